@@ -29,6 +29,7 @@
 #include "decode_mega.cuh"
 #include "f32_stream.cuh"
 #include "mixers.cuh"
+#include "gemm_skinny.cuh"
 #include "gemm_tc.cuh"
 #include "gemv.cuh"
 #include "prefill.cuh"
@@ -59,6 +60,7 @@ static int fail(int code, const char *fmt, ...) {
 
 struct cake_b200_ctx;
 static int wait_loads(cake_b200_ctx *c);
+static int check_waits(cake_b200_ctx *c);
 extern "C" const char *cake_b200_last_error(void) { return g_err; }
 extern "C" const char *cake_b200_version(void) { return "cake_b200 0.1 (sm_100a)"; }
 
@@ -133,6 +135,7 @@ struct cake_b200_ctx {
   cake_b200_sampling sampling{};                   // sampler of the decode graph (kind 0 = greedy)
   size_t d_ids_cap = 0, d_pen_cap = 0;
   uint32_t *h_pin = nullptr;  // pinned staging (tokens)
+  int *wait_err = nullptr;    // pinned, written by a kernel whose bounded wait ran out; reported by the next entry point
   void *h_pin_x = nullptr;
   size_t h_pin_x_cap = 0;
   int nsplit = 1;
@@ -421,6 +424,11 @@ template <typename T> static int set_smem_attrs_T() {
   CU(cudaFuncSetAttribute(gemm_tc_kernel<T, EPI, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<128>::SMEM_BYTES));      \
   CU(cudaFuncSetAttribute(gemm_tc_kernel<T, EPI, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<256>::SMEM_BYTES));      \
   CU(cudaFuncSetAttribute(gemm_tc_kernel<T, EPI, 256, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<256>::SMEM_BYTES));
+#define SETK(EPI)                                                                                                                 \
+  CU(cudaFuncSetAttribute(gemm_skinny_kernel<T, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, SK_SMEM_MAX));                  \
+  CU(cudaFuncSetAttribute(gemm_skinny_kernel<T, EPI>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+  SETK(TCE_PLAIN) SETK(TCE_RESIDUAL) SETK(TCE_SWIGLU) SETK(TCE_RESIDUAL_F32) SETK(TCE_SOFTCAP_F32) SETK(TCE_ACT)
+#undef SETK
   SETT(TCE_PLAIN) SETT(TCE_RESIDUAL) SETT(TCE_SWIGLU) SETT(TCE_RESIDUAL_F32) SETT(TCE_SOFTCAP_F32) SETT(TCE_ACT)
   CU(cudaFuncSetAttribute(attn_window_tc_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, FT_SMEM_BYTES));
   CU(cudaFuncSetAttribute(attn_window_tc_kernel<T>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
@@ -556,6 +564,8 @@ extern "C" int cake_b200_ctx_create(int device, const cake_b200_config *cfg, cak
   CU(cudaMemset(c->d_step, 0, 4));
   CU(cudaMalloc(&c->token_ring, (size_t)TOKEN_RING * 4));
   CU(cudaMallocHost(&c->h_pin, 64 * 4));
+  CU(cudaMallocHost(&c->wait_err, 4));
+  *c->wait_err = 0;
   CU(cudaMalloc(&c->gbar, 16));
   CU(cudaMemset(c->gbar, 0, 16));
   CU(cudaMalloc(&c->tickets, sizeof(unsigned) * (4 * MK_MAX_LAYERS + 4)));
@@ -620,6 +630,7 @@ extern "C" void cake_b200_ctx_destroy(cake_b200_ctx *c) {
   if (c->side_stream) { cudaStreamSynchronize(c->side_stream); cudaStreamDestroy(c->side_stream); }
   if (c->load_stream) { cudaStreamSynchronize(c->load_stream); cudaStreamDestroy(c->load_stream); }
   if (c->h_pin) cudaFreeHost(c->h_pin);
+  if (c->wait_err) cudaFreeHost(c->wait_err);
   if (c->h_pin_x) cudaFreeHost(c->h_pin_x);
   if (c->mk_tab_host) cudaFreeHost(c->mk_tab_host);
   cudaStreamDestroy(c->stream);
@@ -631,7 +642,7 @@ extern "C" int cake_b200_sync(cake_b200_ctx *c) {
   RC(wait_loads(c));
   if (c->load_stream) CU(cudaStreamSynchronize(c->load_stream));
   CU(cudaStreamSynchronize(c->stream));
-  return CAKE_B200_OK;
+  return check_waits(c);
 }
 extern "C" void *cake_b200_stream(cake_b200_ctx *c) { return c ? (void *)c->stream : nullptr; }
 extern "C" int cake_b200_launch_count(cake_b200_ctx *c, uint64_t *k) {
@@ -730,7 +741,13 @@ static int pipe_mark(cake_b200_ctx *c) {  // compute must not start before the u
   c->load_pending = true;
   return CAKE_B200_OK;
 }
+static int check_waits(cake_b200_ctx *c) {
+  if (*(volatile int *)c->wait_err == 0) return CAKE_B200_OK;
+  *(volatile int *)c->wait_err = 0;
+  return fail(CAKE_B200_ECUDA, "a kernel gave up a wait for its own copies: the results of the calls before this one are not valid");
+}
 static int wait_loads(cake_b200_ctx *c) {
+  RC(check_waits(c));
   if (c->load_pending) {
     CU(cudaStreamWaitEvent(c->stream, c->load_done, 0));
     c->load_pending = false;
@@ -1205,8 +1222,9 @@ static int tmap_init() {
   return CAKE_B200_OK;
 }
 // [rows, K] row-major matrix of D -> 2-D map with a (64 x box_rows) box and 128-byte swizzle
-// K: the visible columns (the TMA unit zero-fills past them); ld: the row stride in elements when it is not K
-static int make_tmap(CUtensorMap *m, const void *ptr, uint64_t rows, uint64_t K, int dtype, uint32_t box_rows, uint64_t ld = 0) {
+// K: the visible columns (the TMA unit zero-fills past them); ld: the row stride in elements when it is not K; wide: L2 fetches
+// 256 bytes at a time (a matrix streamed once: the next k-block's half of them is then already there)
+static int make_tmap(CUtensorMap *m, const void *ptr, uint64_t rows, uint64_t K, int dtype, uint32_t box_rows, uint64_t ld = 0, bool wide = false) {
   RC(tmap_init());
   const cuuint64_t gdim[2] = {K, rows};
   const cuuint64_t gstride[1] = {(ld ? ld : K) * 2};
@@ -1214,7 +1232,7 @@ static int make_tmap(CUtensorMap *m, const void *ptr, uint64_t rows, uint64_t K,
   const cuuint32_t estr[2] = {1, 1};
   const CUresult r = g_encode_tiled(m, dtype == CAKE_B200_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2,
                                     const_cast<void *>(ptr), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                                    CU_TENSOR_MAP_SWIZZLE_128B, wide ? CU_TENSOR_MAP_L2_PROMOTION_L2_256B : CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(CAKE_B200_ECUDA, "cuTensorMapEncodeTiled(rows=%llu, K=%llu) -> CUresult %d", (unsigned long long)rows, (unsigned long long)K, (int)r);
   return CAKE_B200_OK;
 }
@@ -1247,10 +1265,44 @@ struct TcExtra {  // optional modes of the tensor-core GEMM (TcParams in gemm_tc
   int b_kwrap = 0, w_cols = 0, w_ld = 0;  // W's k coordinate wraps at b_kwrap; its visible columns / row stride when not K
   int w_rows = 0;                         // W's visible rows when fewer than N (the rest reads as zeros)
   int a_ld = 0;                           // A's row stride in elements when it is a column range of a wider buffer
+  bool w_live = false;                    // W was written by an earlier kernel of the stream (a cache, not a weight)
+  int group_rows = 0;                     // grouped product: no row block holds more rows than this (0 = unknown)
 };
+// gemm_skinny_kernel's shape for a product, or false where gemm_tc_kernel takes it.
+static bool plan_skinny(const cake_b200_ctx *c, int M, int N, int K, const TcExtra &x, SkParams *p, size_t *smem) {
+  static const int max_rows = []() { const char *e = getenv("SK_ROWS"); return e ? atoi(e) : SK_MAX_ROWS; }();
+  if (x.w_live || x.b_kwrap || x.w_cols || x.w_rows || x.w_ld) return false;
+  const int rows = x.tile_group ? x.group_rows : M;
+  if (rows < 1 || rows > max_rows) return false;
+  p->nt = (rows + 15) / 16 * 16;
+  p->m_tiles = x.tile_group ? M / TC_BM : 1;
+  p->m_step = TC_BM;
+  const int tiles = N / SK_BM * p->m_tiles, sms = c->sm_count;
+  // The cut along K: as many CTAs as stay resident at once (up to three per SM), each with at least two k-blocks.  N = 6144, K = 4096, 16
+  // rows: 48 slices x 1 21.9 us, x 2 14.7, x 4 12.7, x 8 11.2 (three per SM) - 15.3 with rings that let only two in, a second wave.
+  p->split = 1;
+  while (p->split < SK_MAX_SPLIT && tiles * p->split * 2 <= 3 * sms && K / TC_BK >= p->split * 4) p->split *= 2;
+  const int per_sm = std::min(3, (tiles * p->split + sms - 1) / sms);
+  const size_t budget = (size_t)(per_sm == 3 && p->split > 1 ? 74 : 110) * 1024 - 1536;
+  p->stages = std::min(SK_MAX_STAGES, std::max(2, (int)(budget / sk_stage_bytes(p->nt))));
+  *smem = sk_smem_bytes(p->nt, p->stages, p->split);
+  return *smem <= SK_SMEM_MAX;
+}
 template <typename T, int EPI>
 static int gemm_tc_T(cake_b200_ctx *c, const void *A, const void *W, const void *bias, const void *res, void *C, int M, int N, int K,
                      int act = -1, int ldc = 0, float cap = 0.f, const TcExtra &x = TcExtra{}) {
+  SkParams sk{};
+  size_t sk_smem = 0;
+  if (plan_skinny(c, M, N, K, x, &sk, &sk_smem)) {
+    sk.bias = bias; sk.residual = res; sk.C = C; sk.M = M; sk.N = N; sk.K = K; sk.ldc = ldc; sk.cap = cap;
+    sk.act = act >= 0 ? act : (c->cfg.use_gelu_mlp ? 1 : 0);
+    sk.tile_group = x.tile_group; sk.row_scale = x.row_scale; sk.err = c->wait_err;
+    CUtensorMap ma, mw;
+    RC(make_tmap(&ma, A, (uint64_t)M, (uint64_t)K, c->cfg.dtype, (uint32_t)sk.nt, (uint64_t)x.a_ld));
+    RC(make_tmap(&mw, W, (uint64_t)N * x.n_groups, (uint64_t)K, c->cfg.dtype, SK_BM, 0, true));
+    return launch_cluster_pdl(c, gemm_skinny_kernel<T, EPI>, dim3((unsigned)(N / SK_BM * sk.m_tiles * sk.split)), dim3(SK_THREADS), sk_smem,
+                              (unsigned)sk.split, mw, ma, sk);
+  }
   // 128 x 256 tiles when N allows and there are enough tiles to fill the chip; CAKE_B200_TC_BN=128 forces the small tile (A/B aid)
   static const int force_bn = []() { const char *e = getenv("CAKE_B200_TC_BN"); return e ? atoi(e) : 0; }();
   const int tiles_m = (M + TC_BM - 1) / TC_BM;
@@ -2495,6 +2547,7 @@ static int run_sub_mixer(cake_b200_ctx *c, const cake_b200_block *b, cake_b200_c
           for (int g = 0; g < G; g++) {
             TcExtra xs;
             xs.w_rows = nk;   // rows past the visible keys read as zeros
+            xs.w_live = true;
             RC((listed_gemm_tc<T, TCE_SOFTCAP_F32>(c, (const T *)w.qh + (size_t)g * grp * n * sp.dim, (const T *)kc->k[slot] + ((size_t)bb * G + g) * kc->cap * sp.dim,
                                                    nullptr, w.scores + (size_t)g * grp * n * kp, grp * n, kp, sp.dim, 0, 0, 0.f, xs)));
           }
@@ -2505,6 +2558,7 @@ static int run_sub_mixer(cake_b200_ctx *c, const cake_b200_block *b, cake_b200_c
             xv.b_kwrap = kp;
             xv.w_cols = nk;
             xv.w_ld = cap_t;
+            xv.w_live = true;
             RC((listed_gemm_tc<T, TCE_PLAIN>(c, (const T *)w.pw + (size_t)g * grp * n * 2 * kp, (const T *)kc->vt[slot] + ((size_t)bb * G + g) * sp.vdim * cap_t, nullptr,
                                              (T *)w.oh + (size_t)g * grp * n * sp.vdim, grp * n, sp.vdim, 2 * kp, 0, 0, 0.f, xv)));
           }
@@ -2933,6 +2987,7 @@ static int enqueue_routed_ff(cake_b200_ctx *c, const cake_b200_block *b, const M
     TcExtra xg;
     xg.tile_group = w.tile_expert;
     xg.n_groups = mo.experts;
+    xg.group_rows = std::min(M, (int)TC_BM);  // a token chooses an expert at most once
     RC((listed_gemm_tc<T, TCE_SWIGLU>(c, w.sorted, b->m_eg, nullptr, w.act, rows, 2 * mo.ff, H, mo.act, mo.ff, mo.limit, xg)));
     RC((listed_gemm_tc<T, TCE_SOFTCAP_F32>(c, w.act, b->m_ed, nullptr, w.y, rows, H, mo.ff, 0, 0, 0.f, xg)));
   } else if (mo.experts) {
@@ -3041,6 +3096,7 @@ static int enqueue_mixer_layers(cake_b200_ctx *c, cake_b200_block *const *blocks
               const T *ct_b = (const T *)kc->v[l] + (size_t)bb * sp.kv_rank * cap_t;
               TcExtra xs;
               xs.w_rows = nk;   // rows past the visible keys read as zeros
+              xs.w_live = true;
               RC((listed_gemm_tc<T, TCE_SOFTCAP_F32>(c, qa_b, kc_b, nullptr, w.scores, rows, kp, Dk, 0, 0, 0.f, xs)));
               mx::LatentSoftmax sm{w.scores, w.pw, nt, sp.heads, kp, pos0 + t0, sp.scale};
               MX(mx::latent_softmax(st, dt, sm, lc));
@@ -3048,6 +3104,7 @@ static int enqueue_mixer_layers(cake_b200_ctx *c, cake_b200_block *const *blocks
               xv.b_kwrap = kp;
               xv.w_cols = nk;
               xv.w_ld = cap_t;
+              xv.w_live = true;
               RC((listed_gemm_tc<T, TCE_PLAIN>(c, w.pw, ct_b, nullptr, (T *)w.lat + ((size_t)bb * S + t0) * sp.heads * sp.kv_rank, rows, sp.kv_rank,
                                                2 * kp, 0, 0, 0.f, xv)));
             }

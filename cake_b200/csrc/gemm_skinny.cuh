@@ -1,0 +1,258 @@
+// gemm_skinny.cuh — linear layers of a few rows (single tokens, batched steps, short prompts) on tcgen05, sm_100a.
+//
+//   C[M,N] = epilogue( A[M,K] · W[N,K]^T )      same operator, epilogues and rounding points as gemm_tc.cuh
+//
+// Bound: the stream of W out of HBM (2 N K bytes; A and C are a few hundred KB).  gemm_tc_kernel gives a product of at most 128
+// rows N / 128 CTAs, each with one 128 x 64 slice of W in flight per k-block: 32 CTAs for a 4096-wide output pull 1.7 TB/s.
+// Here
+//   * W is the MMA's 128-row operand and the rows of A are its columns (16 .. 256 of them, as many as there are, rounded up to 16),
+//     so that a stage carries 16 KB of W and little else, and a product of up to 256 rows reads W once;
+//   * a 128-row slice of W is cut along K between the S CTAs of a cluster, which brings the grid up to the chip; the S fp32 partial
+//     sums meet in shared memory over the cluster (every CTA finishes nt / S of the rows, sums in rank order: deterministic);
+//   * the first ring of W is requested before griddepcontrol.wait: weights don't depend on the kernel in front.
+// One CTA = one slice, 192 threads: warp 0 TMA producer, warp 1 MMA issuer and TMEM owner, warps 2-5 epilogue (thread = row of W).
+#pragma once
+#include "gemm_tc.cuh"
+
+namespace cake {
+
+constexpr int SK_BM = 128, SK_THREADS = 192, SK_MAX_NT = 256, SK_MAX_SPLIT = 8, SK_MAX_STAGES = 8;
+constexpr int SK_MAX_ROWS = 64, SK_SMEM_MAX = 220 * 1024;
+constexpr int SK_W_BYTES = SK_BM * TC_BK * 2;  // 16 KB of W per stage
+__host__ __device__ inline int sk_stage_bytes(int nt) { return SK_W_BYTES + nt * TC_BK * 2; }
+__host__ inline size_t sk_smem_bytes(int nt, int stages, int split) {
+  size_t ring = (size_t)stages * sk_stage_bytes(nt);
+  if (split > 1 && ring < (size_t)nt * SK_BM * 4) ring = (size_t)nt * SK_BM * 4;  // the partial sums take the ring's place
+  return ring + 1024 /*align*/ + 256 /*barriers*/;
+}
+
+struct SkParams {
+  const void *bias, *residual;
+  void *C;
+  int M, N, K, act, ldc;
+  float cap;
+  const int *tile_group;     // as TcParams: rows sorted by group in blocks of TC_BM; a block's first nt rows are all it uses
+  const float *row_scale;
+  int nt;                    // rows of A per tile (a multiple of 16)
+  int m_tiles, m_step;       // row tiles and the distance between their first rows
+  int split, stages;
+  int *err;                  // host-mapped: a wait that ran out
+};
+
+__device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ uint32_t cluster_map(uint32_t saddr, uint32_t rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void st_cluster_f32(uint32_t addr, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+}
+// mbarrier wait with a bound (a try_wait suspends the thread for a while by itself): past it the wait is given up, the error flag
+// is set, and the kernel runs to its end
+constexpr uint32_t MBAR_WAIT_LIMIT = 1u << 25;
+__device__ __forceinline__ bool mbar_wait_lim(uint64_t *bar, uint32_t parity, int *err) {
+  for (uint32_t i = 0; i < MBAR_WAIT_LIMIT; i++) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    if (ok) return true;
+  }
+  if (err) *(volatile int *)err = 1;
+  return false;
+}
+
+// one output of the epilogues that work element by element: fp32 accumulator of (row m, column n) -> C
+template <typename T, int EPI>
+__device__ __forceinline__ void sk_store(const SkParams &p, int m, int n, float v, float bias) {
+  if (EPI == TCE_SOFTCAP_F32) {
+    reinterpret_cast<float *>(p.C)[(size_t)m * p.N + n] = p.cap > 0.f ? p.cap * tanhf(v / p.cap) : v;
+  } else if (EPI == TCE_RESIDUAL_F32) {
+    const size_t o = (size_t)m * p.N + n;
+    const float rs = p.row_scale ? p.row_scale[m] : 1.0f;
+    reinterpret_cast<float *>(p.C)[o] = fmaf(rs, v, reinterpret_cast<const float *>(p.residual)[o]);
+  } else {
+    const size_t o = (size_t)m * (p.ldc ? p.ldc : p.N) + n;
+    float x;
+    if (EPI == TCE_ACT) x = plain_act<T>(v, p.act);
+    else x = rnd<T>(v);
+    if (EPI == TCE_PLAIN && p.bias) x = rnd<T>(x + bias);
+    if (EPI == TCE_RESIDUAL) x += DT<T>::to_f(reinterpret_cast<const T *>(p.residual)[o]);
+    reinterpret_cast<T *>(p.C)[o] = DT<T>::from_f(x);
+  }
+}
+// two rows of A at column n (lanes of a warp = 32 consecutive columns)
+template <typename T, int EPI>
+__device__ __forceinline__ void sk_store2(const SkParams &p, int m, int m_end, int n, float v0, float v1, float bias) {
+  if (EPI == TCE_SWIGLU) {  // columns 2i and 2i + 1 are gate and up: the even lane finishes row m, the odd lane row m + 1
+    const bool odd = (n & 1) != 0;
+    const float got = __shfl_xor_sync(0xffffffffu, odd ? v0 : v1, 1);
+    const float g = odd ? got : v0, u = odd ? v1 : got;
+    const int row = m + (odd ? 1 : 0);
+    if (row < m_end) reinterpret_cast<T *>(p.C)[(size_t)row * (p.ldc ? p.ldc : p.N / 2) + n / 2] = DT<T>::from_f(gated_pair<T>(g, u, p.act, p.cap));
+  } else {
+    if (m < m_end) sk_store<T, EPI>(p, m, n, v0, bias);
+    if (m + 1 < m_end) sk_store<T, EPI>(p, m + 1, n, v1, bias);
+  }
+}
+
+template <typename T, int EPI>
+__global__ void __launch_bounds__(SK_THREADS)
+gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, const SkParams p) {
+  extern __shared__ unsigned char smem_raw_sk[];
+  unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw_sk) + 1023) & ~(uintptr_t)1023);
+  __shared__ uint64_t full[SK_MAX_STAGES], empty[SK_MAX_STAGES], acc_full;
+  __shared__ uint32_t tmem_ptr;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int S = p.split, nt = p.nt, stage_bytes = sk_stage_bytes(nt);
+  const int unit = (int)blockIdx.x / S, rank = (int)blockIdx.x % S;  // the cluster's CTAs are neighbours along x
+  const int mt = unit % p.m_tiles, n0 = (unit / p.m_tiles) * SK_BM;
+  const int m0 = mt * p.m_step, m_end = min(p.M, m0 + nt);
+  const int kblocks = p.K / TC_BK, kb0 = (int)((long)kblocks * rank / S), kb1 = (int)((long)kblocks * (rank + 1) / S), nkb = kb1 - kb0;
+  uint32_t cols = 32;
+  while ((int)cols < nt) cols <<= 1;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < p.stages; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+    mbar_init(&acc_full, 1);
+    mbar_fence_init();
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_ptr)), "r"(cols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  pdl_launch_dependents();
+  const uint32_t tmem = tmem_ptr;
+
+  int group = 0;
+  if (p.tile_group) {  // written by an earlier kernel: nothing can be requested before it has ended
+    pdl_wait();
+    group = p.tile_group[mt];
+  }
+  const bool live = group >= 0;  // cluster-uniform
+
+  if (warp == 0) {
+    if (lane == 0 && live) {
+      asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
+      asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
+      const int wrow = n0 + group * p.N;
+      const int pre = min(nkb, p.stages);
+      for (int i = 0; i < pre; i++) {
+        mbar_arrive_expect_tx(&full[i], (uint32_t)stage_bytes);
+        tma_load_2d(smem + (size_t)i * stage_bytes, &map_w, (kb0 + i) * TC_BK, wrow, &full[i]);
+      }
+      if (!p.tile_group) pdl_wait();
+      for (int i = 0; i < pre; i++) tma_load_2d(smem + (size_t)i * stage_bytes + SK_W_BYTES, &map_a, (kb0 + i) * TC_BK, m0, &full[i]);
+      int s = 0;
+      uint32_t ph = 0;
+      for (int i = pre; i < nkb; i++) {
+        mbar_wait_lim(&empty[s], ph, p.err);
+        unsigned char *st = smem + (size_t)s * stage_bytes;
+        mbar_arrive_expect_tx(&full[s], (uint32_t)stage_bytes);
+        tma_load_2d(st, &map_w, (kb0 + i) * TC_BK, wrow, &full[s]);
+        tma_load_2d(st + SK_W_BYTES, &map_a, (kb0 + i) * TC_BK, m0, &full[s]);
+        if (++s == p.stages) { s = 0; ph ^= 1u; }
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (!p.tile_group) pdl_wait();  // (also keeps the bounded waits from counting the kernel in front)
+    if (lane == 0 && live) {
+      const uint32_t idesc = tc_idesc<T>(nt);
+      int s = 0;
+      uint32_t ph = 0;
+      for (int i = 0; i < nkb; i++) {
+        mbar_wait_lim(&full[s], ph, p.err);
+        tc_fence_after();
+        const unsigned char *st = smem + (size_t)s * stage_bytes;
+        const uint64_t dw = tc_smem_desc(st), da = tc_smem_desc(st + SK_W_BYTES);
+#pragma unroll
+        for (int k = 0; k < TC_BK / 16; k++) tc_mma_f16(tmem, dw + (uint64_t)(k * 2), da + (uint64_t)(k * 2), idesc, (i | k) ? 1u : 0u);
+        tc_commit(&empty[s]);
+        if (++s == p.stages) { s = 0; ph ^= 1u; }
+      }
+      tc_commit(&acc_full);
+    }
+    __syncwarp();
+  }
+  if (!p.tile_group && warp > 1) pdl_wait();  // the residual, and C's previous readers, belong to the kernels in front
+  const int wq = warp & 3;
+  const int n = n0 + wq * 32 + lane;
+  const uint32_t trow = tmem + ((uint32_t)(wq * 32) << 16);
+  float bias = 0.f;
+  if (warp >= 2 && live) {
+    if (EPI == TCE_PLAIN && p.bias) bias = DT<T>::to_f(reinterpret_cast<const T *>(p.bias)[n]);
+    mbar_wait_lim(&acc_full, 0, p.err);
+    tc_fence_after();
+  }
+  if (S == 1) {
+    if (warp >= 2 && live) {
+      for (int c0 = 0; c0 < nt; c0 += 16) {
+        uint32_t r[16];
+        tc_ld16(trow + (uint32_t)c0, r);
+        if (m0 + c0 < m_end) {
+#pragma unroll
+          for (int j = 0; j < 16; j += 2) sk_store2<T, EPI>(p, m0 + c0 + j, m_end, n, __uint_as_float(r[j]), __uint_as_float(r[j + 1]), bias);
+        }
+      }
+    }
+  } else {
+    // partial sums to the CTA that finishes the row: [source rank][row within its share][128 columns] over the drained ring
+    const int share = nt / S;  // even: nt is a multiple of 16 and S at most 8
+    float *recv = reinterpret_cast<float *>(smem);
+    __syncwarp();
+    cluster_arrive();  // every CTA's ring is drained: its MMAs have read all that was loaded
+    cluster_wait();
+    if (warp >= 2 && live) {
+      const uint32_t base = smem_u32(recv) + (uint32_t)(((size_t)rank * share * SK_BM + wq * 32 + lane) * 4);
+      for (int c0 = 0; c0 < nt; c0 += 16) {
+        if (m0 + c0 >= m_end) break;
+        uint32_t r[16];
+        tc_ld16(trow + (uint32_t)c0, r);
+#pragma unroll
+        for (int j = 0; j < 16; j++) {
+          const int c = c0 + j, to = c / share;
+          st_cluster_f32(cluster_map(base + (uint32_t)((c - to * share) * SK_BM * 4), (uint32_t)to), __uint_as_float(r[j]));
+        }
+      }
+    }
+    __syncwarp();
+    cluster_arrive();
+    cluster_wait();
+    if (warp >= 2 && live) {
+      const float *mine = recv + wq * 32 + lane;
+      for (int c = 0; c < share; c += 2) {
+        const int m = m0 + rank * share + c;
+        if (m >= m_end) break;
+        float v0 = 0.f, v1 = 0.f;
+        for (int q = 0; q < S; q++) {
+          v0 += mine[(q * share + c) * SK_BM];
+          v1 += mine[(q * share + c + 1) * SK_BM];
+        }
+        sk_store2<T, EPI>(p, m, m_end, n, v0, v1, bias);
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
+  }
+}
+
+}  // namespace cake
