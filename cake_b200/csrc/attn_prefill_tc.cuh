@@ -7,8 +7,8 @@
 // P_hi + P_lo (two D operands), O accumulated in fp32, rounded once.  What changes is who multiplies: mma.sync tops out
 // near 465 TFLOP/s on this part (ncu r02: HMMA pipe 50 % active at 231 TFLOP/s), a quarter of what tcgen05 delivers.
 //
-// One CTA = one 128-query tile of one head; two CTAs per SM (2 x 256 TMEM columns, 2 x 97 KB shared memory), so one CTA's
-// softmax overlaps the other's MMAs.  192 threads:
+// One CTA = one tile of 128 query rows (the G query heads of one key head x 128 / G tokens) and a range of keys; two CTAs per SM
+// (2 x 256 TMEM columns, 2 x 97 KB shared memory), so one CTA's softmax overlaps the other's MMAs.  192 threads:
 //   warps 0-3  softmax: thread = query row (TMEM lane).  tcgen05.ld of the 128 x 64 S tile, scale + mask + running max /
 //              sum entirely in-thread (no shuffles), P_hi / P_lo packed to D and stored with tcgen05.st over the S tile they
 //              came from (the MMA takes its A operand from TMEM), lazy rescale of O in TMEM (only when the row max grew by
@@ -20,7 +20,7 @@
 //              and O += P_hi V + P_lo V (8 x M128 N128 K16, P from TMEM, V consumed straight from its [key][hd] cache
 //              layout as an MN-major B operand)
 #pragma once
-#include "gemm_tc.cuh"
+#include "gemm_skinny.cuh"
 
 namespace cake {
 
@@ -35,6 +35,13 @@ __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, i
       "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(
           smem_u32(dst)),
       "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *map, int c0, int c1, int c2, int c3, uint64_t *bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];" ::"r"(
+          smem_u32(dst)),
+      "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
       : "memory");
 }
 __device__ __forceinline__ void tc_st32(uint32_t taddr, const uint32_t (&r)[32]) {
@@ -71,11 +78,22 @@ __device__ __forceinline__ uint64_t ft_desc_mn(const void *tile, uint32_t lbo_by
   return addr | ((uint64_t)(lbo_bytes >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
 }
 
+// Query rows of a tile: the G query heads of one key head side by side, row = token * G + head, so that one pass over K and V serves
+// all of them (a step of one token has G rows, not one) and a tile of a causal prompt spans 128 / G tokens: less of its last key
+// tiles is masked.  `splits` CTAs of a cluster cut the tile's keys between them where tiles alone don't fill the chip (few rows on a
+// long context); each finishes 128 / splits of the columns, with the partial sums and the running maxima exchanged over the cluster.
+struct FtParams {
+  void *y;
+  int S, n_heads, n_kv, pos0;
+  int G, tpt, splits_log2;  // query heads per key head, tokens per tile
+  float scale_log2, tau_log2;
+  int *err;
+};
+
 template <typename T>
 __global__ void __launch_bounds__(FT_THREADS, 2)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-                       const __grid_constant__ CUtensorMap map_v, T *__restrict__ y, int S, int n_heads, int n_kv, int pos0,
-                       float scale_log2, float tau_log2) {
+                       const __grid_constant__ CUtensorMap map_v, const FtParams p) {
   extern __shared__ unsigned char ft_smem_raw[];
   unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(ft_smem_raw) + 1023) & ~(uintptr_t)1023);
   unsigned char *q_s = smem;
@@ -87,11 +105,15 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   uint32_t *tmem_ptr = reinterpret_cast<uint32_t *>(bars + 13);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int mt = gridDim.x - 1 - blockIdx.x;  // heavy (late) query tiles first
-  const int h = blockIdx.y, b = blockIdx.z, kvh = h / (n_heads / n_kv);
-  const int m0 = mt * FT_BM;
-  const int kv_end = pos0 + min(S, m0 + FT_BM);  // keys visible to the last query of this tile
-  const int n_tiles = (kv_end + FT_BN - 1) / FT_BN;
+  const int S = p.S, pos0 = p.pos0, G = p.G, tpt = p.tpt, lg = p.splits_log2, splits = 1 << lg;
+  const int rank = (int)blockIdx.x & (splits - 1);                        // the cluster's CTAs are neighbours along x
+  const int mt = (int)(gridDim.x >> lg) - 1 - (int)(blockIdx.x >> lg);  // heavy (late) query tiles first
+  const int kvh = blockIdx.y, b = blockIdx.z, t0 = mt * tpt;
+  const int kv_end = pos0 + min(S, t0 + tpt);  // keys visible to the last query of this tile
+  const int all_tiles = (kv_end + FT_BN - 1) / FT_BN;
+  const int j0 = (all_tiles * rank) >> lg, n_tiles = ((all_tiles * (rank + 1)) >> lg) - j0;  // 0: fewer tiles than CTAs
+  const int rows = G * min(tpt, S - t0);  // of 128
+  const int row = (warp & 3) * 32 + lane, tok = row / G;  // softmax warps: this thread's query row and its token
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < 13; i++) mbar_init(&bars[i], i == 11 ? 128u : 1u);
@@ -109,38 +131,43 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   const uint32_t tmem_base = *tmem_ptr;
   const uint32_t tmem_o = tmem_base + 128u;  // S/P buffer i at columns 64 i
 
+  const uint32_t lane_addr = (uint32_t)((warp & 3) * 32) << 16;
+  const bool busy = warp < 4 && warp * 32 < rows;  // a warp without rows keeps the barriers' counts and computes nothing
+  float m_run = -INFINITY, l_run = 0.f;            // m_run: reference max of the raw scores (unscaled)
+
   if (warp == 4) {
     // ===================== TMA producer ====================================================================
-    if (lane == 0) {
+    if (lane == 0 && n_tiles > 0) {
       asm volatile("prefetch.tensormap [%0];" ::"l"(&map_q) : "memory");
       asm volatile("prefetch.tensormap [%0];" ::"l"(&map_k) : "memory");
       asm volatile("prefetch.tensormap [%0];" ::"l"(&map_v) : "memory");
-      mbar_arrive_expect_tx(q_full, FT_Q_BYTES);
-      tma_load_3d(q_s, &map_q, h * FT_HD, m0, b, q_full);
-      tma_load_3d(q_s + FT_Q_BYTES / 2, &map_q, h * FT_HD + 64, m0, b, q_full);
-      const int slab = b * n_kv + kvh;
+      mbar_arrive_expect_tx(q_full, (uint32_t)(2 * G * tpt * 128));
+      tma_load_4d(q_s, &map_q, 0, kvh * G, t0, b, q_full);
+      tma_load_4d(q_s + FT_Q_BYTES / 2, &map_q, 64, kvh * G, t0, b, q_full);
+      const int slab = b * p.n_kv + kvh;
       for (int j = 0; j < n_tiles; j++) {
         const int st = j & 1;
         const uint32_t eph = (uint32_t)((j >> 1) - 1) & 1u;  // the stage's previous use (tile j-2) has been consumed
         unsigned char *kd = k_s + st * FT_KV_BYTES, *vd = v_s + st * FT_KV_BYTES;
-        if (j >= 2) mbar_wait(&k_empty[st], eph);
+        if (j >= 2) mbar_wait_lim(&k_empty[st], eph, p.err);
         mbar_arrive_expect_tx(&k_full[st], FT_KV_BYTES);
-        tma_load_3d(kd, &map_k, 0, j * FT_BN, slab, &k_full[st]);
-        tma_load_3d(kd + FT_KV_BYTES / 2, &map_k, 64, j * FT_BN, slab, &k_full[st]);
-        if (j >= 2) mbar_wait(&v_empty[st], eph);
+        tma_load_3d(kd, &map_k, 0, (j0 + j) * FT_BN, slab, &k_full[st]);
+        tma_load_3d(kd + FT_KV_BYTES / 2, &map_k, 64, (j0 + j) * FT_BN, slab, &k_full[st]);
+        if (j >= 2) mbar_wait_lim(&v_empty[st], eph, p.err);
         mbar_arrive_expect_tx(&v_full[st], FT_KV_BYTES);
-        tma_load_3d(vd, &map_v, 0, j * FT_BN, slab, &v_full[st]);
-        tma_load_3d(vd + FT_KV_BYTES / 2, &map_v, 64, j * FT_BN, slab, &v_full[st]);
+        tma_load_3d(vd, &map_v, 0, (j0 + j) * FT_BN, slab, &v_full[st]);
+        tma_load_3d(vd + FT_KV_BYTES / 2, &map_v, 64, (j0 + j) * FT_BN, slab, &v_full[st]);
       }
     }
+    __syncwarp();
   } else if (warp == 5) {
     // ===================== MMA issuer (one thread) =========================================================
-    if (lane == 0) {
+    if (lane == 0 && n_tiles > 0) {
       const uint32_t idesc_s = tc_idesc<T>(FT_BN);                   // M128 N64, A and B K-major
       const uint32_t idesc_o = tc_idesc<T>(FT_HD) | (1u << 16);      // M128 N128, A from TMEM, B (V) MN-major
       auto issue_s = [&](int j) {  // S_j = Q K_j^T into S buffer j&1
         const int st = j & 1;
-        mbar_wait(&k_full[st], (uint32_t)(j >> 1) & 1u);
+        mbar_wait_lim(&k_full[st], (uint32_t)(j >> 1) & 1u, p.err);
         tc_fence_after();
         const unsigned char *kt = k_s + st * FT_KV_BYTES;
 #pragma unroll
@@ -152,14 +179,14 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         tc_commit(&k_empty[st]);
         tc_commit(&s_full[st]);
       };
-      mbar_wait(q_full, 0);
+      mbar_wait_lim(q_full, 0, p.err);
       issue_s(0);
       for (int j = 0; j < n_tiles; j++) {
         const int st = j & 1;
         // S of the next tile first: its buffer held P of tile j-1, whose P V is already queued ahead of it in the pipe
         if (j + 1 < n_tiles) issue_s(j + 1);
-        mbar_wait(p_full, (uint32_t)j & 1u);  // P_j in TMEM (over S_j), O rescaled
-        mbar_wait(&v_full[st], (uint32_t)(j >> 1) & 1u);
+        mbar_wait_lim(p_full, (uint32_t)j & 1u, p.err);  // P_j in TMEM (over S_j), O rescaled
+        mbar_wait_lim(&v_full[st], (uint32_t)(j >> 1) & 1u, p.err);
         tc_fence_after();
         const unsigned char *vt = v_s + st * FT_KV_BYTES;
 #pragma unroll
@@ -174,15 +201,19 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         tc_commit(o_full);
       }
     }
-  } else {
-    // ===================== softmax / correction / epilogue (thread = query row) =============================
-    const int row = warp * 32 + lane;
-    const int qp = pos0 + m0 + row;  // absolute position of this row's query
-    const uint32_t lane_addr = (uint32_t)(warp * 32) << 16;
-    float m_run = -INFINITY, l_run = 0.f;  // m_run: reference max of the raw scores (unscaled)
+    __syncwarp();
+  } else if (!busy) {
+    for (int j = 0; j < n_tiles; j++) {  // (P V of tile j-1 first: an arrival for tile j must not join the barrier's previous phase)
+      if (j > 0) mbar_wait_lim(o_full, (uint32_t)(j - 1) & 1u, p.err);
+      mbar_arrive(p_full);
+    }
+    if (n_tiles > 0) mbar_wait_lim(o_full, (uint32_t)(n_tiles - 1) & 1u, p.err);
+  } else if (n_tiles > 0) {
+    // ===================== softmax / correction (thread = query row) ========================================
+    const int qp = pos0 + t0 + tok;  // absolute position of this row's query
     for (int j = 0; j < n_tiles; j++) {
       const uint32_t tmem_sp = tmem_base + lane_addr + (uint32_t)((j & 1) * 64);
-      mbar_wait(&s_full[j & 1], (uint32_t)(j >> 1) & 1u);
+      mbar_wait_lim(&s_full[j & 1], (uint32_t)(j >> 1) & 1u, p.err);
       tc_fence_after();
       float sv[FT_BN];
       {
@@ -196,10 +227,11 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       }
       // causal mask (attention.rs:314-341) — only tiles reaching past the first row's position need the compare
       float mx = -INFINITY;
-      if (j * FT_BN + FT_BN - 1 > pos0 + m0) {
+      const int k0 = (j0 + j) * FT_BN;
+      if (k0 + FT_BN - 1 > pos0 + t0) {
 #pragma unroll
         for (int i = 0; i < FT_BN; i++) {
-          if (j * FT_BN + i > qp) sv[i] = -INFINITY;
+          if (k0 + i > qp) sv[i] = -INFINITY;
           mx = fmaxf(mx, sv[i]);
         }
       } else {
@@ -211,23 +243,24 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       bool resc = false;
       if (j == 0) {
         m_run = mx;
-      } else if ((mx - m_run) * scale_log2 > tau_log2) {
-        fac = ft_ex2((m_run - mx) * scale_log2);
+      } else if ((mx - m_run) * p.scale_log2 > p.tau_log2) {
+        fac = ft_ex2((m_run - mx) * p.scale_log2);
         m_run = mx;
         resc = true;
       }
       // p = exp((s - m) / sqrt(hd)) = 2^(s c - m c), c = log2(e) / sqrt(hd): one FFMA + one MUFU.EX2 per score; 2^-inf = 0 masks
-      const float mc = m_run * scale_log2;
+      // (a row that has seen no key of this CTA's range yet keeps m = -inf: its scores count from 0)
+      const float mc = m_run == -INFINITY ? 0.f : m_run * p.scale_log2;
       float rs = 0.f;
 #pragma unroll
       for (int i = 0; i < FT_BN; i++) {
-        const float p = ft_ex2(fmaf(sv[i], scale_log2, -mc));
-        sv[i] = p;
-        rs += p;
+        const float e = ft_ex2(fmaf(sv[i], p.scale_log2, -mc));
+        sv[i] = e;
+        rs += e;
       }
       l_run = l_run * fac + rs;
       if (j > 0) {
-        mbar_wait(o_full, (uint32_t)(j - 1) & 1u);  // P V of the previous tile is complete: O stable
+        mbar_wait_lim(o_full, (uint32_t)(j - 1) & 1u, p.err);  // P V of the previous tile is complete: O stable
         tc_fence_after();
         if (__any_sync(0xffffffffu, resc)) {
 #pragma unroll 1
@@ -257,23 +290,82 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       tc_fence_before();
       mbar_arrive(p_full);
     }
-    // ---- epilogue: O / l, one rounding to D (attention.rs:346), store (b, s, h, hd) ---------------------------
-    mbar_wait(o_full, (uint32_t)(n_tiles - 1) & 1u);
+    mbar_wait_lim(o_full, (uint32_t)(n_tiles - 1) & 1u, p.err);  // every MMA of this CTA has completed
     tc_fence_after();
-    const int t = m0 + row;
-    const float inv = 1.0f / l_run;
-    T *dst = y + ((size_t)(b * S + t) * n_heads + h) * FT_HD;
+  }
+  // ---- epilogue: O / l, one rounding to D (attention.rs:346), store (b, s, h, hd) ---------------------------
+  T *dst = reinterpret_cast<T *>(p.y) + ((size_t)(b * S + t0 + tok) * p.n_heads + kvh * G + row - tok * G) * FT_HD;
+  if (splits == 1) {
+    if (busy) {
+      const float inv = 1.0f / l_run;
 #pragma unroll 1
-    for (int c0 = 0; c0 < FT_HD; c0 += 32) {
-      uint32_t r[32];
-      tc_ld32(tmem_o + lane_addr + (uint32_t)c0, r);
-      if (t < S) {
-        uint32_t o[16];
+      for (int c0 = 0; c0 < FT_HD; c0 += 32) {
+        uint32_t r[32];
+        tc_ld32(tmem_o + lane_addr + (uint32_t)c0, r);
+        if (row < rows) {
+          uint32_t o[16];
 #pragma unroll
-        for (int i = 0; i < 16; i++) o[i] = pack2x<T>(__uint_as_float(r[2 * i]) * inv, __uint_as_float(r[2 * i + 1]) * inv);
-        uint4 *d4 = reinterpret_cast<uint4 *>(dst + c0);
+          for (int i = 0; i < 16; i++) o[i] = pack2x<T>(__uint_as_float(r[2 * i]) * inv, __uint_as_float(r[2 * i + 1]) * inv);
+          uint4 *d4 = reinterpret_cast<uint4 *>(dst + c0);
 #pragma unroll
-        for (int i = 0; i < 4; i++) d4[i] = make_uint4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
+          for (int i = 0; i < 4; i++) d4[i] = make_uint4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
+        }
+      }
+    }
+  } else {
+    // merge over the cluster.  Q's place: (m, l) of every CTA, [source][row]; K's and V's: partial sums, [source][column of my share][row]
+    const int sp = splits, share = FT_HD >> lg;
+    float2 *ml = reinterpret_cast<float2 *>(q_s);
+    float *part = reinterpret_cast<float *>(k_s);
+    __syncwarp();
+    cluster_arrive();  // every CTA's operands are consumed
+    cluster_wait();
+    if (busy) {
+      const uint32_t a = smem_u32(ml + rank * FT_BM + row);
+      for (int q = 0; q < sp; q++) {
+        const uint32_t to = cluster_map(a, (uint32_t)q);
+        st_cluster_f32(to, m_run);
+        st_cluster_f32(to + 4, l_run);
+      }
+    }
+    __syncwarp();
+    cluster_arrive();
+    cluster_wait();
+    float inv = 0.f;
+    if (busy) {
+      float M = -INFINITY, L = 0.f;
+      for (int q = 0; q < sp; q++) M = fmaxf(M, ml[q * FT_BM + row].x);
+      for (int q = 0; q < sp; q++) {
+        const float2 v = ml[q * FT_BM + row];
+        L += v.x == -INFINITY ? 0.f : v.y * ft_ex2((v.x - M) * p.scale_log2);
+      }
+      inv = 1.0f / L;
+      const float w = m_run == -INFINITY ? 0.f : ft_ex2((m_run - M) * p.scale_log2);
+      const uint32_t a = smem_u32(part + (size_t)rank * share * FT_BM + row);
+#pragma unroll 1
+      for (int c0 = 0; c0 < FT_HD; c0 += 16) {
+        uint32_t r[16];
+        if (n_tiles > 0) tc_ld16(tmem_o + lane_addr + (uint32_t)c0, r);
+        const uint32_t to = cluster_map(a, (uint32_t)(c0 / share)) + (uint32_t)((c0 % share) * FT_BM * 4);  // share is a multiple of 16
+#pragma unroll
+        for (int i = 0; i < 16; i++) st_cluster_f32(to + (uint32_t)(i * FT_BM * 4), n_tiles > 0 ? __uint_as_float(r[i]) * w : 0.f);
+      }
+    }
+    __syncwarp();
+    cluster_arrive();
+    cluster_wait();
+    if (busy && row < rows) {
+      const float *mine = part + row;
+      uint4 *d4 = reinterpret_cast<uint4 *>(dst + rank * share);
+      for (int c0 = 0; c0 < share; c0 += 8) {
+        float v[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) v[i] = 0.f;
+        for (int q = 0; q < sp; q++)
+#pragma unroll
+          for (int i = 0; i < 8; i++) v[i] += mine[(size_t)(q * share + c0 + i) * FT_BM];
+        d4[c0 / 8] = make_uint4(pack2x<T>(v[0] * inv, v[1] * inv), pack2x<T>(v[2] * inv, v[3] * inv), pack2x<T>(v[4] * inv, v[5] * inv),
+                                pack2x<T>(v[6] * inv, v[7] * inv));
       }
     }
   }

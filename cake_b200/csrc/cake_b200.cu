@@ -336,7 +336,7 @@ static int launch_cluster_pdl(cake_b200_ctx *c, void (*kern)(KArgs...), dim3 gri
   at[1].val.clusterDim.y = 1;
   at[1].val.clusterDim.z = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 2;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
   CU(cudaLaunchKernelEx(&cfg, kern, KArgs(args)...));
   if (c->capturing) c->g_kernels++;
   else c->launches++;
@@ -1255,6 +1255,22 @@ static int make_tmap3(CUtensorMap *m, const void *ptr, uint64_t cols, uint64_t r
   return CAKE_B200_OK;
 }
 
+// the query heads of a fused projection [batch][seq][heads + 2 kv heads][hd] as a 4-D map with a (64 x G heads x tokens) box, 128-byte
+// swizzle: a tile's rows come out token by token, the G heads of one key head side by side; tokens past seq read as zeros
+static int make_tmap_q(CUtensorMap *m, const void *ptr, int hd, uint64_t heads, uint64_t seq, uint64_t batch, int dtype, uint32_t G, uint32_t tokens) {
+  RC(tmap_init());
+  const uint64_t row = heads * (uint64_t)hd * 2;
+  const cuuint64_t gdim[4] = {(cuuint64_t)hd, heads, seq, batch};
+  const cuuint64_t gstride[3] = {(cuuint64_t)hd * 2, row, row * seq};
+  const cuuint32_t box[4] = {64u, G, tokens, 1u};
+  const cuuint32_t estr[4] = {1, 1, 1, 1};
+  const CUresult r = g_encode_tiled(m, dtype == CAKE_B200_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4,
+                                    const_cast<void *>(ptr), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(CAKE_B200_ECUDA, "cuTensorMapEncodeTiled(queries: heads=%llu seq=%llu) -> CUresult %d", (unsigned long long)heads, (unsigned long long)seq, (int)r);
+  return CAKE_B200_OK;
+}
+
 static bool tc_gemm_ok(int M, int N, int K) { return M >= 1 && N % TC_BN == 0 && K % TC_BK == 0; }
 
 // C = epi(A[M,K] W[N,K]^T) on the tensor cores (gemm_tc.cuh)
@@ -1428,15 +1444,20 @@ static int enqueue_prefill_layers(cake_b200_ctx *c, cake_b200_block *const *bloc
         static const float fa_tau = []() { const char *e = getenv("CAKE_B200_FA_TAU"); return e ? (float)atof(e) : 5.545f; }();
         if (hd == 128 && !fa_mma) {
           CUtensorMap mq, mk, mv;
-          const uint64_t nqkv_cols = (uint64_t)(f.n_heads + 2 * f.n_kv_heads) * hd;
-          RC(make_tmap3(&mq, c->pf_qkv, nqkv_cols, nqkv_cols, (uint64_t)S, (uint64_t)S, (uint64_t)B, f.dtype, FT_BM));
+          const int G = f.n_heads / f.n_kv_heads, tpt = FT_BM / G;
+          RC(make_tmap_q(&mq, c->pf_qkv, hd, (uint64_t)(f.n_heads + 2 * f.n_kv_heads), (uint64_t)S, (uint64_t)B, f.dtype, (uint32_t)G, (uint32_t)tpt));
           RC(make_tmap3(&mk, (const T *)kc->k[l] + wsoff, (uint64_t)hd, (uint64_t)hd, (uint64_t)(apos0 + S), (uint64_t)kc->cap,
                         (uint64_t)B * f.n_kv_heads, f.dtype, FT_BN));
           RC(make_tmap3(&mv, (const T *)kc->v[l] + wsoff, (uint64_t)hd, (uint64_t)hd, (uint64_t)(apos0 + S), (uint64_t)kc->cap,
                         (uint64_t)B * f.n_kv_heads, f.dtype, FT_BN));
-          dim3 gt((S + FT_BM - 1) / FT_BM, f.n_heads, B);
-          RC(launch_pdl(c, attn_prefill_tc_kernel<T>, gt, dim3(FT_THREADS), (size_t)FT_SMEM_BYTES, mq, mk, mv, (T *)c->pf_y, S, f.n_heads,
-                        f.n_kv_heads, apos0, sc * 1.4426950408889634f, fa_tau * 1.4426950408889634f));
+          // keys cut between the CTAs of a cluster: as many as stay resident (two per SM), with two key tiles each.  One-token steps of 16
+          // sequences at 1000 positions, 32 / 8 heads: 50 us as one row per tile, 32 x 16 CTAs; about 20 packed and cut in two
+          const int tiles = (S + tpt - 1) / tpt, key_tiles = (apos0 + S + FT_BN - 1) / FT_BN;
+          int lg = 0;
+          while (lg < 3 && ((long)tiles * f.n_kv_heads * B << (lg + 1)) <= 2 * c->sm_count && key_tiles >= 4 << lg) lg++;
+          FtParams fp{c->pf_y, S, f.n_heads, f.n_kv_heads, apos0, G, tpt, lg, sc * 1.4426950408889634f, fa_tau * 1.4426950408889634f, c->wait_err};
+          RC(launch_cluster_pdl(c, attn_prefill_tc_kernel<T>, dim3((unsigned)(tiles << lg), f.n_kv_heads, B), dim3(FT_THREADS), (size_t)FT_SMEM_BYTES,
+                                1u << lg, mq, mk, mv, fp));
         } else if (hd == 128)
           RC(launch_pdl(c, attn_prefill_mma_kernel<T, 128>, grid, block, (size_t)4 * FA_BN * 128 * 2, (const T *)c->pf_qkv,
                         (const T *)kc->k[l] + wsoff, (const T *)kc->v[l] + wsoff, (T *)c->pf_y, S, f.n_heads, f.n_kv_heads, kc->cap, apos0, sc));

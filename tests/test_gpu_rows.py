@@ -27,9 +27,38 @@ def test_rows_of_one_sequence_and_of_a_batch(rows, dtype):
     blk = B200Transformer.load(cfg.layer_name(1), ctx)
     x = rand_x((1, rows, cfg.hidden_size), dtype, seed=rows)
     y = blk.forward(ctx.to_device(x), 0, 1, ctx)
+    ctx.sync()
     _check(to_np(y[0]), om.block_forward(1, x[0].float().numpy(), 0, om.new_cache()), dtype, f"prompt of {rows}")
     ctx.cache = Cache(ctx, rows, 8)   # the same rows as one token each of `rows` sequences
-    y = to_np(blk.forward(ctx.to_device(x.transpose(0, 1)), 0, 1, ctx))
+    y = blk.forward(ctx.to_device(x.transpose(0, 1)), 0, 1, ctx)
+    ctx.sync()
+    y = to_np(y)
     for b in range(0, rows, max(1, rows // 4)):
         _check(y[b], om.block_forward(1, x[0, b:b + 1].float().numpy(), 0, om.new_cache()), dtype, f"row {b} of a batch of {rows}")
     ctx.close()
+
+
+@pytest.mark.parametrize("dtype", ["bf16", "f16"])
+@pytest.mark.parametrize("heads,kv,batch,ctx,seq", [
+    (4, 1, 1, 700, 33),    # 4 heads per tile row group, a tile of 32 tokens and one of 1, keys cut over a cluster
+    (4, 1, 3, 300, 1),     # one token each
+    (3, 1, 1, 260, 50),    # 3 heads: 126 of 128 rows of a tile
+    (2, 2, 1, 0, 130),     # one head per key head: tiles of 128 tokens from an empty cache
+    (8, 1, 1, 63, 2),      # 8 heads, the keys end just past a tile
+])
+def test_attention_of_a_portion_on_a_cached_context(heads, kv, batch, ctx, seq, dtype):
+    cfg = medium_config(num_attention_heads=heads, num_key_value_heads=kv, head_dim=128, max_seq_len=1024)
+    sd = checkpoint(cfg, dtype, seed=37)
+    om, dev = O.OracleModel(cfg, sd, dtype), Context(cfg, sd, dtype)
+    blk = B200Transformer.load(cfg.layer_name(0), dev)
+    dev.cache = Cache(dev, batch, ctx + seq + 3)
+    x = rand_x((batch, ctx + seq, cfg.hidden_size), dtype, seed=heads + seq)
+    if ctx:
+        blk.forward(dev.to_device(x[:, :ctx]), 0, 0, dev)
+    y = blk.forward(dev.to_device(x[:, ctx:]), ctx, 0, dev)
+    dev.sync()
+    y = to_np(y)
+    for b in range(batch):
+        ref = om.block_forward(0, x[b].float().numpy(), 0, om.new_cache())[ctx:]
+        _check(y[b], ref, dtype, f"row {b}")
+    dev.close()
