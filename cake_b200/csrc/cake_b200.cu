@@ -1366,6 +1366,8 @@ template <typename T>
 static int rmsnorm_rows_T(cake_b200_ctx *c, const void *x, const void *w, void *out, int M, int n, float eps) {
   const bool al = (((uintptr_t)x | (uintptr_t)w | (uintptr_t)out) & 15) == 0;
   const dim3 g((unsigned)((M + 7) / 8)), blk(256);
+  if (al && n % 8 == 0 && n <= 8192 && M <= 8 * c->sm_count)  // up to eight waves of the warp-per-row kernel's CTAs would be less than one per SM
+    return launch_pdl(c, rmsnorm_row_block_kernel<T>, dim3((unsigned)M), blk, 0, (const T *)x, (const T *)w, (T *)out, n, eps, 1, 0);
   if (al && n == 1024) return launch_pdl(c, rmsnorm_rows_vec_kernel<T, 4>, g, blk, 0, (const T *)x, (const T *)w, (T *)out, M, eps);
   if (al && n == 2048) return launch_pdl(c, rmsnorm_rows_vec_kernel<T, 8>, g, blk, 0, (const T *)x, (const T *)w, (T *)out, M, eps);
   if (al && n == 4096) return launch_pdl(c, rmsnorm_rows_vec_kernel<T, 16>, g, blk, 0, (const T *)x, (const T *)w, (T *)out, M, eps);
@@ -1427,10 +1429,15 @@ static int enqueue_prefill_layers(cake_b200_ctx *c, cake_b200_block *const *bloc
       const int rope_on = b->use_rope ? 1 : 0;
       {
         const long items = (long)M * (f.n_heads + 2 * f.n_kv_heads);
-        if (hd == 128 && c->rot == 128 && ((uintptr_t)c->cos_t & 3) == 0)  // full rotary on 128-wide heads: token-per-warp vector kernel
-          RC(launch_pdl(c, rope_append_vec_kernel<T>, dim3((unsigned)((M + 3) / 4)), dim3(128), 0, (T *)c->pf_qkv, (T *)kc->k[l], (T *)kc->v[l],
+        if (hd == 128 && c->rot == 128 && ((uintptr_t)c->cos_t & 3) == 0) {  // full rotary on 128-wide heads: token-per-warp vector kernel
+          // warps per token: one where the tokens fill the chip (cos / sin read once), else up to one per four heads (16 tokens of 48
+          // heads: 16 us with one warp each, 4 CTAs)
+          int parts = 1;
+          while (parts * 4 < f.n_heads + 2 * f.n_kv_heads && (long)M * parts < 4l * c->sm_count) parts++;
+          RC(launch_pdl(c, rope_append_vec_kernel<T>, dim3((unsigned)(((long)M * parts + 3) / 4)), dim3(128), 0, (T *)c->pf_qkv, (T *)kc->k[l], (T *)kc->v[l],
                         (const T *)c->cos_t, (const T *)c->sin_t, (const T *)qn, (const T *)kn, B, S, f.n_heads, f.n_kv_heads, kc->cap, pos0,
-                        f.rms_eps, rope_on));
+                        f.rms_eps, rope_on, parts));
+        }
         else
         RC(launch_pdl(c, rope_append_kernel<T>, dim3((unsigned)((items + 3) / 4)), dim3(128), (size_t)4 * hd * 4,
                       (T *)c->pf_qkv, (T *)kc->k[l], (T *)kc->v[l], (const T *)c->cos_t, (const T *)c->sin_t,

@@ -80,42 +80,31 @@ __device__ __forceinline__ void mbar_wait_lim(uint64_t *bar, uint32_t parity, in
   if (left == 0) *(volatile int *)err = 1;
 }
 
-// one output of the epilogues that work element by element: fp32 accumulator of (row m, column n) -> C
+// what an epilogue reads beside the sums, for row m of A at column n (rows past m_end: nothing)
 template <typename T, int EPI>
-__device__ __forceinline__ void sk_store(const SkParams &p, int m, int n, float v, float bias) {
+__device__ __forceinline__ float sk_residual(const SkParams &p, int m, int m_end, int n) {
+  if (m >= m_end) return 0.f;
+  if (EPI == TCE_RESIDUAL) return DT<T>::to_f(reinterpret_cast<const T *>(p.residual)[(size_t)m * (p.ldc ? p.ldc : p.N) + n]);
+  if (EPI == TCE_RESIDUAL_F32) return reinterpret_cast<const float *>(p.residual)[(size_t)m * p.N + n];
+  return 0.f;
+}
+template <typename T, int EPI>
+__device__ __forceinline__ void sk_store(const SkParams &p, int m, int m_end, int n, float v, float bias, float res) {
+  if (m >= m_end) return;
   if (EPI == TCE_SOFTCAP_F32) {
     reinterpret_cast<float *>(p.C)[(size_t)m * p.N + n] = p.cap > 0.f ? p.cap * tanhf(v / p.cap) : v;
   } else if (EPI == TCE_RESIDUAL_F32) {
-    const size_t o = (size_t)m * p.N + n;
-    const float rs = p.row_scale ? p.row_scale[m] : 1.0f;
-    reinterpret_cast<float *>(p.C)[o] = fmaf(rs, v, reinterpret_cast<const float *>(p.residual)[o]);
+    reinterpret_cast<float *>(p.C)[(size_t)m * p.N + n] = fmaf(p.row_scale ? p.row_scale[m] : 1.0f, v, res);
   } else {
-    const size_t o = (size_t)m * (p.ldc ? p.ldc : p.N) + n;
-    float x;
-    if (EPI == TCE_ACT) x = plain_act<T>(v, p.act);
-    else x = rnd<T>(v);
+    float x = EPI == TCE_ACT ? plain_act<T>(v, p.act) : rnd<T>(v);
     if (EPI == TCE_PLAIN && p.bias) x = rnd<T>(x + bias);
-    if (EPI == TCE_RESIDUAL) x += DT<T>::to_f(reinterpret_cast<const T *>(p.residual)[o]);
-    reinterpret_cast<T *>(p.C)[o] = DT<T>::from_f(x);
-  }
-}
-// two rows of A at column n (lanes of a warp = 32 consecutive columns)
-template <typename T, int EPI>
-__device__ __forceinline__ void sk_store2(const SkParams &p, int m, int m_end, int n, float v0, float v1, float bias) {
-  if (EPI == TCE_SWIGLU) {  // columns 2i and 2i + 1 are gate and up: the even lane finishes row m, the odd lane row m + 1
-    const bool odd = (n & 1) != 0;
-    const float got = __shfl_xor_sync(0xffffffffu, odd ? v0 : v1, 1);
-    const float g = odd ? got : v0, u = odd ? v1 : got;
-    const int row = m + (odd ? 1 : 0);
-    if (row < m_end) reinterpret_cast<T *>(p.C)[(size_t)row * (p.ldc ? p.ldc : p.N / 2) + n / 2] = DT<T>::from_f(gated_pair<T>(g, u, p.act, p.cap));
-  } else {
-    if (m < m_end) sk_store<T, EPI>(p, m, n, v0, bias);
-    if (m + 1 < m_end) sk_store<T, EPI>(p, m + 1, n, v1, bias);
+    if (EPI == TCE_RESIDUAL) x += res;
+    reinterpret_cast<T *>(p.C)[(size_t)m * (p.ldc ? p.ldc : p.N) + n] = DT<T>::from_f(x);
   }
 }
 
 template <typename T, int EPI>
-__global__ void __launch_bounds__(SK_THREADS)
+__global__ void __launch_bounds__(SK_THREADS, 2)
 gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, const SkParams p) {
   extern __shared__ unsigned char smem_raw_sk[];
   unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw_sk) + 1023) & ~(uintptr_t)1023);
@@ -200,57 +189,77 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   const int wq = warp & 3;
   const int n = n0 + wq * 32 + lane;
   const uint32_t trow = tmem + ((uint32_t)(wq * 32) << 16);
-  float bias = 0.f;
+  float bias = 0.f, res0 = 0.f, res1 = 0.f;
+  const int share = nt / S, f0 = m0 + rank * share;  // rows this CTA finishes: all of the tile, or its share (an even number) of them
+  float *recv = reinterpret_cast<float *>(smem);     // sums on their way, over the drained ring: [source rank][row within the share][128 columns]
   if (warp >= 2 && live) {
     if (EPI == TCE_PLAIN && p.bias) bias = DT<T>::to_f(reinterpret_cast<const T *>(p.bias)[n]);
+    res0 = sk_residual<T, EPI>(p, f0, m_end, n);
+    res1 = sk_residual<T, EPI>(p, f0 + 1, m_end, n);
     mbar_wait_lim(&acc_full, 0, p.err);
     tc_fence_after();
   }
-  if (S == 1) {
-    if (warp >= 2 && live) {
-      for (int c0 = 0; c0 < nt; c0 += 16) {
-        uint32_t r[16];
-        tc_ld16(trow + (uint32_t)c0, r);
-        if (m0 + c0 < m_end) {
-#pragma unroll
-          for (int j = 0; j < 16; j += 2) sk_store2<T, EPI>(p, m0 + c0 + j, m_end, n, __uint_as_float(r[j]), __uint_as_float(r[j + 1]), bias);
-        }
-      }
-    }
-  } else {
-    // partial sums to the CTA that finishes the row: [source rank][row within its share][128 columns] over the drained ring
-    const int share = nt / S;  // even: nt is a multiple of 16 and S at most 8
-    float *recv = reinterpret_cast<float *>(smem);
+  if (S > 1) {
     __syncwarp();
     cluster_arrive();  // every CTA's ring is drained: its MMAs have read all that was loaded
     cluster_wait();
     if (warp >= 2 && live) {
       const uint32_t base = smem_u32(recv) + (uint32_t)(((size_t)rank * share * SK_BM + wq * 32 + lane) * 4);
-      for (int c0 = 0; c0 < nt; c0 += 16) {
-        if (m0 + c0 >= m_end) break;
+      int to = 0, off = 0;  // row of A -> CTA and place within its share
+      uint32_t dst = cluster_map(base, 0u);
+#pragma unroll 1
+      for (int c0 = 0; c0 < nt && m0 + c0 < m_end; c0 += 16) {
         uint32_t r[16];
         tc_ld16(trow + (uint32_t)c0, r);
 #pragma unroll
         for (int j = 0; j < 16; j++) {
-          const int c = c0 + j, to = c / share;
-          st_cluster_f32(cluster_map(base + (uint32_t)((c - to * share) * SK_BM * 4), (uint32_t)to), __uint_as_float(r[j]));
+          st_cluster_f32(dst, __uint_as_float(r[j]));
+          dst += SK_BM * 4;
+          if (++off == share && to + 1 < S) { off = 0; dst = cluster_map(base, (uint32_t)++to); }
         }
       }
     }
     __syncwarp();
     cluster_arrive();
     cluster_wait();
-    if (warp >= 2 && live) {
-      const float *mine = recv + wq * 32 + lane;
-      for (int c = 0; c < share; c += 2) {
-        const int m = m0 + rank * share + c;
+  }
+  // The last pass is a loop of one pair of rows, not straight-line code: a kernel of a few microseconds runs its epilogue once, and
+  // unrolled over 16 rows it waited for its own instructions (233 -> 315 us for four Nigenex layers).  The residual of the next pair is
+  // requested before this pair is stored: C may be the residual's own buffer.
+  if (warp >= 2 && live) {
+    const int step = S == 1 ? 16 : share;
+    float *mine = recv + wq * 32 + lane;
+#pragma unroll 1
+    for (int c0 = 0; c0 < share && f0 + c0 < m_end; c0 += step) {
+      if (S == 1) {  // through shared memory too: the thread's own column, 16 rows at a time
+        uint32_t r[16];
+        tc_ld16(trow + (uint32_t)c0, r);
+#pragma unroll
+        for (int j = 0; j < 16; j++) mine[j * SK_BM] = __uint_as_float(r[j]);
+      }
+#pragma unroll 1
+      for (int c = 0; c < step; c += 2) {
+        const int m = f0 + c0 + c;
         if (m >= m_end) break;
         float v0 = 0.f, v1 = 0.f;
+#pragma unroll 2
         for (int q = 0; q < S; q++) {
           v0 += mine[(q * share + c) * SK_BM];
           v1 += mine[(q * share + c + 1) * SK_BM];
         }
-        sk_store2<T, EPI>(p, m, m_end, n, v0, v1, bias);
+        if (EPI == TCE_SWIGLU) {  // columns 2i and 2i + 1 are gate and up: the even lane finishes row m, the odd lane row m + 1
+          const bool odd = (n & 1) != 0;
+          const float got = __shfl_xor_sync(0xffffffffu, odd ? v0 : v1, 1);
+          const float g = odd ? got : v0, u = odd ? v1 : got;
+          const int row = m + (odd ? 1 : 0);
+          if (row < m_end) reinterpret_cast<T *>(p.C)[(size_t)row * (p.ldc ? p.ldc : p.N / 2) + n / 2] = DT<T>::from_f(gated_pair<T>(g, u, p.act, p.cap));
+        } else {
+          const float n0r = sk_residual<T, EPI>(p, m + 2, m_end, n), n1r = sk_residual<T, EPI>(p, m + 3, m_end, n);
+          sk_store<T, EPI>(p, m, m_end, n, v0, bias, res0);
+          sk_store<T, EPI>(p, m + 1, m_end, n, v1, bias, res1);
+          res0 = n0r;
+          res1 = n1r;
+        }
       }
     }
   }
