@@ -144,6 +144,10 @@ struct cake_b200_ctx {
   void *pf_h = nullptr, *pf_qkv = nullptr, *pf_y = nullptr, *pf_x1 = nullptr, *pf_gu = nullptr, *pf_mm = nullptr;
   void *io_x = nullptr;
   size_t io_x_cap = 0;
+  // head of a batch: its logits where the caller keeps none, its tokens
+  void *hd_logits = nullptr;
+  size_t hd_logits_rows = 0;
+  uint32_t *hd_tokens = nullptr;
   // layer-list blocks (fp32 residual stream): operands of the matrix products in D, sized on demand
   size_t sp_rows = 0, sp_in_cols = 0, sp_out_cols = 0, sp_logit_rows = 0;
   void *sp_h = nullptr, *sp_hs = nullptr, *sp_in = nullptr, *sp_a = nullptr, *sp_hn = nullptr;
@@ -610,7 +614,7 @@ extern "C" void cake_b200_ctx_destroy(cake_b200_ctx *c) {
                   c->ws_acc, c->part_val, c->part_idx, c->d_step, c->attn_counters, c->argmax_counter, c->d_token,
                   c->token_ring, c->d_ids, c->d_pen, c->pf_h, c->pf_qkv, c->pf_y, c->pf_x1, c->pf_gu, c->pf_mm, c->io_x,
                   c->gbar, c->mk_tab_dev, c->g_tab_dev, c->tickets, c->ring_seq, c->inbox, c->step_trace, c->trace,
-                  c->samp_p, c->samp_noise, c->x0, c->sp_h, c->sp_hs, c->sp_in, c->sp_a, c->sp_hn, c->sp_logits, c->sp_rows_idx, c->mx_ws};
+                  c->samp_p, c->samp_noise, c->hd_logits, c->hd_tokens, c->x0, c->sp_h, c->sp_hs, c->sp_in, c->sp_a, c->sp_hn, c->sp_logits, c->sp_rows_idx, c->mx_ws};
   for (void *b : bufs)
     if (b) cudaFree(b);
   if (c->bigram) cudaFree(c->bigram);
@@ -3529,6 +3533,37 @@ extern "C" int cake_b200_logits(cake_b200_ctx *c, const void *x_dev, int batch, 
   RC(wait_loads(c));
   if (c->cfg.layer_list) return listed_logits_last(c, x_dev, batch, seq, logits_dev, argmax_host);
   const size_t H = c->cfg.hidden, V = c->cfg.vocab, es = c->es;
+  if (batch > 1 && batch <= SK_MAX_ROWS && tc_gemm_ok(batch, (int)V, (int)H) && H <= 8192 && (((uintptr_t)x_dev | (uintptr_t)c->ln_f) & 15) == 0) {
+    // several rows: norm, then one product that reads lm_head once (a GEMV per row read it `batch` times: 2750 us for 16 rows of 128256 x
+    // 4096, 158 us of it for the bytes)
+    RC(pf_reserve(c, (size_t)batch));
+    if (!logits_dev && (size_t)batch > c->hd_logits_rows) {
+      CU(cudaStreamSynchronize(c->stream));
+      if (c->hd_logits) cudaFree(c->hd_logits);
+      c->hd_logits = nullptr; c->hd_logits_rows = 0;
+      CU(cudaMalloc(&c->hd_logits, (size_t)batch * V * es));
+      c->hd_logits_rows = batch;
+    }
+    if (!c->hd_tokens) CU(cudaMalloc(&c->hd_tokens, SK_MAX_ROWS * 4));
+    void *lo = logits_dev ? logits_dev : c->hd_logits;
+    RC(DISPATCH_T(c->cfg.dtype, T_LAMBDA {
+      typedef typename decltype(tag_)::type T;
+      RC(launch_pdl(c, rmsnorm_row_block_kernel<T>, dim3((unsigned)batch), dim3(256), 0, (const T *)x_dev, (const T *)c->ln_f, (T *)c->pf_h, (int)H,
+                    c->cfg.rms_eps, seq, seq - 1));  // the last position of every batch row (text_model.rs:342-346)
+      RC((gemm_tc_T<T, TCE_PLAIN>(c, c->pf_h, c->lm_head, nullptr, nullptr, lo, batch, (int)V, (int)H)));
+      if (argmax_host) {
+        argmax_kernel<T><<<batch, 1024, 0, c->stream>>>((const T *)lo, (int)V, c->hd_tokens);
+        c->launches++;
+      }
+      return CAKE_B200_OK;
+    }));
+    if (argmax_host) {
+      CU(cudaMemcpyAsync(c->h_pin, c->hd_tokens, (size_t)batch * 4, cudaMemcpyDeviceToHost, c->stream));
+      CU(cudaStreamSynchronize(c->stream));
+      for (int b = 0; b < batch; b++) argmax_host[b] = c->h_pin[b];
+    }
+    return CAKE_B200_OK;
+  }
   for (int b = 0; b < batch; b++) {
     const char *row = (const char *)x_dev + ((size_t)b * seq + (seq - 1)) * H * es;  // text_model.rs:342-346
     void *lo = logits_dev ? (char *)logits_dev + (size_t)b * V * es : c->logits;

@@ -1,7 +1,11 @@
 """Steps and prompts of a few rows: the sizes at which the products of a block change their kernel or their tiling, against the
 oracle with the bars of test_gpu_parity.py (same rounding points, fp32 sums in another order)."""
+import ctypes
+
+import numpy as np
 import pytest
 
+from cake_b200.capi import check, lib, ptr
 from cake_b200.model import B200Transformer, Cache, Context
 from oracle import oracle as O
 from tests.util import checkpoint, max_ulp_err, mean_ulp_err, medium_config, rand_x, to_np
@@ -62,3 +66,28 @@ def test_attention_of_a_portion_on_a_cached_context(heads, kv, batch, ctx, seq, 
         ref = om.block_forward(0, x[b].float().numpy(), 0, om.new_cache())[ctx:]
         _check(y[b], ref, dtype, f"row {b}")
     dev.close()
+
+
+@pytest.mark.parametrize("dtype", ["bf16", "f16"])
+@pytest.mark.parametrize("batch,seq,vocab", [(2, 1, 1024), (17, 3, 1024), (64, 1, 1152), (3, 2, 1000)])   # 1000: no tiles, row by row
+def test_head_of_a_batch(batch, seq, vocab, dtype):
+    """Logits of every row's last position against the head of each row alone (another kernel, the same rounding points) and the oracle's
+    first maximum; without a logits buffer the tokens are the same."""
+    cfg = medium_config(vocab_size=vocab)
+    sd = checkpoint(cfg, dtype, seed=41, peaked=True)
+    ctx = Context(cfg, sd, dtype)
+    p = cfg.model_prefix
+    head = [sd[p + ".embed_tokens.weight"], sd[p + ".norm.weight"], sd["lm_head.weight"]]
+    check(lib().cake_b200_head_load(ctx.h, *[ptr(t) for t in head]))
+    x = ctx.to_device(rand_x((batch, seq, cfg.hidden_size), dtype, seed=batch))
+    both, alone = ctx.empty(batch, vocab), ctx.empty(batch, vocab)
+    tok, tok2 = (ctypes.c_uint32 * batch)(), (ctypes.c_uint32 * batch)()
+    check(lib().cake_b200_logits(ctx.h, ptr(x), batch, seq, ptr(both), tok))
+    check(lib().cake_b200_logits(ctx.h, ptr(x), batch, seq, None, tok2))
+    for b in range(batch):
+        check(lib().cake_b200_logits(ctx.h, ptr(x[b]), 1, seq, ptr(alone[b]), None))
+    ctx.sync()
+    _check(to_np(both), to_np(alone), dtype, "logits")
+    first = np.argmax(to_np(both), axis=1)   # numpy's argmax is the first maximum
+    assert list(tok) == list(first) == list(tok2)
+    ctx.close()
