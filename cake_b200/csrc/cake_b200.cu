@@ -440,6 +440,7 @@ template <typename T> static int set_smem_attrs_T() {
   SETW(32) SETW(64) SETW(96) SETW(128)
 #undef SETW
 #undef SETT
+  CU(cudaFuncSetAttribute(sample_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, SAMPLE_SMEM_MAX));
   return CAKE_B200_OK;
 }
 
@@ -3608,6 +3609,14 @@ static int samp_reserve(cake_b200_ctx *c) {
 }
 static SampleArgs to_args(const cake_b200_sampling &s) { return SampleArgs{s.kind, s.top_k, s.temperature, s.top_p, (unsigned long long)s.seed}; }
 
+template <typename T>
+static int launch_sampler(cake_b200_ctx *c, const T *logits, const cake_b200_sampling &s, const float *noise, const int *d_step, int step_bias, uint32_t *ring, int ring_cap) {
+  const size_t part = sample_smem(c->cfg.vocab);
+  const bool in_smem = part <= (size_t)SAMPLE_SMEM_MAX;
+  return launch_pdl(c, sample_kernel<T>, dim3(SAMPLE_CTAS), dim3(SAMPLE_THREADS), in_smem ? part : 0, logits, c->cfg.vocab, to_args(s), c->samp_p,
+                    in_smem ? 1 : 0, noise, d_step, step_bias, c->d_token, ring, ring_cap);
+}
+
 static int apply_repeat_penalty(cake_b200_ctx *c, void *logits_dev, float penalty, const uint32_t *ctx_tokens_host, int n_tokens) {
   // text_model.rs:66-72: de-duplicate, keeping first occurrences
   std::vector<uint32_t> uniq;
@@ -3617,6 +3626,15 @@ static int apply_repeat_penalty(cake_b200_ctx *c, void *logits_dev, float penalt
     if (!dup) uniq.push_back(ctx_tokens_host[i]);
   }
   if (uniq.empty() || penalty == 1.0f) return CAKE_B200_OK;
+  if (uniq.size() <= (size_t)PENALTY_INLINE) {
+    PenaltyTokens pt;
+    memcpy(pt.id, uniq.data(), uniq.size() * 4);
+    return DISPATCH_T(c->cfg.dtype, T_LAMBDA {
+      typedef typename decltype(tag_)::type T;
+      return launch_pdl(c, repeat_penalty_inline_kernel<T>, dim3((unsigned)((uniq.size() + 127) / 128)), dim3(128), 0, (T *)logits_dev, c->cfg.vocab, penalty,
+                        pt, (int)uniq.size());
+    });
+  }
   if (uniq.size() > c->d_pen_cap) {
     CU(cudaStreamSynchronize(c->stream));
     if (c->d_pen) cudaFree(c->d_pen);
@@ -3650,14 +3668,10 @@ extern "C" int cake_b200_sample(cake_b200_ctx *c, void *logits_dev, const cake_b
     CU(cudaStreamSynchronize(c->stream));
     noise_dev = c->samp_noise;
   }
-  set_int_kernel<<<1, 1, 0, c->stream>>>((int *)(c->samp_p + c->cfg.vocab), (int)(step & 0x7fffffff));  // the draw's counter
   RC(DISPATCH_T(c->cfg.dtype, T_LAMBDA {
     typedef typename decltype(tag_)::type T;
-    sample_kernel<T><<<1, SAMPLE_THREADS, 0, c->stream>>>((const T *)logits_dev, c->cfg.vocab, to_args(*s), c->samp_p, noise_dev,
-                                                          (const int *)(c->samp_p + c->cfg.vocab), 0, c->d_token, nullptr, 1);
-    return CAKE_B200_OK;
+    return launch_sampler<T>(c, (const T *)logits_dev, *s, noise_dev, (const int *)nullptr, (int)(step & 0x7fffffff), (uint32_t *)nullptr, 1);
   }));
-  c->launches += 2;
   CU(cudaGetLastError());
   CU(cudaMemcpyAsync(c->h_pin, c->d_token, 4, cudaMemcpyDeviceToHost, c->stream));
   CU(cudaStreamSynchronize(c->stream));
@@ -3810,8 +3824,7 @@ extern "C" int cake_b200_decode_build(cake_b200_ctx *c, cake_b200_block *const *
           // (256 KB, L2-hot) and overwrites d_token / the ring slot of this step; the step counter was already advanced
           RC(DISPATCH_T(c->cfg.dtype, T_LAMBDA {
             typedef typename decltype(tag_)::type T;
-            return launch_pdl(c, sample_kernel<T>, dim3(1), dim3(SAMPLE_THREADS), 0, (const T *)c->logits, c->cfg.vocab, to_args(c->sampling),
-                              c->samp_p, (const float *)nullptr, (const int *)c->d_step, -1, c->d_token, c->token_ring, (int)TOKEN_RING);
+            return launch_sampler<T>(c, (const T *)c->logits, c->sampling, nullptr, (const int *)c->d_step, -1, c->token_ring, (int)TOKEN_RING);
           }));
         }
       } else {

@@ -489,11 +489,11 @@ __global__ void __launch_bounds__(1024) argmax_kernel(const T *__restrict__ logi
 }
 
 // ---- repeat penalty (text_model.rs:60-99) on device, arithmetic in D; tokens are pre-deduplicated --
+// a step's tokens travel with the launch where they fit (a copy to the device and a wait for it took longer than the kernel)
+constexpr int PENALTY_INLINE = 512;
+struct PenaltyTokens { uint32_t id[PENALTY_INLINE]; };
 template <typename T>
-__global__ void repeat_penalty_kernel(T *logits, int V, float penalty, const uint32_t *toks, int n) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const uint32_t t = toks[i];
+__device__ __forceinline__ void penalise(T *logits, int V, float penalty, uint32_t t) {
   if (t >= (uint32_t)V) return;
   const float recip = rnd<T>(1.0f / penalty), pen = rnd<T>(penalty);
   const float sel = DT<T>::to_f(logits[t]);
@@ -501,6 +501,18 @@ __global__ void repeat_penalty_kernel(T *logits, int V, float penalty, const uin
   const float penalized = rnd<T>(sel * mult);
   const float delta = rnd<T>(penalized - sel);
   logits[t] = DT<T>::from_f(sel + delta);
+}
+template <typename T>
+__global__ void repeat_penalty_kernel(T *logits, int V, float penalty, const uint32_t *toks, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) penalise<T>(logits, V, penalty, toks[i]);
+}
+template <typename T>
+__global__ void repeat_penalty_inline_kernel(T *logits, int V, float penalty, const __grid_constant__ PenaltyTokens toks, int n) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) penalise<T>(logits, V, penalty, toks.id[i]);
 }
 
 // ---- synthetic cache fill (bench only) ------------------------------------------------------------

@@ -1,6 +1,6 @@
 // sample.cuh — device-side token samplers: the tail of TextModelBase::next_token
 // (text_model.rs:102-118 create_logits_processor, :429-460 the sampling step) without shipping the logits to the
-// host: one CTA reads the (vocab,) logits of the last position from L2/HBM and writes 4 bytes.
+// host: one cluster of SAMPLE_CTAS CTAs reads the (vocab,) logits of the last position from L2/HBM and writes 4 bytes.
 //
 // The arithmetic behind `LogitsProcessor::sample` lives in candle-transformers 0.9.2 (generation/mod.rs) and
 // candle-nn 0.9.2 (sampling.rs), crates that are not vendored under /root/reference; restated from their published
@@ -20,12 +20,15 @@
 // implementation-defined there; here the candidates are ordered by probability (descending, ties by lower id).
 // Everything is deterministic: reductions and scans use fixed trees, never floating-point atomics.
 #pragma once
-#include "common.cuh"
+#include "gemm_skinny.cuh"
 
 namespace cake {
 
 enum SampleKind { SAMPLE_ARGMAX = 0, SAMPLE_ALL = 1, SAMPLE_TOPK = 2, SAMPLE_TOPP = 3, SAMPLE_TOPK_TOPP = 4, SAMPLE_GUMBEL = 5 };
-constexpr int SAMPLE_THREADS = 1024;
+constexpr int SAMPLE_THREADS = 1024, SAMPLE_CTAS = 8;
+constexpr int SAMPLE_SMEM_MAX = 208 * 1024;  // logits and probabilities of a CTA's part of the vocabulary; those of a larger part stay in global memory
+__host__ __device__ inline int sample_per_thread(int V) { return ((V + SAMPLE_CTAS * SAMPLE_THREADS - 1) / (SAMPLE_CTAS * SAMPLE_THREADS)) | 1; }
+__host__ inline size_t sample_smem(int V) { return (size_t)sample_per_thread(V) * SAMPLE_THREADS * 6; }  // odd: a thread's run of entries has no bank conflicts
 constexpr int SAMPLE_MAX_K = 1024;   // candidates sorted in shared memory (top-k requests above this are refused by the host)
 
 struct SampleArgs {
@@ -53,256 +56,301 @@ __device__ __forceinline__ float sample_uniform(const SampleArgs &s, unsigned st
   return u01(w);
 }
 
-// ---- block-wide helpers over SAMPLE_THREADS threads, fixed reduction order --------------------------------------
-__device__ __forceinline__ float block_sum(float v, float *sh) {
-  v = warp_sum(v);
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
-  __syncthreads();
-  float t = (threadIdx.x < 32) ? sh[threadIdx.x] : 0.f;
-  if (threadIdx.x < 32) t = warp_sum(t);
-  if (threadIdx.x == 0) sh[32] = t;
-  __syncthreads();
-  const float r = sh[32];
-  __syncthreads();
-  return r;
-}
-__device__ __forceinline__ float block_max(float v, float *sh) {
-  v = warp_max(v);
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
-  __syncthreads();
-  float t = (threadIdx.x < 32) ? sh[threadIdx.x] : -INFINITY;
-  if (threadIdx.x < 32) t = warp_max(t);
-  if (threadIdx.x == 0) sh[32] = t;
-  __syncthreads();
-  const float r = sh[32];
-  __syncthreads();
-  return r;
-}
-__device__ __forceinline__ int block_sum_i(int v, int *sh) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
-  __syncthreads();
-  int t = (threadIdx.x < 32) ? sh[threadIdx.x] : 0;
-  if (threadIdx.x < 32) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-  }
-  if (threadIdx.x == 0) sh[32] = t;
-  __syncthreads();
-  const int r = sh[32];
-  __syncthreads();
-  return r;
-}
-__device__ __forceinline__ int block_min_i(int v, int *sh) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = min(v, __shfl_xor_sync(0xffffffffu, v, o));
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
-  __syncthreads();
-  int t = (threadIdx.x < 32) ? sh[threadIdx.x] : 0x7fffffff;
-  if (threadIdx.x < 32) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) t = min(t, __shfl_xor_sync(0xffffffffu, t, o));
-  }
-  if (threadIdx.x == 0) sh[32] = t;
-  __syncthreads();
-  const int r = sh[32];
-  __syncthreads();
-  return r;
-}
+// Bound: latency, not bytes (300 KB of logits): one CTA took 31 bisection passes of 125 dependent loads each over the vocabulary, 380 us for
+// 128256 entries.  The vocabulary is cut between the CTAs of a cluster, which keep their probabilities in shared memory; a pass looks
+// at seven thresholds at once and its sums meet over the cluster; the thresholds are logits, whose 16 bits take six passes (a
+// probability's 30 bits took ten: 97 us).
+// Every reduction has a fixed order (threads, warps, ranks): a draw is a function of (logits, seed, step).
+struct SampleShared {
+  float warp[SAMPLE_THREADS / 32][9];    // a warp's sums (rows of nine: no bank conflicts down a column)
+  float slot[2][SAMPLE_CTAS][8];         // the CTAs' sums, written by the peers; two sets in turn
+  float scan[2][SAMPLE_THREADS / 32 + 1];
+  float c_p[SAMPLE_MAX_K];
+  int c_i[SAMPLE_MAX_K];
+};
 
-// Multinomial draw over w[0..n) in index order (w >= 0): the first i whose inclusive prefix sum exceeds u * total
-// (rand::distributions::WeightedIndex).  Thread t owns the contiguous chunk [t*C, (t+1)*C); chunk sums are combined by a
-// fixed tree, so the result is deterministic.  `keep(i)` masks entries out (TopP).
-template <typename Keep>
-__device__ __forceinline__ int block_multinomial(const float *w, int n, float u, Keep keep, float *shf, int *shi) {
-  const int C = (n + SAMPLE_THREADS - 1) / SAMPLE_THREADS;
-  const int i0 = min(n, (int)threadIdx.x * C), i1 = min(n, i0 + C);
-  float loc = 0.f;
-  for (int i = i0; i < i1; i++) loc += keep(i) ? w[i] : 0.f;
-  // exclusive scan of the 1024 chunk sums: warp scan, then a scan of the 32 warp totals
-  float inc = loc;
+struct SampleCluster {
+  SampleShared &sh;
+  int rank, set = 0;
+  // v[0..N) of every thread of the cluster, combined with `op` in a fixed order; all[r * N + t]: rank r's part, for prefixes
+  template <int N, typename Op> __device__ __forceinline__ void reduce(float (&v)[N], float (&part)[SAMPLE_CTAS][N], float neutral, Op op) {
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const float t = __shfl_up_sync(0xffffffffu, inc, o);
-    if ((int)(threadIdx.x & 31) >= o) inc += t;
+    for (int t = 0; t < N; t++) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v[t] = op(v[t], __shfl_xor_sync(0xffffffffu, v[t], o));
+      if (lane == 0) sh.warp[warp][t] = v[t];
+    }
+    __syncthreads();
+    if (warp < N) {  // one warp per sum
+      float x = sh.warp[lane][warp];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) x = op(x, __shfl_xor_sync(0xffffffffu, x, o));
+      if (lane < SAMPLE_CTAS) st_cluster_f32(cluster_map(smem_u32(&sh.slot[set][rank][warp]), (uint32_t)lane), x);
+    }
+    __syncwarp();
+    cluster_arrive();
+    cluster_wait();
+#pragma unroll
+    for (int t = 0; t < N; t++) {
+      v[t] = neutral;
+#pragma unroll
+      for (int r = 0; r < SAMPLE_CTAS; r++) {
+        part[r][t] = sh.slot[set][r][t];
+        v[t] = op(v[t], part[r][t]);
+      }
+    }
+    set ^= 1;
   }
-  if ((threadIdx.x & 31) == 31) shf[threadIdx.x >> 5] = inc;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    float wt = shf[threadIdx.x], winc = wt;
+  template <int N> __device__ __forceinline__ void sum(float (&v)[N], float (&part)[SAMPLE_CTAS][N]) {
+    reduce<N>(v, part, 0.f, [](float a, float b) { return a + b; });
+  }
+  __device__ __forceinline__ float max1(float x) {
+    float v[1] = {x}, part[SAMPLE_CTAS][1];
+    reduce<1>(v, part, -INFINITY, [](float a, float b) { return fmaxf(a, b); });
+    return v[0];
+  }
+  __device__ __forceinline__ float sum1(float x) {
+    float v[1] = {x}, part[SAMPLE_CTAS][1];
+    sum<1>(v, part);
+    return v[0];
+  }
+  __device__ __forceinline__ int min_i(int x) {  // (vocabulary indices and 0x7fffffff compare as floats' bit patterns do)
+    float v[1] = {__int_as_float(x)}, part[SAMPLE_CTAS][1];
+    reduce<1>(v, part, __int_as_float(0x7fffffff), [](float a, float b) { return __int_as_float(min(__float_as_int(a), __float_as_int(b))); });
+    return __float_as_int(v[0]);
+  }
+  // exclusive prefix over the cluster's threads in vocabulary order, and the total
+  __device__ __forceinline__ float scan(float x, float &total) {
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    float inc = x;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const float t = __shfl_up_sync(0xffffffffu, winc, o);
-      if ((int)threadIdx.x >= o) winc += t;
+      const float t = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += t;
     }
-    shf[32 + threadIdx.x] = winc - wt;  // exclusive prefix of warp totals
-    if (threadIdx.x == 31) shf[64] = winc;  // grand total
+    float *ws = sh.scan[set];
+    if (lane == 31) ws[warp] = inc;
+    __syncthreads();
+    if (tid < 32) {
+      const float wt = ws[tid];
+      float winc = wt;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const float t = __shfl_up_sync(0xffffffffu, winc, o);
+        if (tid >= o) winc += t;
+      }
+      ws[tid] = winc - wt;
+      if (tid == 31) ws[32] = winc;
+    }
+    __syncthreads();
+    const float mine = ws[warp] + (inc - x);
+    if (tid < SAMPLE_CTAS) st_cluster_f32(cluster_map(smem_u32(&sh.slot[set][rank][0]), (uint32_t)tid), ws[32]);
+    __syncwarp();
+    cluster_arrive();
+    cluster_wait();
+    float before = 0.f;
+    total = 0.f;
+#pragma unroll
+    for (int r = 0; r < SAMPLE_CTAS; r++) {
+      if (r == rank) before = total;
+      total += sh.slot[set][r][0];
+    }
+    set ^= 1;
+    return before + mine;
   }
-  __syncthreads();
-  const float total = shf[64];
-  float run = shf[32 + (threadIdx.x >> 5)] + (inc - loc);
-  const float target = u * total;
-  int found = 0x7fffffff;
-  for (int i = i0; i < i1; i++) {
-    if (!keep(i)) continue;
-    run += w[i];
-    if (run > target) { found = i; break; }
+};
+
+// 16-bit floats in rising order as 0 .. 65535, and back
+template <typename T> __device__ __forceinline__ uint32_t sample_key(float x) {
+  const T d = DT<T>::from_f(x);
+  const uint32_t h = *reinterpret_cast<const uint16_t *>(&d);
+  return h & 0x8000u ? ~h & 0xffffu : h | 0x8000u;
+}
+template <typename T> __device__ __forceinline__ float sample_unkey(uint32_t k) {
+  const uint16_t h = (uint16_t)(k & 0x8000u ? k & 0x7fffu : ~k);
+  return DT<T>::to_f(*reinterpret_cast<const T *>(&h));
+}
+// The largest logit at which the entries that are at least as large still reach `want`, in number (COUNT) or in probability: with tau its
+// probability, reach(P >= tau) >= want > reach(P > tau), as probabilities rise with logits.  Seven thresholds a pass.
+template <typename T, bool COUNT>
+__device__ __forceinline__ float sample_threshold(SampleCluster &cl, const T *L, const float *P, int i0, int i1, float want) {
+  uint32_t lo = sample_key<T>(-INFINITY), hi = sample_key<T>(INFINITY) + 1u;
+  while (hi - lo > 1u) {
+    const uint32_t step = max(1u, (hi - lo) / 8u);
+    float m[7], th[7], part[SAMPLE_CTAS][7];
+#pragma unroll
+    for (int t = 0; t < 7; t++) {
+      m[t] = 0.f;
+      th[t] = sample_unkey<T>(min(hi - 1u, lo + (uint32_t)(t + 1) * step));
+    }
+    for (int i = i0; i < i1; i++) {
+      const float x = DT<T>::to_f(L[i]), v = COUNT ? 1.f : P[i];
+#pragma unroll
+      for (int t = 0; t < 7; t++) m[t] += x >= th[t] ? v : 0.f;
+    }
+    cl.sum<7>(m, part);
+    int best = 0;
+#pragma unroll
+    for (int t = 0; t < 7; t++)
+      if (lo + (uint32_t)(t + 1) * step < hi && m[t] >= want && best == t) best = t + 1;  // reach() falls as the threshold rises
+    const uint32_t next = lo + (uint32_t)(best + 1) * step;
+    lo += (uint32_t)best * step;
+    if (best < 7 && next < hi) hi = next;
   }
-  __syncthreads();
-  int r = block_min_i(found, shi);
-  if (r == 0x7fffffff) {  // u*total rounded up to the total itself: the last kept entry (WeightedIndex can return len-1)
-    int last = -1;
-    for (int i = i1 - 1; i >= i0; i--) if (keep(i) && w[i] > 0.f) { last = i; break; }
-    r = -block_min_i(last < 0 ? 0x7fffffff : -last, shi);
-    if (r == -0x7fffffff) r = 0;
-  }
-  return r;
+  return sample_unkey<T>(lo);
 }
 
 // `noise`: nullable; tests pass the uniforms explicitly — vocab floats in [0,1) for Gumbel, one float otherwise.
+// P: scratch of V floats, used when a CTA's part of the vocabulary is larger than its shared memory (in_smem == 0).
 template <typename T>
-__global__ void __launch_bounds__(SAMPLE_THREADS) sample_kernel(const T *__restrict__ logits, int V, SampleArgs s, float *__restrict__ P,
-                                                                 const float *__restrict__ noise, const int *d_step, int step_bias,
-                                                                 uint32_t *token_out, uint32_t *ring, int ring_cap) {
+__global__ void __cluster_dims__(SAMPLE_CTAS, 1, 1) __launch_bounds__(SAMPLE_THREADS)
+sample_kernel(const T *__restrict__ logits, int V, SampleArgs s, float *P_global, int in_smem, const float *__restrict__ noise, const int *d_step,
+              int step_bias, uint32_t *token_out, uint32_t *ring, int ring_cap) {
   pdl_launch_dependents();
   pdl_wait();
-  __shared__ float shf[80];
-  __shared__ int shi[40];
-  __shared__ float c_p[SAMPLE_MAX_K];
-  __shared__ int c_i[SAMPLE_MAX_K];
-  __shared__ int n_cand, chosen;
-  const int tid = threadIdx.x;
-  const unsigned step = (unsigned)(d_step ? *d_step + step_bias : 0);
+  extern __shared__ float sample_smem_p[];
+  __shared__ SampleShared sh;
+  const int tid = threadIdx.x, per = sample_per_thread(V);
+  SampleCluster cl{sh, (int)cluster_rank()};
+  const int base = (int)min((long)V, (long)cl.rank * per * SAMPLE_THREADS);
+  const int n = (int)min((long)V - base, (long)per * SAMPLE_THREADS);  // this CTA's entries: [base, base + n)
+  const T *lg = logits + base;
+  const unsigned step = (unsigned)((d_step ? *d_step : 0) + step_bias);
   auto finish = [&](int tok) {
-    if (tid == 0) {
+    if (cl.rank == 0 && tid == 0) {
       *token_out = (uint32_t)tok;
       if (ring) ring[step % (unsigned)ring_cap] = (uint32_t)tok;
     }
   };
+  cluster_arrive();  // every CTA runs before the first store to a peer
+  cluster_wait();
 
-  if (s.kind == SAMPLE_ARGMAX || s.temperature <= 0.f) {  // Sampling::ArgMax: first maximum wins
-    float best = -INFINITY;
-    int idx = 0x7fffffff;
-    for (int i = tid; i < V; i += SAMPLE_THREADS) {
-      const float v = DT<T>::to_f(logits[i]);
-      if (v > best) { best = v; idx = i; }
-    }
-    const float bm = block_max(best, shf);
-    finish(block_min_i(best == bm ? idx : 0x7fffffff, shi));
-    return;
-  }
-  if (s.kind == SAMPLE_GUMBEL) {
+  if (s.kind == SAMPLE_ARGMAX || s.temperature <= 0.f || s.kind == SAMPLE_GUMBEL) {  // first maximum wins
     // candle_nn::sampling::gumbel_softmax: minus_g = log(-log(u)), u in [1e-7, 0.999); T == 1: logits - minus_g, else
     // logits + minus_g * (-T); argmax
+    const bool gumbel = s.kind == SAMPLE_GUMBEL && s.temperature > 0.f;
     float best = -INFINITY;
     int idx = 0x7fffffff;
-    for (int i = tid; i < V; i += SAMPLE_THREADS) {
-      const float r = noise ? noise[i] : sample_uniform(s, step, (unsigned)i);
-      const float u = 1e-7f + r * (0.999f - 1e-7f);
-      const float minus_g = logf(-logf(u));
-      const float l = DT<T>::to_f(logits[i]);
-      const float v = (s.temperature == 1.0f) ? l - minus_g : l + minus_g * (-s.temperature);
-      if (v > best || (v == best && i < idx)) { best = v; idx = i; }
+    for (int i = tid; i < n; i += SAMPLE_THREADS) {
+      float v = DT<T>::to_f(lg[i]);
+      if (gumbel) {
+        const float r = noise ? noise[base + i] : sample_uniform(s, step, (unsigned)(base + i));
+        const float u = 1e-7f + r * (0.999f - 1e-7f);
+        const float minus_g = logf(-logf(u));
+        v = (s.temperature == 1.0f) ? v - minus_g : v + minus_g * (-s.temperature);
+      }
+      if (v > best) { best = v; idx = base + i; }
     }
-    const float bm = block_max(best, shf);
-    finish(block_min_i(best == bm ? idx : 0x7fffffff, shi));
+    const float bm = cl.max1(best);
+    finish(cl.min_i(best == bm ? idx : 0x7fffffff));
     return;
   }
 
   // ---- prs = softmax(logits * (1/T)) in f32 ------------------------------------------------------------------
+  float *P = in_smem ? sample_smem_p : P_global + base;
+  const T *L = lg;
   const float inv_t = (float)(1.0 / (double)s.temperature);
   float mx = -INFINITY;
-  for (int i = tid; i < V; i += SAMPLE_THREADS) mx = fmaxf(mx, DT<T>::to_f(logits[i]) * inv_t);
-  mx = block_max(mx, shf);
+  T *keep = reinterpret_cast<T *>(sample_smem_p + (size_t)per * SAMPLE_THREADS);
+#pragma unroll 4
+  for (int i = tid; i < n; i += SAMPLE_THREADS) {
+    const T x = lg[i];
+    if (in_smem) keep[i] = x;
+    mx = fmaxf(mx, DT<T>::to_f(x) * inv_t);
+  }
+  if (in_smem) L = keep;
+  mx = cl.max1(mx);
+  auto weight = [&](T x) { return expf(__fsub_rn(__fmul_rn(DT<T>::to_f(x), inv_t), mx)); };  // (no contraction: a threshold's own has the same bits)
   float sum = 0.f;
-  for (int i = tid; i < V; i += SAMPLE_THREADS) {
-    const float e = expf(DT<T>::to_f(logits[i]) * inv_t - mx);
+  for (int i = tid; i < n; i += SAMPLE_THREADS) {
+    const float e = weight(L[i]);
     P[i] = e;
     sum += e;
   }
-  sum = block_sum(sum, shf);
-  for (int i = tid; i < V; i += SAMPLE_THREADS) P[i] = P[i] / sum;
+  sum = cl.sum1(sum);
+  for (int i = tid; i < n; i += SAMPLE_THREADS) P[i] = P[i] / sum;
   __syncthreads();
   const float u = noise ? noise[0] : sample_uniform(s, step, 0xffffffffu);
+  const int i0 = min(n, tid * per), i1 = min(n, i0 + per);  // this thread's run of entries
 
   const bool want_k = (s.kind == SAMPLE_TOPK || s.kind == SAMPLE_TOPK_TOPP) && s.top_k < V;
   const bool want_p = (s.kind == SAMPLE_TOPP || s.kind == SAMPLE_TOPK_TOPP) && s.top_p > 0.f && s.top_p < 1.f;
-  if (!want_k && !want_p) {  // All (also TopK with k >= vocab, TopP with p outside (0,1))
-    finish(block_multinomial(P, V, u, [](int) { return true; }, shf, shi));
+  if (!want_k) {
+    // All (also TopK with k >= vocab, TopP with p outside (0,1)): every entry.  TopP: those above the probability tau at which the running
+    // sum in falling order crosses p, and the first ties at tau until the sum before one reaches p.  Drawn in vocabulary order.
+    uint32_t tau = 0u;
+    float eq_before = 0.f;
+    int need = 0x7fffffff;
+    if (want_p) {
+      tau = __float_as_uint(weight(DT<T>::from_f(sample_threshold<T, false>(cl, L, P, i0, i1, s.top_p))) / sum);
+      float m[1] = {0.f}, part[SAMPLE_CTAS][1], eq = 0.f, n_eq;
+      for (int i = i0; i < i1; i++) {
+        const uint32_t b = __float_as_uint(P[i]);
+        m[0] += b > tau ? P[i] : 0.f;
+        eq += b == tau ? 1.f : 0.f;
+      }
+      cl.sum<1>(m, part);
+      eq_before = cl.scan(eq, n_eq);
+      need = 0;
+      for (float cum = m[0]; cum < s.top_p && (float)need < n_eq; need++) cum += __uint_as_float(tau);
+    }
+    auto kept = [&](uint32_t b, int &rank) { return b > tau || (b == tau && rank++ < need); };
+    int rank = (int)eq_before;
+    float loc = 0.f, total;
+    for (int i = i0; i < i1; i++) loc += kept(__float_as_uint(P[i]), rank) ? P[i] : 0.f;
+    float run = cl.scan(loc, total);
+    const float target = u * total;  // rand::distributions::WeightedIndex: the first entry whose inclusive prefix sum exceeds it
+    int found = 0x7fffffff, last = -1;
+    rank = (int)eq_before;
+    for (int i = i0; i < i1; i++) {
+      if (!kept(__float_as_uint(P[i]), rank)) continue;
+      run += P[i];
+      if (P[i] > 0.f) last = base + i;
+      if (run > target && found == 0x7fffffff) found = base + i;
+    }
+    int r = cl.min_i(found);
+    if (r == 0x7fffffff) {  // u * total rounded up to the total itself: the last kept entry (WeightedIndex can return len-1)
+      r = 0x7ffffffe - cl.min_i(last < 0 ? 0x7fffffff : 0x7ffffffe - last);
+      if (r < 0) r = 0;
+    }
+    finish(r);
     return;
   }
 
-  // ---- the K most probable entries: bisection on the (monotone) bit pattern of the k-th largest probability -----
-  // pure TopP first looks at the SAMPLE_MAX_K most probable tokens: the nucleus almost always lies within them
-  const int K = want_k ? s.top_k : SAMPLE_MAX_K;
-  uint32_t lo = 0u, hi = 0x7f800000u;  // count(P >= lo) >= K always holds for lo = 0
-  while (hi - lo > 1u) {
-    const uint32_t mid = lo + (hi - lo) / 2u;
-    int cnt = 0;
-    for (int i = tid; i < V; i += SAMPLE_THREADS) cnt += (__float_as_uint(P[i]) >= mid);
-    cnt = block_sum_i(cnt, shi);
-    if (cnt >= K) lo = mid; else hi = mid;
+  // ---- the K most probable entries, ties at the K-th in vocabulary order, to the first CTA ---------------------
+  const int K = s.top_k;
+  const uint32_t lo = __float_as_uint(weight(DT<T>::from_f(sample_threshold<T, true>(cl, L, P, i0, i1, (float)K))) / sum);
+  float gt = 0.f, eq = 0.f, n_gt, n_eq;
+  for (int i = i0; i < i1; i++) {
+    const uint32_t b = __float_as_uint(P[i]);
+    gt += b > lo ? 1.f : 0.f;
+    eq += b == lo ? 1.f : 0.f;
   }
-  // lo = bit pattern of the K-th largest probability: take everything above it, then ties in index order up to K
-  {
-    int cnt = 0;
-    for (int i = tid; i < V; i += SAMPLE_THREADS) cnt += (__float_as_uint(P[i]) > lo);
-    const int n_gt = block_sum_i(cnt, shi);
-    if (tid == 0) n_cand = 0;
-    __syncthreads();
-    // deterministic gather: thread t owns a contiguous chunk; exclusive offsets by two integer scans (gt, then ties)
-    const int C = (V + SAMPLE_THREADS - 1) / SAMPLE_THREADS;
-    const int i0 = min(V, tid * C), i1 = min(V, i0 + C);
-    int my_gt = 0, my_eq = 0;
-    for (int i = i0; i < i1; i++) {
-      const uint32_t b = __float_as_uint(P[i]);
-      my_gt += (b > lo);
-      my_eq += (b == lo);
-    }
-    auto excl_scan = [&](int v) -> int {  // exclusive prefix over threads
-      int inc = v;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, inc, o);
-        if ((tid & 31) >= o) inc += t;
-      }
-      if ((tid & 31) == 31) shi[tid >> 5] = inc;
-      __syncthreads();
-      if (tid < 32) {
-        int wt = shi[tid], winc = wt;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int t = __shfl_up_sync(0xffffffffu, winc, o);
-          if (tid >= o) winc += t;
-        }
-        shi[tid] = winc - wt;
-      }
-      __syncthreads();
-      const int r = shi[tid >> 5] + inc - v;
-      __syncthreads();
-      return r;
-    };
-    int off_gt = excl_scan(my_gt), off_eq = excl_scan(my_eq);
-    for (int i = i0; i < i1; i++) {
-      const uint32_t b = __float_as_uint(P[i]);
-      if (b > lo) { c_p[off_gt] = P[i]; c_i[off_gt] = i; off_gt++; }
-      else if (b == lo) {
-        const int slot = n_gt + off_eq;
-        if (slot < K) { c_p[slot] = P[i]; c_i[slot] = i; }
-        off_eq++;
-      }
-    }
-    __syncthreads();
+  int at_gt = (int)cl.scan(gt, n_gt);
+  int at_eq = (int)cl.scan(eq, n_eq) + (int)n_gt;
+  for (int i = i0; i < i1; i++) {
+    const uint32_t b = __float_as_uint(P[i]);
+    if (b < lo) continue;
+    const int at = b > lo ? at_gt++ : at_eq++;
+    if (at >= K) continue;
+    st_cluster_f32(cluster_map(smem_u32(&sh.c_p[at]), 0u), P[i]);
+    st_cluster_f32(cluster_map(smem_u32(&sh.c_i[at]), 0u), __int_as_float(base + i));
   }
+  __syncwarp();
+  cluster_arrive();
+  cluster_wait();
+  if (cl.rank != 0) return;
   // ---- sort the K candidates: probability descending, ties by lower id (bitonic, shared memory) ---------------
-  int n = 1;
-  while (n < K) n <<= 1;
-  for (int i = K + tid; i < n; i += SAMPLE_THREADS) { c_p[i] = -1.f; c_i[i] = 0x7fffffff; }
+  float *c_p = sh.c_p;
+  int *c_i = sh.c_i;
+  int np = 1;
+  while (np < K) np <<= 1;
+  for (int i = K + tid; i < np; i += SAMPLE_THREADS) { c_p[i] = -1.f; c_i[i] = 0x7fffffff; }
   __syncthreads();
-  for (int k2 = 2; k2 <= n; k2 <<= 1)
+  for (int k2 = 2; k2 <= np; k2 <<= 1)
     for (int j = k2 >> 1; j > 0; j >>= 1) {
-      for (int i = tid; i < n; i += SAMPLE_THREADS) {
+      for (int i = tid; i < np; i += SAMPLE_THREADS) {
         const int l = i ^ j;
         if (l > i) {
           const bool up = ((i & k2) == 0);
@@ -315,94 +363,7 @@ __global__ void __launch_bounds__(SAMPLE_THREADS) sample_kernel(const T *__restr
       }
       __syncthreads();
     }
-  // ---- the rest is a short sequential walk over at most 1024 sorted candidates ---------------------------------
-  if (s.kind == SAMPLE_TOPP) {
-    // nucleus inside the top-SAMPLE_MAX_K: keep while the running sum BEFORE the token is < p
-    if (tid == 0) {
-      float cum = 0.f;
-      int m = 0;
-      for (; m < K; m++) {
-        if (cum >= s.top_p) break;
-        cum += c_p[m];
-      }
-      n_cand = (m == K && cum < s.top_p) ? -1 : m;   // -1: the nucleus is larger than the candidate list
-      chosen = m > 0 ? __float_as_int(c_p[m - 1]) : 0;
-    }
-    __syncthreads();
-    if (n_cand >= 0) {
-      // kept set = sorted candidates [0, n_cand): in vocabulary order that is {P > tau} plus the first ties at tau
-      const uint32_t tau = (uint32_t)chosen;
-      int ties_kept = 0;
-      if (tid == 0) {
-        for (int m = 0; m < n_cand; m++) ties_kept += (__float_as_uint(c_p[m]) == tau);
-        shi[39] = ties_kept;
-      }
-      __syncthreads();
-      ties_kept = shi[39];
-      __syncthreads();
-      // rank of a tie = number of equal entries with a lower id: ties are few; count them on the fly
-      finish(block_multinomial(P, V, u, [&](int i) {
-        const uint32_t b = __float_as_uint(P[i]);
-        if (b > tau) return true;
-        if (b != tau) return false;
-        int rank = 0;
-        for (int m = 0; m < K; m++) rank += (__float_as_uint(c_p[m]) == tau && c_i[m] < i);
-        return rank < ties_kept;
-      }, shf, shi));
-      return;
-    }
-    // flat distribution: the nucleus exceeds 1024 tokens.  Bisection on the bit pattern of the probability at which the
-    // descending running sum crosses p (mass reductions by fixed trees), then the same vocabulary-order draw.
-    uint32_t a = 0u, b = 0x7f800000u;  // mass(P >= a) >= p holds for a = 0
-    while (b - a > 1u) {
-      const uint32_t mid = a + (b - a) / 2u;
-      float m = 0.f;
-      for (int i = tid; i < V; i += SAMPLE_THREADS) m += (__float_as_uint(P[i]) >= mid) ? P[i] : 0.f;
-      m = block_sum(m, shf);
-      if (m >= s.top_p) a = mid; else b = mid;
-    }
-    float m_gt = 0.f;
-    for (int i = tid; i < V; i += SAMPLE_THREADS) m_gt += (__float_as_uint(P[i]) > a) ? P[i] : 0.f;
-    m_gt = block_sum(m_gt, shf);
-    const float tauf = __uint_as_float(a);
-    int need = 0;  // ties at tau kept: until the running sum before a tie reaches p
-    { float cum = m_gt; while (cum < s.top_p && need < V) { cum += tauf; need++; } }
-    // ties in index order: keep the first `need` (prefix count of ties by chunks)
-    const int C = (V + SAMPLE_THREADS - 1) / SAMPLE_THREADS;
-    const int i0 = min(V, tid * C), i1 = min(V, i0 + C);
-    int my_eq = 0;
-    for (int i = i0; i < i1; i++) my_eq += (__float_as_uint(P[i]) == a);
-    int inc = my_eq;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int t = __shfl_up_sync(0xffffffffu, inc, o);
-      if ((tid & 31) >= o) inc += t;
-    }
-    if ((tid & 31) == 31) shi[tid >> 5] = inc;
-    __syncthreads();
-    if (tid < 32) {
-      int wt = shi[tid], winc = wt;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, winc, o);
-        if (tid >= o) winc += t;
-      }
-      shi[tid] = winc - wt;
-    }
-    __syncthreads();
-    int eq_before = shi[tid >> 5] + inc - my_eq;
-    __syncthreads();
-    // zero the dropped entries in place (P is scratch), then draw
-    for (int i = i0; i < i1; i++) {
-      const uint32_t bb = __float_as_uint(P[i]);
-      if (bb < a) P[i] = 0.f;
-      else if (bb == a) { if (eq_before >= need) P[i] = 0.f; eq_before++; }
-    }
-    __syncthreads();
-    finish(block_multinomial(P, V, u, [](int) { return true; }, shf, shi));
-    return;
-  }
-  // TopK / TopKThenTopP: draw over the sorted candidates (our defined order: probability descending)
+  // TopK / TopKThenTopP: draw over the sorted candidates (our defined order: probability descending), a short sequential walk
   if (tid == 0) {
     int m = K;
     if (want_p) {  // nucleus rule inside the k candidates (sample_topk_topp: sort, clip, multinomial)
@@ -421,10 +382,8 @@ __global__ void __launch_bounds__(SAMPLE_THREADS) sample_kernel(const T *__restr
       run += c_p[j];
       if (run > target) { pick = j; break; }
     }
-    chosen = c_i[pick < 0 ? 0 : pick];
+    finish(c_i[pick < 0 ? 0 : pick]);
   }
-  __syncthreads();
-  finish(chosen);
 }
 
 }  // namespace cake

@@ -208,3 +208,22 @@ def test_gpu_decode_graph_sampler_equals_cake_b200_sample_on_the_same_logits():
         assert int(toks[7]) == cur    # the ring holds the sampled tokens
     finally:
         ctx.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("vocab", [9, 8193, 300000])   # parts without entries; one entry past a full pass; parts too large for shared memory
+def test_gpu_samplers_at_the_edges_of_the_vocabulary_cut(vocab):
+    rng = np.random.default_rng(vocab)
+    ctx = _ctx(vocab)
+    try:
+        l = torch.from_numpy((rng.standard_normal(vocab) * 3).astype(np.float32)).to(torch.bfloat16)
+        l[rng.integers(0, vocab, 5)] = float(l.max())   # ties at the top
+        lf = l.float().numpy()
+        for kind, T, k, p in [(S.ARGMAX, 0.0, 0, 0.0), (S.ALL, 0.9, 0, 0.0), (S.TOPK, 0.7, 6, 0.0), (S.TOPP, 0.8, 0, 0.9), (S.TOPK_TOPP, 0.8, 8, 0.7)]:
+            for u in (0.0, 0.5, 0.99999):
+                want, (got, _) = S.sample(lf, kind, T, top_k=k, top_p=p, noise=[u]), _gpu_sample(ctx, l, kind, T, k, p, [u])
+                assert got == want or _close_draw(lf, kind, T, k, p, got, want), (kind, u, got, want)
+        noise = rng.random(vocab).astype(np.float32)
+        assert _gpu_sample(ctx, l, S.GUMBEL, 0.7, 0, 0.0, noise)[0] == S.sample(lf, S.GUMBEL, 0.7, noise=noise)
+    finally:
+        ctx.close()
