@@ -427,7 +427,7 @@ template <typename T> static int set_smem_attrs_T() {
 #define SETT(EPI)                                                                                                                  \
   CU(cudaFuncSetAttribute(gemm_tc_kernel<T, EPI, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<128>::SMEM_BYTES));      \
   CU(cudaFuncSetAttribute(gemm_tc_kernel<T, EPI, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<256>::SMEM_BYTES));      \
-  CU(cudaFuncSetAttribute(gemm_tc_kernel<T, EPI, 256, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<256>::SMEM_BYTES));
+  CU(cudaFuncSetAttribute(gemm_tc_kernel<T, EPI, 256, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<256, true>::SMEM_BYTES));
 #define SETK(EPI)                                                                                                                 \
   CU(cudaFuncSetAttribute(gemm_skinny_kernel<T, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, SK_SMEM_MAX));                  \
   CU(cudaFuncSetAttribute(gemm_skinny_kernel<T, EPI>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
@@ -1289,22 +1289,48 @@ struct TcExtra {  // optional modes of the tensor-core GEMM (TcParams in gemm_tc
   bool w_live = false;                    // W was written by an earlier kernel of the stream (a cache, not a weight)
   int group_rows = 0;                     // grouped product: no row block holds more rows than this (0 = unknown)
 };
+// Estimated microseconds of a product on gemm_tc_kernel and on gemm_skinny_kernel, from measurements of both over N 1024 .. 28672, K 1024 ..
+// 14336, 48 .. 2048 rows (one kernel after the other, weights from HBM); within 15 % of them.
+// gemm_tc: rounds of tiles over the chip; a 64-wide k-block takes 0.32 us (128 x 128, six stages in flight), 0.42 us (128 x 256, four) or 0.38
+// us (256 x 256 on a pair of SMs, six): the ring's round trip rather than its bytes.  N = 6144, K = 4096, 512 rows: 192 small tiles are two
+// rounds, 45.6 us, 48 pairs one, 29.8; N = 28672: 896 small tiles 170, 448 large ones 129, 224 pairs 101.
+enum { TC_SMALL = 0, TC_WIDE = 1, TC_PAIR = 2 };
+static double tc_us(const cake_b200_ctx *c, int M, int N, int K, int kind) {
+  if (kind != TC_SMALL && N % 256) return 1e30;
+  if (kind == TC_PAIR && M <= TC_BM) return 1e30;  // the second SM's rows would be empty
+  const long tiles = kind == TC_PAIR ? (long)((M + 255) / 256) * (N / 256) : (long)((M + TC_BM - 1) / TC_BM) * (N / (kind == TC_WIDE ? 256 : 128));
+  const long at_once = kind == TC_PAIR ? c->sm_count / 2 : c->sm_count;
+  static const double kb_us[3] = {0.32, 0.42, 0.38};
+  return std::max((kind == TC_PAIR ? 6.5 : 5.5) + (double)((tiles + at_once - 1) / at_once) * (K / TC_BK) * kb_us[kind], 3.0 + 2.0 * N * K / 5.2e6);
+}
+static int tc_kind(const cake_b200_ctx *c, int M, int N, int K, bool pairs) {
+  int best = pairs ? TC_PAIR : TC_WIDE;
+  for (int k = best - 1; k >= TC_SMALL; k--)
+    if (tc_us(c, M, N, K, k) < tc_us(c, M, N, K, best)) best = k;
+  return best;
+}
+// skinny: what its stages carry at the 8.9 TB/s that all SMs take in together (or W from HBM), and an epilogue that grows with the rows
+static double skinny_us(int nt, int N, int K) {
+  return std::max((double)(N / SK_BM) * (K / TC_BK) * sk_stage_bytes(nt) / 8.9e6, 2.0 * N * K / 6.4e6) + 5.5 + 0.035 * nt;
+}
 // gemm_skinny_kernel's shape for a product, or false where gemm_tc_kernel takes it.
 static bool plan_skinny(const cake_b200_ctx *c, int M, int N, int K, const TcExtra &x, SkParams *p, size_t *smem) {
-  static const int max_rows = []() { const char *e = getenv("SK_ROWS"); return e ? atoi(e) : SK_MAX_ROWS; }();
   if (x.w_live || x.b_kwrap || x.w_cols || x.w_rows || x.w_ld) return false;
   const int rows = x.tile_group ? x.group_rows : M;
-  if (rows < 1 || rows > max_rows) return false;
+  if (rows < 1 || rows > (x.tile_group ? 64 : SK_MAX_ROWS)) return false;
   p->nt = (rows + 15) / 16 * 16;
+  if (!x.tile_group && rows > 64 && skinny_us(p->nt, N, K) >= tc_us(c, M, N, K, tc_kind(c, M, N, K, true))) return false;
   p->m_tiles = x.tile_group ? M / TC_BM : 1;
   p->m_step = TC_BM;
   const int tiles = N / SK_BM * p->m_tiles, sms = c->sm_count;
-  // The cut along K: as many CTAs as stay resident at once (up to three per SM), each with at least two k-blocks.  N = 6144, K = 4096, 16
-  // rows: 48 slices x 1 21.9 us, x 2 14.7, x 4 12.7, x 8 11.2 (three per SM) - 15.3 with rings that let only two in, a second wave.
+  // The cut along K: as many CTAs as stay resident at once (three per SM up to 64 rows, two up to 127, one beyond: a ring has four stages or
+  // more), each with at least two k-blocks.  N = 6144, K = 4096, 16 rows: 48 slices x 1 21.9 us, x 2 14.7, x 4 12.7, x 8 11.2 (three per SM) -
+  // 15.3 with rings that let only two in, a second wave.
+  const int most = p->nt <= 64 ? 3 : p->nt < 128 ? 2 : 1;
   p->split = 1;
-  while (p->split < SK_MAX_SPLIT && tiles * p->split * 2 <= 3 * sms && K / TC_BK >= p->split * 4) p->split *= 2;
-  const int per_sm = std::min(3, (tiles * p->split + sms - 1) / sms);
-  const size_t budget = (size_t)(per_sm == 3 && p->split > 1 ? 74 : 110) * 1024 - 1536;
+  while (p->split < SK_MAX_SPLIT && tiles * p->split * 2 <= most * sms && K / TC_BK >= p->split * 4) p->split *= 2;
+  const int per_sm = std::min(most, (tiles * p->split + sms - 1) / sms);
+  const size_t budget = (size_t)(per_sm == 3 && p->split > 1 ? 74 : most == 1 ? 180 : 110) * 1024 - 1536;
   p->stages = std::min(SK_MAX_STAGES, std::max(2, (int)(budget / sk_stage_bytes(p->nt))));
   *smem = sk_smem_bytes(p->nt, p->stages, p->split);
   return *smem <= SK_SMEM_MAX;
@@ -1324,26 +1350,22 @@ static int gemm_tc_T(cake_b200_ctx *c, const void *A, const void *W, const void 
     return launch_cluster_pdl(c, gemm_skinny_kernel<T, EPI>, dim3((unsigned)(N / SK_BM * sk.m_tiles * sk.split)), dim3(SK_THREADS), sk_smem,
                               (unsigned)sk.split, mw, ma, sk);
   }
-  // 128 x 256 tiles when N allows and there are enough tiles to fill the chip; CAKE_B200_TC_BN=128 forces the small tile (A/B aid)
-  static const int force_bn = []() { const char *e = getenv("CAKE_B200_TC_BN"); return e ? atoi(e) : 0; }();
-  const int tiles_m = (M + TC_BM - 1) / TC_BM;
-  const bool big = force_bn ? force_bn == 256 && N % 256 == 0 : (N % 256 == 0 && tiles_m * (N / 256) >= c->sm_count);
-  const int bn = big ? 256 : 128;
-  // pairs of CTAs sharing the W tile by TMA multicast (gemm_tc.cuh MC): needs an even number of 128-row tiles
-  static const int no_mc = []() { const char *e = getenv("CAKE_B200_TC_MC"); return (e && e[0] == '0') ? 1 : 0; }();
-  const bool mc = big && !no_mc && M % 256 == 0 && (tiles_m / 2) * (N / 256) >= c->sm_count / 2 && !x.tile_group && !x.b_kwrap;
+  // the tile whose rounds over the chip come out shortest; a grouped product's neighbours belong to different groups, and a wrapping W has no halves
+  const bool weight = !x.tile_group && !x.w_live && !x.b_kwrap;
+  const int kind = tc_kind(c, M, N, K, !x.tile_group && !x.b_kwrap);
+  const int tiles_m = (M + TC_BM - 1) / TC_BM, bn = kind == TC_SMALL ? 128 : 256;
   CUtensorMap ma, mb;
   RC(make_tmap(&ma, A, (uint64_t)M, (uint64_t)K, c->cfg.dtype, TC_BM, (uint64_t)x.a_ld));
   RC(make_tmap(&mb, W, x.w_rows ? (uint64_t)x.w_rows : (uint64_t)N * x.n_groups, (uint64_t)(x.w_cols ? x.w_cols : K), c->cfg.dtype,
-               mc ? 128u : (uint32_t)bn, (uint64_t)x.w_ld ? (uint64_t)x.w_ld : (uint64_t)K));
-  TcParams p{bias, res, C, M, N, K, act >= 0 ? act : (c->cfg.use_gelu_mlp ? 1 : 0), ldc, cap, x.tile_group, x.row_scale, x.b_kwrap};
+               kind == TC_PAIR ? 128u : (uint32_t)bn, (uint64_t)x.w_ld ? (uint64_t)x.w_ld : (uint64_t)K));
+  TcParams p{bias, res, C, M, N, K, act >= 0 ? act : (c->cfg.use_gelu_mlp ? 1 : 0), ldc, cap, x.tile_group, x.row_scale, x.b_kwrap, weight ? 1 : 0, c->wait_err};
+  if (kind == TC_PAIR) {
+    const int units = (tiles_m + 1) / 2 * (N / 256), pairs = std::min(units, c->sm_count / 2);
+    return launch_cluster_pdl(c, gemm_tc_kernel<T, EPI, 256, true>, dim3((unsigned)(2 * pairs)), dim3(TC_THREADS), (size_t)TcCfg<256, true>::SMEM_BYTES, 2u, ma, mb, p);
+  }
   const int tiles = tiles_m * (N / bn);
   dim3 grid(tiles < c->sm_count ? tiles : c->sm_count), block(TC_THREADS);
-  if (mc) {
-    dim3 g2((unsigned)(c->sm_count & ~1));
-    return launch_cluster_pdl(c, gemm_tc_kernel<T, EPI, 256, true>, g2, block, (size_t)TcCfg<256>::SMEM_BYTES, 2u, ma, mb, p);
-  }
-  if (big) return launch_pdl(c, gemm_tc_kernel<T, EPI, 256>, grid, block, (size_t)TcCfg<256>::SMEM_BYTES, ma, mb, p);
+  if (kind == TC_WIDE) return launch_pdl(c, gemm_tc_kernel<T, EPI, 256>, grid, block, (size_t)TcCfg<256>::SMEM_BYTES, ma, mb, p);
   return launch_pdl(c, gemm_tc_kernel<T, EPI, 128>, grid, block, (size_t)TcCfg<128>::SMEM_BYTES, ma, mb, p);
 }
 
@@ -3534,7 +3556,7 @@ extern "C" int cake_b200_logits(cake_b200_ctx *c, const void *x_dev, int batch, 
   RC(wait_loads(c));
   if (c->cfg.layer_list) return listed_logits_last(c, x_dev, batch, seq, logits_dev, argmax_host);
   const size_t H = c->cfg.hidden, V = c->cfg.vocab, es = c->es;
-  if (batch > 1 && batch <= SK_MAX_ROWS && tc_gemm_ok(batch, (int)V, (int)H) && H <= 8192 && (((uintptr_t)x_dev | (uintptr_t)c->ln_f) & 15) == 0) {
+  if (batch > 1 && tc_gemm_ok(batch, (int)V, (int)H) && H <= 8192 && (((uintptr_t)x_dev | (uintptr_t)c->ln_f) & 15) == 0) {
     // several rows: norm, then one product that reads lm_head once (a GEMV per row read it `batch` times: 2750 us for 16 rows of 128256 x
     // 4096, 158 us of it for the bytes)
     RC(pf_reserve(c, (size_t)batch));
@@ -3545,7 +3567,7 @@ extern "C" int cake_b200_logits(cake_b200_ctx *c, const void *x_dev, int batch, 
       CU(cudaMalloc(&c->hd_logits, (size_t)batch * V * es));
       c->hd_logits_rows = batch;
     }
-    if (!c->hd_tokens) CU(cudaMalloc(&c->hd_tokens, SK_MAX_ROWS * 4));
+    if (!c->hd_tokens) CU(cudaMalloc(&c->hd_tokens, 64 * 4));
     void *lo = logits_dev ? logits_dev : c->hd_logits;
     RC(DISPATCH_T(c->cfg.dtype, T_LAMBDA {
       typedef typename decltype(tag_)::type T;

@@ -17,7 +17,7 @@
 namespace cake {
 
 constexpr int SK_BM = 128, SK_THREADS = 192, SK_MAX_NT = 256, SK_MAX_SPLIT = 8, SK_MAX_STAGES = 8;
-constexpr int SK_MAX_ROWS = 64, SK_SMEM_MAX = 220 * 1024;
+constexpr int SK_MAX_ROWS = 256, SK_SMEM_MAX = 220 * 1024;
 constexpr int SK_W_BYTES = SK_BM * TC_BK * 2;  // 16 KB of W per stage
 __host__ __device__ inline int sk_stage_bytes(int nt) { return SK_W_BYTES + nt * TC_BK * 2; }
 __host__ inline size_t sk_smem_bytes(int nt, int stages, int split) {
@@ -51,35 +51,9 @@ __device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t (&r)[16]) {
 }
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-__device__ __forceinline__ uint32_t cluster_map(uint32_t saddr, uint32_t rank) {
-  uint32_t r;
-  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
-  return r;
-}
 __device__ __forceinline__ void st_cluster_f32(uint32_t addr, float v) {
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
 }
-// mbarrier wait with a bound (a try_wait suspends the thread for a while by itself): past it the wait is given up, the error flag
-// is set, and the kernel runs to its end.  The loop is one piece of assembly: written in C++ it cost the attention kernel 4 %.
-constexpr uint32_t MBAR_WAIT_LIMIT = 1u << 25;
-__device__ __forceinline__ void mbar_wait_lim(uint64_t *bar, uint32_t parity, int *err) {
-  uint32_t left;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "mov.u32 %0, %3;\n\t"
-      "WAIT_%=:\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "@p bra DONE_%=;\n\t"
-      "sub.u32 %0, %0, 1;\n\t"
-      "setp.ne.u32 q, %0, 0;\n\t"
-      "@q bra WAIT_%=;\n\t"
-      "DONE_%=:\n\t}"
-      : "=&r"(left)
-      : "r"(smem_u32(bar)), "r"(parity), "n"(MBAR_WAIT_LIMIT)
-      : "memory");
-  if (left == 0) *(volatile int *)err = 1;
-}
-
 // what an epilogue reads beside the sums, for row m of A at column n (rows past m_end: nothing)
 template <typename T, int EPI>
 __device__ __forceinline__ float sk_residual(const SkParams &p, int m, int m_end, int n) {

@@ -29,9 +29,9 @@ namespace cake {
 // activity.  128x256 (all 512 TMEM columns: two 128x256 fp32 accumulators) moves 48 KB per 4.2 MFLOP = 87 flop/B.
 constexpr int TC_BM = 128, TC_BK = 64, TC_THREADS = 256;
 constexpr int TC_BN = 128;                     // granularity the host checks N against (BN = 256 when N % 256 == 0)
-template <int BN> struct TcCfg {
-  static constexpr int STAGES = (BN == 256) ? 4 : 6;
-  static constexpr int STAGE_BYTES = (TC_BM + BN) * TC_BK * 2;  // 32 KB | 48 KB
+template <int BN, bool PAIR = false> struct TcCfg {
+  static constexpr int STAGES = (BN == 256 && !PAIR) ? 4 : 6;
+  static constexpr int STAGE_BYTES = (TC_BM + (PAIR ? BN / 2 : BN)) * TC_BK * 2;  // 32 KB | 48 KB | 32 KB
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
 };
 constexpr int TC_SMEM_BYTES = TcCfg<256>::SMEM_BYTES > TcCfg<128>::SMEM_BYTES ? TcCfg<256>::SMEM_BYTES : TcCfg<128>::SMEM_BYTES;
@@ -58,6 +58,8 @@ struct TcParams {
   const float *row_scale = nullptr;
   // k-block coordinate of W wraps at this many elements (0 = never): A = [P_hi | P_lo] against one copy of W
   int b_kwrap = 0;
+  int w_early = 0;  // W is a weight: its first stages are requested before the wait for the kernel in front
+  int *err = nullptr;
 };
 
 // Tile rasterisation: groups of TC_GM m-tiles (16 x 128 rows = 16 MB of A at K=4096) are walked n-major, so the A
@@ -80,18 +82,33 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, i
       "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1)
       : "memory");
 }
-// the same load delivered to the same shared-memory offset of every CTA in cta_mask (and signalling each one's mbarrier)
-__device__ __forceinline__ void tma_load_2d_mc(void *dst, const CUtensorMap *map, int c0, int c1, uint64_t *bar, uint16_t cta_mask) {
+// the same load with its completion counted on a barrier of the pair's first CTA (a shared::cluster address)
+__device__ __forceinline__ void tma_load_2d_pair(void *dst, const CUtensorMap *map, int c0, int c1, uint32_t bar) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.multicast::cluster [%0], [%1, {%3, %4}], [%2], %5;" ::"r"(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
           smem_u32(dst)),
-      "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "h"(cta_mask)
+      "l"(map), "r"(bar), "r"(c0), "r"(c1)
       : "memory");
 }
-__device__ __forceinline__ void tc_commit_mc(uint64_t *bar, uint16_t cta_mask) {  // arrive on the barrier at this offset in every CTA of the mask
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
-               "h"(cta_mask)
+__device__ __forceinline__ void tc_commit_pair(uint64_t *bar) {  // arrive on the barrier at this offset in both CTAs of the pair
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
+               "h"((uint16_t)3)
                : "memory");
+}
+__device__ __forceinline__ void tc_mma_f16_pair(uint32_t tmem_c, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_c),
+      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ uint32_t cluster_map(uint32_t saddr, uint32_t rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -143,21 +160,20 @@ template <> __device__ __forceinline__ uint32_t tc_idesc<__half>(int bn) {
   return (1u << 4) | (0u << 7) | (0u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
 }
 
-// MC (BN == 256 only, launched as clusters of 2 CTAs, M % 256 == 0): the two CTAs of a cluster work on vertically adjacent
-// 128-row tiles of the SAME 256-column panel and share its W tile — each loads one 128-row half of it and multicasts the
-// half into both CTAs' shared memory, so a CTA pulls 16 KB (A) + 16 KB (its W half) instead of 48 KB per k-block out of L2:
-// the operand traffic of a 2-CTA MMA without giving up the independent cta_group::1 accumulators.  A stage may be refilled
-// only when BOTH CTAs have consumed it (the peer's multicast lands in our buffer): every MMA commit arrives on the empty
-// barrier of both CTAs (count 2).
-template <typename T, int EPI, int BN, bool MC = false>
+// PAIR (BN == 256 only, launched as clusters of 2 CTAs): one 256 x 256 tile on two SMs, tcgen05.mma.cta_group::2.  Each CTA loads its own 128
+// rows of A and one 128-row half of the W tile and keeps its 128 rows of the accumulator; the first CTA's MMA thread multiplies both.  A
+// stage is 32 KB for the work that took 48 KB, so six are in flight instead of four: a product of one round over the chip is bound by the
+// ring's round trip (0.42 us per k-block with four stages, the tensor cores need 0.27).
+template <typename T, int EPI, int BN, bool PAIR = false>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const TcParams p) {
-  static_assert(!MC || BN == 256, "multicast variant is built for 128 x 256 tiles");
+  static_assert(!PAIR || BN == 256, "the pair is built for 256 columns");
+  typedef TcCfg<BN, PAIR> Cfg;
   extern __shared__ unsigned char smem_raw_tc[];
   unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw_tc) + 1023) & ~(uintptr_t)1023);
-  uint64_t *full = reinterpret_cast<uint64_t *>(smem + TcCfg<BN>::STAGES * TcCfg<BN>::STAGE_BYTES);
-  uint64_t *empty = full + TcCfg<BN>::STAGES;
-  uint64_t *acc_full = empty + TcCfg<BN>::STAGES;   // [2]
+  uint64_t *full = reinterpret_cast<uint64_t *>(smem + Cfg::STAGES * Cfg::STAGE_BYTES);
+  uint64_t *empty = full + Cfg::STAGES;
+  uint64_t *acc_full = empty + Cfg::STAGES;   // [2]
   uint64_t *acc_empty = acc_full + 2;       // [2]
   uint32_t *tmem_ptr = reinterpret_cast<uint32_t *>(acc_empty + 2);
 
@@ -166,28 +182,33 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   const int kblocks = p.K / TC_BK;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < TcCfg<BN>::STAGES; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], MC ? 2 : 1); }
-    for (int a = 0; a < 2; a++) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], 128); }
+    for (int s = 0; s < Cfg::STAGES; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+    for (int a = 0; a < 2; a++) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], PAIR ? 8 : 4); }  // (a warp of the epilogue arrives once)
     mbar_fence_init();
   }
   if (warp == 2) {  // TMEM: 2 x BN columns = two 128 x BN fp32 accumulators
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_ptr)), "n"(2 * BN) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    if (PAIR) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_ptr)), "n"(2 * BN) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_ptr)), "n"(2 * BN) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (MC) cluster_sync_all();  // the peer's barriers exist before anything is multicast to it
+  if (PAIR) cluster_sync_all();  // the peer's barriers exist before anything arrives on them
   pdl_launch_dependents();
-  pdl_wait();
+  if (!p.w_early || warp != 0) pdl_wait();
   const uint32_t tmem_base = *tmem_ptr;
-  // work distribution: non-MC: one tile per CTA and round; MC: one (256-row, 256-column) unit per cluster and round
-  const uint32_t crank = MC ? cluster_rank() : 0u;
-  const int first = MC ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, stride = MC ? (int)(gridDim.x >> 1) : (int)gridDim.x;
-  const int units_m = MC ? tiles_m / 2 : tiles_m, n_units = units_m * tiles_n;
+  // work distribution: one tile per CTA and round; PAIR: one (256-row, 256-column) unit per cluster and round
+  const uint32_t crank = PAIR ? cluster_rank() : 0u;
+  const int first = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, stride = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
+  const int units_m = PAIR ? (tiles_m + 1) / 2 : tiles_m, n_units = units_m * tiles_n;
   auto unit_tile = [&](int u, int &m0, int &n0) {
     tc_tile(u, units_m, tiles_n, BN, m0, n0);   // m0 in units of TC_BM rows of the unit grid
-    if (MC) m0 = m0 * 2 + (int)crank * TC_BM;
+    if (PAIR) m0 = m0 * 2 + (int)crank * TC_BM;
   };
 
   if (warp == 0) {
@@ -195,8 +216,30 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     if (lane == 0) {
       asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
       asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
-      int s = 0;
+      int s = 0, early = 0;
       uint32_t ph = 0;
+      auto expect = [&](int st) {  // PAIR: the first CTA's barrier counts both CTAs' bytes
+        if (!PAIR) mbar_arrive_expect_tx(&full[st], Cfg::STAGE_BYTES);
+        else if (crank == 0) mbar_arrive_expect_tx(&full[st], 2 * Cfg::STAGE_BYTES);
+      };
+      auto load_a = [&](int st, int kb, int m0) {
+        unsigned char *d = smem + (size_t)st * Cfg::STAGE_BYTES;
+        if (PAIR) tma_load_2d_pair(d, &map_a, kb * TC_BK, m0, cluster_map(smem_u32(&full[st]), 0u));
+        else tma_load_2d(d, &map_a, kb * TC_BK, m0, &full[st]);
+      };
+      auto load_w = [&](int st, int kb, int wrow) {
+        unsigned char *d = smem + (size_t)st * Cfg::STAGE_BYTES + TC_BM * TC_BK * 2;
+        if (PAIR) tma_load_2d_pair(d, &map_b, kb * TC_BK, wrow + (int)crank * 128, cluster_map(smem_u32(&full[st]), 0u));  // a 128-row box: our half of the W tile
+        else tma_load_2d(d, &map_b, p.b_kwrap ? (kb * TC_BK) % p.b_kwrap : kb * TC_BK, wrow, &full[st]);
+      };
+      if (p.w_early) {  // (not a grouped product: the groups are another kernel's output)
+        if (first < n_units) {
+          int m0, n0;
+          unit_tile(first, m0, n0);
+          for (; early < Cfg::STAGES && early < kblocks; early++) { expect(early); load_w(early, early, n0); }
+        }
+        pdl_wait();
+      }
       for (int t = first; t < n_units; t += stride) {
         int m0, n0;
         unit_tile(t, m0, n0);
@@ -207,22 +250,21 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           wrow += g * p.N;
         }
         for (int kb = 0; kb < kblocks; kb++) {
-          mbar_wait(&empty[s], ph ^ 1u);
-          unsigned char *st = smem + (size_t)s * TcCfg<BN>::STAGE_BYTES;
-          mbar_arrive_expect_tx(&full[s], TcCfg<BN>::STAGE_BYTES);
-          tma_load_2d(st, &map_a, kb * TC_BK, m0, &full[s]);
-          if (MC)  // map_b has a 128-row box here: our half of the W tile, delivered to both CTAs
-            tma_load_2d_mc(st + TC_BM * TC_BK * 2 + crank * (128 * TC_BK * 2), &map_b, kb * TC_BK, n0 + (int)crank * 128, &full[s], (uint16_t)3);
-          else
-            tma_load_2d(st + TC_BM * TC_BK * 2, &map_b, p.b_kwrap ? (kb * TC_BK) % p.b_kwrap : kb * TC_BK, wrow, &full[s]);
-          if (++s == TcCfg<BN>::STAGES) { s = 0; ph ^= 1u; }
+          if (early > 0) early--;
+          else {
+            mbar_wait_lim(&empty[s], ph ^ 1u, p.err);
+            expect(s);
+            load_w(s, kb, wrow);
+          }
+          load_a(s, kb, m0);
+          if (++s == Cfg::STAGES) { s = 0; ph ^= 1u; }
         }
       }
     }
   } else if (warp == 1) {
     // ===================== MMA issuer (one thread) =======================================================
-    if (lane == 0) {
-      const uint32_t idesc = tc_idesc<T>(BN);
+    if (lane == 0 && crank == 0) {
+      const uint32_t idesc = PAIR ? tc_idesc<T>(BN) + ((uint32_t)(TC_BM >> 4) << 24) : tc_idesc<T>(BN);  // PAIR: M = 256
       int s = 0;
       uint32_t ph = 0;
       int it = 0;
@@ -235,22 +277,24 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         const int a = it & 1;
         const uint32_t aph = (uint32_t)(it >> 1) & 1u;
         it++;
-        mbar_wait(&acc_empty[a], aph ^ 1u);  // the epilogue has drained this accumulator
+        mbar_wait_lim(&acc_empty[a], aph ^ 1u, p.err);  // the epilogue has drained this accumulator
         tc_fence_after();
         const uint32_t tmem_c = tmem_base + (uint32_t)(a * BN);
         for (int kb = 0; kb < kblocks; kb++) {
-          mbar_wait(&full[s], ph);
+          mbar_wait_lim(&full[s], ph, p.err);
           tc_fence_after();
-          const unsigned char *st = smem + (size_t)s * TcCfg<BN>::STAGE_BYTES;
+          const unsigned char *st = smem + (size_t)s * Cfg::STAGE_BYTES;
           const uint64_t da = tc_smem_desc(st), db = tc_smem_desc(st + TC_BM * TC_BK * 2);
 #pragma unroll
           for (int k = 0; k < TC_BK / 16; k++)  // +32 bytes (2 x 16 B units) per K=16 slab inside the swizzle atom
-            tc_mma_f16(tmem_c, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb | k) ? 1u : 0u);
-          if (MC) tc_commit_mc(&empty[s], (uint16_t)3);  // ... in BOTH CTAs: the peer multicasts into this stage too
-          else tc_commit(&empty[s]);  // arrives when the MMAs above have read the stage
-          if (++s == TcCfg<BN>::STAGES) { s = 0; ph ^= 1u; }
+            if (PAIR) tc_mma_f16_pair(tmem_c, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb | k) ? 1u : 0u);
+            else tc_mma_f16(tmem_c, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb | k) ? 1u : 0u);
+          if (PAIR) tc_commit_pair(&empty[s]);  // arrives (in both CTAs) when the MMAs above have read the stage
+          else tc_commit(&empty[s]);
+          if (++s == Cfg::STAGES) { s = 0; ph ^= 1u; }
         }
-        tc_commit(&acc_full[a]);  // accumulator complete
+        if (PAIR) tc_commit_pair(&acc_full[a]);  // accumulator complete
+        else tc_commit(&acc_full[a]);
       }
     }
   } else if (warp >= 4) {
@@ -268,7 +312,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       const uint32_t aph = (uint32_t)(it >> 1) & 1u;
       it++;
       const int row = m0 + wq * 32 + lane;
-      mbar_wait(&acc_full[a], aph);
+      mbar_wait_lim(&acc_full[a], aph, p.err);
       tc_fence_after();
 #pragma unroll 1
       for (int c0 = 0; c0 < BN; c0 += 32) {
@@ -354,15 +398,20 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
       }
       tc_fence_before();
-      mbar_arrive(&acc_empty[a]);
+      __syncwarp();
+      if (lane == 0) {
+        if (PAIR) mbar_arrive_cluster(cluster_map(smem_u32(&acc_empty[a]), 0u));
+        else mbar_arrive(&acc_empty[a]);
+      }
     }
   }
   tc_fence_before();
   __syncthreads();
-  if (MC) cluster_sync_all();  // nobody leaves while the peer may still signal our barriers
+  if (PAIR) cluster_sync_all();  // nobody leaves while the peer may still signal our barriers or read our operands
   if (warp == 2) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "n"(2 * BN) : "memory");
+    if (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "n"(2 * BN) : "memory");
+    else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "n"(2 * BN) : "memory");
   }
 }
 

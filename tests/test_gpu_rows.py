@@ -91,3 +91,18 @@ def test_head_of_a_batch(batch, seq, vocab, dtype):
     first = np.argmax(to_np(both), axis=1)   # numpy's argmax is the first maximum
     assert list(tok) == list(first) == list(tok2)
     ctx.close()
+
+
+@pytest.mark.parametrize("dtype", ["bf16", "f16"])
+@pytest.mark.parametrize("rows", [129, 200, 257, 300])   # a pair's second tile with one row, between two tiles, three tiles, an odd tile count
+def test_products_of_tile_pairs(rows, dtype):
+    # gate / up: 16384 columns, two rounds of small tiles or one of pairs
+    cfg = medium_config(num_attention_heads=4, num_key_value_heads=1, head_dim=128, intermediate_size=8192)
+    sd = checkpoint(cfg, dtype, seed=43, std=0.03)
+    om, ctx = O.OracleModel(cfg, sd, dtype), Context(cfg, sd, dtype)
+    blk = B200Transformer.load(cfg.layer_name(0), ctx)
+    x = rand_x((1, rows, cfg.hidden_size), dtype, seed=rows)
+    y = blk.forward(ctx.to_device(x), 0, 0, ctx)
+    ctx.sync()
+    _check(to_np(y[0]), om.block_forward(0, x[0].float().numpy(), 0, om.new_cache()), dtype, f"{rows} rows")
+    ctx.close()
