@@ -1288,6 +1288,8 @@ struct TcExtra {  // optional modes of the tensor-core GEMM (TcParams in gemm_tc
   int a_ld = 0;                           // A's row stride in elements when it is a column range of a wider buffer
   bool w_live = false;                    // W was written by an earlier kernel of the stream (a cache, not a weight)
   int group_rows = 0;                     // grouped product: no row block holds more rows than this (0 = unknown)
+  int batch = 1, a_step = 0, c_step = 0;  // side-by-side products: product i reads columns i * a_step .. of A's rows and rows i * N .. of W and
+                                          // writes columns i * c_step .. of C's rows (TCE_PLAIN, with a_ld and ldc)
 };
 // Estimated microseconds of a product on gemm_tc_kernel and on gemm_skinny_kernel, from measurements of both over N 1024 .. 28672, K 1024 ..
 // 14336, 48 .. 2048 rows (one kernel after the other, weights from HBM); within 15 % of them.
@@ -1315,7 +1317,7 @@ static double skinny_us(int nt, int N, int K) {
 }
 // gemm_skinny_kernel's shape for a product, or false where gemm_tc_kernel takes it.
 static bool plan_skinny(const cake_b200_ctx *c, int M, int N, int K, const TcExtra &x, SkParams *p, size_t *smem) {
-  if (x.w_live || x.b_kwrap || x.w_cols || x.w_rows || x.w_ld) return false;
+  if (x.w_live || x.b_kwrap || x.w_cols || x.w_rows || x.w_ld || x.batch > 1) return false;
   const int rows = x.tile_group ? x.group_rows : M;
   if (rows < 1 || rows > (x.tile_group ? 64 : SK_MAX_ROWS)) return false;
   p->nt = (rows + 15) / 16 * 16;
@@ -1352,18 +1354,19 @@ static int gemm_tc_T(cake_b200_ctx *c, const void *A, const void *W, const void 
   }
   // the tile whose rounds over the chip come out shortest; a grouped product's neighbours belong to different groups, and a wrapping W has no halves
   const bool weight = !x.tile_group && !x.w_live && !x.b_kwrap;
-  const int kind = tc_kind(c, M, N, K, !x.tile_group && !x.b_kwrap);
+  const int kind = N % 256 && x.batch > 1 ? (int)TC_SMALL : tc_kind(c, M, N * x.batch, K, !x.tile_group && !x.b_kwrap && N % 256 == 0);
   const int tiles_m = (M + TC_BM - 1) / TC_BM, bn = kind == TC_SMALL ? 128 : 256;
   CUtensorMap ma, mb;
-  RC(make_tmap(&ma, A, (uint64_t)M, (uint64_t)K, c->cfg.dtype, TC_BM, (uint64_t)x.a_ld));
-  RC(make_tmap(&mb, W, x.w_rows ? (uint64_t)x.w_rows : (uint64_t)N * x.n_groups, (uint64_t)(x.w_cols ? x.w_cols : K), c->cfg.dtype,
-               kind == TC_PAIR ? 128u : (uint32_t)bn, (uint64_t)x.w_ld ? (uint64_t)x.w_ld : (uint64_t)K));
-  TcParams p{bias, res, C, M, N, K, act >= 0 ? act : (c->cfg.use_gelu_mlp ? 1 : 0), ldc, cap, x.tile_group, x.row_scale, x.b_kwrap, weight ? 1 : 0, c->wait_err};
+  RC(make_tmap(&ma, A, (uint64_t)M, (uint64_t)K + (uint64_t)(x.batch - 1) * x.a_step, c->cfg.dtype, TC_BM, (uint64_t)x.a_ld));
+  // a W that no other row tile reads again comes from HBM in 256-byte pieces (grouped products: 64 experts of 2816 x 2048, one row block each)
+  RC(make_tmap(&mb, W, x.w_rows ? (uint64_t)x.w_rows : (uint64_t)N * x.n_groups * x.batch, (uint64_t)(x.w_cols ? x.w_cols : K), c->cfg.dtype,
+               kind == TC_PAIR ? 128u : (uint32_t)bn, (uint64_t)x.w_ld ? (uint64_t)x.w_ld : (uint64_t)K, x.tile_group != nullptr));
+  TcParams p{bias, res, C, M, N, K, act >= 0 ? act : (c->cfg.use_gelu_mlp ? 1 : 0), ldc, cap, x.tile_group, x.row_scale, x.b_kwrap, weight ? 1 : 0, x.batch, x.a_step, x.c_step, c->wait_err};
   if (kind == TC_PAIR) {
-    const int units = (tiles_m + 1) / 2 * (N / 256), pairs = std::min(units, c->sm_count / 2);
+    const int units = (tiles_m + 1) / 2 * (N / 256) * x.batch, pairs = std::min(units, c->sm_count / 2);
     return launch_cluster_pdl(c, gemm_tc_kernel<T, EPI, 256, true>, dim3((unsigned)(2 * pairs)), dim3(TC_THREADS), (size_t)TcCfg<256, true>::SMEM_BYTES, 2u, ma, mb, p);
   }
-  const int tiles = tiles_m * (N / bn);
+  const int tiles = tiles_m * (N / bn) * x.batch;
   dim3 grid(tiles < c->sm_count ? tiles : c->sm_count), block(TC_THREADS);
   if (kind == TC_WIDE) return launch_pdl(c, gemm_tc_kernel<T, EPI, 256>, grid, block, (size_t)TcCfg<256>::SMEM_BYTES, ma, mb, p);
   return launch_pdl(c, gemm_tc_kernel<T, EPI, 128>, grid, block, (size_t)TcCfg<128>::SMEM_BYTES, ma, mb, p);
@@ -1484,11 +1487,12 @@ static int enqueue_prefill_layers(cake_b200_ctx *c, cake_b200_block *const *bloc
                         (uint64_t)B * f.n_kv_heads, f.dtype, FT_BN));
           RC(make_tmap3(&mv, (const T *)kc->v[l] + wsoff, (uint64_t)hd, (uint64_t)hd, (uint64_t)(apos0 + S), (uint64_t)kc->cap,
                         (uint64_t)B * f.n_kv_heads, f.dtype, FT_BN));
-          // keys cut between the CTAs of a cluster: as many as stay resident (two per SM), with two key tiles each.  One-token steps of 16
+          // keys cut between the CTAs of a cluster: as many as stay resident (two per SM), with at least three key tiles each
+          // (a prompt of 512 tokens: 14 us in one piece, 17 in two).  One-token steps of 16
           // sequences at 1000 positions, 32 / 8 heads: 50 us as one row per tile, 32 x 16 CTAs; about 20 packed and cut in two
-          const int tiles = (S + tpt - 1) / tpt, key_tiles = (apos0 + S + FT_BN - 1) / FT_BN;
+          const int tiles = (S + tpt - 1) / tpt, key_tiles = (apos0 + S / 2 + FT_BN - 1) / FT_BN;  // (of an average tile)
           int lg = 0;
-          while (lg < 3 && ((long)tiles * f.n_kv_heads * B << (lg + 1)) <= 2 * c->sm_count && key_tiles >= 4 << lg) lg++;
+          while (lg < 3 && ((long)tiles * f.n_kv_heads * B << (lg + 1)) <= 2 * c->sm_count && key_tiles >= 6 << lg) lg++;
           FtParams fp{c->pf_y, S, f.n_heads, f.n_kv_heads, apos0, G, tpt, lg, sc * 1.4426950408889634f, fa_tau * 1.4426950408889634f, c->wait_err};
           RC(launch_cluster_pdl(c, attn_prefill_tc_kernel<T>, dim3((unsigned)(tiles << lg), f.n_kv_heads, B), dim3(FT_THREADS), (size_t)FT_SMEM_BYTES,
                                 1u << lg, mq, mk, mv, fp));
@@ -3131,14 +3135,13 @@ static int enqueue_mixer_layers(cake_b200_ctx *c, cake_b200_block *const *blocks
         MX(mx::latent_prep(st, dt, lp, lc));
         // the unrotated query through the key expansion: qa[m, h, :rank] = q[m, h, :dim] . uk[h]   (uk[h]: [dim, rank])
         // long steps in 16-bit D: one tensor-core product per head on column ranges of the step's buffers
-        const bool heads_tc = b->m_ukt && M >= 512 && sp.dim % TC_BK == 0 && sp.vdim % TC_BN == 0 && qw % 8 == 0;
+        const bool heads_tc = b->m_ukt && M >= 32 && sp.dim % TC_BK == 0 && sp.vdim % TC_BN == 0 && qw % 8 == 0;
         mx::HeadGemm ga{w.proj, b->m_uk, w.qa, M, sp.kv_rank, sp.dim, sp.heads, qw, (long)sp.dim * sp.kv_rank, Dk, b->n_in_pad, sp.kv_rank, sp.heads * Dk, 1};
         if (heads_tc) {
           TcExtra xa;
           xa.a_ld = b->n_in_pad;
-          for (int hh = 0; hh < sp.heads; hh++)
-            RC((listed_gemm_tc<T, TCE_PLAIN>(c, (const T *)w.proj + (size_t)hh * qw, (const T *)b->m_ukt + (size_t)hh * sp.kv_rank * sp.dim, nullptr,
-                                             (T *)w.qa + (size_t)hh * Dk, M, sp.kv_rank, sp.dim, 0, sp.heads * Dk, 0.f, xa)));
+          xa.batch = sp.heads; xa.a_step = qw; xa.c_step = Dk;
+          RC((listed_gemm_tc<T, TCE_PLAIN>(c, w.proj, b->m_ukt, nullptr, w.qa, M, sp.kv_rank, sp.dim, 0, sp.heads * Dk, 0.f, xa)));
         } else MX(mx::head_gemm(st, dt, ga, lc));
         if (w.scores && kc->v[l]) {
           // blocks of lat_tok tokens x heads rows: scores = qa . cache^T on the keys the block's last token sees, softmax with
@@ -3173,9 +3176,8 @@ static int enqueue_mixer_layers(cake_b200_ctx *c, cake_b200_block *const *blocks
         if (heads_tc) {
           TcExtra xa;
           xa.a_ld = sp.heads * sp.kv_rank;
-          for (int hh = 0; hh < sp.heads; hh++)
-            RC((listed_gemm_tc<T, TCE_PLAIN>(c, (const T *)w.lat + (size_t)hh * sp.kv_rank, (const T *)b->m_uv + (size_t)hh * sp.vdim * sp.kv_rank, nullptr,
-                                             (T *)w.att + (size_t)hh * sp.vdim, M, sp.vdim, sp.kv_rank, 0, inner, 0.f, xa)));
+          xa.batch = sp.heads; xa.a_step = sp.kv_rank; xa.c_step = sp.vdim;
+          RC((listed_gemm_tc<T, TCE_PLAIN>(c, w.lat, b->m_uv, nullptr, w.att, M, sp.vdim, sp.kv_rank, 0, inner, 0.f, xa)));
         } else MX(mx::head_gemm(st, dt, gv, lc));
       } else if (sp.kind == CAKE_B200_MIX_RETENTION) {
         const int qk = sp.heads * sp.dim;

@@ -59,6 +59,9 @@ struct TcParams {
   // k-block coordinate of W wraps at this many elements (0 = never): A = [P_hi | P_lo] against one copy of W
   int b_kwrap = 0;
   int w_early = 0;  // W is a weight: its first stages are requested before the wait for the kernel in front
+  // `batch` products in one launch (the heads of a latent-attention layer: 16 launches of 8 CTAs were 158 us for 1000 rows): product h reads
+  // A's columns from h * a_step, W's rows from h * N and writes C's columns from h * c_step (TCE_PLAIN / TCE_RESIDUAL / TCE_ACT rows of ldc)
+  int batch = 1, a_step = 0, c_step = 0;
   int *err = nullptr;
 };
 
@@ -205,10 +208,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   // work distribution: one tile per CTA and round; PAIR: one (256-row, 256-column) unit per cluster and round
   const uint32_t crank = PAIR ? cluster_rank() : 0u;
   const int first = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, stride = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
-  const int units_m = PAIR ? (tiles_m + 1) / 2 : tiles_m, n_units = units_m * tiles_n;
-  auto unit_tile = [&](int u, int &m0, int &n0) {
+  const int units_m = PAIR ? (tiles_m + 1) / 2 : tiles_m, per_product = units_m * tiles_n, n_units = per_product * p.batch;
+  auto unit_tile = [&](int u, int &m0, int &n0) -> int {  // returns the product
+    const int h = p.batch > 1 ? u / per_product : 0;
+    u -= h * per_product;
     tc_tile(u, units_m, tiles_n, BN, m0, n0);   // m0 in units of TC_BM rows of the unit grid
     if (PAIR) m0 = m0 * 2 + (int)crank * TC_BM;
+    return h;
   };
 
   if (warp == 0) {
@@ -222,10 +228,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         if (!PAIR) mbar_arrive_expect_tx(&full[st], Cfg::STAGE_BYTES);
         else if (crank == 0) mbar_arrive_expect_tx(&full[st], 2 * Cfg::STAGE_BYTES);
       };
-      auto load_a = [&](int st, int kb, int m0) {
+      auto load_a = [&](int st, int col, int m0) {
         unsigned char *d = smem + (size_t)st * Cfg::STAGE_BYTES;
-        if (PAIR) tma_load_2d_pair(d, &map_a, kb * TC_BK, m0, cluster_map(smem_u32(&full[st]), 0u));
-        else tma_load_2d(d, &map_a, kb * TC_BK, m0, &full[st]);
+        if (PAIR) tma_load_2d_pair(d, &map_a, col, m0, cluster_map(smem_u32(&full[st]), 0u));
+        else tma_load_2d(d, &map_a, col, m0, &full[st]);
       };
       auto load_w = [&](int st, int kb, int wrow) {
         unsigned char *d = smem + (size_t)st * Cfg::STAGE_BYTES + TC_BM * TC_BK * 2;
@@ -235,15 +241,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       if (p.w_early) {  // (not a grouped product: the groups are another kernel's output)
         if (first < n_units) {
           int m0, n0;
-          unit_tile(first, m0, n0);
-          for (; early < Cfg::STAGES && early < kblocks; early++) { expect(early); load_w(early, early, n0); }
+          const int h = unit_tile(first, m0, n0);
+          for (; early < Cfg::STAGES && early < kblocks; early++) { expect(early); load_w(early, early, h * p.N + n0); }
         }
         pdl_wait();
       }
       for (int t = first; t < n_units; t += stride) {
         int m0, n0;
-        unit_tile(t, m0, n0);
-        int wrow = n0;
+        const int h = unit_tile(t, m0, n0);
+        int wrow = h * p.N + n0;
         if (p.tile_group) {
           const int g = p.tile_group[m0 / TC_BM];
           if (g < 0) continue;
@@ -256,7 +262,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             expect(s);
             load_w(s, kb, wrow);
           }
-          load_a(s, kb, m0);
+          load_a(s, h * p.a_step + kb * TC_BK, m0);
           if (++s == Cfg::STAGES) { s = 0; ph ^= 1u; }
         }
       }
@@ -306,7 +312,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     int it = 0;
     for (int t = first; t < n_units; t += stride) {
       int m0, n0;
-      unit_tile(t, m0, n0);
+      const int h = unit_tile(t, m0, n0);
       if (p.tile_group && p.tile_group[m0 / TC_BM] < 0) continue;
       const int a = it & 1;
       const uint32_t aph = (uint32_t)(it >> 1) & 1u;
@@ -359,7 +365,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             }
           } else {
             uint32_t o[16];
-            const size_t off = (size_t)row * (p.ldc ? p.ldc : p.N) + n0 + c0;  // TCE_PLAIN may write a column range of a wider buffer
+            const size_t off = (size_t)row * (p.ldc ? p.ldc : p.N) + h * p.c_step + n0 + c0;  // TCE_PLAIN may write a column range of a wider buffer
             uint32_t rr[16];  // the residual row segment as four 16-byte loads (scalar 2-byte loads made this epilogue longer
                               // than a K=4096 main loop: ncu r02, o_proj 68 % tensor-pipe active against 88-91 % elsewhere)
             if (EPI == TCE_RESIDUAL) {
