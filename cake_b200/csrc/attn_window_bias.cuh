@@ -21,7 +21,7 @@
 // Nothing here follows a reference file: the reference has none of these modifiers.
 #pragma once
 #include "attn_prefill.cuh"
-#include "common.cuh"
+#include "gemm_skinny.cuh"
 #include "f32_stream.cuh"
 
 namespace cake {
@@ -213,16 +213,22 @@ __global__ void __launch_bounds__(WA_DEC_WARPS * 32) attn_window_decode_kernel(c
 // shuffles, and the registers that fed the dot product also feed the weighted sum (the key is read once).  Every group
 // keeps its own running (m, l, acc) over the keys lo + grp, lo + grp + 64, ... with U rows in flight; the groups merge in a
 // fixed order — shuffles inside a warp, shared memory across the warps — so the result does not depend on timing.
+// Long rows of few items (one token of 16 heads is 16 CTAs, four dependent loads of a group each for 1024 keys): up to eight CTAs of a
+// cluster take every parts-th run of keys and the first merges them over shared memory, again in a fixed order.
+constexpr int WA_DEC_PARTS = 8;
 template <typename T, int NCH>
 __global__ void __launch_bounds__(WA_DEC_WARPS * 32) attn_window_decode_vec_kernel(const WinAttn p) {
   pdl_launch_dependents();
+  const int parts = (int)cluster_size(), rank = parts > 1 ? (int)cluster_rank() : 0;
+  if (parts > 1) cluster_arrive();
   pdl_wait();
   constexpr int NG = WA_DEC_WARPS * 4;  // key groups of a CTA
   constexpr int U = NCH >= 3 ? 2 : 4;   // keys in flight per group
   __shared__ float sm_m[WA_DEC_WARPS], sm_l[WA_DEC_WARPS];
   __shared__ float sm_acc[WA_DEC_WARPS][WA_MAX_HD];
+  __shared__ float pm[WA_DEC_PARTS], pl[WA_DEC_PARTS], pa[WA_DEC_PARTS][WA_MAX_HD];  // first CTA: what the cluster's CTAs found
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, grp = threadIdx.x >> 3, r = threadIdx.x & 7;
-  const int item = blockIdx.x;
+  const int item = blockIdx.x / parts;
   const int h = item % p.heads, t = (item / p.heads) % p.S, b = item / (p.heads * p.S);
   const int hd = p.hd, CH = hd >> 3, G = p.heads / p.n_kv;
   const T *qrow = reinterpret_cast<const T *>(p.qkg) + (size_t)(b * p.S + t) * p.ld;
@@ -244,7 +250,7 @@ __global__ void __launch_bounds__(WA_DEC_WARPS * 32) attn_window_decode_vec_kern
   const int lo = p.window > 0 ? max(0, pi - p.window + 1) : 0;
   const float inv_cap2 = p.softcap > 0.f ? 2.0f / p.softcap : 0.f;
   float m = -INFINITY, l = 0.f;
-  for (int base = lo; base <= pi; base += NG * U) {  // the trip count is the same for every thread: the shuffles below are whole-warp
+  for (int base = lo + rank * NG * U; base <= pi; base += parts * NG * U) {  // the trip count is the same for every thread: the shuffles below are whole-warp
     uint4 kr[U][NCH];
 #pragma unroll
     for (int u = 0; u < U; u++) {
@@ -325,14 +331,39 @@ __global__ void __launch_bounds__(WA_DEC_WARPS * 32) attn_window_decode_vec_kern
   for (int w = 0; w < WA_DEC_WARPS; w++) mx = fmaxf(mx, sm_m[w]);
   float lt = 0.f;
   for (int w = 0; w < WA_DEC_WARPS; w++) lt += sm_m[w] == -INFINITY ? 0.f : sm_l[w] * expf(sm_m[w] - mx);
+  if (parts > 1) {
+    cluster_wait();
+    if (threadIdx.x == 0) {
+      st_cluster_f32(cluster_map(smem_u32(&pm[rank]), 0u), mx);
+      st_cluster_f32(cluster_map(smem_u32(&pl[rank]), 0u), lt);
+    }
+    for (int d = threadIdx.x; d < hd; d += blockDim.x) {
+      float a = 0.f;
+      for (int w = 0; w < WA_DEC_WARPS; w++)
+        if (sm_m[w] != -INFINITY) a = fmaf(sm_acc[w][d], expf(sm_m[w] - mx), a);
+      st_cluster_f32(cluster_map(smem_u32(&pa[rank][d]), 0u), a);
+    }
+    __syncwarp();
+    cluster_arrive();
+    cluster_wait();
+    if (rank != 0) return;
+    mx = -INFINITY;
+    for (int q2 = 0; q2 < parts; q2++) mx = fmaxf(mx, pm[q2]);
+    lt = 0.f;
+    for (int q2 = 0; q2 < parts; q2++) lt += pm[q2] == -INFINITY ? 0.f : pl[q2] * expf(pm[q2] - mx);
+  }
   float gate = 1.0f;
   if (p.gate_col >= 0) gate = 1.0f / (1.0f + expf(-DT<T>::to_f(qrow[p.gate_col + h])));
   const float inv = gate / lt;
   T *yo = reinterpret_cast<T *>(p.y) + (size_t)(b * p.S + t) * p.ldy + h * hd;
   for (int d = threadIdx.x; d < hd; d += blockDim.x) {
     float a = 0.f;
-    for (int w = 0; w < WA_DEC_WARPS; w++)
-      if (sm_m[w] != -INFINITY) a = fmaf(sm_acc[w][d], expf(sm_m[w] - mx), a);
+    if (parts > 1) {
+      for (int q2 = 0; q2 < parts; q2++)
+        if (pm[q2] != -INFINITY) a = fmaf(pa[q2][d], expf(pm[q2] - mx), a);
+    } else
+      for (int w = 0; w < WA_DEC_WARPS; w++)
+        if (sm_m[w] != -INFINITY) a = fmaf(sm_acc[w][d], expf(sm_m[w] - mx), a);
     yo[d] = DT<T>::from_f(a * inv);
   }
 }

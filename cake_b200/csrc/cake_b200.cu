@@ -1708,13 +1708,17 @@ template <typename T> static int listed_attention_vec(cake_b200_ctx *c, const Wi
   if (wa.hd % 8 != 0 || wa.hd > WA_MAX_HD || wa.ld % 8 != 0 || wa.kc != wa.vc || wa.gate_col < -1 ||
       (((uintptr_t)wa.qkg | (uintptr_t)wa.kc) & 15) != 0)
     return CAKE_B200_OK;
-  const dim3 grid((unsigned)((long)wa.B * wa.S * wa.heads)), block(WA_DEC_WARPS * 32);
+  // CTAs per item: while the chip has room and a group of lanes keeps four keys (its loads in flight): 16 heads of 1024 keys take four each
+  const long items = (long)wa.B * wa.S * wa.heads, keys = wa.window > 0 ? std::min(wa.window, wa.pos0 + wa.S) : wa.pos0 + wa.S;
+  int parts = 1;
+  while (parts < WA_DEC_PARTS && keys >= 512l * parts && items * parts * 2 <= 2 * c->sm_count) parts *= 2;
+  const dim3 grid((unsigned)(items * parts)), block(WA_DEC_WARPS * 32);
   *done = true;
   switch ((wa.hd + 63) / 64) {
-    case 1: return launch_pdl(c, attn_window_decode_vec_kernel<T, 1>, grid, block, 0, wa);
-    case 2: return launch_pdl(c, attn_window_decode_vec_kernel<T, 2>, grid, block, 0, wa);
-    case 3: return launch_pdl(c, attn_window_decode_vec_kernel<T, 3>, grid, block, 0, wa);
-    default: return launch_pdl(c, attn_window_decode_vec_kernel<T, 4>, grid, block, 0, wa);
+    case 1: return launch_cluster_pdl(c, attn_window_decode_vec_kernel<T, 1>, grid, block, 0, (unsigned)parts, wa);
+    case 2: return launch_cluster_pdl(c, attn_window_decode_vec_kernel<T, 2>, grid, block, 0, (unsigned)parts, wa);
+    case 3: return launch_cluster_pdl(c, attn_window_decode_vec_kernel<T, 3>, grid, block, 0, (unsigned)parts, wa);
+    default: return launch_cluster_pdl(c, attn_window_decode_vec_kernel<T, 4>, grid, block, 0, (unsigned)parts, wa);
   }
 }
 template <> int listed_attention_vec<float>(cake_b200_ctx *, const WinAttn &, bool *done) { *done = false; return CAKE_B200_OK; }

@@ -394,3 +394,21 @@ def test_greedy_generation_through_master():
         assert ctx.launch_count() > 0
     finally:
         ctx.close()
+
+
+@gpu
+@pytest.mark.parametrize("window", [0, 600])
+def test_single_tokens_on_a_long_row_share_its_keys(window):
+    """One token on 1100 cached keys: the row's keys are cut between CTAs (two to eight of them); whole prompt and plain model agree."""
+    layers = [LayerSpec(heads=2, kv_heads=1, head_dim=64, window=window, scale=0.2, softcap=9.0, ff=32),
+              LayerSpec(heads=3, kv_heads=3, head_dim=136, window=0, scale=0.1, softcap=0.0, ff=0)]
+    cfg = small_config(layers, max_seq=1200)
+    sd = make_listed_checkpoint(cfg, "bf16", seed=18)
+    toks = tokens(1103, cfg.vocab_size, 10)
+    want = plain(cfg, sd, toks, "bf16")[-3:]
+    r = Runner(cfg, sd, "bf16")
+    try:
+        r.run("a", toks[:1100], end=False)
+        assert rel_err(r.run("a", toks[1100:], [1]), want) < TOL["bf16"]
+    finally:
+        r.close()
