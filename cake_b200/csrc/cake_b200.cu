@@ -324,7 +324,7 @@ static int launch_pdl(cake_b200_ctx *c, void (*kern)(KArgs...), dim3 grid, dim3 
   return CAKE_B200_OK;
 }
 
-// the same with a thread-block cluster of `cluster` CTAs along x (TMA multicast between the CTAs of a pair)
+// the same with a thread-block cluster of `cluster` CTAs along x
 template <typename... KArgs, typename... Args>
 static int launch_cluster_pdl(cake_b200_ctx *c, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, unsigned cluster, Args... args) {
   cudaLaunchConfig_t cfg{};
@@ -1559,7 +1559,7 @@ extern "C" int cake_b200_block_load_spec(cake_b200_ctx *c, int layer_idx, const 
   const int rc = [&]() -> int {
     // one input projection: rows cat(q, k, gate); padded with zero rows to the tensor-core tile so that it can take the shape
     b->n_in = (int)(sq + skv + (t->gate ? sp->heads : 0));
-    b->n_in_pad = round_up(b->n_in, b->n_in > 1024 ? 256 : TC_BN);  // wide projections take the 128 x 256 tile
+    b->n_in_pad = round_up(b->n_in, b->n_in > 1024 ? 256 : TC_BN);  // wide projections may take the 256-column tiles
     b->gate_col = t->gate ? (int)(sq + skv) : -1;
     CU(cudaMalloc(&b->w_in, (size_t)b->n_in_pad * H * es + 16));
     CU(cudaMemsetAsync(b->w_in, 0, (size_t)b->n_in_pad * H * es, 0));

@@ -121,7 +121,8 @@ __device__ __forceinline__ void mbar_wait(uint64_t *bar, uint32_t parity) {
       : "memory");
 }
 // mbarrier wait with a bound (a try_wait suspends the thread for a while by itself): past it the wait is given up, the error flag
-// is set, and the kernel runs to its end.  The loop is one piece of assembly: written in C++ it cost the attention kernel 4 %.
+// is set, and the kernel runs to its end.  The loop is one piece of assembly: written in C++ it cost a batch of one-token
+// steps 4 % (133 against 128 us).
 constexpr uint32_t MBAR_WAIT_LIMIT = 1u << 25;
 __device__ __forceinline__ void mbar_wait_lim(uint64_t *bar, uint32_t parity, int *err) {
   uint32_t left;

@@ -9,8 +9,8 @@
 // accumulator is rounded to D before any epilogue op.
 //
 // Structure (one persistent CTA per SM, 256 threads, warp-specialised):
-//   warp 0   TMA producer: cp.async.bulk.tensor.2d of a 128x64 A tile and a 128x64 W tile per k-block into a
-//            6-stage shared-memory ring, 128-byte swizzle, completion on full[] mbarriers
+//   warp 0   TMA producer: cp.async.bulk.tensor.2d of a 128x64 A tile and a W tile (128 or 256 rows, or this CTA's half of 256 as
+//            one of a pair) per k-block into a 4- or 6-stage shared-memory ring, 128-byte swizzle, completion on full[] mbarriers
 //   warp 1   MMA issuer: one thread issues tcgen05.mma.cta_group::1.kind::f16 (M=128, N=128, K=16) x4 per
 //            k-block from shared-memory descriptors into one of two TMEM accumulators (128 lanes x 128
 //            fp32 columns each); tcgen05.commit releases the smem stage / publishes the accumulator

@@ -124,8 +124,8 @@ __global__ void __launch_bounds__(256) rmsnorm_rows_vec_kernel(const T *__restri
 }
 
 // The same operator for a few rows of any length that is a multiple of 8 and at most 8192: one CTA per row, the gains fetched before
-// the wait for the kernel in front.  A warp per row takes 16 loads and 700 dependent instructions of one lane at n = 4096, on two CTAs
-// for 16 rows: 6.3 us.
+// the wait for the kernel in front.  A warp per row holds 128 elements per lane at n = 4096 and puts 16 rows on two CTAs:
+// 6.3 us, against 4.7 for 512 rows here.
 template <typename T>
 __global__ void __launch_bounds__(256) rmsnorm_row_block_kernel(const T *__restrict__ x, const T *__restrict__ w, T *__restrict__ out, int n, float eps,
                                                                 int row_mul, int row_add) {
@@ -441,8 +441,8 @@ __global__ void advance_kernel(int *pos, int *step) {
 }
 
 // ---- argmax over logits already in memory (first maximum wins), one CTA per row --------------------
-// The row in 16-byte loads, four of them in flight per thread, where its address and V allow it: 2-byte loads, one dependent round trip
-// each, took 31 us for 151936 entries.
+// The row in 16-byte loads, four of them in flight per thread, where its address and V allow it (9 us for 151936 entries): 2-byte loads,
+// one dependent round trip each, took 62 us more per token.
 template <typename T>
 __global__ void __launch_bounds__(1024) argmax_kernel(const T *__restrict__ logits, int V, uint32_t *out) {
   __shared__ float bv[32];
