@@ -125,21 +125,19 @@ __device__ __forceinline__ void mbar_wait(uint64_t *bar, uint32_t parity) {
 // steps 4 % (133 against 128 us).
 constexpr uint32_t MBAR_WAIT_LIMIT = 1u << 25;
 __device__ __forceinline__ void mbar_wait_lim(uint64_t *bar, uint32_t parity, int *err) {
-  uint32_t left;
   asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "mov.u32 %0, %3;\n\t"
+      "{\n\t.reg .pred p, q;\n\t.reg .u32 left;\n\t"
+      "mov.u32 left, %3;\n\t"
       "WAIT_%=:\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%0], %1;\n\t"
       "@p bra DONE_%=;\n\t"
-      "sub.u32 %0, %0, 1;\n\t"
-      "setp.ne.u32 q, %0, 0;\n\t"
+      "sub.u32 left, left, 1;\n\t"
+      "setp.ne.u32 q, left, 0;\n\t"
       "@q bra WAIT_%=;\n\t"
-      "DONE_%=:\n\t}"
-      : "=&r"(left)
-      : "r"(smem_u32(bar)), "r"(parity), "n"(MBAR_WAIT_LIMIT)
+      "st.volatile.u32 [%2], 1;\n\t"
+      "DONE_%=:\n\t}" ::"r"(smem_u32(bar)),
+      "r"(parity), "l"(err), "n"(MBAR_WAIT_LIMIT)
       : "memory");
-  if (left == 0) *(volatile int *)err = 1;
 }
 
 // L2 eviction policy for data that is streamed exactly once per token (weights)
