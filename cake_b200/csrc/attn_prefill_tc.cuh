@@ -30,11 +30,12 @@ constexpr int FT_KV_BYTES = FT_BN * FT_HD * 2;  // 16 KB: two 64-key x 64-dim bo
 constexpr int FT_SMEM_BYTES = FT_Q_BYTES + 4 * FT_KV_BYTES + 1024 /*align*/ + 128 /*barriers*/;  // Q + 2 K stages + 2 V stages
 constexpr int FT_TMEM_COLS = 256;               // S/P buffers: columns 0..63 and 64..127 (P_hi | P_lo packed over S), O: 128..255
 
-__device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, int c0, int c1, int c2, uint64_t *bar) {
+__device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, int c0, int c1, int c2, uint64_t *bar, uint32_t yes = 1u) {
   asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(
+      "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %6, 0;\n\t"
+      "@p cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];\n\t}" ::"r"(
           smem_u32(dst)),
-      "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
+      "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(yes)
       : "memory");
 }
 __device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *map, int c0, int c1, int c2, int c3, uint64_t *bar) {
@@ -78,6 +79,22 @@ __device__ __forceinline__ uint64_t ft_desc_mn(const void *tile, uint32_t lbo_by
   return addr | ((uint64_t)(lbo_bytes >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
 }
 
+// barriers: Q, two stages of K, K consumed, V, V consumed, S, then P (128 arrivals), O, and the products of a CTA that gave up a wait
+constexpr int FT_BARS = 14;
+// a CTA that gave up: its copies and products in flight end before it leaves
+__device__ __forceinline__ void ft_drain(uint64_t *bars, int warp, int lane, int k_loads, int v_loads) {
+  if (warp == 4 && lane == 0) {
+    if (k_loads > 0) mbar_drain(&bars[0], 0);
+    for (int i = max(0, k_loads - 2); i < k_loads; i++) mbar_drain(&bars[1 + (i & 1)], (uint32_t)(i >> 1) & 1u);
+    for (int i = max(0, v_loads - 2); i < v_loads; i++) mbar_drain(&bars[5 + (i & 1)], (uint32_t)(i >> 1) & 1u);
+  }
+  if (warp == 5 && lane == 0) {
+    tc_commit(&bars[FT_BARS - 1]);
+    mbar_drain(&bars[FT_BARS - 1], 0);
+  }
+  __syncthreads();
+}
+
 // Query rows of a tile: the G query heads of one key head side by side, row = token * G + head, so that one pass over K and V serves
 // all of them (a step of one token has G rows, not one) and a tile of a causal prompt spans 128 / G tokens: less of its last key
 // tiles is masked.  `splits` CTAs of a cluster cut the tile's keys between them where tiles alone don't fill the chip (few rows on a
@@ -102,7 +119,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   uint64_t *bars = reinterpret_cast<uint64_t *>(v_s + 2 * FT_KV_BYTES);
   uint64_t *q_full = bars, *k_full = bars + 1, *k_empty = bars + 3, *v_full = bars + 5, *v_empty = bars + 7, *s_full = bars + 9,
            *p_full = bars + 11, *o_full = bars + 12;
-  uint32_t *tmem_ptr = reinterpret_cast<uint32_t *>(bars + 13);
+  uint32_t *tmem_ptr = reinterpret_cast<uint32_t *>(bars + FT_BARS);
+  int *gave_up = reinterpret_cast<int *>(tmem_ptr + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int S = p.S, pos0 = p.pos0, G = p.G, tpt = p.tpt, lg = p.splits_log2, splits = 1 << lg;
@@ -116,7 +134,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   const int row = (warp & 3) * 32 + lane, tok = row / G;  // softmax warps: this thread's query row and its token
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < 13; i++) mbar_init(&bars[i], i == 11 ? 128u : 1u);
+    for (int i = 0; i < FT_BARS; i++) mbar_init(&bars[i], i == 11 ? 128u : 1u);
+    *gave_up = 0;
     mbar_fence_init();
   }
   if (warp == 5) {
@@ -135,6 +154,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   const bool busy = warp < 4 && warp * 32 < rows;  // a warp without rows keeps the barriers' counts and computes nothing
   float m_run = -INFINITY, l_run = 0.f;            // m_run: reference max of the raw scores (unscaled)
 
+  int left = MBAR_TRIES;    // of this thread's waits
+  int k_loads = 0, v_loads = 0;  // warp 4: tiles requested
   if (warp == 4) {
     // ===================== TMA producer ====================================================================
     if (lane == 0 && n_tiles > 0) {
@@ -149,14 +170,16 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         const int st = j & 1;
         const uint32_t eph = (uint32_t)((j >> 1) - 1) & 1u;  // the stage's previous use (tile j-2) has been consumed
         unsigned char *kd = k_s + st * FT_KV_BYTES, *vd = v_s + st * FT_KV_BYTES;
-        if (j >= 2) mbar_wait_lim(&k_empty[st], eph, p.err);
-        mbar_arrive_expect_tx(&k_full[st], FT_KV_BYTES);
-        tma_load_3d(kd, &map_k, 0, (j0 + j) * FT_BN, slab, &k_full[st]);
-        tma_load_3d(kd + FT_KV_BYTES / 2, &map_k, 64, (j0 + j) * FT_BN, slab, &k_full[st]);
-        if (j >= 2) mbar_wait_lim(&v_empty[st], eph, p.err);
-        mbar_arrive_expect_tx(&v_full[st], FT_KV_BYTES);
-        tma_load_3d(vd, &map_v, 0, (j0 + j) * FT_BN, slab, &v_full[st]);
-        tma_load_3d(vd + FT_KV_BYTES / 2, &map_v, 64, (j0 + j) * FT_BN, slab, &v_full[st]);
+        if (j >= 2) mbar_wait_lim(&k_empty[st], eph, p.err, left);
+        mbar_arrive_expect_tx_if(left, &k_full[st], FT_KV_BYTES);
+        tma_load_3d(kd, &map_k, 0, (j0 + j) * FT_BN, slab, &k_full[st], left);
+        tma_load_3d(kd + FT_KV_BYTES / 2, &map_k, 64, (j0 + j) * FT_BN, slab, &k_full[st], left);
+        k_loads += left ? 1 : 0;
+        if (j >= 2) mbar_wait_lim(&v_empty[st], eph, p.err, left);
+        mbar_arrive_expect_tx_if(left, &v_full[st], FT_KV_BYTES);
+        tma_load_3d(vd, &map_v, 0, (j0 + j) * FT_BN, slab, &v_full[st], left);
+        tma_load_3d(vd + FT_KV_BYTES / 2, &map_v, 64, (j0 + j) * FT_BN, slab, &v_full[st], left);
+        v_loads += left ? 1 : 0;
       }
     }
     __syncwarp();
@@ -167,7 +190,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       const uint32_t idesc_o = tc_idesc<T>(FT_HD) | (1u << 16);      // M128 N128, A from TMEM, B (V) MN-major
       auto issue_s = [&](int j) {  // S_j = Q K_j^T into S buffer j&1
         const int st = j & 1;
-        mbar_wait_lim(&k_full[st], (uint32_t)(j >> 1) & 1u, p.err);
+        mbar_wait_lim(&k_full[st], (uint32_t)(j >> 1) & 1u, p.err, left);
         tc_fence_after();
         const unsigned char *kt = k_s + st * FT_KV_BYTES;
 #pragma unroll
@@ -176,17 +199,17 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           const uint64_t db = tc_smem_desc(kt + (k >> 2) * (FT_KV_BYTES / 2)) + (uint64_t)((k & 3) * 2);
           tc_mma_f16(tmem_base + (uint32_t)(st * 64), da, db, idesc_s, k ? 1u : 0u);
         }
-        tc_commit(&k_empty[st]);
-        tc_commit(&s_full[st]);
+        tc_commit(&k_empty[st], left);
+        tc_commit(&s_full[st], left);
       };
-      mbar_wait_lim(q_full, 0, p.err);
+      mbar_wait_lim(q_full, 0, p.err, left);
       issue_s(0);
       for (int j = 0; j < n_tiles; j++) {
         const int st = j & 1;
         // S of the next tile first: its buffer held P of tile j-1, whose P V is already queued ahead of it in the pipe
         if (j + 1 < n_tiles) issue_s(j + 1);
-        mbar_wait_lim(p_full, (uint32_t)j & 1u, p.err);  // P_j in TMEM (over S_j), O rescaled
-        mbar_wait_lim(&v_full[st], (uint32_t)(j >> 1) & 1u, p.err);
+        mbar_wait_lim(p_full, (uint32_t)j & 1u, p.err, left);  // P_j in TMEM (over S_j), O rescaled
+        mbar_wait_lim(&v_full[st], (uint32_t)(j >> 1) & 1u, p.err, left);
         tc_fence_after();
         const unsigned char *vt = v_s + st * FT_KV_BYTES;
 #pragma unroll
@@ -197,23 +220,23 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             const uint64_t db = ft_desc_mn(vt + ks * 2048, FT_KV_BYTES / 2);
             tc_mma_f16_ts(tmem_o, ta, db, idesc_o, (j | half | ks) ? 1u : 0u);
           }
-        tc_commit(&v_empty[st]);
-        tc_commit(o_full);
+        tc_commit(&v_empty[st], left);
+        tc_commit(o_full, left);
       }
     }
     __syncwarp();
   } else if (!busy) {
     for (int j = 0; j < n_tiles; j++) {  // (P V of tile j-1 first: an arrival for tile j must not join the barrier's previous phase)
-      if (j > 0) mbar_wait_lim(o_full, (uint32_t)(j - 1) & 1u, p.err);
+      if (j > 0) mbar_wait_lim(o_full, (uint32_t)(j - 1) & 1u, p.err, left);
       mbar_arrive(p_full);
     }
-    if (n_tiles > 0) mbar_wait_lim(o_full, (uint32_t)(n_tiles - 1) & 1u, p.err);
+    if (n_tiles > 0) mbar_wait_lim(o_full, (uint32_t)(n_tiles - 1) & 1u, p.err, left);
   } else if (n_tiles > 0) {
     // ===================== softmax / correction (thread = query row) ========================================
     const int qp = pos0 + t0 + tok;  // absolute position of this row's query
     for (int j = 0; j < n_tiles; j++) {
       const uint32_t tmem_sp = tmem_base + lane_addr + (uint32_t)((j & 1) * 64);
-      mbar_wait_lim(&s_full[j & 1], (uint32_t)(j >> 1) & 1u, p.err);
+      mbar_wait_lim(&s_full[j & 1], (uint32_t)(j >> 1) & 1u, p.err, left);
       tc_fence_after();
       float sv[FT_BN];
       {
@@ -260,7 +283,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       }
       l_run = l_run * fac + rs;
       if (j > 0) {
-        mbar_wait_lim(o_full, (uint32_t)(j - 1) & 1u, p.err);  // P V of the previous tile is complete: O stable
+        mbar_wait_lim(o_full, (uint32_t)(j - 1) & 1u, p.err, left);  // P V of the previous tile is complete: O stable
         tc_fence_after();
         if (__any_sync(0xffffffffu, resc)) {
 #pragma unroll 1
@@ -290,7 +313,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       tc_fence_before();
       mbar_arrive(p_full);
     }
-    mbar_wait_lim(o_full, (uint32_t)(n_tiles - 1) & 1u, p.err);  // every MMA of this CTA has completed
+    mbar_wait_lim(o_full, (uint32_t)(n_tiles - 1) & 1u, p.err, left);  // every MMA of this CTA has completed
     tc_fence_after();
   }
   // ---- epilogue: O / l, one rounding to D (attention.rs:346), store (b, s, h, hd) ---------------------------
@@ -369,8 +392,10 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       }
     }
   }
+  if (!left) *gave_up = 1;
   tc_fence_before();
   __syncthreads();
+  if (*gave_up) ft_drain(bars, warp, lane, k_loads, v_loads);
   if (warp == 5) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "n"(FT_TMEM_COLS) : "memory");

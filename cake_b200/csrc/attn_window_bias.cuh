@@ -44,6 +44,7 @@ struct WinAttn {
   // out_scale: a constant factor of the output
   int pool, chunk, sink_zero;
   float out_scale = 1.f;
+  int *err = nullptr;  // attn_window_tc_kernel: host-mapped, a wait that ran out
 };
 constexpr int WA_MAX_HD = 256;
 

@@ -32,7 +32,8 @@ attn_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
   uint64_t *bars = reinterpret_cast<uint64_t *>(v_s + 2 * FT_KV_BYTES);
   uint64_t *q_full = bars, *k_full = bars + 1, *k_empty = bars + 3, *v_full = bars + 5, *v_empty = bars + 7, *s_full = bars + 9,
            *p_full = bars + 11, *o_full = bars + 12;
-  uint32_t *tmem_ptr = reinterpret_cast<uint32_t *>(bars + 13);
+  uint32_t *tmem_ptr = reinterpret_cast<uint32_t *>(bars + FT_BARS);
+  int *gave_up = reinterpret_cast<int *>(tmem_ptr + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int mt = gridDim.x - 1 - blockIdx.x;  // heavy (late) query tiles first
@@ -51,7 +52,8 @@ attn_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
   const int j_add = j_lo - n_kept;
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < 13; i++) mbar_init(&bars[i], i == 11 ? 128u : 1u);
+    for (int i = 0; i < FT_BARS; i++) mbar_init(&bars[i], i == 11 ? 128u : 1u);
+    *gave_up = 0;
     mbar_fence_init();
   }
   if (warp == 5) {
@@ -66,6 +68,8 @@ attn_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
   const uint32_t tmem_base = *tmem_ptr;
   const uint32_t tmem_o = tmem_base + 128u;  // S/P buffer i at columns 64 i
 
+  int left = MBAR_TRIES;    // of this thread's waits
+  int k_loads = 0, v_loads = 0;  // warp 4: tiles requested
   if (warp == 4) {
     // ===================== TMA producer ====================================================================
     if (lane == 0) {
@@ -80,17 +84,19 @@ attn_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         const int st = j & 1;
         const uint32_t eph = (uint32_t)((j >> 1) - 1) & 1u;  // the stage's previous use (tile j-2) has been consumed
         unsigned char *kd = k_s + st * FT_KV_BYTES, *vd = v_s + st * FT_KV_BYTES;
-        if (j >= 2) mbar_wait(&k_empty[st], eph);
-        mbar_arrive_expect_tx(&k_full[st], FT_KV_BYTES);
+        if (j >= 2) mbar_wait_lim(&k_empty[st], eph, p.err, left);
+        mbar_arrive_expect_tx_if(left, &k_full[st], FT_KV_BYTES);
         const bool pooled = j < n_pool;
         const CUtensorMap *mk = pooled ? &map_pk : &map_k, *mv = pooled ? &map_pv : &map_v;
         const int krow = pooled ? j * FT_BN : (j < n_kept ? j - n_pool : j + j_add) * FT_BN - p.key0;  // rows before the buffer read as zeros and are masked
-        tma_load_3d(kd, mk, 0, krow, slab, &k_full[st]);
-        tma_load_3d(kd + FT_KV_BYTES / 2, mk, 64, krow, slab, &k_full[st]);
-        if (j >= 2) mbar_wait(&v_empty[st], eph);
-        mbar_arrive_expect_tx(&v_full[st], FT_KV_BYTES);
-        tma_load_3d(vd, mv, 0, krow, slab, &v_full[st]);
-        tma_load_3d(vd + FT_KV_BYTES / 2, mv, 64, krow, slab, &v_full[st]);
+        tma_load_3d(kd, mk, 0, krow, slab, &k_full[st], left);
+        tma_load_3d(kd + FT_KV_BYTES / 2, mk, 64, krow, slab, &k_full[st], left);
+        k_loads += left ? 1 : 0;
+        if (j >= 2) mbar_wait_lim(&v_empty[st], eph, p.err, left);
+        mbar_arrive_expect_tx_if(left, &v_full[st], FT_KV_BYTES);
+        tma_load_3d(vd, mv, 0, krow, slab, &v_full[st], left);
+        tma_load_3d(vd + FT_KV_BYTES / 2, mv, 64, krow, slab, &v_full[st], left);
+        v_loads += left ? 1 : 0;
       }
     }
   } else if (warp == 5) {
@@ -100,7 +106,7 @@ attn_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       const uint32_t idesc_o = tc_idesc<T>(FT_HD) | (1u << 16);      // M128 N128, A from TMEM, B (V) MN-major
       auto issue_s = [&](int j) {  // S_j = Q K_j^T into S buffer j&1
         const int st = j & 1;
-        mbar_wait(&k_full[st], (uint32_t)(j >> 1) & 1u);
+        mbar_wait_lim(&k_full[st], (uint32_t)(j >> 1) & 1u, p.err, left);
         tc_fence_after();
         const unsigned char *kt = k_s + st * FT_KV_BYTES;
 #pragma unroll
@@ -109,17 +115,17 @@ attn_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
           const uint64_t db = tc_smem_desc(kt + (k >> 2) * (FT_KV_BYTES / 2)) + (uint64_t)((k & 3) * 2);
           tc_mma_f16(tmem_base + (uint32_t)(st * 64), da, db, idesc_s, k ? 1u : 0u);
         }
-        tc_commit(&k_empty[st]);
-        tc_commit(&s_full[st]);
+        tc_commit(&k_empty[st], left);
+        tc_commit(&s_full[st], left);
       };
-      mbar_wait(q_full, 0);
+      mbar_wait_lim(q_full, 0, p.err, left);
       issue_s(0);
       for (int j = 0; j < n_tiles; j++) {
         const int st = j & 1;
         // S of the next tile first: its buffer held P of tile j-1, whose P V is already queued ahead of it in the pipe
         if (j + 1 < n_tiles) issue_s(j + 1);
-        mbar_wait(p_full, (uint32_t)j & 1u);  // P_j in TMEM (over S_j), O rescaled
-        mbar_wait(&v_full[st], (uint32_t)(j >> 1) & 1u);
+        mbar_wait_lim(p_full, (uint32_t)j & 1u, p.err, left);  // P_j in TMEM (over S_j), O rescaled
+        mbar_wait_lim(&v_full[st], (uint32_t)(j >> 1) & 1u, p.err, left);
         tc_fence_after();
         const unsigned char *vt = v_s + st * FT_KV_BYTES;
 #pragma unroll
@@ -130,8 +136,8 @@ attn_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
             const uint64_t db = ft_desc_mn(vt + ks * 2048, FT_KV_BYTES / 2);
             tc_mma_f16_ts(tmem_o, ta, db, idesc_o, (j | half | ks) ? 1u : 0u);
           }
-        tc_commit(&v_empty[st]);
-        tc_commit(o_full);
+        tc_commit(&v_empty[st], left);
+        tc_commit(o_full, left);
       }
     }
   } else {
@@ -150,7 +156,7 @@ attn_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     const int seen = p.pool > 0 && qp >= p.window ? (qp - p.window + 1) / p.pool : 0;
     for (int j = 0; j < n_tiles; j++) {
       const uint32_t tmem_sp = tmem_base + lane_addr + (uint32_t)((j & 1) * 64);
-      mbar_wait(&s_full[j & 1], (uint32_t)(j >> 1) & 1u);
+      mbar_wait_lim(&s_full[j & 1], (uint32_t)(j >> 1) & 1u, p.err, left);
       tc_fence_after();
       float sv[FT_BN];
       {
@@ -202,7 +208,7 @@ attn_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       }
       l_run = l_run * fac + rs;
       if (j > 0) {
-        mbar_wait(o_full, (uint32_t)(j - 1) & 1u);  // P V of the previous tile is complete: O stable
+        mbar_wait_lim(o_full, (uint32_t)(j - 1) & 1u, p.err, left);  // P V of the previous tile is complete: O stable
         tc_fence_after();
         if (__any_sync(0xffffffffu, resc)) {
 #pragma unroll 1
@@ -233,7 +239,7 @@ attn_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       mbar_arrive(p_full);
     }
     // ---- epilogue: O / l, one rounding to D (attention.rs:346), store (b, s, h, hd) ---------------------------
-    mbar_wait(o_full, (uint32_t)(n_tiles - 1) & 1u);
+    mbar_wait_lim(o_full, (uint32_t)(n_tiles - 1) & 1u, p.err, left);
     tc_fence_after();
     const int t = m0 + row;
     float gate = 1.0f;
@@ -276,8 +282,10 @@ attn_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       }
     }
   }
+  if (!left) *gave_up = 1;
   tc_fence_before();
   __syncthreads();
+  if (*gave_up) ft_drain(bars, warp, lane, k_loads, v_loads);
   if (warp == 5) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "n"(FT_TMEM_COLS) : "memory");

@@ -1669,7 +1669,9 @@ template <typename T> static int listed_attention_tc(cake_b200_ctx *c, const Win
   RC(make_tmap3(&mk, wa.kc, (uint64_t)wa.hd, (uint64_t)wa.hd, (uint64_t)(wa.pos0 + wa.S), (uint64_t)wa.cap, (uint64_t)wa.B * wa.n_kv, c->cfg.dtype, FT_BN));
   dim3 gt((wa.S + FT_BM - 1) / FT_BM, wa.heads, wa.B);
   *done = true;
-  return launch_pdl(c, attn_window_tc_kernel<T>, gt, dim3(FT_THREADS), (size_t)FT_SMEM_BYTES, mq, mk, mk, mk, mk, wa, fa_tau * 1.4426950408889634f);
+  WinAttn wp = wa;
+  wp.err = c->wait_err;
+  return launch_pdl(c, attn_window_tc_kernel<T>, gt, dim3(FT_THREADS), (size_t)FT_SMEM_BYTES, mq, mk, mk, mk, mk, wp, fa_tau * 1.4426950408889634f);
 }
 template <> int listed_attention_tc<float>(cake_b200_ctx *, const WinAttn &, bool *done) { *done = false; return CAKE_B200_OK; }
 // attn_window_tc_kernel with its optional parts (kept first keys, sink, a gate buffer, buffers that start at key0).
@@ -1699,7 +1701,9 @@ template <typename T> static int window_attention_tc(cake_b200_ctx *c, const Win
   }
   dim3 gt((wa.S + FT_BM - 1) / FT_BM, wa.heads, wa.B);
   (void)lc;  // launch_pdl counts
-  return launch_pdl(c, attn_window_tc_kernel<T>, gt, dim3(FT_THREADS), (size_t)FT_SMEM_BYTES, mq, mk, mv, mpk, mpv, wa, fa_tau * 1.4426950408889634f);
+  WinAttn wp = wa;
+  wp.err = c->wait_err;
+  return launch_pdl(c, attn_window_tc_kernel<T>, gt, dim3(FT_THREADS), (size_t)FT_SMEM_BYTES, mq, mk, mv, mpk, mpv, wp, fa_tau * 1.4426950408889634f);
 }
 template <> int window_attention_tc<float>(cake_b200_ctx *, const WinAttn &, int, uint64_t *, const void *, const void *, int) { return CAKE_B200_EINVAL; }
 // steps of a few tokens in 16-bit D with 16-byte rows: eight lanes per key (attn_window_decode_vec_kernel)
@@ -4034,6 +4038,35 @@ extern "C" int cake_b200_decode_trace(cake_b200_ctx *c, uint64_t *out_host, int 
   for (int i = 0; i < n_steps; i++) {
     const size_t slot = (size_t)((c->steps_done - n_steps + i) % MK_STEP_RING) * 8;
     for (int j = 0; j < 8; j++) out_host[(size_t)i * 8 + j] = ring[slot + j];
+  }
+  return CAKE_B200_OK;
+}
+
+/* test aid (not in the public header): a bounded wait for an mbarrier on which `arrivals` of two arrivals happen, with `tries` tries, and the same
+ * wait again by the same thread.  ok_host[i]: whether wait i ended by the arrivals, kcycles[i]: how long it took; synchronises. */
+__global__ void wait_probe_kernel(int arrivals, unsigned tries, int *err, int *ok) {
+  __shared__ uint64_t bar;
+  mbar_init(&bar, 2);
+  mbar_fence_init();
+  for (int i = 0; i < arrivals; i++) mbar_arrive(&bar);
+  int left = (int)tries;
+  for (int i = 0; i < 2; i++) {
+    const long long t0 = clock64();
+    mbar_wait_lim(&bar, 0, err, left);
+    ok[2 + i] = (int)((clock64() - t0) / 1000);
+    ok[i] = left ? 1 : 0;
+  }
+}
+extern "C" int cake_b200_debug_wait(cake_b200_ctx *c, int arrivals, unsigned tries, int *ok_host, int *kcycles) {
+  if (!c || !ok_host || !kcycles || arrivals < 0 || arrivals > 2 || tries < 1 || tries > (unsigned)MBAR_TRIES) return fail(CAKE_B200_EINVAL, "bad debug_wait arguments");
+  CU(cudaSetDevice(c->device));
+  CU(cudaStreamSynchronize(c->stream));
+  wait_probe_kernel<<<1, 1, 0, c->stream>>>(arrivals, tries, c->wait_err, (int *)c->h_pin);
+  CU(cudaGetLastError());
+  CU(cudaStreamSynchronize(c->stream));
+  for (int i = 0; i < 2; i++) {
+    ok_host[i] = (int)c->h_pin[i];
+    kcycles[i] = (int)c->h_pin[2 + i];
   }
   return CAKE_B200_OK;
 }

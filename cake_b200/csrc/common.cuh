@@ -120,23 +120,52 @@ __device__ __forceinline__ void mbar_wait(uint64_t *bar, uint32_t parity) {
       "r"(parity)
       : "memory");
 }
-// mbarrier wait with a bound (a try_wait suspends the thread for a while by itself): past it the wait is given up, the error flag
-// is set, and the kernel runs to its end.  The loop is one piece of assembly: written in C++ it cost a batch of one-token
-// steps 4 % (133 against 128 us).
-constexpr uint32_t MBAR_WAIT_LIMIT = 1u << 25;
-__device__ __forceinline__ void mbar_wait_lim(uint64_t *bar, uint32_t parity, int *err) {
+// mbarrier wait with a bound.  `left` is what the waits of a thread may still spend together in this kernel, MBAR_TRIES at first (1.3 s; a
+// kernel of a million rows takes 0.2); at 0 one has been given up, *err is set, and each later one returns after two tries.  One plain
+// try first; past it a try may suspend the thread for longer (MBAR_TRY_NS asked for, about 5 us seen), so that a wait that succeeds takes
+// few of them.  A ring's round trip bounds many products and a branch that depends on a wait keeps their loops from being unrolled, so there
+// is none: copies, the barriers they count on and commits carry left != 0 as a predicate, and a thread that has given up runs its loop
+// to the end, requests no copy and commits no product.  2000 tokens through four 0.6B layers: 673 us; without the predicates 670, with a branch behind
+// every wait 693, with a look at *err in the loop 690, with a counted loop of plain tries 711.
+// Who gives up marks the CTA; the CTA then lets its copies and products in flight end (mbar_drain), gives its tensor memory back and
+// returns.
+constexpr uint32_t MBAR_TRY_NS = 1000000;
+constexpr int MBAR_TRIES = 1 << 18;
+__device__ __forceinline__ void mbar_wait_lim(uint64_t *bar, uint32_t parity, int *err, int &left) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "@p bra DONE_%=;\n\t"
+      "WAIT_%=:\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %4;\n\t"
+      "@p bra DONE_%=;\n\t"
+      "sub.s32 %0, %0, 1;\n\t"
+      "setp.gt.s32 p, %0, 0;\n\t"
+      "@p bra WAIT_%=;\n\t"
+      "mov.u32 %0, 0;\n\t"
+      "st.volatile.u32 [%3], 1;\n\t"
+      "DONE_%=:\n\t}"
+      : "+r"(left)
+      : "r"(smem_u32(bar)), "r"(parity), "l"(err), "r"(MBAR_TRY_NS)
+      : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_expect_tx_if(uint32_t yes, uint64_t *bar, uint32_t bytes) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(smem_u32(bar)), "r"(bytes), "r"(yes)
+               : "memory");
+}
+// the wait of a CTA that has given up for what it still has in flight, bounded too
+__device__ __forceinline__ void mbar_drain(uint64_t *bar, uint32_t parity) {
   asm volatile(
       "{\n\t.reg .pred p, q;\n\t.reg .u32 left;\n\t"
-      "mov.u32 left, %3;\n\t"
+      "mov.u32 left, %2;\n\t"
       "WAIT_%=:\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%0], %1;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%0], %1, %3;\n\t"
       "@p bra DONE_%=;\n\t"
       "sub.u32 left, left, 1;\n\t"
       "setp.ne.u32 q, left, 0;\n\t"
       "@q bra WAIT_%=;\n\t"
-      "st.volatile.u32 [%2], 1;\n\t"
       "DONE_%=:\n\t}" ::"r"(smem_u32(bar)),
-      "r"(parity), "l"(err), "n"(MBAR_WAIT_LIMIT)
+      "r"(parity), "r"(MBAR_TRIES), "r"(MBAR_TRY_NS)
       : "memory");
 }
 

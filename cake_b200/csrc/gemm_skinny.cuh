@@ -82,8 +82,9 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
 gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, const SkParams p) {
   extern __shared__ unsigned char smem_raw_sk[];
   unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw_sk) + 1023) & ~(uintptr_t)1023);
-  __shared__ uint64_t full[SK_MAX_STAGES], empty[SK_MAX_STAGES], acc_full;
+  __shared__ uint64_t full[SK_MAX_STAGES], empty[SK_MAX_STAGES], acc_full, drained;
   __shared__ uint32_t tmem_ptr;
+  __shared__ int gave_up;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int S = p.split, nt = p.nt, stage_bytes = sk_stage_bytes(nt);
   const int unit = (int)blockIdx.x / S, rank = (int)blockIdx.x % S;  // the cluster's CTAs are neighbours along x
@@ -96,6 +97,8 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   if (threadIdx.x == 0) {
     for (int s = 0; s < p.stages; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
     mbar_init(&acc_full, 1);
+    mbar_init(&drained, 1);
+    gave_up = 0;
     mbar_fence_init();
   }
   if (warp == 1) {
@@ -114,6 +117,8 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     group = p.tile_group[mt];
   }
   const bool live = group >= 0;  // cluster-uniform
+  int issued = 0;                // warp 0: stages requested
+  int left = MBAR_TRIES;    // of this thread's waits
 
   if (warp == 0) {
     if (lane == 0 && live) {
@@ -129,12 +134,14 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       for (int i = 0; i < pre; i++) tma_load_2d(smem + (size_t)i * stage_bytes + SK_W_BYTES, &map_a, (kb0 + i) * TC_BK, m0, &full[i]);
       int s = 0;
       uint32_t ph = 0;
+      issued = pre;
       for (int i = pre; i < nkb; i++) {
-        mbar_wait_lim(&empty[s], ph, p.err);
+        mbar_wait_lim(&empty[s], ph, p.err, left);
         unsigned char *st = smem + (size_t)s * stage_bytes;
-        mbar_arrive_expect_tx(&full[s], (uint32_t)stage_bytes);
-        tma_load_2d(st, &map_w, (kb0 + i) * TC_BK, wrow, &full[s]);
-        tma_load_2d(st + SK_W_BYTES, &map_a, (kb0 + i) * TC_BK, m0, &full[s]);
+        mbar_arrive_expect_tx_if(left, &full[s], (uint32_t)stage_bytes);
+        tma_load_2d(st, &map_w, (kb0 + i) * TC_BK, wrow, &full[s], left);
+        tma_load_2d(st + SK_W_BYTES, &map_a, (kb0 + i) * TC_BK, m0, &full[s], left);
+        issued += left ? 1 : 0;
         if (++s == p.stages) { s = 0; ph ^= 1u; }
       }
     }
@@ -146,16 +153,16 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       int s = 0;
       uint32_t ph = 0;
       for (int i = 0; i < nkb; i++) {
-        mbar_wait_lim(&full[s], ph, p.err);
+        mbar_wait_lim(&full[s], ph, p.err, left);
         tc_fence_after();
         const unsigned char *st = smem + (size_t)s * stage_bytes;
         const uint64_t dw = tc_smem_desc(st), da = tc_smem_desc(st + SK_W_BYTES);
 #pragma unroll
         for (int k = 0; k < TC_BK / 16; k++) tc_mma_f16(tmem, dw + (uint64_t)(k * 2), da + (uint64_t)(k * 2), idesc, (i | k) ? 1u : 0u);
-        tc_commit(&empty[s]);
+        tc_commit(&empty[s], left);
         if (++s == p.stages) { s = 0; ph ^= 1u; }
       }
-      tc_commit(&acc_full);
+      tc_commit(&acc_full, left);
     }
     __syncwarp();
   }
@@ -166,18 +173,20 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   float bias = 0.f, res0 = 0.f, res1 = 0.f;
   const int share = nt / S, f0 = m0 + rank * share;  // rows this CTA finishes: all of the tile, or its share (an even number) of them
   float *recv = reinterpret_cast<float *>(smem);     // sums on their way, over the drained ring: [source rank][row within the share][128 columns]
-  if (warp >= 2 && live) {
+  bool go = warp >= 2 && live;                       // warps that finish rows
+  if (go) {
     if (EPI == TCE_PLAIN && p.bias) bias = DT<T>::to_f(reinterpret_cast<const T *>(p.bias)[n]);
     res0 = sk_residual<T, EPI>(p, f0, m_end, n);
     res1 = sk_residual<T, EPI>(p, f0 + 1, m_end, n);
-    mbar_wait_lim(&acc_full, 0, p.err);
+    mbar_wait_lim(&acc_full, 0, p.err, left);
+    go = __all_sync(0xffffffffu, left != 0);
     tc_fence_after();
   }
   if (S > 1) {
     __syncwarp();
     cluster_arrive();  // every CTA's ring is drained: its MMAs have read all that was loaded
     cluster_wait();
-    if (warp >= 2 && live) {
+    if (go) {
       const uint32_t base = smem_u32(recv) + (uint32_t)(((size_t)rank * share * SK_BM + wq * 32 + lane) * 4);
       int to = 0, off = 0;  // row of A -> CTA and place within its share
       uint32_t dst = cluster_map(base, 0u);
@@ -200,7 +209,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   // The last pass is a loop of one pair of rows, not straight-line code: a kernel of a few microseconds runs its epilogue once, and
   // unrolled over 16 rows it waited for its own instructions (233 -> 315 us for four Nigenex layers).  The residual of the next pair is
   // requested before this pair is stored: C may be the residual's own buffer.
-  if (warp >= 2 && live) {
+  if (go) {
     const int step = S == 1 ? 16 : share;
     float *mine = recv + wq * 32 + lane;
 #pragma unroll 1
@@ -237,8 +246,18 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       }
     }
   }
+  if (!left) gave_up = 1;
   tc_fence_before();
   __syncthreads();
+  if (gave_up) {
+    if (threadIdx.x == 0)
+      for (int i = max(0, issued - p.stages); i < issued; i++) mbar_drain(&full[i % p.stages], (uint32_t)(i / p.stages) & 1u);
+    if (threadIdx.x == 32) {
+      tc_commit(&drained);
+      mbar_drain(&drained, 0);
+    }
+    __syncthreads();
+  }
   if (warp == 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");

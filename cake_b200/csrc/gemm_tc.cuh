@@ -78,24 +78,28 @@ __device__ __forceinline__ void tc_tile(int t, int tiles_m, int tiles_n, int bn,
 }
 
 // ---- PTX wrappers ------------------------------------------------------------------------------------
-__device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, int c0, int c1, uint64_t *bar) {
+// yes == 0: nothing (a predicate, not a branch)
+__device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, int c0, int c1, uint64_t *bar, uint32_t yes = 1u) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
+      "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %5, 0;\n\t"
+      "@p cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n\t}" ::"r"(
           smem_u32(dst)),
-      "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1)
+      "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(yes)
       : "memory");
 }
 // the same load with its completion counted on a barrier of the pair's first CTA (a shared::cluster address)
-__device__ __forceinline__ void tma_load_2d_pair(void *dst, const CUtensorMap *map, int c0, int c1, uint32_t bar) {
+__device__ __forceinline__ void tma_load_2d_pair(void *dst, const CUtensorMap *map, int c0, int c1, uint32_t bar, uint32_t yes) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
+      "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %5, 0;\n\t"
+      "@p cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n\t}" ::"r"(
           smem_u32(dst)),
-      "l"(map), "r"(bar), "r"(c0), "r"(c1)
+      "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(yes)
       : "memory");
 }
-__device__ __forceinline__ void tc_commit_pair(uint64_t *bar) {  // arrive on the barrier at this offset in both CTAs of the pair
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
-               "h"((uint16_t)3)
+__device__ __forceinline__ void tc_commit_pair(uint64_t *bar, uint32_t yes = 1u) {  // arrive on the barrier at this offset in both CTAs of the pair
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t"
+               "@p tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}" ::"r"(smem_u32(bar)),
+               "h"((uint16_t)3), "r"(yes)
                : "memory");
 }
 __device__ __forceinline__ void tc_mma_f16_pair(uint32_t tmem_c, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
@@ -128,8 +132,10 @@ __device__ __forceinline__ uint32_t cluster_size() {
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_commit(uint64_t *bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+__device__ __forceinline__ void tc_commit(uint64_t *bar, uint32_t yes = 1u) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\t"
+               "@p tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)), "r"(yes)
+               : "memory");
 }
 __device__ __forceinline__ void tc_mma_f16(uint32_t tmem_c, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -183,7 +189,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   uint64_t *empty = full + Cfg::STAGES;
   uint64_t *acc_full = empty + Cfg::STAGES;   // [2]
   uint64_t *acc_empty = acc_full + 2;       // [2]
-  uint32_t *tmem_ptr = reinterpret_cast<uint32_t *>(acc_empty + 2);
+  uint64_t *drained = acc_empty + 2;
+  uint32_t *tmem_ptr = reinterpret_cast<uint32_t *>(drained + 1);
+  int *gave_up = reinterpret_cast<int *>(tmem_ptr + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tiles_m = (p.M + TC_BM - 1) / TC_BM, tiles_n = p.N / BN;
@@ -192,6 +200,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   if (threadIdx.x == 0) {
     for (int s = 0; s < Cfg::STAGES; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
     for (int a = 0; a < 2; a++) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], PAIR ? 8 : 4); }  // (a warp of the epilogue arrives once)
+    mbar_init(drained, 1);
+    *gave_up = 0;
     mbar_fence_init();
   }
   if (warp == 2) {  // TMEM: 2 x BN columns = two 128 x BN fp32 accumulators
@@ -222,6 +232,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     return h;
   };
 
+  int issued = 0;              // warp 0: stages requested
+  int left = MBAR_TRIES;  // of this thread's waits
   if (warp == 0) {
     // ===================== TMA producer ==================================================================
     if (lane == 0) {
@@ -230,18 +242,18 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       int s = 0, early = 0;
       uint32_t ph = 0;
       auto expect = [&](int st) {  // PAIR: the first CTA's barrier counts both CTAs' bytes
-        if (!PAIR) mbar_arrive_expect_tx(&full[st], Cfg::STAGE_BYTES);
-        else if (crank == 0) mbar_arrive_expect_tx(&full[st], 2 * Cfg::STAGE_BYTES);
+        if (!PAIR) mbar_arrive_expect_tx_if(left, &full[st], Cfg::STAGE_BYTES);
+        else if (crank == 0) mbar_arrive_expect_tx_if(left, &full[st], 2 * Cfg::STAGE_BYTES);
       };
       auto load_a = [&](int st, int col, int m0) {
         unsigned char *d = smem + (size_t)st * Cfg::STAGE_BYTES;
-        if (PAIR) tma_load_2d_pair(d, &map_a, col, m0, cluster_map(smem_u32(&full[st]), 0u));
-        else tma_load_2d(d, &map_a, col, m0, &full[st]);
+        if (PAIR) tma_load_2d_pair(d, &map_a, col, m0, cluster_map(smem_u32(&full[st]), 0u), left);
+        else tma_load_2d(d, &map_a, col, m0, &full[st], left);
       };
       auto load_w = [&](int st, int kb, int wrow) {
         unsigned char *d = smem + (size_t)st * Cfg::STAGE_BYTES + TC_BM * TC_BK * 2;
-        if (PAIR) tma_load_2d_pair(d, &map_b, kb * TC_BK, wrow + (int)crank * 128, cluster_map(smem_u32(&full[st]), 0u));  // a 128-row box: our half of the W tile
-        else tma_load_2d(d, &map_b, p.b_kwrap ? (kb * TC_BK) % p.b_kwrap : kb * TC_BK, wrow, &full[st]);
+        if (PAIR) tma_load_2d_pair(d, &map_b, kb * TC_BK, wrow + (int)crank * 128, cluster_map(smem_u32(&full[st]), 0u), left);  // a 128-row box: our half of the W tile
+        else tma_load_2d(d, &map_b, p.b_kwrap ? (kb * TC_BK) % p.b_kwrap : kb * TC_BK, wrow, &full[st], left);
       };
       if (p.w_early) {  // (not a grouped product: the groups are another kernel's output)
         if (first < n_units) {
@@ -263,11 +275,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         for (int kb = 0; kb < kblocks; kb++) {
           if (early > 0) early--;
           else {
-            mbar_wait_lim(&empty[s], ph ^ 1u, p.err);
+            mbar_wait_lim(&empty[s], ph ^ 1u, p.err, left);
             expect(s);
             load_w(s, kb, wrow);
           }
           load_a(s, h * p.a_step + kb * TC_BK, m0);
+          issued += left ? 1 : 0;
           if (++s == Cfg::STAGES) { s = 0; ph ^= 1u; }
         }
       }
@@ -288,11 +301,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         const int a = it & 1;
         const uint32_t aph = (uint32_t)(it >> 1) & 1u;
         it++;
-        mbar_wait_lim(&acc_empty[a], aph ^ 1u, p.err);  // the epilogue has drained this accumulator
+        mbar_wait_lim(&acc_empty[a], aph ^ 1u, p.err, left);  // the epilogue has drained this accumulator
         tc_fence_after();
         const uint32_t tmem_c = tmem_base + (uint32_t)(a * BN);
         for (int kb = 0; kb < kblocks; kb++) {
-          mbar_wait_lim(&full[s], ph, p.err);
+          mbar_wait_lim(&full[s], ph, p.err, left);
           tc_fence_after();
           const unsigned char *st = smem + (size_t)s * Cfg::STAGE_BYTES;
           const uint64_t da = tc_smem_desc(st), db = tc_smem_desc(st + TC_BM * TC_BK * 2);
@@ -300,12 +313,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           for (int k = 0; k < TC_BK / 16; k++)  // +32 bytes (2 x 16 B units) per K=16 slab inside the swizzle atom
             if (PAIR) tc_mma_f16_pair(tmem_c, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb | k) ? 1u : 0u);
             else tc_mma_f16(tmem_c, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb | k) ? 1u : 0u);
-          if (PAIR) tc_commit_pair(&empty[s]);  // arrives (in both CTAs) when the MMAs above have read the stage
-          else tc_commit(&empty[s]);
+          if (PAIR) tc_commit_pair(&empty[s], left);  // arrives (in both CTAs) when the MMAs above have read the stage
+          else tc_commit(&empty[s], left);
           if (++s == Cfg::STAGES) { s = 0; ph ^= 1u; }
         }
-        if (PAIR) tc_commit_pair(&acc_full[a]);  // accumulator complete
-        else tc_commit(&acc_full[a]);
+        if (PAIR) tc_commit_pair(&acc_full[a], left);  // accumulator complete
+        else tc_commit(&acc_full[a], left);
       }
     }
   } else if (warp >= 4) {
@@ -323,7 +336,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       const uint32_t aph = (uint32_t)(it >> 1) & 1u;
       it++;
       const int row = m0 + wq * 32 + lane;
-      mbar_wait_lim(&acc_full[a], aph, p.err);
+      mbar_wait_lim(&acc_full[a], aph, p.err, left);
+      if (!__all_sync(0xffffffffu, left != 0)) break;
       tc_fence_after();
 #pragma unroll 1
       for (int c0 = 0; c0 < BN; c0 += 32) {
@@ -360,8 +374,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             const size_t off = (size_t)row * p.N + n0 + c0;
             const float4 *r4 = reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(p.residual) + off);
             float4 *dst = reinterpret_cast<float4 *>(reinterpret_cast<float *>(p.C) + off);
-#pragma unroll
             const float rs = p.row_scale ? p.row_scale[row] : 1.0f;
+#pragma unroll
             for (int j = 0; j < 8; j++) {
               float4 v = r4[j];
               v.x = fmaf(rs, __uint_as_float(r[4 * j]), v.x); v.y = fmaf(rs, __uint_as_float(r[4 * j + 1]), v.y);
@@ -416,8 +430,19 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       }
     }
   }
+  if (!left) *gave_up = 1;
   tc_fence_before();
   __syncthreads();
+  if (*gave_up) {  // (PAIR: the first CTA's barriers count both CTAs' copies and products)
+    if (warp == 0 && lane == 0 && crank == 0)
+      for (int i = max(0, issued - Cfg::STAGES); i < issued; i++) mbar_drain(&full[i % Cfg::STAGES], (uint32_t)(i / Cfg::STAGES) & 1u);
+    if (warp == 1 && lane == 0 && crank == 0) {
+      if (PAIR) tc_commit_pair(drained);
+      else tc_commit(drained);
+      mbar_drain(drained, 0);
+    }
+    __syncthreads();
+  }
   if (PAIR) cluster_sync_all();  // nobody leaves while the peer may still signal our barriers or read our operands
   if (warp == 2) {
     tc_fence_after();
