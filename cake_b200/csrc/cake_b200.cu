@@ -61,6 +61,7 @@ static int fail(int code, const char *fmt, ...) {
 struct cake_b200_ctx;
 static int wait_loads(cake_b200_ctx *c);
 static int check_waits(cake_b200_ctx *c);
+static int sync_results(cake_b200_ctx *c);
 extern "C" const char *cake_b200_last_error(void) { return g_err; }
 extern "C" const char *cake_b200_version(void) { return "cake_b200 0.1 (sm_100a)"; }
 
@@ -135,7 +136,8 @@ struct cake_b200_ctx {
   cake_b200_sampling sampling{};                   // sampler of the decode graph (kind 0 = greedy)
   size_t d_ids_cap = 0, d_pen_cap = 0;
   uint32_t *h_pin = nullptr;  // pinned staging (tokens)
-  int *wait_err = nullptr;    // pinned, written by a kernel whose bounded wait ran out; reported by the next entry point
+  int *wait_err = nullptr;    // pinned, written by a kernel whose bounded wait ran out (check_waits)
+  unsigned wait_failures = 0; // how often that has been reported
   void *h_pin_x = nullptr;
   size_t h_pin_x_cap = 0;
   int nsplit = 1;
@@ -286,6 +288,7 @@ struct cake_b200_cache {
   // cake_b200_embed_at: the last token of every batch row and the position the embedding has reached
   std::vector<uint32_t> last_tok;
   int embed_len = 0;
+  unsigned wait_failures = 0;  // the context's count when the cache was created or cleared: another one, and its rows may be no results
 };
 
 template <typename U> struct TypeTag { typedef U type; };
@@ -646,8 +649,7 @@ extern "C" int cake_b200_sync(cake_b200_ctx *c) {
   CU(cudaSetDevice(c->device));
   RC(wait_loads(c));
   if (c->load_stream) CU(cudaStreamSynchronize(c->load_stream));
-  CU(cudaStreamSynchronize(c->stream));
-  return check_waits(c);
+  return sync_results(c);
 }
 extern "C" void *cake_b200_stream(cake_b200_ctx *c) { return c ? (void *)c->stream : nullptr; }
 extern "C" int cake_b200_launch_count(cake_b200_ctx *c, uint64_t *k) {
@@ -746,10 +748,21 @@ static int pipe_mark(cake_b200_ctx *c) {  // compute must not start before the u
   c->load_pending = true;
   return CAKE_B200_OK;
 }
+// A kernel whose bounded wait ran out has returned without results.  Looked at on entry and, above all, after every synchronisation that
+// hands results to the host.  The context goes on; the caches that were there hold no results until they are cleared.
 static int check_waits(cake_b200_ctx *c) {
   if (*(volatile int *)c->wait_err == 0) return CAKE_B200_OK;
   *(volatile int *)c->wait_err = 0;
-  return fail(CAKE_B200_ECUDA, "a kernel gave up a wait for its own copies: the results of the calls before this one are not valid");
+  c->wait_failures++;
+  return fail(CAKE_B200_ECUDA, "a kernel gave up a wait for its own copies: this call and the ones before it since the last synchronisation have no results");
+}
+static int sync_results(cake_b200_ctx *c) {
+  CU(cudaStreamSynchronize(c->stream));
+  return check_waits(c);
+}
+static int check_cache(const cake_b200_cache *k) {
+  if (k->wait_failures == k->ctx->wait_failures) return CAKE_B200_OK;
+  return fail(CAKE_B200_ESTATE, "a kernel gave up a wait while this cache was in use: clear it and start its sequences again");
 }
 static int wait_loads(cake_b200_ctx *c) {
   RC(check_waits(c));
@@ -879,6 +892,7 @@ extern "C" int cake_b200_cache_create(cake_b200_ctx *c, int batch, int max_seq, 
     (void)cudaGetLastError();
     return fail(CAKE_B200_ECUDA, "cache_create: %s", cudaGetErrorString(e));
   }
+  k->wait_failures = c->wait_failures;
   *out = k;
   return CAKE_B200_OK;
 }
@@ -893,6 +907,7 @@ static int cache_ensure(cake_b200_cache *k, int layer) {
 extern "C" int cake_b200_cache_clear(cake_b200_cache *k) {
   if (!k) return fail(CAKE_B200_EINVAL, "null argument");
   for (auto &l : k->len) l = 0;
+  k->wait_failures = k->ctx->wait_failures;
   k->embed_len = 0;  // recurrent state, histories and the previous token are ignored at position 0: nothing to wipe
   return CAKE_B200_OK;
 }
@@ -952,7 +967,8 @@ extern "C" int cake_b200_cache_read(cake_b200_cache *k, int block_idx, int which
   if (which && !k->v[block_idx]) return fail(CAKE_B200_EINVAL, "layer %d keeps no V cache (its values are its keys)", block_idx);
   const size_t need = (size_t)k->batch * nkv * len * hd * c->es;
   if (bytes < need) return fail(CAKE_B200_EINVAL, "cache_read needs %zu bytes", need);
-  CU(cudaStreamSynchronize(c->stream));
+  RC(sync_results(c));
+  RC(check_cache(k));
   const char *src = (const char *)(which ? k->v[block_idx] : k->k[block_idx]);
   CU(cudaMemcpy2D(out_host, (size_t)len * hd * c->es, src, (size_t)k->cap * hd * c->es, (size_t)len * hd * c->es,
                   (size_t)k->batch * nkv, cudaMemcpyDeviceToHost));
@@ -3276,6 +3292,7 @@ extern "C" int cake_b200_forward_batch(cake_b200_ctx *c, cake_b200_block *const 
     return fail(CAKE_B200_ESTATE, "index_pos %d + seq %d exceeds cache capacity %d", index_pos, seq, kc->cap);
   CU(cudaSetDevice(c->device));
   RC(wait_loads(c));
+  RC(check_cache(kc));
   bool listed = false, mixer = false;
   for (int i = 0; i < n_blocks; i++) {
     if (!blocks[i]) return fail(CAKE_B200_EINVAL, "blocks[%d] is null", i);
@@ -3360,7 +3377,7 @@ extern "C" int cake_b200_forward_batch_host(cake_b200_ctx *c, cake_b200_block *c
   CU(cudaMemcpyAsync(c->io_x, c->h_pin_x, bytes, cudaMemcpyHostToDevice, c->stream));
   RC(cake_b200_forward_batch(c, blocks, block_idx, n_blocks, kc, c->io_x, c->io_x, batch, seq, index_pos));
   CU(cudaMemcpyAsync(c->h_pin_x, c->io_x, bytes, cudaMemcpyDeviceToHost, c->stream));
-  CU(cudaStreamSynchronize(c->stream));
+  RC(sync_results(c));
   memcpy(y_host, c->h_pin_x, bytes);
   return CAKE_B200_OK;
 }
@@ -3460,6 +3477,7 @@ extern "C" int cake_b200_embed_at(cake_b200_ctx *c, cake_b200_cache *kc, const u
   if (c->pos_tab && index_pos + seq > c->pos_rows) return fail(CAKE_B200_ESTATE, "position %d exceeds the %d learned positions", index_pos + seq, c->pos_rows);
   CU(cudaSetDevice(c->device));
   RC(wait_loads(c));
+  RC(check_cache(kc));
   const size_t n = (size_t)batch * seq;
   for (size_t i = 0; i < n; i++)
     if (ids_host[i] >= (uint32_t)c->cfg.vocab) return fail(CAKE_B200_EINVAL, "token id %u at %zu out of range (vocab %d)", ids_host[i], i, c->cfg.vocab);
@@ -3540,7 +3558,7 @@ static int listed_logits_last(cake_b200_ctx *c, const void *x_dev, int batch, in
         c->launches++;
         CU(cudaMemcpyAsync(c->h_pin + b, c->d_token, 4, cudaMemcpyDeviceToHost, c->stream));
       }
-      CU(cudaStreamSynchronize(c->stream));
+      RC(sync_results(c));
       for (int b = 0; b < batch; b++) argmax_host[b] = c->h_pin[b];
     }
     return CAKE_B200_OK;
@@ -3592,7 +3610,7 @@ extern "C" int cake_b200_logits(cake_b200_ctx *c, const void *x_dev, int batch, 
     }));
     if (argmax_host) {
       CU(cudaMemcpyAsync(c->h_pin, c->hd_tokens, (size_t)batch * 4, cudaMemcpyDeviceToHost, c->stream));
-      CU(cudaStreamSynchronize(c->stream));
+      RC(sync_results(c));
       for (int b = 0; b < batch; b++) argmax_host[b] = c->h_pin[b];
     }
     return CAKE_B200_OK;
@@ -3604,7 +3622,7 @@ extern "C" int cake_b200_logits(cake_b200_ctx *c, const void *x_dev, int batch, 
     if (argmax_host) CU(cudaMemcpyAsync(c->h_pin + b, c->d_token, 4, cudaMemcpyDeviceToHost, c->stream));
   }
   if (argmax_host) {
-    CU(cudaStreamSynchronize(c->stream));
+    RC(sync_results(c));
     for (int b = 0; b < batch; b++) argmax_host[b] = c->h_pin[b];
   }
   return CAKE_B200_OK;
@@ -3615,6 +3633,7 @@ extern "C" int cake_b200_repeat_penalty_argmax(cake_b200_ctx *c, void *logits_de
                                                const uint32_t *ctx_tokens_host, int n_tokens, uint32_t *argmax_host) {
   if (!c || !logits_dev || !argmax_host) return fail(CAKE_B200_EINVAL, "null argument");
   CU(cudaSetDevice(c->device));
+  RC(check_waits(c));
   RC(apply_repeat_penalty(c, logits_dev, penalty, ctx_tokens_host, n_tokens));
   RC(DISPATCH_T(c->cfg.dtype, T_LAMBDA {
       typedef typename decltype(tag_)::type T;
@@ -3623,7 +3642,7 @@ extern "C" int cake_b200_repeat_penalty_argmax(cake_b200_ctx *c, void *logits_de
   }));
   c->launches++;
   CU(cudaMemcpyAsync(c->h_pin, c->d_token, 4, cudaMemcpyDeviceToHost, c->stream));
-  CU(cudaStreamSynchronize(c->stream));
+  RC(sync_results(c));
   *argmax_host = c->h_pin[0];
   return CAKE_B200_OK;
 }
@@ -3690,6 +3709,7 @@ extern "C" int cake_b200_sample(cake_b200_ctx *c, void *logits_dev, const cake_b
   if (!c || !logits_dev || !s || !token_host || n_tokens < 0 || (n_tokens > 0 && !ctx_tokens_host)) return fail(CAKE_B200_EINVAL, "null argument");
   RC(check_sampling(c, s));
   CU(cudaSetDevice(c->device));
+  RC(check_waits(c));
   RC(samp_reserve(c));
   RC(apply_repeat_penalty(c, logits_dev, repeat_penalty, ctx_tokens_host, n_tokens));
   const float *noise_dev = nullptr;
@@ -3706,7 +3726,7 @@ extern "C" int cake_b200_sample(cake_b200_ctx *c, void *logits_dev, const cake_b
   }));
   CU(cudaGetLastError());
   CU(cudaMemcpyAsync(c->h_pin, c->d_token, 4, cudaMemcpyDeviceToHost, c->stream));
-  CU(cudaStreamSynchronize(c->stream));
+  RC(sync_results(c));
   *token_host = c->h_pin[0];
   return CAKE_B200_OK;
 }
@@ -3911,6 +3931,7 @@ extern "C" int cake_b200_decode_begin(cake_b200_ctx *c, uint32_t first_token, in
   CU(cudaSetDevice(c->device));
   RC(wait_loads(c));
   cake_b200_cache *kc = c->g_cache;
+  RC(check_cache(kc));
   for (int l : c->g_block_idx)
     if (kc->len[l] != index_pos)
       return fail(CAKE_B200_ESTATE, "block %d: index_pos %d != cache length %d", l, index_pos, kc->len[l]);
@@ -3930,6 +3951,8 @@ extern "C" int cake_b200_decode_run(cake_b200_ctx *c, int n_steps) {
   if (!c || !c->gexec) return fail(CAKE_B200_ESTATE, "decode_build has not been called");
   CU(cudaSetDevice(c->device));
   cake_b200_cache *kc = c->g_cache;
+  RC(check_waits(c));
+  RC(check_cache(kc));
   int cur = c->g_block_idx.empty() ? 0 : kc->len[c->g_block_idx[0]];
   if (!c->g_block_idx.empty() && cur + n_steps > kc->cap)
     return fail(CAKE_B200_ESTATE, "decode_run: %d steps from position %d exceed cache capacity %d", n_steps, cur, kc->cap);
@@ -3943,7 +3966,7 @@ extern "C" int cake_b200_decode_run(cake_b200_ctx *c, int n_steps) {
 extern "C" int cake_b200_decode_tokens(cake_b200_ctx *c, uint32_t *out_host, int n) {
   if (!c || !out_host || n < 0 || n > TOKEN_RING || n > c->steps_done) return fail(CAKE_B200_EINVAL, "bad decode_tokens arguments");
   CU(cudaSetDevice(c->device));
-  CU(cudaStreamSynchronize(c->stream));
+  RC(sync_results(c));
   std::vector<uint32_t> ring(TOKEN_RING);
   CU(cudaMemcpy(ring.data(), c->token_ring, (size_t)TOKEN_RING * 4, cudaMemcpyDeviceToHost));
   for (int i = 0; i < n; i++) out_host[i] = ring[(size_t)(c->steps_done - n + i) % TOKEN_RING];
@@ -3958,7 +3981,7 @@ extern "C" int cake_b200_decode_step_host(cake_b200_ctx *c, uint32_t token_in, u
   CU(cudaMemcpyAsync(c->d_token, c->h_pin + 32, 4, cudaMemcpyHostToDevice, c->stream));
   RC(cake_b200_decode_run(c, 1));
   CU(cudaMemcpyAsync(c->h_pin + 33, c->d_token, 4, cudaMemcpyDeviceToHost, c->stream));
-  CU(cudaStreamSynchronize(c->stream));
+  RC(sync_results(c));
   *token_out = c->h_pin[33];
   return CAKE_B200_OK;
 }
@@ -3968,7 +3991,7 @@ extern "C" int cake_b200_decode_logits(cake_b200_ctx *c, void *logits_host, size
   const size_t need = (size_t)c->cfg.vocab * c->es;
   if (bytes < need) return fail(CAKE_B200_EINVAL, "decode_logits needs %zu bytes", need);
   CU(cudaSetDevice(c->device));
-  CU(cudaStreamSynchronize(c->stream));
+  RC(sync_results(c));
   CU(cudaMemcpy(logits_host, c->logits, need, cudaMemcpyDeviceToHost));
   return CAKE_B200_OK;
 }
@@ -4043,7 +4066,7 @@ extern "C" int cake_b200_decode_trace(cake_b200_ctx *c, uint64_t *out_host, int 
 }
 
 /* test aid (not in the public header): a bounded wait for an mbarrier on which `arrivals` of two arrivals happen, with `tries` tries, and the same
- * wait again by the same thread.  ok_host[i]: whether wait i ended by the arrivals, kcycles[i]: how long it took; synchronises. */
+ * wait again by the same thread.  ok_host[i]: whether wait i ended by the arrivals, kcycles[i]: how long it took; synchronises.  With ok_host NULL it only enqueues the kernel. */
 __global__ void wait_probe_kernel(int arrivals, unsigned tries, int *err, int *ok) {
   __shared__ uint64_t bar;
   mbar_init(&bar, 2);
@@ -4058,15 +4081,16 @@ __global__ void wait_probe_kernel(int arrivals, unsigned tries, int *err, int *o
   }
 }
 extern "C" int cake_b200_debug_wait(cake_b200_ctx *c, int arrivals, unsigned tries, int *ok_host, int *kcycles) {
-  if (!c || !ok_host || !kcycles || arrivals < 0 || arrivals > 2 || tries < 1 || tries > (unsigned)MBAR_TRIES) return fail(CAKE_B200_EINVAL, "bad debug_wait arguments");
+  if (!c || !kcycles || arrivals < 0 || arrivals > 2 || tries < 1 || tries > (unsigned)MBAR_TRIES) return fail(CAKE_B200_EINVAL, "bad debug_wait arguments");
   CU(cudaSetDevice(c->device));
   CU(cudaStreamSynchronize(c->stream));
-  wait_probe_kernel<<<1, 1, 0, c->stream>>>(arrivals, tries, c->wait_err, (int *)c->h_pin);
+  wait_probe_kernel<<<1, 1, 0, c->stream>>>(arrivals, tries, c->wait_err, (int *)(c->h_pin + 48));  // (not the first places: a call behind it copies its tokens there)
   CU(cudaGetLastError());
+  if (!ok_host) return CAKE_B200_OK;
   CU(cudaStreamSynchronize(c->stream));
   for (int i = 0; i < 2; i++) {
-    ok_host[i] = (int)c->h_pin[i];
-    kcycles[i] = (int)c->h_pin[2 + i];
+    ok_host[i] = (int)c->h_pin[48 + i];
+    kcycles[i] = (int)c->h_pin[48 + 2 + i];
   }
   return CAKE_B200_OK;
 }

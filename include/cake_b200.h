@@ -95,7 +95,10 @@ const char *cake_b200_version(void);
 /* ---- context ---------------------------------------------------------------------------------- */
 int cake_b200_ctx_create(int device, const cake_b200_config *cfg, cake_b200_ctx **out);
 void cake_b200_ctx_destroy(cake_b200_ctx *);
-int cake_b200_sync(cake_b200_ctx *);              /* cudaStreamSynchronize(ctx stream) */
+/* cudaStreamSynchronize(ctx stream).  CAKE_B200_ECUDA with "gave up a wait": a kernel's bounded wait for its own copies ran out and its results
+ * are not there.  Every call that synchronises and hands results to the host reports it; the caches that existed then refuse further use
+ * (CAKE_B200_ESTATE) until cake_b200_cache_clear. */
+int cake_b200_sync(cake_b200_ctx *);
 void *cake_b200_stream(cake_b200_ctx *);          /* the cudaStream_t everything is enqueued on */
 int cake_b200_launch_count(cake_b200_ctx *, uint64_t *kernels); /* kernels of this library launched so far (graph replays included) */
 

@@ -6,8 +6,8 @@ import ctypes
 import numpy as np
 import pytest
 
-from cake_b200.capi import CakeB200Error, check, lib
-from cake_b200.model import B200Transformer, Context
+from cake_b200.capi import CakeB200Error, check, lib, ptr
+from cake_b200.model import B200Transformer, Context, sampling_from_args
 from tests.util import checkpoint, medium_config, rand_x, to_np
 
 pytestmark = pytest.mark.gpu
@@ -38,5 +38,54 @@ def test_a_wait_that_runs_out_is_reported_and_the_thread_does_not_wait_again():
         y = blk.forward(x, 0, 0, ctx)
         ctx.sync()
         assert np.isfinite(to_np(y)).all()
+    finally:
+        ctx.close()
+
+
+def test_every_call_that_hands_results_to_the_host_reports_it_and_caches_in_use_are_refused():
+    """The wait runs out while the call is under way (a probe kernel in front of it in the stream): the call itself reports it."""
+    cfg = medium_config()
+    sd = checkpoint(cfg, "bf16", seed=3, peaked=True)
+    ctx = Context(cfg, sd, "bf16")
+    h, L = ctx.h, lib()
+    kcycles = (ctypes.c_int * 2)()
+    try:
+        p = cfg.model_prefix
+        check(L.cake_b200_head_load(h, *[ptr(sd[k]) for k in (p + ".embed_tokens.weight", p + ".norm.weight", "lm_head.weight")]))
+        blk = B200Transformer.load(cfg.layer_name(0), ctx)
+        x = ctx.to_device(rand_x((3, 40, cfg.hidden_size), "bf16", seed=1))
+        row, out = x[:1, :1].contiguous(), np.empty((1, 40, cfg.hidden_size), np.uint16)
+        logits = ctx.to_device(rand_x((3, cfg.vocab_size), "bf16", seed=2))
+        tok = (ctypes.c_uint32 * 3)()
+        samp = sampling_from_args(0.8, None, 0.9, 5)
+        kv = np.empty((1 << 20,), np.uint16)
+        one = (ctypes.c_void_p * 1)(blk.h)
+        zero = (ctypes.c_int * 1)(0)
+        x_host = np.zeros((1, 40, cfg.hidden_size), np.uint16)
+        calls = {
+            "sync": lambda: ctx.sync(),
+            "logits of a batch": lambda: check(L.cake_b200_logits(h, ptr(x), 3, 40, None, tok)),
+            "logits of a row": lambda: check(L.cake_b200_logits(h, ptr(row), 1, 1, None, tok)),
+            "penalty and argmax": lambda: check(L.cake_b200_repeat_penalty_argmax(h, ptr(logits), 1.1, tok, 1, tok)),
+            "sample": lambda: check(L.cake_b200_sample(h, ptr(logits), ctypes.byref(samp), 1.0, tok, 0, 0, None, tok)),
+            "cache_read": lambda: check(L.cake_b200_cache_read(ctx.cache.h, 0, 0, kv.ctypes.data, kv.nbytes)),
+            "forward on host buffers": lambda: check(L.cake_b200_forward_batch_host(h, one, zero, 1, ctx.cache.h, x_host.ctypes.data, out.ctypes.data, 1, 40, 40)),
+        }
+        for name, call in calls.items():
+            ctx.cache.clear()
+            blk.forward(x[:1], 0, 0, ctx)
+            ctx.sync()
+            probe(ctx, 1, 1 << 14, None, kcycles)   # some 70 ms: the host is inside `call` when it runs out
+            with pytest.raises(CakeB200Error, match="gave up a wait"):
+                call()
+            ctx.sync()                                          # reported once
+            with pytest.raises(CakeB200Error, match="clear it"):
+                blk.forward(row, 40, 0, ctx)
+            with pytest.raises(CakeB200Error, match="clear it"):
+                check(L.cake_b200_cache_read(ctx.cache.h, 0, 0, kv.ctypes.data, kv.nbytes))
+            ctx.cache.clear()
+            y = blk.forward(x[:1], 0, 0, ctx)
+            ctx.sync()
+            assert np.isfinite(to_np(y)).all(), name
     finally:
         ctx.close()
