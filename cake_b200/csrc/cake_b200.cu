@@ -1480,9 +1480,9 @@ static int enqueue_prefill_layers(cake_b200_ctx *c, cake_b200_block *const *bloc
           // heads: 16 us with one warp each, 4 CTAs)
           int parts = 1;
           while (parts * 4 < f.n_heads + 2 * f.n_kv_heads && (long)M * parts < 4l * c->sm_count) parts++;
-          RC(launch_pdl(c, rope_append_vec_kernel<T>, dim3((unsigned)(((long)M * parts + 3) / 4)), dim3(128), 0, (T *)c->pf_qkv, (T *)kc->k[l], (T *)kc->v[l],
+          RC(launch_pdl(c, rope_append_vec_kernel<T>, dim3((unsigned)((M + 3) / 4), (unsigned)parts), dim3(128), 0, (T *)c->pf_qkv, (T *)kc->k[l], (T *)kc->v[l],
                         (const T *)c->cos_t, (const T *)c->sin_t, (const T *)qn, (const T *)kn, B, S, f.n_heads, f.n_kv_heads, kc->cap, pos0,
-                        f.rms_eps, rope_on, parts));
+                        f.rms_eps, rope_on));
         }
         else
         RC(launch_pdl(c, rope_append_kernel<T>, dim3((unsigned)((items + 3) / 4)), dim3(128), (size_t)4 * hd * 4,

@@ -288,18 +288,17 @@ template <typename T>
 __global__ void __launch_bounds__(128) rope_append_vec_kernel(T *__restrict__ qkv, T *__restrict__ kcache, T *__restrict__ vcache,
                                                               const T *__restrict__ cos_t, const T *__restrict__ sin_t,
                                                               const T *__restrict__ q_norm, const T *__restrict__ k_norm, int B,
-                                                              int S, int n_heads, int n_kv, int cap, int pos0, float eps, int rope_on, int parts) {
+                                                              int S, int n_heads, int n_kv, int cap, int pos0, float eps, int rope_on) {
   pdl_launch_dependents();
   pdl_wait();
   constexpr int HD = 128, HC = 4;
   const int lane = threadIdx.x & 31;
   const int nh_all = n_heads + 2 * n_kv;
-  // few tokens: `parts` warps share a token's heads (groups of HC of them), or 37 tokens of 32 heads would be 10 CTAs of eight
-  // dependent round trips each
-  const long item = (long)blockIdx.x * 4 + (threadIdx.x >> 5);
-  const long tok = item / parts;
+  // few tokens: `parts` warps (of as many CTAs) share a token's heads, in groups of HC: 37 tokens of 32 heads would be 10 CTAs of eight
+  // dependent round trips each.  (A grid dimension and not a quotient: a 64-bit division in front of the loads cost 4 % of 1000 tokens.)
+  const int parts = gridDim.y, part = blockIdx.y;
+  const long tok = (long)blockIdx.x * 4 + (threadIdx.x >> 5);
   if (tok >= (long)B * S) return;
-  const int part = (int)(item % parts);
   const int t = (int)(tok % S), b = (int)(tok / S), pos = pos0 + t;
   uint32_t *row = reinterpret_cast<uint32_t *>(qkv + (size_t)tok * nh_all * HD);  // 64 words per head
   float2 c = DT<T>::unpack2(reinterpret_cast<const uint32_t *>(cos_t + (size_t)pos * (HD / 2))[lane]);
