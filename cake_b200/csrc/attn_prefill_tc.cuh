@@ -107,7 +107,8 @@ struct FtParams {
   int *err;
 };
 
-template <typename T>
+// SPLIT: clusters that cut the keys; without it every CTA sees its rows' first key in its first tile.
+template <typename T, bool SPLIT>
 __global__ void __launch_bounds__(FT_THREADS, 2)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                        const __grid_constant__ CUtensorMap map_v, const FtParams p) {
@@ -123,7 +124,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   int *gave_up = reinterpret_cast<int *>(tmem_ptr + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int S = p.S, pos0 = p.pos0, G = p.G, tpt = p.tpt, lg = p.splits_log2, splits = 1 << lg;
+  const int S = p.S, pos0 = p.pos0, G = p.G, tpt = p.tpt, lg = SPLIT ? p.splits_log2 : 0, splits = 1 << lg;
   const int rank = (int)blockIdx.x & (splits - 1);                        // the cluster's CTAs are neighbours along x
   const int mt = (int)(gridDim.x >> lg) - 1 - (int)(blockIdx.x >> lg);  // heavy (late) query tiles first
   const int kvh = blockIdx.y, b = blockIdx.z, t0 = mt * tpt;
@@ -273,7 +274,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       }
       // p = exp((s - m) / sqrt(hd)) = 2^(s c - m c), c = log2(e) / sqrt(hd): one FFMA + one MUFU.EX2 per score; 2^-inf = 0 masks
       // (a row that has seen no key of this CTA's range yet keeps m = -inf: its scores count from 0)
-      const float mc = m_run == -INFINITY ? 0.f : m_run * p.scale_log2;
+      const float mc = SPLIT && m_run == -INFINITY ? 0.f : m_run * p.scale_log2;
       float rs = 0.f;
 #pragma unroll
       for (int i = 0; i < FT_BN; i++) {
@@ -318,7 +319,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   }
   // ---- epilogue: O / l, one rounding to D (attention.rs:346), store (b, s, h, hd) ---------------------------
   T *dst = reinterpret_cast<T *>(p.y) + ((size_t)(b * S + t0 + tok) * p.n_heads + kvh * G + row - tok * G) * FT_HD;
-  if (splits == 1) {
+  if (!SPLIT) {
     if (busy) {
       const float inv = 1.0f / l_run;
 #pragma unroll 1

@@ -425,8 +425,10 @@ template <typename T> static int set_smem_attrs_T() {
 #undef SETC
   CU(cudaFuncSetAttribute(attn_prefill_mma_kernel<T, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * FA_BN * 128 * 2));
   CU(cudaFuncSetAttribute(attn_prefill_mma_kernel<T, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * FA_BN * 64 * 2));
-  CU(cudaFuncSetAttribute(attn_prefill_tc_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, FT_SMEM_BYTES));
-  CU(cudaFuncSetAttribute(attn_prefill_tc_kernel<T>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+  CU(cudaFuncSetAttribute(attn_prefill_tc_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, FT_SMEM_BYTES));
+  CU(cudaFuncSetAttribute(attn_prefill_tc_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, FT_SMEM_BYTES));
+  CU(cudaFuncSetAttribute(attn_prefill_tc_kernel<T, false>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+  CU(cudaFuncSetAttribute(attn_prefill_tc_kernel<T, true>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
 #define SETT(EPI)                                                                                                                  \
   CU(cudaFuncSetAttribute(gemm_tc_kernel<T, EPI, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<128>::SMEM_BYTES));      \
   CU(cudaFuncSetAttribute(gemm_tc_kernel<T, EPI, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<256>::SMEM_BYTES));      \
@@ -1510,8 +1512,9 @@ static int enqueue_prefill_layers(cake_b200_ctx *c, cake_b200_block *const *bloc
           int lg = 0;
           while (lg < 3 && ((long)tiles * f.n_kv_heads * B << (lg + 1)) <= 2 * c->sm_count && key_tiles >= 6 << lg) lg++;
           FtParams fp{c->pf_y, S, f.n_heads, f.n_kv_heads, apos0, G, tpt, lg, sc * 1.4426950408889634f, fa_tau * 1.4426950408889634f, c->wait_err};
-          RC(launch_cluster_pdl(c, attn_prefill_tc_kernel<T>, dim3((unsigned)(tiles << lg), f.n_kv_heads, B), dim3(FT_THREADS), (size_t)FT_SMEM_BYTES,
-                                1u << lg, mq, mk, mv, fp));
+          const dim3 ga((unsigned)(tiles << lg), f.n_kv_heads, B), ta(FT_THREADS);
+          if (lg) RC(launch_cluster_pdl(c, attn_prefill_tc_kernel<T, true>, ga, ta, (size_t)FT_SMEM_BYTES, 1u << lg, mq, mk, mv, fp));
+          else RC(launch_pdl(c, attn_prefill_tc_kernel<T, false>, ga, ta, (size_t)FT_SMEM_BYTES, mq, mk, mv, fp));
         } else if (hd == 128)
           RC(launch_pdl(c, attn_prefill_mma_kernel<T, 128>, grid, block, (size_t)4 * FA_BN * 128 * 2, (const T *)c->pf_qkv,
                         (const T *)kc->k[l] + wsoff, (const T *)kc->v[l] + wsoff, (T *)c->pf_y, S, f.n_heads, f.n_kv_heads, kc->cap, apos0, sc));
