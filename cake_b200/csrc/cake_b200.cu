@@ -1309,19 +1309,22 @@ struct TcExtra {  // optional modes of the tensor-core GEMM (TcParams in gemm_tc
   int batch = 1, a_step = 0, c_step = 0;  // side-by-side products: product i reads columns i * a_step .. of A's rows and rows i * N .. of W and
                                           // writes columns i * c_step .. of C's rows (TCE_PLAIN, with a_ld and ldc)
 };
-// Estimated microseconds of a product on gemm_tc_kernel and on gemm_skinny_kernel, from measurements of both over N 1024 .. 28672, K 1024 ..
-// 14336, 48 .. 2048 rows (one kernel after the other, weights from HBM); within 15 % of them.
-// gemm_tc: rounds of tiles over the chip; a 64-wide k-block takes 0.32 us (128 x 128, six stages in flight), 0.42 us (128 x 256, four) or 0.38
-// us (256 x 256 on a pair of SMs, six): the ring's round trip rather than its bytes.  N = 6144, K = 4096, 512 rows: 192 small tiles are two
-// rounds, 45.6 us, 48 pairs one, 29.8; N = 28672: 896 small tiles 170, 448 large ones 129, 224 pairs 101.
+// Estimated microseconds of a product on gemm_tc_kernel and on gemm_skinny_kernel, fitted to both over N 1024 .. 28672, K 1024 .. 14336, 48 ..
+// 4096 rows (one kernel after the other, weights from HBM; mostly within 15 %, the order of the three within 5 %).
+// gemm_tc: a launch with its last epilogue, the k-blocks of the first round (64 wide; the ring's round trip rather than its bytes: 128 x 128 with
+// six stages, 128 x 256 with four, 256 x 256 on a pair of SMs with six), and for every further round of tiles over the chip its k-blocks
+// or, where K is short, the epilogue of the tile in front.  The last round counts as a full one.  Small, wide, pairs in us:
+//   N = 6144, K = 4096:  300 rows 25.0, 31.7, 29.7;  512 rows 45.5, 33.7, 31.6;  1000 rows 73.4, 62.2, 56.4
+//   N = 6144, K = 1024 (gated):  1000 rows 28.7, 34.2, 35.0;  1500 rows 35.2, 34.5, 36.3
 enum { TC_SMALL = 0, TC_WIDE = 1, TC_PAIR = 2 };
 static double tc_us(const cake_b200_ctx *c, int M, int N, int K, int kind) {
   if (kind != TC_SMALL && N % 256) return 1e30;
   if (kind == TC_PAIR && M <= TC_BM) return 1e30;  // the second SM's rows would be empty
   const long tiles = kind == TC_PAIR ? (long)((M + 255) / 256) * (N / 256) : (long)((M + TC_BM - 1) / TC_BM) * (N / (kind == TC_WIDE ? 256 : 128));
-  const long at_once = kind == TC_PAIR ? c->sm_count / 2 : c->sm_count;
-  static const double kb_us[3] = {0.32, 0.42, 0.38};
-  return std::max((kind == TC_PAIR ? 6.5 : 5.5) + (double)((tiles + at_once - 1) / at_once) * (K / TC_BK) * kb_us[kind], 3.0 + 2.0 * N * K / 5.2e6);
+  const long at_once = kind == TC_PAIR ? c->sm_count / 2 : c->sm_count, rounds = (tiles + at_once - 1) / at_once;
+  static const double launch_us[3] = {5.8, 7.5, 10.5}, first_us[3] = {0.29, 0.39, 0.30}, kb_us[3] = {0.32, 0.42, 0.39}, epilogue_us[3] = {6.5, 12.5, 13.0};
+  const int kb = K / TC_BK;
+  return std::max(launch_us[kind] + kb * first_us[kind] + (double)(rounds - 1) * std::max(kb * kb_us[kind], epilogue_us[kind]), 3.0 + 2.0 * N * K / 5.2e6);
 }
 static int tc_kind(const cake_b200_ctx *c, int M, int N, int K, bool pairs) {
   int best = pairs ? TC_PAIR : TC_WIDE;
