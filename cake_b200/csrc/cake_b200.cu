@@ -1991,6 +1991,7 @@ extern "C" int cake_b200_block_load_mixer(cake_b200_ctx *c, int layer_idx, const
         RC(pipe_mark(c));
         RC(wait_loads(c));
         MX(mx::transpose_batched(c->stream, c->cfg.dtype, b->m_uk, b->m_ukt, sp->heads, sp->dim, sp->kv_rank, &c->launches));
+        CU(cudaStreamSynchronize(c->stream));  // a weight is in memory before any launch: products request its first tiles before they wait for the kernel in front
       }
     } else if (sp->kind == CAKE_B200_MIX_RETENTION) {
       RC(upload(c, (void **)&b->m_decay, sp->decay, sp->heads * sizeof(float)));
