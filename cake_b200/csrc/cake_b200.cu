@@ -1317,19 +1317,19 @@ struct TcExtra {  // optional modes of the tensor-core GEMM (TcParams in gemm_tc
 //   N = 6144, K = 4096:  300 rows 25.0, 31.7, 29.7;  512 rows 45.5, 33.7, 31.6;  1000 rows 73.4, 62.2, 56.4
 //   N = 6144, K = 1024 (gated):  1000 rows 28.7, 34.2, 35.0;  1500 rows 35.2, 34.5, 36.3
 enum { TC_SMALL = 0, TC_WIDE = 1, TC_PAIR = 2 };
-static double tc_us(const cake_b200_ctx *c, int M, int N, int K, int kind) {
+static double tc_us(int sms, int M, int N, int K, int kind) {
   if (kind != TC_SMALL && N % 256) return 1e30;
   if (kind == TC_PAIR && M <= TC_BM) return 1e30;  // the second SM's rows would be empty
   const long tiles = kind == TC_PAIR ? (long)((M + 255) / 256) * (N / 256) : (long)((M + TC_BM - 1) / TC_BM) * (N / (kind == TC_WIDE ? 256 : 128));
-  const long at_once = kind == TC_PAIR ? c->sm_count / 2 : c->sm_count, rounds = (tiles + at_once - 1) / at_once;
+  const long at_once = kind == TC_PAIR ? sms / 2 : sms, rounds = (tiles + at_once - 1) / at_once;
   static const double launch_us[3] = {5.8, 7.5, 10.5}, first_us[3] = {0.29, 0.39, 0.30}, kb_us[3] = {0.32, 0.42, 0.39}, epilogue_us[3] = {6.5, 12.5, 13.0};
   const int kb = K / TC_BK;
   return std::max(launch_us[kind] + kb * first_us[kind] + (double)(rounds - 1) * std::max(kb * kb_us[kind], epilogue_us[kind]), 3.0 + 2.0 * N * K / 5.2e6);
 }
-static int tc_kind(const cake_b200_ctx *c, int M, int N, int K, bool pairs) {
+static int tc_kind(int sms, int M, int N, int K, bool pairs) {
   int best = pairs ? TC_PAIR : TC_WIDE;
   for (int k = best - 1; k >= TC_SMALL; k--)
-    if (tc_us(c, M, N, K, k) < tc_us(c, M, N, K, best)) best = k;
+    if (tc_us(sms, M, N, K, k) < tc_us(sms, M, N, K, best)) best = k;
   return best;
 }
 // skinny: what its stages carry at the 8.9 TB/s that all SMs take in together (or W from HBM), and an epilogue that grows with the rows
@@ -1337,15 +1337,15 @@ static double skinny_us(int nt, int N, int K) {
   return std::max((double)(N / SK_BM) * (K / TC_BK) * sk_stage_bytes(nt) / 8.9e6, 2.0 * N * K / 6.4e6) + 5.5 + 0.035 * nt;
 }
 // gemm_skinny_kernel's shape for a product, or false where gemm_tc_kernel takes it.
-static bool plan_skinny(const cake_b200_ctx *c, int M, int N, int K, const TcExtra &x, SkParams *p, size_t *smem) {
+static bool plan_skinny(int sms, int M, int N, int K, const TcExtra &x, SkParams *p, size_t *smem) {
   if (x.w_live || x.b_kwrap || x.w_cols || x.w_rows || x.w_ld || x.batch > 1) return false;
   const int rows = x.tile_group ? x.group_rows : M;
   if (rows < 1 || rows > (x.tile_group ? 64 : SK_MAX_ROWS)) return false;
   p->nt = (rows + 15) / 16 * 16;
-  if (!x.tile_group && rows > 64 && skinny_us(p->nt, N, K) >= tc_us(c, M, N, K, tc_kind(c, M, N, K, true))) return false;
+  if (!x.tile_group && rows > 64 && skinny_us(p->nt, N, K) >= tc_us(sms, M, N, K, tc_kind(sms, M, N, K, true))) return false;
   p->m_tiles = x.tile_group ? M / TC_BM : 1;
   p->m_step = TC_BM;
-  const int tiles = N / SK_BM * p->m_tiles, sms = c->sm_count;
+  const int tiles = N / SK_BM * p->m_tiles;
   // The cut along K: as many CTAs as stay resident at once (three per SM up to 64 rows, two up to 127, one beyond: a ring has four stages or
   // more), each with at least two k-blocks.  N = 6144, K = 4096, 16 rows: 48 slices x 1 21.9 us, x 2 14.7, x 4 12.7, x 8 11.2 (three per SM) -
   // 15.3 with rings that let only two in, a second wave.
@@ -1358,12 +1358,18 @@ static bool plan_skinny(const cake_b200_ctx *c, int M, int N, int K, const TcExt
   *smem = sk_smem_bytes(p->nt, p->stages, p->split);
   return *smem <= SK_SMEM_MAX;
 }
+// gemm_tc_kernel's tile: the one whose rounds over the chip come out shortest; a grouped product's neighbours belong to different groups, and a
+// wrapping W has no halves
+static int plan_tiles(int sms, int M, int N, int K, const TcExtra &x) {
+  if (N % 256 && x.batch > 1) return TC_SMALL;
+  return tc_kind(sms, M, N * x.batch, K, !x.tile_group && !x.b_kwrap && N % 256 == 0);
+}
 template <typename T, int EPI>
 static int gemm_tc_T(cake_b200_ctx *c, const void *A, const void *W, const void *bias, const void *res, void *C, int M, int N, int K,
                      int act = -1, int ldc = 0, float cap = 0.f, const TcExtra &x = TcExtra{}) {
   SkParams sk{};
   size_t sk_smem = 0;
-  if (plan_skinny(c, M, N, K, x, &sk, &sk_smem)) {
+  if (plan_skinny(c->sm_count, M, N, K, x, &sk, &sk_smem)) {
     sk.bias = bias; sk.residual = res; sk.C = C; sk.M = M; sk.N = N; sk.K = K; sk.ldc = ldc; sk.cap = cap;
     sk.act = act >= 0 ? act : (c->cfg.use_gelu_mlp ? 1 : 0);
     sk.tile_group = x.tile_group; sk.row_scale = x.row_scale; sk.err = c->wait_err;
@@ -1373,9 +1379,8 @@ static int gemm_tc_T(cake_b200_ctx *c, const void *A, const void *W, const void 
     return launch_cluster_pdl(c, gemm_skinny_kernel<T, EPI>, dim3((unsigned)(N / SK_BM * sk.m_tiles * sk.split)), dim3(SK_THREADS), sk_smem,
                               (unsigned)sk.split, mw, ma, sk);
   }
-  // the tile whose rounds over the chip come out shortest; a grouped product's neighbours belong to different groups, and a wrapping W has no halves
   const bool weight = !x.tile_group && !x.w_live && !x.b_kwrap;
-  const int kind = N % 256 && x.batch > 1 ? (int)TC_SMALL : tc_kind(c, M, N * x.batch, K, !x.tile_group && !x.b_kwrap && N % 256 == 0);
+  const int kind = plan_tiles(c->sm_count, M, N, K, x);
   const int tiles_m = (M + TC_BM - 1) / TC_BM, bn = kind == TC_SMALL ? 128 : 256;
   CUtensorMap ma, mb;
   RC(make_tmap(&ma, A, (uint64_t)M, (uint64_t)K + (uint64_t)(x.batch - 1) * x.a_step, c->cfg.dtype, TC_BM, (uint64_t)x.a_ld));
@@ -4102,6 +4107,51 @@ extern "C" int cake_b200_debug_wait(cake_b200_ctx *c, int arrivals, unsigned tri
     kcycles[i] = (int)c->h_pin[48 + 2 + i];
   }
   return CAKE_B200_OK;
+}
+
+/* test aids (not in the public header): the kernel of a product of M rows, N columns, K ({0, 1, 2 = gemm_tc_kernel small, wide, pairs; 3 =
+ * gemm_skinny_kernel}, split, stages, shared memory), and one product.  group_rows > 0: grouped, M = 128 x blocks, block i of group
+ * group[i] (device memory; W holds n_groups matrices).  batch > 1: that many side by side. */
+extern "C" int cake_b200_debug_plan(int sms, int M, int N, int K, int group_rows, int batch, int *out4) {
+  if (sms < 2 || !tc_gemm_ok(M, N, K) || batch < 1 || !out4 || (group_rows > 0 && M % TC_BM)) return fail(CAKE_B200_EINVAL, "bad debug_plan arguments");
+  TcExtra x;
+  static const int some_group = 0;
+  if (group_rows > 0) { x.tile_group = &some_group; x.group_rows = group_rows; }
+  x.batch = batch;
+  SkParams sk{};
+  size_t smem = 0;
+  if (plan_skinny(sms, M, N, K, x, &sk, &smem)) {
+    out4[0] = 3; out4[1] = sk.split; out4[2] = sk.stages; out4[3] = (int)smem;
+  } else {
+    out4[0] = plan_tiles(sms, M, N, K, x); out4[1] = 1; out4[2] = 0; out4[3] = 0;
+  }
+  return CAKE_B200_OK;
+}
+extern "C" int cake_b200_debug_product(cake_b200_ctx *c, int epi, const void *A, const void *W, const void *bias, const void *res, void *C, int M, int N, int K,
+                                       int act, float cap, const int *group, int n_groups, int group_rows, const float *row_scale, int batch) {
+  if (!c || !A || !W || !C || !tc_gemm_ok(M, N, K) || batch < 1 || (group && (M % TC_BM || group_rows < 1 || n_groups < 1)) || epi < 0 || epi > TCE_ACT ||
+      ((epi == TCE_RESIDUAL || epi == TCE_RESIDUAL_F32) && !res) || (batch > 1 && (epi != TCE_PLAIN || group)) ||
+      (((uintptr_t)A | (uintptr_t)W | (uintptr_t)C | (uintptr_t)res) & 15))
+    return fail(CAKE_B200_EINVAL, "bad debug_product arguments");
+  CU(cudaSetDevice(c->device));
+  RC(wait_loads(c));
+  TcExtra x;
+  if (group) { x.tile_group = group; x.n_groups = n_groups; x.group_rows = group_rows; }
+  x.row_scale = row_scale;
+  if (batch > 1) { x.batch = batch; x.a_ld = batch * K; x.a_step = K; x.c_step = N; }
+  const int ldc = batch > 1 ? batch * N : 0;
+  RC(DISPATCH_T(c->cfg.dtype, T_LAMBDA {
+    typedef typename decltype(tag_)::type T;
+    switch (epi) {
+      case TCE_PLAIN: return gemm_tc_T<T, TCE_PLAIN>(c, A, W, bias, res, C, M, N, K, act, ldc, cap, x);
+      case TCE_RESIDUAL: return gemm_tc_T<T, TCE_RESIDUAL>(c, A, W, bias, res, C, M, N, K, act, ldc, cap, x);
+      case TCE_SWIGLU: return gemm_tc_T<T, TCE_SWIGLU>(c, A, W, bias, res, C, M, N, K, act, ldc, cap, x);
+      case TCE_RESIDUAL_F32: return gemm_tc_T<T, TCE_RESIDUAL_F32>(c, A, W, bias, res, C, M, N, K, act, ldc, cap, x);
+      case TCE_SOFTCAP_F32: return gemm_tc_T<T, TCE_SOFTCAP_F32>(c, A, W, bias, res, C, M, N, K, act, ldc, cap, x);
+      default: return gemm_tc_T<T, TCE_ACT>(c, A, W, bias, res, C, M, N, K, act, ldc, cap, x);
+    }
+  }));
+  return sync_results(c);
 }
 
 /* profiling aid (not in the public header): copies the megakernel's phase-boundary %globaltimer stamps of

@@ -71,15 +71,16 @@ def test_attention_of_a_portion_on_a_cached_context(heads, kv, batch, ctx, seq, 
 @pytest.mark.parametrize("dtype", ["bf16", "f16"])
 @pytest.mark.parametrize("batch,seq,vocab", [(2, 1, 1024), (17, 3, 1024), (64, 1, 1152), (3, 2, 1000)])   # 1000: no tiles, row by row
 def test_head_of_a_batch(batch, seq, vocab, dtype):
-    """Logits of every row's last position against the head of each row alone (another kernel, the same rounding points) and the oracle's
-    first maximum; without a logits buffer the tokens are the same."""
+    """Logits of every row's last position against the head of each row alone (another kernel, the same rounding points) and against the
+    oracle's head; the tokens are the first maxima of these logits, with and without a logits buffer."""
     cfg = medium_config(vocab_size=vocab)
     sd = checkpoint(cfg, dtype, seed=41, peaked=True)
     ctx = Context(cfg, sd, dtype)
     p = cfg.model_prefix
     head = [sd[p + ".embed_tokens.weight"], sd[p + ".norm.weight"], sd["lm_head.weight"]]
     check(lib().cake_b200_head_load(ctx.h, *[ptr(t) for t in head]))
-    x = ctx.to_device(rand_x((batch, seq, cfg.hidden_size), dtype, seed=batch))
+    x_host = rand_x((batch, seq, cfg.hidden_size), dtype, seed=batch)
+    x = ctx.to_device(x_host)
     both, alone = ctx.empty(batch, vocab), ctx.empty(batch, vocab)
     tok, tok2 = (ctypes.c_uint32 * batch)(), (ctypes.c_uint32 * batch)()
     check(lib().cake_b200_logits(ctx.h, ptr(x), batch, seq, ptr(both), tok))
@@ -88,15 +89,18 @@ def test_head_of_a_batch(batch, seq, vocab, dtype):
         check(lib().cake_b200_logits(ctx.h, ptr(x[b]), 1, seq, ptr(alone[b]), None))
     ctx.sync()
     _check(to_np(both), to_np(alone), dtype, "logits")
+    om = O.OracleModel(cfg, sd, dtype)
+    for b in range(0, batch, max(1, batch // 4)):
+        _check(to_np(both[b]), om.logits(x_host[b].float().numpy()), dtype, f"logits of row {b} against the oracle")
     first = np.argmax(to_np(both), axis=1)   # numpy's argmax is the first maximum
     assert list(tok) == list(first) == list(tok2)
     ctx.close()
 
 
 @pytest.mark.parametrize("dtype", ["bf16", "f16"])
-@pytest.mark.parametrize("rows", [129, 200, 257, 300])   # a pair's second tile with one row, between two tiles, three tiles, an odd tile count
-def test_products_of_tile_pairs(rows, dtype):
-    # gate / up: 16384 columns, two rounds of small tiles or one of pairs
+@pytest.mark.parametrize("rows", [129, 200, 257, 300])   # a second row tile with one row, a ragged one, a third with one row, a ragged third
+def test_products_of_wide_tiles(rows, dtype):
+    # gate / up: 16384 columns, two rounds of small tiles or one of wide ones (pairs of SMs: test_products.py)
     cfg = medium_config(num_attention_heads=4, num_key_value_heads=1, head_dim=128, intermediate_size=8192)
     sd = checkpoint(cfg, dtype, seed=43, std=0.03)
     om, ctx = O.OracleModel(cfg, sd, dtype), Context(cfg, sd, dtype)

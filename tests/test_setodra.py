@@ -391,6 +391,41 @@ def test_other_sizes_bf16_and_tensor_core_shapes():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("dtype", ["bf16", "f16"])
+@pytest.mark.parametrize("rows", [31, 32, 33, 129, 300])   # below, at and above the step at which the heads' expansions become one launch; row tiles
+def test_expansions_of_the_heads_in_one_launch(rows, dtype):
+    """dim, vdim and kv_rank at which the latent layer's per-head products run side by side (three heads, from 32 rows on), as a prompt and as
+    that many one-token rows of a batch."""
+    cfg = make_config([latent(heads=3, dim=128, rot_dim=64, vdim=128, kv_rank=256, scale=0.09)], width=128, vocab=96)
+    sd = make_mixer_checkpoint(cfg, dtype, seed=53)
+    toks = tokens(rows, cfg.vocab_size, seed=rows)
+    r = Runner(cfg, sd, dtype)
+    try:
+        close(r.run("w", toks), plain(cfg, sd, toks), dtype, "prompt")
+        if rows <= 33:
+            from cake_b200.model import Cache
+            r.ctx.cache = Cache(r.ctx, rows, 8)
+            got = r.model.forward(np.array(toks, dtype=np.uint32)[:, None], 0, want=list(range(rows))).cpu().numpy().reshape(rows, -1)
+            close(got, np.concatenate([plain(cfg, sd, [t]) for t in toks]), dtype, "one-token rows")
+    finally:
+        r.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [2, 17, 64, 65])
+def test_experts_of_few_rows_cut_along_k(rows):
+    """Width 1024 and ff 512: the grouped products of up to 64 rows cut their k-blocks over a cluster; 65 rows take the tiles."""
+    cfg = make_config([retention(heads=2, dim=64, vdim=64, rot_dims=32, decay=[0.95, 0.99], moe=moe(experts=4, identity=0, top=2, ff=512, shared_ff=128))], width=1024, vocab=96)
+    sd = make_mixer_checkpoint(cfg, "bf16", seed=57)
+    toks = tokens(rows, cfg.vocab_size, seed=rows)
+    r = Runner(cfg, sd, "bf16")
+    try:
+        close(r.run("w", toks), plain(cfg, sd, toks), "bf16", "prompt")
+    finally:
+        r.close()
+
+
+@pytest.mark.gpu
 def test_long_portions_on_the_tensor_cores():
     """Sizes at which long portions in bf16 take the matrix-product form of the latent attention (several blocks of rows, with
     and without keys from earlier portions) and the grouped expert products, against the plain model and against the same
