@@ -20,7 +20,7 @@
 //              and O += P_hi V + P_lo V (8 x M128 N128 K16, P from TMEM, V consumed straight from its [key][hd] cache
 //              layout as an MN-major B operand)
 #pragma once
-#include "gemm_skinny.cuh"
+#include "gemm_tc.cuh"
 
 namespace cake {
 

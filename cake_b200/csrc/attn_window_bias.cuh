@@ -21,7 +21,7 @@
 // Nothing here follows a reference file: the reference has none of these modifiers.
 #pragma once
 #include "attn_prefill.cuh"
-#include "gemm_skinny.cuh"
+#include "common.cuh"
 #include "f32_stream.cuh"
 
 namespace cake {

@@ -1344,9 +1344,8 @@ static bool plan_skinny(int sms, int M, int N, int K, const TcExtra &x, SkParams
   p->nt = (rows + 15) / 16 * 16;
   if (!x.tile_group && rows > 64 && skinny_us(p->nt, N, K) >= tc_us(sms, M, N, K, tc_kind(sms, M, N, K, true))) return false;
   p->m_tiles = x.tile_group ? M / TC_BM : 1;
-  p->m_step = TC_BM;
   const int tiles = N / SK_BM * p->m_tiles;
-  // The cut along K: as many CTAs as stay resident at once (three per SM up to 64 rows, two up to 127, one beyond: a ring has four stages or
+  // The cut along K: as many CTAs as stay resident at once (three per SM up to 64 rows, two up to 112, one beyond: a ring has three stages or
   // more), each with at least two k-blocks.  N = 6144, K = 4096, 16 rows: 48 slices x 1 21.9 us, x 2 14.7, x 4 12.7, x 8 11.2 (three per SM) -
   // 15.3 with rings that let only two in, a second wave.
   const int most = p->nt <= 64 ? 3 : p->nt < 128 ? 2 : 1;
@@ -1417,7 +1416,7 @@ static int pf_reserve(cake_b200_ctx *c, size_t rows) {
   return CAKE_B200_OK;
 }
 
-// RMSNorm over M rows of n: warp-per-row vector kernel for n = 256 * {4, 8, 16, 32} and 16-byte aligned rows, else the generic one
+// RMSNorm over M rows of n, 16-byte aligned: a CTA per row for few rows, a warp per row for many of n = 1024, 2048, 4096 or 8192; else the generic one
 template <typename T>
 static int rmsnorm_rows_T(cake_b200_ctx *c, const void *x, const void *w, void *out, int M, int n, float eps) {
   const bool al = (((uintptr_t)x | (uintptr_t)w | (uintptr_t)out) & 15) == 0;
@@ -3669,7 +3668,7 @@ static int check_sampling(const cake_b200_ctx *c, const cake_b200_sampling *s) {
   return CAKE_B200_OK;
 }
 static int samp_reserve(cake_b200_ctx *c) {
-  if (!c->samp_p) CU(cudaMalloc(&c->samp_p, (size_t)c->cfg.vocab * 4 + 16));
+  if (!c->samp_p) CU(cudaMalloc(&c->samp_p, (size_t)c->cfg.vocab * 4));
   return CAKE_B200_OK;
 }
 static SampleArgs to_args(const cake_b200_sampling &s) { return SampleArgs{s.kind, s.top_k, s.temperature, s.top_p, (unsigned long long)s.seed}; }

@@ -16,7 +16,7 @@
 
 namespace cake {
 
-constexpr int SK_BM = 128, SK_THREADS = 192, SK_MAX_NT = 256, SK_MAX_SPLIT = 8, SK_MAX_STAGES = 8;
+constexpr int SK_BM = 128, SK_THREADS = 192, SK_MAX_SPLIT = 8, SK_MAX_STAGES = 8;
 constexpr int SK_MAX_ROWS = 256, SK_SMEM_MAX = 220 * 1024;
 constexpr int SK_W_BYTES = SK_BM * TC_BK * 2;  // 16 KB of W per stage
 __host__ __device__ inline int sk_stage_bytes(int nt) { return SK_W_BYTES + nt * TC_BK * 2; }
@@ -34,26 +34,11 @@ struct SkParams {
   const int *tile_group;     // as TcParams: rows sorted by group in blocks of TC_BM; a block's first nt rows are all it uses
   const float *row_scale;
   int nt;                    // rows of A per tile (a multiple of 16)
-  int m_tiles, m_step;       // row tiles and the distance between their first rows
+  int m_tiles;               // row tiles, TC_BM rows apart
   int split, stages;
   int *err;                  // host-mapped: a wait that ran out
 };
 
-__device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-__device__ __forceinline__ void st_cluster_f32(uint32_t addr, float v) {
-  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
-}
 // what an epilogue reads beside the sums, for row m of A at column n (rows past m_end: nothing)
 template <typename T, int EPI>
 __device__ __forceinline__ float sk_residual(const SkParams &p, int m, int m_end, int n) {
@@ -89,7 +74,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   const int S = p.split, nt = p.nt, stage_bytes = sk_stage_bytes(nt);
   const int unit = (int)blockIdx.x / S, rank = (int)blockIdx.x % S;  // the cluster's CTAs are neighbours along x
   const int mt = unit % p.m_tiles, n0 = (unit / p.m_tiles) * SK_BM;
-  const int m0 = mt * p.m_step, m_end = min(p.M, m0 + nt);
+  const int m0 = mt * TC_BM, m_end = min(p.M, m0 + nt);
   const int kblocks = p.K / TC_BK, kb0 = (int)((long)kblocks * rank / S), kb1 = (int)((long)kblocks * (rank + 1) / S), nkb = kb1 - kb0;
   uint32_t cols = 32;
   while ((int)cols < nt) cols <<= 1;

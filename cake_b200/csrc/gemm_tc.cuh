@@ -11,10 +11,10 @@
 // Structure (one persistent CTA per SM, 256 threads, warp-specialised):
 //   warp 0   TMA producer: cp.async.bulk.tensor.2d of a 128x64 A tile and a W tile (128 or 256 rows, or this CTA's half of 256 as
 //            one of a pair) per k-block into a 4- or 6-stage shared-memory ring, 128-byte swizzle, completion on full[] mbarriers
-//   warp 1   MMA issuer: one thread issues tcgen05.mma.cta_group::1.kind::f16 (M=128, N=128, K=16) x4 per
-//            k-block from shared-memory descriptors into one of two TMEM accumulators (128 lanes x 128
-//            fp32 columns each); tcgen05.commit releases the smem stage / publishes the accumulator
-//   warp 2   TMEM allocator (256 columns)
+//   warp 1   MMA issuer: one thread issues tcgen05.mma.kind::f16 (M = 128 with cta_group::1, 256 over a pair of SMs with
+//            cta_group::2; N = 128 or 256; K = 16) x4 per k-block from shared-memory descriptors into one of two TMEM
+//            accumulators (128 lanes x BN fp32 columns each); tcgen05.commit releases the smem stage / publishes the accumulator
+//   warp 2   TMEM allocator (2 x BN columns)
 //   warps 4-7  epilogue: tcgen05.ld 32x32b.x32 (thread = accumulator row), fused epilogue, 16-byte global
 //            stores; overlaps with the MMAs of the next tile through the second accumulator
 #pragma once
@@ -34,7 +34,6 @@ template <int BN, bool PAIR = false> struct TcCfg {
   static constexpr int STAGE_BYTES = (TC_BM + (PAIR ? BN / 2 : BN)) * TC_BK * 2;  // 32 KB | 48 KB | 32 KB
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
 };
-constexpr int TC_SMEM_BYTES = TcCfg<256>::SMEM_BYTES > TcCfg<128>::SMEM_BYTES ? TcCfg<256>::SMEM_BYTES : TcCfg<128>::SMEM_BYTES;
 // TCE_RESIDUAL_F32: C (fp32) = residual (fp32) + accumulator, nothing rounded to D — the output projection of a block whose
 // residual stream is fp32 (f32_stream.cuh)
 // TCE_SOFTCAP_F32: C (fp32) = cap * tanh(accumulator / cap) (cap == 0: the accumulator itself) — fp32 logits of such a model
@@ -109,27 +108,6 @@ __device__ __forceinline__ void tc_mma_f16_pair(uint32_t tmem_c, uint64_t desc_a
       "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-__device__ __forceinline__ uint32_t cluster_map(uint32_t saddr, uint32_t rank) {
-  uint32_t r;
-  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ uint32_t cluster_size() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(r));
-  return r;
-}
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_commit(uint64_t *bar, uint32_t yes = 1u) {
@@ -143,6 +121,16 @@ __device__ __forceinline__ void tc_mma_f16(uint32_t tmem_c, uint64_t desc_a, uin
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_c),
       "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
       : "memory");
+}
+__device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile(

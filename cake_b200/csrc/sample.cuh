@@ -20,7 +20,7 @@
 // implementation-defined there; here the candidates are ordered by probability (descending, ties by lower id).
 // Everything is deterministic: reductions and scans use fixed trees, never floating-point atomics.
 #pragma once
-#include "gemm_skinny.cuh"
+#include "common.cuh"
 
 namespace cake {
 
@@ -72,8 +72,8 @@ struct SampleShared {
 struct SampleCluster {
   SampleShared &sh;
   int rank, set = 0;
-  // v[0..N) of every thread of the cluster, combined with `op` in a fixed order; all[r * N + t]: rank r's part, for prefixes
-  template <int N, typename Op> __device__ __forceinline__ void reduce(float (&v)[N], float (&part)[SAMPLE_CTAS][N], float neutral, Op op) {
+  // v[0..N) of every thread of the cluster, combined with `op` in a fixed order
+  template <int N, typename Op> __device__ __forceinline__ void reduce(float (&v)[N], float neutral, Op op) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 #pragma unroll
     for (int t = 0; t < N; t++) {
@@ -95,29 +95,26 @@ struct SampleCluster {
     for (int t = 0; t < N; t++) {
       v[t] = neutral;
 #pragma unroll
-      for (int r = 0; r < SAMPLE_CTAS; r++) {
-        part[r][t] = sh.slot[set][r][t];
-        v[t] = op(v[t], part[r][t]);
-      }
+      for (int r = 0; r < SAMPLE_CTAS; r++) v[t] = op(v[t], sh.slot[set][r][t]);
     }
     set ^= 1;
   }
-  template <int N> __device__ __forceinline__ void sum(float (&v)[N], float (&part)[SAMPLE_CTAS][N]) {
-    reduce<N>(v, part, 0.f, [](float a, float b) { return a + b; });
+  template <int N> __device__ __forceinline__ void sum(float (&v)[N]) {
+    reduce<N>(v, 0.f, [](float a, float b) { return a + b; });
   }
   __device__ __forceinline__ float max1(float x) {
-    float v[1] = {x}, part[SAMPLE_CTAS][1];
-    reduce<1>(v, part, -INFINITY, [](float a, float b) { return fmaxf(a, b); });
+    float v[1] = {x};
+    reduce<1>(v, -INFINITY, [](float a, float b) { return fmaxf(a, b); });
     return v[0];
   }
   __device__ __forceinline__ float sum1(float x) {
-    float v[1] = {x}, part[SAMPLE_CTAS][1];
-    sum<1>(v, part);
+    float v[1] = {x};
+    sum<1>(v);
     return v[0];
   }
   __device__ __forceinline__ int min_i(int x) {  // (vocabulary indices and 0x7fffffff compare as floats' bit patterns do)
-    float v[1] = {__int_as_float(x)}, part[SAMPLE_CTAS][1];
-    reduce<1>(v, part, __int_as_float(0x7fffffff), [](float a, float b) { return __int_as_float(min(__float_as_int(a), __float_as_int(b))); });
+    float v[1] = {__int_as_float(x)};
+    reduce<1>(v, __int_as_float(0x7fffffff), [](float a, float b) { return __int_as_float(min(__float_as_int(a), __float_as_int(b))); });
     return __float_as_int(v[0]);
   }
   // exclusive prefix over the cluster's threads in vocabulary order, and the total
@@ -178,7 +175,7 @@ __device__ __forceinline__ float sample_threshold(SampleCluster &cl, const T *L,
   uint32_t lo = sample_key<T>(-INFINITY), hi = sample_key<T>(INFINITY) + 1u;
   while (hi - lo > 1u) {
     const uint32_t step = max(1u, (hi - lo) / 8u);
-    float m[7], th[7], part[SAMPLE_CTAS][7];
+    float m[7], th[7];
 #pragma unroll
     for (int t = 0; t < 7; t++) {
       m[t] = 0.f;
@@ -189,7 +186,7 @@ __device__ __forceinline__ float sample_threshold(SampleCluster &cl, const T *L,
 #pragma unroll
       for (int t = 0; t < 7; t++) m[t] += x >= th[t] ? v : 0.f;
     }
-    cl.sum<7>(m, part);
+    cl.sum<7>(m);
     int best = 0;
 #pragma unroll
     for (int t = 0; t < 7; t++)
@@ -284,13 +281,13 @@ sample_kernel(const T *__restrict__ logits, int V, SampleArgs s, float *P_global
     int need = 0x7fffffff;
     if (want_p) {
       tau = __float_as_uint(weight(DT<T>::from_f(sample_threshold<T, false>(cl, L, P, i0, i1, s.top_p))) / sum);
-      float m[1] = {0.f}, part[SAMPLE_CTAS][1], eq = 0.f, n_eq;
+      float m[1] = {0.f}, eq = 0.f, n_eq;
       for (int i = i0; i < i1; i++) {
         const uint32_t b = __float_as_uint(P[i]);
         m[0] += b > tau ? P[i] : 0.f;
         eq += b == tau ? 1.f : 0.f;
       }
-      cl.sum<1>(m, part);
+      cl.sum<1>(m);
       eq_before = cl.scan(eq, n_eq);
       need = 0;
       for (float cum = m[0]; cum < s.top_p && (float)need < n_eq; need++) cum += __uint_as_float(tau);
