@@ -1,12 +1,12 @@
 #!/usr/bin/env python
-"""bench.py — decode tok/s of the sharded transformer-block forward path (BASELINE.json's metric):
+"""bench.py — decode tok/s of the sharded transformer-block forward path (the headline metric):
 Llama-3-8B bf16, bs=1, 2k context, layers sharded over N GPUs of one box (N=1 -> all local).
 
     python bench.py [--gpus N] [--steps K] [--warmup W]          # this repo's CUDA path
     python bench.py --impl reference [...]                        # the reference's CPU path (oracle port)
     torchrun --nproc-per-node N bench.py --gpus N ...             # N > 1, one rank per GPU
-    python bench.py --model 70b [--gpus N]                        # BASELINE configs[3] as the main line
-    python bench.py --workload prefill                            # BASELINE configs[4] as the main line
+    python bench.py --model 70b [--gpus N]                        # 70B decode as the main line
+    python bench.py --workload prefill                            # prefill as the main line
     python bench.py --workload nigenex [--sizes 2k,4k,4k-hd64]    # the Nigenex design beside the closest existing block
     python bench.py --workload setodra [--sizes 1k,2k]            # the Setodra design beside the closest existing model
     python bench.py --workload nuvarax [--sizes 1k,2k]            # the Nuvarax design beside the closest existing model
@@ -25,10 +25,10 @@ explicit L2 flush is needed between steps (stated in config.l2).
 Besides the headline metric the line carries (N = 1 unless noted):
   parity     the first decoded tokens / logits of this very model checked against the oracle (every N), and the
              sha256 of all W+K greedy tokens — identical for every N because the kernels are order-deterministic
-  config0    BASELINE configs[0]: Qwen3-0.6B (f16) greedy 32 tokens, GPU tok/s beside the oracle port on the host
-  config3    BASELINE configs[3]: Llama-3-70B bf16 sharded over the 8 GPUs (only when N = 8, or --model 70b);
+  config0    Qwen3-0.6B (f16) greedy 32 tokens, GPU tok/s beside the oracle port on the host
+  config3    Llama-3-70B bf16 sharded over the 8 GPUs (only when N = 8, or --model 70b);
              config3_one_gpu at N = 1: the same model on ONE B200 (139 GB of weights fit its 180 GB)
-  config4    BASELINE configs[4]: Llama-3-8B bs=32 x 4096 prefill with its own tensor-bound roofline object
+  config4    Llama-3-8B bs=32 x 4096 prefill with its own tensor-bound roofline object
 """
 from __future__ import annotations
 
@@ -103,7 +103,7 @@ def metric_name(model: str) -> str:
 
 
 def bytes_per_token(cfg, L: float, es: int = 2) -> float:
-    """SURVEY.md §8(d): weights + lm_head + norms + embed row + KV read (length L) + KV write."""
+    """weights + lm_head + norms + embed row + KV read (length L) + KV write."""
     H, I, nh, nkv, hd, nl, V = (cfg.hidden_size, cfg.intermediate_size, cfg.num_attention_heads,
                                 cfg.num_key_value_heads, cfg.hd, cfg.num_hidden_layers, cfg.vocab_size)
     per_layer = H * (nh + 2 * nkv) * hd + nh * hd * H + 3 * H * I + 2 * H
@@ -134,7 +134,7 @@ def peaks() -> dict:
 
 class ClockSampler:
     """SM clock + throttle reasons sampled in-process through NVML every 10 ms.  NVML is initialised when the
-    sampler is created — long before any timed region; round 1 forked `nvidia-smi` right before the timed steps and
+    sampler is created — long before any timed region; forking `nvidia-smi` right before the timed steps and
     its driver-wide initialisation (all GPUs of the box) stalled one step of every leg by 10-50 ms."""
     REASONS = {0x8: "hw_slowdown", 0x40: "hw_thermal_slowdown", 0x20: "sw_thermal_slowdown", 0x4: "sw_power_cap"}
 
@@ -552,7 +552,7 @@ def decode_leg(env: Env, model: str, K: int, W: int, n_e2e: int, parity: bool, i
         "dtype": "bf16", "data": "synthetic",
         "config": {"workload": (f"{MODEL_LABEL[model]} bf16, bs=1 decode, 2k context, layers sharded over {world} B200 (contiguous ranges, "
                                 "one hidden-state hand-off per boundary)") if world > 1
-                   else f"{MODEL_LABEL[model]} bf16, 1xB200, bs=1 decode, 2k context" + (" (BASELINE.json configs[1])" if model == "8b" else ""),
+                   else f"{MODEL_LABEL[model]} bf16, 1xB200, bs=1 decode, 2k context",
                    "kv_len_start": CTX_LEN + W, "kv_cache": "synthetic fill to 2048 positions (prefill is outside the metric, master.rs:131-134)",
                    "weights": "random-init N(0,0.02) bf16, HF layout, seed 1234", "greedy": True,
                    "parallelism": f"pp{world}" if world > 1 else "single",
@@ -755,7 +755,7 @@ def parity_leg(env: Env, sh: Shard, all_tokens, cpu_leg: bool):
 
 # ------------------------------------------------------------------------------------------------
 def config0_leg(env: Env) -> dict:
-    """BASELINE configs[0]: Qwen3-0.6B (28 layers, f16 = the reference's default dtype), greedy decode of 32 tokens from
+    """Qwen3-0.6B (28 layers, f16 = the reference's default dtype), greedy decode of 32 tokens from
     one 16-token prompt: the GPU through Master.generate_text (tok/s by the reference's definition, master.rs:131-166)
     and through the decode graph, next to the oracle port on the host cores; tokens compared."""
     import numpy as np
@@ -817,7 +817,7 @@ def config0_leg(env: Env) -> dict:
         nmatch += 1
     wb = 2.0 * (cfg.num_hidden_layers * (cfg.hidden_size * (cfg.size_q + 2 * cfg.size_kv) + cfg.size_q * cfg.hidden_size + 3 * cfg.hidden_size * cfg.intermediate_size)
                 + cfg.vocab_size * cfg.hidden_size)
-    res = {"workload": "Qwen3-0.6B (28 layers, QK-norm, tied head), f16, 16-token prompt, greedy 32 tokens (BASELINE.json configs[0])",
+    res = {"workload": "Qwen3-0.6B (28 layers, QK-norm, tied head), f16, 16-token prompt, greedy 32 tokens",
            "gpu_tok_s_generate_text": out["tok_s"], "gpu_tok_s_decode_graph": graph_tok_s,
            "gpu_hbm_frac_decode_graph": wb * graph_tok_s / 1e9 / peaks()["hbm"],
            "cpu_baseline": {"value": n_new / cpu_s, "unit": "tok/s", "cores": nthreads, "kind": "port",
@@ -831,9 +831,9 @@ def config0_leg(env: Env) -> dict:
 
 
 def prefill_leg(env: Env, reps: int = 3, batch: int = 32, seq: int = 4096) -> dict:
-    """BASELINE configs[4]: Llama-3-8B bf16, bs=32 x 4096 prefill on one B200 — one Forwarder::forward_batch over all
+    """Llama-3-8B bf16, bs=32 x 4096 prefill on one B200 — one Forwarder::forward_batch over all
     32 blocks from an empty cache (x: (32, 4096, 4096)) + ln_f / lm_head on the last position of each row
-    (text_model.rs:336-352).  Tensor-bound: algorithmic FLOPs (SURVEY.md §8d) over the measured time against the
+    (text_model.rs:336-352).  Tensor-bound: algorithmic FLOPs over the measured time against the
     measured sustained bf16 tensor throughput."""
     import torch
     from cake_b200.capi import check, lib, ptr
@@ -883,7 +883,7 @@ def prefill_leg(env: Env, reps: int = 3, batch: int = 32, seq: int = 4096) -> di
     pk = peaks()
     res = {"metric": "prefill tok/s (Llama-3-8B bf16, bs=32 x 4096)", "value": M / (ms / 1e3), "unit": "tok/s", "ms_per_step": ms,
            "steps": reps, "warmup": 1, "finite": finite,
-           "config": {"workload": "Llama-3-8B bf16, 1xB200, bs=32 prefill at 4k seq, all 32 layers + last-position lm_head (BASELINE.json configs[4])",
+           "config": {"workload": "Llama-3-8B bf16, 1xB200, bs=32 prefill at 4k seq, all 32 layers + last-position lm_head",
                       "l2": "activations of one step (1 GB per (32,4096,4096) tensor) larger than L2; no flush needed"},
            "gpu_launches": int(launches), "clocks": clocks,
            "roofline": {"bound": "tensor", "achieved": round(flops / (ms * 1e-3) / 1e12, 1), "peak": pk["tc"], "unit": "TFLOP/s",
@@ -891,7 +891,7 @@ def prefill_leg(env: Env, reps: int = 3, batch: int = 32, seq: int = 4096) -> di
                         "peak_source": pk["src"] + " (sustained cuBLAS bf16, the kernel runs inside a seconds-long step)",
                         "algorithmic_flops_per_step": flops,
                         "flops_split": {"linears": flop_lin, "causal_attention": flop_att, "lm_head": flop_head},
-                        "kernels": "per layer: gemm_tc_kernel (tcgen05, 128x256 tiles, TMA-multicast CTA pairs) x4 + attn_prefill_tc_kernel (tcgen05 flash attention) + rmsnorm_rows_vec x2 + rope_append_vec; ncu: profiles/launches_prefill_r02.csv"}}
+                        "kernels": "per layer: gemm_tc_kernel (tcgen05, 256x256 tiles on SM pairs) x4 + attn_prefill_tc_kernel (tcgen05 flash attention) + rmsnorm_rows_vec x2 + rope_append_vec; ncu: profiles/launches_prefill_r02.csv"}}
     ctx.close()
     torch.cuda.empty_cache()
     return res
@@ -1646,7 +1646,7 @@ def run_cuda(args):
     parity = not args.no_parity and args.model == "8b"
     line = decode_leg(env, args.model, K, W, args.e2e_steps, parity=parity, isolated=(world == 1 and not args.no_isolated),
                       cpu_leg=(world == 1 and not args.no_cpu))
-    # ---- further BASELINE configs riding on the same line -------------------------------------------------------
+    # ---- further workloads riding on the same line -------------------------------------------------------
     if extras != "none" and args.model == "8b":
         if world == 8 or (extras == "all" and world > 1):
             guard = threading.Timer(420.0, lambda: (rank == 0 and emit(line), os._exit(0)))
