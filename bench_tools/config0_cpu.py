@@ -1,4 +1,4 @@
-"""BASELINE.json configs[0] on the CPU: Qwen3-0.6B-shaped synthetic checkpoint (f16, the reference's default dtype),
+"""The smallest workload on the CPU: Qwen3-0.6B-shaped synthetic checkpoint (f16, the reference's default dtype),
 one prompt, 32 greedy tokens, through the oracle port of the reference's CPU path (the cake binary itself cannot be
 built here).  tok/s as the reference defines it: (generated - 1) / time since the first token (master.rs:160-166).
 

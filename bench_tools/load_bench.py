@@ -1,4 +1,4 @@
-"""Weight-load throughput (SURVEY.md §8 f-2): a Llama-3-8B-shaped checkpoint of N layers is written to /dev/shm as sharded
+"""Weight-load throughput: a Llama-3-8B-shaped checkpoint of N layers is written to /dev/shm as sharded
 safetensors, read back through cake_b200.loader (mmap) and uploaded through cake_b200_block_load's pinned double-buffered
 copy pipe into the fused device layouts.   python bench_tools/load_bench.py [n_layers=8]"""
 import ctypes, os, shutil, sys, tempfile, time

@@ -97,7 +97,7 @@ def build(force: bool = False, verbose: bool = False, host: bool = True, quiet: 
 
 def build_trace(defines=("-DMK_TRACE=1",), name="libcake_b200_trace.so") -> str:
     """A/B builds of the same library with extra -D switches, written next to the product library (selected at run time with
-    CAKE_B200_LIB=<path>, bench_tools/ab.sh).  Profiling aid only; nothing in the product uses it."""
+    CAKE_B200_LIB=<path>).  Profiling aid only; nothing in the product uses it."""
     out = os.path.join(HERE, name)
     if os.path.exists(out) and all(os.path.getmtime(out) >= os.path.getmtime(s) for s in sources()):
         return out

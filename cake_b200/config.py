@@ -898,7 +898,7 @@ class CConfig(ctypes.Structure):
         )
 
 
-# Named shapes used by tests / bench (SURVEY.md §8).
+# Named shapes used by tests / bench.
 def llama3_8b(max_seq: int = 8192) -> Config:
     return Config(4096, 14336, 128256, 32, 32, 8, rms_norm_eps=1e-5, rope_theta=500000.0, max_seq_len=max_seq,
                   eos_token_id=[128001, 128009])

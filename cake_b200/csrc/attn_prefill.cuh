@@ -51,7 +51,7 @@ template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile(
 // (stride HD*2 bytes, a multiple of 128) land in 8 different bank groups
 template <int HD> __device__ __forceinline__ uint32_t fa_off(int r, int c) { return (uint32_t)(r * HD * 2 + ((c ^ (r & 7)) << 4)); }
 
-// Occupancy (ncu r02: 189 registers + 80 KB -> 2 CTAs = 2 warps per sub-partition, HMMA pipe 50 % active, issue-bound on
+// Occupancy (ncu: 189 registers + 80 KB -> 2 CTAs = 2 warps per sub-partition, HMMA pipe 50 % active, issue-bound on
 // dependent MMA chains): the Q tile is only needed until its fragments sit in registers, so it is staged in the second V
 // buffer (64 KB per CTA instead of 80), and the register budget is capped for 3 CTAs per SM.
 template <typename T, int HD>

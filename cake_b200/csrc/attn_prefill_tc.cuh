@@ -5,7 +5,7 @@
 // cake-core/src/models/common/attention.rs:299-349 (scores = q k^T * 1/sqrt(hd) in fp32, causal mask, fp32 softmax,
 // probabilities x V, one rounding to D at the end): S in fp32 from D operands, P kept to ~16 mantissa bits as
 // P_hi + P_lo (two D operands), O accumulated in fp32, rounded once.  What changes is who multiplies: mma.sync tops out
-// near 465 TFLOP/s on this part (ncu r02: HMMA pipe 50 % active at 231 TFLOP/s), a quarter of what tcgen05 delivers.
+// near 465 TFLOP/s on this part (ncu: HMMA pipe 50 % active at 231 TFLOP/s), a quarter of what tcgen05 delivers.
 //
 // One CTA = one tile of 128 query rows (the G query heads of one key head x 128 / G tokens) and a range of keys; two CTAs per SM
 // (2 x 256 TMEM columns, 2 x 97 KB shared memory), so one CTA's softmax overlaps the other's MMAs.  192 threads:

@@ -124,7 +124,7 @@ struct cake_b200_ctx {
   int *part_idx = nullptr, *d_step = nullptr;
   unsigned *attn_counters = nullptr, *argmax_counter = nullptr;
   uint32_t *d_token = nullptr, *token_ring = nullptr, *d_ids = nullptr, *d_pen = nullptr;
-  // weight upload pipe (SURVEY.md §8 f-2): mmapped safetensors -> two pinned staging buffers (filled by a few host
+  // weight upload pipe: mmapped safetensors -> two pinned staging buffers (filled by a few host
   // threads) -> cudaMemcpy(2D)Async on a copy stream straight into the fused device layouts
   cudaStream_t load_stream = nullptr;
   void *stage[2] = {nullptr, nullptr};

@@ -30,7 +30,7 @@ template <> struct DT<float> {
   static __device__ __forceinline__ float to_f(float v) { return v; }
   static __device__ __forceinline__ float from_f(float f) { return f; }
 };
-// round-trip through D: the "->D" rounding points of the reference
+// round-trip through D: the "->D" rounding points of the reference (fp32 accumulate, round to D)
 template <typename T> __device__ __forceinline__ float rnd(float f) { return DT<T>::to_f(DT<T>::from_f(f)); }
 
 template <typename T> __device__ __forceinline__ void unpack8(const uint4 &v, float (&f)[8]) {
@@ -43,7 +43,7 @@ template <typename T> __device__ __forceinline__ uint32_t pack2(float a, float b
 }
 
 // the same two roundings in ONE packed conversion (cvt.rn.{bf16x2|f16x2}.f32 = F2FP on the ALU pipe; the scalar F2F goes
-// through the quarter-rate XU pipe, which is what bound the tcgen05 attention's softmax: ncu r02, XU 81 % busy)
+// through the quarter-rate XU pipe, which is what bound the tcgen05 attention's softmax: ncu, XU 81 % busy)
 template <typename T> __device__ __forceinline__ uint32_t pack2x(float a, float b);
 template <> __device__ __forceinline__ uint32_t pack2x<__nv_bfloat16>(float a, float b) {
   const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);

@@ -398,7 +398,7 @@ __device__ __forceinline__ void mk_consume_gemv(MkRing &rg, const MkGeom &g, con
   int r0 = 0, nrows = 0, nloc = 0;
   if (dyn) {
     // A lane's columns are the same for every row of the phase, so its x slice is converted to fp32 ONCE into
-    // registers; per 16-byte weight vector the loop is 1 LDS.128 + 8 converts + 8 FMA (ncu r01: re-reading and
+    // registers; per 16-byte weight vector the loop is 1 LDS.128 + 8 converts + 8 FMA (ncu: re-reading and
     // re-converting x per vector made the loop issue-bound).  Stages arrive with their row in stage_row[].
     float xr[4][8];
 #pragma unroll

@@ -25,7 +25,7 @@
 namespace cake {
 
 // Tile: 128 x BN with BN in {128, 256}.  A 128x128 tile needs 32 KB of operands per 2.1 MFLOP k-block = 64 flop/B, i.e.
-// ~240 GB/s per SM at the tensor peak — more than one SM pulls out of L2, which is what capped round 1 at ~55 % tensor-pipe
+// ~240 GB/s per SM at the tensor peak — more than one SM pulls out of L2, which capped the kernel at ~55 % tensor-pipe
 // activity.  128x256 (all 512 TMEM columns: two 128x256 fp32 accumulators) moves 48 KB per 4.2 MFLOP = 87 flop/B.
 constexpr int TC_BM = 128, TC_BK = 64, TC_THREADS = 256;
 constexpr int TC_BN = 128;                     // granularity the host checks N against (BN = 256 when N % 256 == 0)
@@ -374,7 +374,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             uint32_t o[16];
             const size_t off = (size_t)row * (p.ldc ? p.ldc : p.N) + h * p.c_step + n0 + c0;  // TCE_PLAIN may write a column range of a wider buffer
             uint32_t rr[16];  // the residual row segment as four 16-byte loads (scalar 2-byte loads made this epilogue longer
-                              // than a K=4096 main loop: ncu r02, o_proj 68 % tensor-pipe active against 88-91 % elsewhere)
+                              // than a K=4096 main loop: ncu, o_proj 68 % tensor-pipe active against 88-91 % elsewhere)
             if (EPI == TCE_RESIDUAL) {
               const uint4 *r4 = reinterpret_cast<const uint4 *>(res + off);
 #pragma unroll

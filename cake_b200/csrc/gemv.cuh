@@ -1,6 +1,6 @@
 // gemv.cuh — the decode-time linear layer: out[N] = epilogue( W[N,K] · prologue(x[K]) ), batch 1.
 //
-// This kernel moves >97% of the bytes of a decoded token (SURVEY.md §8d), so it is built around
+// This kernel moves >97% of the bytes of a decoded token, so it is built around
 // HBM streaming, not math:
 //   * persistent grid, one CTA per SM (148); each CTA owns a contiguous row range [r0,r1) so the
 //     weight bytes of a CTA are ONE contiguous stream (row-major W) — perfectly sequential DRAM pages;
@@ -16,7 +16,7 @@
 //     bit-deterministic run to run;
 //   * epilogues fuse what the reference does as separate tensor ops: +bias, +residual (transformer.rs:123,131),
 //     silu(gate)*up on row-interleaved Wgu (mlp.rs:22-28), logits + greedy argmax (text_model.rs:348-352,104-105).
-// Rounding points follow SURVEY.md Appendix A: the matmul result is rounded to D before any epilogue op.
+// Rounding points: the matmul result is rounded to D before any epilogue op.
 #pragma once
 #include "common.cuh"
 
@@ -65,7 +65,7 @@ __host__ __device__ inline size_t gemv_smem_bytes(int K, int KC, int RS, int WPR
   return off + 128;                                      // alignment slack
 }
 
-// Geometry chosen from measurements (bench_tools/gemv_sweep.cu, profiles/gemv_sweep_r01.txt): TMA bulk
+// Geometry chosen from measurements (profiles/gemv_sweep_r01.txt): TMA bulk
 // copies must be large (>= 16 KB; 2 KB copies cap at 4.3 TB/s even with no math) and stages ~32 KB;
 // 2 row slots x 4 column slices keeps every lane busy with one shuffle tree per row per warp.
 template <typename T, int EPI, int RPW>

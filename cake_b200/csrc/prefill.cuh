@@ -1,5 +1,5 @@
 // prefill.cuh — the seq>1 / batch>1 side of the block forward (prompt ingestion), plus the small
-// bookkeeping kernels.  Same rounding points as the decode path.
+// bookkeeping kernels.  Same rounding points as the decode path (fp32 accumulate, round to D).
 //
 // The GEMM here is the generic CUDA-core tile kernel used for correctness bring-up of the prefill
 // path; the tcgen05 (UMMA + TMEM + TMA) GEMM replaces it for large M (see gemm_tc.cuh once present).
@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(256) rmsnorm_strided_kernel(T *__restrict__ x,
 // The same operator at HBM speed for the row lengths the served models have (n = 256 NV): one WARP per row, the row
 // read once with NV 16-byte loads per lane (all in flight together) and kept in registers between the sum of squares
 // and the scaling; 8 rows per CTA.  The one-CTA-per-row kernel above (2-byte accesses, row read twice) ran at 1.85 TB/s
-// on bs=32 x 4096 (ncu r02 launch list: 1.16 ms per call, 2.3 ms of a 51 ms layer).
+// on bs=32 x 4096 (ncu: 1.16 ms per call, 2.3 ms of a 51 ms layer).
 template <typename T, int NV>
 __global__ void __launch_bounds__(256) rmsnorm_rows_vec_kernel(const T *__restrict__ x, const T *__restrict__ w,
                                                                T *__restrict__ out, int rows, float eps) {
@@ -283,7 +283,7 @@ __global__ void __launch_bounds__(128) rope_append_kernel(T *__restrict__ qkv, T
 // both partners of its two rotation pairs, so nothing goes through shared memory; every access is a coalesced 128-byte
 // warp transaction and eight of them are in flight per lane; cos/sin are read once per token instead of once per head.
 // Identical arithmetic and rounding points (QK-norm -> D, products -> D, sum -> D).  The one-warp-per-head kernel above ran
-// at 1.4 TB/s on bs=32 x 4096 (ncu r02 launch list: 2.35 ms per layer).
+// at 1.4 TB/s on bs=32 x 4096 (ncu: 2.35 ms per layer).
 template <typename T>
 __global__ void __launch_bounds__(128) rope_append_vec_kernel(T *__restrict__ qkv, T *__restrict__ kcache, T *__restrict__ vcache,
                                                               const T *__restrict__ cos_t, const T *__restrict__ sin_t,

@@ -1,9 +1,9 @@
-// sample.cuh — device-side token samplers (SURVEY.md §8 f-1): the tail of TextModelBase::next_token
+// sample.cuh — device-side token samplers: the tail of TextModelBase::next_token
 // (text_model.rs:102-118 create_logits_processor, :429-460 the sampling step) without shipping the logits to the
 // host: one cluster of SAMPLE_CTAS CTAs reads the (vocab,) logits of the last position from L2/HBM and writes 4 bytes.
 //
 // The arithmetic behind `LogitsProcessor::sample` lives in candle-transformers 0.9.2 (generation/mod.rs) and
-// candle-nn 0.9.2 (sampling.rs), crates that are not vendored under /root/reference; restated from their published
+// candle-nn 0.9.2 (sampling.rs), crates that are not vendored with the reference; restated from their published
 // algorithm (oracle/sampling.py holds the CPU restatement the tests compare with):
 //   all kinds        logits -> f32
 //   GumbelSoftmax    argmax(logits + T * g),  g = -log(-log(u)),  u ~ U(1e-7, 0.999)      (candle_nn::sampling)

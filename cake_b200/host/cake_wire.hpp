@@ -1,5 +1,5 @@
 // cake_wire.hpp — cake's TCP wire protocol in C++ (header-only, no dependencies), so that a B200 box can be one worker
-// of an unmodified remote cake master (SURVEY.md §8f-3).  Same scope and reference anchors as cake_b200/wire.py:
+// of an unmodified remote cake master.  Same scope and reference anchors as cake_b200/wire.py:
 //
 //   proto/mod.rs:3-10          PROTO_MAGIC, MESSAGE_MAX_SIZE
 //   proto/message.rs:7-48      dtype tags, RawTensor { data, dtype, shape }

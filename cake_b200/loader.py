@@ -1,6 +1,6 @@
 """Weight loading: HF safetensors checkpoints -> host tensors that alias the mmapped shards.
 
-Mirrors the reference's loading path for the block-forward scope (SURVEY.md §8f-2):
+Mirrors the reference's loading path for the block-forward scope:
 
   utils/mod.rs:160-206     model.safetensors | model.safetensors.index.json -> shard list
   utils/mod.rs:250-267     load_var_builder_from_index            (every shard)
@@ -590,7 +590,7 @@ def open_model(path: str, topology: Optional[dict] = None, worker: Optional[str]
 def save_checkpoint(path: str, cfg: Config, tensors: Dict[str, torch.Tensor], arch: str = "LlamaForCausalLM",
                     shard_bytes: Optional[int] = None) -> List[str]:
     """Write an HF-layout checkpoint (config.json + model.safetensors, or shards + index when ``shard_bytes`` is
-    given).  Test / benchmark utility (the synthetic checkpoints of SURVEY.md §8d); tensors are written in name
+    given).  Test / benchmark utility (synthetic checkpoints); tensors are written in name
     order, a new shard starts when the current one would exceed ``shard_bytes``."""
     os.makedirs(path, exist_ok=True)
     with open(os.path.join(path, "config.json"), "w") as f:

@@ -1,4 +1,4 @@
-"""Synthetic HF-layout checkpoints (there are no real weights offline; SURVEY.md §8d).
+"""Synthetic HF-layout checkpoints (there are no real weights offline).
 
 Tensor names and shapes are the ones the reference loads:
   transformer.rs:89-90   {layer}.input_layernorm.weight / post_attention_layernorm.weight  (H)
@@ -79,7 +79,7 @@ def make_layer(cfg: Config, i: int, dtype: str = "bf16", seed: int = 1234, devic
 def make_head(cfg: Config, dtype: str = "bf16", seed: int = 1234, device="cpu", std: float = 0.02,
               peaked: bool = False) -> dict:
     """embed / final norm / lm_head.  ``peaked``: lm_head rows are scaled copies of the embedding rows,
-    which gives large top-1/top-2 logit margins (used for greedy token-id parity, SURVEY.md §8d)."""
+    which gives large top-1/top-2 logit margins (used for greedy token-id parity)."""
     gen = torch.Generator(device=device)
     gen.manual_seed(seed * 1000003 + 999983)
     td = TORCH_DTYPES[dtype]

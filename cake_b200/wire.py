@@ -1,4 +1,4 @@
-"""cake's TCP wire protocol, so that a B200 box can serve an unmodified remote cake master (SURVEY.md §8f-3).
+"""cake's TCP wire protocol, so that a B200 box can serve an unmodified remote cake master.
 
 What is mirrored (reference file:line):
 

@@ -18,7 +18,7 @@
  *   - "_dev" pointers are device memory on the ctx's GPU, everything is enqueued on the ctx's
  *     stream and is asynchronous unless the name ends in _host or the doc says it synchronises.
  *
- * Reference interface each entry replaces (paths relative to /root/reference/cake-core/src):
+ * Reference interface each entry replaces (paths relative to cake-core/src):
  *   cake_b200_ctx_create      Context::from_args device/dtype/config part        cake/mod.rs:114-392
  *   cake_b200_block_load      Forwarder::load -> Transformer::load               cake/mod.rs:513-515, models/common/transformer.rs:79-101,
  *                             (qkv / gate_up fusion done here)                   attention.rs:76-149, mlp.rs:34-59

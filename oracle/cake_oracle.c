@@ -5,7 +5,7 @@
  * import or execute this file.  Only tests/, __graft_entry__.smoke() and bench.py's
  * cpu_baseline / --impl reference legs use it, and there only as the checker / CPU arm.
  *
- * What it restates (all citations relative to /root/reference, commit be522af):
+ * What it restates (all citations relative to the reference, commit be522af):
  *   text_model.rs:266-368   TextModelBase::forward  (embed -> blocks -> ln_f -> last -> lm_head)
  *   transformer.rs:103-135  Transformer::forward    (pre-norm block, two residual adds)
  *   attention.rs:152-357    CausalSelfAttention::forward, generic f32 branch :300-346
@@ -17,7 +17,7 @@
  *   text_model.rs:60-99     apply_repeat_penalty_gpu ; :102-118 ArgMax when temperature<=0
  *
  * The arithmetic underneath those call sites lives in candle 0.9.2 (crates.io, Cargo.lock:817-933),
- * which is NOT vendored under /root/reference and cannot be built here (no Rust toolchain).
+ * which is NOT vendored with the reference and cannot be built here (no Rust toolchain).
  * PARITY PINNING: op level only.  The reference's own tests hold known answers for
  * rms_norm, causal mask, cos(pos 0), silu, cache growth (tests/unit_tests/test_backend_ops.rs:87-98,
  * :204-237; test_cache.rs:25-96; test_backends.rs:29-38) — tests/test_oracle_kat.py checks this file
@@ -28,7 +28,7 @@
  *
  * dtype boundaries mirrored (D = model dtype): every tensor the reference materialises in D is
  * rounded to D here (values are carried in float but are always D-representable):
- *   rms_norm: f32 sum of squares, x*rsqrt*w in f32, one rounding           
+ *   rms_norm: f32 sum of squares, x*rsqrt*w in f32, one rounding          
  *   linear:   D x D products (exact in f32), f32 accumulate, one rounding; bias add rounds again
  *   rope:     per-op rounding in D (half-crate / __nv_bfloat16 operator semantics)
  *   attention core: f32 throughout, one rounding of the result (attention.rs:301-346)

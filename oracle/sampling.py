@@ -3,7 +3,7 @@
 text_model.rs:102-118 maps (temperature, top_k, top_p) to a candle_transformers::generation::Sampling and
 text_model.rs:429-460 calls LogitsProcessor::sample on the (optionally repeat-penalised) logits.  The algorithms live
 in candle-transformers 0.9.2 (generation/mod.rs) and candle-nn 0.9.2 (sampling.rs) — crates.io dependencies that are
-not vendored under /root/reference (Cargo.lock:817-933); restated here from their published source, in float32 with the
+not vendored with the reference (Cargo.lock:817-933); restated here from their published source, in float32 with the
 same operation order:
   sample_argmax            first maximum
   sample_gumbel_softmax    u ~ U(1e-7, 0.999); minus_g = log(-log(u)); T == 1: argmax(l - minus_g) else argmax(l + minus_g * (-T))

@@ -25,7 +25,7 @@ CASES = {
     "llama3_rope_scaled": ("LlamaForCausalLM", dict(rope_theta=500000.0,
                            rope_scaling=RopeScaling(8.0, 1.0, 4.0, 16, "llama3"))),
     "qwen3_tiny": ("Qwen3ForCausalLM", dict(head_dim=32, use_qk_norm=True, tie_word_embeddings=True)),
-    # sibling dense architectures whose block is the same path (SURVEY.md §8f-4)
+    # sibling dense architectures whose block is the same path
     "qwen2_tiny": ("Qwen2ForCausalLM", dict(use_qkv_bias=True, rope_theta=1000000.0, tie_word_embeddings=True)),
     "mistral_tiny": ("MistralForCausalLM", dict(head_dim=32, rope_theta=1000000.0)),
     # Falcon3 checkpoints are Llama blocks with an explicit head_dim (falcon3/config.rs:53-90); HF runs them as Llama
@@ -37,7 +37,7 @@ CASES = {
     "mistral_window": ("MistralForCausalLM", dict(head_dim=32, rope_theta=1000000.0, sliding_window=4)),
     # use_gelu_mlp (mlp.rs:25-26; Gemma-style gelu_tanh gate) through HF's Llama with hidden_act=gelu_pytorch_tanh
     "llama_gelu_tiny": ("LlamaForCausalLM", dict(use_gelu_mlp=True)),
-    # the sibling block structures (SURVEY.md §8f-4, models/{olmo2,gemma3}/block.rs):
+    # the sibling block structures (models/{olmo2,gemma3}/block.rs):
     # OLMo2: no pre-norms, post-attention / post-feedforward norms, QK-norm over the whole projection before the reshape
     "olmo2_tiny": ("Olmo2ForCausalLM", dict(use_qk_norm=True, pre_reshape_qk_norm=True, block_kind="olmo2")),
     # Gemma3: sandwich norms with (1 + w) weights, gelu_tanh MLP, scaled embeddings, per-head QK-norm, tied head.  Every layer

@@ -1,5 +1,5 @@
-"""config.json -> block configuration for the dense architectures whose block is the path built here
-(SURVEY.md §8f-4): per-architecture serde defaults and hard-wired flags of the reference's into_config
+"""config.json -> block configuration for the dense architectures whose block is the path built here:
+per-architecture serde defaults and hard-wired flags of the reference's into_config
 (llama3/config.rs:62-98, qwen2/config.rs:69-105, qwen3/config.rs:55-93, mistral/config.rs:56-93,
 falcon3/config.rs:53-90), arch detection (common/config.rs:175-190, cake/mod.rs:81-109) — the Python mirror and
 the compiled C++ host must agree."""

@@ -1,4 +1,4 @@
-"""Parity at BASELINE.json's full layer dimensions (Llama-3-8B: H=4096, I=14336, 32/8 heads of 128), where every
+"""Parity at full layer dimensions (Llama-3-8B: H=4096, I=14336, 32/8 heads of 128), where every
 kernel runs with its production geometry (32 KB TMA stages, 16-warp megakernel slices, 128x128 UMMA tiles, 64x64
 flash tiles): one block against the oracle, plus size-independent properties at depth."""
 import numpy as np
@@ -83,7 +83,7 @@ def test_llama3_8b_decode_equals_prefill_at_depth():
 
 
 def test_qwen3_0_6b_config0_f16_greedy_against_oracle():
-    """BASELINE.json configs[0] — "Qwen3-0.6B ... greedy decode 32 tokens from one prompt (reference runs this
+    """The smallest workload — "Qwen3-0.6B ... greedy decode 32 tokens from one prompt (reference runs this
     today)" — at the real widths (H=1024, I=3072, 16/8 heads of 128, per-head QK-norm, tied 151 936-row head, the
     reference's default dtype f16, cake/mod.rs:75) with 4 of the 28 layers so the oracle stays fast.  Teacher-forced
     on the oracle's greedy sequence: per-step logits within tolerance; the greedy token must match wherever the
@@ -132,7 +132,7 @@ def _ctx_dtype(cfg, sd, dtype, max_seq):
 
 
 def test_llama3_70b_layer_geometry_matches_oracle():
-    """BASELINE.json configs[3] layer dimensions (H=8192, I=28672, 64/8 heads of 128 -> G=8): rows of 16 KB / 56 KB,
+    """Llama-3-70B layer dimensions (H=8192, I=28672, 64/8 heads of 128 -> G=8): rows of 16 KB / 56 KB,
     i.e. the 2-row and the split-row (2 x 28 KB) stage geometries of the megakernel, and 8 query heads per kv head."""
     from cake_b200.config import llama3_70b
     from cake_b200.model import B200Transformer
@@ -189,7 +189,7 @@ def test_llama3_8b_decode_at_2500_context_multi_tile_attention():
 
 
 def test_llama3_8b_block_batch_gt_1_matches_oracle_per_sequence():
-    """BASELINE configs[4] is bs=32: the Forwarder's (b, s, H) contract with b > 1 at the Llama-3-8B layer widths — a
+    """The Forwarder's (b, s, H) contract with b > 1 at the Llama-3-8B layer widths — a
     (2, 144, H) prefill (tcgen05 GEMMs over 288 rows, flash attention per sequence) and two (2, 1, H) steps — every
     sequence against its own oracle run."""
     from cake_b200.model import B200Transformer, Cache

@@ -1,4 +1,4 @@
-"""Parity AT the benchmarked configuration (BASELINE.json configs[1]): the whole 32-layer Llama-3-8B in bf16 at 2k
+"""Parity AT the benchmarked configuration: the whole 32-layer Llama-3-8B in bf16 at 2k
 context — the exact model `bench.py` times — against the oracle, token by token (text_model.rs:266-368 via the decode
 graph: embed -> 32 blocks -> ln_f -> lm_head -> argmax in one persistent kernel launch per token).
 

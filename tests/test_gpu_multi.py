@@ -79,7 +79,7 @@ def test_two_gpu_ring_equals_single_gpu():
 
 
 def _rank_70b(rank, world, port, q):
-    """BASELINE configs[3] widths (Llama-3-70B: H=8192, I=28672, 64/8 heads of 128 -> 8 query heads per kv head, 16 KB and
+    """Widths of the largest workload (Llama-3-70B: H=8192, I=28672, 64/8 heads of 128 -> 8 query heads per kv head, 16 KB and
     split 56 KB weight rows), 2 layers = one per rank, vocabulary cut to 4096 rows to keep the test small."""
     import torch.distributed as dist
     from cake_b200.config import llama3_70b

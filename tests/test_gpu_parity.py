@@ -3,7 +3,7 @@ same seeded inputs.  Scenarios follow the reference's own block/attention/cache 
 (tests/unit_tests/test_blocks.rs:877-933, test_attention.rs:12-143, test_cache.rs:77-96) — which assert
 shapes/determinism only — plus the numeric comparison the reference never had.
 
-Tolerance (written here, stated in DESIGN.md): floating point, dtype D in {bf16, f16}.  GPU and oracle
+Tolerance: floating point, dtype D in {bf16, f16}.  GPU and oracle
 round at the same points but accumulate fp32 sums in different orders, so a value that lands near a
 rounding boundary can differ by 1 ulp of D and the flip propagates.  Bars:
   one block:            max |err| <= 3 ulp of D at the tensor's scale (tests/util.py ulp_at_scale), i.e.
@@ -38,7 +38,7 @@ def _llama31_scaling():
 
 
 CONFIGS = {
-    # SURVEY.md §8 f-4: an active sliding window (cache.rs:173-205; bites from the second decode step on), the GELU MLP
+    # an active sliding window (cache.rs:173-205; bites from the second decode step on), the GELU MLP
     "medium_window": lambda: medium_config(sliding_window=5),
     "medium_gelu": lambda: medium_config(use_gelu_mlp=True),
     "medium_rope_llama3": lambda: medium_config(rope_scaling=_llama31_scaling(), rope_theta=10000.0),

@@ -1,4 +1,4 @@
-"""The GPU cases that were written after round 1's GPU budget was spent, executed here on the CPU: the very same test
+"""GPU cases executed here on the CPU: the very same test
 functions, with `cake_b200.model.Context` replaced by the CPU stand-in and the library by the oracle-backed emulation
 (tests/fake_b200).  Numerics are trivially exact this way; the point is that the tests' own code — shapes, call
 sequences, expectations on errors, process handling — is known to be right before it meets hardware."""
@@ -64,7 +64,7 @@ def _expand(fn):
 
 
 def test_the_hardware_validated_parity_suite_still_runs(emulated):
-    """tests/test_gpu_parity.py (run on a B200 in round 1) executed over the emulation: a regression net for the host
+    """tests/test_gpu_parity.py executed over the emulation: a regression net for the host
     code those tests go through (loading, forward_batch plumbing, caches, the decode loop API, repeat penalty, error
     paths) whenever it is refactored without a GPU at hand.  Numerics are exact here by construction."""
     import inspect

@@ -1,4 +1,4 @@
-"""Weight loading (SURVEY.md §8f-2): cake_b200/loader.py against the reference's loading rules
+"""Weight loading: cake_b200/loader.py against the reference's loading rules
 (utils/mod.rs:160-384, cake/mod.rs:335-357) — checked with the `safetensors` library as an independent
 writer/reader, with the oracle (tokens from a checkpoint on disk == tokens from the in-memory state dict),
 and on the GPU through Context/TextModelBase."""

@@ -31,7 +31,7 @@ def test_oracle_matches_hf_fixture(name):
 
 @pytest.mark.parametrize("dtype,tol", [("bf16", 0.08), ("f16", 0.01)])
 def test_low_precision_oracle_stays_near_fp32(dtype, tol):
-    # bounds how much of any GPU-vs-oracle gap can be rounding order rather than a bug (SURVEY §8c)
+    # bounds how much of any GPU-vs-oracle gap can be rounding order rather than a bug
     z = np.load(os.path.join(GOLD, "hf_llama_tiny.npz"))
     _, cfg = case_config("llama_tiny")
     sd32 = make_checkpoint(cfg, "f32", seed=int(z["seed"]), std=float(z["std"]))

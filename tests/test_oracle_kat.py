@@ -1,5 +1,5 @@
-"""Pins the CPU oracle against every known-answer test the reference holds for this path
-(SURVEY.md §8c).  Citations are to /root/reference/cake-core/tests/unit_tests/."""
+"""Pins the CPU oracle against every known-answer test the reference holds for this path.
+Citations are to cake-core/tests/unit_tests/."""
 import math
 
 import numpy as np
@@ -30,7 +30,7 @@ def test_silu_known_values():
     # test_backends.rs:29-38 silu(1)*1 ~= 0.731 (+-0.01); test_backend_ops: silu(0)=0
     assert abs(O.silu_mul(1.0, 1.0, "f32") - 0.731) < 0.01
     assert O.silu_mul(0.0, 5.0, "f32") == 0.0
-    # both rounding conventions agree to 2 bf16 ulp on a sweep (tolerance probe, DESIGN.md)
+    # both rounding conventions agree to 2 bf16 ulp on a sweep (tolerance probe)
     for g in np.linspace(-6, 6, 97):
         a, b = O.silu_mul(float(g), 1.5, "bf16", 0), O.silu_mul(float(g), 1.5, "bf16", 1)
         assert abs(a - b) <= 2 ** -6 * max(1.0, abs(a))

@@ -1,4 +1,4 @@
-"""Device-side samplers (SURVEY.md §8 f-1): text_model.rs:102-118 picks a Sampling from (temperature, top_k, top_p) and
+"""Device-side samplers: text_model.rs:102-118 picks a Sampling from (temperature, top_k, top_p) and
 :429-460 draws from the (optionally repeat-penalised) logits.  The CUDA samplers (csrc/sample.cuh, through
 cake_b200_sample / the decode graph) are compared with the CPU restatement oracle/sampling.py with the SAME uniforms
 supplied to both sides — candle's own random stream cannot be reproduced (see the module headers)."""

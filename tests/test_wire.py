@@ -1,4 +1,4 @@
-"""cake's TCP wire protocol (cake_b200/wire.py, SURVEY.md §8f-3).
+"""cake's TCP wire protocol (cake_b200/wire.py).
 
 Scenarios follow the reference's own tests: proto/message.rs:415-1026 (round trips of every message, wire framing,
 invalid magic, oversized message, dtype tags) and tests/protocol.rs (mock echo worker over loopback: handshake,

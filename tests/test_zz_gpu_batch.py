@@ -1,6 +1,6 @@
-"""Two cases written after round 1's GPU budget was spent, hence kept in their own file, last in collection order:
+"""Two cases in their own file, last in collection order:
 
-* batch > 1 through the Forwarder (BASELINE.json configs[4] is a bs=32 prefill; `cake run` itself never builds b > 1,
+* batch > 1 through the Forwarder (a bs=32 prefill is a workload of the benchmark; `cake run` itself never builds b > 1,
   text_model.rs:418-420, so the reference's contract here is the Forwarder's `x: (b, s, H)`): every sequence of the
   batch must equal the oracle run on that sequence alone with its own cache;
 * the Phi-3/4 shape of the block: rotary on the first 3/4 of every head only (`rot < head_dim`), qkv_proj / gate_up_proj
