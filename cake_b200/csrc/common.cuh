@@ -120,9 +120,9 @@ __device__ __forceinline__ void mbar_wait(uint64_t *bar, uint32_t parity) {
       "r"(parity)
       : "memory");
 }
-// mbarrier wait with a bound.  `left` is what the waits of a thread may still spend together in this kernel, MBAR_TRIES at first (1.3 s; a
+// mbarrier wait with a bound.  `left` is what the waits of a thread may still spend together in this kernel, MBAR_TRIES at first (1 s; a
 // kernel of a million rows takes 0.2); at 0 one has been given up, *err is set, and each later one returns after two tries.  One plain
-// try first; past it a try may suspend the thread for longer (MBAR_TRY_NS asked for, about 5 us seen), so that a wait that succeeds takes
+// try first; past it a try may suspend the thread for longer (MBAR_TRY_NS asked for, about 4 us seen), so that a wait that succeeds takes
 // few of them.  A ring's round trip bounds many products and a branch that depends on a wait keeps their loops from being unrolled, so there
 // is none: copies, the barriers they count on and commits carry left != 0 as a predicate, and a thread that has given up runs its loop
 // to the end, requests no copy and commits no product.  2000 tokens through four 0.6B layers: 673 us; without the predicates 670, with a branch behind
