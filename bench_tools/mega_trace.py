@@ -20,18 +20,18 @@ ctx.cache.fill_synthetic(list(range(nl)), 2048, 7); ctx.sync(); m.index_pos = 20
 m.decode_build()
 m.decode_greedy(5, 8)
 L = lib(); L.cake_b200_debug_trace.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int]
-n = 1 + nl * 9 + 4
+n = 1 + nl * 10 + 2
 buf = (ctypes.c_ulonglong * n)()
 check(L.cake_b200_debug_trace(ctx.h, buf, n))
 t = np.array(buf[:], dtype=np.int64); t = (t - t[0]) / 1e3
-# stamps: start, then per layer: [qkv done, barrier done, attn done, barrier done, o done, b, gu done, b, down done, b]
-names = ["qkv", "bar", "attn", "bar", "o", "bar", "gate_up", "bar", "down", "bar"]
+# stamps: start, then per layer: input of qkv gathered, qkv published, attention begins, attention done, o gathered, o published, gate_up .., down ..
+names = ["gather qkv", "qkv", "-", "attn", "gather o", "o", "gather gate_up", "gate_up", "gather down", "down"]
 d = np.diff(t)
 per = {}
 for l in range(nl):
     seg = d[l * 10:(l + 1) * 10]
     for k, v in zip(names, seg):
-        per.setdefault(k if k != "bar" else "bar", []).append(v)
+        per.setdefault(k, []).append(v)
     if l < 3 or l == nl - 1:
         print(f"layer {l}: " + " ".join(f"{k}={v:.1f}" for k, v in zip(names, seg)))
 for k, v in per.items():
@@ -42,14 +42,4 @@ n2 = 2048 + 8
 buf2 = (ctypes.c_ulonglong * n2)()
 check(L.cake_b200_debug_trace(ctx.h, buf2, n2))
 a = np.array(buf2[2048:2056], dtype=np.int64)
-print("attention sub-phases (layer 1, CTA 0) us:", dict(zip(["qprep", "tile_wait", "scores", "softmax", "pv", "partial_wr", "fence+ticket"], np.round(np.diff(a) / 1e3, 2))))
-
-n3 = 2560 + 148
-buf3 = (ctypes.c_ulonglong * n3)()
-check(L.cake_b200_debug_trace(ctx.h, buf3, n3))
-fin = np.array(buf3[2304:2304 + 148], dtype=np.int64) / 1e3
-rel = np.array(buf3[2560:2560 + 148], dtype=np.int64) / 1e3
-fin -= fin.min(); 
-print("gate_up(l=1) finish spread over CTAs us: p50 %.2f p90 %.2f max %.2f ; sorted tail:" % (np.percentile(fin, 50), np.percentile(fin, 90), fin.max()), np.round(np.sort(fin)[-6:], 2))
-print("barrier release after last finisher us: min %.2f max %.2f" % ((rel - rel.min()).min() , (rel.max() - (np.array(buf3[2304:2304+148],dtype=np.int64)/1e3).max())))
-print("slowest CTAs:", np.argsort(fin)[-8:])
+print("attention sub-phases (layer 1, CTA 0) us:", dict(zip(["qprep", "tile_wait", "scores", "softmax", "pv", "published", "merged"], np.round(np.diff(a) / 1e3, 2))))

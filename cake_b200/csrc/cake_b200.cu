@@ -194,7 +194,9 @@ struct cake_b200_ctx {
   bool capturing = false;
   // persistent decode megakernel (decode_mega.cuh); CAKE_B200_PER_OP=1 selects the per-op kernels instead
   bool use_mega = true;
-  unsigned long long *gbar = nullptr;   // [0] grid-barrier counter, [1] launch epoch
+  unsigned long long *gbar = nullptr;   // [0] grid-barrier counter, [1] its value at launch start, [2] layers run (the packets' tags)
+  uint32_t *mk_pk = nullptr;            // the megakernel's packets: xa, qkv, y, xb, mm
+  uint64_t *mk_part = nullptr;          // and those of attention cut over several CTAs
   MkLayer *mk_tab_dev = nullptr, *mk_tab_host = nullptr, *g_tab_dev = nullptr;
   std::vector<const void *> mk_sig;
   unsigned long long *trace = nullptr;  // CAKE_B200_MEGA_TRACE=1
@@ -491,6 +493,22 @@ static void f32_to_D(const std::vector<float> &src, std::vector<uint16_t> &dst, 
   }
 }
 
+// the megakernel's packet vectors in mk_pk, 256 bytes apart; returns the packets in all
+static size_t mk_packet_offsets(const cake_b200_ctx *c, MkPackets *pk) {
+  const cake_b200_config &f = c->cfg;
+  const size_t len[5] = {(size_t)f.hidden, (size_t)c->nqkv, (size_t)f.n_heads * f.head_dim, (size_t)f.hidden, (size_t)f.inter};
+  size_t off[5], n = 0;
+  for (int i = 0; i < 5; i++) {
+    off[i] = n;
+    n += (len[i] + 63) & ~(size_t)63;
+  }
+  if (pk) {
+    uint32_t *b = c->mk_pk;
+    *pk = MkPackets{b + off[0], b + off[1], b + off[2], b + off[3], b + off[4], c->mk_part, c->mk_part + (size_t)f.n_heads * f.head_dim * c->nsplit};
+  }
+  return n;
+}
+
 extern "C" int cake_b200_ctx_create(int device, const cake_b200_config *cfg, cake_b200_ctx **out) {
   if (!cfg || !out) return fail(CAKE_B200_EINVAL, "null argument");
   cake_b200_config listed_cfg;
@@ -576,8 +594,15 @@ extern "C" int cake_b200_ctx_create(int device, const cake_b200_config *cfg, cak
   CU(cudaMallocHost(&c->h_pin, 64 * 4));
   CU(cudaMallocHost(&c->wait_err, 4));
   *c->wait_err = 0;
-  CU(cudaMalloc(&c->gbar, 16));
-  CU(cudaMemset(c->gbar, 0, 16));
+  CU(cudaMalloc(&c->gbar, 24));
+  CU(cudaMemset(c->gbar, 0, 24));
+  {  // tags begin at 1
+    const size_t n = mk_packet_offsets(c, nullptr), parts = (size_t)nh * c->nsplit * (hd + 2);
+    CU(cudaMalloc(&c->mk_pk, n * 4));
+    CU(cudaMemset(c->mk_pk, 0, n * 4));
+    CU(cudaMalloc(&c->mk_part, parts * 8));
+    CU(cudaMemset(c->mk_part, 0, parts * 8));
+  }
   CU(cudaMalloc(&c->tickets, sizeof(unsigned) * (4 * MK_MAX_LAYERS + 4)));
   CU(cudaMalloc(&c->ring_seq, 8));
   CU(cudaMemset(c->ring_seq, 0, 8));
@@ -619,7 +644,7 @@ extern "C" void cake_b200_ctx_destroy(cake_b200_ctx *c) {
   void *bufs[] = {c->cos_t, c->sin_t, c->embed, c->ln_f, c->xa, c->xb, c->qkv, c->y, c->mm, c->logits, c->ws_ml,
                   c->ws_acc, c->part_val, c->part_idx, c->d_step, c->attn_counters, c->argmax_counter, c->d_token,
                   c->token_ring, c->d_ids, c->d_pen, c->pf_h, c->pf_qkv, c->pf_y, c->pf_x1, c->pf_gu, c->pf_mm, c->io_x,
-                  c->gbar, c->mk_tab_dev, c->g_tab_dev, c->tickets, c->ring_seq, c->inbox, c->step_trace, c->trace,
+                  c->gbar, c->mk_pk, c->mk_part, c->mk_tab_dev, c->g_tab_dev, c->tickets, c->ring_seq, c->inbox, c->step_trace, c->trace,
                   c->samp_p, c->samp_noise, c->hd_logits, c->hd_tokens, c->x0, c->sp_h, c->sp_hs, c->sp_in, c->sp_a, c->sp_hn, c->sp_logits, c->sp_rows_idx, c->mx_ws};
   for (void *b : bufs)
     if (b) cudaFree(b);
@@ -1069,30 +1094,18 @@ static int enqueue_decode_layers(cake_b200_ctx *c, cake_b200_block *const *block
 }
 
 // ------------------------------------------------------------------------------------------ megakernel plan + launch
-static int plan_mk_geom(const cake_b200_ctx *c, int N, int K, int G, MkGeom *g, int *partial_floats, int *max_groups) {
+static int plan_mk_geom(const cake_b200_ctx *c, int N, int K, int G, MkGeom *g) {
   const int es = c->es;
   if (K % 64 != 0 || N % G != 0) return fail(CAKE_B200_EINVAL, "mega: K=%d must be a multiple of 64, N=%d of %d", K, N, G);
   int KC = K;
   while ((size_t)KC * es > MK_STAGE_BYTES && (KC / 2) % 64 == 0) KC /= 2;
   const size_t seg = (size_t)KC * es;
   if (seg > MK_STAGE_BYTES) return fail(CAKE_B200_EINVAL, "mega: K=%d cannot be staged", K);
-  int RS = 1;
-  while (RS < 64 && (size_t)(RS * 2) * seg <= MK_STAGE_BYTES) RS *= 2;
-  int WPR, RPW;
-  if (RS >= MK_CW) { WPR = 1; RPW = RS / MK_CW; }
-  else { WPR = MK_CW / RS; RPW = 1; }
-  while (WPR > 1 && ((KC / 8) % WPR != 0)) { WPR /= 2; }  // slices must divide the segment's 16-byte vectors
-  if (RS * RPW < (MK_CW / WPR) * RPW || RS != (MK_CW / WPR) * RPW)  // every row slot must map to a staged row
-    return fail(CAKE_B200_EINVAL, "mega: unsupported geometry N=%d K=%d (KC=%d RS=%d WPR=%d)", N, K, KC, RS, WPR);
-  *g = MkGeom{N, K, KC, RS, WPR, RPW};
-  // per-CTA cap of row groups in one phase: twice the even share (dynamic claiming, decode_mega.cuh mk_split)
-  const int n_groups = (N + RS - 1) / RS;
-  const int cap = 2 * ((n_groups + c->sm_count - 1) / c->sm_count) + 4;
-  if (cap > *max_groups) *max_groups = cap;
-  // *partial_floats collects max(RS*WPR) here and the static-path need; plan_mega multiplies by the global cap
-  if (RS * WPR > *partial_floats % 65536) *partial_floats = (*partial_floats / 65536) * 65536 + RS * WPR;
-  const int pf_static = (((N / G) / c->sm_count) + 1) * G * WPR;
-  if (pf_static > *partial_floats / 65536) *partial_floats = pf_static * 65536 + *partial_floats % 65536;
+  int RSL = 0;
+  while (KC == K && RSL < 4 && ((size_t)2 << RSL) * seg <= MK_STAGE_BYTES) RSL++;
+  if (KC == K && (1 << RSL) < G) return fail(CAKE_B200_EINVAL, "mega: K=%d: a stage does not hold a gate and an up row", K);
+  *g = MkGeom{N, K, KC, RSL, K / KC};
+  mk_plan_split(*g, G, c->sm_count);
   return CAKE_B200_OK;
 }
 
@@ -1107,34 +1120,26 @@ static bool mega_supported(const cake_b200_ctx *c) {
 #undef MK_CASE
   return false;
 }
-static int plan_mega(cake_b200_ctx *c, cake_b200_cache *kc, bool with_head, MkPlan *p) {
+static int plan_mega(cake_b200_ctx *c, cake_b200_cache *kc, int n_layers, bool with_head, MkPlan *p) {
   const cake_b200_config &f = c->cfg;
   MkArgs &a = p->a;
   memset(&a, 0, sizeof(a));
-  int pf = 0, mg = 0;
-  RC(plan_mk_geom(c, c->nqkv, f.hidden, 1, &a.g_qkv, &pf, &mg));
-  RC(plan_mk_geom(c, f.hidden, f.n_heads * f.head_dim, 1, &a.g_o, &pf, &mg));
-  RC(plan_mk_geom(c, 2 * f.inter, f.hidden, 2, &a.g_gu, &pf, &mg));
-  RC(plan_mk_geom(c, f.hidden, f.inter, 1, &a.g_down, &pf, &mg));
-  if (with_head) RC(plan_mk_geom(c, f.vocab, f.hidden, 1, &a.g_head, &pf, &mg));
-  {  // partial-sum scratch: every phase may use up to `mg` groups of its own RS*WPR floats (dynamic), or its static rows
-    const int dyn_need = mg * (pf % 65536), static_need = pf / 65536;
-    pf = dyn_need > static_need ? dyn_need : static_need;
-  }
-  a.partial_floats = pf;
-  a.max_groups = mg;
+  RC(plan_mk_geom(c, c->nqkv, f.hidden, 1, &a.g[0]));
+  RC(plan_mk_geom(c, f.hidden, f.n_heads * f.head_dim, 1, &a.g[1]));
+  RC(plan_mk_geom(c, 2 * f.inter, f.hidden, 2, &a.g[2]));
+  RC(plan_mk_geom(c, f.hidden, f.inter, 1, &a.g[3]));
+  if (with_head) RC(plan_mk_geom(c, f.vocab, f.hidden, 1, &a.g[4]));
+  int whole = 0;  // phases in which every CTA has rows
+  for (int i = 0; i < 4; i++) whole += mk_every_cta(a.g[i]) ? 1 : 0;
+  a.meet = whole < 2;
   a.tickets = c->tickets;
-  {
-    const char *e = getenv("CAKE_B200_L2_PREFETCH");
-    a.l2_prefetch = (e && e[0] >= '1' && e[0] <= '2') ? e[0] - '0' : 0;
-  }
   a.hidden = f.hidden; a.inter = f.inter; a.n_heads = f.n_heads; a.n_kv = f.n_kv_heads; a.hd = f.head_dim;
   a.rot = c->rot; a.cap = kc ? kc->cap : 0; a.nsplit = c->nsplit; a.eps = f.rms_eps;
   a.scale = (float)(1.0 / sqrt((double)f.head_dim));
   a.max_k = f.inter > f.hidden ? f.inter : f.hidden;
   if (f.n_heads * f.head_dim > a.max_k) a.max_k = f.n_heads * f.head_dim;
-  a.xa = c->xa; a.xb = c->xb; a.qkv = c->qkv; a.y = c->y; a.mm = c->mm;
-  a.ws_ml = c->ws_ml; a.ws_acc = c->ws_acc; a.attn_counters = c->attn_counters;
+  mk_packet_offsets(c, &a.pk);
+  a.err = c->wait_err;
   a.cos_t = c->cos_t; a.sin_t = c->sin_t; a.d_pos = kc ? kc->d_pos : nullptr; a.d_step = c->d_step; a.gbar = c->gbar;
   a.vocab = f.vocab; a.embed = c->embed; a.d_token = c->d_token;
   a.ln_f = c->ln_f; a.lm_head = c->lm_head; a.logits = c->logits; a.part_val = c->part_val; a.part_idx = c->part_idx;
@@ -1144,11 +1149,16 @@ static int plan_mega(cake_b200_ctx *c, cake_b200_cache *kc, bool with_head, MkPl
   a.trace_tag = 0;
   a.act = f.use_gelu_mlp ? 1 : 0;
   a.window = f.sliding_window;
-  int ns = MK_MAX_STAGES;
   const size_t limit = 227 * 1024 - 4096;  // the kernel also has ~2.2 KB of static shared memory
-  while (ns > 2 && mk_smem_bytes(a.max_k, pf, mg, ns, c->es) > limit) ns--;
-  a.n_stages = ns;
-  p->smem = mk_smem_bytes(a.max_k, pf, mg, ns, c->es);
+  a.n_layers = n_layers;
+  auto stages = [&](int keep) {
+    a.keep_x = keep;
+    for (a.n_stages = MK_MAX_STAGES; a.n_stages > 2 && mk_layout(a, c->es) > limit;) a.n_stages--;
+    return a.n_stages;
+  };
+  const int without = stages(0);
+  if (stages(1) < without || mk_layout(a, c->es) > limit) stages(0);  // the copy of the residual stream is not worth a stage
+  p->smem = mk_layout(a, c->es);
   if (p->smem > limit) return fail(CAKE_B200_EINVAL, "mega: needs %zu B of shared memory", p->smem);
   return CAKE_B200_OK;
 }
@@ -1177,7 +1187,9 @@ static int launch_mega(cake_b200_ctx *c, const MkPlan &p) {
   cfg.attrs = at;
   cfg.numAttrs = 1;
   const MkArgs &a = p.a;
-  CU(cudaMemsetAsync(c->tickets, 0, sizeof(unsigned) * (4 * (size_t)a.n_layers + 4), c->stream));  // a memset node in the graph
+  bool pool = false;
+  for (int i = a.n_layers ? 0 : 4; i < (a.has_head ? 5 : 4); i++) pool = pool || a.g[i].pool < a.g[i].n_groups;
+  if (pool) CU(cudaMemsetAsync(c->tickets, 0, sizeof(unsigned) * (4 * (size_t)a.n_layers + 4), c->stream));  // a memset node in the graph
   int rc = DISPATCH_T(c->cfg.dtype, T_LAMBDA {
     typedef typename decltype(tag_)::type T;
     return launch_mega_T<T>(c, &cfg, a);
@@ -1210,9 +1222,8 @@ static int enqueue_mega_layers(cake_b200_ctx *c, cake_b200_block *const *blocks,
     c->mk_sig = sig;
   }
   MkPlan p;
-  RC(plan_mega(c, kc, false, &p));
+  RC(plan_mega(c, kc, n, false, &p));
   p.a.layers = c->mk_tab_dev;
-  p.a.n_layers = n;
   p.a.x_in = x_in;
   p.a.x_out = x_out;
   p.a.has_head = 0;
@@ -1222,6 +1233,16 @@ static int enqueue_mega_layers(cake_b200_ctx *c, cake_b200_block *const *blocks,
 
 // ln_f + lm_head + greedy argmax on one hidden row -> logits_out (nullable), token -> c->d_token
 static int enqueue_head(cake_b200_ctx *c, const void *x_row, void *logits_out, bool ring) {
+  if (c->use_mega && mega_supported(c)) {  // the decode kernel without layers: the same logits as a replayed step's, bit for bit
+    MkPlan p;
+    RC(plan_mega(c, nullptr, 0, true, &p));
+    p.a.x_in = x_row;
+    p.a.has_head = 1;
+    p.a.logits = logits_out;
+    p.a.step_trace = nullptr;
+    if (ring) p.a.token_ring = c->token_ring;
+    return launch_mega(c, p);
+  }
   GemvArgs a{};
   a.W = c->lm_head; a.x = x_row; a.norm_w = c->ln_f; a.out = logits_out; a.eps = c->cfg.rms_eps;
   a.N = c->cfg.vocab; a.K = c->cfg.hidden;
@@ -3858,8 +3879,8 @@ extern "C" int cake_b200_decode_build(cake_b200_ctx *c, cake_b200_block *const *
       unsigned long long *inbox_ctr = (unsigned long long *)c->inbox, *peer_ctr = (unsigned long long *)c->peer_inbox;
       void *inbox_x = c->inbox ? c->inbox + INBOX_X_OFF : nullptr, *peer_x = c->peer_inbox ? c->peer_inbox + INBOX_X_OFF : nullptr;
       if (rank == 0) {
-        RC(plan_mega(c, kc, world == 1, &p));
-        p.a.layers = c->g_tab_dev; p.a.n_layers = n_blocks; p.a.x_in = nullptr; p.a.x_out = c->xa;
+        RC(plan_mega(c, kc, n_blocks, world == 1, &p));
+        p.a.layers = c->g_tab_dev; p.a.x_in = nullptr; p.a.x_out = c->xa;
         if (c->cfg.embed_scale != 0.f) {  // text_model.rs:274-276: the scaled embedding row is materialised first
           RC(DISPATCH_T(c->cfg.dtype, T_LAMBDA {
             typedef typename decltype(tag_)::type T;
@@ -3878,8 +3899,8 @@ extern "C" int cake_b200_decode_build(cake_b200_ctx *c, cake_b200_block *const *
             RC(cake_b200_recv(c, c->xa, xbytes, world - 1));
           }
           MkPlan h;
-          RC(plan_mega(c, kc, true, &h));
-          h.a.layers = c->g_tab_dev; h.a.n_layers = 0; h.a.x_in = p2p ? inbox_x : c->xa; h.a.x_out = c->xa;
+          RC(plan_mega(c, kc, 0, true, &h));
+          h.a.layers = c->g_tab_dev; h.a.x_in = p2p ? inbox_x : c->xa; h.a.x_out = c->xa;
           h.a.has_head = 1; h.a.advance = 1; h.a.token_ring = c->token_ring; h.a.trace_tag = 1;
           if (p2p) { h.a.inbox_ctr = inbox_ctr; h.a.ring_seq = c->ring_seq; }
           RC(launch_mega(c, h));
@@ -3894,8 +3915,8 @@ extern "C" int cake_b200_decode_build(cake_b200_ctx *c, cake_b200_block *const *
         }
       } else {
         if (!p2p) RC(cake_b200_recv(c, c->xa, xbytes, rank - 1));
-        RC(plan_mega(c, kc, false, &p));
-        p.a.layers = c->g_tab_dev; p.a.n_layers = n_blocks; p.a.x_in = p2p ? inbox_x : c->xa; p.a.x_out = p2p ? peer_x : c->xa;
+        RC(plan_mega(c, kc, n_blocks, false, &p));
+        p.a.layers = c->g_tab_dev; p.a.x_in = p2p ? inbox_x : c->xa; p.a.x_out = p2p ? peer_x : c->xa;
         p.a.has_head = 0; p.a.advance = 1;
         if (p2p) { p.a.inbox_ctr = inbox_ctr; p.a.peer_ctr = peer_ctr; p.a.ring_seq = c->ring_seq; }
         if (n_blocks > 0) RC(launch_mega(c, p));

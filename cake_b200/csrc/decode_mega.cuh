@@ -5,17 +5,27 @@
 // o_proj 7.2 us streamed vs 5.1 us ideal) — 130 boundaries per token = ~0.4 ms of a 2.3 ms budget.
 // Here the whole walk  [rms_1+qkv -> rope/append/attention -> o_proj+res -> rms_2+gate_up+silu*mul ->
 // down+res] x layers (+ ln_f/lm_head/argmax on the master)  runs inside one grid of one CTA per SM:
-//   * warp 16 is the PRODUCER: it walks the same static phase list and issues TMA bulk copies of the
+//   * one warp is the PRODUCER: it walks the same static phase list and issues TMA bulk copies of the
 //     next weight rows (32 KB stages, evict_first) and of this CTA's K/V cache tile into a 5-6 stage
-//     shared-memory ring.  It never takes part in a grid barrier, so HBM keeps streaming while the
-//     consumers synchronise — the ring (~160 KB/SM, ~24 MB chip-wide) absorbs the bubbles;
-//   * warps 0-15 are CONSUMERS: per phase they wait for the grid barrier that publishes the previous
-//     phase's output vector, stage x (RMS-normalised in-kernel), multiply-accumulate the staged rows in
-//     fp32 and run the fused epilogue;
-//   * grid barriers are a 64-bit monotonic counter in global memory (release: bar.sync + threadfence +
-//     atomicAdd; acquire: ld.acquire poll + threadfence); activations are read with ld.global.cg.
+//     shared-memory ring.  It waits for no other CTA, so HBM keeps streaming while the
+//     consumers exchange a vector — the ring (~160 KB/SM, ~24 MB chip-wide) absorbs the bubbles;
+//   * the other warps are CONSUMERS: per phase they gather the previous phase's output vector (RMS-normalised
+//     in-kernel), multiply-accumulate the staged rows in fp32 and run the fused epilogue;
+//   * a vector travels from phase to phase as PACKETS of 32 bits in global memory (L2): the 16-bit value and a 16-bit tag
+//     that changes with every layer.  A CTA stores the packets of its rows and goes on; whoever needs the vector reads the packets
+//     themselves until their tags are right.  One store and one load lie between two phases where a grid barrier
+//     has the release of the CTA's stores, its arrival, the poll and only then the load of the vector.
+// Bound by HBM where a layer's weights are large (8B: 436 MB a layer) and by the chain of five exchanges per layer where they are not
+// (0.6B: 31 MB, 5 us of stream).  With grid barriers and fp32 conversions in 16 warps: 32 us a layer at 0.6B, 24 tokens 25.1 ms, 8B two layers 187 us; now
+// 15 us, 14.1 ms and 182 us.  An exchange is 1.0 to 1.5 us (a barrier with the staging behind it 3 to 4.5), a product of 12 MB 2.1 us behind it.
 // Arithmetic and rounding points are identical to the per-op kernels (gemv.cuh / attn_decode.cuh); only the
 // fp32 summation order within a dot product differs (tests/test_gpu_parity.py::test_megakernel_equals_per_op_kernels).
+//
+// A packet buffer is written again one layer later; no reader may still be in front of it.  A CTA that has not gathered the input of
+// phase p has published nothing from phase p on, and whoever writes that input again (phase p - 1 of the next layer) has gathered, directly or
+// through others, ALL outputs of phases p .. p - 2 (four of the five phases; a vector is complete only when every owner of a row has published).  So
+// it is enough that every CTA owns rows of at least two phases whatever the tickets say (mk_every_cta); where a model is too small for that,
+// all CTAs meet at one grid barrier per layer, between the gathering of the last phase's input and its output (`meet`).
 #pragma once
 #include "common.cuh"
 #include "gemv.cuh"
@@ -23,10 +33,11 @@
 
 namespace cake {
 
-constexpr int MK_CW = 16;                       // consumer warps
+constexpr int MK_CW = 8;                        // consumer warps: few, so that a thread has 168 registers (what spills lands in L2 beside 220 KB of shared memory)
 constexpr int MK_CT = MK_CW * 32;               // consumer threads
 constexpr int MK_THREADS = (MK_CW + 1) * 32;    // + producer warp
 constexpr int MK_STAGE_BYTES = 32768;
+constexpr int MK_BATCH = 512;                   // row segments whose sums are kept until an epilogue takes them
 constexpr int MK_MAX_STAGES = 6;
 constexpr int MK_MAX_LAYERS = 96;
 
@@ -34,26 +45,35 @@ struct MkLayer {
   const void *wqkv, *wo, *wgu, *wd, *ln1, *ln2, *bqkv, *qn, *kn;
   void *kc, *vc;
 };
-struct MkGeom {  // one decode GEMV type; a stage holds RS row segments of KC columns
-  int N, K, KC, RS, WPR, RPW;
+struct MkGeom {  // one decode GEMV type; a stage holds 2^RSL row segments of KC columns (planned by the host: no divisions in the kernel)
+  int N, K, KC, RSL, nchunk;   // nchunk = K / KC; above 1 a stage holds one segment
+  int n_groups, batch;         // groups of 2^RSL rows; groups between two epilogues
+  int unit, cnt, rem;          // static groups: CTA c has unit * (cnt + (c < rem)) of them
+  int pool;                    // first group of the pool (n_groups: none)
+  float inv_k;                 // 1 / K
+};
+// the vectors that travel as packets (uint32_t: value | tag << 16)
+struct MkPackets {
+  uint32_t *xa, *qkv, *y, *xb, *mm;   // layer output, projections, attention, behind the o product, act(gate) * up
+  uint64_t *acc, *ml;                 // attention of several splits: fp32 values | 32-bit tag << 32; ml holds (max, sum) pairs
 };
 struct MkArgs {
   const MkLayer *layers;
   int n_layers;
-  MkGeom g_qkv, g_o, g_gu, g_down, g_head;
+  MkGeom g[5];               // qkv, o, gate_up, down, head
   int hidden, inter, n_heads, n_kv, hd, rot, cap, nsplit, max_k;
   float eps, scale;
   const void *x_in;          // input hidden state (nullptr on the master: embed row of *d_token)
   const void *embed;
   const uint32_t *d_token;
   void *x_out;               // output hidden state of this shard
-  void *xa, *xb, *qkv, *y, *mm;
-  float *ws_ml, *ws_acc;
-  unsigned *attn_counters;
+  MkPackets pk;
   const void *cos_t, *sin_t;
   int *d_pos, *d_step;
-  unsigned long long *gbar;      // [0] monotonic barrier arrival counter, [1] its value at launch start
-  int has_head, advance, n_stages, vocab, partial_floats;
+  unsigned long long *gbar;      // [0] monotonic barrier arrival counter, [1] its value at launch start, [2] layers run so far (the tags)
+  int has_head, advance, n_stages, vocab;
+  int meet;                      // one grid barrier per layer: some CTA may own no row of a layer (see the top)
+  int keep_x;                    // the residual stream stays in shared memory between the phase that reads it and the one that adds it
   const void *ln_f, *lm_head;
   void *logits;
   float *part_val;
@@ -67,9 +87,8 @@ struct MkArgs {
   const unsigned long long *inbox_ctr;
   unsigned long long *peer_ctr;
   unsigned long long *ring_seq;   // hand-offs received so far (device-resident, never reset)
-  unsigned *tickets;          // [phase] work-claim counters, zeroed before every launch
-  int max_groups;             // per-CTA cap of row groups in one phase (sizes the partial-sum scratch)
-  int l2_prefetch;            // experimental (CAKE_B200_L2_PREFETCH=1): producer prefetches its future rows into L2
+  unsigned *tickets;          // [phase] work-claim counters, zeroed before every launch that has a phase with a pool
+  int off_x, off_res, off_part, off_loc, off_rows;  // shared memory (mk_layout)
   unsigned long long *trace;  // optional: %globaltimer stamps of CTA 0 at phase boundaries (profiling aid)
   // always on (3 stores per launch): %globaltimer of CTA 0 at kernel entry / input acquired / exit, ring of
   // MK_STEP_RING steps x 2 launches (tag 0: the layer launch, tag 1: rank 0's head-only launch when sharded) x 4 u64
@@ -77,6 +96,7 @@ struct MkArgs {
   int trace_tag;
   int act;     // mlp.rs:25-26: 0 silu, 1 gelu_tanh
   int window;  // cache.rs:173-205 sliding window (0 = full context): attention covers the last `window` positions
+  int *err;    // host-mapped: set by a wait for packets that ran out
 };
 constexpr int MK_STEP_RING = 2048;
 __device__ __forceinline__ unsigned long long mk_gtime() {
@@ -85,22 +105,31 @@ __device__ __forceinline__ unsigned long long mk_gtime() {
   return t;
 }
 
+// what the consumers look up per layer, copied to shared memory at the start
+struct MkRow {
+  const void *ln1, *ln2, *bqkv, *qn, *kn;
+  void *kc, *vc;
+};
 __host__ __device__ inline size_t mk_xs_bytes(int max_k, int es) {
   size_t b = (size_t)max_k * es;
   const size_t attn = (size_t)(ATTN_MAX_G * 256 * 4) + (size_t)ATTN_MAX_G * ATTN_TILE * 4 + (size_t)2 * 256 * 4;
   return b > attn ? b : attn;  // the attention phase overlays its scratch on the x buffer
 }
-__host__ __device__ inline size_t mk_smem_bytes(int max_k, int partial_floats, int max_groups, int n_stages, int es) {
-  size_t off = (size_t)n_stages * MK_STAGE_BYTES;
-  off += mk_xs_bytes(max_k, es);
-  off = (off + 15) & ~(size_t)15;
-  off += (size_t)partial_floats * 4;     // partial sums [row][slice]
-  off += (size_t)max_groups * 4;         // first row of each locally processed group
-  off += 128 * 4;                        // scratch
-  off = (off + 7) & ~(size_t)7;
-  off += (size_t)2 * MK_MAX_STAGES * 8;  // mbarriers
-  off += (size_t)MK_MAX_STAGES * 4;      // stage_row
-  return off + 256;
+// Shared memory: barriers, stage rows and scratch at fixed places, the ring, then what the model's sizes decide.
+constexpr int MK_OFF_EMPTY = 8 * MK_MAX_STAGES, MK_OFF_STAGE_ROW = 16 * MK_MAX_STAGES, MK_OFF_SCRATCH = 256, MK_OFF_RING = 1024;
+inline size_t mk_layout(MkArgs &a, int es) {
+  size_t off = MK_OFF_RING + (size_t)a.n_stages * MK_STAGE_BYTES;
+  auto take = [&](size_t bytes) {
+    const size_t at = off;
+    off = (off + bytes + 15) & ~(size_t)15;
+    return (int)at;
+  };
+  a.off_x = take(mk_xs_bytes(a.max_k, es));
+  a.off_res = take(a.keep_x ? (size_t)a.hidden * es : 0);
+  a.off_part = take(MK_BATCH * MK_CW * 4);  // partial sums [row][warp of the row]
+  a.off_loc = take(MK_BATCH * 4);           // first row of each group of a batch
+  a.off_rows = take((size_t)a.n_layers * sizeof(MkRow));
+  return off;
 }
 
 __device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long long *p) {
@@ -108,178 +137,101 @@ __device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long
   asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return v;
 }
-__device__ __forceinline__ uint4 ldcg_v4(const void *p) { return __ldcg(reinterpret_cast<const uint4 *>(p)); }
 
 struct MkRing {
-  unsigned char *ring;
-  uint64_t *full, *empty;
-  int *stage_row;  // first weight row held by a stage, or -1 = end-of-phase marker (dynamic phases)
+  unsigned char *sm;
   int n_stages;
   int s;
   uint32_t ph;
+  __device__ __forceinline__ uint64_t *full() const { return reinterpret_cast<uint64_t *>(sm) + s; }
+  __device__ __forceinline__ uint64_t *empty() const { return reinterpret_cast<uint64_t *>(sm + MK_OFF_EMPTY) + s; }
+  // first weight row held by a stage, or -1 = end-of-phase marker (phases with a pool)
+  __device__ __forceinline__ int &row() const { return reinterpret_cast<int *>(sm + MK_OFF_STAGE_ROW)[s]; }
+  __device__ __forceinline__ unsigned char *data() const { return sm + MK_OFF_RING + (size_t)s * MK_STAGE_BYTES; }
   __device__ __forceinline__ void advance() {
     if (++s == n_stages) { s = 0; ph ^= 1u; }
   }
 };
 
-// rows [r0,r1) of this CTA for a GEMV over N rows with row granularity G
-__device__ __forceinline__ void mk_rows(int N, int G, int &r0, int &r1) {
-  const long units = N / G;
-  r0 = (int)(units * blockIdx.x / gridDim.x) * G;
-  r1 = (int)(units * (blockIdx.x + 1) / gridDim.x) * G;
-}
-
-// Dynamic phases: the N/RS row groups of a GEMV are split into a static part (75 %: CTA c owns groups
-// [c*sg, (c+1)*sg)) and a pool claimed one group at a time through an atomic ticket.  Per-SM HBM bandwidth is
-// not uniform (measured: the slowest CTA of the gate_up phase finished 5.5 us after the fastest with static
-// rows), so fast SMs take more pool groups and all CTAs reach the grid barrier together.  A row's dot product
+// The row groups of a GEMV are split into a static part and a pool claimed one group at a time through an atomic ticket.  Per-SM HBM
+// bandwidth is not uniform (measured: the slowest CTA of the 8B gate_up phase finished 5.5 us after the fastest with static
+// rows), so fast SMs take more pool groups and all CTAs end together: 75 % static (CTA c owns groups [c*cnt, (c+1)*cnt)).  A phase of at most
+// MK_SHORT groups per CTA sits in the ring before its input is there, and the CTA that claims one group more than the others is late:
+// all of it is static, dealt out evenly; so are rows that take several stages (K of more than a stage).  A row's dot product
 // is computed by one CTA with a fixed lane/warp mapping whichever CTA it is -> results stay bit-deterministic.
-struct MkSplit {
-  int n_groups, sg, pool_start;
-};
-__device__ __forceinline__ MkSplit mk_split(const MkGeom &g) {
-  MkSplit sp;
-  sp.n_groups = (g.N + g.RS - 1) / g.RS;
-  sp.sg = (int)(((long)sp.n_groups * 3 / 4) / gridDim.x);
-  sp.pool_start = sp.sg * gridDim.x;
-  return sp;
-}
-__device__ __forceinline__ bool mk_is_dynamic(const MkGeom &g) { return g.K == g.KC && (g.KC / 8) / g.WPR <= 128; }
-
-// L2 prefetch cursor.  HBM idles whenever the consumers sit in a grid barrier or in the attention phase and the
-// shared-memory ring is full (~20 us per layer).  The producer therefore also walks its OWN future static row
-// groups — across phase and layer boundaries — MK_PF_AHEAD groups ahead of the load cursor and issues
-// cp.async.bulk.prefetch.L2 for them: the bytes stream into the 126 MB L2 during those windows and the later
-// TMA loads hit L2.  ~14 x 32 KB x 148 CTAs = 66 MB in flight.
-constexpr int MK_PF_AHEAD = 14;
-struct MkPrefetch {
-  const MkArgs *a;
-  int l, ph, grp;  // layer, phase within the layer (0 qkv, 1 o, 2 gate_up, 3 down; l == n_layers: head), next group
-  int es;
-  __device__ __forceinline__ bool phase(const MkGeom *&g, const void *&W) const {
-    if (l < a->n_layers) {
-      const MkLayer &L = a->layers[l];
-      g = ph == 0 ? &a->g_qkv : ph == 1 ? &a->g_o : ph == 2 ? &a->g_gu : &a->g_down;
-      W = ph == 0 ? L.wqkv : ph == 1 ? L.wo : ph == 2 ? L.wgu : L.wd;
-      return true;
-    }
-    if (l == a->n_layers && a->has_head && ph == 0) { g = &a->g_head; W = a->lm_head; return true; }
-    return false;
-  }
-  __device__ __forceinline__ void step() {  // prefetch one more static group of this CTA, if any is left
-    while (true) {
-      const MkGeom *g;
-      const void *W;
-      if (!phase(g, W)) return;
-      if (mk_is_dynamic(*g)) {
-        const MkSplit sp = mk_split(*g);
-        if (grp < sp.sg) {
-          const int row = ((int)blockIdx.x * sp.sg + grp) * g->RS;
-          const size_t rowb = (size_t)g->K * es;
-          const unsigned bytes = (unsigned)(min(g->RS, g->N - row) * rowb);
-          asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(reinterpret_cast<const unsigned char *>(W) + (size_t)row * rowb), "r"(bytes) : "memory");
-          grp++;
-          return;
-        }
-      }
-      grp = 0;
-      if (l < a->n_layers && ph < 3) ph++;
-      else { l++; ph = 0; }
-    }
-  }
-};
-
-// Targeted variant (l2_prefetch == 2): only while HBM is otherwise idle — right after the attention K/V tiles were
-// issued — pull this CTA's static rows of the following GEMV phases into L2.
-__device__ __forceinline__ void mk_prefetch_static(const MkGeom &g, const void *W, int es, int first, int count) {
-  if (!mk_is_dynamic(g)) return;
-  const MkSplit sp = mk_split(g);
-  const size_t rowb = (size_t)g.K * es;
-  for (int i = first; i < sp.sg && i < first + count; i++) {
-    const int row = ((int)blockIdx.x * sp.sg + i) * g.RS;
-    const unsigned bytes = (unsigned)(min(g.RS, g.N - row) * rowb);
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(reinterpret_cast<const unsigned char *>(W) + (size_t)row * rowb), "r"(bytes) : "memory");
+constexpr int MK_SHORT = 4;
+inline void mk_plan_split(MkGeom &g, int gran, int grid) {  // gran: rows that stay together (gate and up of a pair)
+  g.inv_k = 1.0f / (float)g.K;
+  g.n_groups = (g.N + (1 << g.RSL) - 1) >> g.RSL;
+  g.batch = (MK_BATCH >> g.RSL) / g.nchunk;
+  if (g.nchunk > 1 || g.n_groups <= MK_SHORT * grid) {
+    g.unit = gran > 1 << g.RSL ? gran : 1;
+    g.cnt = g.n_groups / g.unit / grid;
+    g.rem = g.n_groups / g.unit % grid;
+    g.pool = g.n_groups;
+  } else {
+    g.unit = 1;
+    g.cnt = (int)(((long)g.n_groups * 3 / 4) / grid);
+    g.rem = 0;
+    g.pool = g.cnt * grid;
   }
 }
+// every CTA owns at least one row of this phase, whatever the tickets say
+inline bool mk_every_cta(const MkGeom &g) { return g.cnt > 0; }
+__device__ __forceinline__ int mk_first(const MkGeom &g) { return g.unit * ((int)blockIdx.x * g.cnt + min((int)blockIdx.x, g.rem)); }
+__device__ __forceinline__ int mk_count(const MkGeom &g) { return g.unit * (g.cnt + ((int)blockIdx.x < g.rem ? 1 : 0)); }
 
 template <typename T>
-__device__ __forceinline__ void mk_produce_gemv_dyn(MkRing &rg, const MkGeom &g, const void *W, unsigned *ticket, int max_groups,
-                                                    uint64_t pol, MkPrefetch &pf) {
+__device__ __forceinline__ void mk_produce_gemv(MkRing &rg, const MkGeom &g, const void *W, unsigned *ticket, uint64_t pol) {
   constexpr int es = sizeof(T);
-  const MkSplit sp = mk_split(g);
   const size_t rowb = (size_t)g.K * es;
   const unsigned char *Wb = reinterpret_cast<const unsigned char *>(W);
-  int issued = 0;
   auto issue = [&](int grp) {
-    const int row = grp * g.RS, nr = min(g.RS, g.N - row);
-    mbar_wait(&rg.empty[rg.s], rg.ph ^ 1u);
-    rg.stage_row[rg.s] = row;
-    mbar_arrive_expect_tx(&rg.full[rg.s], (uint32_t)(nr * rowb));
-    bulk_g2s(rg.ring + (size_t)rg.s * MK_STAGE_BYTES, Wb + (size_t)row * rowb, (uint32_t)(nr * rowb), &rg.full[rg.s], pol);
-    rg.advance();
-    issued++;
-  };
-  for (int grp = blockIdx.x * sp.sg; grp < (int)(blockIdx.x + 1) * sp.sg; grp++) {
-    issue(grp);
-    if (pf.a->l2_prefetch == 1) pf.step();  // keep the L2 prefetch MK_PF_AHEAD static groups ahead of the load cursor
-  }
-  if (sp.pool_start < sp.n_groups && issued < max_groups) {
-    unsigned next = atomicAdd(ticket, 1u);
-    while (sp.pool_start + (int)next < sp.n_groups) {
-      const int cur = sp.pool_start + (int)next;
-      const bool more = issued + 1 < max_groups;  // a claimed group is never dropped: claim only what fits
-      if (more) next = atomicAdd(ticket, 1u);     // claim ahead: the round trip overlaps the wait for a free stage
-      issue(cur);
-      if (!more) break;
+    const int row = grp << g.RSL, nr = min(1 << g.RSL, g.N - row);
+    const uint32_t bytes = (uint32_t)nr * g.KC * es;   // (several rows only where a row is one segment)
+    for (int k = 0; k < g.K; k += g.KC) {
+      mbar_wait(rg.empty(), rg.ph ^ 1u);
+      rg.row() = row;
+      mbar_arrive_expect_tx(rg.full(), bytes);
+      bulk_g2s(rg.data(), Wb + (size_t)row * rowb + (size_t)k * es, bytes, rg.full(), pol);
+      rg.advance();
     }
+  };
+  const int first = mk_first(g), n = mk_count(g);
+#pragma unroll 1
+  for (int i = 0; i < n; i++) issue(first + i);
+  if (g.pool == g.n_groups) return;
+  unsigned next = atomicAdd(ticket, 1u);
+#pragma unroll 1
+  while (g.pool + (int)next < g.n_groups) {
+    const int cur = g.pool + (int)next;
+    next = atomicAdd(ticket, 1u);  // claim ahead: the round trip overlaps the wait for a free stage
+    issue(cur);
   }
-  mbar_wait(&rg.empty[rg.s], rg.ph ^ 1u);  // end-of-phase marker
-  rg.stage_row[rg.s] = -1;
-  mbar_arrive(&rg.full[rg.s]);
+  mbar_wait(rg.empty(), rg.ph ^ 1u);  // end-of-phase marker: the consumers do not know how many groups were claimed
+  rg.row() = -1;
+  mbar_arrive(rg.full());
   rg.advance();
 }
 
-template <typename T>
-__device__ __forceinline__ void mk_produce_gemv(MkRing &rg, const MkGeom &g, const void *W, int G, uint64_t pol) {
-  constexpr int es = sizeof(T);
-  int r0, r1;
-  mk_rows(g.N, G, r0, r1);
-  const int nchunk = g.K / g.KC;
-  const size_t seg = (size_t)g.KC * es;
-  const unsigned char *Wb = reinterpret_cast<const unsigned char *>(W);
-  for (int row = r0; row < r1; row += g.RS) {
-    const int nr = min(g.RS, r1 - row);
-    for (int j = 0; j < nchunk; j++) {
-      mbar_wait(&rg.empty[rg.s], rg.ph ^ 1u);
-      unsigned char *dst = rg.ring + (size_t)rg.s * MK_STAGE_BYTES;
-      mbar_arrive_expect_tx(&rg.full[rg.s], (uint32_t)(nr * seg));
-      if (nchunk == 1) {
-        bulk_g2s(dst, Wb + (size_t)row * g.K * es, (uint32_t)(nr * seg), &rg.full[rg.s], pol);
-      } else {
-        for (int r = 0; r < nr; r++)
-          bulk_g2s(dst + r * seg, Wb + ((size_t)(row + r) * g.K + (size_t)j * g.KC) * es, (uint32_t)seg, &rg.full[rg.s], pol);
-      }
-      rg.advance();
-    }
-  }
-}
-
 struct MkAttnItem {
-  int active, kvh, split, s0, s1, tile;
+  int active, kvh, split, n_split, s0, s1, tile;
 };
-template <typename T>
-__device__ __forceinline__ MkAttnItem mk_attn_item(const MkArgs &a, int pos) {
+// The visible positions are cut over as many CTAs as have MK_SPLIT_MIN of them each; up to MK_SPLIT_ONE one CTA per key head takes them all:
+// what further CTAs would save of its tile (0.4 us) is less than the exchange of their parts (1.5 us).
+constexpr int MK_SPLIT_MIN = 64, MK_SPLIT_ONE = 128;
+__device__ __forceinline__ MkAttnItem mk_attn_item(const MkArgs &a, int pos, int es) {
   MkAttnItem it;
-  const int items = a.n_kv * a.nsplit;
-  it.active = (int)blockIdx.x < items;
   it.kvh = blockIdx.x / a.nsplit;
   it.split = blockIdx.x % a.nsplit;
   const int Tn = pos + 1;
   int per = (Tn + a.nsplit - 1) / a.nsplit;
-  per = (per + 7) & ~7;
+  per = max((per + 7) & ~7, Tn <= MK_SPLIT_ONE ? MK_SPLIT_ONE : MK_SPLIT_MIN);
+  it.n_split = (Tn + per - 1) / per;
+  it.active = (int)blockIdx.x < a.n_kv * a.nsplit && it.split < it.n_split;
   it.s0 = min(Tn, it.split * per);
   it.s1 = min(Tn, it.s0 + per);
-  const int rows = MK_STAGE_BYTES / (a.hd * (int)sizeof(T));
+  const int rows = MK_STAGE_BYTES / (a.hd * es);
   it.tile = rows < ATTN_TILE ? rows : ATTN_TILE;
   if (!it.active) it.s0 = it.s1 = 0;
   return it;
@@ -290,7 +242,8 @@ __device__ __forceinline__ void mk_produce_attn(MkRing &rg, const MkArgs &a, con
   // sliding window: the visible rows start at ws = pos + 1 - window; everything below works on row indices relative to ws
   const int ws = (a.window > 0 && pos + 1 > a.window) ? pos + 1 - a.window : 0;
   pos -= ws;
-  const MkAttnItem it = mk_attn_item<T>(a, pos);
+  const MkAttnItem it = mk_attn_item(a, pos, (int)sizeof(T));
+  if (!it.active) return;
   const int HD = a.hd;
   const T *kc = reinterpret_cast<const T *>(L.kc) + ((size_t)it.kvh * a.cap + ws) * HD;
   const T *vc = reinterpret_cast<const T *>(L.vc) + ((size_t)it.kvh * a.cap + ws) * HD;
@@ -298,270 +251,466 @@ __device__ __forceinline__ void mk_produce_attn(MkRing &rg, const MkArgs &a, con
     const int t1 = min(it.s1, t0 + it.tile);
     const int nold = min(t1, pos) - t0;  // rows already in the cache (the appended row is handled by the consumers)
     for (int kv = 0; kv < 2; kv++) {
-      mbar_wait(&rg.empty[rg.s], rg.ph ^ 1u);
+      mbar_wait(rg.empty(), rg.ph ^ 1u);
       if (nold > 0) {
         const uint32_t bytes = (uint32_t)nold * HD * sizeof(T);
-        mbar_arrive_expect_tx(&rg.full[rg.s], bytes);
-        bulk_g2s(rg.ring + (size_t)rg.s * MK_STAGE_BYTES, (kv ? vc : kc) + (size_t)t0 * HD, bytes, &rg.full[rg.s], pol);
+        mbar_arrive_expect_tx(rg.full(), bytes);
+        bulk_g2s(rg.data(), (kv ? vc : kc) + (size_t)t0 * HD, bytes, rg.full(), pol);
       } else {
-        mbar_arrive(&rg.full[rg.s]);
+        mbar_arrive(rg.full());
       }
       rg.advance();
     }
   }
+}
+
+// Reciprocals and square roots by the fast instruction and one Newton step, to an ulp.  (The correctly rounded forms end in a call for the rare
+// cases, and a call makes the compiler keep what is live around it in local memory.)
+__device__ __forceinline__ float mk_rsqrt(float v) {   // v > 0, or inf
+  const float y = rsqrtf(v), e = fmaf(-v * y, y, 1.0f);
+  return v == INFINITY ? y : fmaf(0.5f * y, e, y);
+}
+__device__ __forceinline__ float mk_rcp(float v) {     // 2^-126 <= |v| < 2^126
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(v));
+  return fmaf(y, fmaf(-v, y, 1.0f), y);
+}
+// gate_act (common.cuh) without the division: below -60 the 1 of 1 + e^-g is far below an ulp, and g e^g the same value
+template <typename T> __device__ __forceinline__ float mk_gate_act(float g, int act) {
+  if (act) return gate_act<T>(g, 1);
+  return rnd<T>(g < -60.f ? g * expf(g) : g * mk_rcp(1.0f + expf(-g)));
+}
+
+// ---------------------------------------------------------------------------------------- packets
+// A thread's waits for other CTAs share one budget: when it is spent the error word is set, and every later wait of the thread returns at once.
+// A poll is a round trip to L2 (0.6 us or more), so a wait gives up after seconds, and a launch whose waits all give up still ends.
+constexpr int MK_POLLS = 1 << 21;
+struct MkWait {
+  int left;
+  int *err;
+  __device__ __forceinline__ bool again() {
+    if (left <= 0) return false;
+    if (--left == 0) *reinterpret_cast<volatile int *>(err) = 1;
+    return true;
+  }
+};
+__device__ __forceinline__ uint4 pk_load4(const uint32_t *p) {
+  uint4 u;
+  asm volatile("ld.relaxed.gpu.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(u.x), "=r"(u.y), "=r"(u.z), "=r"(u.w) : "l"(p));
+  return u;
+}
+__device__ __forceinline__ uint32_t pk_load(const uint32_t *p) {
+  uint32_t u;
+  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(u) : "l"(p));
+  return u;
+}
+__device__ __forceinline__ uint64_t pk_load64(const uint64_t *p) {
+  uint64_t u;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(u) : "l"(p));
+  return u;
+}
+// tag: in the upper 16 bits
+__device__ __forceinline__ bool pk_stale4(const uint4 &u, uint32_t tag) {
+  return (((u.x ^ tag) | (u.y ^ tag) | (u.z ^ tag) | (u.w ^ tag)) & 0xffff0000u) != 0;
+}
+__device__ __forceinline__ uint2 pk_values4(const uint4 &u) { return make_uint2(__byte_perm(u.x, u.y, 0x5410), __byte_perm(u.z, u.w, 0x5410)); }
+template <typename T> __device__ __forceinline__ void pk_store(uint32_t *p, T v, uint32_t tag) {
+  asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(tag | (uint32_t)*reinterpret_cast<const uint16_t *>(&v)) : "memory");
+}
+__device__ __forceinline__ void pk_store64(uint64_t *p, float v, uint32_t tag) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"((uint64_t)__float_as_uint(v) | (uint64_t)tag << 32) : "memory");
+}
+__device__ __forceinline__ float pk_poll64(const uint64_t *p, uint32_t tag, MkWait &w) {
+  uint64_t u = pk_load64(p);
+  while ((uint32_t)(u >> 32) != tag && w.again()) u = pk_load64(p);
+  return __uint_as_float((uint32_t)u);
+}
+template <typename T> __device__ __forceinline__ T pk_value(uint32_t u) {
+  const uint16_t h = (uint16_t)u;
+  T r;
+  *reinterpret_cast<uint16_t *>(&r) = h;
+  return r;
+}
+template <typename T> __device__ __forceinline__ float4 pk_floats4(const uint4 &u) {
+  const uint2 v = pk_values4(u);
+  const float2 a = DT<T>::unpack2(v.x), b = DT<T>::unpack2(v.y);
+  return make_float4(a.x, a.y, b.x, b.y);
 }
 
 // ---------------------------------------------------------------------------------------- consumers
-__device__ __forceinline__ void mk_grid_sync(unsigned long long *ctr, unsigned long long target, int ct) {
+// `meet`: all CTAs of the grid, once per layer (release: bar.sync + red.release; acquire: poll)
+__device__ __forceinline__ void mk_grid_sync(unsigned long long *ctr, unsigned long long target, int ct, MkWait &w) {
   named_bar_sync(1, MK_CT);  // every consumer thread of this CTA has issued its global writes
   if (ct == 0) {
-    // release: publishes this CTA's writes (ordered before us by the bar.sync above); fire-and-forget
     asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(ctr), "l"(1ULL) : "memory");
-    while (ld_acquire_u64(ctr) < target) {
+    while (ld_acquire_u64(ctr) < target && w.again()) {
     }
   }
-  named_bar_sync(1, MK_CT);  // data written by other SMs is read with ld.global.cg below (L1 is bypassed)
+  named_bar_sync(1, MK_CT);
 }
 
-// x -> shared (D), optionally RMS-normalised.  Activations were written by other SMs: ld.global.cg.
+// x -> shared (D) and, where the phase keeps the residual stream, a second copy; returns this thread's share of the sum of squares.
+// A thread's packets are MK_CT quads apart.  The first four are polled (16 KB per CTA); the others are asked for when those are there, six at a time:
+// polling every packet of a long vector (57 KB per CTA for the 8B down product) would take the L2 bandwidth that the weights need.
 template <typename T>
-__device__ __forceinline__ void mk_stage_x(T *xs, const void *x, const void *norm_w, int K, float eps, float *scratch,
-                                           int ct, int warp, int lane) {
-  constexpr int es = sizeof(T);
-  uint4 *xsv = reinterpret_cast<uint4 *>(xs);
-  const int nv = K * es / 16;
-  const char *xb = reinterpret_cast<const char *>(x);
-  if (norm_w == nullptr) {
-    for (int v = ct; v < nv; v += MK_CT) xsv[v] = ldcg_v4(xb + (size_t)v * 16);
-  } else {
-    float ss = 0.f;
-    for (int v = ct; v < nv; v += MK_CT) {
-      const uint4 u = ldcg_v4(xb + (size_t)v * 16);
-      xsv[v] = u;
-      float f[8];
-      unpack8<T>(u, f);
+__device__ __forceinline__ float mk_gather(T *xs, T *keep, const uint32_t *pk, int K, uint32_t tag, int ct, MkWait &w) {
+  const int nq = K >> 2;
+  float ss = 0.f;
+  auto put = [&](int q, const uint4 &u) {
+    const uint2 v = pk_values4(u);
+    *reinterpret_cast<uint2 *>(xs + 4 * q) = v;
+    if (keep) *reinterpret_cast<uint2 *>(keep + 4 * q) = v;
+    const float2 f0 = DT<T>::unpack2(v.x), f1 = DT<T>::unpack2(v.y);
+    ss += f0.x * f0.x + f0.y * f0.y + f1.x * f1.x + f1.y * f1.y;
+  };
+  uint4 u[6];
+  const int n4 = min(4, (nq - ct + MK_CT - 1) / MK_CT);  // (0 or less: this thread has none)
+  if (n4 > 0) {
+    bool stale;
+    do {
+      stale = false;
 #pragma unroll
-      for (int i = 0; i < 8; i++) ss += f[i] * f[i];
+      for (int i = 0; i < 4; i++)
+        if (i < n4) u[i] = pk_load4(pk + 4 * (ct + i * MK_CT));
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+        if (i < n4) stale = stale || pk_stale4(u[i], tag);
+    } while (stale && w.again());
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+      if (i < n4) put(ct + i * MK_CT, u[i]);
+  }
+#pragma unroll 1
+  for (int q = ct + 4 * MK_CT; q < nq; q += 6 * MK_CT) {
+    bool stale;
+    do {
+      stale = false;
+#pragma unroll
+      for (int i = 0; i < 6; i++)
+        if (q + i * MK_CT < nq) u[i] = pk_load4(pk + 4 * (q + i * MK_CT));
+#pragma unroll
+      for (int i = 0; i < 6; i++)
+        if (q + i * MK_CT < nq) stale = stale || pk_stale4(u[i], tag);
+    } while (stale && w.again());
+#pragma unroll
+    for (int i = 0; i < 6; i++)
+      if (q + i * MK_CT < nq) put(q + i * MK_CT, u[i]);
+  }
+  return ss;
+}
+// the same from a plain vector (the step's input: complete before the launch, or acquired from the inbox)
+template <typename T>
+__device__ __forceinline__ float mk_copy_x(T *xs, T *keep, const T *x, int K, int ct) {
+  float ss = 0.f;
+  for (int q = ct; q < K / 4; q += MK_CT) {
+    const uint2 v = __ldcg(reinterpret_cast<const uint2 *>(x) + q);
+    reinterpret_cast<uint2 *>(xs)[q] = v;
+    if (keep) reinterpret_cast<uint2 *>(keep)[q] = v;
+    const float2 f0 = DT<T>::unpack2(v.x), f1 = DT<T>::unpack2(v.y);
+    ss += f0.x * f0.x + f0.y * f0.y + f1.x * f1.x + f1.y * f1.y;
+  }
+  return ss;
+}
+
+// the largest value of a warp and its index; the smaller index where values are equal
+__device__ __forceinline__ void mk_warp_best(float &best, int &idx) {
+#pragma unroll 1
+  for (int o = 16; o > 0; o >>= 1) {
+    const float ov = __shfl_xor_sync(0xffffffffu, best, o);
+    const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
+    if (ov > best || (ov == best && oi < idx)) { best = ov; idx = oi; }
+  }
+}
+
+// acc += w[0] x[0] and w[1] x[1] of two packed 16-bit pairs: the fused multiply-add that takes 16-bit factors and a 32-bit sum (the product is exact, the
+// sum is rounded once, as with both factors converted to fp32).  It issues at the rate of the 32-bit one (1.13 cycles against 1.10, eight chains),
+// so the conversions are gone: 64 instructions for a stage's 8 vectors of a lane where there were 128 to 192.
+template <typename T> __device__ __forceinline__ void mk_fma2(float &lo, float &hi, uint32_t w, uint32_t x);
+template <> __device__ __forceinline__ void mk_fma2<__nv_bfloat16>(float &lo, float &hi, uint32_t w, uint32_t x) {
+  asm("{\n\t.reg .b16 a, b, c, d;\n\tmov.b32 {a, b}, %2;\n\tmov.b32 {c, d}, %3;\n\tfma.rn.f32.bf16 %0, a, c, %0;\n\tfma.rn.f32.bf16 %1, b, d, %1;\n\t}"
+      : "+f"(lo), "+f"(hi) : "r"(w), "r"(x));
+}
+template <> __device__ __forceinline__ void mk_fma2<__half>(float &lo, float &hi, uint32_t w, uint32_t x) {
+  asm("{\n\t.reg .b16 a, b, c, d;\n\tmov.b32 {a, b}, %2;\n\tmov.b32 {c, d}, %3;\n\tfma.rn.f32.f16 %0, a, c, %0;\n\tfma.rn.f32.f16 %1, b, d, %1;\n\t}"
+      : "+f"(lo), "+f"(hi) : "r"(w), "r"(x));
+}
+// 8 weights times x, into four running sums
+template <typename T> __device__ __forceinline__ void mk_dot8(float (&acc)[4], const uint4 &w, const uint4 &x) {
+  mk_fma2<T>(acc[0], acc[1], w.x, x.x);
+  mk_fma2<T>(acc[2], acc[3], w.y, x.y);
+  mk_fma2<T>(acc[0], acc[1], w.z, x.z);
+  mk_fma2<T>(acc[2], acc[3], w.w, x.w);
+}
+__device__ __forceinline__ bool mk_ready(uint64_t *bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+  return __all_sync(0xffffffffu, ok);
+}
+
+// bookkeeping that a launch keeps in the scratch area, as 64-bit words behind the 32 + 32 words of the reductions
+constexpr int MK_START = 32;
+// stamps of CTA 0 in the optional trace: 1 + 10 per layer: input gathered, output published of qkv, attention (begin, end), o, gate_up, down
+__device__ __forceinline__ void mk_stamp(const MkArgs &a, int l, int ph, int end) {
+  if (a.trace && blockIdx.x == 0 && threadIdx.x == 0) a.trace[1 + 10 * l + 2 * ph + (ph ? 2 : 0) + end] = mk_gtime();
+}
+template <typename T> __device__ __forceinline__ const T *mk_x_in(const MkArgs &a) {
+  if (a.x_in) return reinterpret_cast<const T *>(a.x_in);
+  uint32_t tok = *a.d_token;  // master: the block input is the embedding row of the current token (text_model.rs:271)
+  if (tok >= (uint32_t)a.vocab) tok = 0;  // memory safety only: host entry points reject out-of-range ids (EINVAL); in-kernel argmax ids are < vocab
+  return reinterpret_cast<const T *>(a.embed) + (size_t)tok * a.hidden;
+}
+// 4 values normed: (x * inv) * w, rounded to D
+template <typename T> __device__ __forceinline__ uint2 mk_normed(const uint2 &x, const uint2 &w, float inv) {
+  const float2 a = DT<T>::unpack2(x.x), b = DT<T>::unpack2(x.y), wa = DT<T>::unpack2(w.x), wb = DT<T>::unpack2(w.y);
+  return make_uint2(pack2x<T>(a.x * inv * wa.x, a.y * inv * wa.y), pack2x<T>(b.x * inv * wb.x, b.y * inv * wb.y));
+}
+
+// end-of-step bookkeeping by one thread
+__device__ __forceinline__ void mk_end_of_step(const MkArgs &a, const float *scratch) {
+  if (a.advance) { *a.d_pos += 1; *a.d_step += 1; }
+  if (a.inbox_ctr) *a.ring_seq += 1ULL;
+  a.gbar[1] = reinterpret_cast<const unsigned long long *>(scratch)[MK_START] + (a.meet ? (unsigned long long)a.n_layers * gridDim.x : 0ULL);
+  a.gbar[2] += (unsigned long long)a.n_layers;
+}
+
+// the greedy token, by the CTA that is last
+__device__ __forceinline__ void mk_head_end(const MkArgs &a, float *scratch, float best, int bidx) {
+  const int ct = threadIdx.x, warp = ct >> 5, lane = ct & 31;
+  mk_warp_best(best, bidx);
+  int *scratch_i = reinterpret_cast<int *>(scratch + 32);
+  if (lane == 0) { scratch[warp] = best; scratch_i[warp] = bidx; }
+  named_bar_sync(1, MK_CT);
+  if (warp != 0) return;
+  // a lane per warp's best, then (the CTA that arrives last) the CTAs' bests, 32 at a time: for one thread both are chains of round trips
+  best = lane < MK_CW ? scratch[lane] : -INFINITY;
+  bidx = lane < MK_CW ? scratch_i[lane] : 0x7fffffff;
+  mk_warp_best(best, bidx);
+  unsigned ticket = 0;
+  if (lane == 0) {
+    a.part_val[blockIdx.x] = best;
+    a.part_idx[blockIdx.x] = bidx;
+    __threadfence();
+    ticket = atomicAdd(a.argmax_counter, 1u);
+  }
+  ticket = __shfl_sync(0xffffffffu, ticket, 0);
+  if (ticket != gridDim.x - 1) return;
+  __threadfence();
+  best = -INFINITY;
+  bidx = 0x7fffffff;
+#pragma unroll 1
+  for (unsigned c = lane; c < gridDim.x; c += 32) {
+    const float v = __ldcg(a.part_val + c);
+    const int i = __ldcg(a.part_idx + c);
+    if (v > best || (v == best && i < bidx)) { best = v; bidx = i; }
+  }
+  mk_warp_best(best, bidx);
+  if (lane == 0) {
+    *a.token_out = (uint32_t)bidx;
+    if (a.token_ring) a.token_ring[*a.d_step % a.ring_cap] = (uint32_t)bidx;
+    *a.argmax_counter = 0;
+    mk_end_of_step(a, scratch);  // this is the last CTA of the grid to finish
+  }
+}
+
+// one product of the step: input gathered, staged rows, fused epilogue, packets out.  What only one end of it needs is worked out there: values that
+// live across the loop over the stages cost registers that the loop needs.
+template <typename T>
+__device__ __forceinline__ void mk_gemv_phase(MkRing &rg, const MkArgs &a, unsigned char *sm, int l, int ph, uint32_t tag, int &left) {
+  const int ct = threadIdx.x, warp = ct >> 5, lane = ct & 31;
+  const bool head = l == a.n_layers;
+  const MkGeom &g = a.g[head ? 4 : ph];
+  T *xs = reinterpret_cast<T *>(sm + a.off_x), *res_s = reinterpret_cast<T *>(sm + a.off_res);
+  float *partial = reinterpret_cast<float *>(sm + a.off_part), *scratch = reinterpret_cast<float *>(sm + MK_OFF_SCRATCH);
+  int *loc_row = reinterpret_cast<int *>(sm + a.off_loc);
+  const MkRow &L = reinterpret_cast<const MkRow *>(sm + a.off_rows)[head ? 0 : l];  // (not read for the head)
+  const int RSL = g.RSL, nchunk = g.nchunk;
+  const bool norm = head || ph == 0 || ph == 2;
+  // ---- input
+  const T *norm_w = reinterpret_cast<const T *>(head ? a.ln_f : !norm ? nullptr : ph == 0 ? L.ln1 : L.ln2);
+  uint2 nw[4];  // this thread's norm weights, asked for before the input is waited for
+  if (norm) {
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+      if (ct + i * MK_CT < g.K / 4) nw[i] = reinterpret_cast<const uint2 *>(norm_w)[ct + i * MK_CT];
+  }
+  {
+    T *keep = a.keep_x && norm && !head ? res_s : nullptr;
+    MkWait w{left, a.err};
+    float ss;
+    if (l == 0 && ph == 0) {
+      ss = mk_copy_x<T>(xs, keep, mk_x_in<T>(a), g.K, ct);
+    } else {
+      const uint32_t *in = ph == 0 ? a.pk.xa : ph == 1 ? a.pk.y : ph == 2 ? a.pk.xb : a.pk.mm;
+      ss = mk_gather<T>(xs, keep, in, g.K, ph == 0 ? tag - 0x10000u : tag, ct, w);
     }
-    ss = warp_sum(ss);
-    if (lane == 0) scratch[warp] = ss;
+    if (norm) {
+      ss = warp_sum(ss);
+      if (lane == 0) scratch[warp] = ss;
+    }
     named_bar_sync(1, MK_CT);
+    if (a.meet && ph == 3) mk_grid_sync(a.gbar, reinterpret_cast<unsigned long long *>(scratch)[MK_START] + (unsigned long long)(l + 1) * gridDim.x, ct, w);
+    left = w.left;
+  }
+  if (norm) {  // each thread the values it gathered
     float tot = 0.f;
 #pragma unroll
-    for (int w = 0; w < MK_CW; w++) tot += scratch[w];
-    const float inv = 1.0f / sqrtf(tot / (float)K + eps);
-    const uint4 *wg = reinterpret_cast<const uint4 *>(norm_w);
-    for (int v = ct; v < nv; v += MK_CT) {
-      float f[8], w8[8];
-      unpack8<T>(xsv[v], f);
-      unpack8<T>(wg[v], w8);
-      uint4 o;
-      o.x = pack2<T>(f[0] * inv * w8[0], f[1] * inv * w8[1]);
-      o.y = pack2<T>(f[2] * inv * w8[2], f[3] * inv * w8[3]);
-      o.z = pack2<T>(f[4] * inv * w8[4], f[5] * inv * w8[5]);
-      o.w = pack2<T>(f[6] * inv * w8[6], f[7] * inv * w8[7]);
-      xsv[v] = o;
+    for (int i = 0; i < MK_CW / 4; i++) {
+      const float4 f = reinterpret_cast<const float4 *>(scratch)[i];
+      tot += (f.x + f.y) + (f.z + f.w);
     }
-  }
-  named_bar_sync(1, MK_CT);
-}
-
-struct MkEpi {
-  const void *bias, *residual;
-  void *out;
-  int act;  // EPI_SWIGLU: 0 silu, 1 gelu_tanh
-  // argmax
-  float *part_val;
-  int *part_idx;
-  unsigned *counter;
-  uint32_t *token_out, *token_ring;
-  const int *step;
-  int ring_cap;
-  // end-of-step bookkeeping done by the argmax finaliser
-  int advance;
-  int *d_pos, *d_step;
-  unsigned long long *gbar;
-  unsigned long long next_start;
-  unsigned long long *ring_seq;  // non-null when this launch consumed an inbox hand-off
-};
-
-template <typename T, int EPI>
-__device__ __forceinline__ void mk_consume_gemv(MkRing &rg, const MkGeom &g, const T *xs, float *partial, int *loc_row,
-                                                float *scratch, const MkEpi &e, int ct, int warp, int lane) {
-  constexpr int G = (EPI == EPI_SWIGLU) ? 2 : 1;
-  const int RS = g.RS, WPR = g.WPR, RPW = g.RPW, N = g.N;
-  const int nchunk = g.K / g.KC;
-  const int slots = MK_CW / WPR, slot = warp / WPR, ks = warp % WPR;
-  const int segv = g.KC / 8, nvec = segv / WPR;
-  const uint4 *xsv = reinterpret_cast<const uint4 *>(xs);
-  const bool dyn = mk_is_dynamic(g);
-  int r0 = 0, nrows = 0, nloc = 0;
-  if (dyn) {
-    // A lane's columns are the same for every row of the phase, so its x slice is converted to fp32 ONCE into
-    // registers; per 16-byte weight vector the loop is 1 LDS.128 + 8 converts + 8 FMA (ncu: re-reading and
-    // re-converting x per vector made the loop issue-bound).  Stages arrive with their row in stage_row[].
-    float xr[4][8];
+    const float inv = mk_rsqrt(tot * g.inv_k + a.eps);
+    uint2 *xq = reinterpret_cast<uint2 *>(xs);
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const int v = lane + 32 * i;
-      uint4 u = make_uint4(0u, 0u, 0u, 0u);
-      if (v < nvec) u = xsv[ks * nvec + v];
-      unpack8<T>(u, xr[i]);
-    }
-    const bool v3 = lane + 96 < nvec, v2 = lane + 64 < nvec, v1 = lane + 32 < nvec, v0 = lane < nvec;
-    const uint4 z = make_uint4(0u, 0u, 0u, 0u);
-    while (true) {
-      mbar_wait(&rg.full[rg.s], rg.ph);
-      const int row = rg.stage_row[rg.s];
-      if (row >= 0) {
-        const uint4 *st = reinterpret_cast<const uint4 *>(rg.ring + (size_t)rg.s * MK_STAGE_BYTES) + ks * nvec + lane;
-        for (int r = 0; r < RPW; r++) {
-          const uint4 *rowp = st + (size_t)(slot + r * slots) * segv;
-          const uint4 w0 = v0 ? rowp[0] : z, w1 = v1 ? rowp[32] : z, w2 = v2 ? rowp[64] : z, w3 = v3 ? rowp[96] : z;
-          float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f, wf[8];
-          unpack8<T>(w0, wf);
-          a0 = fmaf(wf[0], xr[0][0], a0); a1 = fmaf(wf[1], xr[0][1], a1); a2 = fmaf(wf[2], xr[0][2], a2); a3 = fmaf(wf[3], xr[0][3], a3);
-          a0 = fmaf(wf[4], xr[0][4], a0); a1 = fmaf(wf[5], xr[0][5], a1); a2 = fmaf(wf[6], xr[0][6], a2); a3 = fmaf(wf[7], xr[0][7], a3);
-          unpack8<T>(w1, wf);
-          a0 = fmaf(wf[0], xr[1][0], a0); a1 = fmaf(wf[1], xr[1][1], a1); a2 = fmaf(wf[2], xr[1][2], a2); a3 = fmaf(wf[3], xr[1][3], a3);
-          a0 = fmaf(wf[4], xr[1][4], a0); a1 = fmaf(wf[5], xr[1][5], a1); a2 = fmaf(wf[6], xr[1][6], a2); a3 = fmaf(wf[7], xr[1][7], a3);
-          unpack8<T>(w2, wf);
-          a0 = fmaf(wf[0], xr[2][0], a0); a1 = fmaf(wf[1], xr[2][1], a1); a2 = fmaf(wf[2], xr[2][2], a2); a3 = fmaf(wf[3], xr[2][3], a3);
-          a0 = fmaf(wf[4], xr[2][4], a0); a1 = fmaf(wf[5], xr[2][5], a1); a2 = fmaf(wf[6], xr[2][6], a2); a3 = fmaf(wf[7], xr[2][7], a3);
-          unpack8<T>(w3, wf);
-          a0 = fmaf(wf[0], xr[3][0], a0); a1 = fmaf(wf[1], xr[3][1], a1); a2 = fmaf(wf[2], xr[3][2], a2); a3 = fmaf(wf[3], xr[3][3], a3);
-          a0 = fmaf(wf[4], xr[3][4], a0); a1 = fmaf(wf[5], xr[3][5], a1); a2 = fmaf(wf[6], xr[3][6], a2); a3 = fmaf(wf[7], xr[3][7], a3);
-          const float v = warp_sum((a0 + a1) + (a2 + a3));
-          if (lane == 0) partial[((size_t)nloc * RS + slot + r * slots) * WPR + ks] = v;  // rows past N: never read
+    for (int i = 0; i < 4; i++)
+      if (ct + i * MK_CT < g.K / 4) xq[ct + i * MK_CT] = mk_normed<T>(xq[ct + i * MK_CT], nw[i], inv);
+#pragma unroll 1
+    for (int q = ct + 4 * MK_CT; q < g.K / 4; q += MK_CT) xq[q] = mk_normed<T>(xq[q], reinterpret_cast<const uint2 *>(norm_w)[q], inv);
+    named_bar_sync(1, MK_CT);
+  }
+  mk_stamp(a, l, ph, 0);
+  // ---- staged rows.  A warp takes two rows of 16, one of 8, or one and the other 8 / RS - 1 warps of its row a part of the columns each: at most
+  // 8 vectors of 16 bytes a lane, 32 lanes side by side.  A lane's columns are the same for every stage: its x stays in registers.
+  const bool pool = g.pool < g.n_groups, two = RSL == 4;
+  const int wl = max(3 - RSL, 0), ks = warp & ((1 << wl) - 1), slot = warp >> wl;
+  const int segv = g.KC / 8, nv = segv >> wl;
+  const int cnt = (nv - lane + 31) >> 5;                  // this lane's vectors of a row
+  const uint4 *xsv = reinterpret_cast<const uint4 *>(xs) + ks * nv + lane;
+  const int at = slot * segv + ks * nv + lane, at4 = two ? at + 8 * segv : at + 128;   // the first four vectors, the other four (of a second row, if two)
+  const uint4 z = make_uint4(0u, 0u, 0u, 0u);
+  float best = -INFINITY;  // (head)
+  int bidx = 0x7fffffff;
+  const int kind = (pool ? 1 : 0) | (nchunk > 1 ? 2 : 0) | (two ? 4 : 0);
+  int base = mk_first(g), left_groups = mk_count(g);
+  bool more = true;
+#pragma unroll 1
+  while (more) {
+    int n_groups = pool ? g.batch : min(g.batch, left_groups);
+    left_groups -= n_groups;
+    more = pool || left_groups > 0;
+    const int n_stages = n_groups * nchunk;
+    uint4 x[8], w[8];
+    auto load_x = [&](const uint4 *xv) {
+#pragma unroll
+      for (int i = 0; i < 8; i++) x[i] = i < cnt ? xv[32 * i] : z;   // (two rows: at most four vectors)
+    };
+    // A stage is read half by half, the halves of the next stage (if it is there) as soon as the registers are free, so that the reads,
+    // the products and the sums over the lanes of neighbouring stages overlap.
+    auto load_a = [&](const uint4 *st) {
+#pragma unroll
+      for (int i = 0; i < 4; i++) w[i] = i < cnt ? st[at + 32 * i] : z;
+    };
+    auto load_b = [&](const uint4 *st) {
+#pragma unroll
+      for (int i = 0; i < 4; i++) w[4 + i] = (two ? i : i + 4) < cnt ? st[at4 + 32 * i] : z;
+    };
+    load_x(xsv);
+    int k = 0;
+    bool ready = false;   // the halves of stage i are already requested
+#pragma unroll 1
+    for (int i = 0; i < n_stages; i++) {
+      int what = kind;  // (opaque: the compiler else writes the loop out once per kind, and the phases no longer fit the instruction cache)
+      asm volatile("" : "+r"(what));
+      if (!ready) {
+        mbar_wait(rg.full(), rg.ph);
+        const uint4 *st = reinterpret_cast<const uint4 *>(rg.data());
+        load_a(st);
+        load_b(st);
+      }
+      if (what & 1) {
+        const int row = rg.row();
+        if (row < 0) {
+          __syncwarp();
+          if (lane == 0) mbar_arrive(rg.empty());
+          rg.advance();
+          n_groups = i;
+          more = false;
+          break;
         }
-        if (ct == 0) loc_row[nloc] = row;
+        if (ct == 0) loc_row[i] = row;
+      }
+      if (what & 2) {  // the columns change from stage to stage
+        load_x(xsv + k * segv);
+        if (++k == nchunk) k = 0;
+      }
+      uint64_t *const done = rg.empty();
+      rg.advance();
+      ready = i + 1 < n_stages && mk_ready(rg.full(), rg.ph);
+      const uint4 *st = reinterpret_cast<const uint4 *>(rg.data());
+      float a0[4] = {0.f, 0.f, 0.f, 0.f}, a1[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int c = 0; c < 4; c++) mk_dot8<T>(a0, w[c], x[c]);
+      if (ready) load_a(st);
+      if (what & 4) {
+#pragma unroll
+        for (int c = 0; c < 4; c++) mk_dot8<T>(a1, w[4 + c], x[c]);
+      } else {
+#pragma unroll
+        for (int c = 0; c < 4; c++) mk_dot8<T>(a1, w[4 + c], x[4 + c]);
       }
       __syncwarp();
-      if (lane == 0) mbar_arrive(&rg.empty[rg.s]);
-      rg.advance();
-      if (row < 0) break;
-      nloc++;
-    }
-  } else {
-    int r1;
-    mk_rows(N, G, r0, r1);
-    nrows = r1 - r0;
-    for (int g0 = 0; g0 < nrows; g0 += RS) {
-      float acc[4][2];
-#pragma unroll
-      for (int r = 0; r < 4; r++) acc[r][0] = acc[r][1] = 0.f;
-      for (int j = 0; j < nchunk; j++) {
-        mbar_wait(&rg.full[rg.s], rg.ph);
-        const uint4 *st = reinterpret_cast<const uint4 *>(rg.ring + (size_t)rg.s * MK_STAGE_BYTES);
-        const uint4 *xc = xsv + (size_t)j * segv + ks * nvec;
-#pragma unroll 2
-        for (int v = lane; v < nvec; v += 32) {
-          float xf[8];
-          unpack8<T>(xc[v], xf);
-#pragma unroll
-          for (int r = 0; r < 4; r++) {
-            if (r < RPW) {
-              float wf[8];
-              unpack8<T>(st[(size_t)(slot + r * slots) * segv + ks * nvec + v], wf);
-#pragma unroll
-              for (int i = 0; i < 8; i++) acc[r][i & 1] = fmaf(wf[i], xf[i], acc[r][i & 1]);
-            }
-          }
-        }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&rg.empty[rg.s]);
-        rg.advance();
+      if (lane == 0) mbar_arrive(done);
+      if (ready) load_b(st);
+      float s0 = (a0[0] + a0[1]) + (a0[2] + a0[3]);
+      const float s1 = (a1[0] + a1[1]) + (a1[2] + a1[3]);
+      float *pt = partial + (((i << RSL) + slot) << wl) + ks;
+      if (what & 4) {  // two rows: half of the lanes for each
+        const bool up = lane & 16;
+        s0 = (up ? s1 : s0) + __shfl_xor_sync(0xffffffffu, up ? s0 : s1, 16);
+      } else {
+        s0 += s1;
+        s0 += __shfl_xor_sync(0xffffffffu, s0, 16);
       }
 #pragma unroll
-      for (int r = 0; r < 4; r++) {
-        if (r < RPW) {
-          const float v = warp_sum(acc[r][0] + acc[r][1]);
-          const int rl = g0 + slot + r * slots;
-          if (lane == 0 && rl < nrows) partial[rl * WPR + ks] = v;
-        }
-      }
+      for (int o = 8; o; o >>= 1) s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+      if ((lane & 15) == 0 && (lane == 0 || (what & 4))) pt[lane ? 8 : 0] = s0;  // (rows past N: never read)
     }
-  }
-  named_bar_sync(1, MK_CT);
-  // local row index li -> global row (dynamic: group list; static: contiguous range)
-  const int n_local = dyn ? nloc * RS : nrows;
-  auto row_of = [&](int li) { return dyn ? loc_row[li / RS] + li % RS : r0 + li; };
-  auto row_sum = [&](int li) {
-    float sum = 0.f;
-    for (int w = 0; w < WPR; w++) sum += partial[(size_t)li * WPR + w];
-    return rnd<T>(sum);
-  };
-  T *out = reinterpret_cast<T *>(e.out);
-  if (EPI == EPI_PLAIN) {
-    const T *bias = reinterpret_cast<const T *>(e.bias);
-    for (int li = ct; li < n_local; li += MK_CT) {
-      const int row = row_of(li);
-      if (row >= N) continue;
-      float v = row_sum(li);
-      if (bias) v = rnd<T>(v + DT<T>::to_f(bias[row]));
-      out[row] = DT<T>::from_f(v);
-    }
-  } else if (EPI == EPI_RESIDUAL) {
-    const T *res = reinterpret_cast<const T *>(e.residual);
-    for (int li = ct; li < n_local; li += MK_CT) {
-      const int row = row_of(li);
-      if (row >= N) continue;
-      const float v = row_sum(li);
-      out[row] = DT<T>::from_f(v + DT<T>::to_f(ldcg_T<T>(res + row)));
-    }
-  } else if (EPI == EPI_SWIGLU) {
-    for (int p = ct; p < n_local / 2; p += MK_CT) {
-      const int row = row_of(2 * p);
-      if (row >= N) continue;
-      const float gte = row_sum(2 * p), up = row_sum(2 * p + 1);
-      const float sl = gate_act<T>(gte, e.act);
-      out[row / 2] = DT<T>::from_f(sl * up);
-    }
-  } else {
-    float best = -INFINITY;
-    int bidx = 0x7fffffff;
-    for (int li = ct; li < n_local; li += MK_CT) {
-      const int row = row_of(li);
-      if (row >= N) continue;
-      const float v = row_sum(li);
-      if (out) out[row] = DT<T>::from_f(v);
-      if (v > best || (v == best && row < bidx)) { best = v; bidx = row; }  // first maximum wins
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, bidx, o);
-      if (ov > best || (ov == best && oi < bidx)) { best = ov; bidx = oi; }
-    }
-    int *scratch_i = reinterpret_cast<int *>(scratch + 32);
-    if (lane == 0) { scratch[warp] = best; scratch_i[warp] = bidx; }
     named_bar_sync(1, MK_CT);
-    if (ct == 0) {
-      for (int w = 1; w < MK_CW; w++)
-        if (scratch[w] > best || (scratch[w] == best && scratch_i[w] < bidx)) { best = scratch[w]; bidx = scratch_i[w]; }
-      e.part_val[blockIdx.x] = best;
-      e.part_idx[blockIdx.x] = bidx;
-      __threadfence();
-      const unsigned ticket = atomicAdd(e.counter, 1u);
-      if (ticket == gridDim.x - 1) {
-        __threadfence();
-        float bv = -INFINITY;
-        int bi = 0x7fffffff;
-        for (unsigned c = 0; c < gridDim.x; c++) {
-          const float v = __ldcg(e.part_val + c);
-          const int i = __ldcg(e.part_idx + c);
-          if (v > bv || (v == bv && i < bi)) { bv = v; bi = i; }
+    const int n_local = n_groups << RSL;
+    auto row_sum = [&](int li) {
+      const float *p = partial + (li * nchunk << wl);
+      float sum = p[0];
+      if (wl > 0) {
+        sum += p[1];
+        if (wl > 1) {
+          sum += p[2] + p[3];
+          if (wl > 2) sum += (p[4] + p[5]) + (p[6] + p[7]);
         }
-        *e.token_out = (uint32_t)bi;
-        if (e.token_ring) e.token_ring[*e.step % e.ring_cap] = (uint32_t)bi;
-        *e.counter = 0;
-        // end-of-step bookkeeping: this is the last CTA of the grid to finish
-        if (e.advance) { *e.d_pos += 1; *e.d_step += 1; }
-        if (e.ring_seq) *e.ring_seq += 1ULL;
-        e.gbar[1] = e.next_start;
+      }
+#pragma unroll 1
+      for (int i = 1 << wl; i < nchunk << wl; i++) sum += p[i];
+      return rnd<T>(sum);
+    };
+#pragma unroll 1
+    for (int li = ct << (ph == 2); li < n_local; li += MK_CT << (ph == 2)) {  // a row, or a gate and an up row
+      const int row = pool ? loc_row[li >> RSL] + (li & ((1 << RSL) - 1)) : (base << RSL) + li;
+      if (row >= g.N) continue;
+      int what = head ? 4 : ph;
+      asm volatile("" : "+r"(what));
+      float v = row_sum(li);
+      if (what == 4) {
+        if (a.logits) reinterpret_cast<T *>(a.logits)[row] = DT<T>::from_f(v);
+        if (v > best || (v == best && row < bidx)) { best = v; bidx = row; }  // first maximum wins
+      } else if (what == 0) {
+        if (L.bqkv) v = rnd<T>(v + DT<T>::to_f(reinterpret_cast<const T *>(L.bqkv)[row]));
+        pk_store<T>(a.pk.qkv + row, DT<T>::from_f(v), tag);
+      } else if (what == 2) {
+        const float up = row_sum(li + 1);
+        pk_store<T>(a.pk.mm + row / 2, DT<T>::from_f(mk_gate_act<T>(v, a.act) * up), tag);
+      } else {  // + residual
+        T q;
+        if (a.keep_x) q = res_s[row];
+        else if (what == 1 && l == 0) q = ldcg_T<T>(mk_x_in<T>(a) + row);
+        else q = pk_value<T>(pk_load((what == 1 ? a.pk.xa : a.pk.xb) + row));  // (gathered by this CTA before)
+        const T o = DT<T>::from_f(v + DT<T>::to_f(q));
+        pk_store<T>((what == 1 ? a.pk.xb : a.pk.xa) + row, o, tag);
+        if (what == 3 && l == a.n_layers - 1 && a.x_out) reinterpret_cast<T *>(a.x_out)[row] = o;
       }
     }
+    base += n_groups;
+    if (more) named_bar_sync(1, MK_CT);  // the batch has been taken
   }
+  if (head) mk_head_end(a, scratch, best, bidx);
+  mk_stamp(a, l, ph, 1);
 }
 
 // Sum G per-lane values over the 16 lanes of a half-warp with a halving butterfly: after log2(G) exchange
@@ -591,15 +740,17 @@ __device__ __forceinline__ float reduce16_heads(float (&s)[G], int lane, int &g_
   return v;
 }
 
-// norm_rope_inplace with the position's cos/sin row already staged in shared memory as fp32 (D values)
+// norm_rope_inplace with the position's cos/sin row already staged in shared memory as fp32 (D values); a lane holds its norm weights
 template <typename T, int HD>
-__device__ __forceinline__ void mk_norm_rope(float *buf, const T *norm_w, float eps, const float *cs, const float *sn, int rot, int lane) {
-  if (norm_w) {
+__device__ __forceinline__ void mk_norm_rope(float *buf, bool norm, const float (&w)[(HD + 31) / 32], float eps, const float *cs, const float *sn, int rot, int lane) {
+  if (norm) {
     float ss = 0.f;
     for (int d = lane; d < HD; d += 32) ss += buf[d] * buf[d];
     ss = warp_sum(ss);
-    const float inv = 1.0f / sqrtf(ss / (float)HD + eps);
-    for (int d = lane; d < HD; d += 32) buf[d] = rnd<T>(buf[d] * inv * DT<T>::to_f(norm_w[d]));
+    const float inv = mk_rsqrt(ss * (1.0f / HD) + eps);
+#pragma unroll
+    for (int i = 0; i < (HD + 31) / 32; i++)
+      if (lane + 32 * i < HD) buf[lane + 32 * i] = rnd<T>(buf[lane + 32 * i] * inv * w[i]);
     __syncwarp();
   }
   const int half = rot / 2;
@@ -615,16 +766,16 @@ __device__ __forceinline__ void mk_norm_rope(float *buf, const T *norm_w, float 
 // Attention phase for this CTA's (kv head, split) item.  Same math as attn_decode_kernel (f32 scores,
 // softmax and PV, one rounding of the result); K/V tiles come from the ring, prefetched by the producer while
 // the qkv GEMV was still running.  G = n_heads / n_kv_heads is a template parameter so that all per-head
-// state lives in registers.
+// state lives in registers.  The heads' packets are polled by the warps that norm and rotate them.  One split: its result is the output.
+// Several: each publishes its columns, maximum and sum as packets, and each merges its share of the columns of all of them, in split order.
 template <typename T, int HD, int G>
-__device__ __forceinline__ void mk_consume_attn(MkRing &rg, const MkArgs &a, const MkLayer &L, int pos, unsigned char *scr,
-                                                const float *rope_cs, int ct, int warp, int lane, unsigned long long *tr) {
+__device__ __forceinline__ void mk_consume_attn(MkRing &rg, const MkArgs &a, const MkRow &L, int pos, unsigned char *scr,
+                                                const float *rope_cs, uint32_t tag32, int &left, unsigned long long *tr) {
+  const int ct = threadIdx.x, warp = ct >> 5, lane = ct & 31;
+  const uint32_t tag = tag32 << 16;
+  MkWait wt{left, a.err};
   auto stamp = [&](int i) {
-    if (tr && ct == 0) {
-      unsigned long long t;
-      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-      tr[i] = t;
-    }
+    if (tr && ct == 0) tr[i] = mk_gtime();
   };
   stamp(0);
   constexpr int LPR = HD / 8;            // lanes per cached row (16 B each); HD in {16,64,128} -> 2, 8, 16
@@ -634,44 +785,41 @@ __device__ __forceinline__ void mk_consume_attn(MkRing &rg, const MkArgs &a, con
   // sliding window (cache.rs:173-205): rows below ws = pos + 1 - window are invisible; indices below are relative to ws
   const int ws = (a.window > 0 && pos + 1 > a.window) ? pos + 1 - a.window : 0;
   pos -= ws;
-  const MkAttnItem it = mk_attn_item<T>(a, pos);
-  float *q_s = reinterpret_cast<float *>(scr);             // [G][HD]
+  const MkAttnItem it = mk_attn_item(a, pos, (int)sizeof(T));
+  float *q_s = reinterpret_cast<float *>(scr);             // [G][HD]; then the parts of a merge
   float *sc = q_s + ATTN_MAX_G * 256;                      // [ATTN_TILE][G]  (position-major: one vector per position)
   float *knew = sc + ATTN_MAX_G * ATTN_TILE;               // [2][HD] appended k / v row
   __shared__ float m_run[ATTN_MAX_G], l_run[ATTN_MAX_G], fac[ATTN_MAX_G];
   __shared__ float wgt[ATTN_MAX_G][ATTN_MAX_SPLIT];
-  __shared__ int is_last;
   if (!it.active) return;  // CTA-uniform; inactive CTAs issue no stages either
 
-  const T *qkv = reinterpret_cast<const T *>(a.qkv);
   const float *cosr = rope_cs, *sinr = rope_cs + 128;  // this step's cos/sin row, staged once per launch
   T *kc = reinterpret_cast<T *>(L.kc) + ((size_t)it.kvh * a.cap + ws) * HD;
   T *vc = reinterpret_cast<T *>(L.vc) + ((size_t)it.kvh * a.cap + ws) * HD;
   const int kvh = it.kvh, split = it.split, s0 = it.s0, s1 = it.s1, TILE = it.tile;
   const bool owner = (pos >= s0 && pos < s1);
 
-  // q for the G heads of this kv head (qkv was written by other SMs: ld.global.cg)
-  for (int g = warp; g < G; g += NW) {
-    const T *src = qkv + (size_t)(kvh * G + g) * HD;
-    float *dst = q_s + g * HD;
-    for (int d = lane; d < HD; d += 32) dst[d] = DT<T>::to_f(ldcg_T<T>(src + d));
+  // q of the G heads of this kv head, a warp each; in the split that holds the position the new key and value too
+#pragma unroll 1
+  for (int h = warp; h < (owner ? G + 2 : G); h += NW) {
+    const bool is_q = h < G, is_k = h == G;
+    float nw[(HD + 31) / 32];
+    const T *norm_w = reinterpret_cast<const T *>(is_q ? L.qn : is_k ? L.kn : nullptr);
+#pragma unroll
+    for (int i = 0; i < (HD + 31) / 32; i++) nw[i] = norm_w && lane + 32 * i < HD ? DT<T>::to_f(norm_w[lane + 32 * i]) : 0.f;
+    const int head = is_q ? kvh * G + h : is_k ? a.n_heads + kvh : a.n_heads + a.n_kv + kvh;
+    float *dst = is_q ? q_s + h * HD : is_k ? knew : knew + HD;
+    if (lane < HD / 4) {
+      const uint32_t *src = a.pk.qkv + (size_t)head * HD + lane * 4;
+      uint4 u = pk_load4(src);
+      while (pk_stale4(u, tag) && wt.again()) u = pk_load4(src);
+      *reinterpret_cast<float4 *>(dst + lane * 4) = pk_floats4<T>(u);
+    }
     __syncwarp();
-    mk_norm_rope<T, HD>(dst, reinterpret_cast<const T *>(L.qn), a.eps, cosr, sinr, a.rot, lane);
-  }
-  if (owner) {
-    if (warp == NW - 1) {
-      const T *src = qkv + (size_t)(a.n_heads + kvh) * HD;
-      for (int d = lane; d < HD; d += 32) knew[d] = DT<T>::to_f(ldcg_T<T>(src + d));
-      __syncwarp();
-      mk_norm_rope<T, HD>(knew, reinterpret_cast<const T *>(L.kn), a.eps, cosr, sinr, a.rot, lane);
-      for (int d = lane; d < HD; d += 32) kc[(size_t)pos * HD + d] = DT<T>::from_f(knew[d]);
-    } else if (warp == NW - 2) {
-      const T *vsrc = qkv + (size_t)(a.n_heads + a.n_kv + kvh) * HD;
-      for (int d = lane; d < HD; d += 32) {
-        const T vv = ldcg_T<T>(vsrc + d);
-        vc[(size_t)pos * HD + d] = vv;
-        knew[HD + d] = DT<T>::to_f(vv);
-      }
+    if (is_q || is_k) mk_norm_rope<T, HD>(dst, norm_w != nullptr, nw, a.eps, cosr, sinr, a.rot, lane);
+    if (!is_q) {
+      T *row = is_k ? kc : vc;
+      for (int d = lane; d < HD; d += 32) row[(size_t)pos * HD + d] = DT<T>::from_f(dst[d]);
     }
   }
   if (ct < ATTN_MAX_G) { m_run[ct] = -INFINITY; l_run[ct] = 0.f; }
@@ -679,11 +827,12 @@ __device__ __forceinline__ void mk_consume_attn(MkRing &rg, const MkArgs &a, con
   stamp(1);
 
   const int grp = lane / LPR, gl = lane % LPR;  // row group within the warp / lane within the row
-  float qreg[G][8];
+  uint4 qreg[G];  // (D values: exact)
 #pragma unroll
-  for (int g = 0; g < G; g++)
-#pragma unroll
-    for (int i = 0; i < 8; i++) qreg[g][i] = q_s[g * HD + gl * 8 + i];
+  for (int g = 0; g < G; g++) {
+    const float *q = q_s + g * HD + gl * 8;
+    qreg[g] = make_uint4(pack2x<T>(q[0], q[1]), pack2x<T>(q[2], q[3]), pack2x<T>(q[4], q[5]), pack2x<T>(q[6], q[7]));
+  }
   float acc[G][8];  // PV accumulator: dims gl*8..+8 of every head, over this half-warp's positions
 #pragma unroll
   for (int g = 0; g < G; g++)
@@ -691,23 +840,21 @@ __device__ __forceinline__ void mk_consume_attn(MkRing &rg, const MkArgs &a, con
     for (int i = 0; i < 8; i++) acc[g][i] = 0.f;
 
   T *Ks = nullptr, *Vs = nullptr;
-  int sk = 0, sv = 0;
+  uint64_t *ek = nullptr, *ev = nullptr;
   for (int t0 = s0; t0 < s1; t0 += TILE) {
     const int tn = min(TILE, s1 - t0);
     if (t0 > s0) {  // release the previous tile's stages (the last tile's are kept for the final reduction)
       __syncwarp();
-      if (lane == 0) { mbar_arrive(&rg.empty[sk]); mbar_arrive(&rg.empty[sv]); }
+      if (lane == 0) { mbar_arrive(ek); mbar_arrive(ev); }
     }
-    sk = rg.s;
-    const uint32_t phk = rg.ph;
+    ek = rg.empty();
+    Ks = reinterpret_cast<T *>(rg.data());
+    mbar_wait(rg.full(), rg.ph);
     rg.advance();
-    sv = rg.s;
-    const uint32_t phv = rg.ph;
+    ev = rg.empty();
+    Vs = reinterpret_cast<T *>(rg.data());
+    mbar_wait(rg.full(), rg.ph);
     rg.advance();
-    Ks = reinterpret_cast<T *>(rg.ring + (size_t)sk * MK_STAGE_BYTES);
-    Vs = reinterpret_cast<T *>(rg.ring + (size_t)sv * MK_STAGE_BYTES);
-    mbar_wait(&rg.full[sk], phk);
-    mbar_wait(&rg.full[sv], phv);
     stamp(2);
     if (owner && pos >= t0 && pos < t0 + tn) {  // drop the appended row into its slot of the staged tiles
       const int slot = pos - t0;
@@ -721,17 +868,14 @@ __device__ __forceinline__ void mk_consume_attn(MkRing &rg, const MkArgs &a, con
     for (int pb = warp * RPWI; pb < tn; pb += NW * RPWI) {  // warp-uniform trip count (shuffles below)
       const int p = pb + grp;
       const bool valid = p < tn;
-      float kf[8];
       uint4 kraw = make_uint4(0u, 0u, 0u, 0u);
       if (valid) kraw = *reinterpret_cast<const uint4 *>(Ks + (size_t)p * HD + gl * 8);
-      unpack8<T>(kraw, kf);
       float sg[G];
 #pragma unroll
       for (int g = 0; g < G; g++) {
-        float sacc = 0.f;
-#pragma unroll
-        for (int i = 0; i < 8; i++) sacc = fmaf(qreg[g][i], kf[i], sacc);
-        sg[g] = sacc;
+        float s4[4] = {0.f, 0.f, 0.f, 0.f};
+        mk_dot8<T>(s4, kraw, qreg[g]);
+        sg[g] = (s4[0] + s4[1]) + (s4[2] + s4[3]);
       }
       if (LPR == 16) {
         int gh;
@@ -793,139 +937,114 @@ __device__ __forceinline__ void mk_consume_attn(MkRing &rg, const MkArgs &a, con
     stamp(5);
   }
 
-  // ---- combine the row groups: lanes of a warp first (shuffles), then the 16 warps through the (dead)
-  //      K/V stage buffers of the last tile -----------------------------------------------------------
+  // ---- combine the row groups: lanes of a warp first (shuffles), then the warps through the (dead)
+  //      K stage of the last tile (an active split has at least one position, so there is one) -------------------------------
 #pragma unroll
   for (int o = LPR; o < 32; o <<= 1)
 #pragma unroll
     for (int g = 0; g < G; g++)
 #pragma unroll
       for (int i = 0; i < 8; i++) acc[g][i] += __shfl_xor_sync(0xffffffffu, acc[g][i], o);
-  const bool have_tile = (s1 > s0);
-  float *red0 = reinterpret_cast<float *>(Ks), *red1 = reinterpret_cast<float *>(Vs);  // 8 warps each: [8][G][HD] <= 32 KB
-  if (have_tile) {
-    if (lane < LPR) {
-      float *dst = (warp < 8 ? red0 : red1) + (size_t)(warp & 7) * G * HD;
+  float *red = reinterpret_cast<float *>(Ks);  // [warp][G][HD] <= 32 KB
+  static_assert(NW * ATTN_MAX_G * 128 * 4 <= MK_STAGE_BYTES, "the warps' sums");
+  if (lane < LPR) {
+    float *dst = red + (size_t)warp * G * HD;
 #pragma unroll
-      for (int g = 0; g < G; g++)
+    for (int g = 0; g < G; g++)
 #pragma unroll
-        for (int i = 0; i < 8; i++) dst[g * HD + lane * 8 + i] = acc[g][i];
-    }
-    named_bar_sync(1, MK_CT);
-    for (int i = ct; i < G * HD; i += MK_CT) {
-      float sum = 0.f;
-#pragma unroll
-      for (int w = 0; w < 8; w++) sum += red0[(size_t)w * G * HD + i];
-#pragma unroll
-      for (int w = 0; w < 8; w++) sum += red1[(size_t)w * G * HD + i];
-      const int g = i / HD, d = i % HD;
-      a.ws_acc[((size_t)(kvh * G + g) * a.nsplit + split) * HD + d] = sum;
-    }
-    __syncwarp();
-    named_bar_sync(1, MK_CT);
-    if (lane == 0) { mbar_arrive(&rg.empty[sk]); mbar_arrive(&rg.empty[sv]); }
-  } else {
-    for (int i = ct; i < G * HD; i += MK_CT) {
-      const int g = i / HD, d = i % HD;
-      a.ws_acc[((size_t)(kvh * G + g) * a.nsplit + split) * HD + d] = 0.f;
-    }
-  }
-  if (ct < G) {
-    a.ws_ml[((size_t)(kvh * G + ct) * a.nsplit + split) * 2 + 0] = m_run[ct];
-    a.ws_ml[((size_t)(kvh * G + ct) * a.nsplit + split) * 2 + 1] = l_run[ct];
-  }
-  stamp(6);
-  named_bar_sync(1, MK_CT);
-  if (ct == 0) {
-    // acq_rel at gpu scope: releases the partials every thread of this CTA wrote before the bar.sync (cumulative)
-    // and, for the last arriver, acquires the other splits' partials
-    unsigned ticket;
-    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(ticket) : "l"(&a.attn_counters[kvh]) : "memory");
-    is_last = (ticket == (unsigned)a.nsplit - 1);
+      for (int i = 0; i < 8; i++) dst[g * HD + lane * 8 + i] = acc[g][i];
   }
   named_bar_sync(1, MK_CT);
-  stamp(7);
-  if (!is_last) return;
-  for (int g = warp; g < G; g += NW) {
-    const int h = kvh * G + g;
-    float m = -INFINITY, l = 0.f;
-    if (lane < a.nsplit) {
-      m = __ldcg(a.ws_ml + ((size_t)h * a.nsplit + lane) * 2);
-      l = __ldcg(a.ws_ml + ((size_t)h * a.nsplit + lane) * 2 + 1);
-    }
-    const float M = warp_max(m);
-    const float w = (m == -INFINITY) ? 0.f : expf(m - M);
-    const float Lsum = warp_sum(w * l);
-    wgt[g][lane] = w / Lsum;
-  }
-  named_bar_sync(1, MK_CT);
-  T *y = reinterpret_cast<T *>(a.y);
+  const int ns = it.n_split;
+  uint64_t *pacc = a.pk.acc + (size_t)kvh * G * HD * a.nsplit, *pml = a.pk.ml + (size_t)kvh * G * a.nsplit * 2;  // [column][split], [head][split][2]
   for (int i = ct; i < G * HD; i += MK_CT) {
-    const int g = i / HD, d = i % HD, h = kvh * G + g;
-    const float *src = a.ws_acc + (size_t)h * a.nsplit * HD + d;
-    float o = 0.f;
-#pragma unroll 8
-    for (int s2 = 0; s2 < a.nsplit; s2++) o = fmaf(wgt[g][s2], __ldcg(src + (size_t)s2 * HD), o);
-    y[(size_t)h * HD + d] = DT<T>::from_f(o);
+    float sum = 0.f;
+#pragma unroll
+    for (int w = 0; w < NW; w++) sum += red[(size_t)w * G * HD + i];
+    if (ns == 1) pk_store<T>(a.pk.y + (size_t)kvh * G * HD + i, DT<T>::from_f(sum * mk_rcp(l_run[i / HD])), tag);
+    else pk_store64(pacc + (size_t)i * ns + split, sum, tag32);
   }
-  if (ct == 0) a.attn_counters[kvh] = 0;
+  if (ns > 1 && ct < G) {
+    pk_store64(pml + ((size_t)ct * ns + split) * 2, m_run[ct], tag32);
+    pk_store64(pml + ((size_t)ct * ns + split) * 2 + 1, l_run[ct], tag32);
+  }
+  __syncwarp();
+  named_bar_sync(1, MK_CT);
+  if (lane == 0) { mbar_arrive(ek); mbar_arrive(ev); }
+  stamp(6);
+  if (ns > 1) {
+    // ---- merge: this split's share of the columns; (column, split) pairs are contiguous, a thread polls one or a few of them
+    const int c0 = G * HD * split / ns, nc = G * HD * (split + 1) / ns - c0, np = nc * ns;
+    for (int i = ct; i < np; i += MK_CT) q_s[i] = pk_poll64(pacc + (size_t)c0 * ns + i, tag32, wt);
+    for (int g = warp; g < G; g += NW) {
+      float m = -INFINITY, l = 0.f;
+      if (lane < ns) {
+        m = pk_poll64(pml + ((size_t)g * ns + lane) * 2, tag32, wt);
+        l = pk_poll64(pml + ((size_t)g * ns + lane) * 2 + 1, tag32, wt);
+      }
+      const float M = warp_max(m);
+      const float w = (m == -INFINITY) ? 0.f : expf(m - M);
+      const float Lsum = warp_sum(w * l);
+      wgt[g][lane] = w * mk_rcp(Lsum);
+    }
+    named_bar_sync(1, MK_CT);
+    for (int i = ct; i < nc; i += MK_CT) {
+      const int g = (c0 + i) / HD;
+      float o = 0.f;
+      for (int s2 = 0; s2 < ns; s2++) o = fmaf(wgt[g][s2], q_s[i * ns + s2], o);
+      pk_store<T>(a.pk.y + (size_t)kvh * G * HD + c0 + i, DT<T>::from_f(o), tag);
+    }
+  }
+  left = wt.left;
+  stamp(7);
 }
 
 // ---------------------------------------------------------------------------------------- the kernel
 template <typename T, int HD, int G>
-__global__ void __launch_bounds__(MK_THREADS, 1) decode_mega_kernel(const MkArgs a) {
+__global__ void __launch_bounds__(MK_THREADS, 1) decode_mega_kernel(const __grid_constant__ MkArgs a) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   constexpr int es = sizeof(T);
-  unsigned char *ring = smem_raw;
-  T *xs = reinterpret_cast<T *>(ring + (size_t)a.n_stages * MK_STAGE_BYTES);
-  size_t off = (size_t)a.n_stages * MK_STAGE_BYTES + mk_xs_bytes(a.max_k, es);
-  off = (off + 15) & ~(size_t)15;
-  float *partial = reinterpret_cast<float *>(smem_raw + off);
-  off += (size_t)a.partial_floats * 4;  // sized by the host: max rows x slices over all GEMV types
-  int *loc_row = reinterpret_cast<int *>(smem_raw + off);
-  off += (size_t)a.max_groups * 4;
-  float *scratch = reinterpret_cast<float *>(smem_raw + off);
-  off += 128 * 4;
-  off = (off + 7) & ~(size_t)7;
-  uint64_t *full = reinterpret_cast<uint64_t *>(smem_raw + off);
-  uint64_t *empty = full + MK_MAX_STAGES;
-  int *stage_row = reinterpret_cast<int *>(empty + MK_MAX_STAGES);
-
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < a.n_stages; s++) {
-      mbar_init(&full[s], 1);
-      mbar_init(&empty[s], MK_CW);
+      mbar_init(reinterpret_cast<uint64_t *>(smem_raw) + s, 1);
+      mbar_init(reinterpret_cast<uint64_t *>(smem_raw + MK_OFF_EMPTY) + s, MK_CW);
     }
     mbar_fence_init();
   }
   __syncthreads();
-  const int pos = *a.d_pos;
-  MkRing rg{ring, full, empty, stage_row, a.n_stages, 0, 0u};
+  const int pos = a.n_layers ? *a.d_pos : 0;
+  MkRing rg{smem_raw, a.n_stages, 0, 0u};
 
   if (warp == MK_CW) {
     // ================= producer: stream weights and K/V tiles through the whole phase list ==========
     if (lane == 0) {
       const uint64_t pol_w = policy_evict_first(), pol_kv = policy_evict_last();
-      MkPrefetch pf{&a, 0, 0, 0, (int)sizeof(T)};
-      if (a.l2_prefetch == 1) for (int i = 0; i < MK_PF_AHEAD; i++) pf.step();
-      auto produce = [&](const MkGeom &g, const void *W, int gran, int phase) {
-        if (mk_is_dynamic(g)) mk_produce_gemv_dyn<T>(rg, g, W, a.tickets + phase, a.max_groups, pol_w, pf);
-        else mk_produce_gemv<T>(rg, g, W, gran, pol_w);
-      };
-      for (int l = 0; l < a.n_layers; l++) {
-        const MkLayer L = a.layers[l];
-        produce(a.g_qkv, L.wqkv, 1, 4 * l + 0);
-        mk_produce_attn<T>(rg, a, L, pos, pol_kv);
-        if (a.l2_prefetch == 2) {
-          mk_prefetch_static(a.g_o, L.wo, (int)sizeof(T), 0, 1 << 20);
-          mk_prefetch_static(a.g_gu, L.wgu, (int)sizeof(T), 0, 10);
+#pragma unroll 1
+      for (int l = 0; l <= a.n_layers; l++) {
+        if (l == a.n_layers && !a.has_head) break;
+        const MkLayer &L = a.layers[l];  // (not read for the head)
+        if (l < a.n_layers) {  // norm weights: one cache line each, into L2 before a consumer asks
+          const int b = blockIdx.x * 128;
+          if (b < a.hidden * es) {
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char *>(L.ln1) + b));
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char *>(L.ln2) + b));
+          }
+          if (L.qn && b < HD * es) {
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char *>(L.qn) + b));
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char *>(L.kn) + b));
+          }
         }
-        produce(a.g_o, L.wo, 1, 4 * l + 1);
-        produce(a.g_gu, L.wgu, 2, 4 * l + 2);
-        produce(a.g_down, L.wd, 1, 4 * l + 3);
+#pragma unroll 1
+        for (int ph = 0; ph < 4; ph++) {
+          const bool head = l == a.n_layers;
+          const MkGeom &g = a.g[head ? 4 : ph];
+          const void *W = head ? a.lm_head : ph == 0 ? L.wqkv : ph == 1 ? L.wo : ph == 2 ? L.wgu : L.wd;
+          mk_produce_gemv<T>(rg, g, W, a.tickets + 4 * l + ph, pol_w);
+          if (head) break;
+          if (ph == 0) mk_produce_attn<T>(rg, a, L, pos, pol_kv);
+        }
       }
-      if (a.has_head) produce(a.g_head, a.lm_head, 1, 4 * a.n_layers);
     }
     return;
   }
@@ -934,31 +1053,24 @@ __global__ void __launch_bounds__(MK_THREADS, 1) decode_mega_kernel(const MkArgs
   const int ct = threadIdx.x;
   __shared__ float rope_cs[256];  // cos (first 128) and sin (last 128) row of this step's position, as fp32
   {
-    const int half = a.rot / 2;
+    const int half = a.n_layers ? a.rot / 2 : 0;
     const T *cr = reinterpret_cast<const T *>(a.cos_t) + (size_t)pos * half, *sr = reinterpret_cast<const T *>(a.sin_t) + (size_t)pos * half;
     if (ct < half) rope_cs[ct] = DT<T>::to_f(cr[ct]);
     else if (ct >= 128 && ct - 128 < half) rope_cs[ct] = DT<T>::to_f(sr[ct - 128]);
-    // visibility: the first named barrier of the first phase orders these writes before any use
-  }
-  // gbar[0] is a monotonic arrival counter; gbar[1] holds its value at the start of this launch (written
-  // by the previous launch's last thread), so barrier k of this launch completes at start + k*grid.
-  const unsigned long long start = *reinterpret_cast<volatile unsigned long long *>(a.gbar + 1);
-  unsigned nbar = 0;
-  int ntrace = 0;
-  auto stamp = [&]() {
-    if (a.trace && blockIdx.x == 0 && ct == 0) {
-      unsigned long long t;
-      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-      a.trace[ntrace++] = t;
+    MkRow *rows = reinterpret_cast<MkRow *>(smem_raw + a.off_rows);
+    for (int l = ct; l < a.n_layers; l += MK_CT) {
+      const MkLayer &L = a.layers[l];
+      rows[l] = MkRow{L.ln1, L.ln2, L.bqkv, L.qn, L.kn, L.kc, L.vc};
     }
-  };
-  auto gsync = [&]() {
-    nbar++;
-    stamp();
-    mk_grid_sync(a.gbar, start + (unsigned long long)nbar * gridDim.x, ct);
-    stamp();
-  };
-  stamp();
+    // gbar[0] is a monotonic arrival counter; gbar[1] holds its value at the start of this launch (written
+    // by the previous launch's last thread), so barrier k of this launch completes at start + k*grid.
+    if (ct == 0) reinterpret_cast<unsigned long long *>(smem_raw + MK_OFF_SCRATCH)[MK_START] = *reinterpret_cast<volatile unsigned long long *>(a.gbar + 1);
+    named_bar_sync(1, MK_CT);
+  }
+  // the tag of layer l's packets is first + l; a buffer is written in every layer, so what is stale in it carries the tag in front
+  const uint32_t first = (uint32_t)*reinterpret_cast<volatile unsigned long long *>(a.gbar + 2) + 1u;
+  int left = MK_POLLS;
+  if (a.trace && blockIdx.x == 0 && ct == 0) a.trace[0] = mk_gtime();
   unsigned long long *const st_rec = (a.step_trace && blockIdx.x == 0 && ct == 0)
       ? a.step_trace + ((size_t)((unsigned)*a.d_step % MK_STEP_RING) * 2 + a.trace_tag) * 4 : nullptr;
   if (st_rec) st_rec[0] = mk_gtime();
@@ -973,78 +1085,23 @@ __global__ void __launch_bounds__(MK_THREADS, 1) decode_mega_kernel(const MkArgs
     named_bar_sync(1, MK_CT);
   }
   if (st_rec) st_rec[1] = mk_gtime();
-  const T *cur = reinterpret_cast<const T *>(a.x_in);
-  if (cur == nullptr) {  // master: the block input is the embedding row of the current token (text_model.rs:271)
-    uint32_t tok = *a.d_token;
-    if (tok >= (uint32_t)a.vocab) tok = 0;  // memory safety only: host entry points reject out-of-range ids (EINVAL); in-kernel argmax ids are < vocab
-    cur = reinterpret_cast<const T *>(a.embed) + (size_t)tok * a.hidden;
-  }
-  MkEpi e{};
-  for (int l = 0; l < a.n_layers; l++) {
-    const MkLayer L = a.layers[l];
-    T *dst = reinterpret_cast<T *>((l == a.n_layers - 1) ? a.x_out : a.xa);
-    // rms_1 + qkv (+bias)
-    mk_stage_x<T>(xs, cur, L.ln1, a.hidden, a.eps, scratch, ct, warp, lane);
-    e = MkEpi{};
-    e.bias = L.bqkv;
-    e.out = a.qkv;
-    mk_consume_gemv<T, EPI_PLAIN>(rg, a.g_qkv, xs, partial, loc_row, scratch, e, ct, warp, lane);
-    gsync();
-    // qk-norm, RoPE, KV append, attention
-    mk_consume_attn<T, HD, G>(rg, a, L, pos, reinterpret_cast<unsigned char *>(xs), rope_cs, ct, warp, lane,
-                           (a.trace && blockIdx.x == 0 && l == 1) ? a.trace + 2048 : nullptr);
-    gsync();
-    // o_proj + residual
-    mk_stage_x<T>(xs, a.y, nullptr, a.n_heads * a.hd, a.eps, scratch, ct, warp, lane);
-    e = MkEpi{};
-    e.residual = cur;
-    e.out = a.xb;
-    mk_consume_gemv<T, EPI_RESIDUAL>(rg, a.g_o, xs, partial, loc_row, scratch, e, ct, warp, lane);
-    gsync();
-    // rms_2 + gate_up + silu*mul
-    mk_stage_x<T>(xs, a.xb, L.ln2, a.hidden, a.eps, scratch, ct, warp, lane);
-    e = MkEpi{};
-    e.out = a.mm;
-    e.act = a.act;
-    mk_consume_gemv<T, EPI_SWIGLU>(rg, a.g_gu, xs, partial, loc_row, scratch, e, ct, warp, lane);
-    if (a.trace && l == 1 && ct == 0) {
-      unsigned long long t;
-      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-      a.trace[2304 + blockIdx.x] = t;
+  // One loop over the phases and one body for the products: as straight-line code of five products the layer's instructions were fetched anew in
+  // every phase.
+#pragma unroll 1
+  for (int l = 0; l <= a.n_layers; l++) {
+    if (l == a.n_layers && !a.has_head) break;
+    const uint32_t tag32 = first + (uint32_t)l;
+#pragma unroll 1
+    for (int ph = 0; ph < 4; ph++) {
+      mk_gemv_phase<T>(rg, a, smem_raw, l, ph, tag32 << 16, left);
+      if (l == a.n_layers) break;
+      if (ph == 0) {  // qk-norm, RoPE, KV append, attention
+        mk_stamp(a, l, 0, 2);
+        mk_consume_attn<T, HD, G>(rg, a, reinterpret_cast<const MkRow *>(smem_raw + a.off_rows)[l], pos, smem_raw + a.off_x, rope_cs, tag32, left,
+                                  a.trace && blockIdx.x == 0 && l == 1 ? a.trace + 2048 : nullptr);
+        mk_stamp(a, l, 0, 3);
+      }
     }
-    gsync();
-    if (a.trace && l == 1 && ct == 0) {
-      unsigned long long t;
-      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-      a.trace[2560 + blockIdx.x] = t;
-    }
-    // down + residual
-    mk_stage_x<T>(xs, a.mm, nullptr, a.inter, a.eps, scratch, ct, warp, lane);
-    e = MkEpi{};
-    e.residual = a.xb;
-    e.out = dst;
-    mk_consume_gemv<T, EPI_RESIDUAL>(rg, a.g_down, xs, partial, loc_row, scratch, e, ct, warp, lane);
-    if (l < a.n_layers - 1 || a.has_head) gsync();
-    cur = dst;
-  }
-  if (a.has_head) {
-    mk_stage_x<T>(xs, cur, a.ln_f, a.hidden, a.eps, scratch, ct, warp, lane);
-    e = MkEpi{};
-    e.out = a.logits;
-    e.part_val = a.part_val;
-    e.part_idx = a.part_idx;
-    e.counter = a.argmax_counter;
-    e.token_out = a.token_out;
-    e.token_ring = a.token_ring;
-    e.step = a.d_step;
-    e.ring_cap = a.ring_cap;
-    e.advance = a.advance;
-    e.d_pos = a.d_pos;
-    e.d_step = a.d_step;
-    e.gbar = a.gbar;
-    e.next_start = start + (unsigned long long)nbar * gridDim.x;
-    e.ring_seq = a.inbox_ctr ? a.ring_seq : nullptr;
-    mk_consume_gemv<T, EPI_ARGMAX>(rg, a.g_head, xs, partial, loc_row, scratch, e, ct, warp, lane);
   }
   if (a.peer_ctr && !a.has_head) {  // our rows of x_out are in the next shard's inbox: release them, one arrival per CTA
     named_bar_sync(1, MK_CT);
@@ -1054,13 +1111,9 @@ __global__ void __launch_bounds__(MK_THREADS, 1) decode_mega_kernel(const MkArgs
     }
   }
   if (st_rec) st_rec[2] = mk_gtime();
-  // bookkeeping without a head: CTA 0 only gets here after passing barriers that every CTA arrived at,
-  // and every CTA read *d_pos, *ring_seq and the barrier start value before its first barrier.
-  if (!a.has_head && blockIdx.x == 0 && ct == 0) {
-    if (a.advance) { *a.d_pos += 1; *a.d_step += 1; }
-    if (a.inbox_ctr) *a.ring_seq += 1ULL;
-    a.gbar[1] = start + (unsigned long long)nbar * gridDim.x;
-  }
+  // bookkeeping without a head: CTA 0 has gathered the last product's input, so every CTA has published something in this launch (mk_every_cta,
+  // or all have met), and every CTA read *d_pos, *ring_seq, the barrier start value and the tag before it did.
+  if (!a.has_head && blockIdx.x == 0 && ct == 0) mk_end_of_step(a, reinterpret_cast<const float *>(smem_raw + MK_OFF_SCRATCH));
 }
 
 }  // namespace cake
