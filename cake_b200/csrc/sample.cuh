@@ -169,10 +169,11 @@ template <typename T> __device__ __forceinline__ float sample_unkey(uint32_t k) 
   return DT<T>::to_f(*reinterpret_cast<const T *>(&h));
 }
 // The largest logit at which the entries that are at least as large still reach `want`, in number (COUNT) or in probability: with tau its
-// probability, reach(P >= tau) >= want > reach(P > tau), as probabilities rise with logits.  Seven thresholds a pass.
+// probability, reach(P >= tau) >= want > reach(P > tau), as probabilities rise with logits.  Seven thresholds a pass.  from, to: logits between which it
+// lies (65536 patterns are six passes; the few hundred between the largest logit and where a nucleus can end are three).
 template <typename T, bool COUNT>
-__device__ __forceinline__ float sample_threshold(SampleCluster &cl, const T *L, const float *P, int i0, int i1, float want) {
-  uint32_t lo = sample_key<T>(-INFINITY), hi = sample_key<T>(INFINITY) + 1u;
+__device__ __forceinline__ float sample_threshold(SampleCluster &cl, const T *L, const float *P, int i0, int i1, float want, float from, float to) {
+  uint32_t lo = sample_key<T>(from), hi = sample_key<T>(to) + 1u;
   while (hi - lo > 1u) {
     const uint32_t step = max(1u, (hi - lo) / 8u);
     float m[7], th[7];
@@ -182,7 +183,9 @@ __device__ __forceinline__ float sample_threshold(SampleCluster &cl, const T *L,
       th[t] = sample_unkey<T>(min(hi - 1u, lo + (uint32_t)(t + 1) * step));
     }
     for (int i = i0; i < i1; i++) {
-      const float x = DT<T>::to_f(L[i]), v = COUNT ? 1.f : P[i];
+      const float x = DT<T>::to_f(L[i]);
+      if (!(x >= th[0])) continue;   // (most entries are below the lowest threshold)
+      const float v = COUNT ? 1.f : P[i];
 #pragma unroll
       for (int t = 0; t < 7; t++) m[t] += x >= th[t] ? v : 0.f;
     }
@@ -248,16 +251,33 @@ sample_kernel(const T *__restrict__ logits, int V, SampleArgs s, float *P_global
   float *P = in_smem ? sample_smem_p : P_global + base;
   const T *L = lg;
   const float inv_t = (float)(1.0 / (double)s.temperature);
-  float mx = -INFINITY;
+  float top = -INFINITY;   // the largest logit (times 1/T rises with it)
   T *keep = reinterpret_cast<T *>(sample_smem_p + (size_t)per * SAMPLE_THREADS);
+  if (in_smem && ((uintptr_t)lg & 15) == 0) {   // 16 bytes a load: one or two round trips to L2 for a thread's entries
+#pragma unroll 3
+    for (int i = tid * 8; i + 8 <= n; i += SAMPLE_THREADS * 8) {
+      const uint4 v = *reinterpret_cast<const uint4 *>(lg + i);
+      *reinterpret_cast<uint4 *>(keep + i) = v;
+      float f[8];
+      unpack8<T>(v, f);
+#pragma unroll
+      for (int e = 0; e < 8; e++) top = fmaxf(top, f[e]);
+    }
+    for (int e = (n & ~7) + tid; e < n; e += SAMPLE_THREADS) {
+      keep[e] = lg[e];
+      top = fmaxf(top, DT<T>::to_f(lg[e]));
+    }
+  } else {
 #pragma unroll 4
-  for (int i = tid; i < n; i += SAMPLE_THREADS) {
-    const T x = lg[i];
-    if (in_smem) keep[i] = x;
-    mx = fmaxf(mx, DT<T>::to_f(x) * inv_t);
+    for (int i = tid; i < n; i += SAMPLE_THREADS) {
+      const T x = lg[i];
+      if (in_smem) keep[i] = x;
+      top = fmaxf(top, DT<T>::to_f(x));
+    }
   }
   if (in_smem) L = keep;
-  mx = cl.max1(mx);
+  top = cl.max1(top);   // (its barriers order the copies, of other entries than a thread reads below)
+  const float mx = __fmul_rn(top, inv_t);
   auto weight = [&](T x) { return expf(__fsub_rn(__fmul_rn(DT<T>::to_f(x), inv_t), mx)); };  // (no contraction: a threshold's own has the same bits)
   float sum = 0.f;
   for (int i = tid; i < n; i += SAMPLE_THREADS) {
@@ -280,7 +300,11 @@ sample_kernel(const T *__restrict__ logits, int V, SampleArgs s, float *P_global
     float eq_before = 0.f;
     int need = 0x7fffffff;
     if (want_p) {
-      tau = __float_as_uint(weight(DT<T>::from_f(sample_threshold<T, false>(cl, L, P, i0, i1, s.top_p))) / sum);
+      // Entries more than d below the largest one have less than V e^(-d / T) / sum of the probability together, which is at most half of 1 - p (sum >= 1):
+      // the nucleus ends above them.  A p within 1e-3 of 1, where the roundings of the sums come near 1 - p, and logits that are not finite search all.
+      const float d = logf(2.f * (float)V / (1.f - s.top_p)) * s.temperature;
+      const bool near = s.top_p < 0.999f && top - d > -INFINITY && top < INFINITY;
+      tau = __float_as_uint(weight(DT<T>::from_f(sample_threshold<T, false>(cl, L, P, i0, i1, s.top_p, near ? top - d : -INFINITY, near ? top : INFINITY))) / sum);
       float m[1] = {0.f}, eq = 0.f, n_eq;
       for (int i = i0; i < i1; i++) {
         const uint32_t b = __float_as_uint(P[i]);
@@ -317,7 +341,7 @@ sample_kernel(const T *__restrict__ logits, int V, SampleArgs s, float *P_global
 
   // ---- the K most probable entries, ties at the K-th in vocabulary order, to the first CTA ---------------------
   const int K = s.top_k;
-  const uint32_t lo = __float_as_uint(weight(DT<T>::from_f(sample_threshold<T, true>(cl, L, P, i0, i1, (float)K))) / sum);
+  const uint32_t lo = __float_as_uint(weight(DT<T>::from_f(sample_threshold<T, true>(cl, L, P, i0, i1, (float)K, -INFINITY, INFINITY))) / sum);
   float gt = 0.f, eq = 0.f, n_gt, n_eq;
   for (int i = i0; i < i1; i++) {
     const uint32_t b = __float_as_uint(P[i]);
