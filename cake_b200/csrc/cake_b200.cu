@@ -3070,9 +3070,13 @@ static MixerScratch mixer_scratch(const cake_b200_ctx *c, const cake_b200_block 
       const size_t rows = (size_t)s.lat_tok * sp.heads, kp = ((size_t)n_keys + TC_BN - 1) / TC_BN * TC_BN;
       s.scores = (float *)take(rows * kp * sizeof(float));
       s.pw = take(rows * 2 * kp * es);
-    } else if (M * sp.heads <= 2048 && n_keys > 128) {
-      s.nsplit = std::min(LATENT_SPLIT_MAX, (n_keys + 127) / 128);
-      s.part = (float *)take(M * sp.heads * s.nsplit * (sp.kv_rank + 2) * sizeof(float));
+    } else if (M * sp.heads <= 2048 && n_keys > 32) {
+      // 32 keys a split while two CTAs per SM take them all, 128 at most: a CTA walks its keys 16 at a time, a few us each (one token, 16 heads, 300
+      // keys: 3 splits 27 us)
+      const int fill = (int)((2 * (size_t)c->sm_count + M * sp.heads - 1) / (M * sp.heads));
+      s.nsplit = std::min(LATENT_SPLIT_MAX, std::max((n_keys + 127) / 128, std::min(fill, (n_keys + 31) / 32)));
+      if (s.nsplit > 1) s.part = (float *)take(M * sp.heads * s.nsplit * (sp.kv_rank + 2) * sizeof(float));
+      else s.nsplit = 0;
     }
   } else {
     s.o32 = (float *)take(M * inner * sizeof(float));

@@ -209,26 +209,114 @@ __global__ void __launch_bounds__(128) latent_attn_split_kernel(const LatentAttn
   for (int c = threadIdx.x; c < p.rank; c += blockDim.x)
     out[2 + c] = (sm_acc[c] * f[0] + sm_acc[p.rank + c] * f[1]) + (sm_acc[2 * p.rank + c] * f[2] + sm_acc[3 * p.rank + c] * f[3]);
 }
+// The same for 16-bit rows of whole 16-byte vectors (Dk and rank multiples of 8): a lane holds the vectors lane + 32 i, so a key is NV loads per lane
+// where the general form has 8 NV of two bytes.  Bound by latency (300 keys of 16 heads are 350 KB): four keys are in flight per warp.
+template <typename T, int NV>
+__global__ void __launch_bounds__(128) latent_attn_split_vec_kernel(const LatentAttn p) {
+  __shared__ float sm_m[4], sm_l[4];
+  extern __shared__ float sm_acc[];  // [4][rank]
+  const int mh = blockIdx.x, split = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int m = mh / p.heads, b = m / p.S, t = m % p.S, n_keys = p.pos0 + t + 1, Dk = p.rank + p.rot, nv = Dk / 8;
+  const int per = ((n_keys + p.nsplit - 1) / p.nsplit + 15) / 16 * 16;
+  const int k0 = split * per, k1 = min(n_keys, k0 + per);
+  const uint4 *q = reinterpret_cast<const uint4 *>(reinterpret_cast<const T *>(p.qa) + (size_t)mh * Dk);
+  const uint4 *kc = reinterpret_cast<const uint4 *>(reinterpret_cast<const T *>(p.cache) + (size_t)b * p.cap * Dk);
+  const uint4 z = make_uint4(0u, 0u, 0u, 0u);
+  float qv[NV][8], acc[NV][8];
+#pragma unroll
+  for (int i = 0; i < NV; i++) {
+    unpack8<T>(lane + 32 * i < nv ? q[lane + 32 * i] : z, qv[i]);
+#pragma unroll
+    for (int e = 0; e < 8; e++) {
+      qv[i][e] *= p.scale;
+      acc[i][e] = 0.f;
+    }
+  }
+  float mx = -INFINITY, l = 0.f;
+  for (int j = k0 + 4 * warp; j < k1; j += 16) {
+    uint4 kv[4][NV];
+    float s[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const uint4 *row = kc + (size_t)(j + u < k1 ? j + u : j) * nv;
+#pragma unroll
+      for (int i = 0; i < NV; i++) kv[u][i] = lane + 32 * i < nv ? row[lane + 32 * i] : z;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      float part = 0.f;
+#pragma unroll
+      for (int i = 0; i < NV; i++) {
+        float f[8];
+        unpack8<T>(kv[u][i], f);
+#pragma unroll
+        for (int e = 0; e < 8; e++) part = fmaf(qv[i][e], f[e], part);
+      }
+      s[u] = warp_sum(part);
+      if (j + u >= k1) s[u] = -INFINITY;
+    }
+    const float mn = fmaxf(fmaxf(mx, fmaxf(s[0], s[1])), fmaxf(s[2], s[3]));
+    const float corr = expf(mx - mn);
+    float pr[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) pr[u] = expf(s[u] - mn);
+    l = l * corr + ((pr[0] + pr[1]) + (pr[2] + pr[3]));
+#pragma unroll
+    for (int i = 0; i < NV; i++) {
+#pragma unroll
+      for (int e = 0; e < 8; e++) acc[i][e] *= corr;
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        float f[8];
+        unpack8<T>(kv[u][i], f);
+#pragma unroll
+        for (int e = 0; e < 8; e++) acc[i][e] = fmaf(pr[u], f[e], acc[i][e]);
+      }
+    }
+    mx = mn;
+  }
+  if (lane == 0) { sm_m[warp] = mx; sm_l[warp] = l; }
+#pragma unroll
+  for (int i = 0; i < NV; i++)
+    if (8 * (lane + 32 * i) < p.rank) {
+#pragma unroll
+      for (int e = 0; e < 8; e++) sm_acc[warp * p.rank + 8 * (lane + 32 * i) + e] = acc[i][e];
+    }
+  __syncthreads();
+  const float M4 = fmaxf(fmaxf(sm_m[0], sm_m[1]), fmaxf(sm_m[2], sm_m[3]));
+  float f[4], L = 0.f;
+#pragma unroll
+  for (int w = 0; w < 4; w++) {
+    f[w] = sm_m[w] == -INFINITY ? 0.f : expf(sm_m[w] - M4);
+    L = fmaf(sm_l[w], f[w], L);
+  }
+  float *out = p.part + ((size_t)mh * p.nsplit + split) * (p.rank + 2);
+  if (threadIdx.x == 0) { out[0] = M4; out[1] = L; }
+  for (int c = threadIdx.x; c < p.rank; c += blockDim.x)
+    out[2 + c] = (sm_acc[c] * f[0] + sm_acc[p.rank + c] * f[1]) + (sm_acc[2 * p.rank + c] * f[2] + sm_acc[3 * p.rank + c] * f[3]);
+}
+// CTA (row-head, 128 columns): a lane per split for the weights, then a column per thread
 template <typename T>
 __global__ void __launch_bounds__(128) latent_attn_merge_kernel(const LatentAttn p) {
-  const int mh = blockIdx.x;
+  __shared__ float w[32], total;
+  const int mh = blockIdx.x, c = blockIdx.y * 128 + threadIdx.x;
   const float *part = p.part + (size_t)mh * p.nsplit * (p.rank + 2);
-  float M = -INFINITY;
-  for (int s = 0; s < p.nsplit; s++) M = fmaxf(M, part[(size_t)s * (p.rank + 2)]);
-  float L = 0.f;
+  if (threadIdx.x < 32) {
+    const int s = threadIdx.x;
+    const float ms = s < p.nsplit ? part[(size_t)s * (p.rank + 2)] : -INFINITY, ls = s < p.nsplit ? part[(size_t)s * (p.rank + 2) + 1] : 0.f;
+    const float M = warp_max(ms), e = ms == -INFINITY ? 0.f : expf(ms - M), L = warp_sum(ms == -INFINITY ? 0.f : ls * e);
+    w[s] = e;
+    if (s == 0) total = L;
+  }
+  __syncthreads();
+  if (c >= p.rank) return;
+  float a = 0.f;
+#pragma unroll 8
   for (int s = 0; s < p.nsplit; s++) {
-    const float ms = part[(size_t)s * (p.rank + 2)];
-    if (ms != -INFINITY) L = fmaf(part[(size_t)s * (p.rank + 2) + 1], expf(ms - M), L);
+    const float v = part[(size_t)s * (p.rank + 2) + 2 + c], e = w[s];
+    a = e == 0.f ? a : fmaf(v, e, a);
   }
-  T *out = reinterpret_cast<T *>(p.lat) + (size_t)mh * p.rank;
-  for (int c = threadIdx.x; c < p.rank; c += blockDim.x) {
-    float a = 0.f;
-    for (int s = 0; s < p.nsplit; s++) {
-      const float ms = part[(size_t)s * (p.rank + 2)];
-      if (ms != -INFINITY) a = fmaf(part[(size_t)s * (p.rank + 2) + 2 + c], expf(ms - M), a);
-    }
-    out[c] = DT<T>::from_f(a / L);
-  }
+  (reinterpret_cast<T *>(p.lat) + (size_t)mh * p.rank)[c] = DT<T>::from_f(a / total);
 }
 
 // four adjacent entries (8- / 16-byte load)
@@ -304,6 +392,13 @@ int latent_softmax(cudaStream_t st, int dtype, const LatentSoftmax &p, uint64_t 
   MX_DONE(1);
 }
 
+template <typename T> static void latent_attn_split_vec(cudaStream_t st, dim3 grid, size_t smem, const LatentAttn &p, const T *) {
+  if constexpr (sizeof(T) == 2) {
+    if (p.rank + p.rot <= 256) latent_attn_split_vec_kernel<T, 1><<<grid, 128, smem, st>>>(p);
+    else if (p.rank + p.rot <= 512) latent_attn_split_vec_kernel<T, 2><<<grid, 128, smem, st>>>(p);
+    else latent_attn_split_vec_kernel<T, 3><<<grid, 128, smem, st>>>(p);
+  }
+}
 int latent_attention(cudaStream_t st, int dtype, const LatentAttn &p, uint64_t *launches) {
   const int Dk = p.rank + p.rot;
   if (Dk > 32 * 24) return (int)cudaErrorInvalidValue;
@@ -311,10 +406,11 @@ int latent_attention(cudaStream_t st, int dtype, const LatentAttn &p, uint64_t *
     const dim3 grid((unsigned)(p.B * p.S * p.heads), (unsigned)p.nsplit);
     const size_t smem = (size_t)4 * p.rank * sizeof(float);
     MX_DISPATCH(dtype, {
-      if (Dk <= 32 * 6) latent_attn_split_kernel<T, 6><<<grid, 128, smem, st>>>(p);
+      if (sizeof(T) == 2 && Dk % 8 == 0 && p.rank % 8 == 0 && (((uintptr_t)p.qa | (uintptr_t)p.cache) & 15) == 0) latent_attn_split_vec(st, grid, smem, p, (const T *)nullptr);
+      else if (Dk <= 32 * 6) latent_attn_split_kernel<T, 6><<<grid, 128, smem, st>>>(p);
       else if (Dk <= 32 * 12) latent_attn_split_kernel<T, 12><<<grid, 128, smem, st>>>(p);
       else latent_attn_split_kernel<T, 24><<<grid, 128, smem, st>>>(p);
-      latent_attn_merge_kernel<T><<<grid.x, 128, 0, st>>>(p);
+      latent_attn_merge_kernel<T><<<dim3(grid.x, (unsigned)((p.rank + 127) / 128)), 128, 0, st>>>(p);
     });
     MX_DONE(2);
   }
@@ -413,7 +509,47 @@ __global__ void __launch_bounds__(128) head_gemv_kernel(const HeadGemm p) {
     if (lane == 0) C[n] = DT<T>::from_f(acc);
   }
 }
+// W[z] stored [K, N] in 16 bits, N in whole 16-byte vectors: CTA (128 columns, row, z), a thread takes 8 columns of every 16th k, so that a CTA has its 32 KB
+// of a K of 128 in flight at once; a thread per column walked k one load behind the other (16 x 128 x 512: 21.9 us).
+template <typename T>
+__global__ void __launch_bounds__(256) head_gemv_kn_kernel(const HeadGemm p) {
+  extern __shared__ float arow[];  // the row of A
+  __shared__ float part[16][128 + 4];
+  const int z = blockIdx.z, m = blockIdx.y, v = threadIdx.x & 15, kg = threadIdx.x >> 4, n = blockIdx.x * 128 + 8 * v;
+  const T *A = reinterpret_cast<const T *>(p.A) + (size_t)z * p.a_zs + (size_t)m * p.lda;
+  const T *W = reinterpret_cast<const T *>(p.W) + (size_t)z * p.w_zs + n;
+  T *C = reinterpret_cast<T *>(p.C) + (size_t)z * p.c_zs + (size_t)m * p.ldc;
+  for (int k = threadIdx.x; k < p.K; k += blockDim.x) arow[k] = DT<T>::to_f(A[k]);
+  __syncthreads();
+  float acc[8] = {};
+  if (n < p.N) {
+#pragma unroll 8
+    for (int k = kg; k < p.K; k += 16) {
+      float f[8];
+      unpack8<T>(*reinterpret_cast<const uint4 *>(W + (size_t)k * p.ldw), f);
+      const float a = arow[k];
+#pragma unroll
+      for (int e = 0; e < 8; e++) acc[e] = fmaf(a, f[e], acc[e]);
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < 8; e++) part[kg][8 * v + e] = acc[e];
+  __syncthreads();
+  const int c = threadIdx.x;
+  if (c >= 128 || blockIdx.x * 128 + c >= p.N) return;
+  float sum = 0.f;
+#pragma unroll
+  for (int g = 0; g < 16; g++) sum += part[g][c];
+  C[blockIdx.x * 128 + c] = DT<T>::from_f(sum);
+}
+template <typename T> static void head_gemv_kn(cudaStream_t st, dim3 grid, const HeadGemm &p, const T *) {
+  if constexpr (sizeof(T) == 2) head_gemv_kn_kernel<T><<<grid, 256, (size_t)p.K * sizeof(float), st>>>(p);
+}
 int head_gemm(cudaStream_t st, int dtype, const HeadGemm &p, uint64_t *launches) {
+  if (p.M <= 8 && p.K <= 8192 && p.w_kn && dtype != 2 && p.N % 8 == 0 && p.ldw % 8 == 0 && p.w_zs % 8 == 0 && ((uintptr_t)p.W & 15) == 0) {
+    MX_DISPATCH(dtype, head_gemv_kn(st, dim3((p.N + 127) / 128, p.M, p.Z), p, (const T *)nullptr));
+    MX_DONE(1);
+  }
   if (p.M <= 8 && p.K <= 8192) {
     const dim3 grid(p.w_kn ? (p.N + 127) / 128 : (p.N + 3) / 4, p.M, p.Z);
     MX_DISPATCH(dtype, (head_gemv_kernel<T><<<grid, 128, (size_t)p.K * sizeof(float), st>>>(p)));
