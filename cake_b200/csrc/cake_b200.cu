@@ -596,7 +596,7 @@ extern "C" int cake_b200_ctx_create(int device, const cake_b200_config *cfg, cak
   *c->wait_err = 0;
   CU(cudaMalloc(&c->gbar, 24));
   CU(cudaMemset(c->gbar, 0, 24));
-  {  // tags begin at 1
+  if (!cfg->layer_list) {  // tags begin at 1
     const size_t n = mk_packet_offsets(c, nullptr), parts = (size_t)nh * c->nsplit * (hd + 2);
     CU(cudaMalloc(&c->mk_pk, n * 4));
     CU(cudaMemset(c->mk_pk, 0, n * 4));

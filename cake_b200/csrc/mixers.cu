@@ -18,6 +18,30 @@ namespace mx {
     else if ((dtype) == 1) { typedef __half T; __VA_ARGS__; } \
     else { typedef __nv_bfloat16 T; __VA_ARGS__; }            \
   } while (0)
+// The kernels here wait for the one in front before their first access (griddepcontrol.wait) and, where they are small, are launched while it ends:
+// without that a step's chain of 24 launches of a few us each paid 2 us of launch latency each time (step through three Setodra blocks 358 -> 315 us).  Not so
+// grids of more than two CTAs per SM, and not a recurrence over many tokens: CTAs placed while the kernel in front still holds most of the chip crowd
+// on the SMs that are free first (1000 tokens: 2200 -> 2434 us with all of them launched early).
+constexpr unsigned MX_EARLY_CTAS = 296;
+constexpr int MX_EARLY_TOKENS = 8;
+template <typename... KArgs, typename... Args>
+static void mx_launch_if(bool early, cudaStream_t st, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, Args... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = early && (size_t)grid.x * grid.y * grid.z <= MX_EARLY_CTAS ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+template <typename... KArgs, typename... Args>
+static void mx_launch(cudaStream_t st, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, Args... args) {
+  mx_launch_if(true, st, kern, grid, block, smem, args...);
+}
 #define MX_DONE(n)                     \
   do {                                 \
     if (launches) *launches += (n);    \
@@ -39,6 +63,8 @@ __device__ __forceinline__ float rotated(const T *v, int i, int dims, const floa
 // ---------------------------------------------------------------------------------------------- latent attention: prep
 template <typename T>
 __global__ void __launch_bounds__(128) latent_prep_kernel(const LatentPrep p) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float red[4];
   const int m = blockIdx.x, b = m / p.S, t = m % p.S, pos = p.pos0 + t;
   const T *row = reinterpret_cast<const T *>(p.proj) + (size_t)m * p.ld;
@@ -70,7 +96,7 @@ __global__ void __launch_bounds__(128) latent_prep_kernel(const LatentPrep p) {
   }
 }
 int latent_prep(cudaStream_t st, int dtype, const LatentPrep &p, uint64_t *launches) {
-  MX_DISPATCH(dtype, (latent_prep_kernel<T><<<p.B * p.S, 128, 0, st>>>(p)));
+  MX_DISPATCH(dtype, (mx_launch(st, latent_prep_kernel<T>, p.B * p.S, 128, 0, p)));
   MX_DONE(1);
 }
 
@@ -78,6 +104,8 @@ int latent_prep(cudaStream_t st, int dtype, const LatentPrep &p, uint64_t *launc
 // One warp per (row, head): lanes split the rank + rot columns of a cached row, four keys per round, running softmax.
 template <typename T, int NR>
 __global__ void __launch_bounds__(128) latent_attn_kernel(const LatentAttn p) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int warp = (int)(((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (warp >= p.B * p.S * p.heads) return;
   const int m = warp / p.heads, h = warp % p.heads, b = m / p.S, t = m % p.S, n_keys = p.pos0 + t + 1;
@@ -139,6 +167,8 @@ __global__ void __launch_bounds__(128) latent_attn_kernel(const LatentAttn p) {
 // merged in shared memory and written as (max, sum, weighted latent); a second kernel merges the splits.
 template <typename T, int NR>
 __global__ void __launch_bounds__(128) latent_attn_split_kernel(const LatentAttn p) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float sm_m[4], sm_l[4];
   extern __shared__ float sm_acc[];  // [4][rank]
   const int mh = blockIdx.x, split = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -213,6 +243,8 @@ __global__ void __launch_bounds__(128) latent_attn_split_kernel(const LatentAttn
 // where the general form has 8 NV of two bytes.  Bound by latency (300 keys of 16 heads are 350 KB): four keys are in flight per warp.
 template <typename T, int NV>
 __global__ void __launch_bounds__(128) latent_attn_split_vec_kernel(const LatentAttn p) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float sm_m[4], sm_l[4];
   extern __shared__ float sm_acc[];  // [4][rank]
   const int mh = blockIdx.x, split = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -298,6 +330,8 @@ __global__ void __launch_bounds__(128) latent_attn_split_vec_kernel(const Latent
 // CTA (row-head, 128 columns): a lane per split for the weights, then a column per thread
 template <typename T>
 __global__ void __launch_bounds__(128) latent_attn_merge_kernel(const LatentAttn p) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float w[32], total;
   const int mh = blockIdx.x, c = blockIdx.y * 128 + threadIdx.x;
   const float *part = p.part + (size_t)mh * p.nsplit * (p.rank + 2);
@@ -343,6 +377,8 @@ template <> __device__ __forceinline__ void store4<__half>(__half *d, const floa
 // moves four consecutive scores per load (16 bytes in, 8 + 8 bytes out)
 template <typename T>
 __global__ void __launch_bounds__(128) latent_softmax_kernel(const LatentSoftmax p) {
+  pdl_launch_dependents();
+  pdl_wait();
   const long row = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (row >= (long)p.n_tok * p.heads) return;
@@ -388,15 +424,15 @@ __global__ void __launch_bounds__(128) latent_softmax_kernel(const LatentSoftmax
 int latent_softmax(cudaStream_t st, int dtype, const LatentSoftmax &p, uint64_t *launches) {
   const long warps = (long)p.n_tok * p.heads;
   if (p.kp % 4) return (int)cudaErrorInvalidValue;
-  MX_DISPATCH(dtype, (latent_softmax_kernel<T><<<(unsigned)((warps + 3) / 4), 128, 0, st>>>(p)));
+  MX_DISPATCH(dtype, (mx_launch(st, latent_softmax_kernel<T>, (unsigned)((warps + 3) / 4), 128, 0, p)));
   MX_DONE(1);
 }
 
 template <typename T> static void latent_attn_split_vec(cudaStream_t st, dim3 grid, size_t smem, const LatentAttn &p, const T *) {
   if constexpr (sizeof(T) == 2) {
-    if (p.rank + p.rot <= 256) latent_attn_split_vec_kernel<T, 1><<<grid, 128, smem, st>>>(p);
-    else if (p.rank + p.rot <= 512) latent_attn_split_vec_kernel<T, 2><<<grid, 128, smem, st>>>(p);
-    else latent_attn_split_vec_kernel<T, 3><<<grid, 128, smem, st>>>(p);
+    if (p.rank + p.rot <= 256) mx_launch(st, latent_attn_split_vec_kernel<T, 1>, grid, 128, smem, p);
+    else if (p.rank + p.rot <= 512) mx_launch(st, latent_attn_split_vec_kernel<T, 2>, grid, 128, smem, p);
+    else mx_launch(st, latent_attn_split_vec_kernel<T, 3>, grid, 128, smem, p);
   }
 }
 int latent_attention(cudaStream_t st, int dtype, const LatentAttn &p, uint64_t *launches) {
@@ -407,19 +443,19 @@ int latent_attention(cudaStream_t st, int dtype, const LatentAttn &p, uint64_t *
     const size_t smem = (size_t)4 * p.rank * sizeof(float);
     MX_DISPATCH(dtype, {
       if (sizeof(T) == 2 && Dk % 8 == 0 && p.rank % 8 == 0 && (((uintptr_t)p.qa | (uintptr_t)p.cache) & 15) == 0) latent_attn_split_vec(st, grid, smem, p, (const T *)nullptr);
-      else if (Dk <= 32 * 6) latent_attn_split_kernel<T, 6><<<grid, 128, smem, st>>>(p);
-      else if (Dk <= 32 * 12) latent_attn_split_kernel<T, 12><<<grid, 128, smem, st>>>(p);
-      else latent_attn_split_kernel<T, 24><<<grid, 128, smem, st>>>(p);
-      latent_attn_merge_kernel<T><<<dim3(grid.x, (unsigned)((p.rank + 127) / 128)), 128, 0, st>>>(p);
+      else if (Dk <= 32 * 6) mx_launch(st, latent_attn_split_kernel<T, 6>, grid, 128, smem, p);
+      else if (Dk <= 32 * 12) mx_launch(st, latent_attn_split_kernel<T, 12>, grid, 128, smem, p);
+      else mx_launch(st, latent_attn_split_kernel<T, 24>, grid, 128, smem, p);
+      mx_launch(st, latent_attn_merge_kernel<T>, dim3(grid.x, (unsigned)((p.rank + 127) / 128)), 128, 0, p);
     });
     MX_DONE(2);
   }
   const long warps = (long)p.B * p.S * p.heads;
   const unsigned grid = (unsigned)((warps + 3) / 4);
   MX_DISPATCH(dtype, {
-    if (Dk <= 32 * 6) latent_attn_kernel<T, 6><<<grid, 128, 0, st>>>(p);
-    else if (Dk <= 32 * 12) latent_attn_kernel<T, 12><<<grid, 128, 0, st>>>(p);
-    else latent_attn_kernel<T, 24><<<grid, 128, 0, st>>>(p);
+    if (Dk <= 32 * 6) mx_launch(st, latent_attn_kernel<T, 6>, grid, 128, 0, p);
+    else if (Dk <= 32 * 12) mx_launch(st, latent_attn_kernel<T, 12>, grid, 128, 0, p);
+    else mx_launch(st, latent_attn_kernel<T, 24>, grid, 128, 0, p);
   });
   MX_DONE(1);
 }
@@ -428,6 +464,8 @@ int latent_attention(cudaStream_t st, int dtype, const LatentAttn &p, uint64_t *
 constexpr int HG_BM = 64, HG_BN = 64, HG_BK = 16;
 template <typename T>
 __global__ void __launch_bounds__(256) head_gemm_kernel(const HeadGemm p) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float As[HG_BK][HG_BM + 4];
   __shared__ float Ws[HG_BK][HG_BN + 4];
   const int z = blockIdx.z;
@@ -481,6 +519,8 @@ __global__ void __launch_bounds__(256) head_gemm_kernel(const HeadGemm p) {
 // else (W[z] stored [N, K]): a warp per output column splits k.  The row of A sits in shared memory.
 template <typename T>
 __global__ void __launch_bounds__(128) head_gemv_kernel(const HeadGemm p) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float arow[];
   const int z = blockIdx.z, m = blockIdx.y;
   const T *A = reinterpret_cast<const T *>(p.A) + (size_t)z * p.a_zs + (size_t)m * p.lda;
@@ -513,6 +553,8 @@ __global__ void __launch_bounds__(128) head_gemv_kernel(const HeadGemm p) {
 // of a K of 128 in flight at once; a thread per column walked k one load behind the other (16 x 128 x 512: 21.9 us).
 template <typename T>
 __global__ void __launch_bounds__(256) head_gemv_kn_kernel(const HeadGemm p) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float arow[];  // the row of A
   __shared__ float part[16][128 + 4];
   const int z = blockIdx.z, m = blockIdx.y, v = threadIdx.x & 15, kg = threadIdx.x >> 4, n = blockIdx.x * 128 + 8 * v;
@@ -543,7 +585,7 @@ __global__ void __launch_bounds__(256) head_gemv_kn_kernel(const HeadGemm p) {
   C[blockIdx.x * 128 + c] = DT<T>::from_f(sum);
 }
 template <typename T> static void head_gemv_kn(cudaStream_t st, dim3 grid, const HeadGemm &p, const T *) {
-  if constexpr (sizeof(T) == 2) head_gemv_kn_kernel<T><<<grid, 256, (size_t)p.K * sizeof(float), st>>>(p);
+  if constexpr (sizeof(T) == 2) mx_launch(st, head_gemv_kn_kernel<T>, grid, 256, (size_t)p.K * sizeof(float), p);
 }
 int head_gemm(cudaStream_t st, int dtype, const HeadGemm &p, uint64_t *launches) {
   if (p.M <= 8 && p.K <= 8192 && p.w_kn && dtype != 2 && p.N % 8 == 0 && p.ldw % 8 == 0 && p.w_zs % 8 == 0 && ((uintptr_t)p.W & 15) == 0) {
@@ -552,16 +594,18 @@ int head_gemm(cudaStream_t st, int dtype, const HeadGemm &p, uint64_t *launches)
   }
   if (p.M <= 8 && p.K <= 8192) {
     const dim3 grid(p.w_kn ? (p.N + 127) / 128 : (p.N + 3) / 4, p.M, p.Z);
-    MX_DISPATCH(dtype, (head_gemv_kernel<T><<<grid, 128, (size_t)p.K * sizeof(float), st>>>(p)));
+    MX_DISPATCH(dtype, (mx_launch(st, head_gemv_kernel<T>, grid, 128, (size_t)p.K * sizeof(float), p)));
     MX_DONE(1);
   }
   dim3 grid((p.N + HG_BN - 1) / HG_BN, (p.M + HG_BM - 1) / HG_BM, p.Z);
-  MX_DISPATCH(dtype, (head_gemm_kernel<T><<<grid, 256, 0, st>>>(p)));
+  MX_DISPATCH(dtype, (mx_launch(st, head_gemm_kernel<T>, grid, 256, 0, p)));
   MX_DONE(1);
 }
 
 template <typename T>
 __global__ void transpose_batched_kernel(const T *__restrict__ in, T *__restrict__ out, int rows, int cols) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ T tile[32][33];
   const size_t z = blockIdx.z;
   const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
@@ -573,7 +617,7 @@ __global__ void transpose_batched_kernel(const T *__restrict__ in, T *__restrict
 }
 int transpose_batched(cudaStream_t st, int dtype, const void *in, void *out, int Z, int rows, int cols, uint64_t *launches) {
   const dim3 grid((cols + 31) / 32, (rows + 31) / 32, Z), block(32, 8);
-  MX_DISPATCH(dtype, (transpose_batched_kernel<T><<<grid, block, 0, st>>>(reinterpret_cast<const T *>(in), reinterpret_cast<T *>(out), rows, cols)));
+  MX_DISPATCH(dtype, (mx_launch(st, transpose_batched_kernel<T>, grid, block, 0, reinterpret_cast<const T *>(in), reinterpret_cast<T *>(out), rows, cols)));
   MX_DONE(1);
 }
 
@@ -582,6 +626,8 @@ int transpose_batched(cudaStream_t st, int dtype, const void *in, void *out, int
 // column j of the rows i = s, s + RS, ...: it updates them and adds S[i][j] q[i] to its partial of o[j].
 template <typename T>
 __global__ void recurrence_kernel(const Recurrence p) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float sm[];
   const int h = blockIdx.x, b = blockIdx.y, dk = p.dk, dv = p.dv;
   const int RS = max(1, (int)blockDim.x / dv);
@@ -654,6 +700,8 @@ __global__ void recurrence_kernel(const Recurrence p) {
 constexpr int RC_TT = 16, RC_CB = 32, RC_RS = 8;
 template <typename T, int R, bool ROPE>
 __global__ void __launch_bounds__(256, R > 16 ? 1 : (ROPE ? 2 : 3)) recurrence_cols_kernel(const Recurrence p) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float sm[];
   constexpr int dk = R * RC_RS;
   float *qs = sm, *ks = qs + RC_TT * dk, *vs = ks + RC_TT * dk, *as = vs + RC_TT * RC_CB, *bs = as + RC_TT, *part = bs + RC_TT;
@@ -790,7 +838,7 @@ template <typename T, int R, bool ROPE> static cudaError_t launch_recurrence_col
     if (e != cudaSuccess) return e;
     attr_dev = dev;
   }
-  recurrence_cols_kernel<T, R, ROPE><<<dim3(p.heads * (p.dv / RC_CB), p.B), 256, smem, st>>>(p);
+  mx_launch_if(p.S <= MX_EARLY_TOKENS, st, recurrence_cols_kernel<T, R, ROPE>, dim3(p.heads * (p.dv / RC_CB), p.B), 256, smem, p);
   return cudaSuccess;
 }
 template <typename T, int R> static cudaError_t launch_recurrence_cols(cudaStream_t st, const Recurrence &p) {
@@ -834,7 +882,7 @@ int recurrence(cudaStream_t st, int dtype, const Recurrence &p, uint64_t *launch
       if (e != cudaSuccess) return (int)e;
       attr_dev = dev;
     }
-    recurrence_kernel<T><<<dim3(p.heads, p.B), threads, smem, st>>>(p);
+    mx_launch_if(p.S <= MX_EARLY_TOKENS, st, recurrence_kernel<T>, dim3(p.heads, p.B), threads, smem, p);
   });
   MX_DONE(1);
 }
@@ -842,6 +890,8 @@ int recurrence(cudaStream_t st, int dtype, const Recurrence &p, uint64_t *launch
 // ---------------------------------------------------------------------------------------------- short convolution
 template <typename T>
 __global__ void __launch_bounds__(256) short_conv_kernel(const ShortConv p) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int m = blockIdx.x, b = m / p.S, t = m % p.S, back = p.taps - 1;
   const T *in = reinterpret_cast<const T *>(p.in);
   const T *w = reinterpret_cast<const T *>(p.w), *bias = reinterpret_cast<const T *>(p.bias);
@@ -864,6 +914,8 @@ __global__ void __launch_bounds__(256) short_conv_kernel(const ShortConv p) {
 constexpr int SC_TOK = 16;
 template <typename T, int TAPS>
 __global__ void __launch_bounds__(128) short_conv_vec_kernel(const ShortConv p) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int c8 = blockIdx.y * blockDim.x + threadIdx.x;
   if (c8 >= p.channels / 8) return;
   const int ch = c8 * 8, chunks = (p.S + SC_TOK - 1) / SC_TOK, b = blockIdx.x / chunks, t0 = (blockIdx.x % chunks) * SC_TOK;
@@ -925,17 +977,19 @@ template <typename T> static void launch_short_conv(cudaStream_t st, const Short
   const bool vec = p.channels % 8 == 0 && p.ld % 8 == 0 && p.col0 % 8 == 0 && p.taps >= 2 && p.taps <= 4 &&
                    (((uintptr_t)p.in | (uintptr_t)p.hist | (uintptr_t)p.out | (uintptr_t)p.bias | (uintptr_t)p.w) & 15) == 0;
   const dim3 gv(p.B * ((p.S + SC_TOK - 1) / SC_TOK), (p.channels / 8 + 127) / 128);
-  if (vec && p.taps == 2) short_conv_vec_kernel<T, 2><<<gv, 128, 0, st>>>(p);
-  else if (vec && p.taps == 3) short_conv_vec_kernel<T, 3><<<gv, 128, 0, st>>>(p);
-  else if (vec && p.taps == 4) short_conv_vec_kernel<T, 4><<<gv, 128, 0, st>>>(p);
-  else short_conv_kernel<T><<<dim3(p.B * p.S, (p.channels + 255) / 256), 256, 0, st>>>(p);
+  if (vec && p.taps == 2) mx_launch(st, short_conv_vec_kernel<T, 2>, gv, 128, 0, p);
+  else if (vec && p.taps == 3) mx_launch(st, short_conv_vec_kernel<T, 3>, gv, 128, 0, p);
+  else if (vec && p.taps == 4) mx_launch(st, short_conv_vec_kernel<T, 4>, gv, 128, 0, p);
+  else mx_launch(st, short_conv_kernel<T>, dim3(p.B * p.S, (p.channels + 255) / 256), 256, 0, p);
 }
 template <> void launch_short_conv<float>(cudaStream_t st, const ShortConv &p) {
-  short_conv_kernel<float><<<dim3(p.B * p.S, (p.channels + 255) / 256), 256, 0, st>>>(p);
+  mx_launch(st, short_conv_kernel<float>, dim3(p.B * p.S, (p.channels + 255) / 256), 256, 0, p);
 }
 // after the convolution: the history becomes the last taps - 1 inputs up to the end of this step (zeros before position 0)
 template <typename T>
 __global__ void short_conv_hist_kernel(const ShortConv p) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int idx = blockIdx.x * blockDim.x + threadIdx.x, back = p.taps - 1;
   if (idx >= p.B * p.channels) return;
   const int b = idx / p.channels, ch = idx % p.channels;
@@ -952,7 +1006,7 @@ __global__ void short_conv_hist_kernel(const ShortConv p) {
 int short_conv(cudaStream_t st, int dtype, const ShortConv &p, uint64_t *launches) {
   MX_DISPATCH(dtype, {
     launch_short_conv<T>(st, p);
-    if (p.taps > 1) short_conv_hist_kernel<T><<<(p.B * p.channels + 255) / 256, 256, 0, st>>>(p);
+    if (p.taps > 1) mx_launch(st, short_conv_hist_kernel<T>, (p.B * p.channels + 255) / 256, 256, 0, p);
   });
   MX_DONE(p.taps > 1 ? 2 : 1);
 }
@@ -962,6 +1016,8 @@ template <typename T> struct Bits16 { typedef T type; };
 template <> struct Bits16<float> { typedef __nv_bfloat16 type; };  // never taken for float (sizeof test); keeps the vector path instantiable
 template <typename T>
 __global__ void __launch_bounds__(128) gate_norm_kernel(const GateNorm p) {
+  pdl_launch_dependents();
+  pdl_wait();
   const long warp = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= (long)p.M * p.parts) return;
@@ -1037,7 +1093,7 @@ __global__ void __launch_bounds__(128) gate_norm_kernel(const GateNorm p) {
 int gate_norm(cudaStream_t st, int dtype, const GateNorm &p, uint64_t *launches) {
   if (p.parts < 1 || p.n % p.parts || (p.w_period && p.w_period != p.n / p.parts)) return (int)cudaErrorInvalidValue;
   const long warps = (long)p.M * p.parts;
-  MX_DISPATCH(dtype, (gate_norm_kernel<T><<<(unsigned)((warps + 3) / 4), 128, 0, st>>>(p)));
+  MX_DISPATCH(dtype, (mx_launch(st, gate_norm_kernel<T>, (unsigned)((warps + 3) / 4), 128, 0, p)));
   MX_DONE(1);
 }
 
@@ -1046,6 +1102,8 @@ constexpr int MOE_MAX_SLOTS = 8;  // experts + identity <= 256
 // NS: slots of 32 experts that a warp's lanes hold
 template <typename T, int NS>
 __global__ void __launch_bounds__(128) moe_router_kernel(const MoePlan p) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (warp >= p.M) return;
   const int m = warp, E = p.experts + p.identity;
@@ -1149,11 +1207,15 @@ __global__ void __launch_bounds__(128) moe_router_kernel(const MoePlan p) {
   if (p.has_shared_gate && lane == 0) p.sgate[m] = 1.0f / (1.0f + expf(-lg[E]));
 }
 __global__ void moe_count_kernel(const int *ids, int n, int experts, int *counts) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n && ids[i] < experts) atomicAdd(&counts[ids[i]], 1);
 }
 // one warp: every expert's pairs start on a multiple of `tile` sorted rows; counts[e] becomes that start (the scatter's cursor)
 __global__ void moe_tiles_kernel(const MoePlan p) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int lane = threadIdx.x;
   int done = 0;  // blocks of `tile` rows handed out so far
   for (int base = 0; base < p.experts; base += 32) {
@@ -1172,6 +1234,8 @@ __global__ void moe_tiles_kernel(const MoePlan p) {
   for (int i = done + lane; i < p.max_tiles; i += 32) p.tile_expert[i] = -1;
 }
 __global__ void moe_scatter_kernel(const int *ids, int n, int experts, int *cursor, int *perm, int *pos_of) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n && ids[i] < experts) {
     const int pos = atomicAdd(&cursor[ids[i]], 1);
@@ -1182,6 +1246,8 @@ __global__ void moe_scatter_kernel(const int *ids, int n, int experts, int *curs
 // few (token, slot) pairs (decoding): count, plan and scatter in one CTA with the counters in shared memory
 constexpr int MOE_SMALL_PAIRS = 1024;
 __global__ void __launch_bounds__(256) moe_plan_small_kernel(const MoePlan p) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ int cnt[32 * MOE_MAX_SLOTS];
   __shared__ int done_s;
   const int ne = p.M * p.top, rows = p.max_tiles * p.tile;
@@ -1227,22 +1293,22 @@ int moe_route(cudaStream_t st, int dtype, const MoePlan &p, uint64_t *launches) 
   const int slots = (p.experts + p.identity + 31) / 32;
   MX_DISPATCH(dtype, {
     const unsigned grid = (unsigned)((p.M + 3) / 4);
-    if (slots <= 1) moe_router_kernel<T, 1><<<grid, 128, 0, st>>>(p);
-    else if (slots <= 2) moe_router_kernel<T, 2><<<grid, 128, 0, st>>>(p);
-    else if (slots <= 4) moe_router_kernel<T, 4><<<grid, 128, 0, st>>>(p);
-    else moe_router_kernel<T, MOE_MAX_SLOTS><<<grid, 128, 0, st>>>(p);
+    if (slots <= 1) mx_launch(st, moe_router_kernel<T, 1>, grid, 128, 0, p);
+    else if (slots <= 2) mx_launch(st, moe_router_kernel<T, 2>, grid, 128, 0, p);
+    else if (slots <= 4) mx_launch(st, moe_router_kernel<T, 4>, grid, 128, 0, p);
+    else mx_launch(st, moe_router_kernel<T, MOE_MAX_SLOTS>, grid, 128, 0, p);
   });
   int n = 1;
   if (p.experts > 0 && p.M * p.top <= MOE_SMALL_PAIRS) {
-    moe_plan_small_kernel<<<1, 256, 0, st>>>(p);
+    mx_launch(st, moe_plan_small_kernel, 1, 256, 0, p);
     n += 1;
   } else if (p.experts > 0) {
     cudaMemsetAsync(p.counts, 0, sizeof(int) * (p.experts + 1), st);
     cudaMemsetAsync(p.perm, 0xff, sizeof(int) * (size_t)p.max_tiles * p.tile, st);
     const int ne = p.M * p.top;
-    moe_count_kernel<<<(ne + 255) / 256, 256, 0, st>>>(p.ids, ne, p.experts, p.counts);
-    moe_tiles_kernel<<<1, 32, 0, st>>>(p);
-    moe_scatter_kernel<<<(ne + 255) / 256, 256, 0, st>>>(p.ids, ne, p.experts, p.counts, p.perm, p.pos_of);
+    mx_launch(st, moe_count_kernel, (ne + 255) / 256, 256, 0, p.ids, ne, p.experts, p.counts);
+    mx_launch(st, moe_tiles_kernel, 1, 32, 0, p);
+    mx_launch(st, moe_scatter_kernel, (ne + 255) / 256, 256, 0, p.ids, ne, p.experts, p.counts, p.perm, p.pos_of);
     n += 3;
   }
   MX_DONE(n);
@@ -1251,6 +1317,8 @@ int moe_route(cudaStream_t st, int dtype, const MoePlan &p, uint64_t *launches) 
 template <typename T>
 __global__ void __launch_bounds__(128) moe_gather_kernel(const T *__restrict__ h, const int *__restrict__ perm, T *__restrict__ sorted, int W, int top,
                                                          const float *__restrict__ wts) {
+  pdl_launch_dependents();
+  pdl_wait();
   const size_t r = blockIdx.x;
   const int e = perm[r];
   T *dst = sorted + r * W;
@@ -1288,7 +1356,7 @@ __global__ void __launch_bounds__(128) moe_gather_kernel(const T *__restrict__ h
   for (int i = threadIdx.x; i < W; i += blockDim.x) dst[i] = src ? src[i] : DT<T>::from_f(0.f);
 }
 int moe_gather(cudaStream_t st, int dtype, const void *h, const int *perm, void *sorted, int rows, int W, int top, uint64_t *launches, const float *wts) {
-  MX_DISPATCH(dtype, (moe_gather_kernel<T><<<rows, 128, 0, st>>>(reinterpret_cast<const T *>(h), perm, reinterpret_cast<T *>(sorted), W, top, wts)));
+  MX_DISPATCH(dtype, (mx_launch(st, moe_gather_kernel<T>, rows, 128, 0, reinterpret_cast<const T *>(h), perm, reinterpret_cast<T *>(sorted), W, top, wts)));
   MX_DONE(1);
 }
 
@@ -1302,6 +1370,8 @@ __device__ __forceinline__ float act_f(float g, int kind) {
 }
 template <typename T, int PHASE>
 __global__ void __launch_bounds__(256) moe_expert_kernel(const MoeExperts p) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int tl = blockIdx.y, e = p.tile_expert[tl];
   if (e < 0) return;
   __shared__ float As[ME_BK][ME_BM + 4];
@@ -1378,14 +1448,16 @@ __global__ void __launch_bounds__(256) moe_expert_kernel(const MoeExperts p) {
 int moe_experts(cudaStream_t st, int dtype, const MoeExperts &p, uint64_t *launches) {
   if (p.tile != ME_BM) return (int)cudaErrorInvalidValue;
   MX_DISPATCH(dtype, {
-    moe_expert_kernel<T, 0><<<dim3((p.ff + ME_BN - 1) / ME_BN, p.max_tiles), 256, 0, st>>>(p);
-    moe_expert_kernel<T, 1><<<dim3((p.W + ME_BN - 1) / ME_BN, p.max_tiles), 256, 0, st>>>(p);
+    mx_launch(st, moe_expert_kernel<T, 0>, dim3((p.ff + ME_BN - 1) / ME_BN, p.max_tiles), 256, 0, p);
+    mx_launch(st, moe_expert_kernel<T, 1>, dim3((p.W + ME_BN - 1) / ME_BN, p.max_tiles), 256, 0, p);
   });
   MX_DONE(2);
 }
 
 template <typename T>
 __global__ void __launch_bounds__(256) moe_combine_kernel(const MoeCombine p) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int m = blockIdx.x;
   const T *h = reinterpret_cast<const T *>(p.h) + (size_t)m * p.W;
   if ((p.W & 3) == 0) {  // 16-byte loads and stores of the fp32 rows
@@ -1419,7 +1491,7 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const MoeCombine p) {
   }
 }
 int moe_combine(cudaStream_t st, int dtype, const MoeCombine &p, uint64_t *launches) {
-  MX_DISPATCH(dtype, (moe_combine_kernel<T><<<dim3(p.M, p.M < 64 ? (p.W + 255) / 256 : 1), 256, 0, st>>>(p)));
+  MX_DISPATCH(dtype, (mx_launch(st, moe_combine_kernel<T>, dim3(p.M, p.M < 64 ? (p.W + 255) / 256 : 1), 256, 0, p)));
   MX_DONE(1);
 }
 
@@ -1441,6 +1513,8 @@ __device__ __forceinline__ void block_sum2(float &a, float &b, float *red /* [64
 // ---------------------------------------------------------------------------------------------- RMS norm of fp32 rows
 template <typename T>
 __global__ void __launch_bounds__(256) rms_rows_kernel(const RmsRows p) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float red[64];
   const int m = blockIdx.x;
   const float *x = p.x + (size_t)m * p.n;
@@ -1457,13 +1531,15 @@ __global__ void __launch_bounds__(256) rms_rows_kernel(const RmsRows p) {
 }
 int rms_rows(cudaStream_t st, int dtype, const RmsRows &p, uint64_t *launches) {
   if (p.M < 1 || p.n < 1 || (!p.out32 && !p.outD)) return (int)cudaErrorInvalidValue;
-  MX_DISPATCH(dtype, (rms_rows_kernel<T><<<p.M, 256, 0, st>>>(p)));
+  MX_DISPATCH(dtype, (mx_launch(st, rms_rows_kernel<T>, p.M, 256, 0, p)));
   MX_DONE(1);
 }
 
 // ---------------------------------------------------------------------------------------------- h + conv(h) over time
 template <typename T>
 __global__ void __launch_bounds__(256) canon_conv_kernel(const CanonConv p) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int m = blockIdx.x, b = m / p.S, t = m % p.S, back = p.taps - 1;
   const T *w = reinterpret_cast<const T *>(p.w);
   const float *hist = p.hist + (size_t)b * back * p.n;
@@ -1484,6 +1560,8 @@ __global__ void __launch_bounds__(256) canon_conv_kernel(const CanonConv p) {
 constexpr int CC_TOK = 16, CC_MAXT = 8;
 template <typename T>
 __global__ void __launch_bounds__(128) canon_conv_vec_kernel(const CanonConv p) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int c4 = blockIdx.y * blockDim.x + threadIdx.x;
   if (c4 >= p.n / 4) return;
   const int ch = c4 * 4, chunks = (p.S + CC_TOK - 1) / CC_TOK, b = blockIdx.x / chunks, t0 = (blockIdx.x % chunks) * CC_TOK, back = p.taps - 1;
@@ -1526,6 +1604,8 @@ __global__ void __launch_bounds__(128) canon_conv_vec_kernel(const CanonConv p) 
 }
 // afterwards: the history becomes the last taps - 1 inputs up to the end of this step (zeros before position 0)
 __global__ void canon_hist_kernel(const CanonConv p) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int idx = blockIdx.x * blockDim.x + threadIdx.x, back = p.taps - 1;
   if (idx >= p.B * p.n) return;
   const int b = idx / p.n, ch = idx % p.n;
@@ -1542,16 +1622,18 @@ int canon_conv(cudaStream_t st, int dtype, const CanonConv &p, uint64_t *launche
   if (p.taps < 1 || p.B < 1 || p.S < 1) return (int)cudaErrorInvalidValue;
   const bool vec = p.n % 4 == 0 && p.taps <= CC_MAXT && (((uintptr_t)p.h | (uintptr_t)p.hist | (uintptr_t)p.out) & 15) == 0;
   MX_DISPATCH(dtype, {
-    if (vec) canon_conv_vec_kernel<T><<<dim3(p.B * ((p.S + CC_TOK - 1) / CC_TOK), (p.n / 4 + 127) / 128), 128, 0, st>>>(p);
-    else canon_conv_kernel<T><<<dim3(p.B * p.S, (p.n + 255) / 256), 256, 0, st>>>(p);
+    if (vec) mx_launch(st, canon_conv_vec_kernel<T>, dim3(p.B * ((p.S + CC_TOK - 1) / CC_TOK), (p.n / 4 + 127) / 128), 128, 0, p);
+    else mx_launch(st, canon_conv_kernel<T>, dim3(p.B * p.S, (p.n + 255) / 256), 256, 0, p);
   });
-  if (p.taps > 1) canon_hist_kernel<<<(p.B * p.n + 255) / 256, 256, 0, st>>>(p);
+  if (p.taps > 1) mx_launch(st, canon_hist_kernel, (p.B * p.n + 255) / 256, 256, 0, p);
   MX_DONE(p.taps > 1 ? 2 : 1);
 }
 
 // ---------------------------------------------------------------------------------------------- sublayer output -> stream
 template <typename T>
 __global__ void __launch_bounds__(256) branch_merge_kernel(const BranchMerge p) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float ys[];  // [n]
   __shared__ float red[64];
   const int m = blockIdx.x, n = p.n;
@@ -1597,7 +1679,7 @@ int branch_merge(cudaStream_t st, int dtype, const BranchMerge &p, uint64_t *lau
       cudaError_t e = cudaFuncSetAttribute(branch_merge_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return (int)e;
     }
-    branch_merge_kernel<T><<<p.M, 256, smem, st>>>(p);
+    mx_launch(st, branch_merge_kernel<T>, p.M, 256, smem, p);
   });
   MX_DONE(1);
 }
@@ -1619,6 +1701,8 @@ template <typename T> __device__ __forceinline__ float4 merge_load(const StreamM
 }
 template <typename T, int NV>
 __global__ void __launch_bounds__(256) stream_merge_kernel(const StreamMerge p) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float red[64];
   const int m = blockIdx.x, n4 = p.n / 4;
   const T *post = reinterpret_cast<const T *>(p.post);
@@ -1656,6 +1740,8 @@ __global__ void __launch_bounds__(256) stream_merge_kernel(const StreamMerge p) 
 }
 template <typename T>
 __global__ void __launch_bounds__(256) stream_merge_any_kernel(const StreamMerge p) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float ys[];  // [n]
   __shared__ float red[64];
   const int m = blockIdx.x;
@@ -1694,11 +1780,11 @@ int stream_merge(cudaStream_t st, int dtype, const StreamMerge &p, uint64_t *lau
         cudaError_t e = cudaFuncSetAttribute(stream_merge_any_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
       }
-      stream_merge_any_kernel<T><<<p.M, 256, smem, st>>>(p);
-    } else if (p.n <= 1024) stream_merge_kernel<T, 1><<<p.M, 256, 0, st>>>(p);
-    else if (p.n <= 2048) stream_merge_kernel<T, 2><<<p.M, 256, 0, st>>>(p);
-    else if (p.n <= 4096) stream_merge_kernel<T, 4><<<p.M, 256, 0, st>>>(p);
-    else stream_merge_kernel<T, 8><<<p.M, 256, 0, st>>>(p);
+      mx_launch(st, stream_merge_any_kernel<T>, p.M, 256, smem, p);
+    } else if (p.n <= 1024) mx_launch(st, stream_merge_kernel<T, 1>, p.M, 256, 0, p);
+    else if (p.n <= 2048) mx_launch(st, stream_merge_kernel<T, 2>, p.M, 256, 0, p);
+    else if (p.n <= 4096) mx_launch(st, stream_merge_kernel<T, 4>, p.M, 256, 0, p);
+    else mx_launch(st, stream_merge_kernel<T, 8>, p.M, 256, 0, p);
   });
   MX_DONE(1);
 }
@@ -1706,6 +1792,8 @@ int stream_merge(cudaStream_t st, int dtype, const StreamMerge &p, uint64_t *lau
 // ---------------------------------------------------------------------------------------------- gated delta rule
 template <typename T>
 __global__ void __launch_bounds__(128) delta_prep_kernel(const DeltaPrep p) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int m = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int G = p.kv_heads, dk = p.dk;
   for (int item = warp; item < 2 * G; item += nw) {
@@ -1731,7 +1819,7 @@ __global__ void __launch_bounds__(128) delta_prep_kernel(const DeltaPrep p) {
 }
 int delta_prep(cudaStream_t st, int dtype, const DeltaPrep &p, uint64_t *launches) {
   if (p.M < 1 || p.heads < 1 || p.kv_heads < 1 || p.dk < 1) return (int)cudaErrorInvalidValue;
-  MX_DISPATCH(dtype, (delta_prep_kernel<T><<<p.M, 128, 0, st>>>(p)));
+  MX_DISPATCH(dtype, (mx_launch(st, delta_prep_kernel<T>, p.M, 128, 0, p)));
   MX_DONE(1);
 }
 
@@ -1742,6 +1830,8 @@ int delta_prep(cudaStream_t st, int dtype, const DeltaPrep &p, uint64_t *launche
 constexpr int DR_TT = 16, DR_CB = 32;
 template <typename T, int R, int RS>
 __global__ void __launch_bounds__(DR_CB * RS) delta_rule_kernel(const DeltaRule p) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float sm[];
   // a lane's slice of a staged q / k row starts R + 4 floats after its neighbour's: the eight 16-byte reads of a quarter-warp
   // then fall into different banks
@@ -1816,6 +1906,8 @@ __global__ void __launch_bounds__(DR_CB * RS) delta_rule_kernel(const DeltaRule 
 // Shared-memory form for any dk: a thread owns one column, which sits in shared memory.
 template <typename T>
 __global__ void __launch_bounds__(DR_CB) delta_rule_smem_kernel(const DeltaRule p) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float sm[];
   const int dk = p.dk, dv = p.dv, ld = (dk + 3) / 4 * 4;
   float *qs = sm, *ks = qs + DR_TT * ld, *vs = ks + DR_TT * ld, *gs = vs + DR_TT * DR_CB, *bs = gs + DR_TT, *Ss = bs + DR_TT;
@@ -1867,7 +1959,7 @@ __global__ void __launch_bounds__(DR_CB) delta_rule_smem_kernel(const DeltaRule 
 }
 template <typename T, int R, int RS> static cudaError_t launch_delta_rule(cudaStream_t st, const DeltaRule &p) {
   const size_t smem = ((size_t)2 * DR_TT * (RS > 1 ? R + 4 : R) * RS + (size_t)DR_TT * DR_CB + 2 * DR_TT) * sizeof(float);
-  delta_rule_kernel<T, R, RS><<<dim3(p.heads * ((p.dv + DR_CB - 1) / DR_CB), p.B), DR_CB * RS, smem, st>>>(p);
+  mx_launch_if(p.S <= MX_EARLY_TOKENS, st, delta_rule_kernel<T, R, RS>, dim3(p.heads * ((p.dv + DR_CB - 1) / DR_CB), p.B), DR_CB * RS, smem, p);
   return cudaSuccess;
 }
 template <typename T> static cudaError_t launch_delta_rule_smem(cudaStream_t st, const DeltaRule &p) {
@@ -1878,7 +1970,7 @@ template <typename T> static cudaError_t launch_delta_rule_smem(cudaStream_t st,
     cudaError_t e = cudaFuncSetAttribute(delta_rule_smem_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  delta_rule_smem_kernel<T><<<dim3(p.heads * ((p.dv + DR_CB - 1) / DR_CB), p.B), DR_CB, smem, st>>>(p);
+  mx_launch_if(p.S <= MX_EARLY_TOKENS, st, delta_rule_smem_kernel<T>, dim3(p.heads * ((p.dv + DR_CB - 1) / DR_CB), p.B), DR_CB, smem, p);
   return cudaSuccess;
 }
 int delta_rule(cudaStream_t st, int dtype, const DeltaRule &p, uint64_t *launches) {
@@ -1903,6 +1995,8 @@ int delta_rule(cudaStream_t st, int dtype, const DeltaRule &p, uint64_t *launche
 constexpr int GP_TT = 32, GP_THREADS = 128, GP_NE = 8;
 template <typename T>
 __global__ void __launch_bounds__(GP_THREADS) gate_prep_kernel(const GatePrep p) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float sm[];
   const int h = blockIdx.x, b = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, dk = p.dk;
   float *ns = sm, *ks = ns + dk, *qs = ks + GP_TT * dk, *as = qs + GP_TT * dk, *bs = as + GP_TT, *es = bs + GP_TT, *dots = es + GP_TT;
@@ -2034,7 +2128,7 @@ int gate_prep(cudaStream_t st, int dtype, const GatePrep &p, uint64_t *launches)
       cudaError_t e = cudaFuncSetAttribute(gate_prep_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return (int)e;
     }
-    gate_prep_kernel<T><<<dim3(p.heads, p.B), GP_THREADS, smem, st>>>(p);
+    mx_launch(st, gate_prep_kernel<T>, dim3(p.heads, p.B), GP_THREADS, smem, p);
   });
   MX_DONE(1);
 }
@@ -2090,6 +2184,8 @@ __device__ __forceinline__ void key_scores8(const T *__restrict__ krow, const fl
 constexpr int TA_MAXO = 16;
 template <typename T, int PHASE>
 __global__ void __launch_bounds__(256) talk_attn_kernel(const TalkAttn p) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float sm[];
   const int NT = blockDim.x, H = p.heads, G = p.kv_heads, dim = p.dim, vdim = p.vdim, grp = H / G;
   float *qs = sm, *M_ = qs + (size_t)H * dim, *L_ = M_ + H, *tk = L_ + H, *ta = tk + H * H, *tb = ta + (size_t)H * NT;
@@ -2251,6 +2347,8 @@ __global__ void __launch_bounds__(256) talk_attn_kernel(const TalkAttn p) {
 // the split form's last step: the key ranges' partial outputs are added in range order, gated and stored in D
 template <typename T>
 __global__ void __launch_bounds__(256) talk_attn_merge_kernel(const TalkAttn p) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int m = blockIdx.x, n_out = p.heads * p.vdim, ns = p.nsplit;
   const float *part = p.part + (size_t)p.B * p.S * ns * p.heads * 2 + (size_t)m * ns * n_out;
   for (int idx = threadIdx.x; idx < n_out; idx += blockDim.x) {
@@ -2276,11 +2374,11 @@ int talk_attention(cudaStream_t st, int dtype, const TalkAttn &p, uint64_t *laun
       if (e == cudaSuccess) e = cudaFuncSetAttribute(talk_attn_kernel<T, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return (int)e;
     }
-    if (!split) talk_attn_kernel<T, 0><<<M, NT, smem, st>>>(p);
+    if (!split) mx_launch(st, talk_attn_kernel<T, 0>, M, NT, smem, p);
     else {
-      talk_attn_kernel<T, 1><<<dim3(M, p.nsplit), NT, smem, st>>>(p);
-      talk_attn_kernel<T, 2><<<dim3(M, p.nsplit), NT, smem, st>>>(p);
-      talk_attn_merge_kernel<T><<<M, 256, 0, st>>>(p);
+      mx_launch(st, talk_attn_kernel<T, 1>, dim3(M, p.nsplit), NT, smem, p);
+      mx_launch(st, talk_attn_kernel<T, 2>, dim3(M, p.nsplit), NT, smem, p);
+      mx_launch(st, talk_attn_merge_kernel<T>, M, 256, 0, p);
     }
   });
   MX_DONE(split ? 3 : 1);
@@ -2289,6 +2387,8 @@ int talk_attention(cudaStream_t st, int dtype, const TalkAttn &p, uint64_t *laun
 // ---- the matrix-product form: softmax + head mixing between the two products
 // pass 1: a warp per (head, token) row: maximum and sum of exp over the keys the token sees
 __global__ void __launch_bounds__(256) talk_softmax_stats_kernel(const TalkSoftmax p) {
+  pdl_launch_dependents();
+  pdl_wait();
   const long row = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (row >= (long)p.heads * p.n_tok) return;
@@ -2313,6 +2413,8 @@ __global__ void __launch_bounds__(256) talk_softmax_stats_kernel(const TalkSoftm
 // keys, and hi and lo leave as 8-byte stores
 template <typename T, int HP>
 __global__ void __launch_bounds__(256) talk_softmax_mix_regs_kernel(const TalkSoftmax p) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ __align__(16) float tk[HP * HP];
   __shared__ float M_[HP], L_[HP];
   const int H = p.heads, NT = blockDim.x, t = blockIdx.x, pos = p.pos_first + t;
@@ -2378,6 +2480,8 @@ __global__ void __launch_bounds__(256) talk_softmax_mix_regs_kernel(const TalkSo
 // pass 2: a CTA per token: every thread normalises the scores of its keys for all heads, mixes them and stores hi | lo
 template <typename T>
 __global__ void __launch_bounds__(256) talk_softmax_mix_kernel(const TalkSoftmax p) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float sm[];
   const int H = p.heads, NT = blockDim.x, t = blockIdx.x, pos = p.pos_first + t;
   float *M_ = sm, *L_ = M_ + H, *tk = L_ + H, *pg = tk + H * H;   // pg[g * NT + tid]
@@ -2417,33 +2521,37 @@ int talk_softmax(cudaStream_t st, int dtype, const TalkSoftmax &p, uint64_t *lau
   const long rows = (long)p.heads * p.n_tok;
   const size_t smem = ((size_t)2 * p.heads + (size_t)p.heads * p.heads + (size_t)p.heads * 256) * sizeof(float);
   if (smem > 200 * 1024) return (int)cudaErrorInvalidValue;
-  talk_softmax_stats_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(p);
+  mx_launch(st, talk_softmax_stats_kernel, (unsigned)((rows + 7) / 8), 256, 0, p);
   MX_DISPATCH(dtype, {
-    if (p.heads <= 4) talk_softmax_mix_regs_kernel<T, 4><<<p.n_tok, 256, 0, st>>>(p);
-    else if (p.heads <= 8) talk_softmax_mix_regs_kernel<T, 8><<<p.n_tok, 256, 0, st>>>(p);
-    else if (p.heads <= 16) talk_softmax_mix_regs_kernel<T, 16><<<p.n_tok, 256, 0, st>>>(p);
-    else if (p.heads <= 32) talk_softmax_mix_regs_kernel<T, 32><<<p.n_tok, 256, 0, st>>>(p);
+    if (p.heads <= 4) mx_launch(st, talk_softmax_mix_regs_kernel<T, 4>, p.n_tok, 256, 0, p);
+    else if (p.heads <= 8) mx_launch(st, talk_softmax_mix_regs_kernel<T, 8>, p.n_tok, 256, 0, p);
+    else if (p.heads <= 16) mx_launch(st, talk_softmax_mix_regs_kernel<T, 16>, p.n_tok, 256, 0, p);
+    else if (p.heads <= 32) mx_launch(st, talk_softmax_mix_regs_kernel<T, 32>, p.n_tok, 256, 0, p);
     else {
       if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(talk_softmax_mix_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
       }
-      talk_softmax_mix_kernel<T><<<p.n_tok, 256, smem, st>>>(p);
+      mx_launch(st, talk_softmax_mix_kernel<T>, p.n_tok, 256, smem, p);
     }
   });
   MX_DONE(2);
 }
 template <typename T>
 __global__ void rows_by_head_kernel(const T *__restrict__ src, int ld, T *__restrict__ dst, int n_tok, int heads, int dim) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int t = blockIdx.x;
   for (int i = threadIdx.x; i < heads * dim; i += blockDim.x) dst[((size_t)(i / dim) * n_tok + t) * dim + i % dim] = src[(size_t)t * ld + i];
 }
 int rows_by_head(cudaStream_t st, int dtype, const void *src, int ld, void *dst, int n_tok, int heads, int dim, uint64_t *launches) {
-  MX_DISPATCH(dtype, (rows_by_head_kernel<T><<<n_tok, 256, 0, st>>>(reinterpret_cast<const T *>(src), ld, reinterpret_cast<T *>(dst), n_tok, heads, dim)));
+  MX_DISPATCH(dtype, (mx_launch(st, rows_by_head_kernel<T>, n_tok, 256, 0, reinterpret_cast<const T *>(src), ld, reinterpret_cast<T *>(dst), n_tok, heads, dim)));
   MX_DONE(1);
 }
 template <typename T>
 __global__ void rows_to_tokens_kernel(const T *__restrict__ o, const T *__restrict__ gate, int ldg, T *__restrict__ out, int ldo, int n_tok, int heads, int vdim) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int t = blockIdx.x;
   for (int i = threadIdx.x; i < heads * vdim; i += blockDim.x) {
     float v = DT<T>::to_f(o[((size_t)(i / vdim) * n_tok + t) * vdim + i % vdim]);
@@ -2453,13 +2561,15 @@ __global__ void rows_to_tokens_kernel(const T *__restrict__ o, const T *__restri
 }
 int rows_to_tokens(cudaStream_t st, int dtype, const void *o, const void *gate, int ldg, void *out, int ldo, int n_tok, int heads, int vdim,
                    uint64_t *launches) {
-  MX_DISPATCH(dtype, (rows_to_tokens_kernel<T><<<n_tok, 256, 0, st>>>(reinterpret_cast<const T *>(o), reinterpret_cast<const T *>(gate), ldg,
+  MX_DISPATCH(dtype, (mx_launch(st, rows_to_tokens_kernel<T>, n_tok, 256, 0, reinterpret_cast<const T *>(o), reinterpret_cast<const T *>(gate), ldg,
                                                                        reinterpret_cast<T *>(out), ldo, n_tok, heads, vdim)));
   MX_DONE(1);
 }
 // a CTA transposes a tile of 32 tokens x 32 value entries through shared memory, so that reads and writes are both contiguous
 template <typename T>
 __global__ void values_transposed_kernel(const T *__restrict__ src, int ld, int col0, T *__restrict__ vt, int S, int kv_heads, int vdim, int cap_t, int pos0) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ T tile[32][33];
   const int b = blockIdx.z, t0 = blockIdx.x * 32, e0 = blockIdx.y * 32, n = kv_heads * vdim;
   for (int r = threadIdx.y; r < 32; r += blockDim.y) {
@@ -2475,26 +2585,30 @@ __global__ void values_transposed_kernel(const T *__restrict__ src, int ld, int 
 int values_transposed_append(cudaStream_t st, int dtype, const void *src, int ld, int col0, void *vt, int B, int S, int kv_heads, int vdim, int cap_t,
                              int pos0, uint64_t *launches) {
   const dim3 grid((S + 31) / 32, (kv_heads * vdim + 31) / 32, B), block(32, 8);
-  MX_DISPATCH(dtype, (values_transposed_kernel<T><<<grid, block, 0, st>>>(reinterpret_cast<const T *>(src), ld, col0, reinterpret_cast<T *>(vt), S, kv_heads,
+  MX_DISPATCH(dtype, (mx_launch(st, values_transposed_kernel<T>, grid, block, 0, reinterpret_cast<const T *>(src), ld, col0, reinterpret_cast<T *>(vt), S, kv_heads,
                                                                           vdim, cap_t, pos0)));
   MX_DONE(1);
 }
 
 template <typename T>
 __global__ void distance_bias_kernel(const T *__restrict__ rel, const int *__restrict__ bucket, float *__restrict__ bias, int len, int heads) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= len * heads) return;
   bias[idx] = DT<T>::to_f(rel[(size_t)bucket[idx / heads] * heads + idx % heads]);
 }
 int distance_bias_table(cudaStream_t st, int dtype, const void *rel, const int *bucket, float *bias, int len, int heads, uint64_t *launches) {
   if (len < 1 || heads < 1) return (int)cudaErrorInvalidValue;
-  MX_DISPATCH(dtype, (distance_bias_kernel<T><<<(len * heads + 255) / 256, 256, 0, st>>>(reinterpret_cast<const T *>(rel), bucket, bias, len, heads)));
+  MX_DISPATCH(dtype, (mx_launch(st, distance_bias_kernel<T>, (len * heads + 255) / 256, 256, 0, reinterpret_cast<const T *>(rel), bucket, bias, len, heads)));
   MX_DONE(1);
 }
 
 // ---------------------------------------------------------------------------------------------- embedding with tables
 template <typename T>
 __global__ void __launch_bounds__(128) embed_tables_kernel(const EmbedTables p) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int r = blockIdx.x, b = r / p.S, t = r % p.S;
   uint32_t id = p.ids[r];
   if (id >= (uint32_t)p.vocab) id = 0;
@@ -2519,13 +2633,15 @@ __global__ void __launch_bounds__(128) embed_tables_kernel(const EmbedTables p) 
 }
 int embed_tables(cudaStream_t st, int dtype, const EmbedTables &p, uint64_t *launches) {
   if (p.B < 1 || p.S < 1 || (p.bigram && p.buckets < 1)) return (int)cudaErrorInvalidValue;
-  MX_DISPATCH(dtype, (embed_tables_kernel<T><<<p.B * p.S, 128, 0, st>>>(p)));
+  MX_DISPATCH(dtype, (mx_launch(st, embed_tables_kernel<T>, p.B * p.S, 128, 0, p)));
   MX_DONE(1);
 }
 // token row, RMS norm over the width with a gain
 template <typename T>
 __global__ void __launch_bounds__(256) embed_norm_kernel(const T *__restrict__ E, const uint32_t *__restrict__ ids, const T *__restrict__ w,
                                                          float *__restrict__ x, int W, float scale, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float red[64];
   const T *row = E + (size_t)ids[blockIdx.x] * W;
   float *out = x + (size_t)blockIdx.x * W;
@@ -2542,6 +2658,8 @@ __global__ void __launch_bounds__(256) embed_norm_kernel(const T *__restrict__ E
 template <typename T, int NV>
 __global__ void __launch_bounds__(256) embed_norm_vec_kernel(const T *__restrict__ E, const uint32_t *__restrict__ ids, const T *__restrict__ w,
                                                              float *__restrict__ x, int W, float scale, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float red[64];
   const T *row = E + (size_t)ids[blockIdx.x] * W;
   float4 *out = reinterpret_cast<float4 *>(x + (size_t)blockIdx.x * W);
@@ -2575,11 +2693,11 @@ int embed_norm(cudaStream_t st, int dtype, const void *E, const uint32_t *ids, c
   const bool vec = W % 4 == 0 && W <= 8192 && (((uintptr_t)E | (uintptr_t)w | (uintptr_t)x) & 15) == 0;
   MX_DISPATCH(dtype, {
     const T *e = reinterpret_cast<const T *>(E), *g = reinterpret_cast<const T *>(w);
-    if (!vec) embed_norm_kernel<T><<<M, 256, 0, st>>>(e, ids, g, x, W, sc, eps);
-    else if (W <= 1024) embed_norm_vec_kernel<T, 1><<<M, 256, 0, st>>>(e, ids, g, x, W, sc, eps);
-    else if (W <= 2048) embed_norm_vec_kernel<T, 2><<<M, 256, 0, st>>>(e, ids, g, x, W, sc, eps);
-    else if (W <= 4096) embed_norm_vec_kernel<T, 4><<<M, 256, 0, st>>>(e, ids, g, x, W, sc, eps);
-    else embed_norm_vec_kernel<T, 8><<<M, 256, 0, st>>>(e, ids, g, x, W, sc, eps);
+    if (!vec) mx_launch(st, embed_norm_kernel<T>, M, 256, 0, e, ids, g, x, W, sc, eps);
+    else if (W <= 1024) mx_launch(st, embed_norm_vec_kernel<T, 1>, M, 256, 0, e, ids, g, x, W, sc, eps);
+    else if (W <= 2048) mx_launch(st, embed_norm_vec_kernel<T, 2>, M, 256, 0, e, ids, g, x, W, sc, eps);
+    else if (W <= 4096) mx_launch(st, embed_norm_vec_kernel<T, 4>, M, 256, 0, e, ids, g, x, W, sc, eps);
+    else mx_launch(st, embed_norm_vec_kernel<T, 8>, M, 256, 0, e, ids, g, x, W, sc, eps);
   });
   MX_DONE(1);
 }
@@ -2587,6 +2705,8 @@ int embed_norm(cudaStream_t st, int dtype, const void *E, const uint32_t *ids, c
 // ---------------------------------------------------------------------------------------------- stream injection
 template <typename T>
 __global__ void __launch_bounds__(256) stream_inject_kernel(float *x, const float *x0, const T *vec, int W) {
+  pdl_launch_dependents();
+  pdl_wait();
   const size_t m = blockIdx.x;
   for (int i = threadIdx.x; i < W; i += blockDim.x) {
     float v = x[m * W + i];
@@ -2595,7 +2715,7 @@ __global__ void __launch_bounds__(256) stream_inject_kernel(float *x, const floa
   }
 }
 int stream_inject(cudaStream_t st, int dtype, float *x, const float *x0, const void *vec, int M, int W, uint64_t *launches) {
-  MX_DISPATCH(dtype, (stream_inject_kernel<T><<<M, 256, 0, st>>>(x, x0, reinterpret_cast<const T *>(vec), W)));
+  MX_DISPATCH(dtype, (mx_launch(st, stream_inject_kernel<T>, M, 256, 0, x, x0, reinterpret_cast<const T *>(vec), W)));
   MX_DONE(1);
 }
 
