@@ -59,7 +59,8 @@ __device__ __forceinline__ float sample_uniform(const SampleArgs &s, unsigned st
 // Bound: latency, not bytes (300 KB of logits): one CTA took 31 bisection passes of 125 dependent loads each over the vocabulary, 380 us for
 // 128256 entries.  The vocabulary is cut between the CTAs of a cluster, which keep their probabilities in shared memory; a pass looks
 // at seven thresholds at once and its sums meet over the cluster; the thresholds are logits, whose 16 bits take six passes (a
-// probability's 30 bits took ten: 97 us).
+// probability's 30 bits took ten: 97 us).  A nucleus is searched between the largest logit and where it can end, three passes, entries below a pass's
+// lowest threshold are passed over, and the logits are read 16 bytes at a time: the call 95 -> 77 us at 128256 entries.
 // Every reduction has a fixed order (threads, warps, ranks): a draw is a function of (logits, seed, step).
 struct SampleShared {
   float warp[SAMPLE_THREADS / 32][9];    // a warp's sums (rows of nine: no bank conflicts down a column)
