@@ -2129,7 +2129,7 @@ int gate_prep(cudaStream_t st, int dtype, const GatePrep &p, uint64_t *launches)
       cudaError_t e = cudaFuncSetAttribute(gate_prep_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return (int)e;
     }
-    mx_launch(st, gate_prep_kernel<T>, dim3(p.heads, p.B), GP_THREADS, smem, p);
+    mx_launch_if(p.S <= MX_EARLY_TOKENS, st, gate_prep_kernel<T>, dim3(p.heads, p.B), GP_THREADS, smem, p);
   });
   MX_DONE(1);
 }
