@@ -116,6 +116,19 @@ __host__ __device__ inline size_t mk_xs_bytes(int max_k, int es) {
   return b > attn ? b : attn;  // the attention phase overlays its scratch on the x buffer
 }
 // Shared memory: barriers, stage rows and scratch at fixed places, the ring, then what the model's sizes decide.
+// A thread that is done with a phase begins the next one at once, so an area is reused only where a barrier of the consumers lies between its
+// last reader and its next writer:
+//   x (off_x)        written by a gather.  Its readers in front: a product's loop, which ends with a barrier before the epilogue; attention's queries,
+//                    scores and new rows, all read before the barrier behind the last tile's sums.  The merge of split attention reads on while
+//                    other threads of the CTA gather already, so its parts lie in the partial sums' area and not here.
+//                    Attention writes over x behind the qkv product's barrier.
+//   partial sums     written by a product's loop, behind the barrier of its gather, and by the merge of attention, behind attention's first barriers: all
+//                    epilogues (and the merge) are over when the CTA's threads have met there.  Batches of one product: the barrier behind an epilogue.
+//   loc (off_loc)    as the partial sums.
+//   residual copy    written by the gathers of qkv and gate_up without a barrier in front: an epilogue reads row r before it publishes r, and a gather writes
+//                    over r only when it has seen that packet.
+//   scratch          a warp's sum of squares: written in front of a gather's barrier, read behind it, and the next one is written after at least
+//                    one product's barriers; the head's winners: behind the last product's barrier.
 constexpr int MK_OFF_EMPTY = 8 * MK_MAX_STAGES, MK_OFF_STAGE_ROW = 16 * MK_MAX_STAGES, MK_OFF_SCRATCH = 256, MK_OFF_RING = 1024;
 inline size_t mk_layout(MkArgs &a, int es) {
   size_t off = MK_OFF_RING + (size_t)a.n_stages * MK_STAGE_BYTES;
@@ -126,7 +139,7 @@ inline size_t mk_layout(MkArgs &a, int es) {
   };
   a.off_x = take(mk_xs_bytes(a.max_k, es));
   a.off_res = take(a.keep_x ? (size_t)a.hidden * es : 0);
-  a.off_part = take(MK_BATCH * MK_CW * 4);  // partial sums [row][warp of the row]
+  a.off_part = take(MK_BATCH * MK_CW * 4);  // partial sums [row][warp of the row]; the parts that the merge of split attention gathers
   a.off_loc = take(MK_BATCH * 4);           // first row of each group of a batch
   a.off_rows = take((size_t)a.n_layers * sizeof(MkRow));
   return off;
@@ -769,7 +782,7 @@ __device__ __forceinline__ void mk_norm_rope(float *buf, bool norm, const float 
 // state lives in registers.  The heads' packets are polled by the warps that norm and rotate them.  One split: its result is the output.
 // Several: each publishes its columns, maximum and sum as packets, and each merges its share of the columns of all of them, in split order.
 template <typename T, int HD, int G>
-__device__ __forceinline__ void mk_consume_attn(MkRing &rg, const MkArgs &a, const MkRow &L, int pos, unsigned char *scr,
+__device__ __forceinline__ void mk_consume_attn(MkRing &rg, const MkArgs &a, const MkRow &L, int pos, unsigned char *scr, float *parts,
                                                 const float *rope_cs, uint32_t tag32, int &left, unsigned long long *tr) {
   const int ct = threadIdx.x, warp = ct >> 5, lane = ct & 31;
   const uint32_t tag = tag32 << 16;
@@ -786,7 +799,7 @@ __device__ __forceinline__ void mk_consume_attn(MkRing &rg, const MkArgs &a, con
   const int ws = (a.window > 0 && pos + 1 > a.window) ? pos + 1 - a.window : 0;
   pos -= ws;
   const MkAttnItem it = mk_attn_item(a, pos, (int)sizeof(T));
-  float *q_s = reinterpret_cast<float *>(scr);             // [G][HD]; then the parts of a merge
+  float *q_s = reinterpret_cast<float *>(scr);             // [G][HD]
   float *sc = q_s + ATTN_MAX_G * 256;                      // [ATTN_TILE][G]  (position-major: one vector per position)
   float *knew = sc + ATTN_MAX_G * ATTN_TILE;               // [2][HD] appended k / v row
   __shared__ float m_run[ATTN_MAX_G], l_run[ATTN_MAX_G], fac[ATTN_MAX_G];
@@ -973,9 +986,11 @@ __device__ __forceinline__ void mk_consume_attn(MkRing &rg, const MkArgs &a, con
   if (lane == 0) { mbar_arrive(ek); mbar_arrive(ev); }
   stamp(6);
   if (ns > 1) {
-    // ---- merge: this split's share of the columns; (column, split) pairs are contiguous, a thread polls one or a few of them
+    // ---- merge: this split's share of the columns; (column, split) pairs are contiguous, a thread polls one or a few of them.  The first warps have all
+    // columns: the others gather the o product's input (over scr) while these still read `parts` and `wgt`.
+    static_assert(G * HD + ATTN_MAX_SPLIT <= MK_BATCH * MK_CW, "the parts of a merge");
     const int c0 = G * HD * split / ns, nc = G * HD * (split + 1) / ns - c0, np = nc * ns;
-    for (int i = ct; i < np; i += MK_CT) q_s[i] = pk_poll64(pacc + (size_t)c0 * ns + i, tag32, wt);
+    for (int i = ct; i < np; i += MK_CT) parts[i] = pk_poll64(pacc + (size_t)c0 * ns + i, tag32, wt);
     for (int g = warp; g < G; g += NW) {
       float m = -INFINITY, l = 0.f;
       if (lane < ns) {
@@ -991,7 +1006,7 @@ __device__ __forceinline__ void mk_consume_attn(MkRing &rg, const MkArgs &a, con
     for (int i = ct; i < nc; i += MK_CT) {
       const int g = (c0 + i) / HD;
       float o = 0.f;
-      for (int s2 = 0; s2 < ns; s2++) o = fmaf(wgt[g][s2], q_s[i * ns + s2], o);
+      for (int s2 = 0; s2 < ns; s2++) o = fmaf(wgt[g][s2], parts[i * ns + s2], o);
       pk_store<T>(a.pk.y + (size_t)kvh * G * HD + c0 + i, DT<T>::from_f(o), tag);
     }
   }
@@ -1097,7 +1112,8 @@ __global__ void __launch_bounds__(MK_THREADS, 1) decode_mega_kernel(const __grid
       if (l == a.n_layers) break;
       if (ph == 0) {  // qk-norm, RoPE, KV append, attention
         mk_stamp(a, l, 0, 2);
-        mk_consume_attn<T, HD, G>(rg, a, reinterpret_cast<const MkRow *>(smem_raw + a.off_rows)[l], pos, smem_raw + a.off_x, rope_cs, tag32, left,
+        mk_consume_attn<T, HD, G>(rg, a, reinterpret_cast<const MkRow *>(smem_raw + a.off_rows)[l], pos, smem_raw + a.off_x,
+                                  reinterpret_cast<float *>(smem_raw + a.off_part), rope_cs, tag32, left,
                                   a.trace && blockIdx.x == 0 && l == 1 ? a.trace + 2048 : nullptr);
         mk_stamp(a, l, 0, 3);
       }

@@ -45,3 +45,33 @@ def test_steps_equal_the_chain_of_kernels(shape, monkeypatch):
     for a, b in zip(outs["0"], outs["1"]):
         assert torch.isfinite(a.float()).all()
         assert max_ulp_err(to_np(a), to_np(b), dtype) <= 2.0
+
+
+@pytest.mark.parametrize("hidden,heads,kv,hd,dtype", [(1024, 16, 2, 128, "bf16"), (4096, 32, 4, 128, "f16"), (512, 8, 2, 64, "f16"), (192, 4, 2, 16, "bf16")])
+def test_attention_cut_over_many_ctas_repeats_itself(hidden, heads, kv, hd, dtype, monkeypatch):
+    """2, 16 to 17 and 32 CTAs per key head (the most): a few threads of a CTA merge the parts while the others gather the next product's input, so every
+    run has the same bits, and they are those of the chain of kernels up to the order of sums."""
+    cfg = Config(hidden_size=hidden, intermediate_size=1024, vocab_size=384, num_hidden_layers=LAYERS, num_attention_heads=heads,
+                 num_key_value_heads=kv, rms_norm_eps=1e-5, rope_theta=10000.0, max_seq_len=4096, head_dim=hd)
+    sd = checkpoint(cfg, dtype, seed=12, std=0.7 * hidden ** -0.5)
+    outs = {}
+    for mode, runs in (("1", 1), ("0", 25)):
+        monkeypatch.setenv("CAKE_B200_PER_OP", mode)
+        ctx = Context(cfg, sd, dtype)
+        blocks = [B200Transformer.load(cfg.layer_name(i), ctx) for i in range(LAYERS)]
+        outs[mode] = []
+        for pos in (129, 1030, 2047, 2300):
+            ctx.cache = Cache(ctx, 1, pos + 1)
+            ctx.cache.fill_synthetic(range(LAYERS), pos, 5)
+            x = ctx.to_device(rand_x((1, 1, hidden), dtype, seed=pos))
+            ys = []
+            for _ in range(runs):   # (the step writes its own position's key and value: the same ones each time)
+                ctx.cache.fill_synthetic(range(LAYERS), pos, 5)
+                ys.append(blocks[0].forward_batch(x, [(b.layer_name(), pos, i) for i, b in enumerate(blocks)], ctx, blocks=blocks))
+            ctx.sync()
+            assert all(torch.equal(y, ys[0]) for y in ys[1:]), pos
+            outs[mode].append(ys[0].cpu())
+        ctx.close()
+    for a, b in zip(outs["0"], outs["1"]):
+        assert torch.isfinite(a.float()).all()
+        assert max_ulp_err(to_np(a), to_np(b), dtype) <= 2.0
