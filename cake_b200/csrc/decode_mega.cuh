@@ -18,7 +18,8 @@
 // Bound by HBM where a layer's weights are large (8B: 436 MB a layer) and by the chain of five exchanges per layer where they are not
 // (0.6B: 31 MB, 5 us of stream).  With grid barriers and fp32 conversions in 16 warps: 32 us a layer at 0.6B, 24 tokens 25.1 ms, 8B two layers 187 us; now
 // 15 us, 14.1 ms and 182 us.  An exchange is 1.0 to 1.5 us (a barrier with the staging behind it 3 to 4.5), a product of 12 MB 2.1 us behind it.
-// Arithmetic and rounding points are identical to the per-op kernels (gemv.cuh / attn_decode.cuh); only the
+// Arithmetic and rounding points are identical to the per-op kernels (gemv.cuh / attn_decode.cuh), correctly rounded divisions and square roots
+// included (a Newton step on the fast instructions in their place saved 0.3 of 14.3 ms over 24 tokens and was an ulp off in places); only the
 // fp32 summation order within a dot product differs (tests/test_gpu_parity.py::test_megakernel_equals_per_op_kernels).
 //
 // A packet buffer is written again one layer later; no reader may still be in front of it.  A CTA that has not gathered the input of
@@ -50,7 +51,6 @@ struct MkGeom {  // one decode GEMV type; a stage holds 2^RSL row segments of KC
   int n_groups, batch;         // groups of 2^RSL rows; groups between two epilogues
   int unit, cnt, rem;          // static groups: CTA c has unit * (cnt + (c < rem)) of them
   int pool;                    // first group of the pool (n_groups: none)
-  float inv_k;                 // 1 / K
 };
 // the vectors that travel as packets (uint32_t: value | tag << 16)
 struct MkPackets {
@@ -174,7 +174,6 @@ struct MkRing {
 // is computed by one CTA with a fixed lane/warp mapping whichever CTA it is -> results stay bit-deterministic.
 constexpr int MK_SHORT = 4;
 inline void mk_plan_split(MkGeom &g, int gran, int grid) {  // gran: rows that stay together (gate and up of a pair)
-  g.inv_k = 1.0f / (float)g.K;
   g.n_groups = (g.N + (1 << g.RSL) - 1) >> g.RSL;
   g.batch = (MK_BATCH >> g.RSL) / g.nchunk;
   if (g.nchunk > 1 || g.n_groups <= MK_SHORT * grid) {
@@ -275,23 +274,6 @@ __device__ __forceinline__ void mk_produce_attn(MkRing &rg, const MkArgs &a, con
       rg.advance();
     }
   }
-}
-
-// Reciprocals and square roots by the fast instruction and one Newton step, to an ulp.  (The correctly rounded forms end in a call for the rare
-// cases, and a call makes the compiler keep what is live around it in local memory.)
-__device__ __forceinline__ float mk_rsqrt(float v) {   // v > 0, or inf
-  const float y = rsqrtf(v), e = fmaf(-v * y, y, 1.0f);
-  return v == INFINITY ? y : fmaf(0.5f * y, e, y);
-}
-__device__ __forceinline__ float mk_rcp(float v) {     // 2^-126 <= |v| < 2^126
-  float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(v));
-  return fmaf(y, fmaf(-v, y, 1.0f), y);
-}
-// gate_act (common.cuh) without the division: below -60 the 1 of 1 + e^-g is far below an ulp, and g e^g the same value
-template <typename T> __device__ __forceinline__ float mk_gate_act(float g, int act) {
-  if (act) return gate_act<T>(g, 1);
-  return rnd<T>(g < -60.f ? g * expf(g) : g * mk_rcp(1.0f + expf(-g)));
 }
 
 // ---------------------------------------------------------------------------------------- packets
@@ -571,7 +553,7 @@ __device__ __forceinline__ void mk_gemv_phase(MkRing &rg, const MkArgs &a, unsig
       const float4 f = reinterpret_cast<const float4 *>(scratch)[i];
       tot += (f.x + f.y) + (f.z + f.w);
     }
-    const float inv = mk_rsqrt(tot * g.inv_k + a.eps);
+    const float inv = 1.0f / sqrtf(tot / (float)g.K + a.eps);
     uint2 *xq = reinterpret_cast<uint2 *>(xs);
 #pragma unroll
     for (int i = 0; i < 4; i++)
@@ -708,7 +690,7 @@ __device__ __forceinline__ void mk_gemv_phase(MkRing &rg, const MkArgs &a, unsig
         pk_store<T>(a.pk.qkv + row, DT<T>::from_f(v), tag);
       } else if (what == 2) {
         const float up = row_sum(li + 1);
-        pk_store<T>(a.pk.mm + row / 2, DT<T>::from_f(mk_gate_act<T>(v, a.act) * up), tag);
+        pk_store<T>(a.pk.mm + row / 2, DT<T>::from_f(gate_act<T>(v, a.act) * up), tag);
       } else {  // + residual
         T q;
         if (a.keep_x) q = res_s[row];
@@ -760,7 +742,7 @@ __device__ __forceinline__ void mk_norm_rope(float *buf, bool norm, const float 
     float ss = 0.f;
     for (int d = lane; d < HD; d += 32) ss += buf[d] * buf[d];
     ss = warp_sum(ss);
-    const float inv = mk_rsqrt(ss * (1.0f / HD) + eps);
+    const float inv = 1.0f / sqrtf(ss / (float)HD + eps);
 #pragma unroll
     for (int i = 0; i < (HD + 31) / 32; i++)
       if (lane + 32 * i < HD) buf[lane + 32 * i] = rnd<T>(buf[lane + 32 * i] * inv * w[i]);
@@ -974,7 +956,7 @@ __device__ __forceinline__ void mk_consume_attn(MkRing &rg, const MkArgs &a, con
     float sum = 0.f;
 #pragma unroll
     for (int w = 0; w < NW; w++) sum += red[(size_t)w * G * HD + i];
-    if (ns == 1) pk_store<T>(a.pk.y + (size_t)kvh * G * HD + i, DT<T>::from_f(sum * mk_rcp(l_run[i / HD])), tag);
+    if (ns == 1) pk_store<T>(a.pk.y + (size_t)kvh * G * HD + i, DT<T>::from_f(sum * (1.0f / l_run[i / HD])), tag);
     else pk_store64(pacc + (size_t)i * ns + split, sum, tag32);
   }
   if (ns > 1 && ct < G) {
@@ -1000,7 +982,7 @@ __device__ __forceinline__ void mk_consume_attn(MkRing &rg, const MkArgs &a, con
       const float M = warp_max(m);
       const float w = (m == -INFINITY) ? 0.f : expf(m - M);
       const float Lsum = warp_sum(w * l);
-      wgt[g][lane] = w * mk_rcp(Lsum);
+      wgt[g][lane] = w / Lsum;
     }
     named_bar_sync(1, MK_CT);
     for (int i = ct; i < nc; i += MK_CT) {

@@ -75,3 +75,53 @@ def test_attention_cut_over_many_ctas_repeats_itself(hidden, heads, kv, hd, dtyp
     for a, b in zip(outs["0"], outs["1"]):
         assert torch.isfinite(a.float()).all()
         assert max_ulp_err(to_np(a), to_np(b), dtype) <= 2.0
+
+
+def _one_hot(n, k, column, scale, dtype):
+    w = torch.zeros(n, k)
+    w[torch.arange(n), column] = scale
+    return w.to(dtype)
+
+
+@pytest.mark.parametrize("part", ["norm and gate", "attention"])
+@pytest.mark.parametrize("act", ["silu", "gelu"])
+def test_what_is_not_a_sum_is_rounded_as_in_the_chain(part, act, monkeypatch):
+    """Weights with one entry per row and inputs whose squares add up without a rounding in any order: what is left are the divisions and square
+    roots of the norm, the gate and the attention, and these are the correctly rounded ones in both forms.  Equal bits; a reciprocal or root
+    that is an ulp off moves about one f16 value in ten thousand."""
+    if part == "attention" and act == "gelu":
+        pytest.skip("the same attention")
+    H, I, heads, kv, hd, steps = 2048, 8192, 16, 16, 128, 96
+    cfg = Config(hidden_size=H, intermediate_size=I, vocab_size=384, num_hidden_layers=1, num_attention_heads=heads, num_key_value_heads=kv,
+                 rms_norm_eps=1e-5, rope_theta=10000.0, max_seq_len=256, head_dim=hd, use_gelu_mlp=act == "gelu")
+    sd = checkpoint(cfg, "f16", seed=3)
+    g, f16, p = torch.Generator().manual_seed(5), torch.float16, cfg.layer_name(0) + "."
+    zero = lambda n, k: torch.zeros(n, k, dtype=f16)
+    qkvo = {n: zero(H, H) for n in ("q", "k", "v", "o")}
+    mlp = {"gate": zero(I, H), "up": zero(I, H), "down": zero(H, I)}
+    i, h = torch.arange(I), torch.arange(H)
+    if part == "attention":   # equal scores: value sums of whole 64ths over the number of positions
+        qkvo["v"], qkvo["o"] = _one_hot(H, H, (3 * h + 1) % H, 1.0, f16), _one_hot(H, H, (5 * h + 2) % H, 1.0, f16)
+        sd[p + "input_layernorm.weight"] = (torch.randint(-128, 129, (H,), generator=g) / 64).to(f16)
+        xs = [(4 * torch.randint(0, 2, (1, 1, H), generator=g) - 2).to(f16) for _ in range(steps)]
+    else:
+        mlp = {"gate": _one_hot(I, H, (3 * i + 1) % H, 4.0, f16), "up": _one_hot(I, H, (7 * i + i // H) % H, 1.0, f16),
+               "down": _one_hot(H, I, (5 * h + 3) % I, 1.0, f16)}
+        xs = [(torch.randint(-64, 65, (1, 1, H), generator=g) / 16).to(f16) for _ in range(steps)]
+    for n, w in qkvo.items():
+        sd[p + f"self_attn.{n}_proj.weight"] = w
+    for n, w in mlp.items():
+        sd[p + f"mlp.{n}_proj.weight"] = w
+    outs = {}
+    for mode in ("0", "1"):
+        monkeypatch.setenv("CAKE_B200_PER_OP", mode)
+        ctx = Context(cfg, sd, "f16")
+        block = B200Transformer.load(cfg.layer_name(0), ctx)
+        ctx.cache = Cache(ctx, 1, steps)
+        dev = [ctx.to_device(x) for x in xs]
+        ys = [block.forward(x, t, 0, ctx) for t, x in enumerate(dev)]
+        ctx.sync()
+        outs[mode] = torch.cat([y.cpu() for y in ys])
+        ctx.close()
+    assert torch.isfinite(outs["0"].float()).all() and outs["0"].float().abs().max() > 1
+    assert torch.equal(outs["0"], outs["1"]), int((outs["0"] != outs["1"]).sum())
