@@ -1094,50 +1094,55 @@ static int enqueue_decode_layers(cake_b200_ctx *c, cake_b200_block *const *block
 }
 
 // ------------------------------------------------------------------------------------------ megakernel plan + launch
-static int plan_mk_geom(const cake_b200_ctx *c, int N, int K, int G, MkGeom *g) {
+// false: a stage cannot hold the rows, or a part of one that all warps have whole vectors of
+static bool plan_mk_geom(const cake_b200_ctx *c, int N, int K, int G, MkGeom *g) {
   const int es = c->es;
-  if (K % 64 != 0 || N % G != 0) return fail(CAKE_B200_EINVAL, "mega: K=%d must be a multiple of 64, N=%d of %d", K, N, G);
+  if (K % 64 != 0 || N % G != 0) return false;
   int KC = K;
   while ((size_t)KC * es > MK_STAGE_BYTES && (KC / 2) % 64 == 0) KC /= 2;
   const size_t seg = (size_t)KC * es;
-  if (seg > MK_STAGE_BYTES) return fail(CAKE_B200_EINVAL, "mega: K=%d cannot be staged", K);
+  if (seg > MK_STAGE_BYTES) return false;
   int RSL = 0;
   while (KC == K && RSL < 4 && ((size_t)2 << RSL) * seg <= MK_STAGE_BYTES) RSL++;
-  if (KC == K && (1 << RSL) < G) return fail(CAKE_B200_EINVAL, "mega: K=%d: a stage does not hold a gate and an up row", K);
   *g = MkGeom{N, K, KC, RSL, K / KC};
+  if (g->nchunk > MK_BATCH / 2) return false;
   mk_plan_split(*g, G, c->sm_count);
-  return CAKE_B200_OK;
+  return true;
 }
 
 struct MkPlan {
   MkArgs a;
   size_t smem;
 };
-static bool mega_supported(const cake_b200_ctx *c) {
-  const int G = c->cfg.n_heads / c->cfg.n_kv_heads;
-#define MK_CASE(HD_, G_) if (c->cfg.head_dim == HD_ && G == G_) return true;
+// The decode kernel's plan for n_layers blocks and, if asked for, the head; false where the chain of kernels (enqueue_decode_layers, the gemv head) has to
+// do it: head sizes and groups without an instance, rows that no stage holds (K of 16448, say), vectors and ring larger than the shared memory (an
+// intermediate size above 71000).  Without layers only the head's sizes count.  The ranks of a sharded model have to agree: see decode_build.
+static bool plan_mega(const cake_b200_ctx *c, const cake_b200_cache *kc, int n_layers, bool with_head, MkPlan *p) {
+  const cake_b200_config &f = c->cfg;
+  if (!c->use_mega || f.layer_list) return false;
+  const int G = f.n_heads / f.n_kv_heads;
+  bool instance = false;
+#define MK_CASE(HD_, G_) instance = instance || (f.head_dim == HD_ && G == G_);
   MK_FOR_ALL(MK_CASE)
 #undef MK_CASE
-  return false;
-}
-static int plan_mega(cake_b200_ctx *c, cake_b200_cache *kc, int n_layers, bool with_head, MkPlan *p) {
-  const cake_b200_config &f = c->cfg;
+  if (!instance) return false;
   MkArgs &a = p->a;
   memset(&a, 0, sizeof(a));
-  RC(plan_mk_geom(c, c->nqkv, f.hidden, 1, &a.g[0]));
-  RC(plan_mk_geom(c, f.hidden, f.n_heads * f.head_dim, 1, &a.g[1]));
-  RC(plan_mk_geom(c, 2 * f.inter, f.hidden, 2, &a.g[2]));
-  RC(plan_mk_geom(c, f.hidden, f.inter, 1, &a.g[3]));
-  if (with_head) RC(plan_mk_geom(c, f.vocab, f.hidden, 1, &a.g[4]));
-  int whole = 0;  // phases in which every CTA has rows
-  for (int i = 0; i < 4; i++) whole += mk_every_cta(a.g[i]) ? 1 : 0;
-  a.meet = whole < 2;
+  a.max_k = f.hidden;
+  if (n_layers) {
+    if (!plan_mk_geom(c, c->nqkv, f.hidden, 1, &a.g[0]) || !plan_mk_geom(c, f.hidden, f.n_heads * f.head_dim, 1, &a.g[1]) ||
+        !plan_mk_geom(c, 2 * f.inter, f.hidden, 2, &a.g[2]) || !plan_mk_geom(c, f.hidden, f.inter, 1, &a.g[3]))
+      return false;
+    int whole = 0;  // phases in which every CTA has rows
+    for (int i = 0; i < 4; i++) whole += mk_every_cta(a.g[i]) ? 1 : 0;
+    a.meet = whole < 2;
+    a.max_k = std::max(std::max(f.hidden, f.inter), f.n_heads * f.head_dim);
+  }
+  if (with_head && !plan_mk_geom(c, f.vocab, f.hidden, 1, &a.g[4])) return false;
   a.tickets = c->tickets;
   a.hidden = f.hidden; a.inter = f.inter; a.n_heads = f.n_heads; a.n_kv = f.n_kv_heads; a.hd = f.head_dim;
   a.rot = c->rot; a.cap = kc ? kc->cap : 0; a.nsplit = c->nsplit; a.eps = f.rms_eps;
   a.scale = (float)(1.0 / sqrt((double)f.head_dim));
-  a.max_k = f.inter > f.hidden ? f.inter : f.hidden;
-  if (f.n_heads * f.head_dim > a.max_k) a.max_k = f.n_heads * f.head_dim;
   mk_packet_offsets(c, &a.pk);
   a.err = c->wait_err;
   a.cos_t = c->cos_t; a.sin_t = c->sin_t; a.d_pos = kc ? kc->d_pos : nullptr; a.d_step = c->d_step; a.gbar = c->gbar;
@@ -1150,7 +1155,7 @@ static int plan_mega(cake_b200_ctx *c, cake_b200_cache *kc, int n_layers, bool w
   a.act = f.use_gelu_mlp ? 1 : 0;
   a.window = f.sliding_window;
   const size_t limit = 227 * 1024 - 4096;  // the kernel also has ~2.2 KB of static shared memory
-  a.n_layers = n_layers;
+  a.n_layers = std::min(n_layers, MK_MAX_LAYERS);  // (more are refused by who launches them)
   auto stages = [&](int keep) {
     a.keep_x = keep;
     for (a.n_stages = MK_MAX_STAGES; a.n_stages > 2 && mk_layout(a, c->es) > limit;) a.n_stages--;
@@ -1159,8 +1164,7 @@ static int plan_mega(cake_b200_ctx *c, cake_b200_cache *kc, int n_layers, bool w
   const int without = stages(0);
   if (stages(1) < without || mk_layout(a, c->es) > limit) stages(0);  // the copy of the residual stream is not worth a stage
   p->smem = mk_layout(a, c->es);
-  if (p->smem > limit) return fail(CAKE_B200_EINVAL, "mega: needs %zu B of shared memory", p->smem);
-  return CAKE_B200_OK;
+  return p->smem <= limit;
 }
 
 template <typename T> static int launch_mega_T(cake_b200_ctx *c, cudaLaunchConfig_t *cfg, const MkArgs &a) {
@@ -1208,7 +1212,7 @@ static void fill_mk_table(MkLayer *tab, cake_b200_block *const *blocks, const in
 }
 
 // x_in -> x_out through n blocks in ONE persistent kernel; position from cache->d_pos
-static int enqueue_mega_layers(cake_b200_ctx *c, cake_b200_block *const *blocks, const int *block_idx, int n,
+static int enqueue_mega_layers(cake_b200_ctx *c, MkPlan &p, cake_b200_block *const *blocks, const int *block_idx, int n,
                                cake_b200_cache *kc, const void *x_in, void *x_out) {
   if (n > MK_MAX_LAYERS) return fail(CAKE_B200_EINVAL, "more than %d blocks in one call", MK_MAX_LAYERS);
   std::vector<const void *> sig;
@@ -1221,8 +1225,6 @@ static int enqueue_mega_layers(cake_b200_ctx *c, cake_b200_block *const *blocks,
     CU(cudaMemcpyAsync(c->mk_tab_dev, c->mk_tab_host, sizeof(MkLayer) * n, cudaMemcpyHostToDevice, c->stream));
     c->mk_sig = sig;
   }
-  MkPlan p;
-  RC(plan_mega(c, kc, n, false, &p));
   p.a.layers = c->mk_tab_dev;
   p.a.x_in = x_in;
   p.a.x_out = x_out;
@@ -1233,9 +1235,8 @@ static int enqueue_mega_layers(cake_b200_ctx *c, cake_b200_block *const *blocks,
 
 // ln_f + lm_head + greedy argmax on one hidden row -> logits_out (nullable), token -> c->d_token
 static int enqueue_head(cake_b200_ctx *c, const void *x_row, void *logits_out, bool ring) {
-  if (c->use_mega && mega_supported(c)) {  // the decode kernel without layers: the same logits as a replayed step's, bit for bit
-    MkPlan p;
-    RC(plan_mega(c, nullptr, 0, true, &p));
+  MkPlan p;
+  if (plan_mega(c, nullptr, 0, true, &p)) {  // the decode kernel without layers: the same logits as a replayed step's, bit for bit
     p.a.x_in = x_row;
     p.a.has_head = 1;
     p.a.logits = logits_out;
@@ -3375,7 +3376,8 @@ extern "C" int cake_b200_forward_batch(cake_b200_ctx *c, cake_b200_block *const 
   if (batch == 1 && seq == 1 && !variant) {
     set_int_kernel<<<1, 1, 0, c->stream>>>(kc->d_pos, index_pos);
     c->launches++;
-    if (c->use_mega && mega_supported(c)) RC(enqueue_mega_layers(c, blocks, block_idx, n_blocks, kc, x_dev, y_dev));
+    MkPlan p;
+    if (plan_mega(c, kc, n_blocks, false, &p)) RC(enqueue_mega_layers(c, p, blocks, block_idx, n_blocks, kc, x_dev, y_dev));
     else RC(enqueue_decode_layers(c, blocks, block_idx, n_blocks, kc, x_dev, y_dev));
   } else {
     RC(enqueue_prefill_layers(c, blocks, block_idx, n_blocks, kc, x_dev, y_dev, batch, seq, index_pos));
@@ -3876,14 +3878,24 @@ extern "C" int cake_b200_decode_build(cake_b200_ctx *c, cake_b200_block *const *
   c->capturing = true;
   c->g_kernels = 0;
   int rc = [&]() -> int {
-    if (c->use_mega && mega_supported(c)) {
+    // non-greedy: a sampler kernel behind the head re-draws the token from the logits it left behind (256 KB, L2-hot) and overwrites d_token /
+    // the ring slot of this step; the step counter was already advanced
+    auto draw = [&]() -> int {
+      if (c->sampling.kind == SAMPLE_ARGMAX || c->sampling.temperature <= 0.f) return CAKE_B200_OK;
+      return DISPATCH_T(c->cfg.dtype, T_LAMBDA {
+        typedef typename decltype(tag_)::type T;
+        return launch_sampler<T>(c, (const T *)c->logits, c->sampling, nullptr, (const int *)c->d_step, -1, c->token_ring, (int)TOKEN_RING);
+      });
+    };
+    // The ranks of a ring hand over in one way: whether the decode kernel does it is decided from the sizes alone, with the most layers a shard may have.
+    MkPlan p, h;
+    if (plan_mega(c, kc, world > 1 ? MK_MAX_LAYERS : n_blocks, true, &p)) {
       // rank 0: [embed+layers(+head if alone)] ; world>1: layers -> send ... recv -> head.  ranks>0: recv -> layers -> send
-      MkPlan p;
       const bool p2p = world > 1 && c->inbox && c->peer_inbox;  // hand-off fused into the kernels (no NCCL node)
       unsigned long long *inbox_ctr = (unsigned long long *)c->inbox, *peer_ctr = (unsigned long long *)c->peer_inbox;
       void *inbox_x = c->inbox ? c->inbox + INBOX_X_OFF : nullptr, *peer_x = c->peer_inbox ? c->peer_inbox + INBOX_X_OFF : nullptr;
       if (rank == 0) {
-        RC(plan_mega(c, kc, n_blocks, world == 1, &p));
+        plan_mega(c, kc, n_blocks, world == 1, &p);
         p.a.layers = c->g_tab_dev; p.a.x_in = nullptr; p.a.x_out = c->xa;
         if (c->cfg.embed_scale != 0.f) {  // text_model.rs:274-276: the scaled embedding row is materialised first
           RC(DISPATCH_T(c->cfg.dtype, T_LAMBDA {
@@ -3902,24 +3914,16 @@ extern "C" int cake_b200_decode_build(cake_b200_ctx *c, cake_b200_block *const *
             RC(cake_b200_send(c, c->xa, xbytes, 1));
             RC(cake_b200_recv(c, c->xa, xbytes, world - 1));
           }
-          MkPlan h;
-          RC(plan_mega(c, kc, 0, true, &h));
+          plan_mega(c, kc, 0, true, &h);
           h.a.layers = c->g_tab_dev; h.a.x_in = p2p ? inbox_x : c->xa; h.a.x_out = c->xa;
           h.a.has_head = 1; h.a.advance = 1; h.a.token_ring = c->token_ring; h.a.trace_tag = 1;
           if (p2p) { h.a.inbox_ctr = inbox_ctr; h.a.ring_seq = c->ring_seq; }
           RC(launch_mega(c, h));
         }
-        if (c->sampling.kind != SAMPLE_ARGMAX && c->sampling.temperature > 0.f) {
-          // non-greedy: a sampler kernel behind the decode kernel re-draws the token from the logits it left behind
-          // (256 KB, L2-hot) and overwrites d_token / the ring slot of this step; the step counter was already advanced
-          RC(DISPATCH_T(c->cfg.dtype, T_LAMBDA {
-            typedef typename decltype(tag_)::type T;
-            return launch_sampler<T>(c, (const T *)c->logits, c->sampling, nullptr, (const int *)c->d_step, -1, c->token_ring, (int)TOKEN_RING);
-          }));
-        }
+        RC(draw());
       } else {
         if (!p2p) RC(cake_b200_recv(c, c->xa, xbytes, rank - 1));
-        RC(plan_mega(c, kc, n_blocks, false, &p));
+        plan_mega(c, kc, n_blocks, false, &p);
         p.a.layers = c->g_tab_dev; p.a.x_in = p2p ? inbox_x : c->xa; p.a.x_out = p2p ? peer_x : c->xa;
         p.a.has_head = 0; p.a.advance = 1;
         if (p2p) { p.a.inbox_ctr = inbox_ctr; p.a.peer_ctr = peer_ctr; p.a.ring_seq = c->ring_seq; }
@@ -3945,7 +3949,7 @@ extern "C" int cake_b200_decode_build(cake_b200_ctx *c, cake_b200_block *const *
     }
     if (rank == 0) RC(enqueue_head(c, c->xa, c->logits, true));
     RC(launch_pdl(c, advance_kernel, dim3(1), dim3(32), 0, kc->d_pos, c->d_step));
-    return CAKE_B200_OK;
+    return rank == 0 ? draw() : CAKE_B200_OK;
   }();
   c->capturing = false;
   cudaGraph_t g = nullptr;

@@ -170,13 +170,13 @@ struct MkRing {
 // bandwidth is not uniform (measured: the slowest CTA of the 8B gate_up phase finished 5.5 us after the fastest with static
 // rows), so fast SMs take more pool groups and all CTAs end together: 75 % static (CTA c owns groups [c*cnt, (c+1)*cnt)).  A phase of at most
 // MK_SHORT groups per CTA sits in the ring before its input is there, and the CTA that claims one group more than the others is late:
-// all of it is static, dealt out evenly; so are rows that take several stages (K of more than a stage).  A row's dot product
+// all of it is static, dealt out evenly; so are rows that take several stages (K of more than a stage), and gate and up rows where a stage holds one row.  A row's dot product
 // is computed by one CTA with a fixed lane/warp mapping whichever CTA it is -> results stay bit-deterministic.
 constexpr int MK_SHORT = 4;
 inline void mk_plan_split(MkGeom &g, int gran, int grid) {  // gran: rows that stay together (gate and up of a pair)
   g.n_groups = (g.N + (1 << g.RSL) - 1) >> g.RSL;
   g.batch = (MK_BATCH >> g.RSL) / g.nchunk;
-  if (g.nchunk > 1 || g.n_groups <= MK_SHORT * grid) {
+  if (g.nchunk > 1 || gran > 1 << g.RSL || g.n_groups <= MK_SHORT * grid) {
     g.unit = gran > 1 << g.RSL ? gran : 1;
     g.cnt = g.n_groups / g.unit / grid;
     g.rem = g.n_groups / g.unit % grid;

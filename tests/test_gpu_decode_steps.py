@@ -1,10 +1,13 @@
 """The decode kernel at the sizes where its plan changes, against the chain of one kernel per operation: rows per stage 16 .. 1 and rows of
 several stages, phases dealt out evenly and with a pool, models too small for every CTA to own rows, one CTA or several per key head."""
+import ctypes
+
 import pytest
 import torch
 
+from cake_b200.capi import check, lib, ptr
 from cake_b200.config import Config
-from cake_b200.model import B200Transformer, Cache, Context
+from cake_b200.model import B200Transformer, Cache, Context, TextModelBase
 from tests.util import checkpoint, max_ulp_err, rand_x, to_np
 
 pytestmark = pytest.mark.gpu
@@ -125,3 +128,44 @@ def test_what_is_not_a_sum_is_rounded_as_in_the_chain(part, act, monkeypatch):
         ctx.close()
     assert torch.isfinite(outs["0"].float()).all() and outs["0"].float().abs().max() > 1
     assert torch.equal(outs["0"], outs["1"]), int((outs["0"] != outs["1"]).sum())
+
+
+EDGE_SHAPES = {  # hidden, inter, heads, kv heads, head size, dtype
+    "a stage holds one row of gate or up": (12288, 1088, 8, 1, 128, "bf16"),
+    "the longest row of one stage": (16384, 320, 8, 2, 64, "f16"),
+    "gate and up rows of two stages": (20480, 704, 8, 2, 64, "bf16"),
+    "no stage holds a row of down": (1024, 16448, 16, 8, 128, "bf16"),   # steps by the chain of kernels, the head by the decode kernel
+    "vectors larger than the shared memory": (512, 73728, 8, 2, 64, "f16"),
+}
+
+
+@pytest.mark.parametrize("shape", EDGE_SHAPES)
+def test_sizes_at_the_edge_of_the_plan_step_and_have_a_head(shape, monkeypatch):
+    hidden, inter, heads, kv, hd, dtype = EDGE_SHAPES[shape]
+    cfg = Config(hidden_size=hidden, intermediate_size=inter, vocab_size=1000, num_hidden_layers=1, num_attention_heads=heads,
+                 num_key_value_heads=kv, rms_norm_eps=1e-5, rope_theta=10000.0, max_seq_len=512, head_dim=hd)
+    sd = checkpoint(cfg, dtype, seed=11, std=0.7 * hidden ** -0.5)
+    outs, toks = {}, {}
+    for mode in ("0", "1"):
+        monkeypatch.setenv("CAKE_B200_PER_OP", mode)
+        ctx = Context(cfg, sd, dtype, max_seq=512)
+        model = TextModelBase.load(ctx)
+        blk = model.blocks[0]
+        outs[mode], toks[mode] = [], []
+        for pos in (0, 200):
+            ctx.cache = Cache(ctx, 1, pos + 4)
+            ctx.cache.fill_synthetic(range(1), pos, 5)
+            y = blk.forward(ctx.to_device(rand_x((1, 1, hidden), dtype, seed=pos)), pos, 0, ctx)
+            lg, tok = ctx.to_device(torch.zeros(1, cfg.vocab_size)), (ctypes.c_uint32 * 1)()
+            check(lib().cake_b200_logits(ctx.h, ptr(y), 1, 1, ptr(lg), tok))
+            outs[mode] += [y.cpu(), lg.cpu()]
+            assert tok[0] == int(torch.argmax(lg.float()))
+        # the captured loop: the same kernels with the token and the position on the device
+        model.decode_build()
+        model.index_pos = 201
+        toks[mode] = model.decode_greedy(7, 3)
+        assert max(toks[mode]) < cfg.vocab_size
+        ctx.close()
+    for a, b in zip(outs["0"], outs["1"]):
+        assert torch.isfinite(a.float()).all()
+        assert max_ulp_err(to_np(a), to_np(b), dtype) <= 2.0

@@ -211,6 +211,13 @@ def test_gpu_decode_graph_sampler_equals_cake_b200_sample_on_the_same_logits():
 
 
 @pytest.mark.gpu
+def test_gpu_decode_graph_sampler_behind_the_chain_of_kernels(monkeypatch):
+    """Models that the decode kernel has no plan for run one kernel per operation in the captured loop, with the same draw behind the head."""
+    monkeypatch.setenv("CAKE_B200_PER_OP", "1")
+    test_gpu_decode_graph_sampler_equals_cake_b200_sample_on_the_same_logits()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("vocab", [9, 8193, 300000])   # parts without entries; one entry past a full pass; parts too large for shared memory
 def test_gpu_samplers_at_the_edges_of_the_vocabulary_cut(vocab):
     rng = np.random.default_rng(vocab)
