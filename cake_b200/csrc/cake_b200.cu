@@ -197,6 +197,7 @@ struct cake_b200_ctx {
   unsigned long long *gbar = nullptr;   // [0] grid-barrier counter, [1] its value at launch start, [2] layers run (the packets' tags)
   uint32_t *mk_pk = nullptr;            // the megakernel's packets: xa, qkv, y, xb, mm
   uint64_t *mk_part = nullptr;          // and those of attention cut over several CTAs
+  int mk_polls = MK_POLLS;              // what the waits of one of its threads may spend
   MkLayer *mk_tab_dev = nullptr, *mk_tab_host = nullptr, *g_tab_dev = nullptr;
   std::vector<const void *> mk_sig;
   unsigned long long *trace = nullptr;  // CAKE_B200_MEGA_TRACE=1
@@ -781,7 +782,7 @@ static int check_waits(cake_b200_ctx *c) {
   if (*(volatile int *)c->wait_err == 0) return CAKE_B200_OK;
   *(volatile int *)c->wait_err = 0;
   c->wait_failures++;
-  return fail(CAKE_B200_ECUDA, "a kernel gave up a wait for its own copies: this call and the ones before it since the last synchronisation have no results");
+  return fail(CAKE_B200_ECUDA, "a kernel gave up a wait (for its copies, or for other parts of its grid): this call and the ones before it since the last synchronisation have no results");
 }
 static int sync_results(cake_b200_ctx *c) {
   CU(cudaStreamSynchronize(c->stream));
@@ -1145,6 +1146,7 @@ static bool plan_mega(const cake_b200_ctx *c, const cake_b200_cache *kc, int n_l
   a.scale = (float)(1.0 / sqrt((double)f.head_dim));
   mk_packet_offsets(c, &a.pk);
   a.err = c->wait_err;
+  a.polls = c->mk_polls; a.inbox_polls = MK_INBOX_POLLS;
   a.cos_t = c->cos_t; a.sin_t = c->sin_t; a.d_pos = kc ? kc->d_pos : nullptr; a.d_step = c->d_step; a.gbar = c->gbar;
   a.vocab = f.vocab; a.embed = c->embed; a.d_token = c->d_token;
   a.ln_f = c->ln_f; a.lm_head = c->lm_head; a.logits = c->logits; a.part_val = c->part_val; a.part_idx = c->part_idx;
@@ -4129,6 +4131,22 @@ extern "C" int cake_b200_debug_wait(cake_b200_ctx *c, int arrivals, unsigned tri
   wait_probe_kernel<<<1, 1, 0, c->stream>>>(arrivals, tries, c->wait_err, (int *)(c->h_pin + 48));  // (not the first places: a call behind it copies its tokens there)
   CU(cudaGetLastError());
   if (!ok_host) return CAKE_B200_OK;
+  CU(cudaStreamSynchronize(c->stream));
+  for (int i = 0; i < 2; i++) {
+    ok_host[i] = (int)c->h_pin[48 + i];
+    kcycles[i] = (int)c->h_pin[48 + 2 + i];
+  }
+  return CAKE_B200_OK;
+}
+
+/* test aids (not in the public header): the decode kernel's kinds of waits (0 a vector of packets, 1 the parts of attention, 2 the grid barrier, 3 the
+ * inbox) with `polls` polls, as debug_wait. */
+extern "C" int cake_b200_debug_packet_wait(cake_b200_ctx *c, int what, int fresh, int polls, int *ok_host, int *kcycles) {
+  if (!c || !ok_host || !kcycles || what < 0 || what > 3 || polls < 1 || polls > MK_POLLS) return fail(CAKE_B200_EINVAL, "bad debug_packet_wait arguments");
+  CU(cudaSetDevice(c->device));
+  CU(cudaStreamSynchronize(c->stream));
+  mk_wait_probe_kernel<<<1, MK_CT, 0, c->stream>>>(what, fresh, polls, c->wait_err, (int *)(c->h_pin + 48));
+  CU(cudaGetLastError());
   CU(cudaStreamSynchronize(c->stream));
   for (int i = 0; i < 2; i++) {
     ok_host[i] = (int)c->h_pin[48 + i];

@@ -97,6 +97,7 @@ struct MkArgs {
   int act;     // mlp.rs:25-26: 0 silu, 1 gelu_tanh
   int window;  // cache.rs:173-205 sliding window (0 = full context): attention covers the last `window` positions
   int *err;    // host-mapped: set by a wait for packets that ran out
+  int polls, inbox_polls;   // what a thread's waits may spend (MK_POLLS, MK_INBOX_POLLS; less in a test)
 };
 constexpr int MK_STEP_RING = 2048;
 __device__ __forceinline__ unsigned long long mk_gtime() {
@@ -278,8 +279,11 @@ __device__ __forceinline__ void mk_produce_attn(MkRing &rg, const MkArgs &a, con
 
 // ---------------------------------------------------------------------------------------- packets
 // A thread's waits for other CTAs share one budget: when it is spent the error word is set, and every later wait of the thread returns at once.
-// A poll is a round trip to L2 (0.6 us or more), so a wait gives up after seconds, and a launch whose waits all give up still ends.
+// A poll is a round trip to L2 (0.2 us in an idle chip, 0.6 us beside the weights), so a thread gives up after half a second or more (the 80 layers of
+// a 70B model are 22 ms), and a launch whose waits all give up still ends.
 constexpr int MK_POLLS = 1 << 21;
+// The wait for the previous shard has a budget of its own, about a minute, as that rank may still read its prompt: MK_INBOX_FAST polls, then one every 8 us.
+constexpr int MK_INBOX_FAST = 1 << 20, MK_INBOX_POLLS = MK_INBOX_FAST + (1 << 23);
 struct MkWait {
   int left;
   int *err;
@@ -342,6 +346,17 @@ __device__ __forceinline__ void mk_grid_sync(unsigned long long *ctr, unsigned l
     }
   }
   named_bar_sync(1, MK_CT);
+}
+
+// ring hand-off: the previous shard pushes our input over NVLink and bumps the counter once per CTA
+__device__ __forceinline__ void mk_inbox_wait(const unsigned long long *ctr, unsigned long long want, MkWait &w) {
+  const int fast = w.left - MK_INBOX_FAST;
+  while (true) {
+    unsigned long long v;
+    asm volatile("ld.acquire.sys.global.u64 %0, [%1];" : "=l"(v) : "l"(ctr) : "memory");
+    if (v >= want || !w.again()) return;
+    if (w.left < fast) __nanosleep(8000);
+  }
 }
 
 // x -> shared (D) and, where the phase keeps the residual stream, a second copy; returns this thread's share of the sum of squares.
@@ -1066,18 +1081,15 @@ __global__ void __launch_bounds__(MK_THREADS, 1) decode_mega_kernel(const __grid
   }
   // the tag of layer l's packets is first + l; a buffer is written in every layer, so what is stale in it carries the tag in front
   const uint32_t first = (uint32_t)*reinterpret_cast<volatile unsigned long long *>(a.gbar + 2) + 1u;
-  int left = MK_POLLS;
+  int left = a.polls;
   if (a.trace && blockIdx.x == 0 && ct == 0) a.trace[0] = mk_gtime();
   unsigned long long *const st_rec = (a.step_trace && blockIdx.x == 0 && ct == 0)
       ? a.step_trace + ((size_t)((unsigned)*a.d_step % MK_STEP_RING) * 2 + a.trace_tag) * 4 : nullptr;
   if (st_rec) st_rec[0] = mk_gtime();
-  if (a.inbox_ctr) {  // ring hand-off: the previous shard pushes our input over NVLink and bumps the counter once per CTA
+  if (a.inbox_ctr) {
     if (ct == 0) {
-      const unsigned long long want = (*reinterpret_cast<volatile unsigned long long *>(a.ring_seq) + 1ULL) * gridDim.x;
-      unsigned long long v;
-      do {
-        asm volatile("ld.acquire.sys.global.u64 %0, [%1];" : "=l"(v) : "l"(a.inbox_ctr) : "memory");
-      } while (v < want);
+      MkWait w{a.inbox_polls, a.err};
+      mk_inbox_wait(a.inbox_ctr, (*reinterpret_cast<volatile unsigned long long *>(a.ring_seq) + 1ULL) * gridDim.x, w);
     }
     named_bar_sync(1, MK_CT);
   }
@@ -1112,6 +1124,40 @@ __global__ void __launch_bounds__(MK_THREADS, 1) decode_mega_kernel(const __grid
   // bookkeeping without a head: CTA 0 has gathered the last product's input, so every CTA has published something in this launch (mk_every_cta,
   // or all have met), and every CTA read *d_pos, *ring_seq, the barrier start value and the tag before it did.
   if (!a.has_head && blockIdx.x == 0 && ct == 0) mk_end_of_step(a, reinterpret_cast<const float *>(smem_raw + MK_OFF_SCRATCH));
+}
+
+// test aid: each kind of wait of the decode kernel on words of its own, twice by the same threads; fresh: what it waits for is there.
+// out[i]: whether wait i ended by that, out[2 + i]: its kcycles (thread 0)
+__global__ void __launch_bounds__(MK_CT) mk_wait_probe_kernel(int what, int fresh, int polls, int *err, int *out) {
+  __shared__ __nv_bfloat16 xs[4 * MK_CT];
+  __shared__ int gave_up;
+  alignas(16) static __device__ uint32_t words[4 * MK_CT];
+  const int ct = threadIdx.x;
+  const uint32_t tag = 7u;
+  if (what < 2) {   // packets with this tag, or the one in front
+    for (int i = ct; i < 4 * MK_CT; i += MK_CT) words[i] = what ? (fresh ? tag : tag - 1u) : (fresh ? tag : tag - 1u) << 16;
+  } else if (ct < 2) {
+    words[ct] = 0u;   // a counter
+  }
+  __threadfence();
+  __syncthreads();
+  MkWait w{polls, err};
+  for (int i = 0; i < 2; i++) {
+    if (ct == 0) gave_up = 0;
+    __syncthreads();
+    unsigned long long *const ctr = reinterpret_cast<unsigned long long *>(words);
+    const long long t0 = clock64();
+    if (what == 0) mk_gather<__nv_bfloat16>(xs, nullptr, words, 4 * MK_CT, tag << 16, ct, w);
+    else if (what == 1) pk_poll64(reinterpret_cast<uint64_t *>(words) + ct, tag, w);
+    else if (what == 2) mk_grid_sync(ctr, (unsigned long long)(i + 1) * (fresh ? 1ULL : 2ULL), ct, w);   // this CTA's arrival is the only one
+    else if (ct == 0) mk_inbox_wait(ctr, fresh ? 0ULL : 1ULL, w);
+    if (w.left <= 0) gave_up = 1;
+    __syncthreads();
+    if (ct == 0) {
+      out[i] = gave_up ? 0 : 1;
+      out[2 + i] = (int)((clock64() - t0) / 1000);
+    }
+  }
 }
 
 }  // namespace cake

@@ -1,6 +1,6 @@
-"""The bounded waits of the tensor-core kernels (mbar_wait_lim): a wait that nothing ends gives up after its limit, sets the error word that
+"""The bounded waits of the tensor-core kernels (mbar_wait_lim) and of the decode kernel (MkWait): a wait that nothing ends gives up after its limit, sets the error word that
 the next synchronising call reports, and the thread's later waits return at once.  Nothing faults: the probe kernel waits on a
-barrier of its own, returns, and the context stays usable."""
+barrier (or packets, or a counter) of its own, returns, and the context stays usable."""
 import ctypes
 
 import numpy as np
@@ -87,5 +87,27 @@ def test_every_call_that_hands_results_to_the_host_reports_it_and_caches_in_use_
             y = blk.forward(x[:1], 0, 0, ctx)
             ctx.sync()
             assert np.isfinite(to_np(y)).all(), name
+    finally:
+        ctx.close()
+
+
+@pytest.mark.parametrize("what", ["a vector of packets", "the parts of attention", "the grid barrier", "the inbox"])
+def test_a_wait_of_the_decode_kernel_that_runs_out(what):
+    cfg = medium_config()
+    ctx = Context(cfg, checkpoint(cfg, "bf16", seed=3), "bf16")
+    kind = ["a vector of packets", "the parts of attention", "the grid barrier", "the inbox"].index(what)
+    ok, kcycles = (ctypes.c_int * 2)(), (ctypes.c_int * 2)()
+    fn = lib().cake_b200_debug_packet_wait
+    fn.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int)]
+    try:
+        check(fn(ctx.h, kind, 1, 4096, ok, kcycles))
+        assert list(ok) == [1, 1]
+        ctx.sync()
+        check(fn(ctx.h, kind, 0, 4096, ok, kcycles))   # the first wait takes all of its polls, the second one none
+        print(f"{what}: 4096 polls {kcycles[0]} kcycles, then {kcycles[1]}")
+        assert list(ok) == [0, 0] and kcycles[0] < 100000 and kcycles[1] <= kcycles[0] / 50
+        with pytest.raises(CakeB200Error, match="gave up a wait"):
+            ctx.sync()
+        ctx.sync()
     finally:
         ctx.close()
