@@ -780,6 +780,7 @@ static int pipe_mark(cake_b200_ctx *c) {  // compute must not start before the u
 // hands results to the host.  The context goes on; the caches that were there hold no results until they are cleared.
 static int check_waits(cake_b200_ctx *c) {
   if (*(volatile int *)c->wait_err == 0) return CAKE_B200_OK;
+  (void)cudaStreamSynchronize(c->stream);   // other threads of that kernel, and the kernels behind it, may give up yet: one report for all of them
   *(volatile int *)c->wait_err = 0;
   c->wait_failures++;
   return fail(CAKE_B200_ECUDA, "a kernel gave up a wait (for its copies, or for other parts of its grid): this call and the ones before it since the last synchronisation have no results");
@@ -4140,7 +4141,7 @@ extern "C" int cake_b200_debug_wait(cake_b200_ctx *c, int arrivals, unsigned tri
 }
 
 /* test aids (not in the public header): the decode kernel's kinds of waits (0 a vector of packets, 1 the parts of attention, 2 the grid barrier, 3 the
- * inbox) with `polls` polls, as debug_wait. */
+ * inbox) with `polls` polls, as debug_wait; and the polls that the waits of the context's next decode kernels may spend (0: as ever). */
 extern "C" int cake_b200_debug_packet_wait(cake_b200_ctx *c, int what, int fresh, int polls, int *ok_host, int *kcycles) {
   if (!c || !ok_host || !kcycles || what < 0 || what > 3 || polls < 1 || polls > MK_POLLS) return fail(CAKE_B200_EINVAL, "bad debug_packet_wait arguments");
   CU(cudaSetDevice(c->device));
@@ -4152,6 +4153,11 @@ extern "C" int cake_b200_debug_packet_wait(cake_b200_ctx *c, int what, int fresh
     ok_host[i] = (int)c->h_pin[48 + i];
     kcycles[i] = (int)c->h_pin[48 + 2 + i];
   }
+  return CAKE_B200_OK;
+}
+extern "C" int cake_b200_debug_polls(cake_b200_ctx *c, int polls) {
+  if (!c || polls < 0 || polls > MK_POLLS) return fail(CAKE_B200_EINVAL, "bad debug_polls arguments");
+  c->mk_polls = polls ? polls : MK_POLLS;
   return CAKE_B200_OK;
 }
 

@@ -5,9 +5,11 @@ import ctypes
 
 import numpy as np
 import pytest
+import torch
 
 from cake_b200.capi import CakeB200Error, check, lib, ptr
-from cake_b200.model import B200Transformer, Context, sampling_from_args
+from cake_b200.config import Config
+from cake_b200.model import B200Transformer, Cache, Context, sampling_from_args
 from tests.util import checkpoint, medium_config, rand_x, to_np
 
 pytestmark = pytest.mark.gpu
@@ -109,5 +111,46 @@ def test_a_wait_of_the_decode_kernel_that_runs_out(what):
         with pytest.raises(CakeB200Error, match="gave up a wait"):
             ctx.sync()
         ctx.sync()
+    finally:
+        ctx.close()
+
+
+@pytest.mark.parametrize("hidden,inter,heads,kv,hd", [(192, 448, 4, 2, 16), (1024, 3072, 16, 8, 128), (2560, 17408, 32, 4, 128)])
+def test_steps_after_one_whose_waits_ran_out(hidden, inter, heads, kv, hd):
+    """Every wait of a step gives up at its second poll: the launch ends, the call that synchronises reports it, and the same session begun again on
+    the same context has the bits that it had before (tags, the barrier's counter and its start went on)."""
+    layers, first = 3, 140
+    cfg = Config(hidden_size=hidden, intermediate_size=inter, vocab_size=384, num_hidden_layers=layers, num_attention_heads=heads,
+                 num_key_value_heads=kv, rms_norm_eps=1e-5, rope_theta=10000.0, max_seq_len=512, head_dim=hd)
+    ctx = Context(cfg, checkpoint(cfg, "bf16", seed=3, std=0.7 * hidden ** -0.5), "bf16")
+    polls = lib().cake_b200_debug_polls
+    polls.argtypes = [ctypes.c_void_p, ctypes.c_int]
+    try:
+        blocks = [B200Transformer.load(cfg.layer_name(i), ctx) for i in range(layers)]
+        ctx.cache = Cache(ctx, 1, first + 4)
+        xs = [ctx.to_device(rand_x((1, 1, hidden), "bf16", seed=t)) for t in range(3)]
+
+        def step(t):
+            return blocks[0].forward_batch(xs[t], [(b.layer_name(), first + t, i) for i, b in enumerate(blocks)], ctx, blocks=blocks)
+
+        def session():
+            ctx.cache.clear()
+            ctx.cache.fill_synthetic(range(layers), first, 5)
+            ys = [step(t) for t in range(3)]
+            ctx.sync()
+            return [y.cpu() for y in ys]
+
+        want = session()
+        for _ in range(2):
+            ctx.cache.clear()
+            ctx.cache.fill_synthetic(range(layers), first, 5)
+            check(polls(ctx.h, 1))
+            step(0)
+            check(polls(ctx.h, 0))
+            with pytest.raises(CakeB200Error, match="gave up a wait"):
+                ctx.sync()
+            with pytest.raises(CakeB200Error, match="clear it"):
+                step(1)
+            assert all(torch.equal(a, b) for a, b in zip(session(), want))
     finally:
         ctx.close()
