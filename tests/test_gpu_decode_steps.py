@@ -20,6 +20,7 @@ SHAPES = {  # hidden, inter, heads, kv heads, head size, dtype
     "16 and 4 rows, even shares": (1024, 3072, 16, 8, 128, "f16"),
     "8 and 2 rows, pools": (2048, 8192, 16, 16, 128, "bf16"),
     "4 rows, rows of two stages": (2560, 17408, 32, 4, 128, "bf16"),
+    "no room for the copy of the residual stream": (2560, 21504, 32, 4, 128, "bf16"),   # 5 stages without it, 4 with it
 }
 
 
