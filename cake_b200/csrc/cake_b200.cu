@@ -3053,6 +3053,15 @@ template <typename Take> static MoeScratch moe_scratch(const cake_b200_ctx *c, c
   if (mo.shared_ff) s.sact = take(M * mo.shared_ff * es);
   return s;
 }
+// The CTAs that a row's keys are cut over in latent attention's vector form (0: a warp per row and head).  A CTA walks its keys 16 at a time, a few us each:
+// 64 keys a split while two CTAs per SM take those of one row, 128 at most.  The rows of the call do not count, so that a row has the same sums
+// alone and in a batch: a step of the 2k model at 300 keys takes 313 us (311 with 32 keys a split, 327 with 128), one of 128 rows 1660
+// (1720 with 32 keys, 1645 with 128).
+static int latent_splits(int sms, size_t rows, int heads, int n_keys) {
+  if (rows * heads > 2048) return 0;
+  const int fill = (2 * sms + heads - 1) / heads, n = std::min(LATENT_SPLIT_MAX, std::max((n_keys + 127) / 128, std::min(fill, (n_keys + 63) / 64)));
+  return n > 1 ? n : 0;
+}
 static MixerScratch mixer_scratch(const cake_b200_ctx *c, const cake_b200_block *b, size_t M, char *base, int S = 1, int n_keys = 1) {
   MixerScratch s{};
   size_t off = 0;
@@ -3074,13 +3083,9 @@ static MixerScratch mixer_scratch(const cake_b200_ctx *c, const cake_b200_block 
       const size_t rows = (size_t)s.lat_tok * sp.heads, kp = ((size_t)n_keys + TC_BN - 1) / TC_BN * TC_BN;
       s.scores = (float *)take(rows * kp * sizeof(float));
       s.pw = take(rows * 2 * kp * es);
-    } else if (M * sp.heads <= 2048 && n_keys > 32) {
-      // 32 keys a split while two CTAs per SM take them all, 128 at most: a CTA walks its keys 16 at a time, a few us each (one token, 16 heads, 300
-      // keys: 3 splits 27 us)
-      const int fill = (int)((2 * (size_t)c->sm_count + M * sp.heads - 1) / (M * sp.heads));
-      s.nsplit = std::min(LATENT_SPLIT_MAX, std::max((n_keys + 127) / 128, std::min(fill, (n_keys + 31) / 32)));
-      if (s.nsplit > 1) s.part = (float *)take(M * sp.heads * s.nsplit * (sp.kv_rank + 2) * sizeof(float));
-      else s.nsplit = 0;
+    } else {
+      s.nsplit = latent_splits(c->sm_count, M, sp.heads, n_keys);
+      if (s.nsplit) s.part = (float *)take(M * sp.heads * s.nsplit * (sp.kv_rank + 2) * sizeof(float));
     }
   } else {
     s.o32 = (float *)take(M * inner * sizeof(float));
@@ -4205,6 +4210,9 @@ extern "C" int cake_b200_debug_product(cake_b200_ctx *c, int epi, const void *A,
   }));
   return sync_results(c);
 }
+
+/* test aid (not in the public header): the split rule of latent attention's vector form */
+extern "C" int cake_b200_debug_latent_splits(int sms, int rows, int heads, int n_keys) { return latent_splits(sms, (size_t)rows, heads, n_keys); }
 
 /* profiling aid (not in the public header): copies the megakernel's phase-boundary %globaltimer stamps of
  * the last launch (CTA 0) to `out`; needs CAKE_B200_MEGA_TRACE=1 at ctx creation. */

@@ -512,3 +512,36 @@ def test_checkpoint_on_disk_through_the_trace_replayer_and_the_generate_command(
     assert res.returncode == 0, res.stderr[-2000:]
     out = [int(t) for t in res.stdout.split("tokens:")[1].splitlines()[0].split()]
     assert len(out) == 5 and all(0 <= t < cfg.vocab_size for t in out)
+
+
+def test_latent_splits_do_not_depend_on_the_rows():
+    """A token's sums over its keys are cut in the same places alone and in a batch (up to the rows from which a warp takes a row and head)."""
+    from cake_b200.capi import lib
+    splits = lib().cake_b200_debug_latent_splits
+    for heads in (1, 3, 8, 16, 40):
+        for n_keys in (1, 33, 64, 65, 129, 300, 1217, 4096, 20000):
+            alone = splits(148, 1, heads, n_keys)
+            assert alone == 0 or 2 <= alone <= 32
+            assert alone >= min(32, (n_keys + 127) // 128) or n_keys <= 128
+            assert {splits(148, rows, heads, n_keys) for rows in (1, 2, 5, 16, 2048 // heads)} == {alone}
+            assert splits(148, 2048 // heads + 1, heads, n_keys) == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", ["bf16", "f16"])
+def test_a_row_decodes_alone_as_in_a_batch(dtype):
+    """The steps of up to eight rows have the bits of each row's steps alone, over the key counts at which latent attention is cut anew."""
+    from cake_b200.model import Cache
+    cfg = make_config([latent(heads=4, dim=128, rot_dim=64, vdim=128, kv_rank=256, scale=0.09)], width=256, vocab=96, max_seq=256)
+    sd = make_mixer_checkpoint(cfg, dtype, seed=57)
+    rows = np.array([tokens(140, cfg.vocab_size, seed=60 + i) for i in range(8)], dtype=np.uint32)
+    r = Runner(cfg, sd, dtype)
+    try:
+        got = {}
+        for n in (1, 3, 8):
+            r.ctx.cache = Cache(r.ctx, n, 140)
+            got[n] = np.stack([r.model.forward(rows[:n, t:t + 1], t, want=list(range(n))).cpu().numpy().reshape(n, -1) for t in range(140)])
+        for n in (3, 8):
+            assert np.array_equal(got[n][:, 0], got[1][:, 0]), n
+    finally:
+        r.close()
