@@ -4211,8 +4211,27 @@ extern "C" int cake_b200_debug_product(cake_b200_ctx *c, int epi, const void *A,
   return sync_results(c);
 }
 
-/* test aid (not in the public header): the split rule of latent attention's vector form */
+/* test aids (not in the public header): the split rule of latent attention's vector form, that attention on given buffers (part: [B S heads, nsplit,
+ * rank + 2] fp32, nsplit 0: none), and a product per head. */
 extern "C" int cake_b200_debug_latent_splits(int sms, int rows, int heads, int n_keys) { return latent_splits(sms, (size_t)rows, heads, n_keys); }
+extern "C" int cake_b200_debug_latent(cake_b200_ctx *c, const void *qa, const void *cache, void *lat, float *part, int B, int S, int heads, int rank, int rot, int cap,
+                                      int pos0, float scale, int nsplit) {
+  if (!c || !qa || !cache || !lat || B < 1 || S < 1 || heads < 1 || rank < 1 || rot < 0 || pos0 < 0 || pos0 + S > cap || nsplit < 0 || nsplit > LATENT_SPLIT_MAX ||
+      (nsplit > 1 && !part))
+    return fail(CAKE_B200_EINVAL, "bad debug_latent arguments");
+  CU(cudaSetDevice(c->device));
+  mx::LatentAttn la{qa, cache, lat, B, S, heads, rank, rot, cap, pos0, scale, part, nsplit};
+  MX(mx::latent_attention(c->stream, c->cfg.dtype, la, &c->launches));
+  return sync_results(c);
+}
+extern "C" int cake_b200_debug_head_gemm(cake_b200_ctx *c, const void *A, const void *W, void *C, int M, int N, int K, int Z, long a_zs, long w_zs, long c_zs, int lda,
+                                         int ldw, int ldc, int w_kn) {
+  if (!c || !A || !W || !C || M < 1 || N < 1 || K < 1 || Z < 1) return fail(CAKE_B200_EINVAL, "bad debug_head_gemm arguments");
+  CU(cudaSetDevice(c->device));
+  mx::HeadGemm g{A, W, C, M, N, K, Z, a_zs, w_zs, c_zs, lda, ldw, ldc, w_kn};
+  MX(mx::head_gemm(c->stream, c->cfg.dtype, g, &c->launches));
+  return sync_results(c);
+}
 
 /* profiling aid (not in the public header): copies the megakernel's phase-boundary %globaltimer stamps of
  * the last launch (CTA 0) to `out`; needs CAKE_B200_MEGA_TRACE=1 at ctx creation. */

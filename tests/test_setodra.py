@@ -527,6 +527,77 @@ def test_latent_splits_do_not_depend_on_the_rows():
             assert splits(148, 2048 // heads + 1, heads, n_keys) == 0
 
 
+@pytest.fixture(params=["bf16", "f16"])
+def kernels(request):
+    """A context whose kernels are called one by one."""
+    from cake_b200.model import Context
+    cfg = make_config([latent()])
+    ctx = Context(cfg, {}, request.param)
+    yield ctx
+    ctx.close()
+
+
+U = {"bf16": 2.0 ** -8, "f16": 2.0 ** -11}   # half the spacing of values around 1
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rank,rot", [(192, 64), (200, 56), (448, 64), (512, 64), (704, 64)])   # one, two and three vectors a lane, whole and partial
+@pytest.mark.parametrize("nsplit,S,pos0", [(5, 1, 299), (32, 1, 700), (2, 3, 30), (3, 2, 0)])   # ragged, the most, several rows, splits without keys
+def test_latent_attention_of_a_step_in_vectors(kernels, rank, rot, nsplit, S, pos0):
+    """The form with 16-byte loads against fp32 torch on the same values, and against the general form, which a base address off by two bytes selects."""
+    import ctypes
+    from cake_b200.capi import check, lib, ptr
+    B, heads, Dk, cap, scale = 2, 3, rank + rot, pos0 + S, (rank + rot) ** -0.5
+    g = torch.Generator(device="cuda:0").manual_seed(rank + nsplit)
+    D = kernels.torch_dtype
+    qa, cache = torch.randn(B * S, heads, Dk, device="cuda:0", generator=g).to(D) * 3, torch.randn(B, cap, Dk, device="cuda:0", generator=g).to(D)
+    lat = torch.empty(2, B * S, heads, rank, device="cuda:0", dtype=D)
+    part = torch.full((B * S * heads, nsplit, rank + 2), float("nan"), device="cuda:0")
+    odd = torch.empty(cache.numel() + 1, device="cuda:0", dtype=D)[1:].view_as(cache).copy_(cache)
+    fn = lib().cake_b200_debug_latent
+    V, I = ctypes.c_void_p, ctypes.c_int
+    fn.argtypes = [V, V, V, V, V, I, I, I, I, I, I, I, ctypes.c_float, I]
+    torch.cuda.synchronize()
+    for out, kv in ((lat[0], cache), (lat[1], odd)):
+        check(fn(kernels.h, ptr(qa), ptr(kv), ptr(out), ptr(part), B, S, heads, rank, rot, cap, pos0, scale, nsplit))
+    s = torch.einsum("bshd,btd->bsht", qa.double().view(B, S, heads, Dk), cache.double()) * scale
+    visible = torch.arange(cap, device="cuda:0")[None, :] <= pos0 + torch.arange(S, device="cuda:0")[:, None]
+    w = s.masked_fill(~visible[None, :, None, :], float("-inf")).softmax(-1)
+    want = torch.einsum("bsht,btr->bshr", w, cache.double()[..., :rank]).view(B * S, heads, rank)
+    # one rounding to D, and what an error of the scores (Dk products, |s| up to 3 sqrt(Dk) scale ~ 15) and of the sums does: 1e-5 of the largest entry of a row
+    bound = U[kernels.dtype] * want.abs() + 2e-5 * want.abs().amax(-1, keepdim=True) + 1e-7
+    for form, got in zip(("vectors", "general"), lat):
+        assert ((got.double() - want).abs() <= bound).all(), (form, ((got.double() - want).abs() / bound).max().item())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("N,K,ldw,lda", [(512, 128, 512, 200), (136, 128, 144, 130), (8, 5, 8, 5), (392, 257, 400, 260), (128, 8192, 128, 8192)])
+@pytest.mark.parametrize("M", [1, 3, 8])
+def test_product_per_head_of_a_step_in_vectors(kernels, M, N, K, ldw, lda):
+    """A weight stored [K, N] with rows of whole 16-byte vectors, N not a multiple of the 128 columns of a CTA, strides larger than the rows; the same with rows
+    one element longer takes the general form."""
+    import ctypes
+    from cake_b200.capi import check, lib, ptr
+    Z, D, dev = 3, kernels.torch_dtype, "cuda:0"
+    g = torch.Generator(device=dev).manual_seed(N + K)
+    fn = lib().cake_b200_debug_head_gemm
+    V, I, L = ctypes.c_void_p, ctypes.c_int, ctypes.c_long
+    fn.argtypes = [V, V, V, V, I, I, I, I, L, L, L, I, I, I, I]
+    a = torch.randn(M, Z, lda, device=dev, generator=g).to(D)
+    w = (torch.randn(Z, K, N, device=dev, generator=g) * K ** -0.5).to(D)
+    want = torch.einsum("mzk,zkn->mzn", a[..., :K].double(), w.double())
+    # fp32 sums of K products in 16 parts, one rounding to D
+    bound = U[kernels.dtype] * want.abs() + (K / 16 + 16) * 2.0 ** -24 * torch.einsum("mzk,zkn->mzn", a[..., :K].double().abs(), w.double().abs())
+    for ld in (ldw, ldw + 1):
+        wz = torch.full((Z, K, ld), float("nan"), device=dev, dtype=D)
+        wz[..., :N] = w
+        out = torch.full((M, Z, N + 24), 7.0, device=dev, dtype=D)
+        torch.cuda.synchronize()
+        check(fn(kernels.h, ptr(a), ptr(wz), ptr(out), M, N, K, Z, lda, K * ld, N + 24, Z * lda, ld, Z * (N + 24), 1))
+        assert ((out[..., :N].double() - want).abs() <= bound).all(), ld
+        assert (out[..., N:] == 7.0).all()
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", ["bf16", "f16"])
 def test_a_row_decodes_alone_as_in_a_batch(dtype):
