@@ -603,7 +603,7 @@ def test_product_per_head_of_a_step_in_vectors(kernels, M, N, K, ldw, lda):
 def test_a_row_decodes_alone_as_in_a_batch(dtype):
     """The steps of up to eight rows have the bits of each row's steps alone, over the key counts at which latent attention is cut anew."""
     from cake_b200.model import Cache
-    cfg = make_config([latent(heads=4, dim=128, rot_dim=64, vdim=128, kv_rank=256, scale=0.09)], width=256, vocab=96, max_seq=256)
+    cfg = make_config([latent(heads=16, dim=128, rot_dim=64, vdim=128, kv_rank=256, scale=0.09)], width=256, vocab=96, max_seq=256)
     sd = make_mixer_checkpoint(cfg, dtype, seed=57)
     rows = np.array([tokens(140, cfg.vocab_size, seed=60 + i) for i in range(8)], dtype=np.uint32)
     r = Runner(cfg, sd, dtype)
