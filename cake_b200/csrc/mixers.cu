@@ -22,8 +22,16 @@ namespace mx {
 // without that a step's chain of 24 launches of a few us each paid 2 us of launch latency each time (step through three Setodra blocks 358 -> 315 us).  Not so
 // grids of more than two CTAs per SM, and not a recurrence over many tokens: CTAs placed while the kernel in front still holds most of the chip crowd
 // on the SMs that are free first (1000 tokens: 2200 -> 2434 us with all of them launched early).
-constexpr unsigned MX_EARLY_CTAS = 296;
-constexpr int MX_EARLY_TOKENS = 8;
+constexpr int MX_EARLY_CTAS_PER_SM = 2, MX_EARLY_TOKENS = 8;
+static size_t mx_early_ctas() {
+  static thread_local int of_dev = -1, ctas = 0;
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess && dev != of_dev && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess) {
+    of_dev = dev;
+    ctas = MX_EARLY_CTAS_PER_SM * sms;
+  }
+  return (size_t)ctas;
+}
 template <typename... KArgs, typename... Args>
 static void mx_launch_if(bool early, cudaStream_t st, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, Args... args) {
   cudaLaunchConfig_t cfg{};
@@ -35,7 +43,7 @@ static void mx_launch_if(bool early, cudaStream_t st, void (*kern)(KArgs...), di
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = early && (size_t)grid.x * grid.y * grid.z <= MX_EARLY_CTAS ? 1 : 0;
+  cfg.numAttrs = early && (size_t)grid.x * grid.y * grid.z <= mx_early_ctas() ? 1 : 0;
   cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
 template <typename... KArgs, typename... Args>
