@@ -59,8 +59,8 @@ __device__ __forceinline__ float sample_uniform(const SampleArgs &s, unsigned st
 // Bound: latency, not bytes (300 KB of logits): one CTA took 31 bisection passes of 125 dependent loads each over the vocabulary, 380 us for
 // 128256 entries.  The vocabulary is cut between the CTAs of a cluster, which keep their probabilities in shared memory; a pass looks
 // at seven thresholds at once and its sums meet over the cluster; the thresholds are logits, whose 16 bits take six passes (a
-// probability's 30 bits took ten: 97 us).  A nucleus is searched between the largest logit and where it can end, three passes, entries below a pass's
-// lowest threshold are passed over, and the logits are read 16 bytes at a time: the call 95 -> 77 us at 128256 entries.
+// probability's 30 bits took ten: 97 us).  A nucleus is searched between the largest logit and where it can end (see sample_threshold), entries below a
+// pass's lowest threshold are passed over, and the logits are read 16 bytes at a time: the call 95 -> 77 us at 128256 bf16 entries, three passes.
 // Every reduction has a fixed order (threads, warps, ranks): a draw is a function of (logits, seed, step).
 struct SampleShared {
   float warp[SAMPLE_THREADS / 32][9];    // a warp's sums (rows of nine: no bank conflicts down a column)
@@ -170,8 +170,10 @@ template <typename T> __device__ __forceinline__ float sample_unkey(uint32_t k) 
   return DT<T>::to_f(*reinterpret_cast<const T *>(&h));
 }
 // The largest logit at which the entries that are at least as large still reach `want`, in number (COUNT) or in probability: with tau its
-// probability, reach(P >= tau) >= want > reach(P > tau), as probabilities rise with logits.  Seven thresholds a pass.  from, to: logits between which it
-// lies (65536 patterns are six passes; the few hundred between the largest logit and where a nucleus can end are three).
+// probability, reach(P >= tau) >= want > reach(P > tau), as probabilities rise with logits.  Seven thresholds a pass, log8 of the patterns from `from` to
+// `to`, between which it lies, passes.  All 65536 are six.  From the largest logit to where a nucleus can end, both above zero, there are a few hundred in
+// bf16 (128 an octave: three passes) and a few thousand in f16 (1024 an octave: four); where the end lies below zero, the range holds every small
+// exponent, some 33000 patterns: five passes, or six.
 template <typename T, bool COUNT>
 __device__ __forceinline__ float sample_threshold(SampleCluster &cl, const T *L, const float *P, int i0, int i1, float want, float from, float to) {
   uint32_t lo = sample_key<T>(from), hi = sample_key<T>(to) + 1u;
