@@ -48,7 +48,7 @@ sys.path.insert(0, ROOT)
 
 def _cpu_plan():
     """Host threads for the CPU legs: the physical cores of ONE socket that this process may use, capped by the
-    container's CPU quota.  (Round 1: the same 32 threads gave 4.5-9.1 tok/s run to run — threads and first-touch
+    container's CPU quota.  (Without that, the same 32 threads gave 4.5-9.1 tok/s run to run — threads and first-touch
     pages spread over two sockets and their SMT siblings.)"""
     allowed = sorted(os.sched_getaffinity(0))
     cores, seen = [], set()
@@ -536,8 +536,7 @@ def decode_leg(env: Env, model: str, K: int, W: int, n_e2e: int, parity: bool, i
     roof = {"bound": "hbm", "kernel": f"decode_mega_kernel<bf16,{cfg.hd},{G}> (all local layers + ln_f + lm_head + argmax)",
             "achieved": round(launch_bytes / (launch_ms * 1e-3) / 1e9, 1), "peak": pk["hbm"], "unit": "GB/s",
             "frac": round(launch_bytes / (launch_ms * 1e-3) / 1e9 / pk["hbm"], 4),
-            "traffic": TRAFFIC_NCU["bytes"] if (world == 1 and model == "8b") else None,
-            "traffic_source": TRAFFIC_NCU["source"] if (world == 1 and model == "8b") else None,
+            "traffic": None,
             "peak_source": pk["src"], "algorithmic_bytes_per_launch": launch_bytes, "launch_ms": launch_ms,
             "launches_per_step": 1 if world == 1 else 2, "share_of_step": 1.0}
     if world > 1:
@@ -588,11 +587,6 @@ def decode_leg(env: Env, model: str, K: int, W: int, n_e2e: int, parity: bool, i
             line["cpu_baseline"] = cpu
     sh.close()
     return line
-
-
-TRAFFIC_NCU = {"bytes": 15280381000 + 8281856,
-               "source": "dram__bytes_read.sum + dram__bytes_write.sum of one decode_mega_kernel launch, ncu --set full at N=1 "
-                         "(profiles/mega_r02_raw.csv); cited from the committed capture, not measured in this run"}
 
 
 def step_stats(traces, K: int, ms_all: float):
@@ -891,7 +885,7 @@ def prefill_leg(env: Env, reps: int = 3, batch: int = 32, seq: int = 4096) -> di
                         "peak_source": pk["src"] + " (sustained cuBLAS bf16, the kernel runs inside a seconds-long step)",
                         "algorithmic_flops_per_step": flops,
                         "flops_split": {"linears": flop_lin, "causal_attention": flop_att, "lm_head": flop_head},
-                        "kernels": "per layer: gemm_tc_kernel (tcgen05, 256x256 tiles on SM pairs) x4 + attn_prefill_tc_kernel (tcgen05 flash attention) + rmsnorm_rows_vec x2 + rope_append_vec; ncu: profiles/launches_prefill_r02.csv"}}
+                        "kernels": "per layer: gemm_tc_kernel (tcgen05, 256x256 tiles on SM pairs) x4 + attn_prefill_tc_kernel (tcgen05 flash attention) + rmsnorm_rows_vec x2 + rope_append_vec"}}
     ctx.close()
     torch.cuda.empty_cache()
     return res

@@ -1,22 +1,23 @@
 """Profiling aid: per-phase timing of the persistent decode megakernel (CTA 0's %globaltimer stamps).
-   CAKE_B200_MEGA_TRACE=1 python bench_tools/mega_trace.py [n_layers]"""
+   python bench_tools/mega_trace.py [n_layers] [llama3_8b | qwen3_0_6b] [context length]"""
 import ctypes, os, sys
 os.environ["CAKE_B200_MEGA_TRACE"] = "1"
 sys.path.insert(0, os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
 import numpy as np, torch
 from cake_b200.capi import lib, check
-from cake_b200.config import llama3_8b
+from cake_b200 import config
 from cake_b200.model import Context, TextModelBase, Cache
 from cake_b200.synth import make_head, make_layer
 
 nl = int(sys.argv[1]) if len(sys.argv) > 1 else 8
-cfg = llama3_8b(max_seq=4096); cfg.num_hidden_layers = nl
+cfg = getattr(config, sys.argv[2] if len(sys.argv) > 2 else "llama3_8b")(max_seq=4096); cfg.num_hidden_layers = nl
+at = int(sys.argv[3]) if len(sys.argv) > 3 else 2048
 sd = make_head(cfg, "bf16", device="cuda")
 for i in range(nl): sd.update(make_layer(cfg, i, "bf16", device="cuda"))
 ctx = Context(cfg, sd, "bf16", max_seq=4096)
-ctx.cache = Cache(ctx, 1, 2304)
+ctx.cache = Cache(ctx, 1, at + 256)
 m = TextModelBase.load(ctx)
-ctx.cache.fill_synthetic(list(range(nl)), 2048, 7); ctx.sync(); m.index_pos = 2048
+ctx.cache.fill_synthetic(list(range(nl)), at, 7); ctx.sync(); m.index_pos = at
 m.decode_build()
 m.decode_greedy(5, 8)
 L = lib(); L.cake_b200_debug_trace.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int]

@@ -66,7 +66,7 @@ struct TcParams {
 
 // Tile rasterisation: groups of TC_GM m-tiles (16 x 128 rows = 16 MB of A at K=4096) are walked n-major, so the A
 // group stays in the 126 MB L2 while each W tile streams once per group.  With plain m-fastest order a 1 GB A
-// (bs=32 x 4k) is re-read for every W tile column: measured 815 TFLOP/s, HBM-bound (profiles/README.md).
+// (bs=32 x 4k) is re-read for every W tile column: measured 815 TFLOP/s, HBM-bound.
 constexpr int TC_GM = 16;
 __device__ __forceinline__ void tc_tile(int t, int tiles_m, int tiles_n, int bn, int &m0, int &n0) {
   const int per_group = TC_GM * tiles_n;

@@ -2,7 +2,7 @@
  * cake_b200.h — C ABI of libcake_b200.so: the B200-native (sm_100a) implementation of cake's
  * sharded transformer-block forward path.
  *
- * This is the drop-in boundary.  A Rust `B200Transformer: Forwarder` (see INTEGRATION.md and
+ * This is the drop-in boundary.  A Rust `B200Transformer: Forwarder` (see
  * rust/b200_transformer.rs) binds exactly these entry points; nothing here mentions torch or candle
  * types — only opaque handles, plain pointers and sizes.  Conventions follow the reference's two
  * existing FFI surfaces (cake-core/src/backends/rocm/ffi.rs:12-51 function table with int status

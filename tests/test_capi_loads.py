@@ -88,7 +88,7 @@ def test_product_never_imports_the_oracle():
 
 
 def test_null_handles_are_errors_not_crashes():
-    """`errors never abort`: every entry point called with null handles / zero sizes returns a
+    """Errors never abort: every entry point called with null handles / zero sizes returns a
     status (or a null/negative value) and leaves a message — checked in a child process so that a regression shows up as
     a failed assertion, not a dead test runner."""
     import subprocess
