@@ -605,6 +605,7 @@ extern "C" int cake_b200_ctx_create(int device, const cake_b200_config *cfg, cak
     CU(cudaMemset(c->mk_part, 0, parts * 8));
   }
   CU(cudaMalloc(&c->tickets, sizeof(unsigned) * (4 * MK_MAX_LAYERS + 4)));
+  CU(cudaMemset(c->tickets, 0, sizeof(unsigned) * (4 * MK_MAX_LAYERS + 4)));
   CU(cudaMalloc(&c->ring_seq, 8));
   CU(cudaMemset(c->ring_seq, 0, 8));
   CU(cudaMalloc(&c->step_trace, sizeof(unsigned long long) * MK_STEP_RING * 8));
@@ -1195,8 +1196,8 @@ static int launch_mega(cake_b200_ctx *c, const MkPlan &p) {
   cfg.numAttrs = 1;
   const MkArgs &a = p.a;
   bool pool = false;
-  for (int i = a.n_layers ? 0 : 4; i < (a.has_head ? 5 : 4); i++) pool = pool || a.g[i].pool < a.g[i].n_groups;
-  if (pool) CU(cudaMemsetAsync(c->tickets, 0, sizeof(unsigned) * (4 * (size_t)a.n_layers + 4), c->stream));  // a memset node in the graph
+  for (int i = 0; a.n_layers && i < 4; i++) pool = pool || a.g[i].pool < a.g[i].n_groups;
+  if (pool) CU(cudaMemsetAsync(c->tickets, 0, sizeof(unsigned) * 4 * (size_t)a.n_layers, c->stream));  // a memset node in the graph
   int rc = DISPATCH_T(c->cfg.dtype, T_LAMBDA {
     typedef typename decltype(tag_)::type T;
     return launch_mega_T<T>(c, &cfg, a);

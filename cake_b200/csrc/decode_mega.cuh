@@ -41,6 +41,7 @@ constexpr int MK_STAGE_BYTES = 32768;
 constexpr int MK_BATCH = 512;                   // row segments whose sums are kept until an epilogue takes them
 constexpr int MK_MAX_STAGES = 6;
 constexpr int MK_MAX_LAYERS = 96;
+constexpr int MK_HEAD_TICKET = 4 * MK_MAX_LAYERS;
 
 struct MkLayer {
   const void *wqkv, *wo, *wgu, *wd, *ln1, *ln2, *bqkv, *qn, *kn;
@@ -87,7 +88,8 @@ struct MkArgs {
   const unsigned long long *inbox_ctr;
   unsigned long long *peer_ctr;
   unsigned long long *ring_seq;   // hand-offs received so far (device-resident, never reset)
-  unsigned *tickets;          // [phase] work-claim counters, zeroed before every launch that has a phase with a pool
+  unsigned *tickets;          // [phase] work-claim counters: a layer's zeroed before every launch that has a layer's phase with a pool,
+                              // the head's (MK_HEAD_TICKET) by the last CTA of the launch in front
   int off_x, off_res, off_part, off_loc, off_rows;  // shared memory (mk_layout)
   unsigned long long *trace;  // optional: %globaltimer stamps of CTA 0 at phase boundaries (profiling aid)
   // always on (3 stores per launch): %globaltimer of CTA 0 at kernel entry / input acquired / exit, ring of
@@ -518,6 +520,7 @@ __device__ __forceinline__ void mk_head_end(const MkArgs &a, float *scratch, flo
     *a.token_out = (uint32_t)bidx;
     if (a.token_ring) a.token_ring[*a.d_step % a.ring_cap] = (uint32_t)bidx;
     *a.argmax_counter = 0;
+    a.tickets[MK_HEAD_TICKET] = 0;   // every CTA's producer has seen the end of the pool.  (A memset node in front of the kernel took 2.5 us of a 50 us head.)
     mk_end_of_step(a, scratch);  // this is the last CTA of the grid to finish
   }
 }
@@ -1052,7 +1055,7 @@ __global__ void __launch_bounds__(MK_THREADS, 1) decode_mega_kernel(const __grid
           const bool head = l == a.n_layers;
           const MkGeom &g = a.g[head ? 4 : ph];
           const void *W = head ? a.lm_head : ph == 0 ? L.wqkv : ph == 1 ? L.wo : ph == 2 ? L.wgu : L.wd;
-          mk_produce_gemv<T>(rg, g, W, a.tickets + 4 * l + ph, pol_w);
+          mk_produce_gemv<T>(rg, g, W, a.tickets + (head ? MK_HEAD_TICKET : 4 * l + ph), pol_w);
           if (head) break;
           if (ph == 0) mk_produce_attn<T>(rg, a, L, pos, pol_kv);
         }
