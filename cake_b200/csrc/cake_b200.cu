@@ -1189,12 +1189,17 @@ static int launch_mega(cake_b200_ctx *c, const MkPlan &p) {
   cfg.blockDim = dim3(MK_THREADS);
   cfg.dynamicSmemBytes = p.smem;
   cfg.stream = c->stream;
+  const MkArgs &a = p.a;
   cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeCooperative;  // all CTAs must be co-resident (grid barriers inside)
-  at[0].val.cooperative = 1;
+  if (a.n_layers || a.inbox_ctr) {
+    at[0].id = cudaLaunchAttributeCooperative;  // all CTAs must be co-resident (they wait for each other's packets)
+    at[0].val.cooperative = 1;
+  } else {  // the head alone: no CTA waits for another
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+  }
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  const MkArgs &a = p.a;
   bool pool = false;
   for (int i = 0; a.n_layers && i < 4; i++) pool = pool || a.g[i].pool < a.g[i].n_groups;
   if (pool) CU(cudaMemsetAsync(c->tickets, 0, sizeof(unsigned) * 4 * (size_t)a.n_layers, c->stream));  // a memset node in the graph

@@ -216,6 +216,7 @@ __device__ __forceinline__ void mk_produce_gemv(MkRing &rg, const MkGeom &g, con
 #pragma unroll 1
   for (int i = 0; i < n; i++) issue(first + i);
   if (g.pool == g.n_groups) return;
+  pdl_wait();   // (a head launched early: its counter is zeroed by a launch in front; else at once)
   unsigned next = atomicAdd(ticket, 1u);
 #pragma unroll 1
   while (g.pool + (int)next < g.n_groups) {
@@ -1065,6 +1066,8 @@ __global__ void __launch_bounds__(MK_THREADS, 1) decode_mega_kernel(const __grid
   }
 
   // ================= consumers ========================================================================
+  // A launch without layers is placed while the kernel in front ends (launch_mega), and its producer streams the static rows meanwhile.
+  pdl_wait();
   const int ct = threadIdx.x;
   __shared__ float rope_cs[256];  // cos (first 128) and sin (last 128) row of this step's position, as fp32
   {
