@@ -17,9 +17,10 @@
 //     has the release of the CTA's stores, its arrival, the poll and only then the load of the vector.
 // Bound by HBM where a layer's weights are large (8B: 436 MB a layer) and by the chain of five exchanges per layer where they are not
 // (0.6B: 31 MB, 5 us of stream).  With grid barriers and fp32 conversions in 16 warps: 32 us a layer at 0.6B, 24 tokens 25.1 ms, 8B two layers 187 us; now
-// 15 us, 14.1 ms and 182 us.  An exchange is 1.0 to 1.5 us (a barrier with the staging behind it 3 to 4.5), a product of 12 MB 2.1 us behind it.
+// 15 us, 14.1 ms and 184 to 186 us.  From a CTA's last row of a phase to the next phase's complete input 0.9 to 1.4 us pass at 0.6B and 3.3 to 4.2 at 8B, where CTAs
+// end further apart (9.5 behind the down product, whose groups are one row of 28 KB); a product of 12 MB takes 2.1 us behind it.
 // Arithmetic and rounding points are identical to the per-op kernels (gemv.cuh / attn_decode.cuh), correctly rounded divisions and square roots
-// included (a Newton step on the fast instructions in their place saved 0.3 of 14.3 ms over 24 tokens and was an ulp off in places); only the
+// included (a Newton step on the fast instructions in their place saved 0.3 ms over 24 tokens and was an ulp off in places); only the
 // fp32 summation order within a dot product differs (tests/test_gpu_parity.py::test_megakernel_equals_per_op_kernels).
 //
 // A packet buffer is written again one layer later; no reader may still be in front of it.  A CTA that has not gathered the input of

@@ -19,7 +19,7 @@ namespace mx {
     else { typedef __nv_bfloat16 T; __VA_ARGS__; }            \
   } while (0)
 // The kernels here wait for the one in front before their first access (griddepcontrol.wait) and, where they are small, are launched while it ends:
-// without that a step's chain of 24 launches of a few us each paid 2 us of launch latency each time (step through three Setodra blocks 358 -> 315 us).  Not so
+// without that a step's chain of 24 launches of a few us each paid 2 us of launch latency each time (step through three Setodra blocks 358 -> 317 us).  Not so
 // grids of more than two CTAs per SM, and not a recurrence over many tokens: CTAs placed while the kernel in front still holds most of the chip crowd
 // on the SMs that are free first (1000 tokens: 2200 -> 2434 us with all of them launched early).
 constexpr int MX_EARLY_CTAS_PER_SM = 2, MX_EARLY_TOKENS = 8;
