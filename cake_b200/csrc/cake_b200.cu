@@ -3061,7 +3061,7 @@ template <typename Take> static MoeScratch moe_scratch(const cake_b200_ctx *c, c
 }
 // The CTAs that a row's keys are cut over in latent attention's vector form (0: a warp per row and head).  A CTA walks its keys 16 at a time, a few us each:
 // 64 keys a split while two CTAs per SM take those of one row, 128 at most.  The rows of the call do not count, so that a row has the same sums
-// alone and in a batch: a step of the 2k model at 300 keys takes 313 us (311 with 32 keys a split, 327 with 128), one of 128 rows 1660
+// alone and in a batch: a step of the 2k model at 300 keys takes 313 us (311 with 32 keys a split), one of 128 rows 1660
 // (1720 with 32 keys, 1645 with 128).
 static int latent_splits(int sms, size_t rows, int heads, int n_keys) {
   if (rows * heads > 2048) return 0;
