@@ -290,7 +290,7 @@ def test_repeat_penalty_matches_oracle():
 def test_megakernel_equals_per_op_kernels(monkeypatch):
     """The persistent decode megakernel (decode_mega.cuh) and the per-op kernel chain (gemv.cuh +
     attn_decode.cuh, CAKE_B200_PER_OP=1) implement the same arithmetic with the same rounding points; only
-    the fp32 summation order inside a dot product differs (16 vs 8 consumer warps slice K differently), so
+    the fp32 summation order inside a dot product differs (lanes and warps slice K differently), so
     outputs agree to <= 2 ulp of D and greedy tokens (peaked head) are identical."""
     from cake_b200.model import B200Transformer, TextModelBase
     cfg = medium_config()
