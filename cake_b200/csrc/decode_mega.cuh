@@ -969,6 +969,7 @@ __device__ __forceinline__ void mk_consume_attn(MkRing &rg, const MkArgs &a, con
 #pragma unroll
       for (int i = 0; i < 8; i++) dst[g * HD + lane * 8 + i] = acc[g][i];
   }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // what was written into the stages (these sums, the appended row) comes before the next copy into them
   named_bar_sync(1, MK_CT);
   const int ns = it.n_split;
   uint64_t *pacc = a.pk.acc + (size_t)kvh * G * HD * a.nsplit, *pml = a.pk.ml + (size_t)kvh * G * a.nsplit * 2;  // [column][split], [head][split][2]
