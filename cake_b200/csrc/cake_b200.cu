@@ -1191,10 +1191,10 @@ static int launch_mega(cake_b200_ctx *c, const MkPlan &p) {
   cfg.stream = c->stream;
   const MkArgs &a = p.a;
   cudaLaunchAttribute at[1];
-  if (a.n_layers || a.inbox_ctr) {
+  if (a.n_layers || c->world > 1) {
     at[0].id = cudaLaunchAttributeCooperative;  // all CTAs must be co-resident (they wait for each other's packets)
     at[0].val.cooperative = 1;
-  } else {  // the head alone: no CTA waits for another
+  } else {  // the head alone: no CTA waits for another (on a rank of a ring it follows a transfer or waits for the inbox, and stays as it was)
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
   }
