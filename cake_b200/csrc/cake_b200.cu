@@ -1403,6 +1403,7 @@ static int gemm_tc_T(cake_b200_ctx *c, const void *A, const void *W, const void 
     sk.bias = bias; sk.residual = res; sk.C = C; sk.M = M; sk.N = N; sk.K = K; sk.ldc = ldc; sk.cap = cap;
     sk.act = act >= 0 ? act : (c->cfg.use_gelu_mlp ? 1 : 0);
     sk.tile_group = x.tile_group; sk.row_scale = x.row_scale; sk.err = c->wait_err;
+    sk.vec = (((uintptr_t)res | (uintptr_t)C) & 15) == 0 && ldc % 4 == 0;
     CUtensorMap ma, mw;
     RC(make_tmap(&ma, A, (uint64_t)M, (uint64_t)K, c->cfg.dtype, (uint32_t)sk.nt, (uint64_t)x.a_ld));
     RC(make_tmap(&mw, W, (uint64_t)N * x.n_groups, (uint64_t)K, c->cfg.dtype, SK_BM, 0, true));

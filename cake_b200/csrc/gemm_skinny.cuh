@@ -36,29 +36,64 @@ struct SkParams {
   int nt;                    // rows of A per tile (a multiple of 16)
   int m_tiles;               // row tiles, TC_BM rows apart
   int split, stages;
+  int vec;                   // C and the residual take accesses of four columns (their addresses and row strides)
   int *err;                  // host-mapped: a wait that ran out
 };
 
-// what an epilogue reads beside the sums, for row m of A at column n (rows past m_end: nothing)
+// What an epilogue reads beside the sums, four columns of row m of A from column n on (nothing where the row is not `in`)
+template <typename T, int EPI> struct SkRes {
+  static constexpr int WORDS = EPI == TCE_RESIDUAL_F32 ? 4 : EPI == TCE_RESIDUAL ? 2 : 1;
+  uint32_t w[WORDS];
+  __device__ __forceinline__ void load(const SkParams &p, bool in, int m, int n) {
+    if (!in) return;
+    if (EPI == TCE_RESIDUAL) {
+      const uint16_t *src = reinterpret_cast<const uint16_t *>(p.residual) + (size_t)m * (p.ldc ? p.ldc : p.N) + n;
+      const uint2 v = p.vec ? *reinterpret_cast<const uint2 *>(src) : make_uint2(src[0] | (uint32_t)src[1] << 16, src[2] | (uint32_t)src[3] << 16);
+      w[0] = v.x; w[WORDS > 1 ? 1 : 0] = v.y;
+    } else if (EPI == TCE_RESIDUAL_F32) {
+      const uint32_t *src = reinterpret_cast<const uint32_t *>(p.residual) + (size_t)m * p.N + n;
+      const uint4 v = p.vec ? *reinterpret_cast<const uint4 *>(src) : make_uint4(src[0], src[1], src[2], src[3]);
+      w[0] = v.x; w[WORDS > 1 ? 1 : 0] = v.y; w[WORDS > 2 ? 2 : 0] = v.z; w[WORDS > 3 ? 3 : 0] = v.w;
+    }
+  }
+};
+// the sums of row m, columns n .. n + 3 -> C
 template <typename T, int EPI>
-__device__ __forceinline__ float sk_residual(const SkParams &p, int m, int m_end, int n) {
-  if (m >= m_end) return 0.f;
-  if (EPI == TCE_RESIDUAL) return DT<T>::to_f(reinterpret_cast<const T *>(p.residual)[(size_t)m * (p.ldc ? p.ldc : p.N) + n]);
-  if (EPI == TCE_RESIDUAL_F32) return reinterpret_cast<const float *>(p.residual)[(size_t)m * p.N + n];
-  return 0.f;
-}
-template <typename T, int EPI>
-__device__ __forceinline__ void sk_store(const SkParams &p, int m, int m_end, int n, float v, float bias, float res) {
-  if (m >= m_end) return;
-  if (EPI == TCE_SOFTCAP_F32) {
-    reinterpret_cast<float *>(p.C)[(size_t)m * p.N + n] = p.cap > 0.f ? p.cap * tanhf(v / p.cap) : v;
-  } else if (EPI == TCE_RESIDUAL_F32) {
-    reinterpret_cast<float *>(p.C)[(size_t)m * p.N + n] = fmaf(p.row_scale ? p.row_scale[m] : 1.0f, v, res);
+__device__ __forceinline__ void sk_store(const SkParams &p, int m, int n, const float (&v)[4], const float (&bias)[4], const SkRes<T, EPI> &res) {
+  if (EPI == TCE_SOFTCAP_F32 || EPI == TCE_RESIDUAL_F32) {
+    float *dst = reinterpret_cast<float *>(p.C) + (size_t)m * p.N + n;
+    const float rs = EPI == TCE_RESIDUAL_F32 && p.row_scale ? p.row_scale[m] : 1.0f;
+    float o[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      if (EPI == TCE_RESIDUAL_F32) o[j] = fmaf(rs, v[j], __uint_as_float(res.w[j % SkRes<T, EPI>::WORDS]));
+      else o[j] = p.cap > 0.f ? p.cap * tanhf(v[j] / p.cap) : v[j];
+    }
+    if (p.vec) *reinterpret_cast<float4 *>(dst) = make_float4(o[0], o[1], o[2], o[3]);
+    else { dst[0] = o[0]; dst[1] = o[1]; dst[2] = o[2]; dst[3] = o[3]; }
+  } else if (EPI == TCE_SWIGLU) {  // columns 2i and 2i + 1 are gate and up
+    T *dst = reinterpret_cast<T *>(p.C) + (size_t)m * (p.ldc ? p.ldc : p.N / 2) + n / 2;
+    const uint32_t u = pack2x<T>(gated_pair<T>(v[0], v[1], p.act, p.cap), gated_pair<T>(v[2], v[3], p.act, p.cap));
+    if (p.vec) *reinterpret_cast<uint32_t *>(dst) = u;
+    else { reinterpret_cast<uint16_t *>(dst)[0] = (uint16_t)u; reinterpret_cast<uint16_t *>(dst)[1] = (uint16_t)(u >> 16); }
   } else {
-    float x = EPI == TCE_ACT ? plain_act<T>(v, p.act) : rnd<T>(v);
-    if (EPI == TCE_PLAIN && p.bias) x = rnd<T>(x + bias);
-    if (EPI == TCE_RESIDUAL) x += res;
-    reinterpret_cast<T *>(p.C)[(size_t)m * (p.ldc ? p.ldc : p.N) + n] = DT<T>::from_f(x);
+    float o[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      o[j] = EPI == TCE_ACT ? plain_act<T>(v[j], p.act) : rnd<T>(v[j]);
+      if (EPI == TCE_PLAIN && p.bias) o[j] = rnd<T>(o[j] + bias[j]);
+      if (EPI == TCE_RESIDUAL) {
+        const float2 r2 = DT<T>::unpack2(res.w[(j / 2) % SkRes<T, EPI>::WORDS]);
+        o[j] += j & 1 ? r2.y : r2.x;
+      }
+    }
+    T *dst = reinterpret_cast<T *>(p.C) + (size_t)m * (p.ldc ? p.ldc : p.N) + n;
+    const uint2 u = make_uint2(pack2x<T>(o[0], o[1]), pack2x<T>(o[2], o[3]));
+    if (p.vec) *reinterpret_cast<uint2 *>(dst) = u;
+    else {
+      uint16_t *d16 = reinterpret_cast<uint16_t *>(dst);
+      d16[0] = (uint16_t)u.x; d16[1] = (uint16_t)(u.x >> 16); d16[2] = (uint16_t)u.y; d16[3] = (uint16_t)(u.y >> 16);
+    }
   }
 }
 
@@ -154,16 +189,24 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   }
   if (!p.tile_group && warp > 1) pdl_wait();  // the residual, and C's previous readers, belong to the kernels in front
   const int wq = warp & 3;
-  const int n = n0 + wq * 32 + lane;
   const uint32_t trow = tmem + ((uint32_t)(wq * 32) << 16);
-  float bias = 0.f, res0 = 0.f, res1 = 0.f;
-  const int share = nt / S, f0 = m0 + rank * share;  // rows this CTA finishes: all of the tile, or its share (an even number) of them
+  const int share = nt / S, f0 = m0 + rank * share;  // rows this CTA finishes: all of the tile, or its share of them
   float *recv = reinterpret_cast<float *>(smem);     // sums on their way, over the drained ring: [source rank][row within the share][128 columns]
   bool go = warp >= 2 && live;                       // warps that finish rows
+  // A warp finishes its 32 columns four rows at a time, a lane four columns of one row: loads and stores of 8 bytes (16 of fp32), and the
+  // residual of four passes is on its way.  (A thread per column took a pair of rows at a time, each behind its residual's way from L2: 0.1
+  // us a row, 35.9 us for N = K = 4096, 200 rows.  Eight columns a lane: the gated form's code is twice as long, and a step of one row,
+  // which runs it once, waits for it: 187 -> 189 us for four Nigenex layers.)
+  const int fr = lane >> 3, fc = wq * 32 + (lane & 7) * 4, fn = n0 + fc;
+  float bias[4] = {0.f, 0.f, 0.f, 0.f};
+  SkRes<T, EPI> res[4];
   if (go) {
-    if (EPI == TCE_PLAIN && p.bias) bias = DT<T>::to_f(reinterpret_cast<const T *>(p.bias)[n]);
-    res0 = sk_residual<T, EPI>(p, f0, m_end, n);
-    res1 = sk_residual<T, EPI>(p, f0 + 1, m_end, n);
+    if (EPI == TCE_PLAIN && p.bias) {
+#pragma unroll
+      for (int j = 0; j < 4; j++) bias[j] = DT<T>::to_f(reinterpret_cast<const T *>(p.bias)[fn + j]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) res[i].load(p, fr + 4 * i < share && f0 + fr + 4 * i < m_end, f0 + fr + 4 * i, fn);
     mbar_wait_lim(&acc_full, 0, p.err, left);
     go = __all_sync(0xffffffffu, left != 0);
     tc_fence_after();
@@ -192,44 +235,37 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     cluster_arrive();
     cluster_wait();
   }
-  // The last pass is a loop of one pair of rows, not straight-line code: a kernel of a few microseconds runs its epilogue once, and
-  // unrolled over 16 rows it waited for its own instructions (233 -> 315 us for four Nigenex layers).  The residual of the next pair is
-  // requested before this pair is stored: C may be the residual's own buffer.
+  // The last pass is a loop, not straight-line code: a kernel of a few microseconds runs its epilogue once, and unrolled over 16 rows it
+  // waited for its own instructions (233 -> 315 us for four Nigenex layers).  A row's residual is read by the lane that stores it, before
+  // it does: C may be the residual's own buffer.
   if (go) {
-    const int step = S == 1 ? 16 : share;
-    float *mine = recv + wq * 32 + lane;
+    const float *src0 = recv + (size_t)fr * SK_BM + fc;
 #pragma unroll 1
-    for (int c0 = 0; c0 < share && f0 + c0 < m_end; c0 += step) {
-      if (S == 1) {  // through shared memory too: the thread's own column, 16 rows at a time
+    for (int c0 = 0; c0 < share && f0 + c0 < m_end; c0 += 4) {
+      const float *src = src0 + (size_t)(S == 1 ? c0 & 12 : c0) * SK_BM;
+      if (S == 1 && !(c0 & 12)) {  // through shared memory too: the warp's own columns, 16 rows at a time
         uint32_t r[16];
         tc_ld16(trow + (uint32_t)c0, r);
+        float *mine = recv + wq * 32 + lane;
+        __syncwarp();
 #pragma unroll
         for (int j = 0; j < 16; j++) mine[j * SK_BM] = __uint_as_float(r[j]);
+        __syncwarp();
       }
-#pragma unroll 1
-      for (int c = 0; c < step; c += 2) {
-        const int m = f0 + c0 + c;
-        if (m >= m_end) break;
-        float v0 = 0.f, v1 = 0.f;
+      const int m = f0 + c0 + fr;
+      SkRes<T, EPI> ahead;
+      ahead.load(p, c0 + fr + 16 < share && m + 16 < m_end, m + 16, fn);
+      if (c0 + fr < share && m < m_end) {
+        float v[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 2
-        for (int q = 0; q < S; q++) {
-          v0 += mine[(q * share + c) * SK_BM];
-          v1 += mine[(q * share + c + 1) * SK_BM];
+        for (int q = 0; q < S; q++, src += (size_t)share * SK_BM) {
+          const float4 x = *reinterpret_cast<const float4 *>(src);
+          v[0] += x.x; v[1] += x.y; v[2] += x.z; v[3] += x.w;
         }
-        if (EPI == TCE_SWIGLU) {  // columns 2i and 2i + 1 are gate and up: the even lane finishes row m, the odd lane row m + 1
-          const bool odd = (n & 1) != 0;
-          const float got = __shfl_xor_sync(0xffffffffu, odd ? v0 : v1, 1);
-          const float g = odd ? got : v0, u = odd ? v1 : got;
-          const int row = m + (odd ? 1 : 0);
-          if (row < m_end) reinterpret_cast<T *>(p.C)[(size_t)row * (p.ldc ? p.ldc : p.N / 2) + n / 2] = DT<T>::from_f(gated_pair<T>(g, u, p.act, p.cap));
-        } else {
-          const float n0r = sk_residual<T, EPI>(p, m + 2, m_end, n), n1r = sk_residual<T, EPI>(p, m + 3, m_end, n);
-          sk_store<T, EPI>(p, m, m_end, n, v0, bias, res0);
-          sk_store<T, EPI>(p, m + 1, m_end, n, v1, bias, res1);
-          res0 = n0r;
-          res1 = n1r;
-        }
+        sk_store<T, EPI>(p, m, fn, v, bias, res[0]);
       }
+      res[0] = res[1]; res[1] = res[2]; res[2] = res[3];
+      res[3] = ahead;
     }
   }
   if (!left) gave_up = 1;
