@@ -8,15 +8,18 @@
 // silu(gate)*up on the row-interleaved Wgu (mlp.rs:22-28).  Rounding points as everywhere: the fp32
 // accumulator is rounded to D before any epilogue op.
 //
-// Structure (one persistent CTA per SM, 256 threads, warp-specialised):
+// Structure (one persistent CTA per SM, 384 threads, warp-specialised):
 //   warp 0   TMA producer: cp.async.bulk.tensor.2d of a 128x64 A tile and a W tile (128 or 256 rows, or this CTA's half of 256 as
 //            one of a pair) per k-block into a 4- or 6-stage shared-memory ring, 128-byte swizzle, completion on full[] mbarriers
 //   warp 1   MMA issuer: one thread issues tcgen05.mma.kind::f16 (M = 128 with cta_group::1, 256 over a pair of SMs with
 //            cta_group::2; N = 128 or 256; K = 16) x4 per k-block from shared-memory descriptors into one of two TMEM
 //            accumulators (128 lanes x BN fp32 columns each); tcgen05.commit releases the smem stage / publishes the accumulator
 //   warp 2   TMEM allocator (2 x BN columns)
-//   warps 4-7  epilogue: tcgen05.ld 32x32b.x32 (thread = accumulator row), fused epilogue, 16-byte global
-//            stores; overlaps with the MMAs of the next tile through the second accumulator
+//   warps 4-11  epilogue: tcgen05.ld 32x32b.x32 (thread = accumulator row, every other warp of the same rows the other half of the
+//            columns), fused epilogue, 16-byte global stores; overlaps with the MMAs of the next tile through the second accumulator.
+//            Two warps per scheduler, because one alone issued an instruction every six cycles: 65,000 cycles for a gated tile of
+//            128 x 256, twice its products' time (64 experts of 2816 x 2048 for 1000 tokens: 230 -> 180 us, an instruction budget of the
+//            divisions and exponentials; four warps per scheduler 176).
 #pragma once
 #include <cuda.h>
 
@@ -27,7 +30,7 @@ namespace cake {
 // Tile: 128 x BN with BN in {128, 256}.  A 128x128 tile needs 32 KB of operands per 2.1 MFLOP k-block = 64 flop/B, i.e.
 // ~240 GB/s per SM at the tensor peak — more than one SM pulls out of L2, which capped the kernel at ~55 % tensor-pipe
 // activity.  128x256 (all 512 TMEM columns: two 128x256 fp32 accumulators) moves 48 KB per 4.2 MFLOP = 87 flop/B.
-constexpr int TC_BM = 128, TC_BK = 64, TC_THREADS = 256;
+constexpr int TC_BM = 128, TC_BK = 64, TC_EPI_WARPS = 8, TC_THREADS = 128 + 32 * TC_EPI_WARPS;
 constexpr int TC_BN = 128;                     // granularity the host checks N against (BN = 256 when N % 256 == 0)
 template <int BN, bool PAIR = false> struct TcCfg {
   static constexpr int STAGES = (BN == 256 && !PAIR) ? 4 : 6;
@@ -187,7 +190,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < Cfg::STAGES; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-    for (int a = 0; a < 2; a++) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], PAIR ? 8 : 4); }  // (a warp of the epilogue arrives once)
+    for (int a = 0; a < 2; a++) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], (PAIR ? 2 : 1) * TC_EPI_WARPS); }  // (a warp of the epilogue arrives once)
     mbar_init(drained, 1);
     *gave_up = 0;
     mbar_fence_init();
@@ -310,11 +313,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       }
     }
   } else if (warp >= 4) {
-    // ===================== epilogue warps (TMEM lanes 32*(warp%4) .. +32) ================================
-    const int wq = warp & 3;
+    // ===================== epilogue warps (TMEM lanes 32*(warp%4) .. +32, every fourth warp the same lanes and another range of columns) ====
+    constexpr int CW = BN / (TC_EPI_WARPS / 4);  // columns of a warp
+    const int wq = warp & 3, cw0 = ((warp - 4) >> 2) * CW;
     const T *bias = reinterpret_cast<const T *>(p.bias);
     const T *res = reinterpret_cast<const T *>(p.residual);
     T *C = reinterpret_cast<T *>(p.C);
+    const int ld = p.ldc ? p.ldc : EPI == TCE_SWIGLU ? p.N / 2 : p.N;
     int it = 0;
     for (int t = first; t < n_units; t += stride) {
       int m0, n0;
@@ -324,26 +329,36 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       const uint32_t aph = (uint32_t)(it >> 1) & 1u;
       it++;
       const int row = m0 + wq * 32 + lane;
+      // the residual of a chunk of 32 columns: the first one is on its way while the products run, the next one while a chunk is finished
+      constexpr int RW = EPI == TCE_RESIDUAL ? 4 : EPI == TCE_RESIDUAL_F32 ? 8 : 1;
+      uint4 rr[RW];
+      auto load_res = [&](int col) {
+        if ((EPI != TCE_RESIDUAL && EPI != TCE_RESIDUAL_F32) || row >= p.M) return;
+        const uint4 *r4 = EPI == TCE_RESIDUAL ? reinterpret_cast<const uint4 *>(res + (size_t)row * ld + h * p.c_step + col)
+                                              : reinterpret_cast<const uint4 *>(reinterpret_cast<const float *>(p.residual) + (size_t)row * p.N + col);
+#pragma unroll
+        for (int j = 0; j < RW; j++) rr[j] = r4[j];
+      };
+      load_res(n0 + cw0);
       mbar_wait_lim(&acc_full[a], aph, p.err, left);
       if (!__all_sync(0xffffffffu, left != 0)) break;
       tc_fence_after();
 #pragma unroll 1
-      for (int c0 = 0; c0 < BN; c0 += 32) {
+      for (int c0 = cw0; c0 < cw0 + CW; c0 += 32) {
         uint32_t r[32];
         tc_ld32(tmem_base + ((uint32_t)(wq * 32) << 16) + (uint32_t)(a * BN + c0), r);
         if (row < p.M) {
           if (EPI == TCE_SWIGLU) {
             uint32_t o[8];
+            auto pairs = [&](int act) {
 #pragma unroll
-            for (int j = 0; j < 8; j++) {
-              float v[2];
-#pragma unroll
-              for (int h = 0; h < 2; h++) {
-                v[h] = gated_pair<T>(__uint_as_float(r[4 * j + 2 * h]), __uint_as_float(r[4 * j + 2 * h + 1]), p.act, p.cap);
-              }
-              o[j] = pack2<T>(v[0], v[1]);
-            }
-            uint4 *dst = reinterpret_cast<uint4 *>(C + (size_t)row * (p.ldc ? p.ldc : p.N / 2) + (n0 + c0) / 2);
+              for (int j = 0; j < 8; j++)
+                o[j] = pack2x<T>(gated_pair<T>(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]), act, p.cap),
+                                 gated_pair<T>(__uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]), act, p.cap));
+            };
+            if (p.act == 0) pairs(0);  // the common one without a branch per pair
+            else pairs(p.act);
+            uint4 *dst = reinterpret_cast<uint4 *>(C + (size_t)row * ld + (n0 + c0) / 2);
             dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
             dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
           } else if (EPI == TCE_SOFTCAP_F32) {
@@ -359,30 +374,22 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
               dst[j] = make_float4(v[0], v[1], v[2], v[3]);
             }
           } else if (EPI == TCE_RESIDUAL_F32) {
-            const size_t off = (size_t)row * p.N + n0 + c0;
-            const float4 *r4 = reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(p.residual) + off);
-            float4 *dst = reinterpret_cast<float4 *>(reinterpret_cast<float *>(p.C) + off);
+            float4 *dst = reinterpret_cast<float4 *>(reinterpret_cast<float *>(p.C) + (size_t)row * p.N + n0 + c0);
             const float rs = p.row_scale ? p.row_scale[row] : 1.0f;
 #pragma unroll
             for (int j = 0; j < 8; j++) {
-              float4 v = r4[j];
-              v.x = fmaf(rs, __uint_as_float(r[4 * j]), v.x); v.y = fmaf(rs, __uint_as_float(r[4 * j + 1]), v.y);
-              v.z = fmaf(rs, __uint_as_float(r[4 * j + 2]), v.z); v.w = fmaf(rs, __uint_as_float(r[4 * j + 3]), v.w);
-              dst[j] = v;
+              const uint4 q = rr[j % RW];
+              r[4 * j] = __float_as_uint(fmaf(rs, __uint_as_float(r[4 * j]), __uint_as_float(q.x)));
+              r[4 * j + 1] = __float_as_uint(fmaf(rs, __uint_as_float(r[4 * j + 1]), __uint_as_float(q.y)));
+              r[4 * j + 2] = __float_as_uint(fmaf(rs, __uint_as_float(r[4 * j + 2]), __uint_as_float(q.z)));
+              r[4 * j + 3] = __float_as_uint(fmaf(rs, __uint_as_float(r[4 * j + 3]), __uint_as_float(q.w)));
             }
+            if (c0 + 32 < cw0 + CW) load_res(n0 + c0 + 32);
+#pragma unroll
+            for (int j = 0; j < 8; j++) reinterpret_cast<uint4 *>(dst)[j] = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
           } else {
             uint32_t o[16];
-            const size_t off = (size_t)row * (p.ldc ? p.ldc : p.N) + h * p.c_step + n0 + c0;  // TCE_PLAIN may write a column range of a wider buffer
-            uint32_t rr[16];  // the residual row segment as four 16-byte loads (scalar 2-byte loads made this epilogue longer
-                              // than a K=4096 main loop: ncu, o_proj 68 % tensor-pipe active against 88-91 % elsewhere)
-            if (EPI == TCE_RESIDUAL) {
-              const uint4 *r4 = reinterpret_cast<const uint4 *>(res + off);
-#pragma unroll
-              for (int j = 0; j < 4; j++) {
-                const uint4 v = r4[j];
-                rr[4 * j] = v.x; rr[4 * j + 1] = v.y; rr[4 * j + 2] = v.z; rr[4 * j + 3] = v.w;
-              }
-            }
+            const size_t off = (size_t)row * ld + h * p.c_step + n0 + c0;  // TCE_PLAIN may write a column range of a wider buffer
 #pragma unroll
             for (int j = 0; j < 16; j++) {
               float v0, v1;
@@ -398,12 +405,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 v1 = rnd<T>(v1 + DT<T>::to_f(bias[n0 + c0 + 2 * j + 1]));
               }
               if (EPI == TCE_RESIDUAL) {
-                const float2 rv = DT<T>::unpack2(rr[j]);
+                const uint4 q = rr[(j / 4) % RW];
+                const float2 rv = DT<T>::unpack2((j & 3) == 0 ? q.x : (j & 3) == 1 ? q.y : (j & 3) == 2 ? q.z : q.w);
                 v0 += rv.x;
                 v1 += rv.y;
               }
-              o[j] = pack2<T>(v0, v1);
+              o[j] = pack2x<T>(v0, v1);
             }
+            if (c0 + 32 < cw0 + CW) load_res(n0 + c0 + 32);
             uint4 *dst = reinterpret_cast<uint4 *>(C + off);
 #pragma unroll
             for (int j = 0; j < 4; j++) dst[j] = make_uint4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
