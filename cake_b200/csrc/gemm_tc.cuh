@@ -185,7 +185,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   int *gave_up = reinterpret_cast<int *>(tmem_ptr + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tiles_m = (p.M + TC_BM - 1) / TC_BM, tiles_n = p.N / BN;
+  int tiles_m = (p.M + TC_BM - 1) / TC_BM;
+  const int tiles_n = p.N / BN;
   const int kblocks = p.K / TC_BK;
 
   if (threadIdx.x == 0) {
@@ -211,6 +212,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   pdl_launch_dependents();
   if (!p.w_early || warp != 0) pdl_wait();
   const uint32_t tmem_base = *tmem_ptr;
+  // (83 of 111 blocks in use, 1000 tokens: dealt out with the empty ones some SMs had 7.8 tiles of 6.2; three layers 1981 -> 1922 us)
+  if (p.tile_group) {  // row blocks behind the last one in use don't count: the tiles are dealt out over the chip without them
+    int used = 0;
+    for (int i = lane; i < tiles_m; i += 32)
+      if (p.tile_group[i] >= 0) used = i + 1;
+    tiles_m = __reduce_max_sync(0xffffffffu, used);
+  }
   // work distribution: one tile per CTA and round; PAIR: one (256-row, 256-column) unit per cluster and round
   const uint32_t crank = PAIR ? cluster_rank() : 0u;
   const int first = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, stride = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
