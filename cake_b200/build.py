@@ -43,6 +43,7 @@ def stale() -> bool:
 UNITS = {
     "cake_b200.o": ("cake_b200.cu", None),
     "mixers.o": ("mixers.cu", ("mixers.cuh", "common.cuh")),
+    "mixers_chunks.o": ("mixers_chunks.cu", ("mixers.cuh", "common.cuh")),
     "mixers_window.o": ("mixers_window.cu", ("mixers.cuh", "common.cuh")),
     "mixers_streams.o": ("mixers_streams.cu", ("mixers.cuh", "common.cuh")),
 }

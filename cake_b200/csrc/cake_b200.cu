@@ -3025,7 +3025,7 @@ static int cache_ensure_mixer(cake_b200_cache *k, int layer, const cake_b200_blo
 // scratch of one block for M rows, carved from the ctx arena (base == nullptr: sizes only)
 struct MixerScratch {
   void *h, *proj, *qa, *lat, *att, *conv, *pw;
-  float *o32, *part, *scores;
+  float *o32, *part, *scores, *rec;
   int nsplit, lat_tok;
   MoeScratch moe;
   size_t total;
@@ -3096,6 +3096,8 @@ static MixerScratch mixer_scratch(const cake_b200_ctx *c, const cake_b200_block 
     }
   } else {
     s.o32 = (float *)take(M * inner * sizeof(float));
+    const size_t rec = mx::recurrence_scratch((int)(M / S), S, sp.heads, sp.kind == CAKE_B200_MIX_STATE_SPACE ? sp.state : sp.dim, sp.vdim);
+    if (rec) s.rec = (float *)take(rec);
     if (sp.kind == CAKE_B200_MIX_STATE_SPACE) s.conv = take(M * (inner + 2 * (size_t)sp.groups * sp.state) * es);
   }
   s.moe = moe_scratch(c, b, M, take);
@@ -3262,6 +3264,7 @@ static int enqueue_mixer_layers(cake_b200_ctx *c, cake_b200_block *const *blocks
         const T *pj = (const T *)w.proj;
         mx::Recurrence r{pj, pj + qk, pj + 2 * qk, b->n_in_pad, b->n_in_pad, b->n_in_pad, 1, nullptr, 0, nullptr, nullptr, nullptr, b->m_decay,
                          1.0f / sqrtf((float)sp.dim), b->m_cos, b->m_sin, sp.rot.dims, kc->rec_state[l], w.o32, B, S, sp.heads, sp.dim, sp.vdim, pos0};
+        r.scratch = w.rec;
         MX(mx::recurrence(st, dt, r, lc));
         mx::GateNorm gn{w.o32, pj + 2 * qk + inner, b->n_in_pad, nullptr, w.att, M, inner, sp.heads, 0, c->cfg.rms_eps};
         MX(mx::gate_norm(st, dt, gn, lc));
@@ -3272,6 +3275,7 @@ static int enqueue_mixer_layers(cake_b200_ctx *c, cake_b200_block *const *blocks
         MX(mx::short_conv(st, dt, sc, lc));
         mx::Recurrence r{cv + inner + gn_, cv + inner, cv, ch, ch, ch, sp.heads / sp.groups, pj + inner + ch, b->n_in_pad, b->m_dt_bias, b->m_a_log, b->m_d,
                          nullptr, 1.0f, nullptr, nullptr, 0, kc->rec_state[l], w.o32, B, S, sp.heads, sp.state, sp.vdim, pos0};
+        r.scratch = w.rec;
         MX(mx::recurrence(st, dt, r, lc));
         mx::GateNorm gn{w.o32, pj, b->n_in_pad, b->m_norm, w.att, M, inner, sp.norm_groups, 1, c->cfg.rms_eps};
         MX(mx::gate_norm(st, dt, gn, lc));
@@ -4216,6 +4220,28 @@ extern "C" int cake_b200_debug_product(cake_b200_ctx *c, int epi, const void *A,
     }
   }));
   return sync_results(c);
+}
+
+/* a test aid (not in the public header): the gated recurrence on given buffers, in chunks where scratch is wanted and its rule takes them.
+ * ptrs: q, k, v, dt, dt_bias, a_log, skip, decay, cos, sin, state, o, a_tok, b_tok; dims: ldq, ldk, ldv, group_div, lddt, rope_dims, B, S, heads, dk, dv,
+ * pos0.  *launches: kernels it took. */
+extern "C" int cake_b200_debug_recurrence(cake_b200_ctx *c, const void *const *ptrs, const int *dims, float kscale, int with_scratch, int *launches) {
+  if (!c || !ptrs || !dims || !launches) return fail(CAKE_B200_EINVAL, "null argument");
+  CU(cudaSetDevice(c->device));
+  RC(wait_loads(c));
+  mx::Recurrence r{ptrs[0], ptrs[1], ptrs[2], dims[0], dims[1], dims[2], dims[3], ptrs[3], dims[4], ptrs[4], ptrs[5], ptrs[6], (const float *)ptrs[7], kscale,
+                   (const float *)ptrs[8], (const float *)ptrs[9], dims[5], (float *)const_cast<void *>(ptrs[10]), (float *)const_cast<void *>(ptrs[11]),
+                   dims[6], dims[7], dims[8], dims[9], dims[10], dims[11]};
+  r.a_tok = (const float *)ptrs[12];
+  r.b_tok = (const float *)ptrs[13];
+  const size_t bytes = with_scratch ? mx::recurrence_scratch(r.B, r.S, r.heads, r.dk, r.dv) : 0;
+  if (bytes) CU(cudaMalloc(&r.scratch, bytes));
+  uint64_t n = 0;
+  const int e = mx::recurrence(c->stream, c->cfg.dtype, r, &n);
+  const int rc = sync_results(c);
+  if (r.scratch) cudaFree(r.scratch);
+  *launches = (int)n;
+  return e ? fail(CAKE_B200_ECUDA, "recurrence: %s", cudaGetErrorString((cudaError_t)e)) : rc;
 }
 
 /* test aids (not in the public header): the split rule of latent attention's vector form, that attention on given buffers (part: [B S heads, nsplit,

@@ -861,7 +861,12 @@ int recurrence(cudaStream_t st, int dtype, const Recurrence &p, uint64_t *launch
     const int e = recurrence_channels(st, dtype, p);
     if (e == (int)cudaSuccess) MX_DONE(1);
     if (e != (int)cudaErrorNotSupported) return e;
-  } else if (p.dk % RC_RS == 0 && p.dv % RC_CB == 0) {
+  }
+  int n_chunk_launches = 0;
+  const int ce = recurrence_chunks(st, dtype, p, &n_chunk_launches);
+  if (ce == (int)cudaSuccess) MX_DONE(n_chunk_launches);
+  if (ce != (int)cudaErrorNotSupported) return ce;
+  if (!p.a_chan && p.dk % RC_RS == 0 && p.dv % RC_CB == 0) {
     cudaError_t e = cudaErrorNotSupported;
     MX_DISPATCH(dtype, {
       switch (p.dk / RC_RS) {

@@ -4,7 +4,7 @@
 // with exponential gates), the gated delta rule, softmax attention whose heads are mixed after the softmax, short causal
 // convolutions, grouped unit norms with gates, norms and merges of sublayer outputs on the fp32 stream, several residual
 // streams and their mixing, embeddings with pair and position tables, and a mixture of experts with identity experts.  The kernels live
-// in mixers.cu, mixers_window.cu and mixers_streams.cu, translation units of their own; the entry points below take plain device pointers and a stream, so that any block
+// in mixers.cu, mixers_chunks.cu, mixers_window.cu and mixers_streams.cu, translation units of their own; the entry points below take plain device pointers and a stream, so that any block
 // structure can combine them.  Every function returns a cudaError_t cast to int and adds its launches to *launches.
 //
 // Nothing here follows a reference file: the reference has none of these layers.
@@ -101,8 +101,16 @@ struct Recurrence {
   // no dt / a_tok / skip); q is multiplied by qscale
   const float *a_chan = nullptr;
   float qscale = 1.f;
+  float *scratch = nullptr;  // recurrence_scratch() bytes, 16-byte aligned; nullptr: always token by token
 };
 int recurrence(cudaStream_t, int dtype, const Recurrence &, uint64_t *launches);
+// The form in chunks of tokens (mixers_chunks.cu); cudaErrorNotSupported for what it does not cover.  Three kernels of together 28 us or more against one
+// that walks its tokens: 16 heads of 128 x 128 in us, walked / in chunks: 128 tokens 31 / 28, 256 59 / 28, 1000 223 / 74; 64 heads of 128 x 64:
+// 192 37 / 41, 256 49 / 41, 1000 181 / 126, 4 x 256 150 / 128.  So from 256 tokens on, whatever the batch.
+constexpr int CHUNK_MIN_TOKENS = 256;
+// its scratch (0: not needed)
+size_t recurrence_scratch(int B, int S, int heads, int dk, int dv);
+int recurrence_chunks(cudaStream_t, int dtype, const Recurrence &, int *n_launches);
 // the register-tiled form with a decay per key channel; cudaErrorNotSupported for shapes it does not cover (recurrence() then
 // takes the kernel with the state in shared memory)
 int recurrence_channels(cudaStream_t, int dtype, const Recurrence &);
