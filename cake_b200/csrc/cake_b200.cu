@@ -437,8 +437,10 @@ template <typename T> static int set_smem_attrs_T() {
   CU(cudaFuncSetAttribute(gemm_tc_kernel<T, EPI, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<256>::SMEM_BYTES));      \
   CU(cudaFuncSetAttribute(gemm_tc_kernel<T, EPI, 256, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<256, true>::SMEM_BYTES));
 #define SETK(EPI)                                                                                                                 \
-  CU(cudaFuncSetAttribute(gemm_skinny_kernel<T, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, SK_SMEM_MAX));                  \
-  CU(cudaFuncSetAttribute(gemm_skinny_kernel<T, EPI>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+  CU(cudaFuncSetAttribute(gemm_skinny_kernel<T, EPI, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SK_SMEM_MAX));                  \
+  CU(cudaFuncSetAttribute(gemm_skinny_kernel<T, EPI, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SK_SMEM_MAX));                  \
+  CU(cudaFuncSetAttribute(gemm_skinny_kernel<T, EPI, true>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));\
+  CU(cudaFuncSetAttribute(gemm_skinny_kernel<T, EPI, false>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
   SETK(TCE_PLAIN) SETK(TCE_RESIDUAL) SETK(TCE_SWIGLU) SETK(TCE_RESIDUAL_F32) SETK(TCE_SOFTCAP_F32) SETK(TCE_ACT)
 #undef SETK
   SETT(TCE_PLAIN) SETT(TCE_RESIDUAL) SETT(TCE_SWIGLU) SETT(TCE_RESIDUAL_F32) SETT(TCE_SOFTCAP_F32) SETT(TCE_ACT)
@@ -1363,9 +1365,10 @@ static int tc_kind(int sms, int M, int N, int K, bool pairs) {
     if (tc_us(sms, M, N, K, k) < tc_us(sms, M, N, K, best)) best = k;
   return best;
 }
-// skinny: what its stages carry at the 8.9 TB/s that all SMs take in together (or W from HBM), and an epilogue that grows with the rows
-static double skinny_us(int nt, int N, int K) {
-  return std::max((double)(N / SK_BM) * (K / TC_BK) * sk_stage_bytes(nt) / 8.9e6, 2.0 * N * K / 6.4e6) + 5.5 + 0.035 * nt;
+// skinny: what a CTA's stages carry at 80 KB/us an SM (or W from HBM), and an exchange and epilogue that grow with the rows (128 rows, four CTAs a slice:
+// N = K = 4096 13.9, K = 14336 29.2; 200 rows 16.5, 35.7; within 15 % where the cut fills the chip)
+static double skinny_us(int sms, int nt, int N, int K, int ctas, int kblocks) {
+  return std::max((double)((ctas + sms - 1) / sms) * kblocks * sk_stage_bytes(nt) / 80e3, 2.0 * N * K / 6.4e6) + 3.5 + 0.03 * nt;
 }
 // gemm_skinny_kernel's shape for a product, or false where gemm_tc_kernel takes it.
 static bool plan_skinny(int sms, int M, int N, int K, const TcExtra &x, SkParams *p, size_t *smem) {
@@ -1373,20 +1376,33 @@ static bool plan_skinny(int sms, int M, int N, int K, const TcExtra &x, SkParams
   const int rows = x.tile_group ? x.group_rows : M;
   if (rows < 1 || rows > (x.tile_group ? 64 : SK_MAX_ROWS)) return false;
   p->nt = (rows + 15) / 16 * 16;
-  if (!x.tile_group && rows > 64 && skinny_us(p->nt, N, K) >= tc_us(sms, M, N, K, tc_kind(sms, M, N, K, true))) return false;
   p->m_tiles = x.tile_group ? M / TC_BM : 1;
   const int tiles = N / SK_BM * p->m_tiles;
-  // The cut along K: as many CTAs as stay resident at once (three per SM up to 64 rows, two up to 112, one beyond: a ring has three stages or
-  // more), each with at least two k-blocks.  N = 6144, K = 4096, 16 rows: 48 slices x 1 21.9 us, x 2 14.7, x 4 12.7, x 8 11.2 (three per SM) -
-  // 15.3 with rings that let only two in, a second wave.
+  // The cut along K, each CTA with at least two k-blocks: as many CTAs as stay resident at once (three per SM up to 64 rows, two up to 112, one
+  // beyond: a ring has three stages or more), but a second one per SM only with four k-blocks each and a third with eight (us, S CTAs per slice:
+  // 37 rows, N = 4096, K = 1024: S = 4 5.9, S = 8 6.8; N = 6144: 2 8.2, 4 6.8, 8 12.6; 16 rows, N = 6144, K = 4096: 2 13.6, 4 12.1, 8 11.3), and
+  // clusters of eight CTAs that fill an SM each only on half of the chip (128 rows, N = K = 2048: S = 4 9.9, S = 8 17.2: the last of sixteen clusters waits
+  // for a free GPC).
   const int most = p->nt <= 64 ? 3 : p->nt < 128 ? 2 : 1;
   p->split = 1;
-  while (p->split < SK_MAX_SPLIT && tiles * p->split * 2 <= most * sms && K / TC_BK >= p->split * 4) p->split *= 2;
-  const int per_sm = std::min(most, (tiles * p->split + sms - 1) / sms);
-  const size_t budget = (size_t)(per_sm == 3 && p->split > 1 ? 74 : most == 1 ? 180 : 110) * 1024 - 1536;
-  p->stages = std::min(SK_MAX_STAGES, std::max(2, (int)(budget / sk_stage_bytes(p->nt))));
-  *smem = sk_smem_bytes(p->nt, p->stages, p->split);
-  return *smem <= SK_SMEM_MAX;
+  while (p->split < SK_MAX_SPLIT) {
+    const int ctas = tiles * p->split * 2, kblocks = K / TC_BK / (p->split * 2);
+    if (ctas > most * sms || kblocks < (ctas <= sms ? 2 : ctas <= 2 * sms ? 4 : 8) || (most == 1 && p->split == 4 && ctas > sms / 2)) break;
+    p->split *= 2;
+  }
+  for (;; p->split /= 2) {  // (240 rows leave no room for the sums of a cluster of eight)
+    const int per_sm = std::min(most, (tiles * p->split + sms - 1) / sms);
+    const size_t budget = (size_t)(per_sm == 3 && p->split > 1 ? 74 : most == 1 ? 180 : 110) * 1024 - 1536;
+    const int kblocks = (K / TC_BK + p->split - 1) / p->split;  // of a CTA: no more stages than that, three at least
+    p->stages = std::min(std::min(SK_MAX_STAGES, std::max(2, (int)(budget / sk_stage_bytes(p->nt)))), std::max(3, kblocks));
+    p->how = p->split > 1 && sk_smem_bytes(p->nt, p->stages, p->split, SK_APART) <= budget + 1280 ? SK_APART : SK_OVER;
+    if (p->split > 1 && p->nt / p->split % 32 == 0 && sk_smem_bytes(p->nt, p->stages, p->split, p->how) > SK_SMEM_MAX) p->how = SK_LEAN;
+    *smem = sk_smem_bytes(p->nt, p->stages, p->split, p->how);
+    if (*smem <= SK_SMEM_MAX || p->split == 1) break;
+  }
+  if (*smem > SK_SMEM_MAX) return false;
+  return x.tile_group || rows <= 64 ||
+         skinny_us(sms, p->nt, N, K, tiles * p->split, (K / TC_BK + p->split - 1) / p->split) < tc_us(sms, M, N, K, tc_kind(sms, M, N, K, true));
 }
 // gemm_tc_kernel's tile: the one whose rounds over the chip come out shortest; a grouped product's neighbours belong to different groups, and a
 // wrapping W has no halves
@@ -1403,11 +1419,11 @@ static int gemm_tc_T(cake_b200_ctx *c, const void *A, const void *W, const void 
     sk.bias = bias; sk.residual = res; sk.C = C; sk.M = M; sk.N = N; sk.K = K; sk.ldc = ldc; sk.cap = cap;
     sk.act = act >= 0 ? act : (c->cfg.use_gelu_mlp ? 1 : 0);
     sk.tile_group = x.tile_group; sk.row_scale = x.row_scale; sk.err = c->wait_err;
-    sk.vec = (((uintptr_t)res | (uintptr_t)C) & 15) == 0 && ldc % 4 == 0;
+    const bool vec = (((uintptr_t)res | (uintptr_t)C) & 15) == 0 && ldc % 4 == 0;
     CUtensorMap ma, mw;
     RC(make_tmap(&ma, A, (uint64_t)M, (uint64_t)K, c->cfg.dtype, (uint32_t)sk.nt, (uint64_t)x.a_ld));
     RC(make_tmap(&mw, W, (uint64_t)N * x.n_groups, (uint64_t)K, c->cfg.dtype, SK_BM, 0, true));
-    return launch_cluster_pdl(c, gemm_skinny_kernel<T, EPI>, dim3((unsigned)(N / SK_BM * sk.m_tiles * sk.split)), dim3(SK_THREADS), sk_smem,
+    return launch_cluster_pdl(c, vec ? gemm_skinny_kernel<T, EPI, true> : gemm_skinny_kernel<T, EPI, false>, dim3((unsigned)(N / SK_BM * sk.m_tiles * sk.split)), dim3(SK_THREADS), sk_smem,
                               (unsigned)sk.split, mw, ma, sk);
   }
   const bool weight = !x.tile_group && !x.w_live && !x.b_kwrap;
@@ -4199,13 +4215,17 @@ extern "C" int cake_b200_debug_product(cake_b200_ctx *c, int epi, const void *A,
                                        int act, float cap, const int *group, int n_groups, int group_rows, const float *row_scale, int batch) {
   if (!c || !A || !W || !C || !tc_gemm_ok(M, N, K) || batch < 1 || (group && (M % TC_BM || group_rows < 1 || n_groups < 1)) || epi < 0 || epi > TCE_ACT ||
       ((epi == TCE_RESIDUAL || epi == TCE_RESIDUAL_F32) && !res) || (batch > 1 && (epi != TCE_PLAIN || group)) ||
-      (((uintptr_t)A | (uintptr_t)W | (uintptr_t)C | (uintptr_t)res) & 15))
+      (((uintptr_t)A | (uintptr_t)W) & 15))
     return fail(CAKE_B200_EINVAL, "bad debug_product arguments");
   CU(cudaSetDevice(c->device));
   RC(wait_loads(c));
   TcExtra x;
   if (group) { x.tile_group = group; x.n_groups = n_groups; x.group_rows = group_rows; }
   x.row_scale = row_scale;
+  SkParams sk{};
+  size_t sk_smem = 0;
+  if ((((uintptr_t)C | (uintptr_t)res) & 15) && !plan_skinny(c->sm_count, M, N, K, x, &sk, &sk_smem))  // (the other kernel's accesses are 16 bytes wide)
+    return fail(CAKE_B200_EINVAL, "bad debug_product arguments");
   if (batch > 1) { x.batch = batch; x.a_ld = batch * K; x.a_step = K; x.c_step = N; }
   const int ldc = batch > 1 ? batch * N : 0;
   RC(DISPATCH_T(c->cfg.dtype, T_LAMBDA {

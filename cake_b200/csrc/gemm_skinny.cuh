@@ -8,7 +8,9 @@
 //   * W is the MMA's 128-row operand and the rows of A are its columns (16 .. 256 of them, as many as there are, rounded up to 16),
 //     so that a stage carries 16 KB of W and little else, and a product of up to 256 rows reads W once;
 //   * a 128-row slice of W is cut along K between the S CTAs of a cluster, which brings the grid up to the chip; the S fp32 partial
-//     sums meet in shared memory over the cluster (every CTA finishes nt / S of the rows, sums in rank order: deterministic);
+//     sums meet in shared memory over the cluster (every CTA finishes nt / S of the rows, sums in rank order: deterministic).  A CTA lays its
+//     sums down in its own shared memory and sends each other CTA's rows there as one bulk copy, counted on a barrier of the receiver:
+//     with a store per sum between two cluster barriers the exchange was 2.1 us of a kernel's 5.1 (37 rows of 1024 x 1024, eight CTAs);
 //   * the first ring of W is requested before griddepcontrol.wait: weights don't depend on the kernel in front.
 // One CTA = one slice, 192 threads: warp 0 TMA producer, warp 1 MMA issuer and TMEM owner, warps 2-5 epilogue (thread = row of W).
 #pragma once
@@ -20,10 +22,22 @@ constexpr int SK_BM = 128, SK_THREADS = 192, SK_MAX_SPLIT = 8, SK_MAX_STAGES = 8
 constexpr int SK_MAX_ROWS = 256, SK_SMEM_MAX = 220 * 1024;
 constexpr int SK_W_BYTES = SK_BM * TC_BK * 2;  // 16 KB of W per stage
 __host__ __device__ inline int sk_stage_bytes(int nt) { return SK_W_BYTES + nt * TC_BK * 2; }
-__host__ inline size_t sk_smem_bytes(int nt, int stages, int split) {
-  size_t ring = (size_t)stages * sk_stage_bytes(nt);
-  if (split > 1 && ring < (size_t)nt * SK_BM * 4) ring = (size_t)nt * SK_BM * 4;  // the partial sums take the ring's place
-  return ring + 1024 /*align*/ + 256 /*barriers*/;
+// Shared memory: the ring; over it, when it has been read, a CTA's own sums [nt][128]; and the sums it receives, [split - 1][nt / split][128], behind
+// the ring (SK_APART: peers may send as soon as they like) or over it, behind the own sums (SK_OVER).  SK_LEAN, 256 rows cut in four: the share that
+// a CTA keeps stays in tensor memory until the last pass fetches it 16 rows at a time, as an uncut slice's rows.
+enum { SK_OVER = 0, SK_APART = 1, SK_LEAN = 2 };
+__host__ __device__ inline int sk_sums_floats(int nt, int split, int how) { return (how == SK_LEAN ? nt / split * (split - 1) : nt) * SK_BM; }
+__host__ __device__ inline int sk_recv_at(int nt, int stages, int split, int how) {  // in floats
+  const int ring = stages * sk_stage_bytes(nt) / 4, sums = sk_sums_floats(nt, split, how);
+  return how == SK_APART && ring > sums ? ring : sums;
+}
+__host__ inline size_t sk_smem_bytes(int nt, int stages, int split, int how) {
+  size_t bytes = (size_t)stages * sk_stage_bytes(nt);
+  if (split > 1) {
+    const size_t end = ((size_t)sk_recv_at(nt, stages, split, how) + (size_t)nt / split * (split - 1) * SK_BM + (how == SK_LEAN ? 16 * SK_BM : 0)) * 4;
+    if (bytes < end) bytes = end;
+  }
+  return bytes + 1024 /*align*/ + 256;
 }
 
 struct SkParams {
@@ -36,45 +50,45 @@ struct SkParams {
   int nt;                    // rows of A per tile (a multiple of 16)
   int m_tiles;               // row tiles, TC_BM rows apart
   int split, stages;
-  int vec;                   // C and the residual take accesses of four columns (their addresses and row strides)
+  int how;                   // SK_OVER, SK_APART or SK_LEAN
   int *err;                  // host-mapped: a wait that ran out
 };
 
 // What an epilogue reads beside the sums, four columns of row m of A from column n on (nothing where the row is not `in`)
-template <typename T, int EPI> struct SkRes {
+template <typename T, int EPI, bool VEC> struct SkRes {
   static constexpr int WORDS = EPI == TCE_RESIDUAL_F32 ? 4 : EPI == TCE_RESIDUAL ? 2 : 1;
   uint32_t w[WORDS];
   __device__ __forceinline__ void load(const SkParams &p, bool in, int m, int n) {
     if (!in) return;
     if (EPI == TCE_RESIDUAL) {
       const uint16_t *src = reinterpret_cast<const uint16_t *>(p.residual) + (size_t)m * (p.ldc ? p.ldc : p.N) + n;
-      const uint2 v = p.vec ? *reinterpret_cast<const uint2 *>(src) : make_uint2(src[0] | (uint32_t)src[1] << 16, src[2] | (uint32_t)src[3] << 16);
+      const uint2 v = VEC ? *reinterpret_cast<const uint2 *>(src) : make_uint2(src[0] | (uint32_t)src[1] << 16, src[2] | (uint32_t)src[3] << 16);
       w[0] = v.x; w[WORDS > 1 ? 1 : 0] = v.y;
     } else if (EPI == TCE_RESIDUAL_F32) {
       const uint32_t *src = reinterpret_cast<const uint32_t *>(p.residual) + (size_t)m * p.N + n;
-      const uint4 v = p.vec ? *reinterpret_cast<const uint4 *>(src) : make_uint4(src[0], src[1], src[2], src[3]);
+      const uint4 v = VEC ? *reinterpret_cast<const uint4 *>(src) : make_uint4(src[0], src[1], src[2], src[3]);
       w[0] = v.x; w[WORDS > 1 ? 1 : 0] = v.y; w[WORDS > 2 ? 2 : 0] = v.z; w[WORDS > 3 ? 3 : 0] = v.w;
     }
   }
 };
 // the sums of row m, columns n .. n + 3 -> C
-template <typename T, int EPI>
-__device__ __forceinline__ void sk_store(const SkParams &p, int m, int n, const float (&v)[4], const float (&bias)[4], const SkRes<T, EPI> &res) {
+template <typename T, int EPI, bool VEC>
+__device__ __forceinline__ void sk_store(const SkParams &p, int m, int n, const float (&v)[4], const float (&bias)[4], const SkRes<T, EPI, VEC> &res) {
   if (EPI == TCE_SOFTCAP_F32 || EPI == TCE_RESIDUAL_F32) {
     float *dst = reinterpret_cast<float *>(p.C) + (size_t)m * p.N + n;
     const float rs = EPI == TCE_RESIDUAL_F32 && p.row_scale ? p.row_scale[m] : 1.0f;
     float o[4];
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-      if (EPI == TCE_RESIDUAL_F32) o[j] = fmaf(rs, v[j], __uint_as_float(res.w[j % SkRes<T, EPI>::WORDS]));
+      if (EPI == TCE_RESIDUAL_F32) o[j] = fmaf(rs, v[j], __uint_as_float(res.w[j % SkRes<T, EPI, VEC>::WORDS]));
       else o[j] = p.cap > 0.f ? p.cap * tanhf(v[j] / p.cap) : v[j];
     }
-    if (p.vec) *reinterpret_cast<float4 *>(dst) = make_float4(o[0], o[1], o[2], o[3]);
+    if (VEC) *reinterpret_cast<float4 *>(dst) = make_float4(o[0], o[1], o[2], o[3]);
     else { dst[0] = o[0]; dst[1] = o[1]; dst[2] = o[2]; dst[3] = o[3]; }
   } else if (EPI == TCE_SWIGLU) {  // columns 2i and 2i + 1 are gate and up
     T *dst = reinterpret_cast<T *>(p.C) + (size_t)m * (p.ldc ? p.ldc : p.N / 2) + n / 2;
     const uint32_t u = pack2x<T>(gated_pair<T>(v[0], v[1], p.act, p.cap), gated_pair<T>(v[2], v[3], p.act, p.cap));
-    if (p.vec) *reinterpret_cast<uint32_t *>(dst) = u;
+    if (VEC) *reinterpret_cast<uint32_t *>(dst) = u;
     else { reinterpret_cast<uint16_t *>(dst)[0] = (uint16_t)u; reinterpret_cast<uint16_t *>(dst)[1] = (uint16_t)(u >> 16); }
   } else {
     float o[4];
@@ -83,13 +97,13 @@ __device__ __forceinline__ void sk_store(const SkParams &p, int m, int n, const 
       o[j] = EPI == TCE_ACT ? plain_act<T>(v[j], p.act) : rnd<T>(v[j]);
       if (EPI == TCE_PLAIN && p.bias) o[j] = rnd<T>(o[j] + bias[j]);
       if (EPI == TCE_RESIDUAL) {
-        const float2 r2 = DT<T>::unpack2(res.w[(j / 2) % SkRes<T, EPI>::WORDS]);
+        const float2 r2 = DT<T>::unpack2(res.w[(j / 2) % SkRes<T, EPI, VEC>::WORDS]);
         o[j] += j & 1 ? r2.y : r2.x;
       }
     }
     T *dst = reinterpret_cast<T *>(p.C) + (size_t)m * (p.ldc ? p.ldc : p.N) + n;
     const uint2 u = make_uint2(pack2x<T>(o[0], o[1]), pack2x<T>(o[2], o[3]));
-    if (p.vec) *reinterpret_cast<uint2 *>(dst) = u;
+    if (VEC) *reinterpret_cast<uint2 *>(dst) = u;
     else {
       uint16_t *d16 = reinterpret_cast<uint16_t *>(dst);
       d16[0] = (uint16_t)u.x; d16[1] = (uint16_t)(u.x >> 16); d16[2] = (uint16_t)u.y; d16[3] = (uint16_t)(u.y >> 16);
@@ -97,12 +111,14 @@ __device__ __forceinline__ void sk_store(const SkParams &p, int m, int n, const 
   }
 }
 
-template <typename T, int EPI>
+// VEC: C and the residual take accesses of four columns (their addresses and row strides); an instance of its own for what does not, since a kernel of
+// a few microseconds pays for instructions on its way that it does not run
+template <typename T, int EPI, bool VEC>
 __global__ void __launch_bounds__(SK_THREADS, 2)
 gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, const SkParams p) {
   extern __shared__ unsigned char smem_raw_sk[];
   unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw_sk) + 1023) & ~(uintptr_t)1023);
-  __shared__ uint64_t full[SK_MAX_STAGES], empty[SK_MAX_STAGES], acc_full, drained;
+  __shared__ uint64_t full[SK_MAX_STAGES], empty[SK_MAX_STAGES], acc_full, drained, got;
   __shared__ uint32_t tmem_ptr;
   __shared__ int gave_up;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -118,8 +134,10 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     for (int s = 0; s < p.stages; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
     mbar_init(&acc_full, 1);
     mbar_init(&drained, 1);
+    mbar_init(&got, 1);
     gave_up = 0;
     mbar_fence_init();
+    if (S > 1) mbar_arrive_expect_tx(&got, (uint32_t)(nt / S * (S - 1) * SK_BM * 4));
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_ptr)), "r"(cols) : "memory");
@@ -129,6 +147,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   __syncthreads();
   tc_fence_after();
   pdl_launch_dependents();
+  if (S > 1 && p.how == SK_APART) cluster_arrive_relaxed();  // this CTA's barrier exists (mbar_fence_init) and its place for sums is free
   const uint32_t tmem = tmem_ptr;
 
   int group = 0;
@@ -191,7 +210,8 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   const int wq = warp & 3;
   const uint32_t trow = tmem + ((uint32_t)(wq * 32) << 16);
   const int share = nt / S, f0 = m0 + rank * share;  // rows this CTA finishes: all of the tile, or its share of them
-  float *recv = reinterpret_cast<float *>(smem);     // sums on their way, over the drained ring: [source rank][row within the share][128 columns]
+  float *sums = reinterpret_cast<float *>(smem);     // this CTA's sums, over its drained ring: [row of A][128 columns]
+  const int recv = sk_recv_at(nt, p.stages, S, p.how);  // the others', from here on: [rank but this][row within the share][128 columns]
   bool go = warp >= 2 && live;                       // warps that finish rows
   // A warp finishes its 32 columns four rows at a time, a lane four columns of one row: loads and stores of 8 bytes (16 of fp32), and the
   // residual of four passes is on its way.  (A thread per column took a pair of rows at a time, each behind its residual's way from L2: 0.1
@@ -199,7 +219,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   // which runs it once, waits for it: 187 -> 189 us for four Nigenex layers.)
   const int fr = lane >> 3, fc = wq * 32 + (lane & 7) * 4, fn = n0 + fc;
   float bias[4] = {0.f, 0.f, 0.f, 0.f};
-  SkRes<T, EPI> res[4];
+  SkRes<T, EPI, VEC> res[4];
   if (go) {
     if (EPI == TCE_PLAIN && p.bias) {
 #pragma unroll
@@ -213,56 +233,75 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   }
   if (S > 1) {
     __syncwarp();
-    cluster_arrive();  // every CTA's ring is drained: its MMAs have read all that was loaded
-    cluster_wait();
-    if (go) {
-      const uint32_t base = smem_u32(recv) + (uint32_t)(((size_t)rank * share * SK_BM + wq * 32 + lane) * 4);
-      int to = 0, off = 0;  // row of A -> CTA and place within its share
-      uint32_t dst = cluster_map(base, 0u);
+    if (p.how != SK_APART) cluster_arrive();  // this CTA's ring is drained: its MMAs have read all that was loaded
+    if (warp >= 2) {
+      if (go) {
 #pragma unroll 1
-      for (int c0 = 0; c0 < nt && m0 + c0 < m_end; c0 += 16) {
-        uint32_t r[16];
-        tc_ld16(trow + (uint32_t)c0, r);
+        for (int c0 = 0; c0 < nt; c0 += 32) {  // (the accumulator has a power of two of columns, 32 at least)
+          uint32_t r[32];
+          float *dst = sums + (size_t)c0 * SK_BM + wq * 32 + lane;
+          if (p.how == SK_LEAN) {
+            if (c0 / share == rank) continue;
+            if (c0 / share > rank) dst -= share * SK_BM;
+          }
+          tc_ld32(trow + (uint32_t)c0, r);
 #pragma unroll
-        for (int j = 0; j < 16; j++) {
-          st_cluster_f32(dst, __uint_as_float(r[j]));
-          dst += SK_BM * 4;
-          if (++off == share && to + 1 < S) { off = 0; dst = cluster_map(base, (uint32_t)++to); }
+          for (int j = 0; j < 16; j++) dst[j * SK_BM] = __uint_as_float(r[j]);
+          if (c0 + 16 < nt)
+#pragma unroll
+            for (int j = 16; j < 32; j++) dst[j * SK_BM] = __uint_as_float(r[j]);
         }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      } else if (live) gave_up = 1;
+      __syncwarp();
+      cluster_wait();
+      named_bar_sync(1, SK_THREADS - 64);
+      if (warp == 2 && lane < S - 1 && live && !*(volatile int *)&gave_up) {  // a lane per receiver, every CTA beginning with another one
+        const int to = (rank + 1 + lane) & (S - 1);
+        const uint32_t bytes = (uint32_t)(share * SK_BM * 4), slot = (uint32_t)(rank - (rank > to)) * bytes;
+        bulk_s2s(cluster_map(smem_u32(sums + recv) + slot, (uint32_t)to), smem_u32(sums) + (uint32_t)(to - (p.how == SK_LEAN && to > rank)) * bytes, bytes, cluster_map(smem_u32(&got), (uint32_t)to));
       }
+      __syncwarp();
+      if (go) {
+        mbar_wait_lim(&got, 0, p.err, left);
+        go = __all_sync(0xffffffffu, left != 0);
+      }
+      cluster_arrive_relaxed();  // (waited for at the end: nobody leaves while sums are on their way)
+    } else {
+      cluster_wait();
+      cluster_arrive_relaxed();
     }
-    __syncwarp();
-    cluster_arrive();
-    cluster_wait();
   }
   // The last pass is a loop, not straight-line code: a kernel of a few microseconds runs its epilogue once, and unrolled over 16 rows it
   // waited for its own instructions (233 -> 315 us for four Nigenex layers).  A row's residual is read by the lane that stores it, before
   // it does: C may be the residual's own buffer.
   if (go) {
-    const float *src0 = recv + (size_t)fr * SK_BM + fc;
+    const bool kept = S == 1 || p.how == SK_LEAN;  // own rows are still in tensor memory
+    const int own16 = S == 1 ? 0 : recv + (S - 1) * share * SK_BM;
 #pragma unroll 1
     for (int c0 = 0; c0 < share && f0 + c0 < m_end; c0 += 4) {
-      const float *src = src0 + (size_t)(S == 1 ? c0 & 12 : c0) * SK_BM;
-      if (S == 1 && !(c0 & 12)) {  // through shared memory too: the warp's own columns, 16 rows at a time
+      if (kept && !(c0 & 12)) {  // through shared memory too: the warp's own columns, 16 rows at a time
         uint32_t r[16];
-        tc_ld16(trow + (uint32_t)c0, r);
-        float *mine = recv + wq * 32 + lane;
+        tc_ld16(trow + (uint32_t)(rank * share + c0), r);
+        float *mine = sums + own16 + wq * 32 + lane;
         __syncwarp();
 #pragma unroll
         for (int j = 0; j < 16; j++) mine[j * SK_BM] = __uint_as_float(r[j]);
         __syncwarp();
       }
       const int m = f0 + c0 + fr;
-      SkRes<T, EPI> ahead;
+      SkRes<T, EPI, VEC> ahead;
       ahead.load(p, c0 + fr + 16 < share && m + 16 < m_end, m + 16, fn);
       if (c0 + fr < share && m < m_end) {
+        const int at = (c0 + fr) * SK_BM + fc, stride = share * SK_BM, own = kept ? own16 + ((c0 & 12) + fr) * SK_BM + fc : at + rank * stride;
         float v[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 2
-        for (int q = 0; q < S; q++, src += (size_t)share * SK_BM) {
-          const float4 x = *reinterpret_cast<const float4 *>(src);
+        for (int q = 0; q < S; q++) {  // in rank order
+          const int off = q == rank ? own : recv + at + (q - (q > rank)) * stride;
+          const float4 x = *reinterpret_cast<const float4 *>(sums + off);
           v[0] += x.x; v[1] += x.y; v[2] += x.z; v[3] += x.w;
         }
-        sk_store<T, EPI>(p, m, fn, v, bias, res[0]);
+        sk_store<T, EPI, VEC>(p, m, fn, v, bias, res[0]);
       }
       res[0] = res[1]; res[1] = res[2]; res[2] = res[3];
       res[3] = ahead;
@@ -280,6 +319,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     }
     __syncthreads();
   }
+  if (S > 1) cluster_wait();
   if (warp == 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");

@@ -169,3 +169,31 @@ def test_grouped_products(ctx, rows, N, K):
             sl = slice(i * 128, i * 128 + rows)
             want, bound = reference(epi, a[sl], w[e * N:(e + 1) * N], None, res[sl], 0, 0.0, ctx.D, None)
             near(c[sl], want, bound, (epi, i))
+
+
+# sums that meet over a cluster: (M, N, K), CTAs of a slice; received behind the ring or over it, shares of 2 .. 128 rows, a share that is half empty
+EXCHANGES = [(1, 1024, 1024, 8), (16, 6144, 4096, 8), (37, 4096, 1024, 4), (49, 1024, 2048, 8), (64, 2048, 4096, 8), (97, 4096, 1024, 4), (112, 2048, 2048, 8),
+             (193, 2048, 2048, 4), (209, 1024, 4096, 8), (225, 1024, 4096, 4), (250, 2048, 4096, 4)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M,N,K,split", EXCHANGES)
+def test_sums_of_a_cluster(ctx, M, N, K, split):
+    """Every cut along K gives the same as a plain product, for C and residual that take wide accesses and, two bytes off, for those that don't."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    kind, got_split = plan(M, N, K, sms=sms)[:2]
+    if sms == SMS:
+        assert (kind, got_split) == (SKINNY, split)
+    a, w, g = operands(ctx, M, N, K, M + N)
+    res = torch.randn(M, N, device=a.device, generator=g)
+    for epi in (RESIDUAL, RESIDUAL_F32, SWIGLU, PLAIN):
+        r = res.to(ctx.D) if epi == RESIDUAL else res if epi == RESIDUAL_F32 else None
+        want, bound = reference(epi, a, w, None, r, 0, 0.0, ctx.D, None)
+        near(product(ctx, epi, a, w, M, N, K, None, r), want, bound, epi)
+        if kind != SKINNY:
+            continue
+        c = torch.full((want.numel() + 1,), float("nan"), device=a.device, dtype=torch.float32 if epi == RESIDUAL_F32 else ctx.D)[1:]
+        off = torch.cat([r.flatten()[:1], r.flatten()])[1:] if r is not None else None
+        torch.cuda.synchronize()
+        check(lib().cake_b200_debug_product(ctx.h, epi, ptr(a), ptr(w), None, ptr(off) if off is not None else None, ptr(c), M, N, K, 0, 0.0, None, 0, 0, None, 1))
+        near(c.view(want.shape), want, bound, (epi, "two bytes off"))
