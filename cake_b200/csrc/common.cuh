@@ -229,6 +229,14 @@ __device__ __forceinline__ void bulk_g2s(void *dst_smem, const void *src_gmem, u
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// 1 in one lane of a whole warp.  The thread that issues tcgen05 products is picked this way and the warp runs the loop with it: behind lane == 0 the
+// operands of every product make their own way to the uniform registers, 411 cycles a k-block of four products against 270 (128 x 16 x 64; 294 at N = 128).
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+  return r;
+}
+
 __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }

@@ -188,21 +188,25 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     __syncwarp();
   } else if (warp == 1) {
     if (!p.tile_group) pdl_wait();  // (also keeps the bounded waits from counting the kernel in front)
-    if (lane == 0 && live) {
-      const uint32_t idesc = tc_idesc<T>(nt);
+    if (live) {
+      const uint32_t idesc = tc_idesc<T>(nt), one = elect_one();
+      const uint64_t dw0 = tc_smem_desc(smem), da0 = tc_smem_desc(smem + SK_W_BYTES);
       int s = 0;
       uint32_t ph = 0;
+#pragma unroll 1
       for (int i = 0; i < nkb; i++) {
         mbar_wait_lim(&full[s], ph, p.err, left);
         tc_fence_after();
-        const unsigned char *st = smem + (size_t)s * stage_bytes;
-        const uint64_t dw = tc_smem_desc(st), da = tc_smem_desc(st + SK_W_BYTES);
+        const uint64_t dw = dw0 + (uint64_t)(s * (stage_bytes >> 4)), da = da0 + (uint64_t)(s * (stage_bytes >> 4));
+        if (one) {
 #pragma unroll
-        for (int k = 0; k < TC_BK / 16; k++) tc_mma_f16(tmem, dw + (uint64_t)(k * 2), da + (uint64_t)(k * 2), idesc, (i | k) ? 1u : 0u);
-        tc_commit(&empty[s], left);
+          for (int k = 0; k < TC_BK / 16; k++) tc_mma_f16(tmem, dw + (uint64_t)(k * 2), da + (uint64_t)(k * 2), idesc, (i | k) ? 1u : 0u);
+          tc_commit(&empty[s], left);
+        }
+        __syncwarp();
         if (++s == p.stages) { s = 0; ph ^= 1u; }
       }
-      tc_commit(&acc_full, left);
+      if (one) tc_commit(&acc_full, left);
     }
     __syncwarp();
   }

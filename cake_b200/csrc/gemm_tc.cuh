@@ -33,8 +33,8 @@ namespace cake {
 constexpr int TC_BM = 128, TC_BK = 64, TC_EPI_WARPS = 8, TC_THREADS = 128 + 32 * TC_EPI_WARPS;
 constexpr int TC_BN = 128;                     // granularity the host checks N against (BN = 256 when N % 256 == 0)
 template <int BN, bool PAIR = false> struct TcCfg {
-  static constexpr int STAGES = (BN == 256 && !PAIR) ? 4 : 6;
-  static constexpr int STAGE_BYTES = (TC_BM + (PAIR ? BN / 2 : BN)) * TC_BK * 2;  // 32 KB | 48 KB | 32 KB
+  static constexpr int STAGES = PAIR ? (BN == 256 ? 6 : 8) : BN == 256 ? 4 : 6;
+  static constexpr int STAGE_BYTES = (TC_BM + (PAIR ? BN / 2 : BN)) * TC_BK * 2;  // 32 KB | 48 KB | 32 KB, 24 KB
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
 };
 // TCE_RESIDUAL_F32: C (fp32) = residual (fp32) + accumulator, nothing rounded to D — the output projection of a block whose
@@ -172,7 +172,6 @@ template <> __device__ __forceinline__ uint32_t tc_idesc<__half>(int bn) {
 template <typename T, int EPI, int BN, bool PAIR = false>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const TcParams p) {
-  static_assert(!PAIR || BN == 256, "the pair is built for 256 columns");
   typedef TcCfg<BN, PAIR> Cfg;
   extern __shared__ unsigned char smem_raw_tc[];
   unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw_tc) + 1023) & ~(uintptr_t)1023);
@@ -251,7 +250,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       };
       auto load_w = [&](int st, int kb, int wrow) {
         unsigned char *d = smem + (size_t)st * Cfg::STAGE_BYTES + TC_BM * TC_BK * 2;
-        if (PAIR) tma_load_2d_pair(d, &map_b, kb * TC_BK, wrow + (int)crank * 128, cluster_map(smem_u32(&full[st]), 0u), left);  // a 128-row box: our half of the W tile
+        if (PAIR) tma_load_2d_pair(d, &map_b, kb * TC_BK, wrow + (int)crank * (BN / 2), cluster_map(smem_u32(&full[st]), 0u), left);  // our half of the W tile
         else tma_load_2d(d, &map_b, p.b_kwrap ? (kb * TC_BK) % p.b_kwrap : kb * TC_BK, wrow, &full[st], left);
       };
       if (p.w_early) {  // (not a grouped product: the groups are another kernel's output)
@@ -285,8 +284,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       }
     }
   } else if (warp == 1) {
-    // ===================== MMA issuer (one thread) =======================================================
-    if (lane == 0 && crank == 0) {
+    // ===================== MMA issuer (one thread; the warp runs the loop with it) ========================
+    if (crank == 0) {
+      const uint32_t one = elect_one();
+      const uint64_t da0 = tc_smem_desc(smem), db0 = tc_smem_desc(smem + TC_BM * TC_BK * 2);
       const uint32_t idesc = PAIR ? tc_idesc<T>(BN) + ((uint32_t)(TC_BM >> 4) << 24) : tc_idesc<T>(BN);  // PAIR: M = 256
       int s = 0;
       uint32_t ph = 0;
@@ -306,18 +307,23 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         for (int kb = 0; kb < kblocks; kb++) {
           mbar_wait_lim(&full[s], ph, p.err, left);
           tc_fence_after();
-          const unsigned char *st = smem + (size_t)s * Cfg::STAGE_BYTES;
-          const uint64_t da = tc_smem_desc(st), db = tc_smem_desc(st + TC_BM * TC_BK * 2);
+          const uint64_t da = da0 + (uint64_t)(s * (Cfg::STAGE_BYTES >> 4)), db = db0 + (uint64_t)(s * (Cfg::STAGE_BYTES >> 4));
+          if (one) {
 #pragma unroll
-          for (int k = 0; k < TC_BK / 16; k++)  // +32 bytes (2 x 16 B units) per K=16 slab inside the swizzle atom
-            if (PAIR) tc_mma_f16_pair(tmem_c, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb | k) ? 1u : 0u);
-            else tc_mma_f16(tmem_c, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb | k) ? 1u : 0u);
-          if (PAIR) tc_commit_pair(&empty[s], left);  // arrives (in both CTAs) when the MMAs above have read the stage
-          else tc_commit(&empty[s], left);
+            for (int k = 0; k < TC_BK / 16; k++)  // +32 bytes (2 x 16 B units) per K=16 slab inside the swizzle atom
+              if (PAIR) tc_mma_f16_pair(tmem_c, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb | k) ? 1u : 0u);
+              else tc_mma_f16(tmem_c, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb | k) ? 1u : 0u);
+            if (PAIR) tc_commit_pair(&empty[s], left);  // arrives (in both CTAs) when the MMAs above have read the stage
+            else tc_commit(&empty[s], left);
+          }
+          __syncwarp();
           if (++s == Cfg::STAGES) { s = 0; ph ^= 1u; }
         }
-        if (PAIR) tc_commit_pair(&acc_full[a], left);  // accumulator complete
-        else tc_commit(&acc_full[a], left);
+        if (one) {
+          if (PAIR) tc_commit_pair(&acc_full[a], left);  // accumulator complete
+          else tc_commit(&acc_full[a], left);
+        }
+        __syncwarp();
       }
     }
   } else if (warp >= 4) {
