@@ -185,23 +185,27 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     }
     __syncwarp();
   } else if (warp == 5) {
-    // ===================== MMA issuer (one thread) =========================================================
-    if (lane == 0 && n_tiles > 0) {
+    // ===================== MMA issuer (one thread; the warp runs the loop with it) ==========================
+    if (n_tiles > 0) {
+      const uint32_t one = elect_one();
       const uint32_t idesc_s = tc_idesc<T>(FT_BN);                   // M128 N64, A and B K-major
       const uint32_t idesc_o = tc_idesc<T>(FT_HD) | (1u << 16);      // M128 N128, A from TMEM, B (V) MN-major
       auto issue_s = [&](int j) {  // S_j = Q K_j^T into S buffer j&1
         const int st = j & 1;
         mbar_wait_lim(&k_full[st], (uint32_t)(j >> 1) & 1u, p.err, left);
         tc_fence_after();
-        const unsigned char *kt = k_s + st * FT_KV_BYTES;
+        const uint64_t q0 = tc_smem_desc(q_s), kt = tc_smem_desc(k_s) + (uint64_t)(st * (FT_KV_BYTES >> 4));
+        if (one) {
 #pragma unroll
-        for (int k = 0; k < FT_HD / 16; k++) {  // head dims 16k..16k+15: box k/4, 32-byte slab k%4 inside the swizzle row
-          const uint64_t da = tc_smem_desc(q_s + (k >> 2) * (FT_Q_BYTES / 2)) + (uint64_t)((k & 3) * 2);
-          const uint64_t db = tc_smem_desc(kt + (k >> 2) * (FT_KV_BYTES / 2)) + (uint64_t)((k & 3) * 2);
-          tc_mma_f16(tmem_base + (uint32_t)(st * 64), da, db, idesc_s, k ? 1u : 0u);
+          for (int k = 0; k < FT_HD / 16; k++) {  // head dims 16k..16k+15: box k/4, 32-byte slab k%4 inside the swizzle row
+            const uint64_t da = q0 + (uint64_t)((k >> 2) * (FT_Q_BYTES / 2 >> 4) + (k & 3) * 2);
+            const uint64_t db = kt + (uint64_t)((k >> 2) * (FT_KV_BYTES / 2 >> 4) + (k & 3) * 2);
+            tc_mma_f16(tmem_base + (uint32_t)(st * 64), da, db, idesc_s, k ? 1u : 0u);
+          }
+          tc_commit(&k_empty[st], left);
+          tc_commit(&s_full[st], left);
         }
-        tc_commit(&k_empty[st], left);
-        tc_commit(&s_full[st], left);
+        __syncwarp();
       };
       mbar_wait_lim(q_full, 0, p.err, left);
       issue_s(0);
@@ -212,17 +216,19 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         mbar_wait_lim(p_full, (uint32_t)j & 1u, p.err, left);  // P_j in TMEM (over S_j), O rescaled
         mbar_wait_lim(&v_full[st], (uint32_t)(j >> 1) & 1u, p.err, left);
         tc_fence_after();
-        const unsigned char *vt = v_s + st * FT_KV_BYTES;
+        const uint64_t vt = ft_desc_mn(v_s, FT_KV_BYTES / 2) + (uint64_t)(st * (FT_KV_BYTES >> 4));
+        if (one) {
 #pragma unroll
-        for (int half = 0; half < 2; half++)
+          for (int half = 0; half < 2; half++)
 #pragma unroll
-          for (int ks = 0; ks < FT_BN / 16; ks++) {  // keys 16ks..16ks+15 = 8 packed columns of P_hi (0..31) or P_lo (32..63)
-            const uint32_t ta = tmem_base + (uint32_t)(st * 64 + half * 32 + ks * 8);
-            const uint64_t db = ft_desc_mn(vt + ks * 2048, FT_KV_BYTES / 2);
-            tc_mma_f16_ts(tmem_o, ta, db, idesc_o, (j | half | ks) ? 1u : 0u);
-          }
-        tc_commit(&v_empty[st], left);
-        tc_commit(o_full, left);
+            for (int ks = 0; ks < FT_BN / 16; ks++) {  // keys 16ks..16ks+15 = 8 packed columns of P_hi (0..31) or P_lo (32..63)
+              const uint32_t ta = tmem_base + (uint32_t)(st * 64 + half * 32 + ks * 8);
+              tc_mma_f16_ts(tmem_o, ta, vt + (uint64_t)(ks * (2048 >> 4)), idesc_o, (j | half | ks) ? 1u : 0u);
+            }
+          tc_commit(&v_empty[st], left);
+          tc_commit(o_full, left);
+        }
+        __syncwarp();
       }
     }
     __syncwarp();
