@@ -441,6 +441,10 @@ template <typename T> static int set_smem_attrs_T() {
   CU(cudaFuncSetAttribute(gemm_skinny_kernel<T, EPI, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SK_SMEM_MAX));                  \
   CU(cudaFuncSetAttribute(gemm_skinny_kernel<T, EPI, true>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));\
   CU(cudaFuncSetAttribute(gemm_skinny_kernel<T, EPI, false>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+  CU(cudaFuncSetAttribute(gemm_skinny_two_kernel<T, TCE_SWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, SK_SMEM_MAX));
+  CU(cudaFuncSetAttribute(gemm_skinny_two_kernel<T, TCE_SOFTCAP_F32>, cudaFuncAttributeMaxDynamicSharedMemorySize, SK_SMEM_MAX));
+  CU(cudaFuncSetAttribute(gemm_skinny_two_kernel<T, TCE_SWIGLU>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+  CU(cudaFuncSetAttribute(gemm_skinny_two_kernel<T, TCE_SOFTCAP_F32>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
   SETK(TCE_PLAIN) SETK(TCE_RESIDUAL) SETK(TCE_SWIGLU) SETK(TCE_RESIDUAL_F32) SETK(TCE_SOFTCAP_F32) SETK(TCE_ACT)
 #undef SETK
   SETT(TCE_PLAIN) SETT(TCE_RESIDUAL) SETT(TCE_SWIGLU) SETT(TCE_RESIDUAL_F32) SETT(TCE_SOFTCAP_F32) SETT(TCE_ACT)
@@ -1339,6 +1343,7 @@ struct TcExtra {  // optional modes of the tensor-core GEMM (TcParams in gemm_tc
   int a_ld = 0;                           // A's row stride in elements when it is a column range of a wider buffer
   bool w_live = false;                    // W was written by an earlier kernel of the stream (a cache, not a weight)
   int group_rows = 0;                     // grouped product: no row block holds more rows than this (0 = unknown)
+  bool a_shared = false;                  // grouped product of up to 64 rows: A is these rows, and every row block multiplies all of them
   int batch = 1, a_step = 0, c_step = 0;  // side-by-side products: product i reads columns i * a_step .. of A's rows and rows i * N .. of W and
                                           // writes columns i * c_step .. of C's rows (TCE_PLAIN, with a_ld and ldc)
 };
@@ -1371,13 +1376,7 @@ static double skinny_us(int sms, int nt, int N, int K, int ctas, int kblocks) {
   return std::max((double)((ctas + sms - 1) / sms) * kblocks * sk_stage_bytes(nt) / 80e3, 2.0 * N * K / 6.4e6) + 3.5 + 0.03 * nt;
 }
 // gemm_skinny_kernel's shape for a product, or false where gemm_tc_kernel takes it.
-static bool plan_skinny(int sms, int M, int N, int K, const TcExtra &x, SkParams *p, size_t *smem) {
-  if (x.w_live || x.b_kwrap || x.w_cols || x.w_rows || x.w_ld || x.batch > 1) return false;
-  const int rows = x.tile_group ? x.group_rows : M;
-  if (rows < 1 || rows > (x.tile_group ? 64 : SK_MAX_ROWS)) return false;
-  p->nt = (rows + 15) / 16 * 16;
-  p->m_tiles = x.tile_group ? M / TC_BM : 1;
-  const int tiles = N / SK_BM * p->m_tiles;
+static bool cut_skinny(int sms, int tiles, int k_min, int k_max, SkParams *p, size_t *smem) {  // slices of W in all, the shortest and the longest K
   // The cut along K, each CTA with at least two k-blocks: as many CTAs as stay resident at once (three per SM up to 64 rows, two up to 112, one
   // beyond: a ring has three stages or more), but a second one per SM only with four k-blocks each and a third with eight (us, S CTAs per slice:
   // 37 rows, N = 4096, K = 1024: S = 4 5.9, S = 8 6.8; N = 6144: 2 8.2, 4 6.8, 8 12.6; 16 rows, N = 6144, K = 4096: 2 13.6, 4 12.1, 8 11.3), and
@@ -1386,21 +1385,32 @@ static bool plan_skinny(int sms, int M, int N, int K, const TcExtra &x, SkParams
   const int most = p->nt <= 64 ? 3 : p->nt < 128 ? 2 : 1;
   p->split = 1;
   while (p->split < SK_MAX_SPLIT) {
-    const int ctas = tiles * p->split * 2, kblocks = K / TC_BK / (p->split * 2);
+    const int ctas = tiles * p->split * 2, kblocks = k_min / TC_BK / (p->split * 2);
     if (ctas > most * sms || kblocks < (ctas <= sms ? 2 : ctas <= 2 * sms ? 4 : 8) || (most == 1 && p->split == 4 && ctas > sms / 2)) break;
     p->split *= 2;
   }
   for (;; p->split /= 2) {  // (240 rows leave no room for the sums of a cluster of eight)
     const int per_sm = std::min(most, (tiles * p->split + sms - 1) / sms);
     const size_t budget = (size_t)(per_sm == 3 && p->split > 1 ? 74 : most == 1 ? 180 : 110) * 1024 - 1536;
-    const int kblocks = (K / TC_BK + p->split - 1) / p->split;  // of a CTA: no more stages than that, three at least
+    const int kblocks = (k_max / TC_BK + p->split - 1) / p->split;  // of a CTA: no more stages than that, three at least
     p->stages = std::min(std::min(SK_MAX_STAGES, std::max(2, (int)(budget / sk_stage_bytes(p->nt)))), std::max(3, kblocks));
     p->how = p->split > 1 && sk_smem_bytes(p->nt, p->stages, p->split, SK_APART) <= budget + 1280 ? SK_APART : SK_OVER;
     if (p->split > 1 && p->nt / p->split % 32 == 0 && sk_smem_bytes(p->nt, p->stages, p->split, p->how) > SK_SMEM_MAX) p->how = SK_LEAN;
     *smem = sk_smem_bytes(p->nt, p->stages, p->split, p->how);
     if (*smem <= SK_SMEM_MAX || p->split == 1) break;
   }
-  if (*smem > SK_SMEM_MAX) return false;
+  return *smem <= SK_SMEM_MAX;
+}
+static bool plan_skinny(int sms, int M, int N, int K, const TcExtra &x, SkParams *p, size_t *smem) {
+  if (x.w_live || x.b_kwrap || x.w_cols || x.w_rows || x.w_ld || x.batch > 1) return false;
+  const int rows = x.tile_group ? x.group_rows : M;
+  if (rows < 1 || rows > (x.tile_group ? 64 : SK_MAX_ROWS)) return false;
+  p->rows = rows;
+  p->nt = (rows + 15) / 16 * 16;
+  p->a_shared = x.a_shared ? 1 : 0;
+  p->m_tiles = x.tile_group ? M / TC_BM : 1;
+  const int tiles = N / SK_BM * p->m_tiles;
+  if (!cut_skinny(sms, tiles, K, K, p, smem)) return false;
   return x.tile_group || rows <= 64 ||
          skinny_us(sms, p->nt, N, K, tiles * p->split, (K / TC_BK + p->split - 1) / p->split) < tc_us(sms, M, N, K, tc_kind(sms, M, N, K, true));
 }
@@ -1421,7 +1431,7 @@ static int gemm_tc_T(cake_b200_ctx *c, const void *A, const void *W, const void 
     sk.tile_group = x.tile_group; sk.row_scale = x.row_scale; sk.err = c->wait_err;
     const bool vec = (((uintptr_t)res | (uintptr_t)C) & 15) == 0 && ldc % 4 == 0;
     CUtensorMap ma, mw;
-    RC(make_tmap(&ma, A, (uint64_t)M, (uint64_t)K, c->cfg.dtype, (uint32_t)sk.nt, (uint64_t)x.a_ld));
+    RC(make_tmap(&ma, A, (uint64_t)(x.a_shared ? sk.rows : M), (uint64_t)K, c->cfg.dtype, (uint32_t)sk.nt, (uint64_t)x.a_ld));
     RC(make_tmap(&mw, W, (uint64_t)N * x.n_groups, (uint64_t)K, c->cfg.dtype, SK_BM, 0, true));
     return launch_cluster_pdl(c, vec ? gemm_skinny_kernel<T, EPI, true> : gemm_skinny_kernel<T, EPI, false>, dim3((unsigned)(N / SK_BM * sk.m_tiles * sk.split)), dim3(SK_THREADS), sk_smem,
                               (unsigned)sk.split, mw, ma, sk);
@@ -1443,6 +1453,40 @@ static int gemm_tc_T(cake_b200_ctx *c, const void *A, const void *W, const void 
   dim3 grid(tiles < c->sm_count ? tiles : c->sm_count), block(TC_THREADS);
   if (kind == TC_WIDE) return launch_pdl(c, gemm_tc_kernel<T, EPI, 256>, grid, block, (size_t)TcCfg<256>::SMEM_BYTES, ma, mb, p);
   return launch_pdl(c, gemm_tc_kernel<T, EPI, 128>, grid, block, (size_t)TcCfg<128>::SMEM_BYTES, ma, mb, p);
+}
+
+// Two products of up to 64 rows in one launch, the first one grouped (gemm_skinny_two_kernel); 16-byte aligned outputs.  *done: false where no plan fits.
+struct TwoGemm { const void *A, *W; void *C; int M, N, K, act, ldc; float cap; };
+template <typename T, int EPI>
+static int gemm_two_T(cake_b200_ctx *c, const TwoGemm &a, const TcExtra &xa, const TwoGemm &b, bool *done) {
+  *done = false;
+  const TwoGemm *g[2] = {&a, &b};
+  const TcExtra *x[2] = {&xa, nullptr};
+  const TcExtra plain;
+  x[1] = &plain;
+  SkParams p[2]{};
+  CUtensorMap ma[2], mw[2];
+  const int rows = xa.group_rows, tiles_a = a.N / SK_BM * (a.M / TC_BM), tiles_b = b.N / SK_BM;
+  if (rows < 1 || rows > 64 || b.M != rows) return CAKE_B200_OK;
+  p[0].nt = (rows + 15) / 16 * 16;
+  size_t smem = 0;
+  if (!cut_skinny(c->sm_count, tiles_a + tiles_b, std::min(a.K, b.K), std::max(a.K, b.K), &p[0], &smem)) return CAKE_B200_OK;
+  p[1] = p[0];
+  for (int i = 0; i < 2; i++) {
+    const TwoGemm &q = *g[i];
+    if ((uintptr_t)q.C & 15 || q.ldc % 4) return CAKE_B200_OK;
+    p[i].C = q.C; p[i].M = q.M; p[i].N = q.N; p[i].K = q.K; p[i].act = q.act; p[i].ldc = q.ldc; p[i].cap = q.cap;
+    p[i].rows = rows;
+    p[i].m_tiles = i == 0 ? q.M / TC_BM : 1;
+    p[i].tile_group = x[i]->tile_group;
+    p[i].a_shared = x[i]->a_shared ? 1 : 0;
+    p[i].err = c->wait_err;
+    RC(make_tmap(&ma[i], q.A, (uint64_t)(x[i]->a_shared ? rows : q.M), (uint64_t)q.K, c->cfg.dtype, (uint32_t)p[i].nt));
+    RC(make_tmap(&mw[i], q.W, (uint64_t)q.N * x[i]->n_groups, (uint64_t)q.K, c->cfg.dtype, SK_BM, 0, true));
+  }
+  *done = true;
+  return launch_cluster_pdl(c, gemm_skinny_two_kernel<T, EPI>, dim3((unsigned)((tiles_a + tiles_b) * p[0].split)), dim3(SK_THREADS), smem, (unsigned)p[0].split,
+                            mw[0], ma[0], mw[1], ma[1], p[0], p[1], tiles_a * p[0].split);
 }
 
 // ------------------------------------------------------------------------------------------ prefill path (any batch / seq)
@@ -2602,11 +2646,13 @@ template <typename Take> static SubScratch sub_scratch(const cake_b200_ctx *c, c
   } else s.f3 = (float *)take(M * sp.heads * sizeof(float));
   return s;
 }
+constexpr int MOE_FEW_TOKENS = 64;  // as many rows as a grouped product on gemm_skinny_kernel has
 struct MoeScratch {
   void *act, *sact, *sorted;
-  float *wts, *sgate, *y, *logits;
+  float *wts, *sgate, *y, *ys, *logits;
   int *ids, *counts, *perm, *pos_of, *tile_expert;
   int max_tiles, tile;
+  bool few;  // enqueue_few_ff may take the call
 };
 static bool moe_on_tc(const cake_b200_ctx *c, const cake_b200_block *b);
 template <typename Take> static MoeScratch moe_scratch(const cake_b200_ctx *c, const cake_b200_block *b, size_t M, Take &&take);
@@ -3074,6 +3120,8 @@ template <typename Take> static MoeScratch moe_scratch(const cake_b200_ctx *c, c
     if (s.tile == TC_BM) s.sorted = take(rows * H * es);
   }
   if (mo.shared_ff) s.sact = take(M * mo.shared_ff * es);
+  s.few = s.sorted && M <= MOE_FEW_TOKENS && nt <= (size_t)mx::MOE_SMALL_PAIRS;
+  if (s.few && mo.shared_ff) s.ys = (float *)take(M * H * sizeof(float));
   return s;
 }
 // The CTAs that a row's keys are cut over in latent attention's vector form (0: a warp per row and head).  A CTA walks its keys 16 at a time, a few us each:
@@ -3121,6 +3169,36 @@ static MixerScratch mixer_scratch(const cake_b200_ctx *c, const cake_b200_block 
   return s;
 }
 
+// The products and the sum of a routed feed-forward of up to MOE_FEW_TOKENS tokens, planned by_token
+template <typename T>
+static int enqueue_few_ff(cake_b200_ctx *c, const cake_b200_block *b, const MoeScratch &w, const void *h, const float *x, float *out, int M, uint64_t *lc) {
+  const cake_b200_moe_spec &mo = b->ms.moe;
+  const int H = c->cfg.hidden, rows = w.max_tiles * w.tile;
+  TcExtra xg;
+  xg.tile_group = w.tile_expert;
+  xg.n_groups = mo.experts;
+  xg.group_rows = M;
+  xg.a_shared = true;
+  const bool shared_tc = mo.shared_ff && listed_tc<T>(c, M, 2 * mo.shared_ff, H) && listed_tc<T>(c, M, H, mo.shared_ff);
+  bool up = false, down = false;
+  if constexpr (sizeof(T) == 2) {
+    if (shared_tc) {
+      RC((gemm_two_T<T, TCE_SWIGLU>(c, {h, b->m_eg, w.act, rows, 2 * mo.ff, H, mo.act, mo.ff, mo.limit}, xg,
+                                    {h, b->wgu, w.sact, M, 2 * mo.shared_ff, H, mo.act, mo.shared_ff, mo.shared_limit}, &up)));
+      if (up) {
+        xg.a_shared = false;
+        RC((gemm_two_T<T, TCE_SOFTCAP_F32>(c, {w.act, b->m_ed, w.y, rows, H, mo.ff, 0, 0, 0.f}, xg, {w.sact, b->wd, w.ys, M, H, mo.shared_ff, 0, 0, 0.f}, &down)));
+      }
+    }
+  }
+  if (!up) RC((listed_gemm_tc<T, TCE_SWIGLU>(c, h, b->m_eg, nullptr, w.act, rows, 2 * mo.ff, H, mo.act, mo.ff, mo.limit, xg)));
+  xg.a_shared = false;
+  if (!down) RC((listed_gemm_tc<T, TCE_SOFTCAP_F32>(c, w.act, b->m_ed, nullptr, w.y, rows, H, mo.ff, 0, 0, 0.f, xg)));
+  mx::MoeCombine mc{x, out, h, w.y, w.wts, w.ids, w.pos_of, M, H, mo.top, mo.experts};
+  if (down) { mc.shared = w.ys; mc.shared_gate = b->shared_gated ? w.sgate : nullptr; }
+  MX(mx::moe_combine(c->stream, c->cfg.dtype, mc, lc));
+  return mo.shared_ff && !down ? enqueue_shared_ff<T>(c, b, w, h, out, out, M) : CAKE_B200_OK;
+}
 // The routed feed-forward on normed rows h [M, hidden] in D: out = (x ? x : 0) + sum over a token's chosen experts of weight *
 // expert(h) (+ weight * h for identity experts) + sigmoid(shared gate) * shared expert(h); out may alias x.
 template <typename T>
@@ -3135,7 +3213,12 @@ static int enqueue_routed_ff(cake_b200_ctx *c, const cake_b200_block *b, const M
   mx::MoePlan mp{w.logits, NP, b->m_corr, b->shared_gated ? 1 : 0, M, H, mo.experts, mo.identity, mo.top, mo.scale, w.ids, w.wts,
                  w.sgate, w.tile, w.counts, w.perm, w.pos_of, w.tile_expert, w.max_tiles, mo.logit_bias, mo.groups, mo.groups_keep, mo.plain_weights,
                  mo.sigmoid_scores};
+  // a few tokens: every expert that one of them chose multiplies all of them (its tile has room for sixteen anyway), so nothing is sorted or gathered; the
+  // shared expert's products join those of the experts
+  const bool few = w.few && out && !mo.weigh_input && M <= MOE_FEW_TOKENS;
+  mp.by_token = few ? 1 : 0;
   MX(mx::moe_route(st, dt, mp, lc));
+  if (few) return enqueue_few_ff<T>(c, b, w, h, x, out, M, lc);
   if (mo.experts && w.sorted) {  // grouped products: sorted rows of h -> act(gate) * up -> down, expert e at row e * N of the stacked weights
     const int rows = w.max_tiles * w.tile;
     MX(mx::moe_gather(st, dt, h, w.perm, w.sorted, rows, H, mo.top, lc, mo.weigh_input ? w.wts : nullptr));

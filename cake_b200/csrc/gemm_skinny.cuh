@@ -45,9 +45,10 @@ struct SkParams {
   void *C;
   int M, N, K, act, ldc;
   float cap;
-  const int *tile_group;     // as TcParams: rows sorted by group in blocks of TC_BM; a block's first nt rows are all it uses
+  const int *tile_group;     // as TcParams: rows sorted by group in blocks of TC_BM; a block's first `rows` rows are all it uses
   const float *row_scale;
-  int nt;                    // rows of A per tile (a multiple of 16)
+  int nt, rows;              // rows of A per tile: as columns of the MMA (a multiple of 16), and those of them that are there
+  int a_shared;              // every row block multiplies the same rows of A, the first ones
   int m_tiles;               // row tiles, TC_BM rows apart
   int split, stages;
   int how;                   // SK_OVER, SK_APART or SK_LEAN
@@ -114,8 +115,7 @@ __device__ __forceinline__ void sk_store(const SkParams &p, int m, int n, const 
 // VEC: C and the residual take accesses of four columns (their addresses and row strides); an instance of its own for what does not, since a kernel of
 // a few microseconds pays for instructions on its way that it does not run
 template <typename T, int EPI, bool VEC>
-__global__ void __launch_bounds__(SK_THREADS, 2)
-gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, const SkParams p) {
+__device__ __forceinline__ void sk_product(const CUtensorMap &map_w, const CUtensorMap &map_a, const SkParams &p, const int block) {
   extern __shared__ unsigned char smem_raw_sk[];
   unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw_sk) + 1023) & ~(uintptr_t)1023);
   __shared__ uint64_t full[SK_MAX_STAGES], empty[SK_MAX_STAGES], acc_full, drained, got;
@@ -123,9 +123,9 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   __shared__ int gave_up;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int S = p.split, nt = p.nt, stage_bytes = sk_stage_bytes(nt);
-  const int unit = (int)blockIdx.x / S, rank = (int)blockIdx.x % S;  // the cluster's CTAs are neighbours along x
+  const int unit = block / S, rank = block % S;  // the cluster's CTAs are neighbours along x
   const int mt = unit % p.m_tiles, n0 = (unit / p.m_tiles) * SK_BM;
-  const int m0 = mt * TC_BM, m_end = min(p.M, m0 + nt);
+  const int m0 = mt * TC_BM, m_end = min(p.M, m0 + p.rows), a0 = p.a_shared ? 0 : m0;
   const int kblocks = p.K / TC_BK, kb0 = (int)((long)kblocks * rank / S), kb1 = (int)((long)kblocks * (rank + 1) / S), nkb = kb1 - kb0;
   uint32_t cols = 32;
   while ((int)cols < nt) cols <<= 1;
@@ -170,7 +170,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         tma_load_2d(smem + (size_t)i * stage_bytes, &map_w, (kb0 + i) * TC_BK, wrow, &full[i]);
       }
       if (!p.tile_group) pdl_wait();
-      for (int i = 0; i < pre; i++) tma_load_2d(smem + (size_t)i * stage_bytes + SK_W_BYTES, &map_a, (kb0 + i) * TC_BK, m0, &full[i]);
+      for (int i = 0; i < pre; i++) tma_load_2d(smem + (size_t)i * stage_bytes + SK_W_BYTES, &map_a, (kb0 + i) * TC_BK, a0, &full[i]);
       int s = 0;
       uint32_t ph = 0;
       issued = pre;
@@ -180,7 +180,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         unsigned char *st = smem + (size_t)s * stage_bytes;
         mbar_arrive_expect_tx_if(left, &full[s], (uint32_t)stage_bytes);
         tma_load_2d(st, &map_w, (kb0 + i) * TC_BK, wrow, &full[s], left);
-        tma_load_2d(st + SK_W_BYTES, &map_a, (kb0 + i) * TC_BK, m0, &full[s], left);
+        tma_load_2d(st + SK_W_BYTES, &map_a, (kb0 + i) * TC_BK, a0, &full[s], left);
         issued += left ? 1 : 0;
         if (++s == p.stages) { s = 0; ph ^= 1u; }
       }
@@ -328,6 +328,22 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
   }
+}
+
+template <typename T, int EPI, bool VEC>
+__global__ void __launch_bounds__(SK_THREADS, 2)
+gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, const SkParams p) {
+  sk_product<T, EPI, VEC>(map_w, map_a, p, (int)blockIdx.x);
+}
+// Two products of one epilogue side by side: the clusters from first_ctas on work on the second (a routed feed-forward's experts and its shared expert, which
+// alone are too short to come up to speed).  Both are cut into clusters of the same size.
+template <typename T, int EPI>
+__global__ void __launch_bounds__(SK_THREADS, 2)
+gemm_skinny_two_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w2,
+                       const __grid_constant__ CUtensorMap map_a2, const SkParams p, const SkParams p2, const int first_ctas) {
+  const bool second = (int)blockIdx.x >= first_ctas;
+  const SkParams q = second ? p2 : p;
+  sk_product<T, EPI, true>(second ? map_w2 : map_w, second ? map_a2 : map_a, q, (int)blockIdx.x - (second ? first_ctas : 0));
 }
 
 }  // namespace cake

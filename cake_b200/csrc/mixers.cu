@@ -1114,13 +1114,8 @@ int gate_norm(cudaStream_t st, int dtype, const GateNorm &p, uint64_t *launches)
 // ---------------------------------------------------------------------------------------------- router
 constexpr int MOE_MAX_SLOTS = 8;  // experts + identity <= 256
 // NS: slots of 32 experts that a warp's lanes hold
-template <typename T, int NS>
-__global__ void __launch_bounds__(128) moe_router_kernel(const MoePlan p) {
-  pdl_launch_dependents();
-  pdl_wait();
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (warp >= p.M) return;
-  const int m = warp, E = p.experts + p.identity;
+template <typename T, int NS> __device__ __forceinline__ void route_token(const MoePlan &p, const int m, const int lane) {
+  const int E = p.experts + p.identity;
   const float *lg = p.logits + (size_t)m * p.ld;
   const T *corr = reinterpret_cast<const T *>(p.correction);
   float z[NS];
@@ -1220,6 +1215,43 @@ __global__ void __launch_bounds__(128) moe_router_kernel(const MoePlan p) {
   }
   if (p.has_shared_gate && lane == 0) p.sgate[m] = 1.0f / (1.0f + expf(-lg[E]));
 }
+template <typename T, int NS>
+__global__ void __launch_bounds__(128) moe_router_kernel(const MoePlan p) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (warp >= p.M) return;
+  route_token<T, NS>(p, warp, lane);
+}
+// by_token: the choices and the plan in one CTA
+template <typename T, int NS>
+__global__ void __launch_bounds__(512) moe_route_few_kernel(const MoePlan p) {
+  pdl_launch_dependents();
+  pdl_wait();
+  __shared__ int first[32 * MOE_MAX_SLOTS];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ne = p.M * p.top;
+  for (int e = threadIdx.x; e < p.experts; e += blockDim.x) first[e] = 0;
+  for (int m = warp; m < p.M; m += blockDim.x >> 5) route_token<T, NS>(p, m, lane);
+  __syncthreads();
+  for (int i = threadIdx.x; i < ne; i += blockDim.x)
+    if (p.ids[i] < p.experts) first[p.ids[i]] = 1;
+  __syncthreads();
+  if (warp == 0) {
+    int done = 0;
+    for (int base = 0; base < p.experts; base += 32) {
+      const int e = base + lane;
+      const bool used = e < p.experts && first[e];
+      const unsigned who = __ballot_sync(0xffffffffu, used);
+      const int at = done + __popc(who & ((1u << lane) - 1u));
+      if (used) { first[e] = at; p.tile_expert[at] = e; }
+      done += __popc(who);
+    }
+    for (int i = done + lane; i < p.max_tiles; i += 32) p.tile_expert[i] = -1;
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < ne; i += blockDim.x)
+    if (p.ids[i] < p.experts) p.pos_of[i] = first[p.ids[i]] * p.tile + i / p.top;
+}
 __global__ void moe_count_kernel(const int *ids, int n, int experts, int *counts) {
   pdl_launch_dependents();
   pdl_wait();
@@ -1258,7 +1290,6 @@ __global__ void moe_scatter_kernel(const int *ids, int n, int experts, int *curs
   }
 }
 // few (token, slot) pairs (decoding): count, plan and scatter in one CTA with the counters in shared memory
-constexpr int MOE_SMALL_PAIRS = 1024;
 __global__ void __launch_bounds__(256) moe_plan_small_kernel(const MoePlan p) {
   pdl_launch_dependents();
   pdl_wait();
@@ -1305,6 +1336,16 @@ int moe_route(cudaStream_t st, int dtype, const MoePlan &p, uint64_t *launches) 
     return (int)cudaErrorInvalidValue;
   if (p.logit_bias && !p.correction) return (int)cudaErrorInvalidValue;
   const int slots = (p.experts + p.identity + 31) / 32;
+  if (p.by_token) {
+    if (p.experts < 1 || p.M > p.tile || p.M * p.top > MOE_SMALL_PAIRS) return (int)cudaErrorInvalidValue;
+    MX_DISPATCH(dtype, {
+      if (slots <= 1) mx_launch(st, moe_route_few_kernel<T, 1>, 1, 512, 0, p);
+      else if (slots <= 2) mx_launch(st, moe_route_few_kernel<T, 2>, 1, 512, 0, p);
+      else if (slots <= 4) mx_launch(st, moe_route_few_kernel<T, 4>, 1, 512, 0, p);
+      else mx_launch(st, moe_route_few_kernel<T, MOE_MAX_SLOTS>, 1, 512, 0, p);
+    });
+    MX_DONE(1);
+  }
   MX_DISPATCH(dtype, {
     const unsigned grid = (unsigned)((p.M + 3) / 4);
     if (slots <= 1) mx_launch(st, moe_router_kernel<T, 1>, grid, 128, 0, p);
@@ -1474,6 +1515,7 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const MoeCombine p) {
   pdl_wait();
   const int m = blockIdx.x;
   const T *h = reinterpret_cast<const T *>(p.h) + (size_t)m * p.W;
+  const float sg = p.shared && p.shared_gate ? p.shared_gate[m] : 1.f;
   if ((p.W & 3) == 0) {  // 16-byte loads and stores of the fp32 rows
     const float4 *x4 = p.x ? reinterpret_cast<const float4 *>(p.x + (size_t)m * p.W) : nullptr;
     float4 *o4 = reinterpret_cast<float4 *>(p.x_out + (size_t)m * p.W);
@@ -1490,6 +1532,10 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const MoeCombine p) {
           s.z = fmaf(w, DT<T>::to_f(h[4 * i + 2]), s.z); s.w = fmaf(w, DT<T>::to_f(h[4 * i + 3]), s.w);
         }
       }
+      if (p.shared) {
+        const float4 y = reinterpret_cast<const float4 *>(p.shared + (size_t)m * p.W)[i];
+        s.x = fmaf(sg, y.x, s.x); s.y = fmaf(sg, y.y, s.y); s.z = fmaf(sg, y.z, s.z); s.w = fmaf(sg, y.w, s.w);
+      }
       o4[i] = s;
     }
     return;
@@ -1501,7 +1547,8 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const MoeCombine p) {
       const int e = p.ids[pr];
       s = fmaf(p.wts ? p.wts[pr] : 1.f, e < p.experts ? p.y[(size_t)p.pos_of[pr] * p.W + i] : DT<T>::to_f(h[i]), s);
     }
-    p.x_out[(size_t)m * p.W + i] = (p.x ? p.x[(size_t)m * p.W + i] : 0.f) + s;
+    s += p.x ? p.x[(size_t)m * p.W + i] : 0.f;
+    p.x_out[(size_t)m * p.W + i] = p.shared ? fmaf(sg, p.shared[(size_t)m * p.W + i], s) : s;
   }
 }
 int moe_combine(cudaStream_t st, int dtype, const MoeCombine &p, uint64_t *launches) {

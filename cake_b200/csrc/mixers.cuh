@@ -182,7 +182,11 @@ struct MoePlan {
   // score s may be chosen; plain_weights: the weights are the scores s (times scale), not renormalised.  correction may be nullptr
   int groups = 0, groups_keep = 0, plain_weights = 0;
   int sigmoid_scores = 0;  // 1: s = sigmoid(z) instead of the softmax
+  // 1: a block of `tile` rows per expert that any token chose (in order of the experts), where token m has row m: pos_of = block * tile + m; perm is not
+  // written.  M <= tile, at most MOE_SMALL_PAIRS pairs
+  int by_token = 0;
 };
+constexpr int MOE_SMALL_PAIRS = 1024;
 int moe_route(cudaStream_t, int dtype, const MoePlan &, uint64_t *launches);
 
 // sorted[r] = h[perm[r] / top] (zeros for padding rows): the operand of a grouped product on the tensor cores
@@ -214,6 +218,7 @@ struct MoeCombine {
   const float *y, *wts;  // wts nullptr: every weight is one
   const int *ids, *pos_of;
   int M, W, top, experts;
+  const float *shared = nullptr, *shared_gate = nullptr;  // [M, W] the shared expert's output, added last, times [M] its gate
 };
 int moe_combine(cudaStream_t, int dtype, const MoeCombine &, uint64_t *launches);
 
