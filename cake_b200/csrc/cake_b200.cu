@@ -1658,6 +1658,31 @@ static int enqueue_prefill_layers(cake_b200_ctx *c, cake_b200_block *const *bloc
 // ------------------------------------------------------------------------------------------ layer-list blocks (fp32 residual stream)
 // include/cake_b200.h, cake_b200_layer_spec: parallel block, scalar/vector RMS norm in fp32, token shift, attention with
 // soft cap / distance bias / window / keys as values / head gate (attn_window_bias.cuh), gated feed-forward.
+// RMS norm of M rows of the fp32 stream (norm_shift_rows_kernel's arguments): a few rows of a step take the kernel that holds them in registers.  At 1000 rows
+// that one is the slower (three Setodra layers 1701 -> 1717 us).
+struct NormRows {
+  const float *x;
+  const int *rows;
+  int row_mul, row_add;
+  const void *g;
+  int g_stride;
+  const void *shift;
+  const float *state_in;
+  float *state_out;
+  void *h, *hs;
+  int M, S, n, pos0;
+  float g_add;
+};
+template <typename T> static int norm_rows(cake_b200_ctx *c, const NormRows &a) {
+  const float eps = c->cfg.rms_eps;
+  if (sizeof(T) == 2 && a.M <= 2 * c->sm_count && a.n % 4 == 0 && a.n <= 16 * NORM_THREADS && (a.g_stride == 0 || a.g_stride == 1) && (!a.shift || a.S == 1) &&
+      (((uintptr_t)a.g | (uintptr_t)a.shift) & 7) == 0)
+    return launch_pdl(c, norm_few_rows_kernel<T>, dim3((unsigned)a.M), dim3(NORM_THREADS), 0, a.x, a.rows, a.row_mul, a.row_add, (const T *)a.g, a.g_stride, (const T *)a.shift,
+                      a.state_in, a.state_out, (T *)a.h, (T *)a.hs, a.n, eps, a.pos0, a.g_add);
+  return launch_pdl(c, norm_shift_rows_kernel<T>, dim3((unsigned)a.M), dim3(256), 0, a.x, a.rows, a.row_mul, a.row_add, (const T *)a.g, a.g_stride, (const T *)a.shift, a.state_in,
+                    a.state_out, (T *)a.h, (T *)a.hs, a.S, a.n, eps, a.pos0, a.g_add);
+}
+
 static int round_up(int v, int m) { return (v + m - 1) / m * m; }
 
 extern "C" int cake_b200_block_load_spec(cake_b200_ctx *c, int layer_idx, const cake_b200_layer_spec *sp,
@@ -1891,9 +1916,8 @@ static int enqueue_listed_layers(cake_b200_ctx *c, cake_b200_block *const *block
       // 1. h = norm(x) (for the feed-forward) and its token-shifted copy (for the mixer)
       const int cs = kc->shift_cur[l];
       const T *mix_in = (const T *)(b->shift ? c->sp_hs : c->sp_h);
-      RC(launch_pdl(c, norm_shift_rows_kernel<T>, dim3(M), dim3(256), 0, cur, (const int *)nullptr, 1, 0, (const T *)b->g, sp.scalar_norm ? 0 : 1,
-                    (const T *)b->shift, (const float *)kc->shift_state[cs][l], kc->shift_state[cs ^ 1][l], (T *)c->sp_h, (T *)c->sp_hs, S, H,
-                    c->cfg.rms_eps, pos0, 0.f));
+      RC(norm_rows<T>(c, {cur, nullptr, 1, 0, b->g, sp.scalar_norm ? 0 : 1, b->shift, (const float *)kc->shift_state[cs][l], kc->shift_state[cs ^ 1][l], c->sp_h,
+                          c->sp_hs, M, S, H, pos0, 0.f}));
       // 2. q | k | gate logits in one product
       RowsGemm gi{mix_in, b->w_in, nullptr, c->sp_in, M, b->n_in, H, H, b->n_in_pad, 0, 0.f};
       if (listed_tc<T>(c, M, b->n_in_pad, H)) RC((listed_gemm_tc<T, TCE_PLAIN>(c, mix_in, b->w_in, nullptr, c->sp_in, M, b->n_in_pad, H, 0, 0)));
@@ -3300,8 +3324,7 @@ static int enqueue_mixer_layers(cake_b200_ctx *c, cake_b200_block *const *blocks
       x_in_h = false;
       const MixerScratch w = mixer_scratch(c, b, (size_t)M, (char *)c->mx_ws, S, pos0 + S);
       // 1. h = norm1(x); every input projection of the mixer in one product
-      RC(launch_pdl(c, norm_shift_rows_kernel<T>, dim3(M), dim3(256), 0, cur, (const int *)nullptr, 1, 0, (const T *)b->ln1, 1, (const T *)nullptr,
-                    (const float *)nullptr, (float *)nullptr, (T *)w.h, (T *)nullptr, S, H, c->cfg.rms_eps, pos0, 0.f));
+      RC(norm_rows<T>(c, {cur, nullptr, 1, 0, b->ln1, 1, nullptr, nullptr, nullptr, w.h, nullptr, M, S, H, pos0, 0.f}));
       RowsGemm gi{w.h, b->w_in, nullptr, w.proj, M, b->n_in, H, H, b->n_in_pad, 0, 0.f};
       if (listed_tc<T>(c, M, b->n_in_pad, H)) RC((listed_gemm_tc<T, TCE_PLAIN>(c, w.h, b->w_in, nullptr, w.proj, M, b->n_in_pad, H, 0, 0)));
       else RC((gemm_rows_T<T, RE_STORE>(c, gi)));
@@ -3387,8 +3410,7 @@ static int enqueue_mixer_layers(cake_b200_ctx *c, cake_b200_block *const *blocks
       cur = x_out;
       // 4. x <- x + routed experts(norm2(x)) + gate * shared expert
       if (sp.moe.experts + sp.moe.identity > 0) {
-        RC(launch_pdl(c, norm_shift_rows_kernel<T>, dim3(M), dim3(256), 0, cur, (const int *)nullptr, 1, 0, (const T *)b->ln2, 1, (const T *)nullptr,
-                      (const float *)nullptr, (float *)nullptr, (T *)w.h, (T *)nullptr, S, H, c->cfg.rms_eps, pos0, 0.f));
+        RC(norm_rows<T>(c, {cur, nullptr, 1, 0, b->ln2, 1, nullptr, nullptr, nullptr, w.h, nullptr, M, S, H, pos0, 0.f}));
         RC(enqueue_routed_ff<T>(c, b, w.moe, w.h, cur, x_out, M, lc));
       }
     }
@@ -3689,10 +3711,8 @@ static int listed_logits(cake_b200_ctx *c, const void *x_dev, const int *rows_ho
                        c->cfg.streams, c->cfg.rms_eps, rows_host ? c->sp_rows_idx : nullptr, row_mul, row_add};
       MX(mx::stream_mix(c->stream, c->cfg.dtype, sm, &c->launches));
     } else
-    RC(launch_pdl(c, norm_shift_rows_kernel<T>, dim3(n), dim3(256), 0, (const float *)x_dev, (const int *)(rows_host ? c->sp_rows_idx : nullptr),
-                  row_mul, row_add, (const T *)c->ln_f,
-                  c->cfg.scalar_final_norm ? 0 : 1, (const T *)nullptr, (const float *)nullptr, (float *)nullptr, (T *)c->sp_hn, (T *)nullptr, 1,
-                  (int)H, c->cfg.rms_eps, 0, c->final_norm_offset));
+    RC(norm_rows<T>(c, {(const float *)x_dev, (const int *)(rows_host ? c->sp_rows_idx : nullptr), row_mul, row_add, c->ln_f, c->cfg.scalar_final_norm ? 0 : 1, nullptr,
+                        nullptr, nullptr, c->sp_hn, nullptr, n, 1, (int)H, 0, c->final_norm_offset}));
     RowsGemm g{c->sp_hn, c->lm_head, nullptr, out_dev ? out_dev : c->sp_logits, n, (int)V, (int)H, (int)H, (int)V, 0, c->cfg.logit_softcap};
     if (listed_tc<T>(c, n, (int)V, (int)H))
       return listed_gemm_tc<T, TCE_SOFTCAP_F32>(c, c->sp_hn, c->lm_head, nullptr, g.C, n, (int)V, (int)H, 0, 0, c->cfg.logit_softcap);

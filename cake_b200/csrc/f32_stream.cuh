@@ -153,6 +153,69 @@ __global__ void __launch_bounds__(256) norm_shift_rows_kernel(const float *__res
   }
 }
 
+constexpr int NORM_THREADS = 256;
+// The kernel above for a few rows of up to 4096 values in 16-bit D, n % 4 == 0, weights on 8 bytes: no shift, or steps of one token (S == 1), so that no row needs
+// the one before it.  The row stays in registers and everything is asked for at once, the weights before the kernel in front has ended: one
+// trip to memory where there were four (step through three Setodra layers, six norms of a row of 2048, 258 -> 243 us).  The same sums and roundings.
+template <typename T>
+__global__ void __launch_bounds__(NORM_THREADS) norm_few_rows_kernel(const float *__restrict__ x, const int *__restrict__ rows, int row_mul, int row_add, const T *__restrict__ g,
+                                                                     int g_stride, const T *__restrict__ shift, const float *__restrict__ state_in, float *__restrict__ state_out,
+                                                                     T *__restrict__ h_out, T *__restrict__ hs_out, int n, float eps, int pos0, float g_add) {
+  pdl_launch_dependents();
+  constexpr int PER = 4;
+  __shared__ float red[NORM_THREADS / 32];
+  const int r = blockIdx.x, b = r;
+  const bool from_state = shift && pos0 > 0;  // t == 0
+  uint2 gr[PER], sr[PER];
+#pragma unroll
+  for (int e = 0; e < PER; e++) {
+    const int i = threadIdx.x + NORM_THREADS * e;
+    gr[e] = sr[e] = make_uint2(0u, 0u);
+    if (i >= n / 4) continue;
+    if (g_stride) gr[e] = reinterpret_cast<const uint2 *>(g)[i];
+    if (shift) sr[e] = reinterpret_cast<const uint2 *>(shift)[i];
+  }
+  const float g0 = g_stride ? 0.f : DT<T>::to_f(g[0]);
+  pdl_wait();
+  x += (rows ? (size_t)rows[r] : (size_t)r * row_mul + row_add) * n;
+  float4 v[PER], u[PER];
+  float ss = 0.f;
+#pragma unroll
+  for (int e = 0; e < PER; e++) {
+    const int i = threadIdx.x + NORM_THREADS * e;
+    v[e] = u[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i >= n / 4) continue;
+    v[e] = reinterpret_cast<const float4 *>(x)[i];
+    if (from_state) u[e] = reinterpret_cast<const float4 *>(state_in + (size_t)b * n)[i];
+  }
+#pragma unroll
+  for (int e = 0; e < PER; e++) {
+    ss = fmaf(v[e].x, v[e].x, ss); ss = fmaf(v[e].y, v[e].y, ss); ss = fmaf(v[e].z, v[e].z, ss); ss = fmaf(v[e].w, v[e].w, ss);
+  }
+  ss = warp_sum(ss);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
+  __syncthreads();
+  float tot = 0.f;
+#pragma unroll
+  for (int i = 0; i < NORM_THREADS / 32; i++) tot += red[i];
+  const float inv = 1.0f / sqrtf(tot / (float)n + eps);
+  typedef typename EmbedBits<T>::type B;
+#pragma unroll
+  for (int e = 0; e < PER; e++) {
+    const int i = threadIdx.x + NORM_THREADS * e;
+    if (i >= n / 4) continue;
+    const float2 ga = DT<B>::unpack2(gr[e].x), gb = DT<B>::unpack2(gr[e].y);
+    const float gi[4] = {(g_stride ? ga.x : g0) + g_add, (g_stride ? ga.y : g0) + g_add, (g_stride ? gb.x : g0) + g_add, (g_stride ? gb.y : g0) + g_add};
+    const float h[4] = {v[e].x * inv * gi[0], v[e].y * inv * gi[1], v[e].z * inv * gi[2], v[e].w * inv * gi[3]};
+    if (h_out) store4<T>(h_out + (size_t)r * n + 4 * i, h[0], h[1], h[2], h[3]);
+    if (shift) {
+      const float2 sa = DT<B>::unpack2(sr[e].x), sb = DT<B>::unpack2(sr[e].y);
+      store4<T>(hs_out + (size_t)r * n + 4 * i, h[0] + (u[e].x - h[0]) * sa.x, h[1] + (u[e].y - h[1]) * sa.y, h[2] + (u[e].z - h[2]) * sb.x, h[3] + (u[e].w - h[3]) * sb.y);
+      *reinterpret_cast<float4 *>(state_out + (size_t)b * n + 4 * i) = make_float4(h[0], h[1], h[2], h[3]);
+    }
+  }
+}
+
 // ---- generic GEMM with the fp32-stream epilogues --------------------------------------------------------------------------
 enum { RE_STORE = 0, RE_GATE_UP = 1, RE_RESIDUAL_F32 = 2, RE_SOFTCAP_F32 = 3, RE_ACT = 4 };
 struct RowsGemm {

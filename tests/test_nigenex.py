@@ -412,3 +412,22 @@ def test_single_tokens_on_a_long_row_share_its_keys(window):
         assert rel_err(r.run("a", toks[1100:], [1]), want) < TOL["bf16"]
     finally:
         r.close()
+
+
+@gpu
+@pytest.mark.parametrize("width", [36, 1028, 2048, 4096, 4100])
+def test_steps_of_a_few_tokens(width):
+    """Rows that a norm holds in registers and rows that it does not (wider than 4096), projections that share a launch (2048, 4096) and ones that don't; steps
+    of one, of a few and of eight and nine tokens, where the attention that lays its own keys down ends."""
+    layers = [LayerSpec(heads=4, kv_heads=2, head_dim=64, window=11, scale=0.125, softcap=30.0, ff=128),
+              LayerSpec(heads=2, kv_heads=1, head_dim=64, window=0, scale=0.125, softcap=0.0, ff=64)]
+    cfg = small_config(layers, width=width)
+    sd = make_listed_checkpoint(cfg, "bf16", seed=19)
+    toks = tokens(47, cfg.vocab_size, 11)
+    want = plain(cfg, sd, toks, "bf16")
+    r = Runner(cfg, sd, "bf16")
+    try:
+        assert rel_err(r.run("a", toks, [5, 1, 1, 3, 8, 9, 1, 2]), want) < TOL["bf16"]
+        assert rel_err(r.run("b", toks, [1]), want) < TOL["bf16"]
+    finally:
+        r.close()
