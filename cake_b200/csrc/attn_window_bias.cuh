@@ -45,6 +45,7 @@ struct WinAttn {
   int pool, chunk, sink_zero;
   float out_scale = 1.f;
   int *err = nullptr;  // attn_window_tc_kernel: host-mapped, a wait that ran out
+  int k_col = -1;      // attn_window_decode_vec_kernel: the step's own keys are still in qkg, from this column on (a head after the other), and join the cache here
 };
 constexpr int WA_MAX_HD = 256;
 
@@ -213,7 +214,8 @@ __global__ void __launch_bounds__(WA_DEC_WARPS * 32) attn_window_decode_kernel(c
 // holds the 16-byte pieces r, r + 8, ... of the row (NCH of them), so a warp's loads are whole rows, a score costs three
 // shuffles, and the registers that fed the dot product also feed the weighted sum (the key is read once).  Every group
 // keeps its own running (m, l, acc) over the keys lo + grp, lo + grp + 64, ... with U rows in flight; the groups merge in a
-// fixed order — shuffles inside a warp, shared memory across the warps — so the result does not depend on timing.
+// fixed order — shuffles inside a warp, shared memory across the warps — so the result does not depend on timing.  The step's own keys may still lie in the
+// projection (k_col): a kernel that only appended them was 2.7 us of a layer's step.
 // Long rows of few items (one token of 16 heads is 16 CTAs, four dependent loads of a group each for 1024 keys): up to eight CTAs of a
 // cluster take every parts-th run of keys and the first merges them over shared memory, again in a fixed order.
 constexpr int WA_DEC_PARTS = 8;
@@ -250,6 +252,10 @@ __global__ void __launch_bounds__(WA_DEC_WARPS * 32) attn_window_decode_vec_kern
   const int pi = p.pos0 + t;
   const int lo = p.window > 0 ? max(0, pi - p.window + 1) : 0;
   const float inv_cap2 = p.softcap > 0.f ? 2.0f / p.softcap : 0.f;
+  const int own = p.k_col >= 0 ? p.pos0 : pi + 1;  // keys from here on are the step's
+  const T *step_k = p.k_col >= 0 ? reinterpret_cast<const T *>(p.qkg) + (size_t)b * p.S * p.ld + p.k_col + (size_t)(h / G) * hd : nullptr;
+  if (p.k_col >= 0 && rank == 0 && h % G == 0 && (int)threadIdx.x < CH)  // one CTA per key row lays it down; nobody reads it there in this step
+    reinterpret_cast<uint4 *>(const_cast<T *>(kc) + (size_t)pi * hd)[threadIdx.x] = reinterpret_cast<const uint4 *>(step_k + (size_t)t * p.ld)[threadIdx.x];
   float m = -INFINITY, l = 0.f;
   for (int base = lo + rank * NG * U; base <= pi; base += parts * NG * U) {  // the trip count is the same for every thread: the shuffles below are whole-warp
     uint4 kr[U][NCH];
@@ -260,7 +266,7 @@ __global__ void __launch_bounds__(WA_DEC_WARPS * 32) attn_window_decode_vec_kern
       for (int c = 0; c < NCH; c++) {
         const int ch = r + 8 * c;
         kr[u][c] = make_uint4(0u, 0u, 0u, 0u);
-        if (j <= pi && ch < CH) kr[u][c] = reinterpret_cast<const uint4 *>(kc + (size_t)j * hd)[ch];
+        if (j <= pi && ch < CH) kr[u][c] = reinterpret_cast<const uint4 *>(j < own ? kc + (size_t)j * hd : step_k + (size_t)(j - own) * p.ld)[ch];
       }
     }
 #pragma unroll

@@ -441,10 +441,12 @@ template <typename T> static int set_smem_attrs_T() {
   CU(cudaFuncSetAttribute(gemm_skinny_kernel<T, EPI, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SK_SMEM_MAX));                  \
   CU(cudaFuncSetAttribute(gemm_skinny_kernel<T, EPI, true>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));\
   CU(cudaFuncSetAttribute(gemm_skinny_kernel<T, EPI, false>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
-  CU(cudaFuncSetAttribute(gemm_skinny_two_kernel<T, TCE_SWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, SK_SMEM_MAX));
-  CU(cudaFuncSetAttribute(gemm_skinny_two_kernel<T, TCE_SOFTCAP_F32>, cudaFuncAttributeMaxDynamicSharedMemorySize, SK_SMEM_MAX));
-  CU(cudaFuncSetAttribute(gemm_skinny_two_kernel<T, TCE_SWIGLU>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
-  CU(cudaFuncSetAttribute(gemm_skinny_two_kernel<T, TCE_SOFTCAP_F32>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+  CU(cudaFuncSetAttribute(gemm_skinny_two_kernel<T, TCE_SWIGLU, TCE_SWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, SK_SMEM_MAX));
+  CU(cudaFuncSetAttribute(gemm_skinny_two_kernel<T, TCE_PLAIN, TCE_SWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, SK_SMEM_MAX));
+  CU(cudaFuncSetAttribute(gemm_skinny_two_kernel<T, TCE_PLAIN, TCE_SWIGLU>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+  CU(cudaFuncSetAttribute(gemm_skinny_two_kernel<T, TCE_SOFTCAP_F32, TCE_SOFTCAP_F32>, cudaFuncAttributeMaxDynamicSharedMemorySize, SK_SMEM_MAX));
+  CU(cudaFuncSetAttribute(gemm_skinny_two_kernel<T, TCE_SWIGLU, TCE_SWIGLU>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+  CU(cudaFuncSetAttribute(gemm_skinny_two_kernel<T, TCE_SOFTCAP_F32, TCE_SOFTCAP_F32>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
   SETK(TCE_PLAIN) SETK(TCE_RESIDUAL) SETK(TCE_SWIGLU) SETK(TCE_RESIDUAL_F32) SETK(TCE_SOFTCAP_F32) SETK(TCE_ACT)
 #undef SETK
   SETT(TCE_PLAIN) SETT(TCE_RESIDUAL) SETT(TCE_SWIGLU) SETT(TCE_RESIDUAL_F32) SETT(TCE_SOFTCAP_F32) SETT(TCE_ACT)
@@ -1455,9 +1457,10 @@ static int gemm_tc_T(cake_b200_ctx *c, const void *A, const void *W, const void 
   return launch_pdl(c, gemm_tc_kernel<T, EPI, 128>, grid, block, (size_t)TcCfg<128>::SMEM_BYTES, ma, mb, p);
 }
 
-// Two products of up to 64 rows in one launch, the first one grouped (gemm_skinny_two_kernel); 16-byte aligned outputs.  *done: false where no plan fits.
+// Two products of the same up to 64 rows in one launch, the first one grouped or not (gemm_skinny_two_kernel); 16-byte aligned outputs.  *done: false
+// where no plan fits.
 struct TwoGemm { const void *A, *W; void *C; int M, N, K, act, ldc; float cap; };
-template <typename T, int EPI>
+template <typename T, int EPI, int EPI2>
 static int gemm_two_T(cake_b200_ctx *c, const TwoGemm &a, const TcExtra &xa, const TwoGemm &b, bool *done) {
   *done = false;
   const TwoGemm *g[2] = {&a, &b};
@@ -1466,7 +1469,7 @@ static int gemm_two_T(cake_b200_ctx *c, const TwoGemm &a, const TcExtra &xa, con
   x[1] = &plain;
   SkParams p[2]{};
   CUtensorMap ma[2], mw[2];
-  const int rows = xa.group_rows, tiles_a = a.N / SK_BM * (a.M / TC_BM), tiles_b = b.N / SK_BM;
+  const int rows = xa.tile_group ? xa.group_rows : a.M, m_tiles = xa.tile_group ? a.M / TC_BM : 1, tiles_a = a.N / SK_BM * m_tiles, tiles_b = b.N / SK_BM;
   if (rows < 1 || rows > 64 || b.M != rows) return CAKE_B200_OK;
   p[0].nt = (rows + 15) / 16 * 16;
   size_t smem = 0;
@@ -1477,7 +1480,7 @@ static int gemm_two_T(cake_b200_ctx *c, const TwoGemm &a, const TcExtra &xa, con
     if ((uintptr_t)q.C & 15 || q.ldc % 4) return CAKE_B200_OK;
     p[i].C = q.C; p[i].M = q.M; p[i].N = q.N; p[i].K = q.K; p[i].act = q.act; p[i].ldc = q.ldc; p[i].cap = q.cap;
     p[i].rows = rows;
-    p[i].m_tiles = i == 0 ? q.M / TC_BM : 1;
+    p[i].m_tiles = i == 0 ? m_tiles : 1;
     p[i].tile_group = x[i]->tile_group;
     p[i].a_shared = x[i]->a_shared ? 1 : 0;
     p[i].err = c->wait_err;
@@ -1485,7 +1488,7 @@ static int gemm_two_T(cake_b200_ctx *c, const TwoGemm &a, const TcExtra &xa, con
     RC(make_tmap(&mw[i], q.W, (uint64_t)q.N * x[i]->n_groups, (uint64_t)q.K, c->cfg.dtype, SK_BM, 0, true));
   }
   *done = true;
-  return launch_cluster_pdl(c, gemm_skinny_two_kernel<T, EPI>, dim3((unsigned)((tiles_a + tiles_b) * p[0].split)), dim3(SK_THREADS), smem, (unsigned)p[0].split,
+  return launch_cluster_pdl(c, gemm_skinny_two_kernel<T, EPI, EPI2>, dim3((unsigned)((tiles_a + tiles_b) * p[0].split)), dim3(SK_THREADS), smem, (unsigned)p[0].split,
                             mw[0], ma[0], mw[1], ma[1], p[0], p[1], tiles_a * p[0].split);
 }
 
@@ -1852,11 +1855,15 @@ template <typename T> static int window_attention_tc(cake_b200_ctx *c, const Win
 }
 template <> int window_attention_tc<float>(cake_b200_ctx *, const WinAttn &, int, uint64_t *, const void *, const void *, int) { return CAKE_B200_EINVAL; }
 // steps of a few tokens in 16-bit D with 16-byte rows: eight lanes per key (attn_window_decode_vec_kernel)
+// steps of a few tokens that attn_window_decode_vec_kernel takes
+template <typename T> static bool listed_attention_in_vectors(const WinAttn &wa) {
+  static const bool no_mma = []() { const char *e = getenv("CAKE_B200_NO_TC"); return e && e[0] == '1'; }();
+  return sizeof(T) == 2 && !no_mma && wa.S <= 8 && wa.hd % 8 == 0 && wa.hd <= WA_MAX_HD && wa.ld % 8 == 0 && wa.kc == wa.vc && wa.gate_col >= -1 &&
+         (((uintptr_t)wa.qkg | (uintptr_t)wa.kc) & 15) == 0;
+}
 template <typename T> static int listed_attention_vec(cake_b200_ctx *c, const WinAttn &wa, bool *done) {
   *done = false;
-  if (wa.hd % 8 != 0 || wa.hd > WA_MAX_HD || wa.ld % 8 != 0 || wa.kc != wa.vc || wa.gate_col < -1 ||
-      (((uintptr_t)wa.qkg | (uintptr_t)wa.kc) & 15) != 0)
-    return CAKE_B200_OK;
+  if (!listed_attention_in_vectors<T>(wa)) return CAKE_B200_OK;
   // CTAs per item: while the chip has room and a group of lanes keeps four keys (its loads in flight): 16 heads of 1024 keys take four each
   const long items = (long)wa.B * wa.S * wa.heads, keys = wa.window > 0 ? std::min(wa.window, wa.pos0 + wa.S) : wa.pos0 + wa.S;
   int parts = 1;
@@ -1881,7 +1888,7 @@ template <typename T> static int listed_attention(cake_b200_ctx *c, const WinAtt
     RC(listed_attention_mma<T>(c, wa, &done));
     if (done) return CAKE_B200_OK;
   }
-  if (wa.S <= 8 && !no_mma) {
+  if (wa.S <= 8) {
     bool done = false;
     RC(listed_attention_vec<T>(c, wa, &done));
     if (done) return CAKE_B200_OK;
@@ -1918,21 +1925,31 @@ static int enqueue_listed_layers(cake_b200_ctx *c, cake_b200_block *const *block
       const T *mix_in = (const T *)(b->shift ? c->sp_hs : c->sp_h);
       RC(norm_rows<T>(c, {cur, nullptr, 1, 0, b->g, sp.scalar_norm ? 0 : 1, b->shift, (const float *)kc->shift_state[cs][l], kc->shift_state[cs ^ 1][l], c->sp_h,
                           c->sp_hs, M, S, H, pos0, 0.f}));
-      // 2. q | k | gate logits in one product
+      // 2. q | k | gate logits in one product, and beside it (a few rows) the feed-forward's input half: act(gate h) * (up h), written next to the
+      // attention's output (one token, four layers of 2048 162 -> 160.5 us, 2 x 5 tokens, three layers, 129.5 -> 120.9)
+      const bool in_tc = listed_tc<T>(c, M, b->n_in_pad, H), up_tc = sp.ff > 0 && listed_tc<T>(c, M, 2 * sp.ff, H) && sq % 8 == 0 && b->k_out % 8 == 0;
+      bool both = false;
+      if constexpr (sizeof(T) == 2) {
+        if (in_tc && up_tc)
+          RC((gemm_two_T<T, TCE_PLAIN, TCE_SWIGLU>(c, {mix_in, b->w_in, c->sp_in, M, b->n_in_pad, H, 0, 0, 0.f}, TcExtra{},
+                                                   {c->sp_h, b->wgu, (T *)c->sp_a + sq, M, 2 * sp.ff, H, sp.act, b->k_out, 0.f}, &both)));
+      }
       RowsGemm gi{mix_in, b->w_in, nullptr, c->sp_in, M, b->n_in, H, H, b->n_in_pad, 0, 0.f};
-      if (listed_tc<T>(c, M, b->n_in_pad, H)) RC((listed_gemm_tc<T, TCE_PLAIN>(c, mix_in, b->w_in, nullptr, c->sp_in, M, b->n_in_pad, H, 0, 0)));
+      if (both) {
+      } else if (in_tc) RC((listed_gemm_tc<T, TCE_PLAIN>(c, mix_in, b->w_in, nullptr, c->sp_in, M, b->n_in_pad, H, 0, 0)));
       else RC((gemm_rows_T<T, RE_STORE>(c, gi)));
-      // 3. the step's keys join the cache, then attention reads keys (= values) only from there
-      RC(launch_pdl(c, rows_to_cache_kernel<T>, dim3(M), dim3(128), 0, (const T *)c->sp_in, (T *)kc->k[l], S, b->n_in_pad, sq, sp.kv_heads, hd,
-                    kc->cap, pos0));
+      // 3. the step's keys join the cache, then attention reads keys (= values) only from there; the kernel for steps of a few tokens lays them down itself
       WinAttn wa{c->sp_in, kc->k[l], kc->k[l], b->r1, b->r2, c->sp_a, B, S, sp.heads, sp.kv_heads, hd, kc->cap, pos0, b->n_in_pad, b->k_out,
                  b->gate_col, sp.window, sp.scale, sp.softcap};
+      if (listed_attention_in_vectors<T>(wa) && sq % 8 == 0) wa.k_col = sq;
+      else
+        RC(launch_pdl(c, rows_to_cache_kernel<T>, dim3(M), dim3(128), 0, (const T *)c->sp_in, (T *)kc->k[l], S, b->n_in_pad, sq, sp.kv_heads, hd,
+                      kc->cap, pos0));
       RC(listed_attention<T>(c, wa));
-      // 4. feed-forward input half: act(gate h) * (up h), written next to the attention output
-      if (sp.ff > 0) {
+      // 4. the feed-forward's input half, where it has not been done yet
+      if (sp.ff > 0 && !both) {
         RowsGemm gu{c->sp_h, b->wgu, nullptr, (T *)c->sp_a + sq, M, 2 * sp.ff, H, H, b->k_out, sp.act, 0.f};
-        if (listed_tc<T>(c, M, 2 * sp.ff, H) && sq % 8 == 0 && b->k_out % 8 == 0)
-          RC((listed_gemm_tc<T, TCE_SWIGLU>(c, c->sp_h, b->wgu, nullptr, (T *)c->sp_a + sq, M, 2 * sp.ff, H, sp.act, b->k_out)));
+        if (up_tc) RC((listed_gemm_tc<T, TCE_SWIGLU>(c, c->sp_h, b->wgu, nullptr, (T *)c->sp_a + sq, M, 2 * sp.ff, H, sp.act, b->k_out)));
         else RC((gemm_rows_T<T, RE_GATE_UP>(c, gu)));
       }
       // 5. x <- x + [attention | ff] . [o | down]^T
@@ -3207,11 +3224,11 @@ static int enqueue_few_ff(cake_b200_ctx *c, const cake_b200_block *b, const MoeS
   bool up = false, down = false;
   if constexpr (sizeof(T) == 2) {
     if (shared_tc) {
-      RC((gemm_two_T<T, TCE_SWIGLU>(c, {h, b->m_eg, w.act, rows, 2 * mo.ff, H, mo.act, mo.ff, mo.limit}, xg,
+      RC((gemm_two_T<T, TCE_SWIGLU, TCE_SWIGLU>(c, {h, b->m_eg, w.act, rows, 2 * mo.ff, H, mo.act, mo.ff, mo.limit}, xg,
                                     {h, b->wgu, w.sact, M, 2 * mo.shared_ff, H, mo.act, mo.shared_ff, mo.shared_limit}, &up)));
       if (up) {
         xg.a_shared = false;
-        RC((gemm_two_T<T, TCE_SOFTCAP_F32>(c, {w.act, b->m_ed, w.y, rows, H, mo.ff, 0, 0, 0.f}, xg, {w.sact, b->wd, w.ys, M, H, mo.shared_ff, 0, 0, 0.f}, &down)));
+        RC((gemm_two_T<T, TCE_SOFTCAP_F32, TCE_SOFTCAP_F32>(c, {w.act, b->m_ed, w.y, rows, H, mo.ff, 0, 0, 0.f}, xg, {w.sact, b->wd, w.ys, M, H, mo.shared_ff, 0, 0, 0.f}, &down)));
       }
     }
   }

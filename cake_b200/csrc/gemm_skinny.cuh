@@ -335,15 +335,21 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
 gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, const SkParams p) {
   sk_product<T, EPI, VEC>(map_w, map_a, p, (int)blockIdx.x);
 }
-// Two products of one epilogue side by side: the clusters from first_ctas on work on the second (a routed feed-forward's experts and its shared expert, which
-// alone are too short to come up to speed).  Both are cut into clusters of the same size.
-template <typename T, int EPI>
+// Two products side by side, the clusters from first_ctas on work on the second: a routed feed-forward's experts and its shared expert, or a block's
+// attention projections and the input half of its feed-forward, which alone are too short to come up to speed.  Both are cut into clusters of the same size.
+template <typename T, int EPI, int EPI2>
 __global__ void __launch_bounds__(SK_THREADS, 2)
 gemm_skinny_two_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w2,
                        const __grid_constant__ CUtensorMap map_a2, const SkParams p, const SkParams p2, const int first_ctas) {
   const bool second = (int)blockIdx.x >= first_ctas;
-  const SkParams q = second ? p2 : p;
-  sk_product<T, EPI, true>(second ? map_w2 : map_w, second ? map_a2 : map_a, q, (int)blockIdx.x - (second ? first_ctas : 0));
+  if (EPI == EPI2) {
+    const SkParams q = second ? p2 : p;
+    sk_product<T, EPI, true>(second ? map_w2 : map_w, second ? map_a2 : map_a, q, (int)blockIdx.x - (second ? first_ctas : 0));
+  } else if (second) {
+    sk_product<T, EPI2, true>(map_w2, map_a2, p2, (int)blockIdx.x - first_ctas);
+  } else {
+    sk_product<T, EPI, true>(map_w, map_a, p, (int)blockIdx.x);
+  }
 }
 
 }  // namespace cake
