@@ -1338,6 +1338,7 @@ static bool tc_gemm_ok(int M, int N, int K) { return M >= 1 && N % TC_BN == 0 &&
 // C = epi(A[M,K] W[N,K]^T) on the tensor cores (gemm_tc.cuh)
 struct TcExtra {  // optional modes of the tensor-core GEMM (TcParams in gemm_tc.cuh)
   const int *tile_group = nullptr;  // grouped product: W holds n_groups stacked [N, K] matrices
+  const int *tile_rows = nullptr;   // grouped product of more than 64 rows: rows of a block that are there
   int n_groups = 1;
   const float *row_scale = nullptr;
   int b_kwrap = 0, w_cols = 0, w_ld = 0;  // W's k coordinate wraps at b_kwrap; its visible columns / row stride when not K
@@ -1442,11 +1443,11 @@ static int gemm_tc_T(cake_b200_ctx *c, const void *A, const void *W, const void 
   const int kind = plan_tiles(c->sm_count, M, N, K, x);
   const int tiles_m = (M + TC_BM - 1) / TC_BM, bn = kind == TC_SMALL ? 128 : 256;
   CUtensorMap ma, mb;
-  RC(make_tmap(&ma, A, (uint64_t)M, (uint64_t)K + (uint64_t)(x.batch - 1) * x.a_step, c->cfg.dtype, TC_BM, (uint64_t)x.a_ld));
+  RC(make_tmap(&ma, A, (uint64_t)M, (uint64_t)K + (uint64_t)(x.batch - 1) * x.a_step, c->cfg.dtype, x.tile_group ? TC_BM / 2 : TC_BM, (uint64_t)x.a_ld));
   // a W that no other row tile reads again comes from HBM in 256-byte pieces (grouped products: 64 experts of 2816 x 2048, one row block each)
   RC(make_tmap(&mb, W, x.w_rows ? (uint64_t)x.w_rows : (uint64_t)N * x.n_groups * x.batch, (uint64_t)(x.w_cols ? x.w_cols : K), c->cfg.dtype,
                kind == TC_PAIR ? 128u : (uint32_t)bn, (uint64_t)x.w_ld ? (uint64_t)x.w_ld : (uint64_t)K, x.tile_group != nullptr));
-  TcParams p{bias, res, C, M, N, K, act >= 0 ? act : (c->cfg.use_gelu_mlp ? 1 : 0), ldc, cap, x.tile_group, x.row_scale, x.b_kwrap, weight ? 1 : 0, x.batch, x.a_step, x.c_step, c->wait_err};
+  TcParams p{bias, res, C, M, N, K, act >= 0 ? act : (c->cfg.use_gelu_mlp ? 1 : 0), ldc, cap, x.tile_group, x.tile_rows, x.row_scale, x.b_kwrap, weight ? 1 : 0, x.batch, x.a_step, x.c_step, c->wait_err};
   if (kind == TC_PAIR) {
     const int units = (tiles_m + 1) / 2 * (N / 256) * x.batch, pairs = std::min(units, c->sm_count / 2);
     return launch_cluster_pdl(c, gemm_tc_kernel<T, EPI, 256, true>, dim3((unsigned)(2 * pairs)), dim3(TC_THREADS), (size_t)TcCfg<256, true>::SMEM_BYTES, 2u, ma, mb, p);
@@ -2691,7 +2692,7 @@ constexpr int MOE_FEW_TOKENS = 64;  // as many rows as a grouped product on gemm
 struct MoeScratch {
   void *act, *sact, *sorted;
   float *wts, *sgate, *y, *ys, *logits;
-  int *ids, *counts, *perm, *pos_of, *tile_expert;
+  int *ids, *counts, *perm, *pos_of, *tile_expert, *tile_rows;
   int max_tiles, tile;
   bool few;  // enqueue_few_ff may take the call
 };
@@ -3155,6 +3156,7 @@ template <typename Take> static MoeScratch moe_scratch(const cake_b200_ctx *c, c
   s.perm = (int *)take(rows * sizeof(int));
   s.pos_of = (int *)take(nt * sizeof(int));
   s.tile_expert = (int *)take(s.max_tiles * sizeof(int));
+  s.tile_rows = (int *)take(s.max_tiles * sizeof(int));
   if (mo.experts) {
     s.act = take(rows * mo.ff * es);
     s.y = (float *)take(rows * H * sizeof(float));
@@ -3258,13 +3260,15 @@ static int enqueue_routed_ff(cake_b200_ctx *c, const cake_b200_block *b, const M
   // shared expert's products join those of the experts
   const bool few = w.few && out && !mo.weigh_input && M <= MOE_FEW_TOKENS;
   mp.by_token = few ? 1 : 0;
+  mp.tile_rows = w.tile_rows;
   MX(mx::moe_route(st, dt, mp, lc));
   if (few) return enqueue_few_ff<T>(c, b, w, h, x, out, M, lc);
   if (mo.experts && w.sorted) {  // grouped products: sorted rows of h -> act(gate) * up -> down, expert e at row e * N of the stacked weights
     const int rows = w.max_tiles * w.tile;
-    MX(mx::moe_gather(st, dt, h, w.perm, w.sorted, rows, H, mo.top, lc, mo.weigh_input ? w.wts : nullptr));
+    MX(mx::moe_gather(st, dt, h, w.ids, w.pos_of, mo.experts, w.sorted, M * mo.top, H, mo.top, lc, mo.weigh_input ? w.wts : nullptr));
     TcExtra xg;
     xg.tile_group = w.tile_expert;
+    xg.tile_rows = w.tile_rows;
     xg.n_groups = mo.experts;
     xg.group_rows = std::min(M, (int)TC_BM);  // a token chooses an expert at most once
     RC((listed_gemm_tc<T, TCE_SWIGLU>(c, w.sorted, b->m_eg, nullptr, w.act, rows, 2 * mo.ff, H, mo.act, mo.ff, mo.limit, xg)));

@@ -56,6 +56,7 @@ struct TcParams {
   // names the group of a row block (< 0: the block is empty and skipped), and group g multiplies by rows g * N .. g * N + N - 1
   // of W (map_b covers all groups).  nullptr: one group.
   const int *tile_group = nullptr;
+  const int *tile_rows = nullptr;  // grouped: rows of a block that are there (nullptr: all TC_BM); the others are neither read nor written
   // TCE_RESIDUAL_F32: optional [M] fp32, C = residual + row_scale[m] * accumulator (a per-row gate on the product)
   const float *row_scale = nullptr;
   // k-block coordinate of W wraps at this many elements (0 = never): A = [P_hi | P_lo] against one copy of W
@@ -239,14 +240,18 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
       int s = 0, early = 0;
       uint32_t ph = 0;
+      int a_boxes = 2;  // a grouped product's A comes in boxes of 64 rows: experts of 1000 tokens have 50 rows for the most part
       auto expect = [&](int st) {  // PAIR: the first CTA's barrier counts both CTAs' bytes
-        if (!PAIR) mbar_arrive_expect_tx_if(left, &full[st], Cfg::STAGE_BYTES);
+        if (!PAIR) mbar_arrive_expect_tx_if(left, &full[st], Cfg::STAGE_BYTES - (2 - a_boxes) * (TC_BM / 2 * TC_BK * 2));
         else if (crank == 0) mbar_arrive_expect_tx_if(left, &full[st], 2 * Cfg::STAGE_BYTES);
       };
       auto load_a = [&](int st, int col, int m0) {
         unsigned char *d = smem + (size_t)st * Cfg::STAGE_BYTES;
         if (PAIR) tma_load_2d_pair(d, &map_a, col, m0, cluster_map(smem_u32(&full[st]), 0u), left);
-        else tma_load_2d(d, &map_a, col, m0, &full[st], left);
+        else {
+          tma_load_2d(d, &map_a, col, m0, &full[st], left);
+          if (p.tile_group && a_boxes > 1) tma_load_2d(d + TC_BM / 2 * TC_BK * 2, &map_a, col, m0 + TC_BM / 2, &full[st], left);
+        }
       };
       auto load_w = [&](int st, int kb, int wrow) {
         unsigned char *d = smem + (size_t)st * Cfg::STAGE_BYTES + TC_BM * TC_BK * 2;
@@ -269,6 +274,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           const int g = p.tile_group[m0 / TC_BM];
           if (g < 0) continue;
           wrow += g * p.N;
+          a_boxes = p.tile_rows && p.tile_rows[m0 / TC_BM] <= TC_BM / 2 ? 1 : 2;
         }
         for (int kb = 0; kb < kblocks; kb++) {
           if (early > 0) early--;
@@ -342,12 +348,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       const int a = it & 1;
       const uint32_t aph = (uint32_t)(it >> 1) & 1u;
       it++;
-      const int row = m0 + wq * 32 + lane;
+      const int row = m0 + wq * 32 + lane, m_end = p.tile_rows ? min(p.M, m0 + p.tile_rows[m0 / TC_BM]) : p.M;
       // the residual of a chunk of 32 columns: the first one is on its way while the products run, the next one while a chunk is finished
       constexpr int RW = EPI == TCE_RESIDUAL ? 4 : EPI == TCE_RESIDUAL_F32 ? 8 : 1;
       uint4 rr[RW];
       auto load_res = [&](int col) {
-        if ((EPI != TCE_RESIDUAL && EPI != TCE_RESIDUAL_F32) || row >= p.M) return;
+        if ((EPI != TCE_RESIDUAL && EPI != TCE_RESIDUAL_F32) || row >= m_end) return;
         const uint4 *r4 = EPI == TCE_RESIDUAL ? reinterpret_cast<const uint4 *>(res + (size_t)row * ld + h * p.c_step + col)
                                               : reinterpret_cast<const uint4 *>(reinterpret_cast<const float *>(p.residual) + (size_t)row * p.N + col);
 #pragma unroll
@@ -358,10 +364,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       if (!__all_sync(0xffffffffu, left != 0)) break;
       tc_fence_after();
 #pragma unroll 1
-      for (int c0 = cw0; c0 < cw0 + CW; c0 += 32) {
+      for (int c0 = cw0; c0 < cw0 + CW && m0 + wq * 32 < m_end; c0 += 32) {
         uint32_t r[32];
         tc_ld32(tmem_base + ((uint32_t)(wq * 32) << 16) + (uint32_t)(a * BN + c0), r);
-        if (row < p.M) {
+        if (row < m_end) {
           if (EPI == TCE_SWIGLU) {
             uint32_t o[8];
             auto pairs = [&](int act) {

@@ -185,13 +185,14 @@ struct MoePlan {
   // 1: a block of `tile` rows per expert that any token chose (in order of the experts), where token m has row m: pos_of = block * tile + m; perm is not
   // written.  M <= tile, at most MOE_SMALL_PAIRS pairs
   int by_token = 0;
+  int *tile_rows = nullptr;  // [max_tiles] or nullptr: rows of a block that are there (not by_token)
 };
 constexpr int MOE_SMALL_PAIRS = 1024;
 int moe_route(cudaStream_t, int dtype, const MoePlan &, uint64_t *launches);
 
 // sorted[r] = h[perm[r] / top] (zeros for padding rows): the operand of a grouped product on the tensor cores
 // (wts [M, top] != nullptr: times the pair's weight, rounded to D once)
-int moe_gather(cudaStream_t, int dtype, const void *h, const int *perm, void *sorted, int rows, int W, int top, uint64_t *launches,
+int moe_gather(cudaStream_t, int dtype, const void *h, const int *ids, const int *pos_of, int experts, void *sorted, int pairs, int W, int top, uint64_t *launches,
                const float *wts = nullptr);
 
 // CUDA-core experts for every shape and D = float: act = f(Wg h) * (Wu h), then y[sorted row] = Wd act

@@ -426,6 +426,23 @@ def test_experts_of_few_rows_cut_along_k(rows):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("dtype", ["bf16", "f16"])
+@pytest.mark.parametrize("rows", [1, 16, 33, 64, 90, 260, 500])
+@pytest.mark.parametrize("shared", [0, 64, 320])
+def test_routed_feed_forward_at_any_number_of_rows(rows, shared, dtype):
+    """Steps whose experts all multiply all rows, with no shared expert, one of a single k-block and one longer than the experts; and prompts whose blocks hold
+    less than 64, up to 128 or more rows of an expert.  Some tokens choose an identity expert."""
+    cfg = make_config([retention(heads=2, dim=64, vdim=64, rot_dims=32, decay=[0.95, 0.99], moe=moe(experts=4, identity=1, top=2, ff=192, shared_ff=shared))], width=256, vocab=96)
+    sd = make_mixer_checkpoint(cfg, dtype, seed=59)
+    toks = tokens(rows, cfg.vocab_size, seed=rows)
+    r = Runner(cfg, sd, dtype)
+    try:
+        close(r.run("w", toks), plain(cfg, sd, toks), dtype, "prompt")
+    finally:
+        r.close()
+
+
+@pytest.mark.gpu
 def test_long_portions_on_the_tensor_cores():
     """Sizes at which long portions in bf16 take the matrix-product form of the latent attention (several blocks of rows, with
     and without keys from earlier portions) and the grouped expert products, against the plain model and against the same
