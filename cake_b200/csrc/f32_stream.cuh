@@ -154,11 +154,11 @@ __global__ void __launch_bounds__(256) norm_shift_rows_kernel(const float *__res
 }
 
 constexpr int NORM_THREADS = 256;
-// The kernel above for a few rows of up to 4096 values in 16-bit D, n % 4 == 0, weights on 8 bytes: no shift, or steps of one token (S == 1), so that no row needs
+// The kernel above for rows of up to 4096 values in 16-bit D, n % 4 == 0, weights on 8 bytes: no shift, or steps of one token (S == 1), so that no row needs
 // the one before it.  The row stays in registers and everything is asked for at once, the weights before the kernel in front has ended: one
 // trip to memory where there were four (step through three Setodra layers, six norms of a row of 2048, 258 -> 243 us).  The same sums and roundings.
 template <typename T>
-__global__ void __launch_bounds__(NORM_THREADS) norm_few_rows_kernel(const float *__restrict__ x, const int *__restrict__ rows, int row_mul, int row_add, const T *__restrict__ g,
+__global__ void __launch_bounds__(NORM_THREADS) norm_rows_kernel(const float *__restrict__ x, const int *__restrict__ rows, int row_mul, int row_add, const T *__restrict__ g,
                                                                      int g_stride, const T *__restrict__ shift, const float *__restrict__ state_in, float *__restrict__ state_out,
                                                                      T *__restrict__ h_out, T *__restrict__ hs_out, int n, float eps, int pos0, float g_add) {
   pdl_launch_dependents();
