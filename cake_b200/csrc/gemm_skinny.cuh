@@ -270,6 +270,7 @@ __device__ __forceinline__ void sk_product(const CUtensorMap &map_w, const CUten
         mbar_wait_lim(&got, 0, p.err, left);
         go = __all_sync(0xffffffffu, left != 0);
       }
+      if (!go && live) mbar_drain(&got, 0);  // gave up: what peers have sent all the same lands before anybody leaves
       cluster_arrive_relaxed();  // (waited for at the end: nobody leaves while sums are on their way)
     } else {
       cluster_wait();
