@@ -69,42 +69,65 @@ __device__ __forceinline__ float rotated(const T *v, int i, int dims, const floa
 }
 
 // ---------------------------------------------------------------------------------------------- latent attention: prep
+// Steps of a few rows: the first CTA of a row norms its latent and lays the cache row down, the others rotate its heads' queries (one CTA took 9.3 us for
+// the 16 heads of one row, a trip to memory per pass of its loops).
 template <typename T>
 __global__ void __launch_bounds__(128) latent_prep_kernel(const LatentPrep p) {
   pdl_launch_dependents();
   pdl_wait();
   __shared__ float red[4];
-  const int m = blockIdx.x, b = m / p.S, t = m % p.S, pos = p.pos0 + t;
+  const int m = blockIdx.x, b = m / p.S, t = m % p.S, pos = p.pos0 + t, part = blockIdx.y, parts = gridDim.y;
   const T *row = reinterpret_cast<const T *>(p.proj) + (size_t)m * p.ld;
   const T *kv = row + p.kv_col;
   const int Dk = p.rank + p.rot, half = p.rope_dims >> 1;
   const float *cs = p.cos_t + (size_t)pos * half, *sn = p.sin_t + (size_t)pos * half;
-  float ss = 0.f;
-  for (int i = threadIdx.x; i < p.rank; i += blockDim.x) {
-    const float v = DT<T>::to_f(kv[i]);
-    ss = fmaf(v, v, ss);
+  if (part == 0) {
+    constexpr int PER = 4;  // entries of a thread that stay in registers; a longer rank is read again
+    const T *w = reinterpret_cast<const T *>(p.norm_w);
+    T rv[PER], rw[PER];
+    float ss = 0.f;
+#pragma unroll
+    for (int e = 0; e < PER; e++) {
+      const int i = threadIdx.x + 128 * e;
+      rv[e] = rw[e] = DT<T>::from_f(0.f);
+      if (i < p.rank) { rv[e] = kv[i]; rw[e] = w[i]; }
+    }
+#pragma unroll
+    for (int e = 0; e < PER; e++) {
+      const float v = DT<T>::to_f(rv[e]);
+      ss = fmaf(v, v, ss);
+    }
+    for (int i = threadIdx.x + 128 * PER; i < p.rank; i += 128) {
+      const float v = DT<T>::to_f(kv[i]);
+      ss = fmaf(v, v, ss);
+    }
+    ss = warp_sum(ss);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
+    __syncthreads();
+    const float inv = 1.0f / sqrtf((red[0] + red[1] + red[2] + red[3]) / (float)p.rank + p.eps);
+    T *crow = reinterpret_cast<T *>(p.cache) + ((size_t)b * p.cap + pos) * Dk;
+    T *ct = p.cache_t ? reinterpret_cast<T *>(p.cache_t) + (size_t)b * p.rank * p.cap_t + pos : nullptr;
+    auto lay = [&](int i, T x, T g) {
+      const T c = DT<T>::from_f(DT<T>::to_f(x) * inv * DT<T>::to_f(g));
+      crow[i] = c;
+      if (ct) ct[(size_t)i * p.cap_t] = c;
+    };
+#pragma unroll
+    for (int e = 0; e < PER; e++)
+      if ((int)threadIdx.x + 128 * e < p.rank) lay(threadIdx.x + 128 * e, rv[e], rw[e]);
+    for (int i = threadIdx.x + 128 * PER; i < p.rank; i += 128) lay(i, kv[i], w[i]);
+    for (int i = threadIdx.x; i < p.rot; i += 128) crow[p.rank + i] = DT<T>::from_f(rotated<T>(kv + p.rank, i, p.rope_dims, cs, sn));
+    if (parts > 1) return;
   }
-  ss = warp_sum(ss);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
-  __syncthreads();
-  const float inv = 1.0f / sqrtf((red[0] + red[1] + red[2] + red[3]) / (float)p.rank + p.eps);
-  T *crow = reinterpret_cast<T *>(p.cache) + ((size_t)b * p.cap + pos) * Dk;
-  const T *w = reinterpret_cast<const T *>(p.norm_w);
-  T *ct = p.cache_t ? reinterpret_cast<T *>(p.cache_t) + (size_t)b * p.rank * p.cap_t + pos : nullptr;
-  for (int i = threadIdx.x; i < p.rank; i += blockDim.x) {
-    const T c = DT<T>::from_f(DT<T>::to_f(kv[i]) * inv * DT<T>::to_f(w[i]));
-    crow[i] = c;
-    if (ct) ct[(size_t)i * p.cap_t] = c;
-  }
-  for (int i = threadIdx.x; i < p.rot; i += blockDim.x) crow[p.rank + i] = DT<T>::from_f(rotated<T>(kv + p.rank, i, p.rope_dims, cs, sn));
   T *qa = reinterpret_cast<T *>(p.qa) + (size_t)m * p.heads * Dk;
-  for (int i = threadIdx.x; i < p.heads * p.rot; i += blockDim.x) {
+  for (int i = (parts > 1 ? part - 1 : 0) * 128 + threadIdx.x; i < p.heads * p.rot; i += (parts > 1 ? parts - 1 : 1) * 128) {
     const int h = i / p.rot, r = i % p.rot;
     qa[(size_t)h * Dk + p.rank + r] = DT<T>::from_f(rotated<T>(row + (size_t)h * (p.dim + p.rot) + p.dim, r, p.rope_dims, cs, sn));
   }
 }
 int latent_prep(cudaStream_t st, int dtype, const LatentPrep &p, uint64_t *launches) {
-  MX_DISPATCH(dtype, (mx_launch(st, latent_prep_kernel<T>, p.B * p.S, 128, 0, p)));
+  const int parts = p.B * p.S <= 16 ? 1 + (p.heads * p.rot + 127) / 128 : 1;
+  MX_DISPATCH(dtype, (mx_launch(st, latent_prep_kernel<T>, dim3(p.B * p.S, parts), 128, 0, p)));
   MX_DONE(1);
 }
 
@@ -929,7 +952,6 @@ constexpr int SC_TOK = 16;
 template <typename T, int TAPS>
 __global__ void __launch_bounds__(128) short_conv_vec_kernel(const ShortConv p) {
   pdl_launch_dependents();
-  pdl_wait();
   const int c8 = blockIdx.y * blockDim.x + threadIdx.x;
   if (c8 >= p.channels / 8) return;
   const int ch = c8 * 8, chunks = (p.S + SC_TOK - 1) / SC_TOK, b = blockIdx.x / chunks, t0 = (blockIdx.x % chunks) * SC_TOK;
@@ -957,6 +979,7 @@ __global__ void __launch_bounds__(128) short_conv_vec_kernel(const ShortConv p) 
       for (int e = 0; e < 8; e++) bias[e] = 0.f;
     }
   }
+  pdl_wait();
 #pragma unroll
   for (int jt = 0; jt < TAPS - 1; jt++) {  // the rows before the chunk: this step's, the history's, or zeros before position 0
     const int tt = t0 - (TAPS - 1) + jt;
@@ -986,8 +1009,18 @@ __global__ void __launch_bounds__(128) short_conv_vec_kernel(const ShortConv p) 
 #pragma unroll
       for (int e = 0; e < 8; e++) x[jt][e] = x[jt + 1][e];
   }
+  // A portion of one chunk: this thread has read all that its channels' history had to give, so it leaves the new one behind (a launch of its own
+  // where chunks read the history that another one would overwrite)
+  if (chunks == 1) {
+    T *h = reinterpret_cast<T *>(p.hist) + (size_t)b * (TAPS - 1) * p.channels + ch;
+#pragma unroll
+    for (int jt = 0; jt < TAPS - 1; jt++)
+      *reinterpret_cast<uint4 *>(h + (size_t)jt * p.channels) =
+          make_uint4(pack2x<T>(x[jt][0], x[jt][1]), pack2x<T>(x[jt][2], x[jt][3]), pack2x<T>(x[jt][4], x[jt][5]), pack2x<T>(x[jt][6], x[jt][7]));
+  }
 }
-template <typename T> static void launch_short_conv(cudaStream_t st, const ShortConv &p) {
+// true: the history is done too
+template <typename T> static bool launch_short_conv(cudaStream_t st, const ShortConv &p) {
   const bool vec = p.channels % 8 == 0 && p.ld % 8 == 0 && p.col0 % 8 == 0 && p.taps >= 2 && p.taps <= 4 &&
                    (((uintptr_t)p.in | (uintptr_t)p.hist | (uintptr_t)p.out | (uintptr_t)p.bias | (uintptr_t)p.w) & 15) == 0;
   const dim3 gv(p.B * ((p.S + SC_TOK - 1) / SC_TOK), (p.channels / 8 + 127) / 128);
@@ -995,9 +1028,11 @@ template <typename T> static void launch_short_conv(cudaStream_t st, const Short
   else if (vec && p.taps == 3) mx_launch(st, short_conv_vec_kernel<T, 3>, gv, 128, 0, p);
   else if (vec && p.taps == 4) mx_launch(st, short_conv_vec_kernel<T, 4>, gv, 128, 0, p);
   else mx_launch(st, short_conv_kernel<T>, dim3(p.B * p.S, (p.channels + 255) / 256), 256, 0, p);
+  return vec && p.S <= SC_TOK;
 }
-template <> void launch_short_conv<float>(cudaStream_t st, const ShortConv &p) {
+template <> bool launch_short_conv<float>(cudaStream_t st, const ShortConv &p) {
   mx_launch(st, short_conv_kernel<float>, dim3(p.B * p.S, (p.channels + 255) / 256), 256, 0, p);
+  return false;
 }
 // after the convolution: the history becomes the last taps - 1 inputs up to the end of this step (zeros before position 0)
 template <typename T>
@@ -1018,11 +1053,12 @@ __global__ void short_conv_hist_kernel(const ShortConv p) {
   }
 }
 int short_conv(cudaStream_t st, int dtype, const ShortConv &p, uint64_t *launches) {
+  bool done = false;
   MX_DISPATCH(dtype, {
-    launch_short_conv<T>(st, p);
-    if (p.taps > 1) mx_launch(st, short_conv_hist_kernel<T>, (p.B * p.channels + 255) / 256, 256, 0, p);
+    done = launch_short_conv<T>(st, p) || p.taps < 2;
+    if (!done) mx_launch(st, short_conv_hist_kernel<T>, (p.B * p.channels + 255) / 256, 256, 0, p);
   });
-  MX_DONE(p.taps > 1 ? 2 : 1);
+  MX_DONE(done ? 1 : 2);
 }
 
 // ---------------------------------------------------------------------------------------------- gated unit norm
@@ -1047,6 +1083,58 @@ __global__ void __launch_bounds__(128) gate_norm_kernel(const GateNorm p) {
   // parts whose rows start on 16 bytes: four entries per lane and load
   const bool vec = sizeof(T) == 2 && (len & 3) == 0 && (p.n & 3) == 0 && (p.ldg & 3) == 0 && (p.ldo & 3) == 0 &&
                    ((uintptr_t)p.o & 15) == 0 && ((uintptr_t)p.out & 7) == 0 && (((uintptr_t)p.gate | (uintptr_t)(p.w ? p.w : p.gate)) & 7) == 0;
+  // A part of up to 512 entries stays in registers and is asked for at once; longer ones are read twice, a trip to memory per pass of either loop.  Bound by
+  // those trips: eight parts of 512 took 8.2 us as loops; with the convolution's history and the latent rows below, a step through three Setodra blocks
+  // went from 245.4 to 236.4 us and a prompt of 1000 tokens from 1565 to 1559.
+  if (vec && len <= 512) {
+    typedef typename Bits16<T>::type B;
+    constexpr int PER = 4;
+    float4 ov[PER];
+    uint2 gr[PER], wr[PER];
+#pragma unroll
+    for (int e = 0; e < PER; e++) {
+      const int i = lane + 32 * e;
+      ov[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+      gr[e] = wr[e] = make_uint2(0u, 0u);
+      if (i < len / 4) {
+        ov[e] = reinterpret_cast<const float4 *>(o)[i];
+        gr[e] = reinterpret_cast<const uint2 *>(gate)[i];
+        if (w) wr[e] = reinterpret_cast<const uint2 *>(w)[i];
+      }
+    }
+    float v[PER][4], gs[PER][4];
+#pragma unroll
+    for (int e = 0; e < PER; e++) {
+      if (lane + 32 * e >= len / 4) continue;
+      const float2 ga = DT<B>::unpack2(gr[e].x), gb = DT<B>::unpack2(gr[e].y);
+      gs[e][0] = gact(ga.x); gs[e][1] = gact(ga.y); gs[e][2] = gact(gb.x); gs[e][3] = gact(gb.y);
+      v[e][0] = ov[e].x; v[e][1] = ov[e].y; v[e][2] = ov[e].z; v[e][3] = ov[e].w;
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        if (p.row_div) v[e][k] /= rdiv;
+        if (p.gate_first) v[e][k] *= gs[e][k];
+        ss = fmaf(v[e][k], v[e][k], ss);
+      }
+    }
+    ss = warp_sum(ss);
+    const float inv = 1.0f / sqrtf(ss / (float)len + p.eps);
+#pragma unroll
+    for (int e = 0; e < PER; e++) {
+      const int i = lane + 32 * e;
+      if (i >= len / 4) continue;
+      const float2 wa = DT<B>::unpack2(wr[e].x), wb = DT<B>::unpack2(wr[e].y);
+      const float wv[4] = {wa.x, wa.y, wb.x, wb.y};
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        float r = v[e][k] * inv;
+        if (w) r *= wv[k];
+        if (!p.gate_first) r *= gs[e][k];
+        v[e][k] = r * p.out_scale;
+      }
+      *reinterpret_cast<uint2 *>(out + 4 * i) = make_uint2(pack2x<B>(v[e][0], v[e][1]), pack2x<B>(v[e][2], v[e][3]));
+    }
+    return;
+  }
   if (vec) {
     const float4 *o4 = reinterpret_cast<const float4 *>(o);
     const uint2 *g2 = reinterpret_cast<const uint2 *>(gate), *w2 = reinterpret_cast<const uint2 *>(w);

@@ -443,6 +443,24 @@ def test_routed_feed_forward_at_any_number_of_rows(rows, shared, dtype):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("dtype", ["bf16", "f16"])
+@pytest.mark.parametrize("taps,parts,vdim,rank", [(2, 1, 64, 512), (3, 1, 80, 520), (4, 1, 128, 200), (4, 2, 128, 513), (2, 8, 2, 40)])
+def test_small_kernels_of_a_step(taps, parts, vdim, rank, dtype):
+    """Portions of up to 16 tokens leave their convolution's history behind in the convolution's own launch, and up to 16 rows of a latent cache share their
+    queries' rotation out; a norm's part of up to 512 entries (512, 640, 1024, 512 and 2 here) and a rank of up to 512 stay in registers."""
+    cfg = make_config([mamba(heads=8, vdim=vdim, state=24, groups=1, conv=taps, norm_groups=parts, moe=None),
+                       latent(heads=5, dim=24, rot_dim=40, vdim=24, kv_rank=rank, moe=None)], width=64, vocab=96)
+    sd = make_mixer_checkpoint(cfg, dtype, seed=61)
+    toks = tokens(61, cfg.vocab_size, seed=taps)
+    r = Runner(cfg, sd, dtype)
+    try:
+        close(r.run("p", toks, cuts=[1, 2, 16, 17, 3, 1]), plain(cfg, sd, toks), dtype, "portions")
+        close(r.run("w", toks), plain(cfg, sd, toks), dtype, "whole")
+    finally:
+        r.close()
+
+
+@pytest.mark.gpu
 def test_long_portions_on_the_tensor_cores():
     """Sizes at which long portions in bf16 take the matrix-product form of the latent attention (several blocks of rows, with
     and without keys from earlier portions) and the grouped expert products, against the plain model and against the same
