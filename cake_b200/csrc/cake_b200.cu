@@ -1354,7 +1354,9 @@ struct TcExtra {  // optional modes of the tensor-core GEMM (TcParams in gemm_tc
 // 4096 rows (one kernel after the other, weights from HBM; mostly within 15 %, the order of the three within 5 %).
 // gemm_tc: a launch with its last epilogue, the k-blocks of the first round (64 wide; the ring's round trip rather than its bytes: 128 x 128 with
 // six stages, 128 x 256 with four, 256 x 256 on a pair of SMs with six), and for every further round of tiles over the chip its k-blocks
-// or, where K is short, the epilogue of the tile in front.  The last round counts as a full one.  Small, wide, pairs in us:
+// or, where K is short, the epilogue of the tile in front.  The last round counts as a full one.  Fitted
+// when the epilogue had four warps; refitted to the eight it has, the choice came out worse where a model's products follow one another (a prompt of 250
+// tokens, 28 layers of 1024: 587 -> 606 us; 1500 tokens, layer-list blocks: 871 -> 891).  Small, wide, pairs in us, as fitted:
 //   N = 6144, K = 4096:  300 rows 25.0, 31.7, 29.7;  512 rows 45.5, 33.7, 31.6;  1000 rows 73.4, 62.2, 56.4
 //   N = 6144, K = 1024 (gated):  1000 rows 28.7, 34.2, 35.0;  1500 rows 35.2, 34.5, 36.3
 enum { TC_SMALL = 0, TC_WIDE = 1, TC_PAIR = 2 };
@@ -1378,7 +1380,7 @@ static int tc_kind(int sms, int M, int N, int K, bool pairs) {
 static double skinny_us(int sms, int nt, int N, int K, int ctas, int kblocks) {
   return std::max((double)((ctas + sms - 1) / sms) * kblocks * sk_stage_bytes(nt) / 80e3, 2.0 * N * K / 6.4e6) + 3.5 + 0.03 * nt;
 }
-// gemm_skinny_kernel's shape for a product, or false where gemm_tc_kernel takes it.
+// A skinny launch's cluster size, stages and exchange; false where no cut fits shared memory.
 static bool cut_skinny(int sms, int tiles, int k_min, int k_max, SkParams *p, size_t *smem) {  // slices of W in all, the shortest and the longest K
   // The cut along K, each CTA with at least two k-blocks: as many CTAs as stay resident at once (three per SM up to 64 rows, two up to 112, one
   // beyond: a ring has three stages or more), but a second one per SM only with four k-blocks each and a third with eight (us, S CTAs per slice:
@@ -1404,6 +1406,7 @@ static bool cut_skinny(int sms, int tiles, int k_min, int k_max, SkParams *p, si
   }
   return *smem <= SK_SMEM_MAX;
 }
+// gemm_skinny_kernel's shape for a product, or false where gemm_tc_kernel takes it.
 static bool plan_skinny(int sms, int M, int N, int K, const TcExtra &x, SkParams *p, size_t *smem) {
   if (x.w_live || x.b_kwrap || x.w_cols || x.w_rows || x.w_ld || x.batch > 1) return false;
   const int rows = x.tile_group ? x.group_rows : M;

@@ -4,6 +4,7 @@
 //   norm_shift_rows_kernel   RMS norm in fp32 with a scalar or a vector gain, and the token shift
 //                            hs = h + (h_prev - h) * shift  (h_prev = the previous position's h, zeros at position 0);
 //                            the operands of the matrix products leave in D
+//   norm_rows_kernel         the same for 16-bit D and rows of up to 4096 entries: a row stays in its CTA's registers
 //   gemm_rows_kernel         C = A[M,K] · W[N,K]^T on the CUDA cores, fp32 accumulation, with the epilogues this block needs:
 //                            store in D | act(gate) * up on row-interleaved gate/up | fp32 residual add | soft-capped fp32
 //                            logits | act(C) in D.  It serves every shape and D = float (true fp32: one FFMA per product, no TF32); the

@@ -18,8 +18,8 @@
 //   warps 4-11  epilogue: tcgen05.ld 32x32b.x32 (thread = accumulator row, every other warp of the same rows the other half of the
 //            columns), fused epilogue, 16-byte global stores; overlaps with the MMAs of the next tile through the second accumulator.
 //            Two warps per scheduler, because one alone issued an instruction every six cycles: 65,000 cycles for a gated tile of
-//            128 x 256, twice its products' time (64 experts of 2816 x 2048 for 1000 tokens: 230 -> 180 us, an instruction budget of the
-//            divisions and exponentials; four warps per scheduler 176).
+//            128 x 256, twice its products' time (64 experts of 2816 x 2048 for 1000 tokens: 230 -> 180 us; four warps per scheduler 176, since
+//            by then the scheduler is busy with the exponentials and divisions themselves).
 #pragma once
 #include <cuda.h>
 
@@ -33,8 +33,8 @@ namespace cake {
 constexpr int TC_BM = 128, TC_BK = 64, TC_EPI_WARPS = 8, TC_THREADS = 128 + 32 * TC_EPI_WARPS;
 constexpr int TC_BN = 128;                     // granularity the host checks N against (BN = 256 when N % 256 == 0)
 template <int BN, bool PAIR = false> struct TcCfg {
-  static constexpr int STAGES = PAIR ? (BN == 256 ? 6 : 8) : BN == 256 ? 4 : 6;
-  static constexpr int STAGE_BYTES = (TC_BM + (PAIR ? BN / 2 : BN)) * TC_BK * 2;  // 32 KB | 48 KB | 32 KB, 24 KB
+  static constexpr int STAGES = (BN == 256 && !PAIR) ? 4 : 6;
+  static constexpr int STAGE_BYTES = (TC_BM + (PAIR ? BN / 2 : BN)) * TC_BK * 2;  // 32 KB | 48 KB | 32 KB
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
 };
 // TCE_RESIDUAL_F32: C (fp32) = residual (fp32) + accumulator, nothing rounded to D — the output projection of a block whose
@@ -173,6 +173,7 @@ template <> __device__ __forceinline__ uint32_t tc_idesc<__half>(int bn) {
 template <typename T, int EPI, int BN, bool PAIR = false>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const TcParams p) {
+  static_assert(!PAIR || BN == 256, "the pair is built for 256 columns");
   typedef TcCfg<BN, PAIR> Cfg;
   extern __shared__ unsigned char smem_raw_tc[];
   unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw_tc) + 1023) & ~(uintptr_t)1023);
@@ -212,8 +213,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   pdl_launch_dependents();
   if (!p.w_early || warp != 0) pdl_wait();
   const uint32_t tmem_base = *tmem_ptr;
-  // (83 of 111 blocks in use, 1000 tokens: dealt out with the empty ones some SMs had 7.8 tiles of 6.2; three layers 1981 -> 1922 us)
-  if (p.tile_group) {  // row blocks behind the last one in use don't count: the tiles are dealt out over the chip without them
+  // Row blocks behind the last one in use don't count: the tiles are dealt out over the chip without them (83 of 111 blocks in use, 1000 tokens: dealt out
+  // with the empty ones some SMs had 7.8 tiles of 6.2; three layers 1981 -> 1922 us).
+  if (p.tile_group) {
     int used = 0;
     for (int i = lane; i < tiles_m; i += 32)
       if (p.tile_group[i] >= 0) used = i + 1;
@@ -255,7 +257,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       };
       auto load_w = [&](int st, int kb, int wrow) {
         unsigned char *d = smem + (size_t)st * Cfg::STAGE_BYTES + TC_BM * TC_BK * 2;
-        if (PAIR) tma_load_2d_pair(d, &map_b, kb * TC_BK, wrow + (int)crank * (BN / 2), cluster_map(smem_u32(&full[st]), 0u), left);  // our half of the W tile
+        if (PAIR) tma_load_2d_pair(d, &map_b, kb * TC_BK, wrow + (int)crank * 128, cluster_map(smem_u32(&full[st]), 0u), left);  // a 128-row box: our half of the W tile
         else tma_load_2d(d, &map_b, p.b_kwrap ? (kb * TC_BK) % p.b_kwrap : kb * TC_BK, wrow, &full[st], left);
       };
       if (p.w_early) {  // (not a grouped product: the groups are another kernel's output)
