@@ -13,6 +13,7 @@
 #include <atomic>
 #include <algorithm>
 #include <chrono>
+#include <memory>
 #include <mutex>
 #include <thread>
 #include <set>
@@ -3166,7 +3167,8 @@ template <typename Take> static MoeScratch moe_scratch(const cake_b200_ctx *c, c
     if (s.tile == TC_BM) s.sorted = take(rows * H * es);
   }
   if (mo.shared_ff) s.sact = take(M * mo.shared_ff * es);
-  s.few = s.sorted && M <= MOE_FEW_TOKENS && nt <= (size_t)mx::MOE_SMALL_PAIRS;
+  // (by the sizes alone: the pass that adds up the bytes has no addresses)
+  s.few = mo.experts && s.tile == TC_BM && M <= MOE_FEW_TOKENS && nt <= (size_t)mx::MOE_SMALL_PAIRS;
   if (s.few && mo.shared_ff) s.ys = (float *)take(M * H * sizeof(float));
   return s;
 }
@@ -4317,6 +4319,30 @@ extern "C" int cake_b200_debug_packet_wait(cake_b200_ctx *c, int what, int fresh
 extern "C" int cake_b200_debug_polls(cake_b200_ctx *c, int polls) {
   if (!c || polls < 0 || polls > MK_POLLS) return fail(CAKE_B200_EINVAL, "bad debug_polls arguments");
   c->mk_polls = polls ? polls : MK_POLLS;
+  return CAKE_B200_OK;
+}
+
+/* test aid (not in the public header), needs no GPU: the scratch of a routed feed-forward of M tokens, {bytes that are added up before it is allocated, end of the
+ * last piece that is dealt out of it, offset of the shared expert's sums (0: none)}. */
+extern "C" int cake_b200_debug_routed_scratch(int dtype, int hidden, int experts, int identity, int top, int ff, int shared_ff, int M, long long *out3) {
+  if (!out3 || hidden < 1 || experts < 0 || identity < 0 || top < 1 || M < 1) return fail(CAKE_B200_EINVAL, "bad debug_routed_scratch arguments");
+  std::unique_ptr<cake_b200_ctx> c(new cake_b200_ctx());
+  std::unique_ptr<cake_b200_block> b(new cake_b200_block());
+  c->cfg.dtype = dtype; c->cfg.hidden = hidden;
+  c->es = dtype == CAKE_B200_F32 ? 4 : 2;
+  cake_b200_moe_spec &mo = b->ms.moe;
+  mo.experts = experts; mo.identity = identity; mo.top = top; mo.ff = ff; mo.shared_ff = shared_ff;
+  char *const base = (char *)256;  // never read: places only
+  for (int i = 0; i < 2; i++) {
+    size_t off = 0;
+    const MoeScratch s = moe_scratch(c.get(), b.get(), (size_t)M, [&](size_t bytes) -> void * {
+      void *p = i ? base + off : nullptr;
+      off += (bytes + 255) / 256 * 256;
+      return p;
+    });
+    out3[i] = (long long)off;
+    if (i) out3[2] = s.ys ? (char *)s.ys - base : 0;
+  }
   return CAKE_B200_OK;
 }
 

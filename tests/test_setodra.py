@@ -425,6 +425,23 @@ def test_experts_of_few_rows_cut_along_k(rows):
         r.close()
 
 
+@pytest.mark.parametrize("dtype", [0, 1, 2])   # bf16, f16, f32
+@pytest.mark.parametrize("rows", [1, 2, 33, 64, 65, 1000])
+@pytest.mark.parametrize("hidden,experts,top,ff,shared", [(256, 4, 2, 192, 320), (256, 4, 2, 192, 0), (2048, 64, 6, 1408, 2816), (256, 130, 32, 64, 64), (40, 5, 2, 24, 40), (256, 0, 1, 0, 64)])
+def test_scratch_of_a_routed_feed_forward_holds_every_piece(hidden, experts, top, ff, shared, rows, dtype):
+    """What is added up before the scratch is allocated is what is dealt out of it; steps of up to 64 tokens keep their shared expert's sums in it."""
+    import ctypes
+    from cake_b200.capi import check, lib
+    fn, out = lib().cake_b200_debug_routed_scratch, (ctypes.c_longlong * 3)()
+    check(fn(dtype, hidden, experts, 1, top, ff, shared, rows, out))
+    asked, end, sums = out
+    assert asked == end
+    if dtype != 2 and shared and experts and hidden % 128 == 0 and ff % 64 == 0 and rows <= 64 and rows * top <= 1024:
+        assert 0 < sums and sums + rows * hidden * 4 <= asked
+    else:
+        assert sums == 0
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", ["bf16", "f16"])
 @pytest.mark.parametrize("rows", [1, 16, 33, 64, 90, 260, 500])
