@@ -1348,6 +1348,7 @@ struct TcExtra {  // optional modes of the tensor-core GEMM (TcParams in gemm_tc
   bool w_live = false;                    // W was written by an earlier kernel of the stream (a cache, not a weight)
   int group_rows = 0;                     // grouped product: no row block holds more rows than this (0 = unknown)
   bool a_shared = false;                  // grouped product of up to 64 rows: A is these rows, and every row block multiplies all of them
+  bool row_tiles = false;                 // an output of one or two slices of W, whatever the rows: they may be dealt out in tiles of TC_BM
   int batch = 1, a_step = 0, c_step = 0;  // side-by-side products: product i reads columns i * a_step .. of A's rows and rows i * N .. of W and
                                           // writes columns i * c_step .. of C's rows (TCE_PLAIN, with a_ld and ldc)
 };
@@ -1410,14 +1411,19 @@ static bool cut_skinny(int sms, int tiles, int k_min, int k_max, SkParams *p, si
 // gemm_skinny_kernel's shape for a product, or false where gemm_tc_kernel takes it.
 static bool plan_skinny(int sms, int M, int N, int K, const TcExtra &x, SkParams *p, size_t *smem) {
   if (x.w_live || x.b_kwrap || x.w_cols || x.w_rows || x.w_ld || x.batch > 1) return false;
-  const int rows = x.tile_group ? x.group_rows : M;
+  // Row tiles (a router: N = 128 for the most part): gemm_tc_kernel has a CTA per 128 rows and cuts nothing along K, eight CTAs for 1000 tokens (K = 2048: 15.0 ->
+  // 10.6 us, three routed layers 1577 -> 1560; 260 tokens 1138 -> 1119).  Only where clusters of eight with four k-blocks each find room: at K = 1024 nothing is won
+  // (700 tokens 633 and 634), with clusters of two 4 x 1500 tokens took 6290 us and not 6190.
+  const bool tiled = x.row_tiles && !x.tile_group && M > SK_MAX_ROWS;
+  const int rows = x.tile_group ? x.group_rows : tiled ? TC_BM : M;
   if (rows < 1 || rows > (x.tile_group ? 64 : SK_MAX_ROWS)) return false;
   p->rows = rows;
   p->nt = (rows + 15) / 16 * 16;
   p->a_shared = x.a_shared ? 1 : 0;
-  p->m_tiles = x.tile_group ? M / TC_BM : 1;
+  p->m_tiles = x.tile_group ? M / TC_BM : tiled ? (M + TC_BM - 1) / TC_BM : 1;
   const int tiles = N / SK_BM * p->m_tiles;
   if (!cut_skinny(sms, tiles, K, K, p, smem)) return false;
+  if (tiled) return p->split == SK_MAX_SPLIT && K / TC_BK >= 4 * SK_MAX_SPLIT;
   return x.tile_group || rows <= 64 ||
          skinny_us(sms, p->nt, N, K, tiles * p->split, (K / TC_BK + p->split - 1) / p->split) < tc_us(sms, M, N, K, tc_kind(sms, M, N, K, true));
 }
@@ -3256,7 +3262,9 @@ static int enqueue_routed_ff(cake_b200_ctx *c, const cake_b200_block *b, const M
   cudaStream_t st = c->stream;
   const int NP = round_up(mo.experts + mo.identity + 1, TC_BN);
   RowsGemm gr{h, b->m_router, nullptr, w.logits, M, NP, H, H, NP, 0, 0.f};
-  if (listed_tc<T>(c, M, NP, H)) RC((listed_gemm_tc<T, TCE_SOFTCAP_F32>(c, h, b->m_router, nullptr, w.logits, M, NP, H, 0, 0)));
+  TcExtra xr;
+  xr.row_tiles = true;
+  if (listed_tc<T>(c, M, NP, H)) RC((listed_gemm_tc<T, TCE_SOFTCAP_F32>(c, h, b->m_router, nullptr, w.logits, M, NP, H, 0, 0, 0.f, xr)));
   else RC((gemm_rows_T<T, RE_SOFTCAP_F32>(c, gr)));
   mx::MoePlan mp{w.logits, NP, b->m_corr, b->shared_gated ? 1 : 0, M, H, mo.experts, mo.identity, mo.top, mo.scale, w.ids, w.wts,
                  w.sgate, w.tile, w.counts, w.perm, w.pos_of, w.tile_expert, w.max_tiles, mo.logit_bias, mo.groups, mo.groups_keep, mo.plain_weights,

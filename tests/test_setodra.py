@@ -460,6 +460,21 @@ def test_routed_feed_forward_at_any_number_of_rows(rows, shared, dtype):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("rows", [256, 257, 384, 500])
+@pytest.mark.parametrize("experts", [6, 130])   # a router of one slice of 128 columns and of two
+def test_router_of_many_rows(rows, experts):
+    """Above 256 rows a router's product deals them out in tiles of 128 and cuts K: the last tile holds one row, 128 and 116 here."""
+    cfg = make_config([retention(heads=2, dim=64, vdim=64, rot_dims=32, decay=[0.95, 0.99], moe=moe(experts=experts, identity=1, top=2, ff=64, shared_ff=0))], width=2048, vocab=96)
+    sd = make_mixer_checkpoint(cfg, "bf16", seed=67)
+    toks = tokens(rows, cfg.vocab_size, seed=rows)
+    r = Runner(cfg, sd, "bf16")
+    try:
+        close(r.run("w", toks), plain(cfg, sd, toks), "bf16", "prompt")
+    finally:
+        r.close()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("dtype", ["bf16", "f16"])
 @pytest.mark.parametrize("taps,parts,vdim,rank", [(2, 1, 64, 512), (3, 1, 80, 520), (4, 1, 128, 200), (4, 2, 128, 513), (2, 8, 2, 40)])
 def test_small_kernels_of_a_step(taps, parts, vdim, rank, dtype):
