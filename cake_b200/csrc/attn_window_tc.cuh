@@ -108,6 +108,7 @@ attn_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       auto issue_s = [&](int j) {  // S_j = Q K_j^T into S buffer j&1
         const int st = j & 1;
         mbar_wait_lim(&k_full[st], (uint32_t)(j >> 1) & 1u, p.err, left);
+        __syncwarp();  // every lane has seen this phase before one of them begins what completes the next
         tc_fence_after();
         const uint64_t q0 = tc_smem_desc(q_s), kt = tc_smem_desc(k_s) + (uint64_t)(st * (FT_KV_BYTES >> 4));
         if (one) {
@@ -130,6 +131,7 @@ attn_window_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         if (j + 1 < n_tiles) issue_s(j + 1);
         mbar_wait_lim(p_full, (uint32_t)j & 1u, p.err, left);  // P_j in TMEM (over S_j), O rescaled
         mbar_wait_lim(&v_full[st], (uint32_t)(j >> 1) & 1u, p.err, left);
+        __syncwarp();
         tc_fence_after();
         const uint64_t vt = ft_desc_mn(v_s, FT_KV_BYTES / 2) + (uint64_t)(st * (FT_KV_BYTES >> 4));
         if (one) {

@@ -196,6 +196,7 @@ __device__ __forceinline__ void sk_product(const CUtensorMap &map_w, const CUten
 #pragma unroll 1
       for (int i = 0; i < nkb; i++) {
         mbar_wait_lim(&full[s], ph, p.err, left);
+        __syncwarp();  // every lane has seen this phase before one of them begins what completes the next
         tc_fence_after();
         const uint64_t dw = dw0 + (uint64_t)(s * (stage_bytes >> 4)), da = da0 + (uint64_t)(s * (stage_bytes >> 4));
         if (one) {

@@ -314,6 +314,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         const uint32_t tmem_c = tmem_base + (uint32_t)(a * BN);
         for (int kb = 0; kb < kblocks; kb++) {
           mbar_wait_lim(&full[s], ph, p.err, left);
+          __syncwarp();  // every lane has seen this phase before one of them begins what completes the next
           tc_fence_after();
           const uint64_t da = da0 + (uint64_t)(s * (Cfg::STAGE_BYTES >> 4)), db = db0 + (uint64_t)(s * (Cfg::STAGE_BYTES >> 4));
           if (one) {
