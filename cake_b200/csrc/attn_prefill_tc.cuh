@@ -88,7 +88,7 @@ __device__ __forceinline__ void ft_drain(uint64_t *bars, int warp, int lane, int
     for (int i = max(0, k_loads - 2); i < k_loads; i++) mbar_drain(&bars[1 + (i & 1)], (uint32_t)(i >> 1) & 1u);
     for (int i = max(0, v_loads - 2); i < v_loads; i++) mbar_drain(&bars[5 + (i & 1)], (uint32_t)(i >> 1) & 1u);
   }
-  if (warp == 5 && lane == 0) {
+  if (warp == 5 && elect_one()) {
     tc_commit(&bars[FT_BARS - 1]);
     mbar_drain(&bars[FT_BARS - 1], 0);
   }

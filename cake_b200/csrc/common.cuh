@@ -231,6 +231,7 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 
 // 1 in one lane of a whole warp.  The thread that issues tcgen05 products is picked this way and the warp runs the loop with it: behind lane == 0 the
 // operands of every product make their own way to the uniform registers, 411 cycles a k-block of four products against 270 (128 x 16 x 64; 294 at N = 128).
+// The same lane every time (elect.sync picks one lane per mask), which a commit needs: it counts the products of its own thread.
 __device__ __forceinline__ uint32_t elect_one() {
   uint32_t r;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));

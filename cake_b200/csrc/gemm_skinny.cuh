@@ -319,7 +319,7 @@ __device__ __forceinline__ void sk_product(const CUtensorMap &map_w, const CUten
   if (gave_up) {
     if (threadIdx.x == 0)
       for (int i = max(0, issued - p.stages); i < issued; i++) mbar_drain(&full[i % p.stages], (uint32_t)(i / p.stages) & 1u);
-    if (threadIdx.x == 32) {
+    if (warp == 1 && elect_one()) {
       tc_commit(&drained);
       mbar_drain(&drained, 0);
     }

@@ -456,7 +456,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   if (*gave_up) {  // (PAIR: the first CTA's barriers count both CTAs' copies and products)
     if (warp == 0 && lane == 0 && crank == 0)
       for (int i = max(0, issued - Cfg::STAGES); i < issued; i++) mbar_drain(&full[i % Cfg::STAGES], (uint32_t)(i / Cfg::STAGES) & 1u);
-    if (warp == 1 && lane == 0 && crank == 0) {
+    if (warp == 1 && crank == 0 && elect_one()) {
       if (PAIR) tc_commit_pair(drained);
       else tc_commit(drained);
       mbar_drain(drained, 0);

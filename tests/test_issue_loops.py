@@ -35,3 +35,20 @@ def test_every_lane_has_seen_a_phase_before_one_issues(name):
         if re.search(r"\bif \(one\)", x):
             assert not open_wait, f"{name}: a lane issues behind a wait that others may still be in"
     assert waits == KERNELS[name]
+
+
+@pytest.mark.parametrize("name", KERNELS)
+def test_the_lane_that_issues_is_the_one_that_commits(name):
+    """A commit counts the products of its own thread: one by another lane completes at once, and a CTA that gave up would hand its tensor memory back
+    under products in flight."""
+    guard, commits = [], 0   # the lines that opened the enclosing blocks
+    for x in lines(name):
+        if re.search(r"\btc_commit(_pair)?\(", x) and "__device__" not in x:
+            commits += 1
+            assert any("if (one)" in g or "elect_one()" in g for g in guard + [x]), f"{name}: {x.strip()}"
+        for ch in x:
+            if ch == "{":
+                guard.append(x)
+            elif ch == "}":
+                guard.pop()
+    assert commits >= 3
