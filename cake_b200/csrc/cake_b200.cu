@@ -1408,8 +1408,9 @@ static bool cut_skinny(int sms, int tiles, int k_min, int k_max, SkParams *p, si
   }
   return *smem <= SK_SMEM_MAX;
 }
-// gemm_skinny_kernel's shape for a product, or false where gemm_tc_kernel takes it.
-static bool plan_skinny(int sms, int M, int N, int K, const TcExtra &x, SkParams *p, size_t *smem) {
+// gemm_skinny_kernel's shape for a product, or false where gemm_tc_kernel takes it.  `unaligned`: C or the residual is not on 16 bytes, which only
+// gemm_skinny_kernel can write or read, so it takes whatever it can.
+static bool plan_skinny(int sms, int M, int N, int K, const TcExtra &x, SkParams *p, size_t *smem, bool unaligned = false) {
   if (x.w_live || x.b_kwrap || x.w_cols || x.w_rows || x.w_ld || x.batch > 1) return false;
   // Row tiles (a router: N = 128 for the most part): gemm_tc_kernel has a CTA per 128 rows and cuts nothing along K, eight CTAs for 1000 tokens (K = 2048: 15.0 ->
   // 10.6 us, three routed layers 1577 -> 1560; 260 tokens 1138 -> 1119).  Only where clusters of eight with four k-blocks each find room: at K = 1024 nothing is won
@@ -1424,7 +1425,7 @@ static bool plan_skinny(int sms, int M, int N, int K, const TcExtra &x, SkParams
   const int tiles = N / SK_BM * p->m_tiles;
   if (!cut_skinny(sms, tiles, K, K, p, smem)) return false;
   if (tiled) return p->split == SK_MAX_SPLIT && K / TC_BK >= 4 * SK_MAX_SPLIT;
-  return x.tile_group || rows <= 64 ||
+  return x.tile_group || rows <= 64 || unaligned ||
          skinny_us(sms, p->nt, N, K, tiles * p->split, (K / TC_BK + p->split - 1) / p->split) < tc_us(sms, M, N, K, tc_kind(sms, M, N, K, true));
 }
 // gemm_tc_kernel's tile: the one whose rounds over the chip come out shortest; a grouped product's neighbours belong to different groups, and a
@@ -1438,17 +1439,19 @@ static int gemm_tc_T(cake_b200_ctx *c, const void *A, const void *W, const void 
                      int act = -1, int ldc = 0, float cap = 0.f, const TcExtra &x = TcExtra{}) {
   SkParams sk{};
   size_t sk_smem = 0;
-  if (plan_skinny(c->sm_count, M, N, K, x, &sk, &sk_smem)) {
+  const bool aligned = (((uintptr_t)res | (uintptr_t)C) & 15) == 0;
+  if (plan_skinny(c->sm_count, M, N, K, x, &sk, &sk_smem, !aligned)) {
     sk.bias = bias; sk.residual = res; sk.C = C; sk.M = M; sk.N = N; sk.K = K; sk.ldc = ldc; sk.cap = cap;
     sk.act = act >= 0 ? act : (c->cfg.use_gelu_mlp ? 1 : 0);
     sk.tile_group = x.tile_group; sk.row_scale = x.row_scale; sk.err = c->wait_err;
-    const bool vec = (((uintptr_t)res | (uintptr_t)C) & 15) == 0 && ldc % 4 == 0;
+    const bool vec = aligned && ldc % 4 == 0;
     CUtensorMap ma, mw;
     RC(make_tmap(&ma, A, (uint64_t)(x.a_shared ? sk.rows : M), (uint64_t)K, c->cfg.dtype, (uint32_t)sk.nt, (uint64_t)x.a_ld));
     RC(make_tmap(&mw, W, (uint64_t)N * x.n_groups, (uint64_t)K, c->cfg.dtype, SK_BM, 0, true));
     return launch_cluster_pdl(c, vec ? gemm_skinny_kernel<T, EPI, true> : gemm_skinny_kernel<T, EPI, false>, dim3((unsigned)(N / SK_BM * sk.m_tiles * sk.split)), dim3(SK_THREADS), sk_smem,
                               (unsigned)sk.split, mw, ma, sk);
   }
+  if (!aligned) return fail(CAKE_B200_EINVAL, "a call of %d rows needs its output on an address that is a multiple of 16", M);
   const bool weight = !x.tile_group && !x.w_live && !x.b_kwrap;
   const int kind = plan_tiles(c->sm_count, M, N, K, x);
   const int tiles_m = (M + TC_BM - 1) / TC_BM, bn = kind == TC_SMALL ? 128 : 256;
@@ -4383,10 +4386,6 @@ extern "C" int cake_b200_debug_product(cake_b200_ctx *c, int epi, const void *A,
   TcExtra x;
   if (group) { x.tile_group = group; x.n_groups = n_groups; x.group_rows = group_rows; }
   x.row_scale = row_scale;
-  SkParams sk{};
-  size_t sk_smem = 0;
-  if ((((uintptr_t)C | (uintptr_t)res) & 15) && !plan_skinny(c->sm_count, M, N, K, x, &sk, &sk_smem))  // (the other kernel's accesses are 16 bytes wide)
-    return fail(CAKE_B200_EINVAL, "bad debug_product arguments");
   if (batch > 1) { x.batch = batch; x.a_ld = batch * K; x.a_step = K; x.c_step = N; }
   const int ldc = batch > 1 ? batch * N : 0;
   RC(DISPATCH_T(c->cfg.dtype, T_LAMBDA {

@@ -5,7 +5,7 @@ import ctypes
 import pytest
 import torch
 
-from cake_b200.capi import check, lib, ptr
+from cake_b200.capi import CakeB200Error, check, lib, ptr
 from cake_b200.model import Context
 from tests.util import checkpoint, medium_config
 
@@ -196,4 +196,25 @@ def test_sums_of_a_cluster(ctx, M, N, K, split):
         off = torch.cat([r.flatten()[:1], r.flatten()])[1:] if r is not None else None
         torch.cuda.synchronize()
         check(lib().cake_b200_debug_product(ctx.h, epi, ptr(a), ptr(w), None, ptr(off) if off is not None else None, ptr(c), M, N, K, 0, 0.0, None, 0, 0, None, 1))
+        near(c.view(want.shape), want, bound, (epi, "two bytes off"))
+
+
+# shapes of 65 .. 256 rows that the estimates give to gemm_tc_kernel, whose accesses are 16 bytes wide, and one with more rows than gemm_skinny_kernel has
+@pytest.mark.gpu
+@pytest.mark.parametrize("M,N,K", [(227, 256, 2048), (254, 128, 2048), (215, 6144, 14336), (257, 256, 2048)])
+def test_outputs_on_any_address(ctx, M, N, K):
+    """A caller's output two bytes off a 16-byte address: as many rows as the kernel for any address has go there, more are refused before a launch."""
+    a, w, g = operands(ctx, M, N, K, M + N)
+    res = torch.randn(M, N, device=a.device, generator=g).to(ctx.D)
+    for epi, r in ((PLAIN, None), (RESIDUAL, res)):
+        want, bound = reference(epi, a, w, None, r, 0, 0.0, ctx.D, None)
+        near(product(ctx, epi, a, w, M, N, K, None, r), want, bound, epi)
+        c = torch.full((want.numel() + 1,), float("nan"), device=a.device, dtype=ctx.D)[1:]
+        torch.cuda.synchronize()
+        call = lambda: check(lib().cake_b200_debug_product(ctx.h, epi, ptr(a), ptr(w), None, ptr(r) if r is not None else None, ptr(c), M, N, K, 0, 0.0, None, 0, 0, None, 1))  # noqa: E731
+        if M > 256:
+            with pytest.raises(CakeB200Error, match="multiple of 16"):
+                call()
+            continue
+        call()
         near(c.view(want.shape), want, bound, (epi, "two bytes off"))
