@@ -199,6 +199,7 @@ struct cake_b200_ctx {
   uint32_t *mk_pk = nullptr;            // the megakernel's packets: xa, qkv, y, xb, mm
   uint64_t *mk_part = nullptr;          // and those of attention cut over several CTAs
   int mk_polls = MK_POLLS;              // what the waits of one of its threads may spend
+  int sk_tries = 0;                     // SkParams::tries
   MkLayer *mk_tab_dev = nullptr, *mk_tab_host = nullptr, *g_tab_dev = nullptr;
   std::vector<const void *> mk_sig;
   unsigned long long *trace = nullptr;  // CAKE_B200_MEGA_TRACE=1
@@ -1443,7 +1444,7 @@ static int gemm_tc_T(cake_b200_ctx *c, const void *A, const void *W, const void 
   if (plan_skinny(c->sm_count, M, N, K, x, &sk, &sk_smem, !aligned)) {
     sk.bias = bias; sk.residual = res; sk.C = C; sk.M = M; sk.N = N; sk.K = K; sk.ldc = ldc; sk.cap = cap;
     sk.act = act >= 0 ? act : (c->cfg.use_gelu_mlp ? 1 : 0);
-    sk.tile_group = x.tile_group; sk.row_scale = x.row_scale; sk.err = c->wait_err;
+    sk.tile_group = x.tile_group; sk.row_scale = x.row_scale; sk.err = c->wait_err; sk.tries = c->sk_tries;
     const bool vec = aligned && ldc % 4 == 0;
     CUtensorMap ma, mw;
     RC(make_tmap(&ma, A, (uint64_t)(x.a_shared ? sk.rows : M), (uint64_t)K, c->cfg.dtype, (uint32_t)sk.nt, (uint64_t)x.a_ld));
@@ -4325,6 +4326,11 @@ extern "C" int cake_b200_debug_packet_wait(cake_b200_ctx *c, int what, int fresh
     ok_host[i] = (int)c->h_pin[48 + i];
     kcycles[i] = (int)c->h_pin[48 + 2 + i];
   }
+  return CAKE_B200_OK;
+}
+extern "C" int cake_b200_debug_tries(cake_b200_ctx *c, int tries) {
+  if (!c || tries < 0 || tries > MBAR_TRIES) return fail(CAKE_B200_EINVAL, "bad debug_tries arguments");
+  c->sk_tries = tries;
   return CAKE_B200_OK;
 }
 extern "C" int cake_b200_debug_polls(cake_b200_ctx *c, int polls) {

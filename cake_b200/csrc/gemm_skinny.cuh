@@ -53,6 +53,7 @@ struct SkParams {
   int split, stages;
   int how;                   // SK_OVER, SK_APART or SK_LEAN
   int *err;                  // host-mapped: a wait that ran out
+  int tries;                 // 0, or (a test's) what a thread's waits may spend instead of MBAR_TRIES; those of a cluster's first CTA nothing
 };
 
 // What an epilogue reads beside the sums, four columns of row m of A from column n on (nothing where the row is not `in`)
@@ -157,7 +158,7 @@ __device__ __forceinline__ void sk_product(const CUtensorMap &map_w, const CUten
   }
   const bool live = group >= 0;  // cluster-uniform
   int issued = 0;                // warp 0: stages requested
-  int left = MBAR_TRIES;    // of this thread's waits
+  int left = !p.tries ? MBAR_TRIES : rank ? p.tries : 0;  // of this thread's waits
 
   if (warp == 0) {
     if (lane == 0 && live) {

@@ -154,3 +154,39 @@ def test_steps_after_one_whose_waits_ran_out(hidden, inter, heads, kv, hd):
             assert all(torch.equal(a, b) for a, b in zip(session(), want))
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("M,N,K,split", [(16, 6144, 4096, 8), (37, 4096, 1024, 4), (225, 1024, 4096, 4), (250, 2048, 4096, 4)])
+def test_sums_of_a_cluster_that_never_come(M, N, K, split):
+    """The first CTA of every cluster gives up at its first wait and sends nothing, the others wait for its sums until their tries are spent: all of them let what
+    is in flight end and leave, the call reports it, and the next product on the same context has the bits that it had before.  Sums received
+    behind the ring, over it, and with a share kept in tensor memory."""
+    from tests.test_products import SKINNY, plan
+    cfg = medium_config()
+    ctx = Context(cfg, checkpoint(cfg, "bf16", seed=3), "bf16")
+    V, I = ctypes.c_void_p, ctypes.c_int
+    fn, tries = lib().cake_b200_debug_product, lib().cake_b200_debug_tries
+    fn.argtypes = [V, I, V, V, V, V, V, I, I, I, I, ctypes.c_float, V, I, I, V, I]
+    tries.argtypes = [V, I]
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    if sms == 148:
+        assert plan(M, N, K, sms=sms)[:2] == (SKINNY, split)
+    g = torch.Generator(device="cuda:0").manual_seed(M)
+    a, w = (torch.randn(n, K, device="cuda:0", generator=g).bfloat16() for n in (M, N))
+
+    def product():
+        c = torch.zeros(M, N, device="cuda:0", dtype=torch.bfloat16)
+        torch.cuda.synchronize()
+        check(fn(ctx.h, 0, ptr(a), ptr(w), None, None, ptr(c), M, N, K, 0, 0.0, None, 0, 0, None, 1))
+        return c
+    try:
+        want = product()
+        for n in (1, 1024):
+            check(tries(ctx.h, n))
+            with pytest.raises(CakeB200Error, match="gave up a wait"):
+                product()
+            check(tries(ctx.h, 0))
+            for _ in range(3):
+                assert torch.equal(product(), want)
+    finally:
+        ctx.close()
