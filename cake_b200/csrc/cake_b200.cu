@@ -1869,22 +1869,18 @@ template <typename T> static int window_attention_tc(cake_b200_ctx *c, const Win
   return launch_pdl(c, attn_window_tc_kernel<T>, gt, dim3(FT_THREADS), (size_t)FT_SMEM_BYTES, mq, mk, mv, mpk, mpv, wp, fa_tau * 1.4426950408889634f);
 }
 template <> int window_attention_tc<float>(cake_b200_ctx *, const WinAttn &, int, uint64_t *, const void *, const void *, int) { return CAKE_B200_EINVAL; }
-// steps of a few tokens in 16-bit D with 16-byte rows: eight lanes per key (attn_window_decode_vec_kernel)
-// steps of a few tokens that attn_window_decode_vec_kernel takes
+// steps of a few tokens that attn_window_decode_vec_kernel takes: 16-bit D, rows of 16-byte pieces
 template <typename T> static bool listed_attention_in_vectors(const WinAttn &wa) {
   static const bool no_mma = []() { const char *e = getenv("CAKE_B200_NO_TC"); return e && e[0] == '1'; }();
   return sizeof(T) == 2 && !no_mma && wa.S <= 8 && wa.hd % 8 == 0 && wa.hd <= WA_MAX_HD && wa.ld % 8 == 0 && wa.kc == wa.vc && wa.gate_col >= -1 &&
          (((uintptr_t)wa.qkg | (uintptr_t)wa.kc) & 15) == 0;
 }
-template <typename T> static int listed_attention_vec(cake_b200_ctx *c, const WinAttn &wa, bool *done) {
-  *done = false;
-  if (!listed_attention_in_vectors<T>(wa)) return CAKE_B200_OK;
+template <typename T> static int listed_attention_vec(cake_b200_ctx *c, const WinAttn &wa) {
   // CTAs per item: while the chip has room and a group of lanes keeps four keys (its loads in flight): 16 heads of 1024 keys take four each
   const long items = (long)wa.B * wa.S * wa.heads, keys = wa.window > 0 ? std::min(wa.window, wa.pos0 + wa.S) : wa.pos0 + wa.S;
   int parts = 1;
   while (parts < WA_DEC_PARTS && keys >= 512l * parts && items * parts * 2 <= 2 * c->sm_count) parts *= 2;
   const dim3 grid((unsigned)(items * parts)), block(WA_DEC_WARPS * 32);
-  *done = true;
   switch ((wa.hd + 63) / 64) {
     case 1: return launch_cluster_pdl(c, attn_window_decode_vec_kernel<T, 1>, grid, block, 0, (unsigned)parts, wa);
     case 2: return launch_cluster_pdl(c, attn_window_decode_vec_kernel<T, 2>, grid, block, 0, (unsigned)parts, wa);
@@ -1892,8 +1888,15 @@ template <typename T> static int listed_attention_vec(cake_b200_ctx *c, const Wi
     default: return launch_cluster_pdl(c, attn_window_decode_vec_kernel<T, 4>, grid, block, 0, (unsigned)parts, wa);
   }
 }
-template <> int listed_attention_vec<float>(cake_b200_ctx *, const WinAttn &, bool *done) { *done = false; return CAKE_B200_OK; }
-template <typename T> static int listed_attention(cake_b200_ctx *c, const WinAttn &wa) {
+template <> int listed_attention_vec<float>(cake_b200_ctx *, const WinAttn &) { return CAKE_B200_EINVAL; }
+// The step's keys, columns k_col .. of wa.qkg, join the cache, and its queries attend to all of them.  The kernel for steps of a few tokens lays the keys down
+// itself; for every other one, which reads keys from the cache only, a kernel in front of it does.
+template <typename T> static int listed_attention(cake_b200_ctx *c, WinAttn wa, int k_col) {
+  if (listed_attention_in_vectors<T>(wa)) {  // (hd % 8 == 0: k_col, behind whole heads, is on 16 bytes too)
+    wa.k_col = k_col;
+    return listed_attention_vec<T>(c, wa);
+  }
+  RC(launch_pdl(c, rows_to_cache_kernel<T>, dim3(wa.B * wa.S), dim3(128), 0, (const T *)wa.qkg, (T *)const_cast<void *>(wa.kc), wa.S, wa.ld, k_col, wa.n_kv, wa.hd, wa.cap, wa.pos0));
   static const bool no_mma = []() { const char *e = getenv("CAKE_B200_NO_TC"); return e && e[0] == '1'; }();
   const long items = (long)wa.B * wa.S * wa.heads;
   if (wa.S >= 16 && !no_mma && wa.ld % 8 == 0 && wa.ldy % 2 == 0) {
@@ -1901,11 +1904,6 @@ template <typename T> static int listed_attention(cake_b200_ctx *c, const WinAtt
     RC(listed_attention_tc<T>(c, wa, &done));
     if (done) return CAKE_B200_OK;
     RC(listed_attention_mma<T>(c, wa, &done));
-    if (done) return CAKE_B200_OK;
-  }
-  if (wa.S <= 8) {
-    bool done = false;
-    RC(listed_attention_vec<T>(c, wa, &done));
     if (done) return CAKE_B200_OK;
   }
   if (wa.S <= 8) return launch_pdl(c, attn_window_decode_kernel<T>, dim3((unsigned)items), dim3(WA_DEC_WARPS * 32), 0, wa);
@@ -1953,14 +1951,10 @@ static int enqueue_listed_layers(cake_b200_ctx *c, cake_b200_block *const *block
       if (both) {
       } else if (in_tc) RC((listed_gemm_tc<T, TCE_PLAIN>(c, mix_in, b->w_in, nullptr, c->sp_in, M, b->n_in_pad, H, 0, 0)));
       else RC((gemm_rows_T<T, RE_STORE>(c, gi)));
-      // 3. the step's keys join the cache, then attention reads keys (= values) only from there; the kernel for steps of a few tokens lays them down itself
+      // 3. the step's keys (= values) join the cache, and attention
       WinAttn wa{c->sp_in, kc->k[l], kc->k[l], b->r1, b->r2, c->sp_a, B, S, sp.heads, sp.kv_heads, hd, kc->cap, pos0, b->n_in_pad, b->k_out,
                  b->gate_col, sp.window, sp.scale, sp.softcap};
-      if (listed_attention_in_vectors<T>(wa) && sq % 8 == 0) wa.k_col = sq;
-      else
-        RC(launch_pdl(c, rows_to_cache_kernel<T>, dim3(M), dim3(128), 0, (const T *)c->sp_in, (T *)kc->k[l], S, b->n_in_pad, sq, sp.kv_heads, hd,
-                      kc->cap, pos0));
-      RC(listed_attention<T>(c, wa));
+      RC(listed_attention<T>(c, wa, sq));
       // 4. the feed-forward's input half, where it has not been done yet
       if (sp.ff > 0 && !both) {
         RowsGemm gu{c->sp_h, b->wgu, nullptr, (T *)c->sp_a + sq, M, 2 * sp.ff, H, H, b->k_out, sp.act, 0.f};
