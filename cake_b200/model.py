@@ -259,6 +259,10 @@ class B200Transformer(Forwarder):
             pass
 
 
+# what a walk over local blocks asks them; TextModelBase passes it by for one token, where all of it is as defined here
+_LOCAL_METHODS = {"forward_batch": B200Transformer.forward_batch, "ident": B200Transformer.ident, "layer_name": B200Transformer.layer_name}
+
+
 class ListedBlock(B200Transformer):
     """A layer of a layer-list model (``Config.layers``; ``cake_b200_block_load_spec``): same Forwarder surface and the same
     ``cake_b200_forward_batch`` call as the Llama-family block, with an fp32 activation."""
@@ -569,9 +573,14 @@ class TextModelBase:
         return logits
 
     def _local_run(self):
-        """All blocks as one run of this process: (handles, cache slots, count), or None where a block lives elsewhere or is of another make."""
+        """All blocks as one run of this process: (handles, cache slots, count), or None where a block lives elsewhere, is of another make, or has a
+        method of its own or a wrapped one (a tracer's) on its class or on itself, which then is to be asked."""
         for cls in set(map(type, self.blocks)):
-            if not issubclass(cls, B200Transformer) or cls.forward_batch is not B200Transformer.forward_batch or cls.ident is not Forwarder.ident:
+            if not issubclass(cls, B200Transformer) or any(getattr(cls, name) is not own for name, own in _LOCAL_METHODS.items()):
+                return None
+        for blk in self.blocks:
+            own = blk.__dict__
+            if "forward_batch" in own or "ident" in own or "layer_name" in own:
                 return None
         if not self.blocks or self.ctx.cache is None or any([blk.h is None for blk in self.blocks]):
             return None

@@ -5,6 +5,7 @@ import pytest
 import torch
 
 from cake_b200.model import B200Transformer, Cache, Context, TextModelBase
+from tests.cpu_ctx import CpuContext, use_emulation
 from tests.util import checkpoint, medium_config
 
 
@@ -72,3 +73,44 @@ def test_threads_have_rows_of_their_own(model):
     t.join()
     model.ctx.sync()
     assert len({r.data_ptr() for pair in rows.values() for r in pair}) == 4
+
+
+@pytest.mark.parametrize("where", ["nowhere", "a block", "its class", "the base class", "a block's place", "a block's name"])
+def test_who_asks_a_block_is_not_passed_by(where, monkeypatch, tmp_path):
+    """A tracer on one block, on all blocks of a make, on where they say they live or what they are called: asked for the prompt, and for every token behind it."""
+    use_emulation(monkeypatch, tmp_path)
+    cfg = medium_config()
+    ctx = CpuContext(cfg, checkpoint(cfg, "bf16", seed=3), "bf16")
+    try:
+        m = TextModelBase.load(ctx)
+        asked = []
+
+        def traced(method):
+            def call(*args, **kw):
+                asked.append(method.__name__)
+                return method(*args, **kw)
+            return call
+
+        class Own(B200Transformer):
+            forward_batch = traced(B200Transformer.forward_batch)
+
+        first = m.blocks[0]
+        if where == "a block":
+            first.forward_batch = traced(first.forward_batch)
+        elif where == "its class":
+            first.__class__ = Own
+        elif where == "the base class":
+            monkeypatch.setattr(B200Transformer, "forward_batch", traced(B200Transformer.forward_batch))
+        elif where == "a block's place":
+            first.ident = traced(first.ident)
+        elif where == "a block's name":
+            first.layer_name = traced(first.layer_name)
+        assert (m._local_run() is None) == (where != "nowhere")
+        m.forward([[3, 5, 7]], 0)
+        per_call = len(asked)
+        assert bool(per_call) == (where != "nowhere")
+        for i in range(2):
+            m.forward([[9 + i]], 3 + i)
+        assert len(asked) == 3 * per_call
+    finally:
+        ctx.close()
