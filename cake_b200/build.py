@@ -42,6 +42,7 @@ def stale() -> bool:
 # translation units of the library: object file -> (source, the files it depends on besides itself; None = everything in csrc/)
 UNITS = {
     "cake_b200.o": ("cake_b200.cu", None),
+    "decode_mega.o": ("decode_mega.cu", ("decode_mega.cuh", "gemv.cuh", "attn_decode.cuh", "common.cuh")),
     "mixers.o": ("mixers.cu", ("mixers.cuh", "common.cuh")),
     "mixers_chunks.o": ("mixers_chunks.cu", ("mixers.cuh", "common.cuh")),
     "mixers_window.o": ("mixers_window.cu", ("mixers.cuh", "common.cuh")),

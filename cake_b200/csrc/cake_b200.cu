@@ -310,9 +310,6 @@ template <typename F> static inline int dispatch_T3(int dtype, F &&f) {
 #define DISPATCH_T(dtype, ...) dispatch_T((dtype), __VA_ARGS__)
 #define T_LAMBDA [&](auto tag_) -> int
 
-// (head_dim, query heads per kv head) combinations the megakernel is instantiated for
-#define MK_FOR_ALL(X) X(16, 2) X(16, 4) X(64, 2) X(64, 4) X(128, 1) X(128, 2) X(128, 4) X(128, 8)
-
 // ------------------------------------------------------------------------------------------ launch helper (PDL)
 template <typename... KArgs, typename... Args>
 static int launch_pdl(cake_b200_ctx *c, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, Args... args) {
@@ -423,11 +420,6 @@ template <typename T> static int set_smem_attrs_T() {
   CU(cudaFuncSetAttribute(attn_decode_kernel<T, HD>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
   SETB(16) SETB(32) SETB(64) SETB(128) SETB(256)
 #undef SETB
-#define SETC(HD, G)                                                                                                  \
-  CU(cudaFuncSetAttribute(decode_mega_kernel<T, HD, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxs - 4096));  \
-  CU(cudaFuncSetAttribute(decode_mega_kernel<T, HD, G>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
-  MK_FOR_ALL(SETC)
-#undef SETC
   CU(cudaFuncSetAttribute(attn_prefill_mma_kernel<T, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * FA_BN * 128 * 2));
   CU(cudaFuncSetAttribute(attn_prefill_mma_kernel<T, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * FA_BN * 64 * 2));
   CU(cudaFuncSetAttribute(attn_prefill_tc_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, FT_SMEM_BYTES));
@@ -567,6 +559,10 @@ extern "C" int cake_b200_ctx_create(int device, const cake_b200_config *cfg, cak
   CU(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
   RC(set_smem_attrs_T<__nv_bfloat16>());
   RC(set_smem_attrs_T<__half>());
+  if (const void *k = mk_kernel(cfg->dtype, cfg->head_dim, cfg->n_heads / cfg->n_kv_heads)) {
+    CU(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 4096));
+    CU(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+  }
   // RoPE tables -> D
   std::vector<float> cs, sn;
   rope_tables_host(*cfg, cs, sn, c->rot);
@@ -1134,11 +1130,7 @@ static bool plan_mega(const cake_b200_ctx *c, const cake_b200_cache *kc, int n_l
   const cake_b200_config &f = c->cfg;
   if (!c->use_mega || f.layer_list) return false;
   const int G = f.n_heads / f.n_kv_heads;
-  bool instance = false;
-#define MK_CASE(HD_, G_) instance = instance || (f.head_dim == HD_ && G == G_);
-  MK_FOR_ALL(MK_CASE)
-#undef MK_CASE
-  if (!instance) return false;
+  if (!mk_kernel(f.dtype, f.head_dim, G)) return false;
   MkArgs &a = p->a;
   memset(&a, 0, sizeof(a));
   a.max_k = f.hidden;
@@ -1181,18 +1173,6 @@ static bool plan_mega(const cake_b200_ctx *c, const cake_b200_cache *kc, int n_l
   return p->smem <= limit;
 }
 
-template <typename T> static int launch_mega_T(cake_b200_ctx *c, cudaLaunchConfig_t *cfg, const MkArgs &a) {
-  const int G = c->cfg.n_heads / c->cfg.n_kv_heads;
-#define MK_CASE(HD_, G_)                                                \
-  if (c->cfg.head_dim == HD_ && G == G_) {                              \
-    CU(cudaLaunchKernelEx(cfg, decode_mega_kernel<T, HD_, G_>, a));     \
-    return CAKE_B200_OK;                                                \
-  }
-  MK_FOR_ALL(MK_CASE)
-#undef MK_CASE
-  return fail(CAKE_B200_EINVAL, "megakernel: head_dim %d with %d query heads per kv head is not instantiated", c->cfg.head_dim, G);
-}
-
 static int launch_mega(cake_b200_ctx *c, const MkPlan &p) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(c->sm_count);
@@ -1213,11 +1193,11 @@ static int launch_mega(cake_b200_ctx *c, const MkPlan &p) {
   bool pool = false;
   for (int i = 0; a.n_layers && i < 4; i++) pool = pool || a.g[i].pool < a.g[i].n_groups;
   if (pool) CU(cudaMemsetAsync(c->tickets, 0, sizeof(unsigned) * 4 * (size_t)a.n_layers, c->stream));  // a memset node in the graph
-  int rc = DISPATCH_T(c->cfg.dtype, T_LAMBDA {
-    typedef typename decltype(tag_)::type T;
-    return launch_mega_T<T>(c, &cfg, a);
-  });
-  RC(rc);
+  const int G = c->cfg.n_heads / c->cfg.n_kv_heads;
+  const void *k = mk_kernel(c->cfg.dtype, c->cfg.head_dim, G);
+  if (!k) return fail(CAKE_B200_EINVAL, "megakernel: head_dim %d with %d query heads per kv head is not instantiated", c->cfg.head_dim, G);
+  void *args[1] = {(void *)&a};
+  CU(cudaLaunchKernelExC(&cfg, k, args));
   if (c->capturing) c->g_kernels++;
   else c->launches++;
   return CAKE_B200_OK;
@@ -4313,8 +4293,7 @@ extern "C" int cake_b200_debug_packet_wait(cake_b200_ctx *c, int what, int fresh
   if (!c || !ok_host || !kcycles || what < 0 || what > 3 || polls < 1 || polls > MK_POLLS) return fail(CAKE_B200_EINVAL, "bad debug_packet_wait arguments");
   CU(cudaSetDevice(c->device));
   CU(cudaStreamSynchronize(c->stream));
-  mk_wait_probe_kernel<<<1, MK_CT, 0, c->stream>>>(what, fresh, polls, c->wait_err, (int *)(c->h_pin + 48));
-  CU(cudaGetLastError());
+  CU(mk_wait_probe(c->stream, what, fresh, polls, c->wait_err, (int *)(c->h_pin + 48)));
   CU(cudaStreamSynchronize(c->stream));
   for (int i = 0; i < 2; i++) {
     ok_host[i] = (int)c->h_pin[48 + i];

@@ -1134,38 +1134,10 @@ __global__ void __launch_bounds__(MK_THREADS, 1) decode_mega_kernel(const __grid
   if (!a.has_head && blockIdx.x == 0 && ct == 0) mk_end_of_step(a, reinterpret_cast<const float *>(smem_raw + MK_OFF_SCRATCH));
 }
 
+// The decode kernel for a data type, head size and number of query heads per key head; nullptr: no instance (decode_mega.cu)
+const void *mk_kernel(int dtype, int head_dim, int group);
 // test aid: each kind of wait of the decode kernel on words of its own, twice by the same threads; fresh: what it waits for is there.
 // out[i]: whether wait i ended by that, out[2 + i]: its kcycles (thread 0)
-__global__ void __launch_bounds__(MK_CT) mk_wait_probe_kernel(int what, int fresh, int polls, int *err, int *out) {
-  __shared__ __nv_bfloat16 xs[4 * MK_CT];
-  __shared__ int gave_up;
-  alignas(16) static __device__ uint32_t words[4 * MK_CT];
-  const int ct = threadIdx.x;
-  const uint32_t tag = 7u;
-  if (what < 2) {   // packets with this tag, or the one in front
-    for (int i = ct; i < 4 * MK_CT; i += MK_CT) words[i] = what ? (fresh ? tag : tag - 1u) : (fresh ? tag : tag - 1u) << 16;
-  } else if (ct < 2) {
-    words[ct] = 0u;   // a counter
-  }
-  __threadfence();
-  __syncthreads();
-  MkWait w{polls, err};
-  for (int i = 0; i < 2; i++) {
-    if (ct == 0) gave_up = 0;
-    __syncthreads();
-    unsigned long long *const ctr = reinterpret_cast<unsigned long long *>(words);
-    const long long t0 = clock64();
-    if (what == 0) mk_gather<__nv_bfloat16>(xs, nullptr, words, 4 * MK_CT, tag << 16, ct, w);
-    else if (what == 1) pk_poll64(reinterpret_cast<uint64_t *>(words) + ct, tag, w);
-    else if (what == 2) mk_grid_sync(ctr, (unsigned long long)(i + 1) * (fresh ? 1ULL : 2ULL), ct, w);   // this CTA's arrival is the only one
-    else if (ct == 0) mk_inbox_wait(ctr, fresh ? 0ULL : 1ULL, w);
-    if (w.left <= 0) gave_up = 1;
-    __syncthreads();
-    if (ct == 0) {
-      out[i] = gave_up ? 0 : 1;
-      out[2 + i] = (int)((clock64() - t0) / 1000);
-    }
-  }
-}
+cudaError_t mk_wait_probe(cudaStream_t, int what, int fresh, int polls, int *err, int *out);
 
 }  // namespace cake
