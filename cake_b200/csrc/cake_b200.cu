@@ -3141,7 +3141,7 @@ template <typename Take> static MoeScratch moe_scratch(const cake_b200_ctx *c, c
   s.wts = (float *)take(nt * sizeof(float));
   s.sgate = (float *)take(M * sizeof(float));
   s.counts = (int *)take((mo.experts + 1) * sizeof(int));
-  s.perm = (int *)take(rows * sizeof(int));
+  if (s.tile != TC_BM) s.perm = (int *)take(rows * sizeof(int));  // (the kernels on the CUDA cores look up their rows; the products' are gathered)
   s.pos_of = (int *)take(nt * sizeof(int));
   s.tile_expert = (int *)take(s.max_tiles * sizeof(int));
   s.tile_rows = (int *)take(s.max_tiles * sizeof(int));

@@ -1376,7 +1376,7 @@ __global__ void moe_scatter_kernel(const int *ids, int n, int experts, int *curs
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n && ids[i] < experts) {
     const int pos = atomicAdd(&cursor[ids[i]], 1);
-    perm[pos] = i;
+    if (perm) perm[pos] = i;
     pos_of[i] = pos;
   }
 }
@@ -1386,7 +1386,7 @@ __global__ void __launch_bounds__(256) moe_plan_small_kernel(const MoePlan p) {
   pdl_wait();
   __shared__ int cnt[32 * MOE_MAX_SLOTS];
   __shared__ int done_s;
-  const int ne = p.M * p.top, rows = p.max_tiles * p.tile;
+  const int ne = p.M * p.top, rows = p.perm ? p.max_tiles * p.tile : 0;
   for (int e = threadIdx.x; e < p.experts; e += blockDim.x) cnt[e] = 0;
   for (int r = threadIdx.x; r < rows; r += blockDim.x) p.perm[r] = -1;
   __syncthreads();
@@ -1419,7 +1419,7 @@ __global__ void __launch_bounds__(256) moe_plan_small_kernel(const MoePlan p) {
   for (int i = threadIdx.x; i < ne; i += blockDim.x)
     if (p.ids[i] < p.experts) {
       const int pos = atomicAdd(&cnt[p.ids[i]], 1);
-      p.perm[pos] = i;
+      if (p.perm) p.perm[pos] = i;
       p.pos_of[i] = pos;
     }
 }
@@ -1431,7 +1431,7 @@ int moe_route(cudaStream_t st, int dtype, const MoePlan &p, uint64_t *launches) 
   if (p.logit_bias && !p.correction) return (int)cudaErrorInvalidValue;
   const int slots = (p.experts + p.identity + 31) / 32;
   if (p.by_token) {
-    if (p.experts < 1 || p.M > p.tile || p.M * p.top > MOE_SMALL_PAIRS) return (int)cudaErrorInvalidValue;
+    if (p.experts < 1 || p.perm || p.M > p.tile || p.M * p.top > MOE_SMALL_PAIRS) return (int)cudaErrorInvalidValue;
     MX_DISPATCH(dtype, {
       if (slots <= 1) mx_launch(st, moe_route_few_kernel<T, 1>, 1, 512, 0, p);
       else if (slots <= 2) mx_launch(st, moe_route_few_kernel<T, 2>, 1, 512, 0, p);
@@ -1453,7 +1453,7 @@ int moe_route(cudaStream_t st, int dtype, const MoePlan &p, uint64_t *launches) 
     n += 1;
   } else if (p.experts > 0) {
     cudaMemsetAsync(p.counts, 0, sizeof(int) * (p.experts + 1), st);
-    cudaMemsetAsync(p.perm, 0xff, sizeof(int) * (size_t)p.max_tiles * p.tile, st);
+    if (p.perm) cudaMemsetAsync(p.perm, 0xff, sizeof(int) * (size_t)p.max_tiles * p.tile, st);
     const int ne = p.M * p.top;
     mx_launch(st, moe_count_kernel, (ne + 255) / 256, 256, 0, p.ids, ne, p.experts, p.counts);
     mx_launch(st, moe_tiles_kernel, 1, 32, 0, p);

@@ -171,7 +171,7 @@ struct MoePlan {
   // grouping of the (token, slot) pairs by expert: every expert's pairs start on a multiple of `tile` sorted rows
   int tile;
   int *counts;           // [experts + 1] scratch
-  int *perm;             // [max_tiles * tile]: sorted row -> m * top + slot, or -1 (padding)
+  int *perm;             // [max_tiles * tile]: sorted row -> m * top + slot, or -1 (padding); nullptr where nobody asks (moe_gather goes by pos_of)
   int *pos_of;           // [M * top]: m * top + slot -> sorted row (pairs of identity experts: untouched)
   int *tile_expert;      // [max_tiles]: the expert of a block of `tile` sorted rows, or -1 (unused block)
   int max_tiles;
@@ -182,16 +182,17 @@ struct MoePlan {
   // score s may be chosen; plain_weights: the weights are the scores s (times scale), not renormalised.  correction may be nullptr
   int groups = 0, groups_keep = 0, plain_weights = 0;
   int sigmoid_scores = 0;  // 1: s = sigmoid(z) instead of the softmax
-  // 1: a block of `tile` rows per expert that any token chose (in order of the experts), where token m has row m: pos_of = block * tile + m; perm is not
-  // written.  M <= tile, at most MOE_SMALL_PAIRS pairs
+  // 1: a block of `tile` rows per expert that any token chose (in order of the experts), where token m has row m: pos_of = block * tile + m; perm has to be
+  // nullptr.  M <= tile, at most MOE_SMALL_PAIRS pairs
   int by_token = 0;
   int *tile_rows = nullptr;  // [max_tiles] or nullptr: rows of a block that are there (not by_token)
 };
 constexpr int MOE_SMALL_PAIRS = 1024;
 int moe_route(cudaStream_t, int dtype, const MoePlan &, uint64_t *launches);
 
-// sorted[r] = h[perm[r] / top] (zeros for padding rows): the operand of a grouped product on the tensor cores
-// (wts [M, top] != nullptr: times the pair's weight, rounded to D once)
+// sorted[pos_of[i]] = h[i / top] for every (token, slot) pair i of an expert: the operand of a grouped product on the tensor cores (wts [M, top] !=
+// nullptr: times the pair's weight, rounded to D once).  Rows that belong to no pair are not written, here nor by the products behind it: what lies there is of
+// an earlier call or nobody's, and must not be read.
 int moe_gather(cudaStream_t, int dtype, const void *h, const int *ids, const int *pos_of, int experts, void *sorted, int pairs, int W, int top, uint64_t *launches,
                const float *wts = nullptr);
 

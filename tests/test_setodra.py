@@ -436,6 +436,14 @@ def test_scratch_of_a_routed_feed_forward_holds_every_piece(hidden, experts, top
     check(fn(dtype, hidden, experts, 1, top, ff, shared, rows, out))
     asked, end, sums = out
     assert asked == end
+    tc, pairs, up = dtype != 2 and hidden % 128 == 0 and ff % 64 == 0 and experts > 0, rows * top, lambda n: (n + 255) // 256 * 256
+    tile, es = 128 if tc else 64, 4 if dtype == 2 else 2
+    tiles = -(-pairs // tile) + min(experts, pairs)
+    pieces = [rows * -(-(experts + 2) // 128) * 128 * 4, pairs * 4, pairs * 4, rows * 4, (experts + 1) * 4, pairs * 4, tiles * 4, tiles * 4, rows * shared * es]
+    if experts:
+        pieces += [tiles * tile * ff * es, tiles * tile * hidden * 4]
+    pieces += [tiles * tile * hidden * es] if tc else [tiles * tile * 4]   # gathered rows, or where each comes from: not both
+    assert end == sum(map(up, pieces)) + (up(rows * hidden * 4) if sums else 0)
     if dtype != 2 and shared and experts and hidden % 128 == 0 and ff % 64 == 0 and rows <= 64 and rows * top <= 1024:
         assert 0 < sums and sums + rows * hidden * 4 <= asked
     else:
@@ -444,12 +452,12 @@ def test_scratch_of_a_routed_feed_forward_holds_every_piece(hidden, experts, top
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", ["bf16", "f16"])
-@pytest.mark.parametrize("rows", [1, 16, 33, 64, 90, 260, 500])
+@pytest.mark.parametrize("rows", [1, 16, 33, 64, 90, 260, 500, 510])   # (510, three experts each: more than 1024 pairs are counted, planned and placed by kernels of their own)
 @pytest.mark.parametrize("shared", [0, 64, 320])
 def test_routed_feed_forward_at_any_number_of_rows(rows, shared, dtype):
     """Steps whose experts all multiply all rows, with no shared expert, one of a single k-block and one longer than the experts; and prompts whose blocks hold
     less than 64, up to 128 or more rows of an expert.  Some tokens choose an identity expert."""
-    cfg = make_config([retention(heads=2, dim=64, vdim=64, rot_dims=32, decay=[0.95, 0.99], moe=moe(experts=4, identity=1, top=2, ff=192, shared_ff=shared))], width=256, vocab=96)
+    cfg = make_config([retention(heads=2, dim=64, vdim=64, rot_dims=32, decay=[0.95, 0.99], moe=moe(experts=4, identity=1, top=3 if rows == 510 else 2, ff=192, shared_ff=shared))], width=256, vocab=96)
     sd = make_mixer_checkpoint(cfg, dtype, seed=59)
     toks = tokens(rows, cfg.vocab_size, seed=rows)
     r = Runner(cfg, sd, dtype)
