@@ -104,7 +104,7 @@ struct Recurrence {
   float *scratch = nullptr;  // recurrence_scratch() bytes, 16-byte aligned; nullptr: always token by token
 };
 int recurrence(cudaStream_t, int dtype, const Recurrence &, uint64_t *launches);
-// The form in chunks of tokens (mixers_chunks.cu); cudaErrorNotSupported for what it does not cover.  Three kernels of together 28 us or more against one
+// The form in chunks of tokens (mixers_chunks.cu); cudaErrorNotSupported for what it does not cover, factors per token and decays per channel among it.  Three kernels of together 28 us or more against one
 // that walks its tokens: 16 heads of 128 x 128 in us, walked / in chunks: 128 tokens 31 / 28, 256 59 / 28, 1000 223 / 74; 64 heads of 128 x 64:
 // 192 37 / 41, 256 49 / 41, 1000 181 / 126, 4 x 256 150 / 128.  So from 256 tokens on, whatever the batch.
 constexpr int CHUNK_MIN_TOKENS = 256;

@@ -108,10 +108,6 @@ template <typename T> __device__ __forceinline__ void ch_factors(const Recurrenc
       a = expf(-expf(DT<T>::to_f(reinterpret_cast<const T *>(p.a_log)[h])) * d);
       b = d;
     }
-    if (p.a_tok) {
-      a = p.a_tok[(m0 + t) * p.heads + h];
-      b = p.b_tok[(m0 + t) * p.heads + h];
-    }
   }
   as[t] = a;
   bs[t] = b;
@@ -368,7 +364,7 @@ template <typename T, int DK, bool ROPE> static cudaError_t launch_chunks(cudaSt
   return cudaGetLastError();
 }
 int recurrence_chunks(cudaStream_t st, int dtype, const Recurrence &p, int *n_launches) {
-  const int at_once = p.scratch && !p.a_chan && p.qscale == 1.f ? chunks_at_once(p.B, p.S, p.heads, p.dk, p.dv) : 0;
+  const int at_once = p.scratch && !p.a_chan && !p.a_tok && p.qscale == 1.f ? chunks_at_once(p.B, p.S, p.heads, p.dk, p.dv) : 0;
   const bool rope = p.cos_t && p.rope_dims > 0;
   const uintptr_t in_align = dtype == 2 ? 15 : 7;
   if (!at_once || (rope && p.rope_dims != p.dk) || p.ldq % 4 || p.ldk % 4 || p.ldv % 4 || (((uintptr_t)p.q | (uintptr_t)p.k | (uintptr_t)p.v) & in_align) ||

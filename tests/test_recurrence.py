@@ -23,7 +23,7 @@ def ctx(request):
 
 def inputs(ctx, form, B, S, H, dk, dv, group, pos0, seed=0):
     """What the three designs hand over: retention (fixed decays, rotation), a state-space layer (input-dependent decays, groups of heads that
-    share q and k, a skip), a matrix memory (factors per token)."""
+    share q and k, a skip; "forgetful": now and then a step so large that nothing of the tokens in front is left), a matrix memory (factors per token)."""
     g = torch.Generator(device="cuda:0").manual_seed(seed)
     rnd = lambda *s: torch.randn(*s, generator=g, device="cuda:0")  # noqa: E731
     q, k, v = rnd(B * S, H // group * dk).to(ctx.D), rnd(B * S, H // group * dk).to(ctx.D), rnd(B * S, H * dv).to(ctx.D)
@@ -33,8 +33,11 @@ def inputs(ctx, form, B, S, H, dk, dv, group, pos0, seed=0):
         f = 10000.0 ** (-torch.arange(dk // 2, device="cuda:0", dtype=torch.float64) * 2 / dk)
         a = torch.arange(pos0 + S, device="cuda:0", dtype=torch.float64)[:, None] * f
         d["cos"], d["sin"] = a.cos().float(), a.sin().float()
-    elif form == "ssd":
+    elif form in ("ssd", "forgetful"):
         d["dt"], d["dt_bias"], d["a_log"], d["skip"] = rnd(B * S, H).to(ctx.D), (rnd(H) * 0.7 - 1).to(ctx.D), (rnd(H) * 0.7 - 0.5).to(ctx.D), (rnd(H) * 0.2 + 1).to(ctx.D)
+        if form == "forgetful":
+            d["a_log"].clamp_(min=1.0)
+            d["dt"][::7] = 50.0   # a decay of exp(-50 e): 0 in fp32
     else:
         a = torch.rand(B * S, H, generator=g, device="cuda:0")
         a[::7] = 0.0   # a token that forgets everything in front of it
@@ -85,7 +88,7 @@ def rel(x, y):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("form,group,dk,dv", [("retention", 1, 128, 128), ("ssd", 4, 128, 64), ("factors", 1, 64, 64), ("ssd", 2, 64, 192)])
+@pytest.mark.parametrize("form,group,dk,dv", [("retention", 1, 128, 128), ("ssd", 4, 128, 64), ("forgetful", 1, 64, 64), ("ssd", 2, 64, 192)])
 @pytest.mark.parametrize("B,S,pos0", [(1, CHUNK_MIN, 0), (2, CHUNK_MIN + 1, 5), (1, 319, 0), (2, 320, 64), (1, 1000, 17)])
 def test_chunks_against_a_scan(ctx, form, group, dk, dv, B, S, pos0):
     H = 8
@@ -105,7 +108,7 @@ def test_chunks_against_a_scan(ctx, form, group, dk, dv, B, S, pos0):
 def test_states_held_at_once_are_bounded(ctx, B, launches):
     """A batch whose states don't all fit goes through the tokens in several passes (8 of 11 chunks, then 3), a large one walks them."""
     S, H, dk, dv = 700, 16, 128, 128
-    d = inputs(ctx, "factors", B, S, H, dk, dv, 1, 3, seed=1)
+    d = inputs(ctx, "ssd", B, S, H, dk, dv, 1, 3, seed=1)
     o1, s1, n1 = call(ctx, d, B, S, H, dk, dv, 1, 3, 1.0, 0)
     o2, s2, n2 = call(ctx, d, B, S, H, dk, dv, 1, 3, 1.0, 1)
     assert n1 == 1 and n2 == launches
@@ -115,8 +118,9 @@ def test_states_held_at_once_are_bounded(ctx, B, launches):
 @pytest.mark.gpu
 def test_an_infinity_reaches_no_token_in_front_of_it(ctx):
     S, H, dk, dv = 300, 4, 64, 64
-    d = inputs(ctx, "factors", 1, S, H, dk, dv, 1, 0, seed=2)
-    d["a_tok"].clamp_(min=0.1)
+    d = inputs(ctx, "ssd", 1, S, H, dk, dv, 1, 0, seed=2)
+    d["dt"].clamp_(max=1.0)
+    d["a_log"].clamp_(max=0.0)   # no decay below exp(-1.3): what follows keeps something of it
     o0, _, _ = call(ctx, d, 1, S, H, dk, dv, 1, 0, 1.0, 1)
     d["v"][133] = float("inf")
     o1, _, n = call(ctx, d, 1, S, H, dk, dv, 1, 0, 1.0, 1)
@@ -124,7 +128,7 @@ def test_an_infinity_reaches_no_token_in_front_of_it(ctx):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("what", ["few tokens", "key size", "value size", "row stride"])
+@pytest.mark.parametrize("what", ["few tokens", "key size", "value size", "row stride", "factors"])
 def test_what_chunks_do_not_cover_walks_the_tokens(ctx, what):
     S, H, dk, dv = 300, 4, 64, 64
     if what == "few tokens":
@@ -133,7 +137,7 @@ def test_what_chunks_do_not_cover_walks_the_tokens(ctx, what):
         dk = 96
     if what == "value size":
         dv = 32
-    d = inputs(ctx, "factors", 1, S, H, dk, dv, 1, 0, seed=3)
+    d = inputs(ctx, "factors" if what == "factors" else "ssd", 1, S, H, dk, dv, 1, 0, seed=3)
     if what == "row stride":
         d["v"] = torch.cat([d["v"], d["v"][:, :1]], 1)
     want, want_state = scan(dict(d, v=d["v"][:, :H * dv]), 1, S, H, dk, dv, 1, 0, 1.0)
