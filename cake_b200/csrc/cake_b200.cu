@@ -1673,10 +1673,11 @@ struct NormRows {
 };
 template <typename T> static int norm_rows(cake_b200_ctx *c, const NormRows &a) {
   const float eps = c->cfg.rms_eps;
-  if (sizeof(T) == 2 && a.n % 4 == 0 && a.n <= 16 * NORM_THREADS && (a.g_stride == 0 || a.g_stride == 1) && (!a.shift || a.S == 1) &&
-      (((uintptr_t)a.g | (uintptr_t)a.shift) & 7) == 0)
-    return launch_pdl(c, norm_rows_kernel<T>, dim3((unsigned)a.M), dim3(NORM_THREADS), 0, a.x, a.rows, a.row_mul, a.row_add, (const T *)a.g, a.g_stride, (const T *)a.shift,
-                      a.state_in, a.state_out, (T *)a.h, (T *)a.hs, a.n, eps, a.pos0, a.g_add);
+  if constexpr (sizeof(T) == 2) {
+    if (a.n % 4 == 0 && a.n <= 16 * NORM_THREADS && (a.g_stride == 0 || a.g_stride == 1) && (!a.shift || a.S == 1) && (((uintptr_t)a.g | (uintptr_t)a.shift) & 7) == 0)
+      return launch_pdl(c, norm_rows_kernel<T>, dim3((unsigned)a.M), dim3(NORM_THREADS), 0, a.x, a.rows, a.row_mul, a.row_add, (const T *)a.g, a.g_stride, (const T *)a.shift,
+                        a.state_in, a.state_out, (T *)a.h, (T *)a.hs, a.n, eps, a.pos0, a.g_add);
+  }
   return launch_pdl(c, norm_shift_rows_kernel<T>, dim3((unsigned)a.M), dim3(256), 0, a.x, a.rows, a.row_mul, a.row_add, (const T *)a.g, a.g_stride, (const T *)a.shift, a.state_in,
                     a.state_out, (T *)a.h, (T *)a.hs, a.S, a.n, eps, a.pos0, a.g_add);
 }

@@ -200,17 +200,16 @@ __global__ void __launch_bounds__(NORM_THREADS) norm_rows_kernel(const float *__
 #pragma unroll
   for (int i = 0; i < NORM_THREADS / 32; i++) tot += red[i];
   const float inv = 1.0f / sqrtf(tot / (float)n + eps);
-  typedef typename EmbedBits<T>::type B;
 #pragma unroll
   for (int e = 0; e < PER; e++) {
     const int i = threadIdx.x + NORM_THREADS * e;
     if (i >= n / 4) continue;
-    const float2 ga = DT<B>::unpack2(gr[e].x), gb = DT<B>::unpack2(gr[e].y);
+    const float2 ga = DT<T>::unpack2(gr[e].x), gb = DT<T>::unpack2(gr[e].y);
     const float gi[4] = {(g_stride ? ga.x : g0) + g_add, (g_stride ? ga.y : g0) + g_add, (g_stride ? gb.x : g0) + g_add, (g_stride ? gb.y : g0) + g_add};
     const float h[4] = {v[e].x * inv * gi[0], v[e].y * inv * gi[1], v[e].z * inv * gi[2], v[e].w * inv * gi[3]};
     if (h_out) store4<T>(h_out + (size_t)r * n + 4 * i, h[0], h[1], h[2], h[3]);
     if (shift) {
-      const float2 sa = DT<B>::unpack2(sr[e].x), sb = DT<B>::unpack2(sr[e].y);
+      const float2 sa = DT<T>::unpack2(sr[e].x), sb = DT<T>::unpack2(sr[e].y);
       store4<T>(hs_out + (size_t)r * n + 4 * i, h[0] + (u[e].x - h[0]) * sa.x, h[1] + (u[e].y - h[1]) * sa.y, h[2] + (u[e].z - h[2]) * sb.x, h[3] + (u[e].w - h[3]) * sb.y);
       *reinterpret_cast<float4 *>(state_out + (size_t)b * n + 4 * i) = make_float4(h[0], h[1], h[2], h[3]);
     }
