@@ -1337,8 +1337,8 @@ struct TcExtra {  // optional modes of the tensor-core GEMM (TcParams in gemm_tc
 // 4096 rows (one kernel after the other, weights from HBM; mostly within 15 %, the order of the three within 5 %).
 // gemm_tc: a launch with its last epilogue, the k-blocks of the first round (64 wide; the ring's round trip rather than its bytes: 128 x 128 with
 // six stages, 128 x 256 with four, 256 x 256 on a pair of SMs with six), and for every further round of tiles over the chip its k-blocks
-// or, where K is short, the epilogue of the tile in front.  The last round counts as a full one.  Fitted
-// when the epilogue had four warps; refitted to the eight it has, the choice came out worse where a model's products follow one another (a prompt of 250
+// or, where K is short, the epilogue of the tile in front.  The last round counts as a full one.  These are not the present kernel's times: they were fitted
+// when the epilogue had four warps.  What they choose is kept because it is the faster choice where both were timed; refitted to the eight it has, the choice came out worse where a model's products follow one another (a prompt of 250
 // tokens, 28 layers of 1024: 587 -> 606 us; 1500 tokens, layer-list blocks: 871 -> 891).  Small, wide, pairs in us, as fitted:
 //   N = 6144, K = 4096:  300 rows 25.0, 31.7, 29.7;  512 rows 45.5, 33.7, 31.6;  1000 rows 73.4, 62.2, 56.4
 //   N = 6144, K = 1024 (gated):  1000 rows 28.7, 34.2, 35.0;  1500 rows 35.2, 34.5, 36.3
@@ -1395,7 +1395,8 @@ static bool plan_skinny(int sms, int M, int N, int K, const TcExtra &x, SkParams
   if (x.w_live || x.b_kwrap || x.w_cols || x.w_rows || x.w_ld || x.batch > 1) return false;
   // Row tiles (a router: N = 128 for the most part): gemm_tc_kernel has a CTA per 128 rows and cuts nothing along K, eight CTAs for 1000 tokens (K = 2048: 15.0 ->
   // 10.6 us, three routed layers 1577 -> 1560; 260 tokens 1138 -> 1119).  Only where clusters of eight with four k-blocks each find room: at K = 1024 nothing is won
-  // (700 tokens 633 and 634), with clusters of two 4 x 1500 tokens took 6290 us and not 6190.
+  // (700 tokens 633 and 634), with clusters of two 4 x 1500 tokens took 6290 us and not 6190, and with clusters of four 1200 tokens 1789 and not 1801, but 1500 and
+  // 2200 what they take without (2032 and 2040, 2647 and 2658).
   const bool tiled = x.row_tiles && !x.tile_group && M > SK_MAX_ROWS;
   const int rows = x.tile_group ? x.group_rows : tiled ? TC_BM : M;
   if (rows < 1 || rows > (x.tile_group ? 64 : SK_MAX_ROWS)) return false;
